@@ -47,6 +47,7 @@ extern "C" {
 #define OF3_FLAG_OUTGOING 4    /* trimul: outgoing edges (else incoming) */
 #define OF3_FLAG_TRANSPOSED 8  /* triangle attention around the ending node */
 #define OF3_FLAG_ADA_LN 16     /* attention pair bias: adaptive LayerNorm conditioning on s */
+#define OF3_FLAG_NO_TRANSITION_MASK 32 /* blocks: the transitions ignore the mask (_mask_trans = False) */
 
 /* Message for the last non-zero return code seen by the calling thread. */
 const char* of3_last_error_string(void);
@@ -218,6 +219,45 @@ int of3_cond_transition_forward(const void* a, const void* s, const void* mask, 
                                 long long rows, int c_a, int c_s, int n, int dtype, int flags,
                                 const of3_cond_transition_params* p, void* workspace,
                                 size_t workspace_bytes, void* stream);
+
+/* ---- Whole blocks ------------------------------------------------------------------------
+ * One call per block instead of one per layer: the block's layers are enqueued by native code (a block of a short
+ * sequence is some thirty launches of a few microseconds, and issuing them one layer at a time from a scripting
+ * language takes longer than they run).
+ * of3_pair_block_forward replaces PairBlock.forward (openfold3/core/model/latent/base_blocks.py:406-480), in place on
+ * z [B, N, N, c_z]; pair_mask [B, N, N] or NULL.
+ * of3_pairformer_block_forward replaces PairFormerBlock.forward (openfold3/core/model/latent/pairformer.py:124-213), in
+ * place on z and s [B, N, c_s]; single_mask [B, N] or NULL. With side_stream != NULL (and widths for which the pair-bias
+ * projection has a kernel of its own: c_z = 128, 16 heads) the single track runs on side_stream behind the pair stack
+ * of the same block, so that it overlaps the pair stack of the next block: the caller makes side_stream wait for
+ * stream before the first block and stream wait for side_stream after the last one (of3_stream_wait), and gives the
+ * single track a workspace of its own. */
+typedef struct {
+    of3_trimul_params tri_mul_out, tri_mul_in;
+    of3_triattn_params tri_att_start, tri_att_end;
+    of3_transition_params pair_transition;
+} of3_pair_block_params;
+typedef struct {
+    of3_pair_block_params pair;
+    of3_attn_pair_bias_params attn;
+    of3_transition_params single_transition;
+} of3_pairformer_block_params;
+typedef struct {
+    int B, N, c_z, c_hidden_mul, no_heads_pair, c_hidden_pair_att, pair_transition_n;
+    int c_s, no_heads_single, c_hidden_single, single_transition_n;   /* unused by of3_pair_block_* */
+    float inf_pair, inf_single;
+} of3_block_dims;
+
+size_t of3_pair_block_workspace_bytes(const of3_block_dims* dims, int dtype, int flags);
+int of3_pair_block_forward(void* z, const void* pair_mask, const of3_block_dims* dims, int dtype, int flags,
+                           const of3_pair_block_params* p, void* workspace, size_t workspace_bytes, void* stream);
+size_t of3_pairformer_block_workspace_bytes(const of3_block_dims* dims, int dtype, int flags, int side);
+int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, const void* pair_mask,
+                                 const of3_block_dims* dims, int dtype, int flags, const of3_pairformer_block_params* p,
+                                 void* workspace, size_t workspace_bytes, void* side_workspace,
+                                 size_t side_workspace_bytes, void* stream, void* side_stream);
+/* Work enqueued on `waiter` from now on starts after everything enqueued on `signaler` so far. */
+int of3_stream_wait(void* waiter, void* signaler);
 
 /* ---- Row-sharded ("DAP") pair stack: phase entry points --------------------------------------
  * No counterpart in the reference (it has data-parallel DDP / ZeRO only;

@@ -1,11 +1,9 @@
 // extern "C" entry points: argument checks, kernel-family selection, workspace sizing.
 #include "modules.cuh"
 
-using namespace of3;
+namespace of3 {
 
-namespace {
-
-bool use_fast(int dtype, int flags) {
+static bool use_fast(int dtype, int flags) {
     return dtype == OF3_DTYPE_BF16 && !(flags & OF3_FLAG_FORCE_GENERIC);
 }
 
@@ -86,7 +84,9 @@ int cond_dispatch(const void* a, const void* s, const void* mask, void* out, lon
                                            (float*)out, rows, c_a, c_s, n, flags, p, ws, st);
 }
 
-}  // namespace
+}  // namespace of3
+
+using namespace of3;
 
 extern "C" {
 

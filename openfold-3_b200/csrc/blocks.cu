@@ -1,0 +1,185 @@
+// Whole blocks of the Pairformer behind one C call each: the same layer launches in the same order as the module entry
+// points of api.cu, issued by native code. A pair block is 13 launches and the single track of a block 9 more; from
+// Python, one layer call at a time, they cost about 13 us of host time each (400 us per block: the 4-block trunk at
+// N = 37 took 1.6 ms for 0.3 ms of device work, and so did N = 256).
+#include "generic_ops.cuh"
+#include "modules.cuh"
+#include "runtime.cuh"
+
+using namespace of3;
+
+namespace {
+
+// Layers of one stack call share the workspace: each starts at its beginning.
+struct Scratch {
+    void* base;
+    size_t cap;
+    size_t need = 0;
+    template <typename F>
+    int run(F&& f) {
+        Arena ws(base, cap);
+        const int rc = f(ws);
+        if (ws.off > need) need = ws.off;
+        return rc;
+    }
+};
+
+int pair_block(void* z, const void* mask, const of3_block_dims& D, int dtype, int flags, const of3_pair_block_params* p,
+               Scratch& ws, cudaStream_t st) {
+    const int f = (flags & OF3_FLAG_FORCE_GENERIC) | OF3_FLAG_ADD_RESIDUAL;
+    int rc;
+    if ((rc = ws.run([&](Arena& a) {
+             return trimul_dispatch(z, mask, z, D.B, D.N, D.c_z, D.c_hidden_mul, dtype, f | OF3_FLAG_OUTGOING,
+                                    &p->tri_mul_out, a, st);
+         })))
+        return rc;
+    if ((rc = ws.run([&](Arena& a) {
+             return trimul_dispatch(z, mask, z, D.B, D.N, D.c_z, D.c_hidden_mul, dtype, f, &p->tri_mul_in, a, st);
+         })))
+        return rc;
+    if ((rc = ws.run([&](Arena& a) {
+             return triattn_dispatch(z, mask, z, D.B, D.N, D.c_z, D.no_heads_pair, D.c_hidden_pair_att, D.inf_pair, dtype,
+                                     f, &p->tri_att_start, a, st);
+         })))
+        return rc;
+    if ((rc = ws.run([&](Arena& a) {
+             return triattn_dispatch(z, mask, z, D.B, D.N, D.c_z, D.no_heads_pair, D.c_hidden_pair_att, D.inf_pair, dtype,
+                                     f | OF3_FLAG_TRANSPOSED, &p->tri_att_end, a, st);
+         })))
+        return rc;
+    return ws.run([&](Arena& a) {
+        return transition_dispatch(z, (flags & OF3_FLAG_NO_TRANSITION_MASK) ? nullptr : mask, z,
+                                   (long long)D.B * D.N * D.N, D.c_z, D.pair_transition_n, dtype, f, &p->pair_transition, a,
+                                   st);
+    });
+}
+
+// How the single track gets its pair bias: projected ahead of it (bf16 bias tiles of the tensor-core attention, or an
+// fp32 tensor), or by the attention layer itself.
+enum BiasForm { kBiasInLayer, kBiasTiles, kBiasF32 };
+BiasForm bias_form(const of3_block_dims& D, int dtype, int flags) {
+    if (D.c_z != 128 || D.no_heads_single != 16 || (flags & OF3_FLAG_FORCE_GENERIC)) return kBiasInLayer;
+    if (dtype == OF3_DTYPE_BF16)
+        return fast::attn_pair_bias_supported(D.B, D.B, D.N, D.c_s, 0, D.c_z, D.no_heads_single, D.c_hidden_single, flags)
+                   ? kBiasTiles
+                   : kBiasInLayer;
+    return kBiasF32;
+}
+size_t bias_bytes(const of3_block_dims& D, BiasForm f) {
+    if (f == kBiasTiles) return (size_t)D.B * of3_pair_bias_tiles_elems(D.N) * sizeof(__nv_bfloat16);
+    return f == kBiasF32 ? (size_t)D.B * D.no_heads_single * D.N * D.N * sizeof(float) : 0;
+}
+
+int project_bias(const void* z, void* bias, const of3_block_dims& D, BiasForm form, const of3_attn_pair_bias_params* p,
+                 cudaStream_t st) {
+    if (form == kBiasTiles)
+        return fast::pair_bias_tiles_c128_h16((const __nv_bfloat16*)z, (const __nv_bfloat16*)p->ln_z_w,
+                                              (const __nv_bfloat16*)p->ln_z_b, (const __nv_bfloat16*)p->w_z,
+                                              (__nv_bfloat16*)bias, D.B, D.N, st);
+    return generic::pair_bias_c128_h16<float>((const float*)z, (const float*)p->ln_z_w, (const float*)p->ln_z_b,
+                                              (const float*)p->w_z, (float*)bias, D.B, (long long)D.N * D.N, st);
+}
+
+int single_track(void* s, const void* z, const void* bias, BiasForm form, const void* mask, const of3_block_dims& D,
+                 int dtype, int flags, const of3_pairformer_block_params* p, Scratch& ws, cudaStream_t st) {
+    const int f = (flags & OF3_FLAG_FORCE_GENERIC) | OF3_FLAG_ADD_RESIDUAL;
+    int rc = ws.run([&](Arena& a) {
+        if (form == kBiasTiles)
+            return fast::attn_pair_bias((const __nv_bfloat16*)s, nullptr, nullptr, (const __nv_bfloat16*)mask,
+                                        (__nv_bfloat16*)s, D.B, D.B, D.N, D.c_s, 0, D.no_heads_single, D.c_hidden_single,
+                                        D.inf_single, f, &p->attn, a, st, nullptr, (const __nv_bfloat16*)bias);
+        if (form == kBiasF32)
+            return generic::attn_pair_bias<float>((const float*)s, nullptr, nullptr, (const float*)mask, (float*)s, D.B,
+                                                  D.B, D.N, D.c_s, 0, D.c_z, D.no_heads_single, D.c_hidden_single,
+                                                  D.inf_single, f, &p->attn, a, st, (const float*)bias);
+        return apb_dispatch(s, z, nullptr, mask, s, D.B, D.B, D.N, D.c_s, 0, D.c_z, D.no_heads_single, D.c_hidden_single,
+                            D.inf_single, dtype, f, &p->attn, a, st);
+    });
+    if (rc) return rc;
+    return ws.run([&](Arena& a) {
+        return transition_dispatch(s, (flags & OF3_FLAG_NO_TRANSITION_MASK) ? nullptr : mask, s, (long long)D.B * D.N,
+                                   D.c_s, D.single_transition_n, dtype, f, &p->single_transition, a, st);
+    });
+}
+
+bool dims_ok(const of3_block_dims* d) {
+    return d && d->B > 0 && d->N > 0 && d->c_z > 0 && d->c_hidden_mul > 0 && d->no_heads_pair > 0 &&
+           d->c_hidden_pair_att > 0 && d->pair_transition_n > 0;
+}
+bool single_dims_ok(const of3_block_dims* d) {
+    return d->c_s > 0 && d->no_heads_single > 0 && d->c_hidden_single > 0 && d->single_transition_n > 0;
+}
+#define CHECK_BLOCK(what)                                                                                        \
+    OF3_REQUIRE(dtype == OF3_DTYPE_BF16 || dtype == OF3_DTYPE_F32, OF3_ERR_ARG, what ": bad dtype %d", dtype);    \
+    OF3_REQUIRE(dims_ok(dims), OF3_ERR_ARG, what ": non-positive size")
+
+}  // namespace
+
+extern "C" {
+
+int of3_stream_wait(void* waiter, void* signaler) {
+    return stream_wait((cudaStream_t)waiter, (cudaStream_t)signaler);
+}
+
+size_t of3_pair_block_workspace_bytes(const of3_block_dims* dims, int dtype, int flags) {
+    if (!dims_ok(dims)) return 0;
+    of3_pair_block_params p = {};
+    Scratch ws{nullptr, 0};
+    if (pair_block(nullptr, nullptr, *dims, dtype, flags, &p, ws, nullptr)) return 0;
+    return ws.need + 256;
+}
+
+int of3_pair_block_forward(void* z, const void* pair_mask, const of3_block_dims* dims, int dtype, int flags,
+                           const of3_pair_block_params* p, void* workspace, size_t workspace_bytes, void* stream) {
+    CHECK_BLOCK("pair_block");
+    OF3_REQUIRE(z && p && workspace, OF3_ERR_ARG, "pair_block: null pointer argument");
+    Scratch ws{workspace, workspace_bytes};
+    return pair_block(z, pair_mask, *dims, dtype, flags, p, ws, (cudaStream_t)stream);
+}
+
+// side = 0: the main stream's workspace: the largest layer, then the projected pair bias, which outlives the next
+// block's layers; side = 1: the single track's.
+size_t of3_pairformer_block_workspace_bytes(const of3_block_dims* dims, int dtype, int flags, int side) {
+    if (!dims_ok(dims) || !single_dims_ok(dims)) return 0;
+    of3_pairformer_block_params p = {};
+    Scratch ws{nullptr, 0};
+    const BiasForm form = bias_form(*dims, dtype, flags);
+    if (side) {
+        if (single_track(nullptr, nullptr, nullptr, form, nullptr, *dims, dtype, flags, &p, ws, nullptr)) return 0;
+        return ws.need + 256;
+    }
+    if (pair_block(nullptr, nullptr, *dims, dtype, flags, &p.pair, ws, nullptr)) return 0;
+    return align_up(ws.need, 256) + bias_bytes(*dims, form) + 256;
+}
+
+int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, const void* pair_mask,
+                                 const of3_block_dims* dims, int dtype, int flags, const of3_pairformer_block_params* p,
+                                 void* workspace, size_t workspace_bytes, void* side_workspace,
+                                 size_t side_workspace_bytes, void* stream, void* side_stream) {
+    CHECK_BLOCK("pairformer_block");
+    OF3_REQUIRE(single_dims_ok(dims), OF3_ERR_ARG, "pairformer_block: non-positive single-track size");
+    OF3_REQUIRE(s && z && p && workspace && side_workspace, OF3_ERR_ARG, "pairformer_block: null pointer argument");
+    cudaStream_t main = (cudaStream_t)stream;
+    const BiasForm form = bias_form(*dims, dtype, flags);
+    const size_t tail = bias_bytes(*dims, form);
+    OF3_REQUIRE(workspace_bytes >= tail, OF3_ERR_WORKSPACE, "pairformer_block: workspace too small");
+    const size_t head = (workspace_bytes - tail) / 256 * 256;
+    void* bias = (char*)workspace + head;
+    Scratch ws{workspace, head}, ws_side{side_workspace, side_workspace_bytes};
+    int rc;
+    if ((rc = pair_block(z, pair_mask, *dims, dtype, flags, &p->pair, ws, main))) return rc;
+    if (form == kBiasInLayer || side_stream == nullptr) {
+        if (form != kBiasInLayer && (rc = project_bias(z, bias, *dims, form, &p->attn, main))) return rc;
+        return single_track(s, z, bias, form, single_mask, *dims, dtype, flags, p, ws_side, main);
+    }
+    // The pair stack never reads s, so the single track (a chain of small, launch-bound kernels) runs on the side
+    // stream under the next block's pair stack. What it needs of z, the pair bias, is projected here, before the next
+    // block overwrites z, into the one bias buffer: behind the previous block's single track, which read it.
+    cudaStream_t side = (cudaStream_t)side_stream;
+    if ((rc = stream_wait(main, side))) return rc;
+    if ((rc = project_bias(z, bias, *dims, form, &p->attn, main))) return rc;
+    if ((rc = stream_wait(side, main))) return rc;
+    return single_track(s, nullptr, bias, form, single_mask, *dims, dtype, flags, p, ws_side, side);
+}
+
+}  // extern "C"

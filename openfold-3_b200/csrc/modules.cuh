@@ -94,6 +94,20 @@ int transition_wide(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bflo
                     int n, int flags, const of3_transition_params* p, Arena& ws, cudaStream_t st);
 }  // namespace fast
 
+// Kernel-family selection behind the module entry points (api.cu); with ws.base == nullptr they only measure the
+// workspace.
+int trimul_dispatch(const void* z, const void* mask, void* out, int B, int N, int c_z, int c_h, int dtype, int flags,
+                    const of3_trimul_params* p, Arena& ws, cudaStream_t st);
+int triattn_dispatch(const void* z, const void* mask, void* out, int B, int N, int c_z, int H, int d, float inf,
+                     int dtype, int flags, const of3_triattn_params* p, Arena& ws, cudaStream_t st);
+int transition_dispatch(const void* x, const void* mask, void* out, long long rows, int c, int n, int dtype, int flags,
+                        const of3_transition_params* p, Arena& ws, cudaStream_t st);
+int apb_dispatch(const void* a, const void* z, const void* s, const void* mask, void* out, int Ba, int Bz, int N,
+                 int c_a, int c_s, int c_z, int H, int d, float inf, int dtype, int flags,
+                 const of3_attn_pair_bias_params* p, Arena& ws, cudaStream_t st);
+int cond_dispatch(const void* a, const void* s, const void* mask, void* out, long long rows, int c_a, int c_s, int n,
+                  int dtype, int flags, const of3_cond_transition_params* p, Arena& ws, cudaStream_t st);
+
 int contract_nt_bf16(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, int batch,
                      int M, int N, int K, int lda, int ldb, int ldo, long long a_bs, long long b_bs,
                      long long o_bs, cudaStream_t stream, int rows_per_block = 0, long long row_block_stride = 0,

@@ -6,9 +6,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <memory>
 #include <mutex>
-#include <string>
-#include <unordered_map>
 #include <vector>
 
 namespace of3 {
@@ -53,6 +52,33 @@ int sm_count() {
     return g_sm_count[dev];
 }
 
+// An event is free again as soon as the wait on it is enqueued (a wait refers to the record before it), so each device
+// needs one per thread that is inside this function at the same time.
+static std::vector<cudaEvent_t> g_order_events[kMaxDevices];
+
+int stream_wait(cudaStream_t waiter, cudaStream_t signaler) {
+    int dev = 0;
+    OF3_CUDA_CHECK(cudaGetDevice(&dev));
+    OF3_REQUIRE(dev >= 0 && dev < kMaxDevices, OF3_ERR_ARG, "stream_wait: device %d", dev);
+    cudaEvent_t e = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (!g_order_events[dev].empty()) {
+            e = g_order_events[dev].back();
+            g_order_events[dev].pop_back();
+        }
+    }
+    if (e == nullptr) OF3_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    cudaError_t r = cudaEventRecord(e, signaler);
+    if (r == cudaSuccess) r = cudaStreamWaitEvent(waiter, e, 0);
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        g_order_events[dev].push_back(e);
+    }
+    OF3_CUDA_CHECK(r);
+    return OF3_OK;
+}
+
 static unsigned g_configured[kMaxDevices] = {0};
 
 bool device_configured(int key) {
@@ -90,11 +116,43 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-static std::unordered_map<std::string, CUtensorMap> g_tmaps;
-static const size_t kMaxCachedTmaps = 8192;
+// Encoded maps, per thread (no lock) and direct-mapped (bounded: callers with ever-new buffers replace old entries).
+// A launch needs up to five maps; looked up by string key in one locked hash table they cost about 1 us per launch.
+struct TmapKey {
+    uint64_t base, dims[5], strides[4], box[5];
+    int32_t rank, swizzle;
+};
+struct TmapEntry {
+    TmapKey key;
+    bool used;
+    CUtensorMap map;
+};
+static const unsigned kTmapSlots = 1024;
+static thread_local std::unique_ptr<TmapEntry[]> t_tmaps;
 
 int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                    const uint64_t* strides_bytes, const uint32_t* box, int swizzle) {
+    TmapKey key;
+    memset(&key, 0, sizeof(key));
+    key.base = (uint64_t)(uintptr_t)base;
+    key.rank = rank;
+    key.swizzle = swizzle;
+    for (int i = 0; i < rank; ++i) {
+        key.dims[i] = dims[i];
+        key.box[i] = box[i];
+        if (i > 0) key.strides[i - 1] = strides_bytes[i - 1];
+    }
+    uint64_t words[sizeof(TmapKey) / 8], h = 1469598103934665603ull;
+    static_assert(sizeof(TmapKey) % 8 == 0, "key of whole words");
+    memcpy(words, &key, sizeof(key));
+    for (uint64_t w : words) h = (h ^ w) * 1099511628211ull, h ^= h >> 29;
+    if (!t_tmaps) t_tmaps.reset(new TmapEntry[kTmapSlots]());
+    TmapEntry& e = t_tmaps[h % kTmapSlots];
+    // a tensor map holds no device state: the same arguments give the same 128 bytes on every device of the process
+    if (e.used && memcmp(&e.key, &key, sizeof(key)) == 0) {
+        *out = e.map;
+        return OF3_OK;
+    }
     EncodeTiledFn fn = encode_fn();
     OF3_REQUIRE(fn != nullptr, OF3_ERR_DRIVER, "cuTensorMapEncodeTiled entry point unavailable");
     OF3_REQUIRE(((uintptr_t)base & 15) == 0, OF3_ERR_ALIGN, "tensor map base not 16-byte aligned");
@@ -113,25 +171,6 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
             gstr[i - 1] = strides_bytes[i - 1];
         }
     }
-    // cache key: every argument of the encoding (a tensor map holds no device state: the same
-    // arguments give the same 128 bytes on every device of the process)
-    std::string key;
-    key.reserve(8 + 4 + rank * 20 + 4);
-    auto put = [&key](const void* p, size_t n) { key.append((const char*)p, n); };
-    put(&base, sizeof(base));
-    put(&rank, sizeof(rank));
-    put(gdim, rank * sizeof(cuuint64_t));
-    put(gstr, (rank - 1) * sizeof(cuuint64_t));
-    put(bx, rank * sizeof(cuuint32_t));
-    put(&swizzle, sizeof(swizzle));
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        auto it = g_tmaps.find(key);
-        if (it != g_tmaps.end()) {
-            *out = it->second;
-            return OF3_OK;
-        }
-    }
     CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base),
                     gdim, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     swizzle == 1 ? CU_TENSOR_MAP_SWIZZLE_128B
@@ -139,11 +178,9 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     OF3_REQUIRE(r == CUDA_SUCCESS, OF3_ERR_DRIVER, "cuTensorMapEncodeTiled failed with CUresult %d",
                 (int)r);
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        if (g_tmaps.size() >= kMaxCachedTmaps) g_tmaps.clear();  // bounded: callers with ever-new buffers
-        g_tmaps.emplace(std::move(key), *out);
-    }
+    e.key = key;
+    e.map = *out;
+    e.used = true;
     return OF3_OK;
 }
 

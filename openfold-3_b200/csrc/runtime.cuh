@@ -8,8 +8,8 @@ namespace of3 {
 
 // Encodes a tiled bf16 tensor map. dims/strides are innermost-first; strides_bytes has
 // rank-1 entries (stride of dim 1.., the innermost is dense). Returns OF3_OK or an error code.
-// swizzle: 0 none, 1 (or true) 128-byte, 2 64-byte. Encoded maps are kept in a locked cache keyed by
-// every argument, so a steady-state launch costs a lookup instead of a driver call per operand.
+// swizzle: 0 none, 1 (or true) 128-byte, 2 64-byte. Encoded maps are kept in a per-thread cache keyed
+// by every argument, so a steady-state launch costs a lookup instead of a driver call per operand.
 int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                    const uint64_t* strides_bytes, const uint32_t* box, int swizzle);
 
@@ -28,6 +28,9 @@ struct LaunchScope {
     LaunchScope(int kernel_id, cudaStream_t st);
     ~LaunchScope();
 };
+
+// Work enqueued on `waiter` from now on starts after everything enqueued on `signaler` so far.
+int stream_wait(cudaStream_t waiter, cudaStream_t signaler);
 
 // Number of SMs of the current device (cached per device).
 int sm_count();

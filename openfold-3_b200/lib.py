@@ -17,6 +17,7 @@ LIB_PATH = Path(__file__).resolve().parent / "libof3b200.so"
 
 DTYPE_BF16, DTYPE_F32 = 0, 1
 FLAG_ADD_RESIDUAL, FLAG_FORCE_GENERIC, FLAG_OUTGOING, FLAG_TRANSPOSED, FLAG_ADA_LN = 1, 2, 4, 8, 16
+FLAG_NO_TRANSITION_MASK = 32
 MODULE_TRIMUL, MODULE_TRIATTN, MODULE_TRANSITION = 1, 2, 3
 
 _lib = None
@@ -37,6 +38,22 @@ AttnPairBiasParams = _struct("AttnPairBiasParams", [
     "ln_z_w", "ln_z_b", "w_z", "w_q", "b_q", "w_k", "w_v", "w_g", "w_o"])
 CondTransitionParams = _struct("CondTransitionParams", [
     "ada_ln_s_w", "ada_w_g", "ada_b_g", "ada_w_s", "w_a", "w_b", "w_g", "b_g", "w_out"])
+
+
+class PairBlockParams(ctypes.Structure):
+    _fields_ = [("tri_mul_out", TrimulParams), ("tri_mul_in", TrimulParams), ("tri_att_start", TriattnParams),
+                ("tri_att_end", TriattnParams), ("pair_transition", TransitionParams)]
+
+
+class PairformerBlockParams(ctypes.Structure):
+    _fields_ = [("pair", PairBlockParams), ("attn", AttnPairBiasParams), ("single_transition", TransitionParams)]
+
+
+class BlockDims(ctypes.Structure):
+    _fields_ = [(n, c_int) for n in (
+        "B", "N", "c_z", "c_hidden_mul", "no_heads_pair", "c_hidden_pair_att", "pair_transition_n", "c_s",
+        "no_heads_single", "c_hidden_single", "single_transition_n")] + [("inf_pair", c_float), ("inf_single", c_float)]
+
 
 # name -> (restype, argtypes); the same list is checked against include/of3b200.h by the tests
 SIGNATURES = {
@@ -69,6 +86,14 @@ SIGNATURES = {
     "of3_cond_transition_forward": (c_int, [c_void_p] * 4 + [c_longlong, c_int, c_int, c_int, c_int, c_int,
                                             ctypes.POINTER(CondTransitionParams), c_void_p, c_size_t,
                                             c_void_p]),
+    "of3_pair_block_workspace_bytes": (c_size_t, [ctypes.POINTER(BlockDims), c_int, c_int]),
+    "of3_pair_block_forward": (c_int, [c_void_p] * 2 + [ctypes.POINTER(BlockDims), c_int, c_int,
+                                                        ctypes.POINTER(PairBlockParams), c_void_p, c_size_t, c_void_p]),
+    "of3_pairformer_block_workspace_bytes": (c_size_t, [ctypes.POINTER(BlockDims), c_int, c_int, c_int]),
+    "of3_pairformer_block_forward": (c_int, [c_void_p] * 4 + [ctypes.POINTER(BlockDims), c_int, c_int,
+                                                              ctypes.POINTER(PairformerBlockParams), c_void_p, c_size_t,
+                                                              c_void_p, c_size_t, c_void_p, c_void_p]),
+    "of3_stream_wait": (c_int, [c_void_p, c_void_p]),
     "of3_dap_pitch": (c_int, [c_int, c_int]),
     "of3_dap_triattn_image_elems": (c_longlong, [c_int, c_int]),
     "of3_dap_triattn_bias_elems": (c_longlong, [c_int, c_int]),
@@ -185,15 +210,17 @@ def dtype_code(dtype: torch.dtype) -> int:
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 
 
-def workspace(nbytes: int, device: torch.device) -> torch.Tensor:
-    """Grow-only scratch buffer per (device, stream); owned by torch, handed to the library per call."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
+def workspace(nbytes: int, device: torch.device, stream: torch.cuda.Stream | None = None) -> torch.Tensor:
+    """Grow-only scratch buffer per (device, stream; default the current one); owned by torch, handed to the library
+    per call."""
+    st = torch.cuda.current_stream(device) if stream is None else stream
+    key = (device.index if device.index is not None else torch.cuda.current_device(), st.cuda_stream)
     buf = _workspaces.get(key)
     if buf is None or buf.numel() < nbytes:
         buf = None
         _workspaces.pop(key, None)
-        buf = torch.empty(int(nbytes * 1.0) + 1024, dtype=torch.uint8, device=device)
+        with torch.cuda.stream(st):   # allocated on the stream that uses it
+            buf = torch.empty(int(nbytes * 1.0) + 1024, dtype=torch.uint8, device=device)
         _workspaces[key] = buf
     return buf
 
@@ -209,6 +236,44 @@ def _stream(device):
 def _require_cuda(t: torch.Tensor, name: str):
     if not t.is_cuda:
         raise RuntimeError(f"{name} must be a CUDA tensor: the B200 library has no CPU path")
+
+
+class BlockPlan:
+    """What the block entry points need besides the tensors of a call, for one shape: sizes and workspace bytes."""
+
+    __slots__ = ("dims", "ref", "bytes_main", "bytes_side", "bytes_pair")
+
+    def __init__(self, dims: BlockDims, dtype: int, flags: int, single: bool):
+        lib = load()
+        self.dims, self.ref = dims, ctypes.byref(dims)
+        self.bytes_pair = lib.of3_pair_block_workspace_bytes(self.ref, dtype, flags)
+        self.bytes_main = lib.of3_pairformer_block_workspace_bytes(self.ref, dtype, flags, 0) if single else 0
+        self.bytes_side = lib.of3_pairformer_block_workspace_bytes(self.ref, dtype, flags, 1) if single else 0
+
+
+def pair_block_forward(z, pair_mask, plan: BlockPlan, dtype: int, flags: int, params):
+    """One PairBlock in place on z [B, N, N, c_z]; params: a reference to PairBlockParams."""
+    ws = workspace(plan.bytes_pair, z.device)
+    _check(_lib.of3_pair_block_forward(z.data_ptr(), _ptr(pair_mask), plan.ref, dtype, flags, params, ws.data_ptr(),
+                                       ws.numel(), _stream(z.device)), "of3_pair_block_forward")
+
+
+def pairformer_block_forward(s, z, single_mask, pair_mask, plan: BlockPlan, dtype: int, flags: int, params, side=None):
+    """One PairFormerBlock in place on s [B, N, c_s] and z [B, N, N, c_z], the single track on the stream ``side``."""
+    ws = workspace(plan.bytes_main, z.device)
+    main = torch.cuda.current_stream(z.device)
+    if side is None:   # one stream, one after the other: but the pair bias lies in the first workspace
+        ws_side = torch.empty(plan.bytes_side, dtype=torch.uint8, device=z.device)
+    else:
+        ws_side = workspace(plan.bytes_side, z.device, side)
+    _check(_lib.of3_pairformer_block_forward(s.data_ptr(), z.data_ptr(), _ptr(single_mask), _ptr(pair_mask), plan.ref,
+                                             dtype, flags, params, ws.data_ptr(), ws.numel(), ws_side.data_ptr(),
+                                             ws_side.numel(), main.cuda_stream, None if side is None else side.cuda_stream),
+           "of3_pairformer_block_forward")
+
+
+def stream_wait(waiter, signaler):
+    _check(load().of3_stream_wait(waiter.cuda_stream, signaler.cuda_stream), "of3_stream_wait")
 
 
 def trimul_forward(z, mask, out, params, c_h: int, outgoing: bool, add_residual: bool):

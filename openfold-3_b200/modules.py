@@ -13,6 +13,7 @@ Forward only: autograd and training-mode dropout are not provided and raise.
 
 from __future__ import annotations
 
+import ctypes
 import math
 from functools import partialmethod
 
@@ -24,13 +25,32 @@ from . import lib
 
 
 # --------------------------------------------------------------------------- primitives
+_structure_epoch = 0   # counts changes of what a cached block plan was built from (submodules, parameters, constants)
+
+
+class _Tracked(nn.Module):
+    """Base of this package's modules: assigning a public attribute (a submodule, a parameter, a constant such as
+    ``inf``) makes the block plans built so far be built again. Values of parameters are checked at every call."""
+
+    def __setattr__(self, name, value):
+        if name[0] != "_":
+            global _structure_epoch
+            _structure_epoch += 1
+        super().__setattr__(name, value)
+
+    def __delattr__(self, name):
+        global _structure_epoch
+        _structure_epoch += 1
+        super().__delattr__(name)
+
+
 def _trunc_normal_(w: torch.Tensor, scale: float, fan: int):
     # variance-scaled truncated normal on [-2, 2] sigma; 0.8796... is the std of that truncation
     std = math.sqrt(scale / max(1, fan)) / 0.87962566103423978
     nn.init.trunc_normal_(w, mean=0.0, std=std, a=-2.0 * std, b=2.0 * std)
 
 
-class Linear(nn.Linear):
+class Linear(_Tracked, nn.Linear):
     """Parameter holder with the reference's named initialisers
     (openfold3/core/model/primitives/linear.py:38-138). Called alone it is a plain library GEMM."""
 
@@ -64,7 +84,7 @@ class Linear(nn.Linear):
                 raise ValueError("Invalid init string.")
 
 
-class LayerNorm(nn.Module):
+class LayerNorm(_Tracked):
     """Parameter holder (openfold3/core/model/primitives/normalization.py:33-86)."""
 
     def __init__(self, c_in: int, create_scale: bool = True, create_offset: bool = True, eps=1e-5):
@@ -81,7 +101,7 @@ class LayerNorm(nn.Module):
         return nn.functional.layer_norm(x, self.c_in, w, b, self.eps)
 
 
-class AdaLN(nn.Module):
+class AdaLN(_Tracked):
     """Parameter holder for adaptive LayerNorm
     (openfold3/core/model/primitives/normalization.py:89-140); the arithmetic is fused into
     the kernels of the modules that own it."""
@@ -95,7 +115,7 @@ class AdaLN(nn.Module):
         self.linear_s = Linear(c_s, c_a, **linear_init_params.linear_s)
 
 
-class SwiGLU(nn.Module):
+class SwiGLU(_Tracked):
     """Parameter holder (openfold3/core/model/primitives/activations.py:33-61)."""
 
     def __init__(self, c_in: int, c_out: int, linear_init_params=lin_init.swiglu_init):
@@ -105,7 +125,7 @@ class SwiGLU(nn.Module):
         self.linear_b = Linear(c_in, c_out, **linear_init_params.linear_b)
 
 
-class Attention(nn.Module):
+class Attention(_Tracked):
     """Parameter holder for gated multi-head attention
     (openfold3/core/model/primitives/attention.py:199-268). ``c_hidden`` is per head."""
 
@@ -122,7 +142,7 @@ class Attention(nn.Module):
             self.linear_g = Linear(c_q, c_hidden * no_heads, **linear_init_params.linear_g)
 
 
-class DropoutRowwise(nn.Module):
+class DropoutRowwise(_Tracked):
     """Identity in eval mode (openfold3/core/model/primitives/dropout.py:57-58); training-mode
     shared dropout is outside the forward-only scope."""
 
@@ -171,6 +191,68 @@ class _PackedParams:
         return self._val
 
 
+class _BlockPlans:
+    """A block's parameters as the native block entry point takes them, and its plans per shape.
+
+    ``get`` returns a reference to the parameter struct, rebuilt when a parameter has another address or version, or
+    the module tree another structure, than when it was built; ``None`` when the block has to take the layer-by-layer
+    path (hooks on its submodules, or a submodule that is not this package's)."""
+
+    def __init__(self):
+        self._epoch = -1
+        self._plans = {}
+
+    def __reduce__(self):   # a copied or unpickled module builds its own
+        return (_BlockPlans, ())
+
+    def _build(self, block, dtype, device):
+        self._epoch = _structure_epoch
+        self._hooks, self._ref, self._plans = [], None, {}
+        plain = block._plan_submodules()
+        if plain is None:
+            return
+        for m in plain:
+            self._hooks += [m._forward_hooks, m._forward_pre_hooks]
+        self._slots = [(m._parameters, n) for m in block.modules() for n, t in m._parameters.items() if t is not None]
+        self._dtype, self._device = dtype, device
+        tensors = [d[n] for d, n in self._slots]
+        self._ptrs, self._versions = [t.data_ptr() for t in tensors], [t._version for t in tensors]
+        self._struct, self._keep = block._native_params(dtype, device)
+        self._ref = ctypes.byref(self._struct)
+
+    def get(self, block, dtype, device):
+        if self._epoch == _structure_epoch and self._ref is not None and dtype == self._dtype and device == self._device:
+            try:
+                tensors = [d[n] for d, n in self._slots]
+                if [t.data_ptr() for t in tensors] == self._ptrs and [t._version for t in tensors] == self._versions:
+                    return None if any(self._hooks) else self._ref
+            except (KeyError, AttributeError, RuntimeError):   # replaced by something else, or without versions
+                return None
+        elif self._epoch == _structure_epoch and self._ref is None:
+            return None
+        self._build(block, dtype, device)
+        return None if any(self._hooks) else self._ref
+
+    def plan(self, block, B, N, dtype, flags):
+        p = self._plans.get((B, N, dtype, flags))
+        if p is None:
+            if len(self._plans) >= 64:
+                self._plans.clear()
+            p = self._plans[(B, N, dtype, flags)] = block._native_plan(B, N, dtype, flags)
+        return p
+
+
+def _native_state(block, z):
+    """(parameter reference, dtype code) for the native path of ``block`` on z [*, N, N, c], or None."""
+    if not z.is_cuda or block.training or z.dtype not in (torch.bfloat16, torch.float32):
+        return None
+    try:
+        ref = block._plans.get(block, z.dtype, z.device)
+    except RuntimeError:   # parameters that track no versions (inference tensors): nothing to key a plan on
+        return None
+    return None if ref is None else (ref, lib.dtype_code(z.dtype))
+
+
 def _mask_like(mask, shape, dtype):
     if mask is None:
         return None
@@ -178,7 +260,7 @@ def _mask_like(mask, shape, dtype):
 
 
 # --------------------------------------------------------------------------- triangle multiplication
-class TriangleMultiplicativeUpdate(nn.Module):
+class TriangleMultiplicativeUpdate(_Tracked):
     """AF3 Algorithms 12/13. Drop-in for
     openfold3/core/model/layers/triangular_multiplicative_update.py:123-503."""
 
@@ -226,7 +308,7 @@ class TriangleMultiplicationIncoming(TriangleMultiplicativeUpdate):
 
 
 # --------------------------------------------------------------------------- triangle attention
-class TriangleAttention(nn.Module):
+class TriangleAttention(_Tracked):
     """AF3 Algorithms 14/15. Drop-in for openfold3/core/model/layers/triangular_attention.py:30-179."""
 
     def __init__(self, c_in, c_hidden, no_heads, starting=True, inf=1e9, linear_init_params=lin_init.tri_att_init):
@@ -271,7 +353,7 @@ class TriangleAttentionEndingNode(TriangleAttention):
 
 
 # --------------------------------------------------------------------------- transitions
-class SwiGLUTransition(nn.Module):
+class SwiGLUTransition(_Tracked):
     """AF3 Algorithm 11. Drop-in for openfold3/core/model/layers/transition.py:225-271."""
 
     def __init__(self, c_in: int, n: int, linear_init_params=lin_init.swiglu_transition_init):
@@ -301,7 +383,7 @@ class SwiGLUTransition(nn.Module):
         return self._run(x, mask, in_place=False)
 
 
-class ConditionedTransitionBlock(nn.Module):
+class ConditionedTransitionBlock(_Tracked):
     """AF3 Algorithm 25. Drop-in for openfold3/core/model/layers/transition.py:274-380."""
 
     def __init__(self, c_a: int, c_s: int, n: int, linear_init_params=lin_init.cond_transition_init):
@@ -336,7 +418,7 @@ class ConditionedTransitionBlock(nn.Module):
 
 
 # --------------------------------------------------------------------------- attention with pair bias
-class AttentionPairBias(nn.Module):
+class AttentionPairBias(_Tracked):
     """AF3 Algorithm 24. Drop-in for openfold3/core/model/layers/attention_pair_bias.py:33-227."""
 
     def __init__(self, c_q, c_k, c_v, c_s, c_z, c_hidden, no_heads, use_ada_layer_norm=False, gating=True,
@@ -455,7 +537,7 @@ class AttentionPairBias(nn.Module):
 
 
 # --------------------------------------------------------------------------- blocks and stacks
-class PairBlock(nn.Module):
+class PairBlock(_Tracked):
     """Pair stack of one block. Drop-in for openfold3/core/model/latent/base_blocks.py:219-480."""
 
     def __init__(self, c_z, c_hidden_mul, c_hidden_pair_att, no_heads_pair, transition_type, transition_n,
@@ -477,6 +559,47 @@ class PairBlock(nn.Module):
         self.pair_transition = SwiGLUTransition(c_in=c_z, n=transition_n,
                                                 linear_init_params=linear_init_params.pair_transition.swiglu)
         self.ps_dropout_row_layer = DropoutRowwise(pair_dropout)
+        self._plans = _BlockPlans()
+
+    def _plan_submodules(self):
+        """The submodules whose hooks the layer-by-layer path runs, or None if one is not this package's own."""
+        own = {"tri_mul_out": TriangleMultiplicationOutgoing, "tri_mul_in": TriangleMultiplicationIncoming,
+               "tri_att_start": TriangleAttention, "tri_att_end": TriangleAttention, "pair_transition": SwiGLUTransition,
+               "ps_dropout_row_layer": DropoutRowwise}
+        if type(self) is not PairBlock or any(type(self._modules.get(n)) is not c for n, c in own.items()):
+            return None
+        dims = {(m.c_z, m.c_hidden) for m in (self.tri_mul_out, self.tri_mul_in)}
+        att = {(m.c_in, m.c_hidden, m.no_heads, m.inf) for m in (self.tri_att_start, self.tri_att_end)}
+        if len(dims) != 1 or len(att) != 1 or self.tri_mul_in._outgoing or not self.tri_mul_out._outgoing:
+            return None
+        if self.ps_dropout_row_layer.training:
+            return None
+        return [self.tri_mul_out, self.tri_mul_in, self.ps_dropout_row_layer]
+
+    def _native_params(self, dtype, device):
+        parts = [m._params(dtype, device) for m in (self.tri_mul_out, self.tri_mul_in, self.tri_att_start,
+                                                    self.tri_att_end, self.pair_transition)]
+        kinds = (lib.TrimulParams, lib.TrimulParams, lib.TriattnParams, lib.TriattnParams, lib.TransitionParams)
+        return lib.PairBlockParams(*[k(*[t.data_ptr() for t in p]) for k, p in zip(kinds, parts)]), parts
+
+    def _native_dims(self, B, N):
+        mul, att = self.tri_mul_out, self.tri_att_start
+        return lib.BlockDims(B=B, N=N, c_z=mul.c_z, c_hidden_mul=mul.c_hidden, no_heads_pair=att.no_heads,
+                             c_hidden_pair_att=att.c_hidden, pair_transition_n=self.pair_transition.n, inf_pair=att.inf)
+
+    def _native_plan(self, B, N, dtype, flags):
+        return lib.BlockPlan(self._native_dims(B, N), dtype, flags, single=False)
+
+    def _run_native(self, z, pair_mask, mask_trans):
+        """In place on the contiguous z with the prepared mask; False if the native path does not take this call."""
+        st = _native_state(self, z)
+        if st is None:
+            return False
+        N = z.shape[-2]
+        flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
+        plan = self._plans.plan(self, z.numel() // (N * N * z.shape[-1]), N, st[1], flags)
+        lib.pair_block_forward(z, pair_mask, plan, st[1], flags, st[0])
+        return True
 
     def tri_mul_out_in(self, z, pair_mask, inplace_safe, use_cueq_triangle_kernels=False):
         z = z if inplace_safe and z.is_contiguous() else z.clone(memory_format=torch.contiguous_format)
@@ -499,6 +622,9 @@ class PairBlock(nn.Module):
         _forward_only(self, z)
         self.ps_dropout_row_layer(z)  # raises in training mode with a non-zero rate
         z = z if inplace_safe and z.is_contiguous() else z.clone(memory_format=torch.contiguous_format)
+        pair_mask = _mask_like(pair_mask, z.shape[:-1], z.dtype)
+        if self._run_native(z, pair_mask, _mask_trans):
+            return z
         z = self.tri_mul_out_in(z, pair_mask, inplace_safe=True)
         z = self.tri_att_start_end(z, _attn_chunk_size, pair_mask, use_deepspeed_evo_attention,
                                    use_cueq_triangle_kernels, use_lma, inplace_safe=True)
@@ -506,7 +632,7 @@ class PairBlock(nn.Module):
         return z
 
 
-class PairFormerBlock(nn.Module):
+class PairFormerBlock(_Tracked):
     """Block of AF3 Algorithm 17. Drop-in for openfold3/core/model/latent/pairformer.py:38-213."""
 
     def __init__(self, c_s, c_z, c_hidden_pair_bias, no_heads_pair_bias, c_hidden_mul, c_hidden_pair_att,
@@ -524,11 +650,53 @@ class PairFormerBlock(nn.Module):
                                                 linear_init_params=linear_init_params.att_pair_bias)
         self.single_transition = SwiGLUTransition(c_in=c_s, n=transition_n,
                                                   linear_init_params=linear_init_params.transition)
+        self._plans = _BlockPlans()
+
+    def _plan_submodules(self):
+        own = {"pair_stack": PairBlock, "attn_pair_bias": AttentionPairBias, "single_transition": SwiGLUTransition}
+        if type(self) is not PairFormerBlock or any(type(self._modules.get(n)) is not c for n, c in own.items()):
+            return None
+        inner = self.pair_stack._plan_submodules()
+        if inner is None or self.attn_pair_bias.use_ada_layer_norm:
+            return None
+        return [self.pair_stack, *inner]
+
+    def _native_params(self, dtype, device):
+        pair, keep = self.pair_stack._native_params(dtype, device)
+        attn, trans = self.attn_pair_bias._params(dtype, device), self.single_transition._params(dtype, device)
+        ptr = lambda ts: [None if t is None else t.data_ptr() for t in ts]  # noqa: E731
+        return (lib.PairformerBlockParams(pair, lib.AttnPairBiasParams(*ptr(attn)), lib.TransitionParams(*ptr(trans))),
+                (keep, attn, trans))
+
+    def _native_plan(self, B, N, dtype, flags):
+        d, a = self.pair_stack._native_dims(B, N), self.attn_pair_bias
+        d.c_s, d.no_heads_single, d.c_hidden_single = a.c_q, a.no_heads, a.c_hidden
+        d.single_transition_n, d.inf_single = self.single_transition.n, a.inf
+        return lib.BlockPlan(d, dtype, flags, single=True)
+
+    def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None):
+        """In place on contiguous s and z with prepared masks; False if the native path does not take this call."""
+        st = _native_state(self, z)
+        N = z.shape[-2]
+        if st is None or s.dtype != z.dtype or s.shape[:-1] != z.shape[:-2]:
+            return False
+        flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
+        plan = self._plans.plan(self, z.numel() // (N * N * z.shape[-1]), N, st[1], flags)
+        lib.pairformer_block_forward(s, z, single_mask, pair_mask, plan, st[1], flags, st[0], side)
+        return True
 
     def forward(self, s, z, single_mask, pair_mask, chunk_size=None, use_deepspeed_evo_attention=False,
                 use_cueq_triangle_kernels=False, use_lma=False, inplace_safe=False, _mask_trans=True,
                 _attn_chunk_size=None):
         _forward_only(self, s, z)
+        if z.is_cuda and not self.training:
+            z = z if inplace_safe and z.is_contiguous() else z.clone(memory_format=torch.contiguous_format)
+            s = s if inplace_safe and s.is_contiguous() else s.clone(memory_format=torch.contiguous_format)
+            inplace_safe = True
+            pair_mask = _mask_like(pair_mask, z.shape[:-1], z.dtype)
+            single_mask = _mask_like(single_mask, s.shape[:-1], s.dtype)
+            if self._run_native(s, z, single_mask, pair_mask, _mask_trans):
+                return s, z
         z = self.pair_stack(z=z, pair_mask=pair_mask, chunk_size=chunk_size, inplace_safe=inplace_safe,
                             _mask_trans=_mask_trans, _attn_chunk_size=_attn_chunk_size)
         s = s if inplace_safe and s.is_contiguous() else s.clone(memory_format=torch.contiguous_format)
@@ -537,7 +705,7 @@ class PairFormerBlock(nn.Module):
         return s, z
 
 
-class PairFormerStack(nn.Module):
+class PairFormerStack(_Tracked):
     """AF3 Algorithm 17. Drop-in for openfold3/core/model/latent/pairformer.py:217-464."""
 
     def __init__(self, c_s, c_z, c_hidden_pair_bias, no_heads_pair_bias, c_hidden_mul, c_hidden_pair_att,
@@ -569,6 +737,9 @@ class PairFormerStack(nn.Module):
             z = z.clone(memory_format=torch.contiguous_format)
         if not (inplace_safe and s.is_contiguous()):
             s = s.clone(memory_format=torch.contiguous_format)
+        if z.is_cuda:   # prepared once for all blocks
+            pair_mask = _mask_like(pair_mask, z.shape[:-1], z.dtype)
+            single_mask = _mask_like(single_mask, s.shape[:-1], s.dtype)
         if not (self.overlap_single_track and z.is_cuda and len(self.blocks) > 1
                 and self.blocks[0].attn_pair_bias.can_hoist_pair_bias(z)):
             for b in self.blocks:
@@ -582,23 +753,23 @@ class PairFormerStack(nn.Module):
         side = self._side_streams.get(z.device)
         if side is None:
             side = self._side_streams[z.device] = torch.cuda.Stream(z.device)
-        side.wait_stream(main)
+        lib.stream_wait(side, main)
         for b in self.blocks:
+            if b._run_native(s, z, single_mask, pair_mask, _mask_trans, side):
+                continue
             z = b.pair_stack(z=z, pair_mask=pair_mask, chunk_size=chunk_size, inplace_safe=True,
                              _mask_trans=_mask_trans)
             bias = b.attn_pair_bias.project_pair_bias(z)
             bias.record_stream(side)   # allocated on the main stream, last read on the second one
-            ready = torch.cuda.Event()
-            ready.record(main)
+            lib.stream_wait(side, main)
             with torch.cuda.stream(side):
-                side.wait_event(ready)
                 b.attn_pair_bias._run(s, z, None, single_mask, in_place=True, pair_bias=bias)
                 b.single_transition._run(s, single_mask if _mask_trans else None, in_place=True)
-        main.wait_stream(side)
+        lib.stream_wait(main, side)
         return s, z
 
 
-class PairStack(nn.Module):
+class PairStack(_Tracked):
     """Consecutive ``PairBlock``s applied to one pair tensor: the "pair stack only" workloads. The reference has no
     class for it; its callers keep a ``nn.ModuleList`` of ``PairBlock``s and call them in sequence with the same
     pair mask (openfold3/core/model/latent/template_module.py:148-189), which is what ``forward`` does.
@@ -620,12 +791,14 @@ class PairStack(nn.Module):
         _forward_only(self, z)
         if not (inplace_safe and z.is_contiguous()):
             z = z.clone(memory_format=torch.contiguous_format)
+        if z.is_cuda:   # prepared once for all blocks
+            pair_mask = _mask_like(pair_mask, z.shape[:-1], z.dtype)
         for b in self.blocks:
             z = b(z, pair_mask, inplace_safe=True, _mask_trans=_mask_trans)
         return z
 
 
-class DiffusionTransformerBlock(nn.Module):
+class DiffusionTransformerBlock(_Tracked):
     """AF3 Algorithm 23 block. Drop-in for openfold3/core/model/layers/diffusion_transformer.py:30-179
     (the ``n_query is None`` token-level branch)."""
 
@@ -655,7 +828,7 @@ class DiffusionTransformerBlock(nn.Module):
         return a
 
 
-class DiffusionTransformer(nn.Module):
+class DiffusionTransformer(_Tracked):
     """AF3 Algorithm 23. Drop-in for openfold3/core/model/layers/diffusion_transformer.py:182-322."""
 
     def __init__(self, c_a, c_s, c_z, c_hidden, no_heads, no_blocks, n_transition, use_ada_layer_norm,
