@@ -22,6 +22,7 @@ class GraphedModule:
     """
 
     def __init__(self, fn, *example_args, warmup: int = 2):
+        self._fn = fn   # the graph reads what the function holds: its weights, a pair tensor it closes over
         self._static_in = [None if a is None else a.detach().clone() for a in example_args]
         if not all(a is None or a.is_cuda for a in self._static_in):
             raise ValueError("GraphedModule needs CUDA example arguments")
