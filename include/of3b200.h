@@ -165,11 +165,10 @@ int of3_transition_forward(const void* x, const void* mask, void* out, long long
  * a, out: [Ba, N, c_a]; z: [Bz, N, N, c_z] with Ba a multiple of Bz (samples sharing one pair
  * tensor are consecutive); s: [Ba, N, c_s] (AdaLN only, else NULL); mask: [Ba, N] or NULL.
  * out may alias a.
- * Launch grouping (bf16 kernels; an optimisation, never a requirement): linear layers that read the
- * same input run as ONE launch when their weights lie back to back in memory -- here w_q, w_g, w_k,
- * w_v in this order (w_g == w_q + H*d*c_a elements, ...) and ada_w_g, ada_w_s; in
- * of3_cond_transition_params ada_w_g, ada_w_s and w_a, w_b; in of3_transition_params w_a, w_b.
- * Otherwise each layer is its own launch, with the same result. */
+ * Launch grouping (bf16 kernels; an optimisation, never a requirement): the three projections of the conditioning run
+ * as ONE launch when their weights lie back to back in memory: here ada_w_g, ada_w_s, w_ada_out in this order
+ * (ada_w_s == ada_w_g + c_a*c_s elements, ...), in of3_cond_transition_params ada_w_g, ada_w_s, w_g. Otherwise each is
+ * its own launch, with the same result. */
 typedef struct {
     const void* ln_a_w;      /* [c_a] layer_norm_a.weight              (LayerNorm variant) */
     const void* ln_a_b;      /* [c_a] layer_norm_a.bias                (LayerNorm variant) */
@@ -256,6 +255,23 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
                                  const of3_block_dims* dims, int dtype, int flags, const of3_pairformer_block_params* p,
                                  void* workspace, size_t workspace_bytes, void* side_workspace,
                                  size_t side_workspace_bytes, void* stream, void* side_stream);
+/* of3_diffusion_stack_forward replaces the block loop of DiffusionTransformer.forward (openfold3/core/model/layers/
+ * diffusion_transformer.py:263-322, 116-179), in place on a [Ba, N, c_a]: per block attention with pair bias (AdaLN
+ * variant with OF3_FLAG_ADA_LN), then the conditioned transition. s [Ba, N, c_s]; z [Bz, N, N, c_z] (Ba a multiple of
+ * Bz, samples that share a pair tensor consecutive), or bias[block]: the blocks' pair biases, projected earlier
+ * (of3_pair_bias_project_tiles for the bf16 tensor-core attention, else of3_pair_bias_project), and z NULL.
+ * The projections of s are computed for several blocks per launch when those of all layers lie back to back:
+ * [block][attention, transition][gate, shift, output gate][c_a][c_s]. */
+typedef struct {
+    int Ba, Bz, N, c_a, c_s, c_z, H, d, n;
+    float inf;
+} of3_diffusion_dims;
+size_t of3_diffusion_stack_workspace_bytes(const of3_diffusion_dims* dims, int dtype, int flags, int blocks,
+                                           int with_bias);
+int of3_diffusion_stack_forward(void* a, const void* s, const void* z, const void* mask, const void* const* bias,
+                                const of3_diffusion_dims* dims, int dtype, int flags, int blocks,
+                                const of3_attn_pair_bias_params* attn, const of3_cond_transition_params* transition,
+                                void* workspace, size_t workspace_bytes, void* stream);
 /* Work enqueued on `waiter` from now on starts after everything enqueued on `signaler` so far. */
 int of3_stream_wait(void* waiter, void* signaler);
 

@@ -1,7 +1,8 @@
 """Builds the C-ABI CUDA library (sm_100a only) in-tree with nvcc.
 
 The library is a plain shared object (``extern "C"`` entry points, raw pointers and sizes);
-it does not link against torch. ``build()`` recompiles only translation units whose sources
+it does not link against torch. Beside it stands a small CPython extension that does: it reads
+the addresses and versions of a module's parameters. ``build()`` recompiles only translation units whose sources
 (or headers) are newer than their object files.
 """
 
@@ -10,6 +11,7 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -18,6 +20,8 @@ CSRC = PKG_DIR / "csrc"
 OBJ_DIR = PKG_DIR / "build"
 LIB_PATH = PKG_DIR / "libof3b200.so"
 INCLUDE_DIR = PKG_DIR.parent / "include"
+WATCH_SRC = CSRC / "host" / "param_watch.cpp"
+WATCH_PATH = PKG_DIR / ("_param_watch" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 NVCC_FLAGS = [
     "-gencode",
@@ -48,11 +52,28 @@ def _stale(obj: Path, src: Path, headers: list[Path]) -> bool:
     return any(p.stat().st_mtime > t for p in [src, *headers])
 
 
+def _build_watch(force: bool) -> None:
+    if not force and not _stale(WATCH_PATH, WATCH_SRC, []):
+        return
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", str(WATCH_SRC), "-o", str(WATCH_PATH),
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", str(root / "include"), "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"),
+           "-I", sysconfig.get_paths()["include"], "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10",
+           f"-Wl,-rpath,{root / 'lib'}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compile every ``csrc/*.cu`` for sm_100a and link ``libof3b200.so``. Returns its path."""
     OBJ_DIR.mkdir(exist_ok=True)
     headers = sorted(CSRC.glob("*.cuh")) + sorted(INCLUDE_DIR.glob("*.h"))
     nvcc = _nvcc()
+    _build_watch(force)
     jobs = []
     objs = []
     for src in sources():

@@ -1,10 +1,13 @@
-// Whole blocks of the Pairformer behind one C call each: the same layer launches in the same order as the module entry
-// points of api.cu, issued by native code. A pair block is 13 launches and the single track of a block 9 more; from
+// Whole blocks of the Pairformer, and the whole diffusion token stack, behind one C call each: the same layers in the
+// same order as the module entry points of api.cu, issued by native code. A pair block is 13 launches and the single track of a block 9 more; from
 // Python, one layer call at a time, they cost about 13 us of host time each (400 us per block: the 4-block trunk at
 // N = 37 took 1.6 ms for 0.3 ms of device work, and so did N = 256).
+#include "fast_single.cuh"
 #include "generic_ops.cuh"
 #include "modules.cuh"
 #include "runtime.cuh"
+
+#include <vector>
 
 using namespace of3;
 
@@ -102,6 +105,99 @@ int single_track(void* s, const void* z, const void* bias, BiasForm form, const 
     });
 }
 
+// ---------------------------------------------------------------- diffusion token stack
+// Room for the conditioning projections of one group of blocks. s is the same for all blocks, so a launch can cover
+// several of them: with few rows the projections of one block (6 matrices of c_a x c_s) fill a fraction of the chip and
+// cost a launch each; with many rows one block fills it, and its planes should stay in L2 until they are read.
+constexpr size_t kCondGroupBytes = 32u << 20;
+
+int diffusion_stack(void* a, const void* s, const void* z, const void* mask, const void* const* bias,
+                    const of3_diffusion_dims& D, int dtype, int flags, int blocks, const of3_attn_pair_bias_params* pa,
+                    const of3_cond_transition_params* pt, Scratch& ws, cudaStream_t st) {
+    typedef __nv_bfloat16 bf16;
+    const int f = (flags & (OF3_FLAG_FORCE_GENERIC | OF3_FLAG_ADA_LN)) | OF3_FLAG_ADD_RESIDUAL;
+    const long long rows = (long long)D.Ba * D.N;
+    const void* tmask = (flags & OF3_FLAG_NO_TRANSITION_MASK) ? nullptr : mask;
+    const bool fast_attn = dtype == OF3_DTYPE_BF16 &&
+                           fast::attn_pair_bias_supported(D.Ba, D.Bz, D.N, D.c_a, D.c_s, D.c_z, D.H, D.d, f);
+    const bool fast_trans = dtype == OF3_DTYPE_BF16 && fast::cond_transition_supported(D.c_a, D.c_s, D.n, f);
+    int rc;
+    if (!(fast_attn && fast_trans && (flags & OF3_FLAG_ADA_LN))) {
+        for (int b = 0; b < blocks; ++b) {
+            rc = ws.run([&](Arena& A) {
+                if (bias != nullptr && fast_attn)
+                    return fast::attn_pair_bias((const bf16*)a, nullptr, (const bf16*)s, (const bf16*)mask, (bf16*)a, D.Ba,
+                                                D.Bz, D.N, D.c_a, D.c_s, D.H, D.d, D.inf, f, pa + b, A, st, nullptr,
+                                                (const bf16*)bias[b]);
+                if (bias != nullptr && dtype == OF3_DTYPE_F32)
+                    return generic::attn_pair_bias<float>((const float*)a, nullptr, (const float*)s, (const float*)mask,
+                                                          (float*)a, D.Ba, D.Bz, D.N, D.c_a, D.c_s, D.c_z, D.H, D.d,
+                                                          D.inf, f, pa + b, A, st, (const float*)bias[b]);
+                if (bias != nullptr)
+                    return generic::attn_pair_bias<bf16>((const bf16*)a, nullptr, (const bf16*)s, (const bf16*)mask,
+                                                         (bf16*)a, D.Ba, D.Bz, D.N, D.c_a, D.c_s, D.c_z, D.H, D.d, D.inf,
+                                                         f, pa + b, A, st, (const float*)bias[b]);
+                return apb_dispatch(a, z, s, mask, a, D.Ba, D.Bz, D.N, D.c_a, D.c_s, D.c_z, D.H, D.d, D.inf, dtype, f,
+                                    pa + b, A, st);
+            });
+            if (rc) return rc;
+            rc = ws.run([&](Arena& A) {
+                return cond_dispatch(a, s, tmask, a, rows, D.c_a, D.c_s, D.n, dtype, f & ~OF3_FLAG_ADA_LN, pt + b, A, st);
+            });
+            if (rc) return rc;
+        }
+        return OF3_OK;
+    }
+    const size_t per_block = (size_t)rows * 6 * D.c_a * sizeof(bf16);
+    int group = per_block ? (int)(kCondGroupBytes / per_block) : 1;
+    if (group < 1) group = 1;
+    if (group > blocks) group = blocks;
+    if (group > fast::kMaxCondBatch / 2) group = fast::kMaxCondBatch / 2;
+    return ws.run([&](Arena& A) -> int {
+        bf16* planes = (bf16*)A.take(group * per_block);
+        bf16* sn = (bf16*)A.take((size_t)(2 * group + 1) * rows * D.c_s * sizeof(bf16));
+        const size_t mark = A.off;
+        size_t need = A.off;
+        for (int b0 = 0; b0 < blocks; b0 += group) {
+            const int nb = blocks - b0 < group ? blocks - b0 : group;
+            if (A.base) {
+                OF3_REQUIRE(A.ok(), OF3_ERR_WORKSPACE, "diffusion stack: workspace too small (%zu needed)", A.off);
+                fast::CondLayer layer[fast::kMaxCondBatch];
+                for (int i = 0; i < nb; ++i) {
+                    layer[2 * i] = fast::cond_layer(pa + b0 + i);
+                    layer[2 * i + 1] = fast::cond_layer(pt + b0 + i);
+                }
+                const int rc = fast::conditioning((const bf16*)s, layer, 2 * nb, rows, D.c_a, D.c_s, sn, planes, st);
+                if (rc) return rc;
+            }
+            for (int i = 0; i < nb; ++i) {
+                const int b = b0 + i;
+                const bf16* cond = planes ? planes + (size_t)i * 6 * rows * D.c_a : (const bf16*)256;
+                A.off = mark;
+                int rc = fast::attn_pair_bias((const bf16*)a, (const bf16*)z, (const bf16*)s, (const bf16*)mask, (bf16*)a,
+                                              D.Ba, D.Bz, D.N, D.c_a, D.c_s, D.H, D.d, D.inf, f, pa + b, A, st, nullptr,
+                                              bias ? (const bf16*)bias[b] : nullptr, cond);
+                if (rc) return rc;
+                need = A.off > need ? A.off : need;
+                A.off = mark;
+                rc = fast::cond_transition((const bf16*)a, (const bf16*)s, (const bf16*)tmask, (bf16*)a, rows, D.c_a, D.c_s,
+                                           D.n, f, pt + b, A, st, planes ? cond + 3 * rows * D.c_a : cond);
+                if (rc) return rc;
+                need = A.off > need ? A.off : need;
+                if (!A.base) break;   // sizing: the blocks are alike
+            }
+            if (!A.base) break;
+        }
+        A.off = need;
+        return OF3_OK;
+    });
+}
+
+bool diffusion_dims_ok(const of3_diffusion_dims* d) {
+    return d && d->Ba > 0 && d->Bz > 0 && d->Ba % d->Bz == 0 && d->N > 0 && d->c_a > 0 && d->c_s > 0 && d->c_z > 0 &&
+           d->H > 0 && d->d > 0 && d->n > 0;
+}
+
 bool dims_ok(const of3_block_dims* d) {
     return d && d->B > 0 && d->N > 0 && d->c_z > 0 && d->c_hidden_mul > 0 && d->no_heads_pair > 0 &&
            d->c_hidden_pair_att > 0 && d->pair_transition_n > 0;
@@ -145,7 +241,8 @@ size_t of3_pairformer_block_workspace_bytes(const of3_block_dims* dims, int dtyp
     Scratch ws{nullptr, 0};
     const BiasForm form = bias_form(*dims, dtype, flags);
     if (side) {
-        if (single_track(nullptr, nullptr, nullptr, form, nullptr, *dims, dtype, flags, &p, ws, nullptr)) return 0;
+        // a bias pointer that is never read: the projected form takes no room here
+        if (single_track(nullptr, nullptr, form == kBiasTiles ? (const void*)256 : nullptr, form, nullptr, *dims, dtype, flags, &p, ws, nullptr)) return 0;
         return ws.need + 256;
     }
     if (pair_block(nullptr, nullptr, *dims, dtype, flags, &p.pair, ws, nullptr)) return 0;
@@ -180,6 +277,31 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
     if ((rc = project_bias(z, bias, *dims, form, &p->attn, main))) return rc;
     if ((rc = stream_wait(side, main))) return rc;
     return single_track(s, nullptr, bias, form, single_mask, *dims, dtype, flags, p, ws_side, side);
+}
+
+size_t of3_diffusion_stack_workspace_bytes(const of3_diffusion_dims* dims, int dtype, int flags, int blocks,
+                                           int with_bias) {
+    if (!diffusion_dims_ok(dims) || blocks <= 0) return 0;
+    Scratch ws{nullptr, 0};
+    const std::vector<of3_attn_pair_bias_params> pas(blocks, of3_attn_pair_bias_params{});
+    const std::vector<of3_cond_transition_params> pts(blocks, of3_cond_transition_params{});
+    const std::vector<const void*> bias(blocks, (const void*)256);   // never read: says that the bias takes no room here
+    if (diffusion_stack(nullptr, nullptr, nullptr, nullptr, with_bias ? bias.data() : nullptr, *dims, dtype, flags, blocks,
+                        pas.data(), pts.data(), ws, nullptr))
+        return 0;
+    return ws.need + 256;
+}
+
+int of3_diffusion_stack_forward(void* a, const void* s, const void* z, const void* mask, const void* const* bias,
+                                const of3_diffusion_dims* dims, int dtype, int flags, int blocks,
+                                const of3_attn_pair_bias_params* attn, const of3_cond_transition_params* transition,
+                                void* workspace, size_t workspace_bytes, void* stream) {
+    OF3_REQUIRE(dtype == OF3_DTYPE_BF16 || dtype == OF3_DTYPE_F32, OF3_ERR_ARG, "diffusion_stack: bad dtype %d", dtype);
+    OF3_REQUIRE(diffusion_dims_ok(dims) && blocks > 0, OF3_ERR_ARG, "diffusion_stack: bad sizes");
+    OF3_REQUIRE(a && s && (z || bias) && attn && transition && workspace, OF3_ERR_ARG,
+                "diffusion_stack: null pointer argument");
+    Scratch ws{workspace, workspace_bytes};
+    return diffusion_stack(a, s, z, mask, bias, *dims, dtype, flags, blocks, attn, transition, ws, (cudaStream_t)stream);
 }
 
 }  // extern "C"

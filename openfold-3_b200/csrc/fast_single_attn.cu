@@ -2,9 +2,9 @@
 // the streaming core of the triangle attention (csrc/fast_triattn.cu) with one (pair tensor, head, 128 queries) and
 // two samples per CTA.
 //
-//   single_pack     q / k / v rows [rows, H*d] (outputs of the linear layers) -> pre-swizzled operand tiles: q with
-//                   its bias added and scaled by log2(e)/sqrt(d), K-dim padded with zeros to 32 (d = 24) or 64
-//                   (d = 48); k likewise per key block of 32; v transposed [d rows][32 keys]; keys >= N are zeros
+//   operand images  q / k / v projections as pre-swizzled operand tiles (linear.cu): q with its bias added and scaled
+//                   by log2(e)/sqrt(d), K-dim padded with zeros to 32 (d = 24) or 64 (d = 48); k likewise per key
+//                   block of 32; v transposed [d rows][32 keys]; keys >= N are zeros
 //   single_bias     pair bias fp32 [zh][nq][N] -> bf16 tiles [zh][key block][nq][32], pre-scaled by log2(e), each
 //                   64-byte row in the 64-byte swizzle of a K-major A operand (callers that project the bias
 //                   themselves get these tiles straight from csrc/fast_pairbias.cu and skip this kernel)
@@ -15,9 +15,11 @@
 // Queries may be a window of nq rows of the sample (row-sharded callers); keys and values are always all N rows.
 // Reference: openfold3/core/model/layers/attention_pair_bias.py:123-227,
 //            openfold3/core/model/primitives/attention.py:94-135, 270-310.
+#include "fast_single.cuh"
 #include "modules.cuh"
 #include "rowtile.cuh"
 #include "runtime.cuh"
+#include "single_attn.cuh"
 
 namespace of3 {
 namespace fast {
@@ -27,11 +29,11 @@ using namespace umma;
 using namespace rowtile;
 typedef __nv_bfloat16 bf16;
 
-constexpr int kKidSingleAttn = 8;    // operand images: accounted with the single track's small kernels
+constexpr int kKidSingleAttn = 8;    // bias conversion: accounted with the single track's small kernels
 constexpr int kKidSingleCore = 11;   // the attention core
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kBQ = 128;   // queries per CTA and line
-constexpr int kBK = 32;    // keys per step
+constexpr int kBQ = kSingleBQ;   // queries per CTA and line
+constexpr int kBK = kSingleBK;   // keys per step
 constexpr int kLines = 2;  // samples per CTA: they share the pair-bias tiles
 constexpr int kThreads = 32 * (1 + kLines + 4 * kLines);  // producer, one MMA warp per line, softmax warps
 constexpr float kRescaleThreshold = 8.0f;
@@ -39,9 +41,9 @@ constexpr int kMaxKeysSingle = 8192;  // one flag byte per key block, 256 of the
 
 template <int D>
 struct Cfg {
-    static constexpr int kKD = (D <= 32) ? 32 : 64;      // K dim of Q K^T after zero padding
+    static constexpr int kKD = SingleImage<D>::kKD;
     static constexpr int kKSteps = (D + 15) / 16;        // K = 16 steps that hold data
-    static constexpr int kDV = (D <= 32) ? 32 : 48;      // rows of the V^T tile = columns of O
+    static constexpr int kDV = SingleImage<D>::kDV;
     static constexpr int kStages = (D <= 32) ? 4 : 3;    // ring of K + bias tiles
     static constexpr int kVStages = (D <= 32) ? 4 : 2;   // ring of V tiles (two CTAs of 16 x 48 heads must fit an SM)
     static constexpr uint32_t kQBytes = kBQ * kKD * 2;   // 8 or 16 KB
@@ -64,83 +66,6 @@ struct Cfg {
     // in place once S has been read out; O [64, 64 + kON): kDV channels, then the sum of the row's P
     static constexpr uint32_t kColO = 64;
 };
-
-// 16-byte chunk c of row r inside a K-major tile with rows of kKD bf16: 64-byte rows use the 64-byte swizzle,
-// 128-byte rows the 128-byte swizzle (what the tcgen05 descriptors of umma.cuh expect).
-template <int KD>
-__device__ __forceinline__ uint32_t tile_chunk_off(int r, int c) {
-    return KD == 32 ? (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) : (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4));
-}
-
-
-// ---------------------------------------------------------------- operand images
-// q and k: one thread per 16-byte chunk of a tile row (reads of a warp run along the rows of the source, each
-// tile row is written whole). blockIdx.y: 0 = q tiles [bh][query tile][128][KD], 1 = k tiles [bh][key block][32][KD].
-template <int D>
-__global__ void __launch_bounds__(256)
-single_pack_qk_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ q_bias,
-                      bf16* __restrict__ q_img, bf16* __restrict__ k_img, int BB, int N, int nq, int H, float qscale) {
-    constexpr int KD = Cfg<D>::kKD, CH = KD / 8;
-    const bool is_q = blockIdx.y == 0;
-    const int rows_src = is_q ? nq : N;
-    const int tile_rows = is_q ? kBQ : kBK;
-    const int rows_pad = (rows_src + tile_rows - 1) / tile_rows * tile_rows;
-    const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
-    const int c = (int)(idx % CH);
-    const int h = (int)((idx / CH) % H);
-    const int pos = (int)((idx / ((long long)CH * H)) % rows_pad);
-    const long long bb = idx / ((long long)CH * H * rows_pad);
-    if (bb >= BB) return;
-    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-    if (pos < rows_src && c * 8 < D) {
-        const long long off = (bb * rows_src + pos) * (long long)(H * D) + h * D + c * 8;
-        w = *reinterpret_cast<const uint4*>((is_q ? q : k) + off);
-        if (is_q) {
-            uint4 bq = make_uint4(0u, 0u, 0u, 0u);
-            if (q_bias) bq = *reinterpret_cast<const uint4*>(q_bias + h * D + c * 8);
-            w.x = pack_bf16x2((bf16lo(w.x) + bf16lo(bq.x)) * qscale, (bf16hi(w.x) + bf16hi(bq.x)) * qscale);
-            w.y = pack_bf16x2((bf16lo(w.y) + bf16lo(bq.y)) * qscale, (bf16hi(w.y) + bf16hi(bq.y)) * qscale);
-            w.z = pack_bf16x2((bf16lo(w.z) + bf16lo(bq.z)) * qscale, (bf16hi(w.z) + bf16hi(bq.z)) * qscale);
-            w.w = pack_bf16x2((bf16lo(w.w) + bf16lo(bq.w)) * qscale, (bf16hi(w.w) + bf16hi(bq.w)) * qscale);
-        }
-    }
-    const long long tile = (bb * H + h) * (rows_pad / tile_rows) + pos / tile_rows;
-    uint8_t* dst = reinterpret_cast<uint8_t*>(is_q ? q_img : k_img) + tile * tile_rows * (long long)(KD * 2);
-    *reinterpret_cast<uint4*>(dst + tile_chunk_off<KD>(pos % tile_rows, c)) = w;
-}
-
-// v: block = (key block of 32, sample); the 32 source rows pass through shared memory and leave transposed,
-// v tiles [bh][key block][DV][32 keys] with the 64-byte swizzle. Dynamic shared memory: 32 * H * D * 2 bytes.
-template <int D>
-__global__ void __launch_bounds__(256)
-single_pack_v_kernel(const bf16* __restrict__ v, bf16* __restrict__ v_img, int N, int H) {
-    constexpr int DV = Cfg<D>::kDV;
-    extern __shared__ __align__(16) uint8_t vs_raw[];
-    bf16* vs = reinterpret_cast<bf16*>(vs_raw);
-    const int kb = blockIdx.x, nkb = gridDim.x;
-    const long long bb = blockIdx.y;
-    const int HD = H * D, cpr = HD / 8;
-    for (int idx = threadIdx.x; idx < kBK * cpr; idx += 256) {
-        const int r = idx / cpr, c = idx % cpr;
-        const int key = kb * kBK + r;
-        uint4 w = make_uint4(0u, 0u, 0u, 0u);
-        if (key < N) w = *reinterpret_cast<const uint4*>(v + (bb * N + key) * (long long)HD + c * 8);
-        *reinterpret_cast<uint4*>(vs + r * HD + c * 8) = w;
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < H * DV * 4; idx += 256) {
-        const int kc = idx & 3, dd = (idx >> 2) % DV, h = idx / (4 * DV);
-        uint32_t w[4] = {0u, 0u, 0u, 0u};
-        if (dd < D) {
-            const unsigned short* col = reinterpret_cast<const unsigned short*>(vs) + h * D + dd;
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                w[e] = (uint32_t)col[(kc * 8 + 2 * e) * HD] | ((uint32_t)col[(kc * 8 + 2 * e + 1) * HD] << 16);
-        }
-        bf16* tile = v_img + (((bb * H + h) * nkb + kb) * (long long)DV + dd) * kBK;
-        *reinterpret_cast<uint4*>(tile + ((kc ^ ((dd >> 1) & 3)) << 3)) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-}
 
 // pair bias fp32 [zh][nq][N] -> bf16 tiles [zh][key block][nq][32], times log2(e); block = (query row, zh)
 __global__ void __launch_bounds__(256)
@@ -254,6 +179,8 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr;
+    grid_trigger();
+    grid_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -532,66 +459,16 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
 }
 
 template <int D>
-struct Images {
-    size_t q, k, v, tb;  // bytes
-    Images(int BB, int Bz, int N, int nq, int H) {
-        const size_t n_qt = ceil_div(nq, kBQ), nkb = ceil_div(N, kBK);
-        q = (size_t)BB * H * n_qt * Cfg<D>::kQBytes;
-        k = (size_t)BB * H * nkb * Cfg<D>::kKBytes;
-        v = (size_t)BB * H * nkb * Cfg<D>::kVBytes;
-        tb = (size_t)Bz * H * nkb * nq * kBK * sizeof(bf16);
-    }
-};
-
-template <int D>
-int attn_tc_impl(const bf16* q, const bf16* k, const bf16* v, const bf16* g, const bf16* q_bias, const float* pb,
-                 const bf16* mask, bf16* out, int BB, int N, int nq, int H, float inf, int rpb, Arena& ws,
-                 cudaStream_t st, const bf16* z, const bf16* ln_z_w, const bf16* ln_z_b, const bf16* w_z,
-                 const bf16* bias_tiles) {
-    const int Bz = BB / rpb;
-    const Images<D> im(BB, Bz, N, nq, H);
-    bf16* q_img = (bf16*)ws.take(im.q);
-    bf16* k_img = (bf16*)ws.take(im.k);
-    bf16* v_img = (bf16*)ws.take(im.v);
-    bf16* tb_img = (bf16*)ws.take(im.tb);
-    if (!ws.base) return OF3_OK;
-    OF3_REQUIRE(ws.ok(), OF3_ERR_WORKSPACE, "single attention: workspace too small (%zu needed)", ws.off);
+int core_impl(const SingleImages& im, const bf16* g, const bf16* tb, const bf16* mask, bf16* out, int BB, int N, int nq,
+              int H, float inf, int rpb, cudaStream_t st) {
     const int nkb = ceil_div(N, kBK), n_qt = ceil_div(nq, kBQ);
-    constexpr int CH = Cfg<D>::kKD / 8;
-    {
-        const long long nq_chunks = (long long)BB * n_qt * kBQ * H * CH, nk_chunks = (long long)BB * nkb * kBK * H * CH;
-        const long long most = nq_chunks > nk_chunks ? nq_chunks : nk_chunks;
-        LaunchScope scope(kKidSingleAttn, st);
-        single_pack_qk_kernel<D><<<dim3((unsigned)((most + 255) / 256), 2), 256, 0, st>>>(
-            q, k, q_bias, q_img, k_img, BB, N, nq, H, kLog2e * rsqrtf((float)D));
-    }
-    {
-        const size_t smem = (size_t)kBK * H * D * sizeof(bf16);
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(single_pack_v_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem));
-        LaunchScope scope(kKidSingleAttn, st);
-        single_pack_v_kernel<D><<<dim3(nkb, BB), 256, smem, st>>>(v, v_img, N, H);
-    }
-    if (bias_tiles != nullptr) {
-        tb_img = const_cast<bf16*>(bias_tiles);   // projected earlier, in this kernel's layout
-    } else if (pb != nullptr) {
-        LaunchScope scope(kKidSingleAttn, st);
-        single_bias_kernel<<<dim3(nq, Bz * H), 256, 0, st>>>(pb, tb_img, N, nq, nkb);
-    } else {   // straight from the pair tensor: no fp32 bias in between
-        OF3_REQUIRE(z != nullptr && w_z != nullptr && nq == N && H == 16, OF3_ERR_ARG,
-                    "single attention: neither a pair bias nor a whole pair tensor to project it from");
-        const int rc = pair_bias_tiles_c128_h16(z, ln_z_w, ln_z_b, w_z, tb_img, Bz, N, st);
-        if (rc) return rc;
-    }
-    OF3_CUDA_CHECK(cudaGetLastError());
     const uint32_t smem = Cfg<D>::dyn_bytes(nkb * kBK);
     // the size depends on N and function attributes are per device: set on every launch (a host-side store)
     OF3_CUDA_CHECK(cudaFuncSetAttribute(single_core_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const long long grid = (long long)Bz * H * n_qt * ceil_div(rpb, kLines);
+    const long long grid = (long long)(BB / rpb) * H * n_qt * ceil_div(rpb, kLines);
     LaunchScope scope(kKidSingleCore, st);
-    single_core_kernel<D><<<(unsigned)grid, kThreads, smem, st>>>(q_img, k_img, v_img, tb_img, mask, g, out, N, nq, H,
-                                                                  rpb, inf, device_status_ptr());
-    OF3_CUDA_CHECK(cudaGetLastError());
+    OF3_CUDA_CHECK(launch_chained(single_core_kernel<D>, dim3((unsigned)grid), kThreads, smem, st, im.q, im.k, im.v, tb,
+                                  mask, g, out, N, nq, H, rpb, inf, device_status_ptr()));
     return OF3_OK;
 }
 
@@ -599,28 +476,46 @@ int attn_tc_impl(const bf16* q, const bf16* k, const bf16* v, const bf16* g, con
 
 // d in {24, 48}; H * d a multiple of 8 (16-byte rows per head); N within the mask row a CTA keeps.
 bool single_attn_tc_supported(int N, int H, int d) {
-    if (!(d == 24 || d == 48) || N < 1 || N > kMaxKeysSingle) return false;
+    if (!(d == 24 || d == 48) || N < 1 || N > kMaxKeysSingle || H * d % 64 != 0) return false;
     const size_t smem = d == 24 ? Cfg<24>::dyn_bytes(ceil_div(N, kBK) * kBK) : Cfg<48>::dyn_bytes(ceil_div(N, kBK) * kBK);
-    return smem <= 227 * 1024 && (size_t)kBK * H * d * sizeof(bf16) <= 160 * 1024;
+    return smem <= 227 * 1024;
+}
+
+SingleImages take_single_images(Arena& ws, int BB, int N, int nq, int H, int d) {
+    const size_t n_qt = ceil_div(nq, kBQ), nkb = ceil_div(N, kBK), bh = (size_t)BB * H;
+    SingleImages im;
+    im.q = (bf16*)ws.take(bh * n_qt * (d == 24 ? Cfg<24>::kQBytes : Cfg<48>::kQBytes));
+    im.k = (bf16*)ws.take(bh * nkb * (d == 24 ? Cfg<24>::kKBytes : Cfg<48>::kKBytes));
+    im.v = (bf16*)ws.take(bh * nkb * (d == 24 ? Cfg<24>::kVBytes : Cfg<48>::kVBytes));
+    return im;
 }
 
 // Gated attention with pair bias over BB samples of N keys and nq query rows each:
 //   out[bb, i, h, :] = sigmoid(g[bb, i, h, :]) * softmax_j((q[bb, i, h] + q_bias[h]) . k[bb, j, h] / sqrt(d)
 //                                                       + inf * (mask[bb, j] - 1) + pair_bias[bb / rpb, h, i, j]) v
-// q, g, out: [BB, nq, H*d]; k, v: [BB, N, H*d]; pair_bias fp32 [BB / rpb, H, nq, N]; mask [BB, N] or null.
-// With ws.base == nullptr only the workspace need is accumulated.
-int single_attn_tc(const bf16* q, const bf16* k, const bf16* v, const bf16* g, const bf16* q_bias,
-                   const float* pair_bias, const bf16* mask, bf16* out, int BB, int N, int nq, int H, int d, float inf,
-                   int rows_per_bias, Arena& ws, cudaStream_t st, const bf16* z, const bf16* ln_z_w, const bf16* ln_z_b,
-                   const bf16* w_z, const bf16* bias_tiles) {
+// g, out: [BB, nq, H*d]; mask [BB, N] or null; tb: room for the bias tiles where they are not given.
+int single_attn(const SingleImages& im, const bf16* g, const SingleBias& bias, bf16* tb, const bf16* mask, bf16* out,
+                int BB, int N, int nq, int H, int d, float inf, int rows_per_bias, cudaStream_t st) {
     OF3_REQUIRE(single_attn_tc_supported(N, H, d), OF3_ERR_SHAPE, "single attention: N %d, H %d, d %d not supported",
                 N, H, d);
     OF3_REQUIRE(rows_per_bias > 0 && BB % rows_per_bias == 0, OF3_ERR_SHAPE,
                 "single attention: %d samples do not divide into groups of %d", BB, rows_per_bias);
-    return d == 24 ? attn_tc_impl<24>(q, k, v, g, q_bias, pair_bias, mask, out, BB, N, nq, H, inf, rows_per_bias, ws, st,
-                                      z, ln_z_w, ln_z_b, w_z, bias_tiles)
-                   : attn_tc_impl<48>(q, k, v, g, q_bias, pair_bias, mask, out, BB, N, nq, H, inf, rows_per_bias, ws, st,
-                                      z, ln_z_w, ln_z_b, w_z, bias_tiles);
+    const int Bz = BB / rows_per_bias;
+    const bf16* tiles = tb;
+    if (bias.tiles != nullptr) {
+        tiles = bias.tiles;   // projected earlier, in this kernel's layout
+    } else if (bias.f32 != nullptr) {
+        LaunchScope scope(kKidSingleAttn, st);
+        single_bias_kernel<<<dim3(nq, Bz * H), 256, 0, st>>>(bias.f32, tb, N, nq, ceil_div(N, kBK));
+        OF3_CUDA_CHECK(cudaGetLastError());
+    } else {   // straight from the pair tensor: no fp32 bias in between
+        OF3_REQUIRE(bias.z != nullptr && bias.w != nullptr && nq == N && H == 16, OF3_ERR_ARG,
+                    "single attention: neither a pair bias nor a whole pair tensor to project it from");
+        const int rc = pair_bias_tiles_c128_h16(bias.z, bias.ln_w, bias.ln_b, bias.w, tb, Bz, N, st);
+        if (rc) return rc;
+    }
+    return d == 24 ? core_impl<24>(im, g, tiles, mask, out, BB, N, nq, H, inf, rows_per_bias, st)
+                   : core_impl<48>(im, g, tiles, mask, out, BB, N, nq, H, inf, rows_per_bias, st);
 }
 
 }  // namespace fast

@@ -1,0 +1,469 @@
+// Linear layers on tcgen05 with their consumers in the epilogue (bf16 operands, fp32 accumulation): the projections of
+// the single track (c_s = 384) and of the diffusion token stack (c_a = 768, c_s = 384).
+//
+//   y = x W^T, x [rows][k], W [n][k], both K-major. Persistent CTA: warp 0 TMA producer (128-byte swizzled k-blocks of
+//   64), warp 1 MMA issuer (128 x BN x 16, accumulators double-buffered in TMEM), warps 2..9 the epilogue (two per 32
+//   rows, each half of the columns; thread = row).
+//
+// What bounds them: a few hundred 128-row tiles with k = 384 .. 1536 are 3 - 15 us of L2 -> shared-memory traffic (every
+// tile streams its A and B panels) and, for short sequences, launch and fill latency; the separate passes that read the
+// products back (attention operand images, silu * mul, gates, residuals) cost as much again as 11 launches per block.
+// So the product leaves the SM in the form its consumer reads, and BN is chosen per call (pick_bn).
+#include "linear.cuh"
+#include "modules.cuh"
+#include "rowtile.cuh"
+#include "runtime.cuh"
+#include "single_attn.cuh"
+
+namespace of3 {
+namespace fast {
+namespace {
+
+using namespace umma;
+typedef __nv_bfloat16 bf16;
+
+constexpr int kKid = 10;
+constexpr int kBM = 128, kBK = 64;
+constexpr int kThreads = 32 * (2 + 8);
+constexpr float kLog2e = 1.4426950408889634f;
+
+enum Epi { kEpiStore, kEpiImages, kEpiSwiglu, kEpiResidual };
+
+template <int BN>
+struct LinCfg {
+    static constexpr int kABytes = kBM * kBK * 2;
+    static constexpr int kStageBytes = kABytes + BN * kBK * 2;
+    static constexpr int kStages = BN == 256 ? 4 : (BN == 192 ? 5 : (BN == 128 ? 6 : 8));
+    static constexpr int kAccStride = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);
+    static constexpr int kTmemCols = 2 * kAccStride;
+    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+};
+
+struct LinMaps {
+    CUtensorMap a, w[4];
+};
+struct EpiArgs {
+    // kEpiStore
+    bf16* y;
+    int raw_slice;
+    // kEpiImages
+    AttnImages im;
+    int kind[4];
+    float qscale;
+    // kEpiSwiglu, kEpiResidual
+    bf16* out;
+    const bf16 *residual, *gate, *gate_bias, *mask;
+};
+
+__device__ __forceinline__ float sigmoid_of(float x) { return 1.0f / (1.0f + __expf(-x)); }
+
+// One column group of 16 of this thread's row as attention operand images; `kind` is uniform over the tile.
+template <int D>
+__device__ __forceinline__ void store_images(const AttnImages& im, int kind, float qscale, const uint32_t (&r)[16],
+                                             int col0, long long row) {
+    constexpr int KD = SingleImage<D>::kKD, DV = SingleImage<D>::kDV;
+    const int HD = im.H * D;
+    if (kind == kOutG) {
+        uint32_t o[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = pack_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+        stg256(im.g + row * HD + col0, o);
+        return;
+    }
+    const int n = im.rows_per_sample;
+    const long long bb = row / n;
+    const int pos = (int)(row - bb * n);
+    const int nkb = (n + kSingleBK - 1) / kSingleBK, n_qt = (n + kSingleBQ - 1) / kSingleBQ;
+    const int pad = nkb * kSingleBK - n;   // keys past the end of the last block: zeros, written by the first rows
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int col = col0 + half * 8;
+        const int h = col / D, d0 = col - h * D;
+        if (kind == kOutV) {
+            // tile [DV][32 keys], 64-byte rows: a warp's 32 consecutive keys fill one row of one tile
+            auto put = [&](int p, bool live) {
+                const int kc = (p & 31) >> 3;
+                bf16* tile = im.v + (((bb * im.H + h) * nkb + (p >> 5)) * (long long)DV) * kSingleBK;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const int dd = d0 + e;
+                    tile[dd * kSingleBK + (((kc ^ ((dd >> 1) & 3)) << 3) | (p & 7))] =
+                        __float2bfloat16_rn(live ? __uint_as_float(r[half * 8 + e]) : 0.f);
+                }
+            };
+            put(pos, true);
+            for (int p = n + pos; p < n + pad; p += n) put(p, false);
+            continue;
+        }
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[half * 8 + e]);
+        if (kind == kOutQ) {
+            if (im.q_bias) {
+                uint32_t b[4];
+                ld_row8_any(im.q_bias + col, b);
+                #pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] += (e & 1) ? bf16hi(b[e >> 1]) : bf16lo(b[e >> 1]);
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] *= qscale;
+        }
+        const uint4 v = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
+                                   pack_bf16x2(f[6], f[7]));
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        const int c = d0 >> 3;
+        const bool last = D < KD && D <= 32 && c == D / 8 - 1;   // 24 channels: chunk 3 of the row pads K with zeros
+        if (kind == kOutQ) {
+            uint8_t* t = reinterpret_cast<uint8_t*>(im.q) +
+                         ((bb * im.H + h) * n_qt + (pos >> 7)) * (long long)(kSingleBQ * KD * 2);
+            *reinterpret_cast<uint4*>(t + single_chunk_off<KD>(pos & 127, c)) = v;
+            if (last) *reinterpret_cast<uint4*>(t + single_chunk_off<KD>(pos & 127, c + 1)) = zero;
+        } else {
+            uint8_t* t0 = reinterpret_cast<uint8_t*>(im.k) + (bb * im.H + h) * nkb * (long long)(kSingleBK * KD * 2);
+            uint8_t* t = t0 + (pos >> 5) * (long long)(kSingleBK * KD * 2);
+            *reinterpret_cast<uint4*>(t + single_chunk_off<KD>(pos & 31, c)) = v;
+            if (last) *reinterpret_cast<uint4*>(t + single_chunk_off<KD>(pos & 31, c + 1)) = zero;
+            for (int p = n + pos; p < n + pad; p += n) {
+                uint8_t* tp = t0 + (p >> 5) * (long long)(kSingleBK * KD * 2);
+                *reinterpret_cast<uint4*>(tp + single_chunk_off<KD>(p & 31, c)) = zero;
+                if (last) *reinterpret_cast<uint4*>(tp + single_chunk_off<KD>(p & 31, c + 1)) = zero;
+            }
+        }
+    }
+}
+
+template <int BN, int EPI, int D>
+__global__ void __launch_bounds__(kThreads, 1)
+linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long rows, int K, int n, int num_mats,
+              int* status) {
+    using Cfg = LinCfg<BN>;
+    constexpr int S = Cfg::kStages;
+    constexpr int kWRows = EPI == kEpiSwiglu ? BN / 2 : BN;   // rows of each weight matrix in a tile
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
+    const uint32_t bars = sbase + S * Cfg::kStageBytes;
+    auto full = [&](int s) { return bars + 8u * s; };
+    auto empty = [&](int s) { return bars + 8u * (S + s); };
+    auto tfull = [&](int a) { return bars + 8u * (2 * S + a); };
+    auto tempty = [&](int a) { return bars + 8u * (2 * S + 2 + a); };
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + S * Cfg::kStageBytes + 8 * (2 * S + 4));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + S * Cfg::kStageBytes + 8 * (2 * S + 4) + 8);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int num_mt = (int)((rows + kBM - 1) / kBM);
+    const int nt_per_mat = n / kWRows;
+    // kEpiSwiglu: matrices 0 and 1 share a tile; otherwise a tile lies inside one matrix
+    const int num_nt = EPI == kEpiSwiglu ? nt_per_mat : nt_per_mat * num_mats;
+    const int num_kb = K / kBK;
+    const int num_tiles = num_mt * num_nt;
+    // a tile: row tile mt (innermost: concurrent CTAs share the weight panel), matrix g, column tile inside it
+    struct Tile { int mt, g, nt; };
+    auto tile_of = [&](int t) {
+        Tile c;
+        c.mt = t % num_mt;
+        const int q = t / num_mt;
+        c.g = EPI == kEpiSwiglu ? 0 : q / nt_per_mat;
+        c.nt = EPI == kEpiSwiglu ? q : q % nt_per_mat;
+        return c;
+    };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < S; ++s) {
+            mbar_init(full(s), 1);
+            mbar_init(empty(s), 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(tfull(a), 1);
+            mbar_init(tempty(a), 8);
+        }
+        *abort_flag = 0;
+        mbar_fence_init();
+        prefetch_tmap(&maps.a);
+        prefetch_tmap(&maps.w[0]);
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32((const void*)tmem_ptr), Cfg::kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    grid_trigger();
+    const uint32_t tmem_base = *tmem_ptr;
+
+    if (warp == 0) {
+        // ---------------------------------------------------------------- TMA producer
+        if (lane == 0) {
+            auto load_w = [&](const Tile& c, int kb, int s) {
+                const uint32_t sw = sbase + s * Cfg::kStageBytes + Cfg::kABytes;
+                if constexpr (EPI == kEpiSwiglu) {
+                    tma_load_2d(sw, &maps.w[0], full(s), kb * kBK, c.nt * kWRows);
+                    tma_load_2d(sw + kWRows * 128, &maps.w[1], full(s), kb * kBK, c.nt * kWRows);
+                } else if constexpr (EPI == kEpiStore) {
+                    tma_load_2d(sw, &maps.w[0], full(s), kb * kBK, c.g * n + c.nt * BN);
+                } else {
+                    tma_load_2d(sw, &maps.w[c.g], full(s), kb * kBK, c.nt * BN);
+                }
+            };
+            auto load_a = [&](const Tile& c, int kb, int s) {
+                const int slice = EPI == kEpiStore ? (c.g % 3 == 2 ? ep.raw_slice : c.g / 3) : 0;
+                tma_load_3d(sbase + s * Cfg::kStageBytes, &maps.a, full(s), kb * kBK, c.mt * kBM, slice);
+            };
+            // the weight panels of the first stages do not depend on the kernel before this one
+            const Tile first = tile_of(blockIdx.x);
+            const int ahead = num_kb < S ? num_kb : S;
+            for (int kb = 0; kb < ahead; ++kb) {
+                mbar_arrive_expect_tx(full(kb), Cfg::kStageBytes);
+                load_w(first, kb, kb);
+            }
+            grid_wait();
+            for (int kb = 0; kb < ahead; ++kb) load_a(first, kb, kb);
+            uint32_t it = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+                const Tile c = tile_of(t);
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    if (it < (uint32_t)ahead) continue;
+                    const int s = it % S;
+                    if (!mbar_wait(empty(s), ((it / S) & 1u) ^ 1u, abort_flag)) {
+                        report_wait_failure(status, abort_flag, kKid, 1);
+                        ok = false;
+                        break;
+                    }
+                    mbar_arrive_expect_tx(full(s), Cfg::kStageBytes);
+                    load_a(c, kb, s);
+                    load_w(c, kb, s);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------- MMA issuer
+        if (lane == 0) {
+            constexpr uint32_t idesc = idesc_bf16_f32(kBM, BN);
+            uint32_t it = 0, tc = 0;
+            bool ok = true;
+            for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tc) {
+                const uint32_t acc = tc & 1u;
+                if (!mbar_wait(tempty(acc), ((tc >> 1) & 1u) ^ 1u, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKid, 2);
+                    break;
+                }
+                tc_fence_after_sync();
+                const uint32_t d = tmem_base + acc * Cfg::kAccStride;
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    const int s = it % S;
+                    if (!mbar_wait(full(s), (it / S) & 1u, abort_flag)) {
+                        report_wait_failure(status, abort_flag, kKid, 3);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    const uint32_t sa = sbase + s * Cfg::kStageBytes;
+                    const uint64_t ad = smem_desc_k_sw128(sa), bd = smem_desc_k_sw128(sa + Cfg::kABytes);
+#pragma unroll
+                    for (int k4 = 0; k4 < kBK / 16; ++k4)
+                        mma_bf16(d, ad + 2u * k4, bd + 2u * k4, idesc, (kb | k4) != 0 ? 1u : 0u);
+                    mma_commit(empty(s));
+                }
+                if (ok) mma_commit(tfull(acc));
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------- epilogue: thread = row, half of the columns
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        constexpr int kCols = EPI == kEpiSwiglu ? BN / 4 : BN / 2;   // result columns per thread and tile
+        grid_wait();
+        uint32_t tc = 0;
+        for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tc) {
+            const Tile c = tile_of(t);
+            const uint32_t acc = tc & 1u;
+            const long long row = (long long)c.mt * kBM + quad * 32 + lane;
+            const bool live = row < rows;
+            if (!mbar_wait(tfull(acc), (tc >> 1) & 1u, abort_flag)) {
+                if (lane == 0) report_wait_failure(status, abort_flag, kKid, 4);
+                break;
+            }
+            tc_fence_after_sync();
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * Cfg::kAccStride + half * kCols;
+            float mk = 1.0f;
+            if constexpr (EPI == kEpiResidual) {
+                if (ep.mask != nullptr && live) mk = __bfloat162float(ep.mask[row]);
+            }
+#pragma unroll 1
+            for (int c0 = 0; c0 < kCols; c0 += 16) {
+                uint32_t r[16], r2[16];
+                tmem_ld16(taddr + c0, r);
+                if constexpr (EPI == kEpiSwiglu) tmem_ld16(taddr + BN / 2 + c0, r2);
+                tmem_ld_wait();
+                const int col = c.nt * kWRows + half * kCols + c0;   // column inside the matrix
+                if (!live) continue;
+                if constexpr (EPI == kEpiImages) {
+                    store_images<D>(ep.im, ep.kind[c.g], ep.qscale, r, col, row);
+                } else {
+                    uint32_t o[8];
+                    if constexpr (EPI == kEpiStore) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            o[e] = pack_bf16x2(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+                        stg256(ep.y + ((long long)c.g * rows + row) * n + col, o);
+                    } else if constexpr (EPI == kEpiSwiglu) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const float a0 = __uint_as_float(r[2 * e]), a1 = __uint_as_float(r[2 * e + 1]);
+                            o[e] = pack_bf16x2(a0 * sigmoid_of(a0) * __uint_as_float(r2[2 * e]),
+                                               a1 * sigmoid_of(a1) * __uint_as_float(r2[2 * e + 1]));
+                        }
+                        stg256(ep.out + row * n + col, o);
+                    } else {
+                        float v[16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) v[e] = mk * __uint_as_float(r[e]);
+                        if (ep.gate != nullptr) {
+                            uint32_t g[8], b[8];
+                            ld_row16(ep.gate + row * n + col, g);
+                            ld_row16_any(ep.gate_bias + col, b);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                v[2 * e] *= sigmoid_of(bf16lo(g[e]) + bf16lo(b[e]));
+                                v[2 * e + 1] *= sigmoid_of(bf16hi(g[e]) + bf16hi(b[e]));
+                            }
+                        }
+                        if (ep.residual != nullptr) {
+                            uint32_t z[8];
+                            ld_row16_any(ep.residual + row * n + col, z);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                v[2 * e] += bf16lo(z[e]);
+                                v[2 * e + 1] += bf16hi(z[e]);
+                            }
+                        }
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) o[e] = pack_bf16x2(v[2 * e], v[2 * e + 1]);
+                        st_row16_any(ep.out + row * n + col, o);
+                    }
+                }
+            }
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty(acc));
+        }
+    }
+
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, Cfg::kTmemCols);
+    }
+}
+
+// Column tile: the number of waves of 148 CTAs times the panels a tile streams (128 rows of x and BN of the weights per
+// k-block, plus a constant for its fill and epilogue). Wide tiles move fewer bytes, narrow ones fill the chip when there
+// are few rows; a BN that does not divide the matrix is out.
+int pick_bn(long long rows, int n, int mats, bool swiglu) {
+    const long long sms = sm_count(), mt = (rows + kBM - 1) / kBM;
+    const int cand[4] = {256, 192, 128, 64};
+    int best = 0;
+    long long best_cost = 0;
+    for (int bn : cand) {
+        const int wr = swiglu ? bn / 2 : bn;
+        if (n % wr != 0 || (swiglu && (bn == 64 || bn == 192))) continue;
+        const long long tiles = mt * (n / wr) * (swiglu ? 1 : mats);
+        const long long cost = (tiles + sms - 1) / sms * (128 + bn + 64);
+        if (best == 0 || cost < best_cost) {
+            best = bn;
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
+template <int BN, int EPI, int D>
+int launch(const LinearIn& in, const EpiArgs& ep, int slices, int w_rows, cudaStream_t st) {
+    using Cfg = LinCfg<BN>;
+    constexpr int kWRows = EPI == kEpiSwiglu ? BN / 2 : BN;
+    LinMaps maps;
+    int rc;
+    {
+        uint64_t dims[3] = {(uint64_t)in.k, (uint64_t)in.rows, (uint64_t)slices};
+        uint64_t str[2] = {(uint64_t)in.k * 2, (uint64_t)in.rows * in.k * 2};
+        uint32_t box[3] = {kBK, kBM, 1};
+        if ((rc = make_tmap_bf16(&maps.a, in.x, 3, dims, str, box, 1))) return rc;
+    }
+    const int tensors = EPI == kEpiStore ? 1 : in.num_w;
+    for (int i = 0; i < tensors; ++i) {
+        uint64_t dims[2] = {(uint64_t)in.k, (uint64_t)w_rows};
+        uint64_t str[1] = {(uint64_t)in.k * 2};
+        uint32_t box[2] = {kBK, (uint32_t)kWRows};
+        if ((rc = make_tmap_bf16(&maps.w[i], in.w[i], 2, dims, str, box, 1))) return rc;
+    }
+    for (int i = tensors; i < 4; ++i) maps.w[i] = maps.w[0];
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(linear_kernel<BN, EPI, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            Cfg::kSmemBytes));
+        configured.mark();
+    }
+    const long long tiles = ((in.rows + kBM - 1) / kBM) * (in.n / kWRows) * (EPI == kEpiSwiglu ? 1 : in.num_w);
+    OF3_REQUIRE(tiles < (1LL << 31) && in.rows < (1LL << 31), OF3_ERR_SHAPE, "linear: too many rows");
+    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+    LaunchScope scope(kKid, st);
+    OF3_CUDA_CHECK(launch_chained(linear_kernel<BN, EPI, D>, grid, kThreads, Cfg::kSmemBytes, st, maps, ep, in.rows, in.k,
+                                  in.n, in.num_w, device_status_ptr()));
+    return OF3_OK;
+}
+
+template <int EPI, int D>
+int dispatch(const LinearIn& in, const EpiArgs& ep, int slices, int w_rows, cudaStream_t st) {
+    OF3_REQUIRE(in.k % kBK == 0 && in.n % 64 == 0, OF3_ERR_SHAPE, "linear: widths %d x %d are not multiples of 64", in.n,
+                in.k);
+    switch (pick_bn(in.rows, in.n, in.num_w, EPI == kEpiSwiglu)) {
+        case 256: return launch<256, EPI, D>(in, ep, slices, w_rows, st);
+        case 192:
+            if constexpr (EPI != kEpiSwiglu) return launch<192, EPI, D>(in, ep, slices, w_rows, st);
+        case 128: return launch<128, EPI, D>(in, ep, slices, w_rows, st);
+        default:
+            if constexpr (EPI != kEpiSwiglu) return launch<64, EPI, D>(in, ep, slices, w_rows, st);
+            return OF3_ERR_SHAPE;
+    }
+}
+
+}  // namespace
+
+int linear_conditioning(const bf16* x, long long rows, int k, int n, const bf16* w, int layers, int slices,
+                        int raw_slice, bf16* y, cudaStream_t st) {
+    LinearIn in{x, rows, k, n, {w}, 3 * layers};
+    EpiArgs ep = {};
+    ep.y = y;
+    ep.raw_slice = raw_slice;
+    return dispatch<kEpiStore, 0>(in, ep, slices, 3 * layers * n, st);
+}
+
+int linear_attn_images(const LinearIn& in, const LinearOut* kinds, const AttnImages& im, cudaStream_t st) {
+    EpiArgs ep = {};
+    ep.im = im;
+    for (int i = 0; i < in.num_w; ++i) ep.kind[i] = kinds[i];
+    ep.qscale = kLog2e * (1.0f / sqrtf((float)im.D));
+    return im.D == 24 ? dispatch<kEpiImages, 24>(in, ep, 1, in.n, st) : dispatch<kEpiImages, 48>(in, ep, 1, in.n, st);
+}
+
+int linear_swiglu(const LinearIn& in, bf16* h, cudaStream_t st) {
+    EpiArgs ep = {};
+    ep.out = h;
+    return dispatch<kEpiSwiglu, 0>(in, ep, 1, in.n, st);
+}
+
+int linear_residual(const LinearIn& in, const bf16* residual, const bf16* gate, const bf16* gate_bias, const bf16* mask,
+                    bf16* out, cudaStream_t st) {
+    EpiArgs ep = {};
+    ep.out = out;
+    ep.residual = residual;
+    ep.gate = gate;
+    ep.gate_bias = gate_bias;
+    ep.mask = mask;
+    return dispatch<kEpiResidual, 0>(in, ep, 1, in.n, st);
+}
+
+}  // namespace fast
+}  // namespace of3

@@ -58,28 +58,20 @@ int triattn_finish(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloa
 bool transition_supported(int c, int n);
 int transition(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bfloat16* out, long long rows,
                int flags, const of3_transition_params* p, Arena& ws, cudaStream_t st);
-// gated attention with pair bias on the tensor pipe: q, g, out [BB, nq, H*d]; k, v [BB, N, H*d]; pair_bias fp32
-// [BB / rows_per_bias, H, nq, N]; with ws.base == nullptr only the workspace need is accumulated
+// gated attention with pair bias on the tensor pipe (fast_single.cuh)
 bool single_attn_tc_supported(int N, int H, int d);
-// pair_bias == nullptr: the bias tiles are projected straight from z (whole pair tensors only: nq == N) with the
-// LayerNorm weight / bias ln_z_w / ln_z_b and linear_z.weight w_z
-int single_attn_tc(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* g,
-                   const __nv_bfloat16* q_bias, const float* pair_bias, const __nv_bfloat16* mask, __nv_bfloat16* out,
-                   int BB, int N, int nq, int H, int d, float inf, int rows_per_bias, Arena& ws, cudaStream_t st,
-                   const __nv_bfloat16* z = nullptr, const __nv_bfloat16* ln_z_w = nullptr,
-                   const __nv_bfloat16* ln_z_b = nullptr, const __nv_bfloat16* w_z = nullptr,
-                   const __nv_bfloat16* bias_tiles = nullptr);   // bias_tiles: from pair_bias_tiles_c128_h16
 // single-track layers (bf16): linears on the tcgen05 contraction kernel, attention on single_attn_tc
 // (LayerNorm variant of the trunk, or with OF3_FLAG_ADA_LN the conditioned variant of the diffusion stack)
 bool attn_pair_bias_supported(int Ba, int Bz, int N, int c_a, int c_s, int c_z, int H, int d, int flags);
 int attn_pair_bias(const __nv_bfloat16* a, const __nv_bfloat16* z, const __nv_bfloat16* s, const __nv_bfloat16* mask,
                    __nv_bfloat16* out, int Ba, int Bz, int N, int c_a, int c_s, int H, int d, float inf, int flags,
                    const of3_attn_pair_bias_params* p, Arena& ws, cudaStream_t st, const float* pair_bias,
-                   const __nv_bfloat16* bias_tiles = nullptr);
+                   const __nv_bfloat16* bias_tiles = nullptr,
+                   const __nv_bfloat16* cond = nullptr);   // planes of `conditioning` (fast_single.cuh), or computed here
 bool cond_transition_supported(int c_a, int c_s, int n, int flags);
 int cond_transition(const __nv_bfloat16* a, const __nv_bfloat16* s, const __nv_bfloat16* mask, __nv_bfloat16* out,
                     long long rows, int c_a, int c_s, int n, int flags, const of3_cond_transition_params* p, Arena& ws,
-                    cudaStream_t st);
+                    cudaStream_t st, const __nv_bfloat16* cond = nullptr);
 int attn_pair_bias_rows(const __nv_bfloat16* a, const float* pair_bias_rows, const __nv_bfloat16* mask,
                         __nv_bfloat16* out_rows, int N, int row0, int R, int c_a, int H, int d, float inf, int flags,
                         const of3_attn_pair_bias_params* p, Arena& ws, cudaStream_t st);

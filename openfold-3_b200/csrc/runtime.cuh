@@ -2,6 +2,7 @@
 // driver entry point (no link-time dependency on libcuda), launch-attribute helpers.
 #pragma once
 #include <cuda.h>
+#include <atomic>
 #include "common.cuh"
 
 namespace of3 {
@@ -32,6 +33,24 @@ struct LaunchScope {
 // Work enqueued on `waiter` from now on starts after everything enqueued on `signaler` so far.
 int stream_wait(cudaStream_t waiter, cudaStream_t signaler);
 
+// Launches a kernel that calls umma::grid_wait() before it touches anything another kernel wrote: its prologue (barrier
+// set-up, tensor-memory allocation, weight loads) overlaps the end of the kernel before it in the stream.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
@@ -40,5 +59,24 @@ int sm_count();
 // marks them once cudaFuncSetAttribute has succeeded there. Guarded by the runtime's mutex.
 bool device_configured(int key);
 void device_mark_configured(int key);
+
+// The same for launch sites that are templates: a static object of one instantiation.
+class PerDeviceOnce {
+    std::atomic<unsigned long long> bits_{0};
+    static int device() {
+        int dev = 0;
+        return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? dev : -1;
+    }
+
+  public:
+    bool done() const {
+        const int d = device();
+        return d >= 0 && ((bits_.load(std::memory_order_acquire) >> d) & 1ull);
+    }
+    void mark() {
+        const int d = device();
+        if (d >= 0) bits_.fetch_or(1ull << d, std::memory_order_release);
+    }
+};
 
 }  // namespace of3

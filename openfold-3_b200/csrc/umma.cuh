@@ -92,6 +92,15 @@ __device__ __forceinline__ void tc_fence_after_sync() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
+// ---------------------------------------------------------------- programmatic dependent launch
+// A kernel launched with launch_chained (runtime.cuh) may start while the kernel before it in the stream still runs:
+// grid_wait() returns once that kernel (and with it everything before it) has completed and its writes are visible;
+// no thread reads or writes what another kernel of the stream may touch before it -- weights excepted, which only
+// ordinary kernels write. grid_trigger() lets the next kernel start; it comes after the CTA's TMEM allocation, so that
+// a waiting successor never holds tensor memory that a CTA of this grid still needs.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- TMA (tiled; destination = the issuing CTA)
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -247,6 +256,49 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
+// 32 bytes of global memory per thread (one full sector); p 32-byte aligned
+__device__ __forceinline__ void stg256(void* p, const uint32_t (&o)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(o[0]), "r"(o[1]), "r"(o[2]),
+                 "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7])
+                 : "memory");
+}
+__device__ __forceinline__ void ld_row16(const __nv_bfloat16* p, uint32_t (&o)[8]) {
+    const uint4 a = *reinterpret_cast<const uint4*>(p), b = *reinterpret_cast<const uint4*>(p + 8);
+    o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+    o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+}
+
+// Rows of the caller's own tensors: vector accesses where the address allows them.
+__device__ __forceinline__ void ld_row8_any(const __nv_bfloat16* p, uint32_t* o) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        const uint4 a = *reinterpret_cast<const uint4*>(p);
+        o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
+    } else {
+        const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[e] = (uint32_t)u[2 * e] | ((uint32_t)u[2 * e + 1] << 16);
+    }
+}
+__device__ __forceinline__ void ld_row16_any(const __nv_bfloat16* p, uint32_t (&o)[8]) {
+    ld_row8_any(p, o);
+    ld_row8_any(p + 8, o + 4);
+}
+__device__ __forceinline__ void st_row16_any(__nv_bfloat16* p, const uint32_t (&o)[8]) {
+    if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
+        stg256(p, o);
+    } else if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        *reinterpret_cast<uint4*>(p) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(p + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+    } else {
+        unsigned short* u = reinterpret_cast<unsigned short*>(p);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            u[2 * e] = (unsigned short)(o[e] & 0xffffu);
+            u[2 * e + 1] = (unsigned short)(o[e] >> 16);
+        }
+    }
+}
+
 // 16 consecutive fp32 columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(

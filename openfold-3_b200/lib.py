@@ -55,6 +55,10 @@ class BlockDims(ctypes.Structure):
         "no_heads_single", "c_hidden_single", "single_transition_n")] + [("inf_pair", c_float), ("inf_single", c_float)]
 
 
+class DiffusionDims(ctypes.Structure):
+    _fields_ = [(n, c_int) for n in ("Ba", "Bz", "N", "c_a", "c_s", "c_z", "H", "d", "n")] + [("inf", c_float)]
+
+
 # name -> (restype, argtypes); the same list is checked against include/of3b200.h by the tests
 SIGNATURES = {
     "of3_last_error_string": (c_char_p, []),
@@ -93,6 +97,11 @@ SIGNATURES = {
     "of3_pairformer_block_forward": (c_int, [c_void_p] * 4 + [ctypes.POINTER(BlockDims), c_int, c_int,
                                                               ctypes.POINTER(PairformerBlockParams), c_void_p, c_size_t,
                                                               c_void_p, c_size_t, c_void_p, c_void_p]),
+    "of3_diffusion_stack_workspace_bytes": (c_size_t, [ctypes.POINTER(DiffusionDims)] + [c_int] * 4),
+    "of3_diffusion_stack_forward": (c_int, [c_void_p] * 5 + [ctypes.POINTER(DiffusionDims), c_int, c_int, c_int,
+                                                             ctypes.POINTER(AttnPairBiasParams),
+                                                             ctypes.POINTER(CondTransitionParams), c_void_p, c_size_t,
+                                                             c_void_p]),
     "of3_stream_wait": (c_int, [c_void_p, c_void_p]),
     "of3_dap_pitch": (c_int, [c_int, c_int]),
     "of3_dap_triattn_image_elems": (c_longlong, [c_int, c_int]),
@@ -270,6 +279,24 @@ def pairformer_block_forward(s, z, single_mask, pair_mask, plan: BlockPlan, dtyp
                                              dtype, flags, params, ws.data_ptr(), ws.numel(), ws_side.data_ptr(),
                                              ws_side.numel(), main.cuda_stream, None if side is None else side.cuda_stream),
            "of3_pairformer_block_forward")
+
+
+class DiffusionPlan:
+    __slots__ = ("dims", "ref", "bytes", "blocks")
+
+    def __init__(self, dims: DiffusionDims, dtype: int, flags: int, blocks: int, with_bias: bool):
+        self.dims, self.ref, self.blocks = dims, ctypes.byref(dims), blocks
+        self.bytes = load().of3_diffusion_stack_workspace_bytes(self.ref, dtype, flags, blocks, int(with_bias))
+
+
+def diffusion_stack_forward(a, s, z, mask, biases, plan: DiffusionPlan, dtype: int, flags: int, params):
+    """All blocks of a diffusion token stack in place on a [Ba, N, c_a]; biases: projected pair bias per block, or
+    Nones (projected from z in the call); params: the two arrays of parameter structs."""
+    ws = workspace(plan.bytes, a.device)
+    bias = None if biases[0] is None else (c_void_p * plan.blocks)(*[t.data_ptr() for t in biases])
+    _check(_lib.of3_diffusion_stack_forward(a.data_ptr(), s.data_ptr(), z.data_ptr(), _ptr(mask), bias, plan.ref, dtype,
+                                            flags, plan.blocks, params[0], params[1], ws.data_ptr(), ws.numel(),
+                                            _stream(a.device)), "of3_diffusion_stack_forward")
 
 
 def stream_wait(waiter, signaler):

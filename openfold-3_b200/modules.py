@@ -191,15 +191,24 @@ class _PackedParams:
         return self._val
 
 
-class _BlockPlans:
-    """A block's parameters as the native block entry point takes them, and its plans per shape.
+def _param_watch():
+    try:
+        from . import _param_watch as w
+    except ImportError as e:
+        raise RuntimeError("the _param_watch extension is missing: build it first (python __graft_entry__.py)") from e
+    return w
 
-    ``get`` returns a reference to the parameter struct, rebuilt when a parameter has another address or version, or
-    the module tree another structure, than when it was built; ``None`` when the block has to take the layer-by-layer
-    path (hooks on its submodules, or a submodule that is not this package's)."""
+
+class _BlockPlans:
+    """A block's (or stack's) parameters as its native entry point takes them, and its plans per shape.
+
+    ``get`` returns the parameter structs, rebuilt when a parameter has another address or version, or the module tree
+    another structure, than when they were built; ``None`` when the call has to take the layer-by-layer path (hooks on
+    submodules, a submodule that is not this package's, parameters that track no versions)."""
 
     def __init__(self):
         self._epoch = -1
+        self._ref = None
         self._plans = {}
 
     def __reduce__(self):   # a copied or unpickled module builds its own
@@ -208,49 +217,44 @@ class _BlockPlans:
     def _build(self, block, dtype, device):
         self._epoch = _structure_epoch
         self._hooks, self._ref, self._plans = [], None, {}
+        self._dtype, self._device = dtype, device
         plain = block._plan_submodules()
         if plain is None:
             return
         for m in plain:
             self._hooks += [m._forward_hooks, m._forward_pre_hooks]
-        self._slots = [(m._parameters, n) for m in block.modules() for n, t in m._parameters.items() if t is not None]
-        self._dtype, self._device = dtype, device
-        tensors = [d[n] for d, n in self._slots]
-        self._ptrs, self._versions = [t.data_ptr() for t in tensors], [t._version for t in tensors]
-        self._struct, self._keep = block._native_params(dtype, device)
-        self._ref = ctypes.byref(self._struct)
+        w = _param_watch()
+        self._changed = w.changed
+        self._watch = w.make([(m._parameters, n) for m in block.modules() for n, t in m._parameters.items()
+                              if t is not None])
+        if self._watch is not None:
+            self._ref, self._keep = block._native_params(dtype, device)
 
     def get(self, block, dtype, device):
-        if self._epoch == _structure_epoch and self._ref is not None and dtype == self._dtype and device == self._device:
-            try:
-                tensors = [d[n] for d, n in self._slots]
-                if [t.data_ptr() for t in tensors] == self._ptrs and [t._version for t in tensors] == self._versions:
-                    return None if any(self._hooks) else self._ref
-            except (KeyError, AttributeError, RuntimeError):   # replaced by something else, or without versions
-                return None
-        elif self._epoch == _structure_epoch and self._ref is None:
-            return None
-        self._build(block, dtype, device)
-        return None if any(self._hooks) else self._ref
+        if (self._epoch != _structure_epoch or dtype != self._dtype or device != self._device
+                or (self._ref is not None and self._changed(self._watch))):
+            self._build(block, dtype, device)
+        return None if self._ref is None or any(self._hooks) else self._ref
 
-    def plan(self, block, B, N, dtype, flags):
-        p = self._plans.get((B, N, dtype, flags))
+    def plan(self, block, *key):
+        p = self._plans.get(key)
         if p is None:
             if len(self._plans) >= 64:
                 self._plans.clear()
-            p = self._plans[(B, N, dtype, flags)] = block._native_plan(B, N, dtype, flags)
+            p = self._plans[key] = block._native_plan(*key)
         return p
 
 
 def _native_state(block, z):
-    """(parameter reference, dtype code) for the native path of ``block`` on z [*, N, N, c], or None."""
+    """(parameter structs, dtype code) for the native path of ``block`` on z, or None."""
     if not z.is_cuda or block.training or z.dtype not in (torch.bfloat16, torch.float32):
         return None
-    try:
-        ref = block._plans.get(block, z.dtype, z.device)
-    except RuntimeError:   # parameters that track no versions (inference tensors): nothing to key a plan on
-        return None
+    ref = block._plans.get(block, z.dtype, z.device)
     return None if ref is None else (ref, lib.dtype_code(z.dtype))
+
+
+def _pointers(tensors):
+    return [None if t is None else t.data_ptr() for t in tensors]
 
 
 def _mask_like(mask, shape, dtype):
@@ -395,12 +399,16 @@ class ConditionedTransitionBlock(_Tracked):
         self.linear_out = Linear(n * c_a, c_a, **linear_init_params.linear_out)
         self._packed = _PackedParams()
 
-    def _params(self, dtype, device):
+    def _tensors(self):
         ln = self.layer_norm
-        return self._packed.get(
-            (ln.layer_norm_s.weight, ln.linear_g.weight, ln.linear_g.bias, ln.linear_s.weight,
-             self.swiglu.linear_a.weight, self.swiglu.linear_b.weight, self.linear_g.weight,
-             self.linear_g.bias, self.linear_out.weight), dtype, device, adjacent=((1, 3), (4, 5)))
+        return (ln.layer_norm_s.weight, ln.linear_g.weight, ln.linear_g.bias, ln.linear_s.weight,
+                self.swiglu.linear_a.weight, self.swiglu.linear_b.weight, self.linear_g.weight,
+                self.linear_g.bias, self.linear_out.weight)
+
+    _cond_group = (1, 3, 6)   # the three projections of s among _tensors()
+
+    def _params(self, dtype, device):
+        return self._packed.get(self._tensors(), dtype, device, adjacent=(self._cond_group, (4, 5)))
 
     def _run(self, a, s, mask, in_place: bool):
         ac = a.contiguous().view(-1, self.c_a)
@@ -443,7 +451,7 @@ class AttentionPairBias(_Tracked):
                              linear_init_params=linear_init_params.mha)
         self._packed = _PackedParams()
 
-    def _params(self, dtype, device):
+    def _tensors(self):
         if self.use_ada_layer_norm:
             ln = self.layer_norm_a
             head = (None, None, ln.layer_norm_s.weight, ln.linear_g.weight, ln.linear_g.bias,
@@ -451,11 +459,15 @@ class AttentionPairBias(_Tracked):
         else:
             head = (self.layer_norm_a.weight, self.layer_norm_a.bias, None, None, None, None, None, None)
         m = self.mha
-        return self._packed.get(
-            head + (self.layer_norm_z.weight, self.layer_norm_z.bias, self.linear_z.weight,
-                    m.linear_q.weight, m.linear_q.bias, m.linear_k.weight, m.linear_v.weight,
-                    m.linear_g.weight, m.linear_o.weight), dtype, device,
-            adjacent=((11, 15, 13, 14), (3, 5)))   # q, g, k, v projections; the two AdaLN projections
+        return head + (self.layer_norm_z.weight, self.layer_norm_z.bias, self.linear_z.weight,
+                       m.linear_q.weight, m.linear_q.bias, m.linear_k.weight, m.linear_v.weight,
+                       m.linear_g.weight, m.linear_o.weight)
+
+    _cond_group = (3, 5, 6)   # the three projections of s among _tensors()
+
+    def _params(self, dtype, device):
+        return self._packed.get(self._tensors(), dtype, device,
+                                adjacent=((11, 15, 13, 14), self._cond_group))   # q, g, k, v; the projections of s
 
     def can_hoist_pair_bias(self, z) -> bool:
         """Whether ``project_pair_bias`` has a kernel for this layer (c_z = 128, 16 heads, bf16 or fp32)."""
@@ -480,22 +492,13 @@ class AttentionPairBias(_Tracked):
             return lib.pair_bias_project_tiles(zc, prm[8], prm[9], prm[10])
         return lib.pair_bias_project(zc, prm[8], prm[9], prm[10])
 
-    def _run(self, a, z, s, mask, in_place: bool, high_precision: bool = False, pair_bias=None):
-        """``high_precision`` (the reference's ``use_high_precision_attention``, which computes logits and softmax
-        in fp32: openfold3/core/model/primitives/attention.py:99-120, 314-339): bf16 inputs are evaluated by the
-        fp32 validation kernels (true fp32 products everywhere) and the result is rounded once at the end."""
-        if high_precision and a.dtype != torch.float32:
-            f32 = lambda t: None if t is None else t.float()
-            upd = self._run(f32(a), f32(z), f32(s), f32(mask), in_place=False)
-            if in_place:
-                a.add_(upd.to(a.dtype))
-                return a
-            return upd.to(a.dtype)
+    def _operands(self, a, z, s, mask):
+        """a [Ba, N, C], z [Bz, N, N, C_z], s, mask as the kernels take them: samples that share a pair tensor are
+        consecutive."""
         N = a.shape[-2]
         batch = a.shape[:-2]
         ac = a.contiguous().view(-1, N, self.c_q)
-        Ba = ac.shape[0]
-        # z's batch dims broadcast against a's; samples that share one pair tensor must be consecutive
+        # z's batch dims broadcast against a's
         zb = z.shape[:-3]
         zb = (1,) * (len(batch) - len(zb)) + tuple(zb)
         lead = 0
@@ -512,8 +515,23 @@ class AttentionPairBias(_Tracked):
             sc = s.expand(*batch, N, self.c_s).contiguous().view(-1, N, self.c_s)
         m = _mask_like(mask, a.shape[:-1], a.dtype)
         m = None if m is None else m.view(-1, N)
+        assert ac.shape[0] % zc.shape[0] == 0
+        return ac, zc, sc, m
+
+    def _run(self, a, z, s, mask, in_place: bool, high_precision: bool = False, pair_bias=None):
+        """``high_precision`` (the reference's ``use_high_precision_attention``, which computes logits and softmax
+        in fp32: openfold3/core/model/primitives/attention.py:99-120, 314-339): bf16 inputs are evaluated by the
+        fp32 validation kernels (true fp32 products everywhere) and the result is rounded once at the end."""
+        if high_precision and a.dtype != torch.float32:
+            f32 = lambda t: None if t is None else t.float()
+            upd = self._run(f32(a), f32(z), f32(s), f32(mask), in_place=False)
+            if in_place:
+                a.add_(upd.to(a.dtype))
+                return a
+            return upd.to(a.dtype)
+        N = a.shape[-2]
+        ac, zc, sc, m = self._operands(a, z, s, mask)
         out = ac if in_place else torch.empty_like(ac)
-        assert Ba % zc.shape[0] == 0
         if pair_bias is not None and pair_bias.dtype == torch.bfloat16:   # bias tiles of the tensor-core attention
             assert pair_bias.shape == (zc.shape[0], 16, (N + 31) // 32, N, 32) and a.dtype == torch.bfloat16
             lib.attn_pair_bias_forward_pretiles(ac, pair_bias, sc, m, out, self._params(a.dtype, a.device),
@@ -580,7 +598,7 @@ class PairBlock(_Tracked):
         parts = [m._params(dtype, device) for m in (self.tri_mul_out, self.tri_mul_in, self.tri_att_start,
                                                     self.tri_att_end, self.pair_transition)]
         kinds = (lib.TrimulParams, lib.TrimulParams, lib.TriattnParams, lib.TriattnParams, lib.TransitionParams)
-        return lib.PairBlockParams(*[k(*[t.data_ptr() for t in p]) for k, p in zip(kinds, parts)]), parts
+        return lib.PairBlockParams(*[k(*_pointers(p)) for k, p in zip(kinds, parts)]), parts
 
     def _native_dims(self, B, N):
         mul, att = self.tri_mul_out, self.tri_att_start
@@ -664,9 +682,8 @@ class PairFormerBlock(_Tracked):
     def _native_params(self, dtype, device):
         pair, keep = self.pair_stack._native_params(dtype, device)
         attn, trans = self.attn_pair_bias._params(dtype, device), self.single_transition._params(dtype, device)
-        ptr = lambda ts: [None if t is None else t.data_ptr() for t in ts]  # noqa: E731
-        return (lib.PairformerBlockParams(pair, lib.AttnPairBiasParams(*ptr(attn)), lib.TransitionParams(*ptr(trans))),
-                (keep, attn, trans))
+        return (lib.PairformerBlockParams(pair, lib.AttnPairBiasParams(*_pointers(attn)),
+                                          lib.TransitionParams(*_pointers(trans))), (keep, attn, trans))
 
     def _native_plan(self, B, N, dtype, flags):
         d, a = self.pair_stack._native_dims(B, N), self.attn_pair_bias
@@ -851,30 +868,99 @@ class DiffusionTransformer(_Tracked):
         # in every call (what the reference does).
         self.hoist_pair_bias = True
         self._bias_cache = None   # (weakref to z, z._version, parameter versions, [bias per block])
+        self._plans = _BlockPlans()
 
-    def _pair_biases(self, z):
+    def _plan_submodules(self):
+        blocks = list(self.blocks)
+        own = {"attention_pair_bias": AttentionPairBias, "conditioned_transition": ConditionedTransitionBlock}
+        if type(self) is not DiffusionTransformer or not blocks:
+            return None
+        for b in blocks:
+            if type(b) is not DiffusionTransformerBlock or any(type(b._modules.get(n)) is not c for n, c in own.items()):
+                return None
+        kinds = {(b.attention_pair_bias.c_q, b.attention_pair_bias.c_s, b.attention_pair_bias.c_z,
+                  b.attention_pair_bias.no_heads, b.attention_pair_bias.c_hidden, b.attention_pair_bias.inf,
+                  b.attention_pair_bias.use_ada_layer_norm, b.conditioned_transition.c_a, b.conditioned_transition.c_s,
+                  b.conditioned_transition.n) for b in blocks}
+        k = next(iter(kinds))
+        return blocks if len(kinds) == 1 and k[0] == k[7] and k[1] == k[8] else None
+
+    def _native_params(self, dtype, device):
+        """Parameter structs of all blocks. The projections of s lie back to back over the whole stack (the library
+        computes those of several blocks in one launch)."""
+        conv = lambda t: None if t is None else t.detach().to(device=device, dtype=dtype).contiguous()  # noqa: E731
+        layers = [m for b in self.blocks for m in (b.attention_pair_bias, b.conditioned_transition)]
+        cond = None
+        if self.blocks[0].attention_pair_bias.use_ada_layer_norm:
+            raw = [m._tensors() for m in layers]
+            cond = torch.stack([r[i].detach().to(device=device, dtype=dtype) for m, r in zip(layers, raw)
+                                for i in m._cond_group]).view(len(layers), 3, *raw[0][layers[0]._cond_group[0]].shape)
+        vals = []
+        for n, m in enumerate(layers):
+            group = m._cond_group if cond is not None else ()
+            t = [None if i in group else conv(t) for i, t in enumerate(m._tensors())]
+            for j, i in enumerate(group):
+                t[i] = cond[n, j]
+            vals.append(t)
+        attn = (lib.AttnPairBiasParams * len(self.blocks))(*[lib.AttnPairBiasParams(*_pointers(v)) for v in vals[0::2]])
+        trans = (lib.CondTransitionParams * len(self.blocks))(
+            *[lib.CondTransitionParams(*_pointers(v)) for v in vals[1::2]])
+        return (attn, trans), vals
+
+    def _native_plan(self, Ba, Bz, N, dtype, flags, with_bias):
+        m = self.blocks[0].attention_pair_bias
+        dims = lib.DiffusionDims(Ba=Ba, Bz=Bz, N=N, c_a=m.c_q, c_s=m.c_s, c_z=m.c_z, H=m.no_heads, d=m.c_hidden,
+                                 n=self.blocks[0].conditioned_transition.n, inf=m.inf)
+        return lib.DiffusionPlan(dims, dtype, flags, len(self.blocks), with_bias)
+
+    def _run_native(self, a, s, z, mask, mask_trans):
+        """In place on the contiguous a; False if the native path does not take this call."""
+        st = _native_state(self, a)
+        if st is None or z.dtype != a.dtype or s is None or s.dtype != a.dtype:
+            return False
+        m0 = self.blocks[0].attention_pair_bias
+        if not m0.use_ada_layer_norm:   # the attention takes no s then, the transitions still do
+            return False
+        ac, zc, sc, m = m0._operands(a, z, s, mask)
+        biases = self._pair_biases(z, token=st[0])
+        flags = (lib.extra_flags | lib.FLAG_ADA_LN) | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
+        plan = self._plans.plan(self, ac.shape[0], zc.shape[0], a.shape[-2], st[1], flags, biases[0] is not None)
+        lib.diffusion_stack_forward(ac, sc, zc, m, biases, plan, st[1], flags, st[0])
+        return True
+
+    def _pair_biases(self, z, token=None):
+        """The projected pair bias of every block, or Nones. ``token``: an object that stands for unchanged parameters
+        while it is the same (the native path's parameter structs)."""
         import weakref
 
-        apbs = [b.attention_pair_bias for b in self.blocks]
-        if not (self.hoist_pair_bias and all(m.can_hoist_pair_bias(z) for m in apbs)):
-            return [None] * len(apbs)
-        pv = tuple((m.layer_norm_z.weight._version, m.linear_z.weight._version, m.linear_z.weight.data_ptr())
-                   for m in apbs)
         try:
             zv = z._version
         except RuntimeError:   # inference tensors do not track versions: nothing to key the cache on
-            return [m.project_pair_bias(z) for m in apbs]
+            zv = None
         c = self._bias_cache
-        if c is not None and c[0]() is z and c[1] == zv and c[2] == pv:
+        if (self.hoist_pair_bias and token is not None and c is not None and c[4] is token and c[0]() is z
+                and c[1] == zv and lib.extra_flags == 0):
             return c[3]
-        biases = [m.project_pair_bias(z) for m in apbs]
-        self._bias_cache = (weakref.ref(z), zv, pv, biases)
+        apbs = [b.attention_pair_bias for b in self.blocks]
+        if not (self.hoist_pair_bias and all(m.can_hoist_pair_bias(z) for m in apbs)):
+            return [None] * len(apbs)
+        if zv is None:
+            return [m.project_pair_bias(z) for m in apbs]
+        pv = tuple((m.layer_norm_z.weight._version, m.linear_z.weight._version, m.linear_z.weight.data_ptr())
+                   for m in apbs)
+        if c is not None and c[0]() is z and c[1] == zv and c[2] == pv:
+            biases = c[3]
+        else:
+            biases = [m.project_pair_bias(z) for m in apbs]
+        self._bias_cache = (weakref.ref(z), zv, pv, biases, token)
         return biases
 
     def forward(self, a, s, z, mask=None, use_deepspeed_evo_attention=False, use_cueq_triangle_kernels=False,
                 use_lma=False, use_high_precision_attention=False, _mask_trans=True):
         _forward_only(self, a, s, z)
         a = a.clone(memory_format=torch.contiguous_format)
+        if not use_high_precision_attention and self._run_native(a, s, z, mask, _mask_trans):
+            return a
         biases = self._pair_biases(z)
         for b, pb in zip(self.blocks, biases):
             a = b(a, s, z, mask=mask, use_high_precision_attention=use_high_precision_attention,
