@@ -15,7 +15,7 @@ int trimul_dispatch(const void* z, const void* mask, void* out, int B, int N, in
                     int dtype, int flags, const of3_trimul_params* p, Arena& ws, cudaStream_t st) {
     if (use_fast(dtype, flags) && fast::trimul_supported(c_z, c_h))
         return fast::trimul((const __nv_bfloat16*)z, (const __nv_bfloat16*)mask, (__nv_bfloat16*)out,
-                            B, N, flags, p, ws, st);
+                            B, N, c_z, flags, p, ws, st);
     if (dtype == OF3_DTYPE_BF16)
         return generic::trimul<__nv_bfloat16>((const __nv_bfloat16*)z, (const __nv_bfloat16*)mask,
                                               (__nv_bfloat16*)out, B, N, c_z, c_h, flags, p, ws, st);
@@ -28,7 +28,7 @@ int triattn_dispatch(const void* z, const void* mask, void* out, int B, int N, i
                      cudaStream_t st) {
     if (use_fast(dtype, flags) && fast::triattn_supported(c_z, H, d, N))
         return fast::triattn((const __nv_bfloat16*)z, (const __nv_bfloat16*)mask, (__nv_bfloat16*)out,
-                             B, N, inf, flags, p, ws, st);
+                             B, N, c_z, inf, flags, p, ws, st);
     if (dtype == OF3_DTYPE_BF16)
         return generic::triattn<__nv_bfloat16>((const __nv_bfloat16*)z, (const __nv_bfloat16*)mask,
                                                (__nv_bfloat16*)out, B, N, c_z, H, d, inf, flags, p,
@@ -42,7 +42,7 @@ int transition_dispatch(const void* x, const void* mask, void* out, long long ro
                         cudaStream_t st) {
     if (use_fast(dtype, flags) && fast::transition_supported(c, n))
         return fast::transition((const __nv_bfloat16*)x, (const __nv_bfloat16*)mask,
-                                (__nv_bfloat16*)out, rows, flags, p, ws, st);
+                                (__nv_bfloat16*)out, rows, c, flags, p, ws, st);
     if (use_fast(dtype, flags) && fast::transition_wide_supported(c, n))
         return fast::transition_wide((const __nv_bfloat16*)x, (const __nv_bfloat16*)mask, (__nv_bfloat16*)out, rows,
                                      c, n, flags, p, ws, st);

@@ -374,7 +374,7 @@ int attn_pair_bias_rows(const bf16* a, const float* pair_bias_rows, const bf16* 
 }
 
 // SwiGLU transition for widths without the fused row-tile kernel (bf16, c a multiple of 64).
-bool transition_wide_supported(int c, int n) { return c % 64 == 0 && c <= kMaxRowWidth && !(c == 128 && n == 4); }
+bool transition_wide_supported(int c, int n) { return c % 64 == 0 && c <= kMaxRowWidth && !transition_supported(c, n); }
 
 int transition_wide(const bf16* x, const bf16* mask, bf16* out, long long rows, int c, int n, int flags,
                     const of3_transition_params* p, Arena& ws, cudaStream_t st) {

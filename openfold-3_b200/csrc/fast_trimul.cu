@@ -1,4 +1,4 @@
-// Triangle multiplicative update, bf16 / tcgen05 family (c_z = c_hidden = 128).
+// Triangle multiplicative update, bf16 / tcgen05 family (c_z = c_hidden = 128, or 64 in the template stack).
 //
 // Three kernels per layer, all fed by TMA:
 //   trimul_in   z tile -> LayerNorm_in (in place) -> the four projections a_p, a_g, b_p, b_g TRANSPOSED
@@ -44,24 +44,30 @@ __device__ __forceinline__ TileCoord tile_coord(long long t, int R, int tiles_pe
 // =====================================================================================
 // trimul_in
 // =====================================================================================
+// 128 channels: the four weights are four A operands and a tile makes two jobs, its a and its b projection. 64
+// channels: the A operands are [a_p; b_p] and [a_g; b_g], 128 rows each, and a tile is one job.
+template <int C>
 struct InSmem {
-    static constexpr uint32_t kW = 0;                          // 2 k-blocks x [512 rows x 128 B]
-    static constexpr uint32_t kWKb = 512 * 128;                // 65536
-    static constexpr uint32_t kZ = 2 * kWKb;                   // 2 stages x 32768
-    static constexpr uint32_t kGamma = kZ + 2 * kTileBytes;    // 128 floats
+    static constexpr int kJobs = C / 64;                       // GEMM pairs (projection, gate) per tile
+    static constexpr int kStages = C == 128 ? 2 : 4;           // z tiles in flight
+    static constexpr uint32_t kW = 0;                          // C / 64 k-blocks x [4 C rows x 128 B]
+    static constexpr uint32_t kWKb = 4 * C * 128;
+    static constexpr uint32_t kZ = C / 64 * kWKb;              // stages of one tile
+    static constexpr uint32_t kGamma = kZ + kStages * tile_bytes<C>();   // C floats
     static constexpr uint32_t kBeta = kGamma + 512;
-    static constexpr uint32_t kMask = kBeta + 512;             // 4 x 128 floats: 0.5 * mask of the tile's positions
-    static constexpr uint32_t kBars = kMask + 4 * 512;
-    static constexpr uint32_t kTotal = kBars + 128;
+    static constexpr uint32_t kMask = kBeta + 512;             // ring of 128 floats: 0.5 * mask of the tile's positions
+    static constexpr int kMaskRing = C == 128 ? 4 : 8;
+    static constexpr uint32_t kBars = kMask + kMaskRing * 512;
+    static constexpr uint32_t kTotal = kBars + 192;
     static constexpr uint32_t kDyn = kTotal + 1024;
 };
 
 // outgoing: tmZ is 3-D {c, second index, b*N + first index}; incoming: 4-D {c, second, first, b}
 constexpr int kInLnWarps = 8;    // two threads per position
-constexpr int kInEpiSets = 2;    // epilogue warp sets: a / b projection x first / second half of the tile's positions
+constexpr int kInEpiSets = 2;    // epilogue warp sets, one per TMEM slot
 constexpr int kInThreads = 32 * (2 + kInLnWarps + 4 * kInEpiSets);  // producer, MMA, LayerNorm and epilogue warps
 
-template <bool kOutgoing>
+template <int C, bool kOutgoing>
 __global__ void __launch_bounds__(kInThreads, 1)
 trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmWap,
                  const __grid_constant__ CUtensorMap tmWag, const __grid_constant__ CUtensorMap tmWbp,
@@ -69,21 +75,23 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                  const __nv_bfloat16* __restrict__ ln_w, const __nv_bfloat16* __restrict__ ln_b,
                  __nv_bfloat16* __restrict__ a_t, __nv_bfloat16* __restrict__ b_t, int B, int R,
                  int N, int ld, int group_shift, long long group_stride, int wide_stores, int* status) {
+    using Sm = InSmem<C>;
+    constexpr int kSt = Sm::kStages;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
-    float* gamma = reinterpret_cast<float*>(gbase + InSmem::kGamma);
-    float* beta = reinterpret_cast<float*>(gbase + InSmem::kBeta);
-    float* mask05 = reinterpret_cast<float*>(gbase + InSmem::kMask);
-    const uint32_t bars = sbase + InSmem::kBars;
+    float* gamma = reinterpret_cast<float*>(gbase + Sm::kGamma);
+    float* beta = reinterpret_cast<float*>(gbase + Sm::kBeta);
+    float* mask05 = reinterpret_cast<float*>(gbase + Sm::kMask);
+    const uint32_t bars = sbase + Sm::kBars;
     const uint32_t w_full = bars;
     auto z_full = [&](int s) { return bars + 8u * (1 + s); };
-    auto z_empty = [&](int s) { return bars + 8u * (3 + s); };
-    auto a_ready = [&](int s) { return bars + 8u * (5 + s); };
-    auto slot_full = [&](int q) { return bars + 8u * (7 + q); };
-    auto slot_empty = [&](int q) { return bars + 8u * (9 + q); };
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + InSmem::kBars + 96);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + InSmem::kBars + 104);
+    auto z_empty = [&](int s) { return bars + 8u * (1 + kSt + s); };
+    auto a_ready = [&](int s) { return bars + 8u * (1 + 2 * kSt + s); };
+    auto slot_full = [&](int q) { return bars + 8u * (1 + 3 * kSt + q); };
+    auto slot_empty = [&](int q) { return bars + 8u * (3 + 3 * kSt + q); };
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 160);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 168);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_per_line = (N + kRows - 1) / kRows;
@@ -91,18 +99,20 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
 
     if (threadIdx.x == 0) {
         mbar_init(w_full, 1);
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < kSt; ++s) {
             mbar_init(z_full(s), 1);
             mbar_init(z_empty(s), 1);
             mbar_init(a_ready(s), kInLnWarps);
-            mbar_init(slot_full(s), 1);
-            mbar_init(slot_empty(s), 2 * kInEpiSets);
+        }
+        for (int q = 0; q < 2; ++q) {
+            mbar_init(slot_full(q), 1);
+            mbar_init(slot_empty(q), 4);
         }
         *abort_flag = 0;
         mbar_fence_init();
         prefetch_tmap(&tmZ);
     }
-    if (threadIdx.x < 128) {
+    if (threadIdx.x < C) {
         gamma[threadIdx.x] = __bfloat162float(ln_w[threadIdx.x]);
         beta[threadIdx.x] = __bfloat162float(ln_b[threadIdx.x]);
     }
@@ -114,27 +124,29 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr;
+    grid_trigger();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
-            mbar_arrive_expect_tx(w_full, 2 * InSmem::kWKb);
-            const CUtensorMap* wm[4] = {&tmWap, &tmWag, &tmWbp, &tmWbg};
+            mbar_arrive_expect_tx(w_full, C / 64 * Sm::kWKb);
+            // slab order: C = 128: a_p, a_g, b_p, b_g; C = 64: a_p, b_p | a_g, b_g
+            const CUtensorMap* wm[4] = {&tmWap, C == 128 ? &tmWag : &tmWbp, C == 128 ? &tmWbp : &tmWag, &tmWbg};
             for (int w = 0; w < 4; ++w)
-                for (int kb = 0; kb < 2; ++kb)
-                    tma_load_2d(sbase + InSmem::kW + kb * InSmem::kWKb + w * 128 * 128, wm[w], w_full,
-                                kb * 64, 0);
+                for (int kb = 0; kb < C / 64; ++kb)
+                    tma_load_2d(sbase + Sm::kW + kb * Sm::kWKb + w * C * 128, wm[w], w_full, kb * 64, 0);
+            grid_wait();
             uint32_t it = 0;
             for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
-                const int s = it & 1;
-                if (!mbar_wait(z_empty(s), ((it >> 1) & 1u) ^ 1u, abort_flag)) {
+                const int s = it % kSt;
+                if (!mbar_wait(z_empty(s), ((it / kSt) & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidIn, 1);
                     break;
                 }
                 const TileCoord tc = tile_coord(t, R, tiles_per_line);
-                mbar_arrive_expect_tx(z_full(s), kTileBytes);
-                const uint32_t dst = sbase + InSmem::kZ + s * kTileBytes;
-                for (int kb = 0; kb < 2; ++kb) {
+                mbar_arrive_expect_tx(z_full(s), tile_bytes<C>());
+                const uint32_t dst = sbase + Sm::kZ + s * tile_bytes<C>();
+                for (int kb = 0; kb < C / 64; ++kb) {
                     if (kOutgoing)
                         tma_load_3d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tc.t0,
                                     tc.b * R + tc.fixed);
@@ -152,14 +164,15 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
             if (!ok) report_wait_failure(status, abort_flag, kKidIn, 2);
             uint32_t it = 0;
             for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
-                const int s = it & 1;
-                if (!mbar_wait(a_ready(s), (it >> 1) & 1u, abort_flag)) {
+                const int s = it % kSt;
+                if (!mbar_wait(a_ready(s), (it / kSt) & 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidIn, 3);
                     break;
                 }
-                const uint32_t ztile = sbase + InSmem::kZ + s * kTileBytes;
-                for (int q = 0; q < 2; ++q) {
-                    if (!mbar_wait(slot_empty(q), (it & 1u) ^ 1u, abort_flag)) {
+                const uint32_t ztile = sbase + Sm::kZ + s * tile_bytes<C>();
+                for (int q = 0; q < Sm::kJobs; ++q) {
+                    const uint32_t job = it * Sm::kJobs + q, slot = job & 1u;
+                    if (!mbar_wait(slot_empty(slot), ((job >> 1) & 1u) ^ 1u, abort_flag)) {
                         report_wait_failure(status, abort_flag, kKidIn, 4);
                         ok = false;
                         break;
@@ -167,18 +180,18 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                     tc_fence_after_sync();
                     // D[channel][position] = W[channel][:] . LN(z)[position][:]: projection, then gate
                     for (int hg = 0; hg < 2; ++hg) {
-                        const uint32_t w_tile = sbase + InSmem::kW + (q * 2 + hg) * 128 * 128;
+                        const uint32_t w_tile = sbase + Sm::kW + (q * 2 + hg) * 128 * 128;
 #pragma unroll
-                        for (int kb = 0; kb < 2; ++kb) {
-                            const uint64_t ad = smem_desc_k_sw128(w_tile + kb * InSmem::kWKb);
+                        for (int kb = 0; kb < C / 64; ++kb) {
+                            const uint64_t ad = smem_desc_k_sw128(w_tile + kb * Sm::kWKb);
                             const uint64_t bd = smem_desc_k_sw128(ztile + kb * kKBlockBytes);
 #pragma unroll
                             for (int k4 = 0; k4 < 4; ++k4)
-                                mma_bf16(tmem_base + q * 256 + hg * 128, ad + 2u * k4, bd + 2u * k4, idesc,
+                                mma_bf16(tmem_base + slot * 256 + hg * 128, ad + 2u * k4, bd + 2u * k4, idesc,
                                          (kb != 0 || k4 != 0) ? 1u : 0u);
                         }
                     }
-                    mma_commit(slot_full(q));
+                    mma_commit(slot_full(slot));
                 }
                 if (ok) mma_commit(z_empty(s));
             }
@@ -188,19 +201,20 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         // lanes 0..15 their first 64 channels, lanes 16..31 the other 64 (statistics joined by one shuffle)
         const int row = (warp - 2) * 16 + (lane & 15);
         const int half = lane >> 4;
+        grid_wait();
         uint32_t it = 0;
         for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
-            const int s = it & 1;
-            if (!mbar_wait(z_full(s), (it >> 1) & 1u, abort_flag)) {
+            const int s = it % kSt;
+            if (!mbar_wait(z_full(s), (it / kSt) & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidIn, 5);
                 break;
             }
-            const uint32_t tile = sbase + InSmem::kZ + s * kTileBytes;
-            uint32_t raw[32];
-            load_half_row(tile, row, half, raw);
+            const uint32_t tile = sbase + Sm::kZ + s * tile_bytes<C>();
+            uint32_t raw[C / 4];
+            load_half_row<C>(tile, row, half, raw);
             float mean, rstd;
-            half_row_stats(raw, mean, rstd);
-            store_normalized_half_row(tile, row, half, raw, mean, rstd, gamma, beta);
+            half_row_stats<C>(raw, mean, rstd);
+            store_normalized_half_row<C>(tile, row, half, raw, mean, rstd, gamma, beta);
             const TileCoord tc = tile_coord(t, R, tiles_per_line);
             const int k = tc.t0 + row;
             float m = 0.f;   // positions past the end of the line are never stored
@@ -212,9 +226,10 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                     m = 0.5f * __bfloat162float(mask[lin]);
                 }
             }
-            // four mask buffers: the epilogue of tile `it` may still read its buffer while tile it + 2 is normalised;
-            // tile it + 4 cannot get here before that epilogue has released its TMEM slot
-            if (half == 0) mask05[(it & 3) * 128 + row] = m;
+            // The epilogue of tile `it` may still read its buffer while the next kStages tiles are normalised (and, with
+            // one job per tile, one tile more waits for the other TMEM slot); by tile it + kMaskRing it has released
+            // its slot
+            if (half == 0) mask05[(it % Sm::kMaskRing) * 128 + row] = m;
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(a_ready(s));
@@ -223,31 +238,34 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         // ---------------------------------------------------------------- epilogue warps: the first four take the a
         // projection (TMEM slot 0), the other four the b projection (slot 1); thread = output channel, columns =
         // positions
-        const int set = (warp - 2 - kInLnWarps) >> 2;
-        const int q = set / (kInEpiSets / 2), khalf = set % (kInEpiSets / 2);
-        constexpr int kSpan = kRows / (kInEpiSets / 2);   // positions per set
+        const int set = (warp - 2 - kInLnWarps) >> 2;   // TMEM slot of this set's jobs
         const int quad = warp & 3;
-        const int c = quad * 32 + lane;
+        const int lch = quad * 32 + lane;
+        const bool is_b = C == 128 ? set == 1 : lch >= 64;
+        const int c = lch & (C - 1);
         const long long cs = (long long)R * ld;
         // channel c lives at (c >> group_shift) * group_stride + (c & group_mask) * R * ld: one contiguous plane
-        // [128][R][ld] by default, or one group of channels per destination rank when the planes are about to be
+        // [C][R][ld] by default, or one group of channels per destination rank when the planes are about to be
         // exchanged
-        __nv_bfloat16* plane = (q == 0 ? a_t : b_t) + (long long)(c >> group_shift) * group_stride +
+        __nv_bfloat16* plane = (is_b ? b_t : a_t) + (long long)(c >> group_shift) * group_stride +
                                (long long)(c & ((1 << group_shift) - 1)) * cs;
-        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + q * 256;
-        uint32_t it = 0;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + set * 256;
+        grid_wait();
+        uint32_t it = 0, use = 0;
         for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+            if (C == 64 && (it & 1u) != (uint32_t)set) continue;   // one job per tile: the sets take turns
             const TileCoord tc = tile_coord(t, R, tiles_per_line);
             const int kmax = (N - tc.t0 < kRows) ? N - tc.t0 : kRows;   // positions of the tile that exist
-            if (!mbar_wait(slot_full(q), it & 1u, abort_flag)) {
+            if (!mbar_wait(slot_full(set), use & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidIn, 6);
                 break;
             }
+            ++use;
             tc_fence_after_sync();
-            const float* mk = mask05 + (it & 3) * 128;
+            const float* mk = mask05 + (it % Sm::kMaskRing) * 128;
             // the line pitch ld is a multiple of 8 elements, so a 16-byte store that starts below N ends inside the
             // row; with a pitch that is a multiple of 16 (and 32-byte aligned planes) the same holds for 32 bytes
-            __nv_bfloat16* dst = plane + (long long)tc.b * ((kC >> group_shift) * group_stride) +
+            __nv_bfloat16* dst = plane + (long long)tc.b * ((C >> group_shift) * group_stride) +
                                  (long long)tc.fixed * ld + tc.t0;
             // 16 positions per pass; the TMEM load of the next pass is in flight while this one is computed
             auto emit = [&](const uint32_t (&p)[16], const uint32_t (&g)[16], int k0) {
@@ -276,8 +294,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                     if (k0 + 8 < kmax) *reinterpret_cast<uint4*>(dst + k0 + 8) = make_uint4(o[4], o[5], o[6], o[7]);
                 }
             };
-            const int k_begin = khalf * kSpan;
-            const int k_end = (kmax < (khalf + 1) * kSpan) ? kmax : (khalf + 1) * kSpan;
+            const int k_begin = 0, k_end = kmax;
             uint32_t pa[16], ga[16], pb[16], gb[16];
             if (k_begin < k_end) {
                 tmem_ld16(taddr + k_begin, pa);
@@ -302,7 +319,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
             }
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(slot_empty(q));
+            if (lane == 0) mbar_arrive(slot_empty(set));
         }
     }
 
@@ -332,17 +349,17 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
-    float* gamma = reinterpret_cast<float*>(gbase + InSmem::kGamma);
-    float* beta = reinterpret_cast<float*>(gbase + InSmem::kBeta);
-    const uint32_t bars = sbase + InSmem::kBars;
+    float* gamma = reinterpret_cast<float*>(gbase + InSmem<128>::kGamma);
+    float* beta = reinterpret_cast<float*>(gbase + InSmem<128>::kBeta);
+    const uint32_t bars = sbase + InSmem<128>::kBars;
     const uint32_t w_full = bars;
     auto z_full = [&](int s) { return bars + 8u * (1 + s); };
     auto z_empty = [&](int s) { return bars + 8u * (3 + s); };
     auto a_ready = [&](int s) { return bars + 8u * (5 + s); };
     auto slot_full = [&](int q) { return bars + 8u * (7 + q); };
     auto slot_empty = [&](int q) { return bars + 8u * (9 + q); };
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + InSmem::kBars + 96);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + InSmem::kBars + 104);
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + InSmem<128>::kBars + 96);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + InSmem<128>::kBars + 104);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_per_line = (N + kRows - 1) / kRows;
@@ -373,16 +390,19 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr;
+    grid_trigger();
+    if (warp != 0 && warp != 1) grid_wait();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
-            mbar_arrive_expect_tx(w_full, 2 * InSmem::kWKb);
+            mbar_arrive_expect_tx(w_full, 2 * InSmem<128>::kWKb);
             const CUtensorMap* wm[4] = {&tmWap, &tmWag, &tmWbp, &tmWbg};
             for (int w = 0; w < 4; ++w)
                 for (int kb = 0; kb < 2; ++kb)
-                    tma_load_2d(sbase + InSmem::kW + kb * InSmem::kWKb + w * 128 * 128, wm[w], w_full,
+                    tma_load_2d(sbase + InSmem<128>::kW + kb * InSmem<128>::kWKb + w * 128 * 128, wm[w], w_full,
                                 kb * 64, 0);
+            grid_wait();
             uint32_t it = 0;
             for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
                 const int s = it & 1;
@@ -392,7 +412,7 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 }
                 const TileCoord tc = tile_coord(t, R, tiles_per_line);
                 mbar_arrive_expect_tx(z_full(s), kTileBytes);
-                const uint32_t dst = sbase + InSmem::kZ + s * kTileBytes;
+                const uint32_t dst = sbase + InSmem<128>::kZ + s * kTileBytes;
                 for (int kb = 0; kb < 2; ++kb) {
                     if (kOutgoing)
                         tma_load_3d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tc.t0,
@@ -423,8 +443,8 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                         break;
                     }
                     tc_fence_after_sync();
-                    mma_k128(tmem_base + q * 256, sbase + InSmem::kZ + s * kTileBytes,
-                             sbase + InSmem::kW + q * 256 * 128, InSmem::kWKb, idesc, false);
+                    mma_k128(tmem_base + q * 256, sbase + InSmem<128>::kZ + s * kTileBytes,
+                             sbase + InSmem<128>::kW + q * 256 * 128, InSmem<128>::kWKb, idesc, false);
                     mma_commit(slot_full(q));
                 }
                 if (ok) mma_commit(z_empty(s));
@@ -440,7 +460,7 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidIn, 5);
                 break;
             }
-            const uint32_t tile = sbase + InSmem::kZ + s * kTileBytes;
+            const uint32_t tile = sbase + InSmem<128>::kZ + s * kTileBytes;
             uint32_t raw[64];
             load_row(tile, row, raw);
             float mean, rstd;
@@ -527,29 +547,35 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
 // =====================================================================================
 // trimul_out
 // =====================================================================================
+template <int C>
 struct OutSmem {
-    static constexpr uint32_t kWg = 0;                        // [128 x 128] as 2 k-blocks of 16 KB
-    static constexpr uint32_t kWz = kTileBytes;
-    static constexpr uint32_t kZ = 2 * kTileBytes;            // 2 groups x 32768 (z tile, then output)
-    static constexpr uint32_t kX = kZ + 2 * kTileBytes;       // 2 groups x 32768 (x tile [c][j], then A)
-    static constexpr uint32_t kParams = kX + 2 * kTileBytes;  // gamma_in, beta_in, gamma_out, beta_out
+    static constexpr uint32_t kWBytes = C * C * 2;            // a weight as C / 64 k-blocks of [C rows x 128 B]
+    static constexpr uint32_t kWg = 0;
+    static constexpr uint32_t kWz = kWBytes;
+    static constexpr uint32_t kZ = 2 * kWBytes;                    // 2 groups: z tile, then output
+    static constexpr uint32_t kX = kZ + 2 * tile_bytes<C>();       // 2 groups: x tile [c][j], then A
+    static constexpr uint32_t kParams = kX + 2 * tile_bytes<C>();  // gamma_in, beta_in, gamma_out, beta_out
     static constexpr uint32_t kBars = kParams + 4 * 512;
     static constexpr uint32_t kTotal = kBars + 128;
     static constexpr uint32_t kDyn = kTotal + 1024;
 };
 
-__global__ void __launch_bounds__(320, 1)
+// 64 channels: half the registers, tiles and tensor memory, so two CTAs share an SM (four tiles in flight)
+template <int C>
+__global__ void __launch_bounds__(320, C == 128 ? 1 : 2)
 trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmX,
                   const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ CUtensorMap tmWg,
                   const __grid_constant__ CUtensorMap tmWz, const __nv_bfloat16* __restrict__ ln_in_w,
                   const __nv_bfloat16* __restrict__ ln_in_b, const __nv_bfloat16* __restrict__ ln_out_w,
                   const __nv_bfloat16* __restrict__ ln_out_b, int B, int R, int N, int add_residual,
                   int* status) {
+    using Sm = OutSmem<C>;
+    constexpr int kTm = 2 * C;   // tensor-memory columns of a group: gate, update
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
-    float* prm = reinterpret_cast<float*>(gbase + OutSmem::kParams);
-    const uint32_t bars = sbase + OutSmem::kBars;
+    float* prm = reinterpret_cast<float*>(gbase + Sm::kParams);
+    const uint32_t bars = sbase + Sm::kBars;
     const uint32_t w_full = bars;
     // The x buffer is free as soon as the group's GEMMs have read it (the result goes over the z buffer), so
     // the next x tile is fetched during the epilogue; the z buffer is free once the output store has read it,
@@ -561,8 +587,8 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     auto d_full = [&](int g) { return bars + 8u * (7 + g); };   // MMAs of the group's tile done
     auto z_full = [&](int g) { return bars + 8u * (9 + g); };   // TMA landed: z tile
     auto x_empty = [&](int g) { return bars + 8u * (11 + g); };  // MMAs have read the x buffer
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + OutSmem::kBars + 112);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + OutSmem::kBars + 116);
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 112);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 116);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_per_line = (N + kRows - 1) / kRows;
@@ -586,29 +612,32 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
         prefetch_tmap(&tmX);
         prefetch_tmap(&tmOut);
     }
-    if (threadIdx.x < 128) {
+    if (threadIdx.x < C) {
         prm[threadIdx.x] = __bfloat162float(ln_in_w[threadIdx.x]);
         prm[128 + threadIdx.x] = __bfloat162float(ln_in_b[threadIdx.x]);
         prm[256 + threadIdx.x] = __bfloat162float(ln_out_w[threadIdx.x]);
         prm[384 + threadIdx.x] = __bfloat162float(ln_out_b[threadIdx.x]);
     }
     if (warp == 1) {
-        tmem_alloc(smem_u32((const void*)tmem_ptr), 512);
+        tmem_alloc(smem_u32((const void*)tmem_ptr), 2 * kTm);
         tmem_relinquish();
     }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr;
+    grid_trigger();
+    if (warp >= 2) grid_wait();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
-            mbar_arrive_expect_tx(w_full, 2 * kTileBytes);
-            for (int kb = 0; kb < 2; ++kb) {
-                tma_load_2d(sbase + OutSmem::kWg + kb * kKBlockBytes, &tmWg, w_full, kb * 64, 0);
-                tma_load_2d(sbase + OutSmem::kWz + kb * kKBlockBytes, &tmWz, w_full, kb * 64, 0);
+            mbar_arrive_expect_tx(w_full, 2 * Sm::kWBytes);
+            for (int kb = 0; kb < C / 64; ++kb) {
+                tma_load_2d(sbase + Sm::kWg + kb * C * 128, &tmWg, w_full, kb * 64, 0);
+                tma_load_2d(sbase + Sm::kWz + kb * C * 128, &tmWz, w_full, kb * 64, 0);
             }
+            grid_wait();
             for (long long lt = 0; lt < my_tiles; ++lt) {
                 const int g = (int)(lt & 1);
                 const uint32_t use = (uint32_t)(lt >> 1);
@@ -618,22 +647,22 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                     break;
                 }
                 // x tile: all 128 channels of positions (fixed, t0 .. t0+127), layout [c][j]
-                mbar_arrive_expect_tx(x_full(g), kTileBytes);
-                tma_load_3d(sbase + OutSmem::kX + g * kTileBytes, &tmX, x_full(g), tc.t0, tc.fixed, tc.b * kC);
+                mbar_arrive_expect_tx(x_full(g), tile_bytes<C>());
+                tma_load_3d(sbase + Sm::kX + g * tile_bytes<C>(), &tmX, x_full(g), tc.t0, tc.fixed, tc.b * C);
                 if (!mbar_wait(z_empty(g), (use & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidOut, 6);
                     break;
                 }
-                mbar_arrive_expect_tx(z_full(g), kTileBytes);
-                const uint32_t zdst = sbase + OutSmem::kZ + g * kTileBytes;
-                for (int kb = 0; kb < 2; ++kb)
+                mbar_arrive_expect_tx(z_full(g), tile_bytes<C>());
+                const uint32_t zdst = sbase + Sm::kZ + g * tile_bytes<C>();
+                for (int kb = 0; kb < C / 64; ++kb)
                     tma_load_3d(zdst + kb * kKBlockBytes, &tmZ, z_full(g), kb * 64, tc.t0, tc.b * R + tc.fixed);
             }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
         if (lane == 0) {
-            constexpr uint32_t idesc = idesc_bf16_f32(128, 128);
+            constexpr uint32_t idesc = idesc_bf16_f32(128, C);
             bool ok = mbar_wait(w_full, 0, abort_flag);
             if (!ok) report_wait_failure(status, abort_flag, kKidOut, 2);
             for (long long lt = 0; lt < my_tiles && ok; ++lt) {
@@ -644,11 +673,11 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                     break;
                 }
                 tc_fence_after_sync();
-                // gate = LN_in(z) W_g^T -> columns [0,128); update = LN_out(x) W_z^T -> [128,256)
-                mma_k128(tmem_base + g * 256, sbase + OutSmem::kZ + g * kTileBytes, sbase + OutSmem::kWg,
-                         kKBlockBytes, idesc, false);
-                mma_k128(tmem_base + g * 256 + 128, sbase + OutSmem::kX + g * kTileBytes,
-                         sbase + OutSmem::kWz, kKBlockBytes, idesc, false);
+                // gate = LN_in(z) W_g^T -> columns [0,C); update = LN_out(x) W_z^T -> [C,2C)
+                mma_rows<C>(tmem_base + g * kTm, sbase + Sm::kZ + g * tile_bytes<C>(), sbase + Sm::kWg, C * 128, idesc,
+                            false);
+                mma_rows<C>(tmem_base + g * kTm + C, sbase + Sm::kX + g * tile_bytes<C>(), sbase + Sm::kWz, C * 128, idesc,
+                            false);
                 mma_commit(d_full(g));
                 mma_commit(x_empty(g));
             }
@@ -659,8 +688,8 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         const int gtid = (warp - 2 - g * 4) * 32 + lane;  // 0..127 inside the group
-        const uint32_t ztile = sbase + OutSmem::kZ + g * kTileBytes;
-        const uint32_t xtile = sbase + OutSmem::kX + g * kTileBytes;
+        const uint32_t ztile = sbase + Sm::kZ + g * tile_bytes<C>();
+        const uint32_t xtile = sbase + Sm::kX + g * tile_bytes<C>();
         for (long long lt = g; lt < my_tiles; lt += 2) {
             const uint32_t use = (uint32_t)(lt >> 1);
             const TileCoord tc = tile_coord(blockIdx.x + lt * gridDim.x, R, tiles_per_line);
@@ -669,31 +698,31 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                 break;
             }
             float mean, rstd;
-            // --- x column of this position: 128 channels, [c][j] layout, stride 256 B
+            // --- x column of this position: C channels, [c][j] layout, stride 256 B
             {
-                uint32_t xraw[64];
+                uint32_t xraw[C / 2];
                 const uint32_t col = xtile + row * 2;
 #pragma unroll
-                for (int i = 0; i < 64; ++i) {
+                for (int i = 0; i < C / 2; ++i) {
                     uint32_t lo, hi;
                     if ((i & 7) == 0) asm volatile("" ::: "memory");  // cap the loads in flight per batch
                     asm volatile("ld.shared.u16 %0, [%1];" : "=r"(lo) : "r"(col + (2 * i) * 256));
                     asm volatile("ld.shared.u16 %0, [%1];" : "=r"(hi) : "r"(col + (2 * i + 1) * 256));
                     xraw[i] = lo | (hi << 16);
                 }
-                row_stats(xraw, mean, rstd);
+                row_stats<C>(xraw, mean, rstd);
                 group_sync(1 + g, 128);  // everyone has read its column before rows overwrite the buffer
-                store_normalized_row(xtile, row, xraw, mean, rstd, prm + 256, prm + 384);
+                store_normalized_row<C>(xtile, row, xraw, mean, rstd, prm + 256, prm + 384);
             }
             // --- z row: keep the raw values for the residual, normalise in place (A operand 1)
             if (!mbar_wait(z_full(g), use & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidOut, 7);
                 break;
             }
-            uint32_t zraw[64];
-            load_row(ztile, row, zraw);
-            row_stats(zraw, mean, rstd);
-            store_normalized_row(ztile, row, zraw, mean, rstd, prm, prm + 128);
+            uint32_t zraw[C / 2];
+            load_row<C>(ztile, row, zraw);
+            row_stats<C>(zraw, mean, rstd);
+            store_normalized_row<C>(ztile, row, zraw, mean, rstd, prm, prm + 128);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(a_ready(g));
@@ -703,12 +732,12 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                 break;
             }
             tc_fence_after_sync();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * 256;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * kTm;
 #pragma unroll
-            for (int cb = 0; cb < 8; ++cb) {  // 16 channels per step
+            for (int cb = 0; cb < C / 16; ++cb) {  // 16 channels per step
                 uint32_t gate[16], upd[16];
                 tmem_ld16(taddr + cb * 16, gate);
-                tmem_ld16(taddr + 128 + cb * 16, upd);
+                tmem_ld16(taddr + C + cb * 16, upd);
                 tmem_ld_wait();
 #pragma unroll
                 for (int ch = 0; ch < 2; ++ch) {
@@ -732,7 +761,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
             fence_proxy_async_smem();
             group_sync(1 + g, 128);
             if (gtid == 0) {
-                for (int kb = 0; kb < 2; ++kb)
+                for (int kb = 0; kb < C / 64; ++kb)
                     tma_store_3d(&tmOut, ztile + kb * kKBlockBytes, kb * 64, tc.t0, tc.b * R + tc.fixed);
                 tma_store_commit();
                 tma_store_wait_read<0>();
@@ -746,158 +775,182 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     __syncthreads();
     if (warp == 1) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, 512);
+        tmem_dealloc(tmem_base, 2 * kTm);
     }
 }
 
-int weight_tmap(CUtensorMap* m, const void* w, int rows) {
-    uint64_t dims[2] = {128, (uint64_t)rows};
-    uint64_t str[1] = {256};
-    uint32_t box[2] = {64, 128};
+int weight_tmap(CUtensorMap* m, const void* w, int C) {
+    uint64_t dims[2] = {(uint64_t)C, (uint64_t)C};
+    uint64_t str[1] = {(uint64_t)C * 2};
+    uint32_t box[2] = {64, (uint32_t)C};
     return make_tmap_bf16(m, w, 2, dims, str, box, true);
 }
 
-}  // namespace
-
-
-bool trimul_supported(int c_z, int c_h) { return c_z == 128 && c_h == 128; }
-
-static int set_attrs() {
-    if (!device_configured(5)) {
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_in_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, InSmem::kDyn));
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_in_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, InSmem::kDyn));
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_in_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, InSmem::kDyn));
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_in_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, InSmem::kDyn));
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OutSmem::kDyn));
-        device_mark_configured(5);
-    }
-    return OF3_OK;
-}
-
 // z as lines: {c, position, b*R + line}
-static int line_tmap(CUtensorMap* m, const void* z, int B, int R, int N) {
-    uint64_t dims[3] = {128, (uint64_t)N, (uint64_t)B * R};
-    uint64_t str[2] = {256, (uint64_t)N * 256};
+int line_tmap(CUtensorMap* m, const void* z, int B, int R, int N, int C) {
+    uint64_t dims[3] = {(uint64_t)C, (uint64_t)N, (uint64_t)B * R};
+    uint64_t str[2] = {(uint64_t)C * 2, (uint64_t)N * C * 2};
     uint32_t box[3] = {64, 128, 1};
     return make_tmap_bf16(m, z, 3, dims, str, box, 1);
 }
 
-// a_t[(b*128 + c)][line][k], b_t likewise, from R lines of N positions per sample: z is [B][R][N][128].
-// transposed_walk: z is [B][N][R][128] and a line runs along its FIRST index (line = second index),
+template <int C, bool kOutgoing>
+int launch_in(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensorMap* w, const __nv_bfloat16* mask,
+              const __nv_bfloat16* lw, const __nv_bfloat16* lb, __nv_bfloat16* a_t, __nv_bfloat16* b_t, int B, int R,
+              int N, int ld, int group_shift, long long group_stride, int wide) {
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_in_kernel<C, kOutgoing>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            InSmem<C>::kDyn));
+        configured.mark();
+    }
+    LaunchScope scope(kKidIn, st);
+    OF3_CUDA_CHECK(launch_chained(trimul_in_kernel<C, kOutgoing>, grid, kInThreads, InSmem<C>::kDyn, st, tmZ, w[0], w[1],
+                                  w[2], w[3], mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift, group_stride, wide,
+                                  device_status_ptr()));
+    return OF3_OK;
+}
+template <bool kOutgoing>
+int launch_in_rows(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensorMap* w, const __nv_bfloat16* mask,
+                   const __nv_bfloat16* lw, const __nv_bfloat16* lb, __nv_bfloat16* a_t, __nv_bfloat16* b_t, int B, int R,
+                   int N, int ld, int group_shift, long long group_stride) {
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_in_rows_kernel<kOutgoing>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            InSmem<128>::kDyn));
+        configured.mark();
+    }
+    LaunchScope scope(kKidIn, st);
+    OF3_CUDA_CHECK(launch_chained(trimul_in_rows_kernel<kOutgoing>, grid, kInRowsThreads, InSmem<128>::kDyn, st, tmZ, w[0],
+                                  w[1], w[2], w[3], mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift, group_stride,
+                                  device_status_ptr()));
+    return OF3_OK;
+}
+template <int C>
+int launch_out(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensorMap& tmX, const CUtensorMap& tmOut,
+               const CUtensorMap& tmWg, const CUtensorMap& tmWz, const of3_trimul_params* p, int B, int R, int N,
+               int add_residual) {
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_out_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            OutSmem<C>::kDyn));
+        configured.mark();
+    }
+    typedef const __nv_bfloat16* P;
+    LaunchScope scope(kKidOut, st);
+    OF3_CUDA_CHECK(launch_chained(trimul_out_kernel<C>, grid, 320, OutSmem<C>::kDyn, st, tmZ, tmX, tmOut, tmWg, tmWz,
+                                  (P)p->ln_in_w, (P)p->ln_in_b, (P)p->ln_out_w, (P)p->ln_out_b, B, R, N, add_residual,
+                                  device_status_ptr()));
+    return OF3_OK;
+}
+
+}  // namespace
+
+bool trimul_supported(int c_z, int c_h) { return c_z == c_h && (c_z == 128 || c_z == 64); }
+
+// a_t[(b*C + c)][line][k], b_t likewise, from R lines of N positions per sample: z is [B][R][N][C].
+// transposed_walk: z is [B][N][R][C] and a line runs along its FIRST index (line = second index),
 // which makes the incoming update the same K-major contraction as the outgoing one; with R != N this
 // is a row shard of N rows seen as R lines of N positions each.
-// groups > 1: the 128 channels are written as `groups` equal groups, group q of a_t at
+// groups > 1: the C channels are written as `groups` equal groups, group q of a_t at
 // a_t + q * group_stride (b_t likewise), so that each group can be sent to another rank as one block.
 int trimul_project(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* a_t, __nv_bfloat16* b_t,
                    int B, int R, int N, int ld, bool transposed_walk, const of3_trimul_params* p,
-                   cudaStream_t st, int groups, long long group_stride) {
+                   cudaStream_t st, int groups, long long group_stride, int C) {
     OF3_REQUIRE(((uintptr_t)z & 15) == 0, OF3_ERR_ALIGN, "trimul: z must be 16-byte aligned");
     OF3_REQUIRE(groups == 1 || groups == 2 || groups == 4 || groups == 8, OF3_ERR_ARG,
                 "trimul: channel groups must be 1, 2, 4 or 8 (got %d)", groups);
-    int group_shift = 7;
+    int group_shift = C == 128 ? 7 : 6;
     for (int g = groups; g > 1; g >>= 1) --group_shift;
-    if (groups == 1) group_stride = (long long)kC * R * ld;
+    if (groups == 1) group_stride = (long long)C * R * ld;
     int rc;
     CUtensorMap tmZ, tmW[4];
     if (!transposed_walk) {
-        if ((rc = line_tmap(&tmZ, z, B, R, N))) return rc;
+        if ((rc = line_tmap(&tmZ, z, B, R, N, C))) return rc;
     } else {  // {c, second (line), first (position), b}
-        uint64_t dims[4] = {128, (uint64_t)R, (uint64_t)N, (uint64_t)B};
-        uint64_t str[3] = {256, (uint64_t)R * 256, (uint64_t)N * R * 256};
+        uint64_t dims[4] = {(uint64_t)C, (uint64_t)R, (uint64_t)N, (uint64_t)B};
+        uint64_t str[3] = {(uint64_t)C * 2, (uint64_t)R * C * 2, (uint64_t)N * R * C * 2};
         uint32_t box[4] = {64, 1, 128, 1};
         if ((rc = make_tmap_bf16(&tmZ, z, 4, dims, str, box, 1))) return rc;
     }
     const void* w4[4] = {p->w_a_p, p->w_a_g, p->w_b_p, p->w_b_g};
     for (int i = 0; i < 4; ++i)
-        if ((rc = weight_tmap(&tmW[i], w4[i], 128))) return rc;
-    if ((rc = set_attrs())) return rc;
+        if ((rc = weight_tmap(&tmW[i], w4[i], C))) return rc;
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     // 32-byte stores need every channel row of a_t / b_t to start on a 32-byte boundary
     const int wide = (ld % 16 == 0 && (group_stride % 16) == 0 && ((uintptr_t)a_t & 31) == 0 && ((uintptr_t)b_t & 31) == 0) ? 1 : 0;
     // a channel plane of R lines: beyond about one 2 MB page the kernel whose stores stay inside one plane wins
-    const bool planes_far_apart = (long long)R * ld * (long long)sizeof(__nv_bfloat16) > (2LL << 20);
-    LaunchScope scope(kKidIn, st);
+    const bool planes_far_apart = C == 128 && (long long)R * ld * (long long)sizeof(__nv_bfloat16) > (2LL << 20);
     const __nv_bfloat16* lw = (const __nv_bfloat16*)p->ln_in_w;
     const __nv_bfloat16* lb = (const __nv_bfloat16*)p->ln_in_b;
-    if (planes_far_apart) {
-        if (!transposed_walk)
-            trimul_in_rows_kernel<true><<<grid, kInRowsThreads, InSmem::kDyn, st>>>(
-                tmZ, tmW[0], tmW[1], tmW[2], tmW[3], mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift, group_stride,
-                device_status_ptr());
-        else
-            trimul_in_rows_kernel<false><<<grid, kInRowsThreads, InSmem::kDyn, st>>>(
-                tmZ, tmW[0], tmW[1], tmW[2], tmW[3], mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift, group_stride,
-                device_status_ptr());
-    } else if (!transposed_walk) {
-        trimul_in_kernel<true><<<grid, kInThreads, InSmem::kDyn, st>>>(
-            tmZ, tmW[0], tmW[1], tmW[2], tmW[3], mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift, group_stride, wide,
-            device_status_ptr());
-    } else {
-        trimul_in_kernel<false><<<grid, kInThreads, InSmem::kDyn, st>>>(
-            tmZ, tmW[0], tmW[1], tmW[2], tmW[3], mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift, group_stride, wide,
-            device_status_ptr());
-    }
-    OF3_CUDA_CHECK(cudaGetLastError());
-    return OF3_OK;
+    if (planes_far_apart)
+        return transposed_walk ? launch_in_rows<false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
+                                                       group_stride)
+                               : launch_in_rows<true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
+                                                      group_stride);
+    if (C == 128)
+        return transposed_walk ? launch_in<128, false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
+                                                       group_stride, wide)
+                               : launch_in<128, true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
+                                                      group_stride, wide);
+    return transposed_walk ? launch_in<64, false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
+                                                  group_stride, wide)
+                           : launch_in<64, true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
+                                                 group_stride, wide);
 }
 
 // x = a_t . b_t^T per channel (a_t: R lines, b_t: all N lines), then LN_out / linear_z / gate / residual
 // on the R lines of z -> out (may alias z).
 int trimul_finish(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* a_t,
                   const __nv_bfloat16* b_t, __nv_bfloat16* x_t, int B, int R, int N, int ld, int add_residual,
-                  const of3_trimul_params* p, cudaStream_t st) {
+                  const of3_trimul_params* p, cudaStream_t st, int C) {
     OF3_REQUIRE(((uintptr_t)z & 15) == 0 && ((uintptr_t)out & 15) == 0, OF3_ERR_ALIGN,
                 "trimul: z/out must be 16-byte aligned");
-    int rc = contract_nt_bf16(a_t, b_t, x_t, B * kC, R, N, N, ld, ld, ld, (long long)R * ld, (long long)N * ld,
+    int rc = contract_nt_bf16(a_t, b_t, x_t, B * C, R, N, N, ld, ld, ld, (long long)R * ld, (long long)N * ld,
                               (long long)R * ld, st);
     if (rc) return rc;
-    return trimul_output(z, out, x_t, B, R, N, ld, add_residual, p, st);
+    return trimul_output(z, out, x_t, B, R, N, ld, add_residual, p, st, C);
 }
 
 // LN_out(x) -> linear_z, gate from LN_in(z), residual: the part of the update after the contraction,
-// on R lines of z with x_t[b*128 + c][line][j] (pitch ld)
+// on R lines of z with x_t[b*C + c][line][j] (pitch ld)
 int trimul_output(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* x_t, int B, int R, int N, int ld,
-                  int add_residual, const of3_trimul_params* p, cudaStream_t st) {
+                  int add_residual, const of3_trimul_params* p, cudaStream_t st, int C) {
     OF3_REQUIRE(((uintptr_t)z & 15) == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)x_t & 15) == 0, OF3_ERR_ALIGN,
                 "trimul: z/out/x must be 16-byte aligned");
     int rc;
     CUtensorMap tmZ, tmOut, tmX, tmWg, tmWz;
-    if ((rc = line_tmap(&tmZ, z, B, R, N))) return rc;
-    if ((rc = line_tmap(&tmOut, out, B, R, N))) return rc;
-    {   // x_t[b*128 + c][line][j], pitch ld: box = 128 positions j x 1 x 128 channels, no swizzle
-        uint64_t dims[3] = {(uint64_t)N, (uint64_t)R, (uint64_t)B * kC};
+    if ((rc = line_tmap(&tmZ, z, B, R, N, C))) return rc;
+    if ((rc = line_tmap(&tmOut, out, B, R, N, C))) return rc;
+    {   // x_t[b*C + c][line][j], pitch ld: box = 128 positions j x 1 x C channels, no swizzle
+        uint64_t dims[3] = {(uint64_t)N, (uint64_t)R, (uint64_t)B * C};
         uint64_t str[2] = {(uint64_t)ld * 2, (uint64_t)R * ld * 2};
-        uint32_t box[3] = {128, 1, 128};
+        uint32_t box[3] = {128, 1, (uint32_t)C};
         if ((rc = make_tmap_bf16(&tmX, x_t, 3, dims, str, box, 0))) return rc;
     }
-    if ((rc = weight_tmap(&tmWg, p->w_g, 128))) return rc;
-    if ((rc = weight_tmap(&tmWz, p->w_z, 128))) return rc;
-    if ((rc = set_attrs())) return rc;
+    if ((rc = weight_tmap(&tmWg, p->w_g, C))) return rc;
+    if ((rc = weight_tmap(&tmWz, p->w_z, C))) return rc;
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
-    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    LaunchScope scope(kKidOut, st);
-    trimul_out_kernel<<<grid, 320, OutSmem::kDyn, st>>>(
-        tmZ, tmX, tmOut, tmWg, tmWz, (const __nv_bfloat16*)p->ln_in_w, (const __nv_bfloat16*)p->ln_in_b,
-        (const __nv_bfloat16*)p->ln_out_w, (const __nv_bfloat16*)p->ln_out_b, B, R, N, add_residual,
-        device_status_ptr());
-    OF3_CUDA_CHECK(cudaGetLastError());
-    return OF3_OK;
+    const int ctas = sm_count() * (C == 128 ? 1 : 2);
+    const int grid = (int)(tiles < ctas ? tiles : ctas);
+    return C == 128 ? launch_out<128>(grid, st, tmZ, tmX, tmOut, tmWg, tmWz, p, B, R, N, add_residual)
+                    : launch_out<64>(grid, st, tmZ, tmX, tmOut, tmWg, tmWz, p, B, R, N, add_residual);
 }
 
-int trimul(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N,
+int trimul(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N, int C,
            int flags, const of3_trimul_params* p, Arena& ws, cudaStream_t st) {
     const int ld = (int)align_up(N, 8);
-    const size_t plane = (size_t)B * kC * N * ld * sizeof(__nv_bfloat16);
+    const size_t plane = (size_t)B * C * N * ld * sizeof(__nv_bfloat16);
     __nv_bfloat16* a_t = (__nv_bfloat16*)ws.take(plane);
     __nv_bfloat16* b_t = (__nv_bfloat16*)ws.take(plane);
     __nv_bfloat16* x_t = (__nv_bfloat16*)ws.take(plane);
     if (!ws.base) return OF3_OK;
     OF3_REQUIRE(ws.ok(), OF3_ERR_WORKSPACE, "trimul: workspace too small (%zu needed)", ws.off);
     const bool outgoing = (flags & OF3_FLAG_OUTGOING) != 0;
-    int rc = trimul_project(z, mask, a_t, b_t, B, N, N, ld, !outgoing, p, st);
+    int rc = trimul_project(z, mask, a_t, b_t, B, N, N, ld, !outgoing, p, st, 1, 0, C);
     if (rc) return rc;
-    return trimul_finish(z, out, a_t, b_t, x_t, B, N, N, ld, (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, st);
+    return trimul_finish(z, out, a_t, b_t, x_t, B, N, N, ld, (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, st, C);
 }
 
 }  // namespace fast

@@ -28,35 +28,35 @@ int cond_transition(const T* a, const T* s, const T* mask, T* out, long long row
 }  // namespace generic
 
 namespace fast {
-// bf16, c_z = c_hidden = 128
+// bf16, c_z = c_hidden = C = 128, or 64 (the template stack)
 bool trimul_supported(int c_z, int c_h);
-int trimul(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N,
+int trimul(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N, int C,
            int flags, const of3_trimul_params* p, Arena& ws, cudaStream_t st);
-// bf16, c_z = 128, 4 heads x 32
+// bf16, 4 heads, c_z = C = 128 (heads of 32) or 64 (heads of 16)
 bool triattn_supported(int c_z, int H, int d, int N);
-int triattn(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N,
+int triattn(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N, int C,
             float inf, int flags, const of3_triattn_params* p, Arena& ws, cudaStream_t st);
 // bf16, c = 128, n = 4
 // phases of the two layers above on R lines of N positions (R == N: whole tensor; R = N / P: a row shard)
 int trimul_project(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* a_t, __nv_bfloat16* b_t,
                    int B, int R, int N, int ld, bool transposed_walk, const of3_trimul_params* p,
-                   cudaStream_t st, int groups = 1, long long group_stride = 0);
+                   cudaStream_t st, int groups = 1, long long group_stride = 0, int C = 128);
 int trimul_output(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* x_t, int B, int R, int N, int ld,
-                  int add_residual, const of3_trimul_params* p, cudaStream_t st);
+                  int add_residual, const of3_trimul_params* p, cudaStream_t st, int C = 128);
 int trimul_finish(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* a_t,
                   const __nv_bfloat16* b_t, __nv_bfloat16* x_t, int B, int R, int N, int ld, int add_residual,
-                  const of3_trimul_params* p, cudaStream_t st);
-size_t triattn_image_elems(int B, int R, int N);
+                  const of3_trimul_params* p, cudaStream_t st, int C = 128);
+size_t triattn_image_elems(int B, int R, int N, int C = 128);
 size_t triattn_bias_elems(int B, int R, int N);  // bf16 elements of the pair-bias image [B*4][key blocks][R][32]
 int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* vt,
                     __nv_bfloat16* tb, int B, int R, int N, int row0, bool transposed,
-                    const of3_triattn_params* p, cudaStream_t st);
+                    const of3_triattn_params* p, cudaStream_t st, int C = 128);
 int triattn_finish(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out,
                    const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* vt,
                    const __nv_bfloat16* tb, __nv_bfloat16* o, int B, int R, int N, float inf,
-                   bool transposed, int add_residual, const of3_triattn_params* p, cudaStream_t st);
+                   bool transposed, int add_residual, const of3_triattn_params* p, cudaStream_t st, int C = 128);
 bool transition_supported(int c, int n);
-int transition(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bfloat16* out, long long rows,
+int transition(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bfloat16* out, long long rows, int c,
                int flags, const of3_transition_params* p, Arena& ws, cudaStream_t st);
 // gated attention with pair bias on the tensor pipe (fast_single.cuh)
 bool single_attn_tc_supported(int N, int H, int d);

@@ -1,7 +1,7 @@
-// Device helpers shared by the "row tile" kernels: a tile is 128 rows (pair positions) of 128
-// bf16 channels held in shared memory as a K-major, 128-byte-swizzled tcgen05 A operand made of
-// two k-blocks [128 rows x 64 channels] (16 KB each) -- exactly what two TMA boxes {64, 128}
-// with CU_TENSOR_MAP_SWIZZLE_128B deposit. One thread owns one row.
+// Device helpers shared by the "row tile" kernels: a tile is 128 rows (pair positions) of C = 128
+// bf16 channels (64 in the template stack) held in shared memory as a K-major, 128-byte-swizzled
+// tcgen05 operand made of C / 64 k-blocks [128 rows x 64 channels] (16 KB each) -- exactly what
+// TMA boxes {64, 128} with CU_TENSOR_MAP_SWIZZLE_128B deposit. One thread owns one row.
 #pragma once
 #include "umma.cuh"
 
@@ -12,6 +12,8 @@ constexpr int kRows = 128;
 constexpr int kC = 128;
 constexpr int kKBlockBytes = kRows * 64 * 2;  // 16384
 constexpr int kTileBytes = 2 * kKBlockBytes;  // 32768
+template <int C>
+__host__ __device__ constexpr int tile_bytes() { return C / 64 * kKBlockBytes; }
 constexpr float kLnEps = 1e-5f;
 
 __device__ __forceinline__ float tanh_approx(float x) {
@@ -70,10 +72,11 @@ __device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
                  : "memory");
 }
 
-// Reads this thread's row (128 bf16) of a swizzled tile into 64 packed registers.
-__device__ __forceinline__ void load_row(uint32_t tile, int row, uint32_t (&raw)[64]) {
+// Reads this thread's row (C bf16) of a swizzled tile into C / 2 packed registers.
+template <int C = kC>
+__device__ __forceinline__ void load_row(uint32_t tile, int row, uint32_t (&raw)[C / 2]) {
 #pragma unroll
-    for (int ch = 0; ch < 16; ++ch) {
+    for (int ch = 0; ch < C / 8; ++ch) {
         const uint4 v = lds128(chunk_addr(tile, row, ch));
         raw[ch * 4 + 0] = v.x;
         raw[ch * 4 + 1] = v.y;
@@ -82,54 +85,57 @@ __device__ __forceinline__ void load_row(uint32_t tile, int row, uint32_t (&raw)
     }
 }
 
-// LayerNorm statistics of 128 packed bf16 values (fp32, two-pass on registers). Eight independent partial sums (a
-// single accumulator is a 128-deep dependent chain, which with two warps per scheduler is pure latency), associated
+// LayerNorm statistics of C packed bf16 values (fp32, two-pass on registers). Eight independent partial sums (a
+// single accumulator is a C-deep dependent chain, which with two warps per scheduler is pure latency), associated
 // exactly like the two-threads-per-row variant below -- four partial sums per half row, the halves added last -- so
 // that kernels that split a row over two threads and kernels that do not produce the same bits.
-__device__ __forceinline__ void row_stats(const uint32_t (&raw)[64], float& mean, float& rstd) {
+template <int C = kC>
+__device__ __forceinline__ void row_stats(const uint32_t (&raw)[C / 2], float& mean, float& rstd) {
     float s[8];
 #pragma unroll
     for (int a = 0; a < 8; ++a) s[a] = 0.f;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
+        for (int i = 0; i < C / 4; i += 4) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a) s[h * 4 + a] += bf16lo(raw[h * 32 + i + a]) + bf16hi(raw[h * 32 + i + a]);
+            for (int a = 0; a < 4; ++a)
+                s[h * 4 + a] += bf16lo(raw[h * (C / 4) + i + a]) + bf16hi(raw[h * (C / 4) + i + a]);
         }
     }
-    mean = (((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]))) * (1.0f / kC);
+    mean = (((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]))) * (1.0f / C);
     float v[8];
 #pragma unroll
     for (int a = 0; a < 8; ++a) v[a] = 0.f;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
+        for (int i = 0; i < C / 4; i += 4) {
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const float x0 = bf16lo(raw[h * 32 + i + a]) - mean, x1 = bf16hi(raw[h * 32 + i + a]) - mean;
+                const float x0 = bf16lo(raw[h * (C / 4) + i + a]) - mean, x1 = bf16hi(raw[h * (C / 4) + i + a]) - mean;
                 v[h * 4 + a] = fmaf(x0, x0, v[h * 4 + a]);
                 v[h * 4 + a] = fmaf(x1, x1, v[h * 4 + a]);
             }
         }
     }
-    const float var = (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]))) * (1.0f / kC);
+    const float var = (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]))) * (1.0f / C);
     rstd = rsqrtf(var + kLnEps);
 }
 
-// Writes LN(raw) * gamma + beta (bf16) as this thread's row of a swizzled tile.
-// gamma/beta: fp32 arrays of 128 in shared memory, 16-byte aligned (broadcast vector reads).
-__device__ __forceinline__ void store_normalized_row(uint32_t tile, int row, const uint32_t (&raw)[64],
-                                                     float mean, float rstd, const float* gamma,
-                                                     const float* beta) {
+// Writes LN(raw) * gamma + beta (bf16) of NCH 16-byte chunks, from chunk `first` of the row on, into a swizzled tile.
+// gamma/beta: fp32 arrays of C in shared memory, 16-byte aligned (broadcast vector reads).
+template <int NCH>
+__device__ __forceinline__ void store_normalized_chunks(uint32_t tile, int row, int first, const uint32_t (&raw)[NCH * 4],
+                                                        float mean, float rstd, const float* gamma, const float* beta) {
     const float nm = -mean * rstd;
 #pragma unroll
-    for (int ch = 0; ch < 16; ++ch) {
-        const float4 g0 = *reinterpret_cast<const float4*>(gamma + ch * 8);
-        const float4 g1 = *reinterpret_cast<const float4*>(gamma + ch * 8 + 4);
-        const float4 b0 = *reinterpret_cast<const float4*>(beta + ch * 8);
-        const float4 b1 = *reinterpret_cast<const float4*>(beta + ch * 8 + 4);
+    for (int ch = 0; ch < NCH; ++ch) {
+        const int c0 = (first + ch) * 8;
+        const float4 g0 = *reinterpret_cast<const float4*>(gamma + c0);
+        const float4 g1 = *reinterpret_cast<const float4*>(gamma + c0 + 4);
+        const float4 b0 = *reinterpret_cast<const float4*>(beta + c0);
+        const float4 b1 = *reinterpret_cast<const float4*>(beta + c0 + 4);
         const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
         const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
         uint32_t o[4];
@@ -140,36 +146,45 @@ __device__ __forceinline__ void store_normalized_row(uint32_t tile, int row, con
             const float b = fmaf(fmaf(bf16hi(raw[ch * 4 + j]), rstd, nm), gg[j * 2 + 1], bb[j * 2 + 1]);
             o[j] = pack_bf16x2(a, b);
         }
-        sts128(chunk_addr(tile, row, ch), make_uint4(o[0], o[1], o[2], o[3]));
+        sts128(chunk_addr(tile, row, first + ch), make_uint4(o[0], o[1], o[2], o[3]));
     }
 }
+template <int C = kC>
+__device__ __forceinline__ void store_normalized_row(uint32_t tile, int row, const uint32_t (&raw)[C / 2],
+                                                     float mean, float rstd, const float* gamma,
+                                                     const float* beta) {
+    store_normalized_chunks<C / 8>(tile, row, 0, raw, mean, rstd, gamma, beta);
+}
 
-// The same three steps with TWO threads per row: lanes 0..15 of a warp hold channels 0..63 of 16 rows, lanes
-// 16..31 channels 64..127 of the same rows (half = lane >> 4); the statistics are joined by one shuffle.
-__device__ __forceinline__ void load_half_row(uint32_t tile, int row, int half, uint32_t (&raw)[32]) {
+// The same three steps with TWO threads per row: lanes 0..15 of a warp hold the first C / 2 channels of 16 rows, lanes
+// 16..31 the others of the same rows (half = lane >> 4); the statistics are joined by one shuffle.
+template <int C = kC>
+__device__ __forceinline__ void load_half_row(uint32_t tile, int row, int half, uint32_t (&raw)[C / 4]) {
 #pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-        const uint4 v = lds128(chunk_addr(tile, row, half * 8 + ch));
+    for (int ch = 0; ch < C / 16; ++ch) {
+        const uint4 v = lds128(chunk_addr(tile, row, half * (C / 16) + ch));
         raw[ch * 4 + 0] = v.x;
         raw[ch * 4 + 1] = v.y;
         raw[ch * 4 + 2] = v.z;
         raw[ch * 4 + 3] = v.w;
     }
 }
-// Sum, and sum of squared deviations, of this thread's 64 of a row's 128 values.
-__device__ __forceinline__ float half_row_sum(const uint32_t (&raw)[32]) {
+// Sum, and sum of squared deviations, of this thread's half of a row's values.
+template <int C = kC>
+__device__ __forceinline__ float half_row_sum(const uint32_t (&raw)[C / 4]) {
     float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < 32; i += 4) {
+    for (int i = 0; i < C / 4; i += 4) {
 #pragma unroll
         for (int a = 0; a < 4; ++a) s[a] += bf16lo(raw[i + a]) + bf16hi(raw[i + a]);
     }
     return (s[0] + s[1]) + (s[2] + s[3]);
 }
-__device__ __forceinline__ float half_row_sqdev(const uint32_t (&raw)[32], float mean) {
+template <int C = kC>
+__device__ __forceinline__ float half_row_sqdev(const uint32_t (&raw)[C / 4], float mean) {
     float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < 32; i += 4) {
+    for (int i = 0; i < C / 4; i += 4) {
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const float x0 = bf16lo(raw[i + a]) - mean, x1 = bf16hi(raw[i + a]) - mean;
@@ -180,57 +195,43 @@ __device__ __forceinline__ float half_row_sqdev(const uint32_t (&raw)[32], float
     return (v[0] + v[1]) + (v[2] + v[3]);
 }
 // the two halves of a row sit 16 lanes apart in one warp
-__device__ __forceinline__ void half_row_stats(const uint32_t (&raw)[32], float& mean, float& rstd) {
-    float sum = half_row_sum(raw);
+template <int C = kC>
+__device__ __forceinline__ void half_row_stats(const uint32_t (&raw)[C / 4], float& mean, float& rstd) {
+    float sum = half_row_sum<C>(raw);
     sum += __shfl_xor_sync(0xffffffffu, sum, 16);
-    mean = sum * (1.0f / kC);
-    float var = half_row_sqdev(raw, mean);
+    mean = sum * (1.0f / C);
+    float var = half_row_sqdev<C>(raw, mean);
     var += __shfl_xor_sync(0xffffffffu, var, 16);
-    rstd = rsqrtf(var * (1.0f / kC) + kLnEps);
+    rstd = rsqrtf(var * (1.0f / C) + kLnEps);
 }
 // the two halves of a row belong to the same lane of two warps of a group of `nthreads` threads: the partial
 // results cross through xch (2 x 256 floats of shared memory) and two named barriers (id)
-__device__ __forceinline__ void half_row_stats_xwarp(const uint32_t (&raw)[32], int row, int half, float* xch, int bar_id,
-                                                     int nthreads, float& mean, float& rstd) {
-    const float sum = half_row_sum(raw);
+template <int C = kC>
+__device__ __forceinline__ void half_row_stats_xwarp(const uint32_t (&raw)[C / 4], int row, int half, float* xch,
+                                                     int bar_id, int nthreads, float& mean, float& rstd) {
+    const float sum = half_row_sum<C>(raw);
     xch[half * 128 + row] = sum;
     group_sync(bar_id, nthreads);
-    mean = (sum + xch[(half ^ 1) * 128 + row]) * (1.0f / kC);
-    const float var = half_row_sqdev(raw, mean);
+    mean = (sum + xch[(half ^ 1) * 128 + row]) * (1.0f / C);
+    const float var = half_row_sqdev<C>(raw, mean);
     xch[256 + half * 128 + row] = var;
     group_sync(bar_id, nthreads);
-    rstd = rsqrtf((var + xch[256 + (half ^ 1) * 128 + row]) * (1.0f / kC) + kLnEps);
+    rstd = rsqrtf((var + xch[256 + (half ^ 1) * 128 + row]) * (1.0f / C) + kLnEps);
 }
-__device__ __forceinline__ void store_normalized_half_row(uint32_t tile, int row, int half, const uint32_t (&raw)[32],
+template <int C = kC>
+__device__ __forceinline__ void store_normalized_half_row(uint32_t tile, int row, int half, const uint32_t (&raw)[C / 4],
                                                           float mean, float rstd, const float* gamma,
                                                           const float* beta) {
-    const float nm = -mean * rstd;
-#pragma unroll
-    for (int ch = 0; ch < 8; ++ch) {
-        const int c0 = (half * 8 + ch) * 8;
-        const float4 g0 = *reinterpret_cast<const float4*>(gamma + c0);
-        const float4 g1 = *reinterpret_cast<const float4*>(gamma + c0 + 4);
-        const float4 b0 = *reinterpret_cast<const float4*>(beta + c0);
-        const float4 b1 = *reinterpret_cast<const float4*>(beta + c0 + 4);
-        const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float a = fmaf(fmaf(bf16lo(raw[ch * 4 + j]), rstd, nm), gg[j * 2], bb[j * 2]);
-            const float b = fmaf(fmaf(bf16hi(raw[ch * 4 + j]), rstd, nm), gg[j * 2 + 1], bb[j * 2 + 1]);
-            o[j] = pack_bf16x2(a, b);
-        }
-        sts128(chunk_addr(tile, row, half * 8 + ch), make_uint4(o[0], o[1], o[2], o[3]));
-    }
+    store_normalized_chunks<C / 16>(tile, row, half * (C / 16), raw, mean, rstd, gamma, beta);
 }
 
-// 8 tcgen05.mma (K = 128 in steps of 16) of one row tile against a weight slab:
-// D[128 x N] (+)= A[128 x 128] * W[N x 128]^T. `w_kb_stride` = bytes between the slab's k-blocks.
-__device__ __forceinline__ void mma_k128(uint32_t d_tmem, uint32_t a_tile, uint32_t w_slab,
+// K / 16 tcgen05.mma of one row tile against a weight slab:
+// D[128 x N] (+)= A[128 x K] * W[N x K]^T. `w_kb_stride` = bytes between the slab's k-blocks.
+template <int K = kC>
+__device__ __forceinline__ void mma_rows(uint32_t d_tmem, uint32_t a_tile, uint32_t w_slab,
                                          uint32_t w_kb_stride, uint32_t idesc, bool accumulate) {
 #pragma unroll
-    for (int kb = 0; kb < 2; ++kb) {
+    for (int kb = 0; kb < K / 64; ++kb) {
         const uint64_t ad = umma::smem_desc_k_sw128(a_tile + kb * kKBlockBytes);
         const uint64_t bd = umma::smem_desc_k_sw128(w_slab + kb * w_kb_stride);
 #pragma unroll
@@ -238,6 +239,10 @@ __device__ __forceinline__ void mma_k128(uint32_t d_tmem, uint32_t a_tile, uint3
             umma::mma_bf16(d_tmem, ad + 2u * k4, bd + 2u * k4, idesc,
                            (accumulate || kb != 0 || k4 != 0) ? 1u : 0u);
     }
+}
+__device__ __forceinline__ void mma_k128(uint32_t d_tmem, uint32_t a_tile, uint32_t w_slab,
+                                         uint32_t w_kb_stride, uint32_t idesc, bool accumulate) {
+    mma_rows<128>(d_tmem, a_tile, w_slab, w_kb_stride, idesc, accumulate);
 }
 
 }  // namespace rowtile
