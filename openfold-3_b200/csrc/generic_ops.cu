@@ -1,6 +1,7 @@
 // Shape-generic SIMT kernels: see generic_ops.cuh. True fp32 arithmetic throughout.
 #include "generic_ops.cuh"
 #include "runtime.cuh"
+#include "umma.cuh"
 
 namespace of3 {
 namespace generic {
@@ -13,11 +14,6 @@ __device__ __forceinline__ float warp_sum(float v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 __device__ __forceinline__ float sigmoid_acc(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 inline unsigned grid_for(long long n, int per_block) {
@@ -26,172 +22,260 @@ inline unsigned grid_for(long long n, int per_block) {
 }
 
 // ------------------------------------------------------------------ LayerNorm
+// One warp per row; the row stays in registers up to 512 channels.
+constexpr int kLnRegs = 16;
 template <typename TX, typename TP>
-__global__ void layernorm_kernel(const TX* __restrict__ x, const TP* __restrict__ gamma,
-                                 const TP* __restrict__ beta, float* __restrict__ y, long long rows,
-                                 int C, float eps, long long inner, long long outer_stride,
-                                 long long inner_stride) {
+__global__ void __launch_bounds__(kThreads) layernorm_kernel(const TX* __restrict__ x, const TP* __restrict__ gamma,
+                                                             const TP* __restrict__ beta, float* __restrict__ y,
+                                                             long long rows, int C, float eps, RowMap map,
+                                                             const TP* __restrict__ proj_w, int H,
+                                                             float* __restrict__ proj) {
+    umma::grid_trigger();
+    umma::grid_wait();
     const int lane = threadIdx.x & 31;
     const long long r = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     if (r >= rows) return;
-    const TX* xr = x + (r / inner) * outer_stride + (r % inner) * inner_stride;
-    float s = 0.f;
-    for (int c = lane; c < C; c += 32) s += ld_as_float(xr + c);
-    const float mean = warp_sum(s) / (float)C;
-    float v = 0.f;
-    for (int c = lane; c < C; c += 32) {
-        const float d = ld_as_float(xr + c) - mean;
-        v += d * d;
-    }
-    const float rstd = 1.0f / sqrtf(warp_sum(v) / (float)C + eps);
+    const TX* xr = x + (r / map.inner) * map.outer_stride + (r % map.inner) * map.inner_stride;
     float* yr = y + r * C;
-    for (int c = lane; c < C; c += 32) {
-        float o = (ld_as_float(xr + c) - mean) * rstd;
+    const bool in_regs = C <= 32 * kLnRegs;
+    float v[kLnRegs];
+    float s = 0.f;
+    if (in_regs) {
+#pragma unroll
+        for (int i = 0; i < kLnRegs; ++i) {
+            v[i] = lane + 32 * i < C ? ld_as_float(xr + lane + 32 * i) : 0.f;
+            s += v[i];
+        }
+    } else {
+        for (int c = lane; c < C; c += 32) s += ld_as_float(xr + c);
+    }
+    const float mean = warp_sum(s) / (float)C;
+    float q = 0.f;
+    if (in_regs) {
+#pragma unroll
+        for (int i = 0; i < kLnRegs; ++i) {
+            const float d = lane + 32 * i < C ? v[i] - mean : 0.f;
+            q += d * d;
+        }
+    } else {
+        for (int c = lane; c < C; c += 32) {
+            const float d = ld_as_float(xr + c) - mean;
+            q += d * d;
+        }
+    }
+    const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)C + eps);
+    auto norm = [&](float xv, int c) {
+        float o = (xv - mean) * rstd;
         if (gamma) o *= ld_as_float(gamma + c);
         if (beta) o += ld_as_float(beta + c);
-        yr[c] = o;
+        return o;
+    };
+    if (in_regs) {
+#pragma unroll
+        for (int i = 0; i < kLnRegs; ++i) {
+            const int c = lane + 32 * i;
+            if (c < C) {
+                v[i] = norm(v[i], c);
+                if (y) yr[c] = v[i];
+            }
+        }
+    } else if (y) {
+        for (int c = lane; c < C; c += 32) yr[c] = norm(ld_as_float(xr + c), c);
+    }
+    for (int h = 0; h < H; ++h) {
+        float d = 0.f;
+        if (in_regs) {
+#pragma unroll
+            for (int i = 0; i < kLnRegs; ++i)
+                if (lane + 32 * i < C) d = fmaf(v[i], ld_as_float(proj_w + (long long)h * C + lane + 32 * i), d);
+        } else {
+            for (int c = lane; c < C; c += 32)
+                d = fmaf(norm(ld_as_float(xr + c), c), ld_as_float(proj_w + (long long)h * C + c), d);
+        }
+        d = warp_sum(d);
+        if (lane == 0) proj[(long long)h * rows + r] = d;
     }
 }
 
-// ------------------------------------------------------------------ strided batched NT GEMM
-constexpr int kTM = 64, kTN = 64, kTK = 16;
-
-template <typename TW>
-__global__ void __launch_bounds__(256) gemm_nt_kernel(const float* __restrict__ A,
-                                                      const TW* __restrict__ W,
-                                                      const TW* __restrict__ bias,
-                                                      float* __restrict__ out, GemmDesc d) {
-    __shared__ float As[kTK][kTM + 1];
-    __shared__ float Ws[kTK][kTN + 1];
-    const int b = blockIdx.z;
-    const int m0 = blockIdx.y * kTM;
-    const int n0 = blockIdx.x * kTN;
-    const float* Ab = A + (long long)b * d.a_b;
-    const TW* Wb = W + (long long)b * d.w_b;
-    const int tx = threadIdx.x & 15;  // n micro index
-    const int ty = threadIdx.x >> 4;  // m micro index
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-    for (int k0 = 0; k0 < d.K; k0 += kTK) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int idx = threadIdx.x + e * 256;
-            const int kk = idx & 15;
-            const int mm = idx >> 4;
-            const int gm = m0 + mm, gk = k0 + kk;
-            As[kk][mm] = (gm < d.M && gk < d.K) ? Ab[(long long)gm * d.a_m + (long long)gk * d.a_k] : 0.f;
-            const int gn = n0 + mm;
-            Ws[kk][mm] = (gn < d.N && gk < d.K)
-                             ? ld_as_float(Wb + (long long)gn * d.w_n + (long long)gk * d.w_k)
-                             : 0.f;
-        }
+// Rows of channel planes: a block takes 32 rows, passes of 32 x 32 values through shared memory.
+template <typename TP>
+__global__ void __launch_bounds__(kThreads) layernorm_planes_kernel(const float* __restrict__ x,
+                                                                    const TP* __restrict__ gamma,
+                                                                    const TP* __restrict__ beta, float* __restrict__ y,
+                                                                    long long rows, int C, float eps) {
+    __shared__ float part[8][33], mean_s[32], rstd_s[32], tile[32][33];
+    umma::grid_trigger();
+    umma::grid_wait();
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const long long r0 = (long long)blockIdx.x * 32, r = r0 + lane;
+    auto reduce = [&](float v) {   // sum over the 8 warps, per lane
+        part[wp][lane] = v;
         __syncthreads();
+        float s = 0.f;
 #pragma unroll
-        for (int kk = 0; kk < kTK; ++kk) {
-            float a[4], w[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = Ws[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-        }
+        for (int i = 0; i < 8; ++i) s += part[i][lane];
         __syncthreads();
+        return s;
+    };
+    float s = 0.f;
+    for (int c = wp; c < C; c += 8) s += r < rows ? x[(long long)c * rows + r] : 0.f;
+    const float mean = reduce(s) / (float)C;
+    float q = 0.f;
+    for (int c = wp; c < C; c += 8) {
+        const float d = (r < rows ? x[(long long)c * rows + r] : 0.f) - mean;
+        q += d * d;
     }
-    float* ob = out + (long long)b * d.o_b;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gm = m0 + ty * 4 + i;
-        if (gm >= d.M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= d.N) continue;
-            float v = acc[i][j];
-            if (bias) v += ld_as_float(bias + gn);
-            ob[(long long)gm * d.o_m + (long long)gn * d.o_n] = v;
+    const float rstd = 1.0f / sqrtf(reduce(q) / (float)C + eps);
+    if (wp == 0) {
+        mean_s[lane] = mean;
+        rstd_s[lane] = rstd;
+    }
+    for (int c0 = 0; c0 < C; c0 += 32) {
+        __syncthreads();
+        for (int c = wp; c < 32; c += 8)
+            tile[c][lane] = (c0 + c < C && r < rows) ? x[(long long)(c0 + c) * rows + r] : 0.f;
+        __syncthreads();
+        const int c = c0 + lane;
+        if (c < C) {
+            const float gm = gamma ? ld_as_float(gamma + c) : 1.f, bt = beta ? ld_as_float(beta + c) : 0.f;
+            for (int i = wp; i < 32; i += 8)
+                if (r0 + i < rows) y[(r0 + i) * C + c] = (tile[lane][i] - mean_s[i]) * rstd_s[i] * gm + bt;
         }
     }
 }
 
 // ------------------------------------------------------------------ streaming attention
-constexpr int kAttWarps = 8;
+// Block = 64 queries of one (bb, head), 256 threads as 16 x 16: thread (ty, tx) holds the 4 x 4 logits of queries 4 ty..
+// and keys 4 tx.., and DC = DP / 16 output channels of its four queries. Q and K lie transposed in shared memory, P goes
+// through it; a row's maximum and sum are joined over the 16 threads of a half warp. FMA-pipe bound: 16 FMA per two
+// 16-byte shared-memory reads. (One warp per query, two shared-memory reads per FMA: 121 us per layer at N = 128, 4 x 32.)
 constexpr int kAttMaxD = 64;
+constexpr int kAttQ = 64, kAttK = 64, kAttP = 68;   // pitch: 16-byte aligned rows
+template <int DP>
+constexpr int att_smem_floats() { return 2 * DP * kAttP + kAttK * DP + kAttK * kAttP + kAttK; }
 
-__global__ void __launch_bounds__(kAttWarps * 32)
-attention_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                 const float* __restrict__ v, const float* __restrict__ mask_bias,
-                 const float* __restrict__ pair_bias, float* __restrict__ out, int N, int H, int d,
-                 float scale, long long rows_per_bias) {
-    __shared__ float Ks[32][kAttMaxD + 1];
-    __shared__ float Vs[32][kAttMaxD + 1];
-    __shared__ float Qs[kAttWarps][kAttMaxD];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+template <int DP, typename T>
+__global__ void __launch_bounds__(256) attention_kernel(const float* __restrict__ q, const float* __restrict__ k,
+                                                        const float* __restrict__ v, const float* g,
+                                                        const T* __restrict__ mask, long long mask_row,
+                                                        long long mask_k, float inf, const float* __restrict__ pair_bias,
+                                                        float* out, int N, int H, int d, float scale,
+                                                        long long rows_per_bias) {
+    constexpr int DC = DP / 16;
+    extern __shared__ __align__(16) float att_smem[];
+    float* Qs = att_smem;                     // [DP][kAttP]
+    float* Ks = Qs + DP * kAttP;              // [DP][kAttP]
+    float* Vs = Ks + DP * kAttP;              // [64][DP]
+    float* Ps = Vs + kAttK * DP;              // [64 keys][kAttP]
+    float* Ms = Ps + kAttK * kAttP;           // [64]
+    umma::grid_trigger();
+    umma::grid_wait();
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const long long bb = blockIdx.x;
-    const int h = blockIdx.y;
-    const int qi = blockIdx.z * kAttWarps + warp;
-    const bool q_valid = qi < N;
-    const long long row_pitch = (long long)H * d;
-    const float* qrow = q + (bb * N + (q_valid ? qi : 0)) * row_pitch + (long long)h * d;
-    for (int c = lane; c < d; c += 32) Qs[warp][c] = qrow[c];
-    const float* pb = pair_bias
-                          ? pair_bias + (((bb / rows_per_bias) * H + h) * (long long)N +
-                                         (q_valid ? qi : 0)) * N
-                          : nullptr;
-    const float* mb = mask_bias ? mask_bias + bb * N : nullptr;
-    float m = -INFINITY, l = 0.f, o0 = 0.f, o1 = 0.f;
-    for (int k0 = 0; k0 < N; k0 += 32) {
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < 32 * d; idx += kAttWarps * 32) {
-            const int kk = idx / d, c = idx % d;
-            const int gk = k0 + kk;
-            float kv = 0.f, vv = 0.f;
-            if (gk < N) {
-                const long long off = (bb * N + gk) * row_pitch + (long long)h * d + c;
-                kv = k[off];
-                vv = v[off];
-            }
-            Ks[kk][c] = kv;
-            Vs[kk][c] = vv;
-        }
-        __syncthreads();
-        const int gk = k0 + lane;
-        float s = -INFINITY;
-        if (gk < N) {
-            float dot = 0.f;
-            for (int c = 0; c < d; ++c) dot = fmaf(Qs[warp][c], Ks[lane][c], dot);
-            s = dot * scale;
-            if (mb) s += mb[gk];
-            if (pb) s += pb[gk];
-        }
-        const float m_new = fmaxf(m, warp_max(s));
-        const float p = (gk < N) ? expf(s - m_new) : 0.f;
-        const float corr = expf(m - m_new);
-        l = l * corr + warp_sum(p);
-        o0 *= corr;
-        o1 *= corr;
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j) {
-            const float pj = __shfl_sync(0xffffffffu, p, j);
-            o0 = fmaf(pj, Vs[j][lane], o0);
-            if (d > 32) o1 = fmaf(pj, Vs[j][(lane + 32) < kAttMaxD ? lane + 32 : 0], o1);
-        }
-        m = m_new;
+    const int h = blockIdx.y, q0 = blockIdx.z * kAttQ;
+    const long long pitch = (long long)H * d, base = bb * N * pitch + (long long)h * d;
+    for (int idx = threadIdx.x; idx < kAttQ * DP; idx += 256) {
+        const int i = idx / DP, c = idx % DP;
+        Qs[c * kAttP + i] = (q0 + i < N && c < d) ? q[base + (q0 + i) * pitch + c] : 0.f;
     }
-    if (q_valid) {
-        float* orow = out + (bb * N + qi) * row_pitch + (long long)h * d;
-        const float inv = 1.0f / l;
-        if (lane < d) orow[lane] = o0 * inv;
-        if (lane + 32 < d) orow[lane + 32] = o1 * inv;
+    const float* pb = pair_bias ? pair_bias + ((bb / rows_per_bias) * H + h) * (long long)N * N : nullptr;
+    float m[4], l[4], o[4][DC];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < DC; ++c) o[i][c] = 0.f;
+    }
+    for (int k0 = 0; k0 < N; k0 += kAttK) {
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < kAttK * DP; idx += 256) {
+            const int i = idx / DP, c = idx % DP;
+            const bool in = k0 + i < N && c < d;
+            const long long off = base + (k0 + i) * pitch + c;
+            Ks[c * kAttP + i] = in ? k[off] : 0.f;
+            Vs[i * DP + c] = in ? v[off] : 0.f;
+        }
+        if (threadIdx.x < kAttK) {
+            const int kk = k0 + threadIdx.x;
+            Ms[threadIdx.x] = kk >= N ? -INFINITY
+                              : (mask ? inf * (ld_as_float(mask + bb * mask_row + kk * mask_k) - 1.0f) : 0.f);
+        }
+        __syncthreads();
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 8
+        for (int c = 0; c < DP; ++c) {
+            const float4 a = *reinterpret_cast<const float4*>(&Qs[c * kAttP + ty * 4]);
+            const float4 b = *reinterpret_cast<const float4*>(&Ks[c * kAttP + tx * 4]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] = fmaf(av[i], bv[j], s[i][j]);
+        }
+        float p[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int qi = q0 + ty * 4 + i;
+            float mx = -INFINITY;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int kk = k0 + tx * 4 + j;
+                float x = s[i][j] * scale + Ms[tx * 4 + j];
+                if (pb && qi < N && kk < N) x += pb[(long long)qi * N + kk];
+                s[i][j] = x;
+                mx = fmaxf(mx, x);
+            }
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+            const float m_new = fmaxf(m[i], mx);   // finite: the first block holds a key < N
+            const float corr = expf(m[i] - m_new);
+            m[i] = m_new;
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                p[i][j] = expf(s[i][j] - m_new);
+                sum += p[i][j];
+            }
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+            l[i] = l[i] * corr + sum;
+#pragma unroll
+            for (int c = 0; c < DC; ++c) o[i][c] *= corr;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(&Ps[(tx * 4 + j) * kAttP + ty * 4]) = make_float4(p[0][j], p[1][j], p[2][j], p[3][j]);
+        __syncthreads();
+#pragma unroll 8
+        for (int kk = 0; kk < kAttK; ++kk) {
+            const float4 a = *reinterpret_cast<const float4*>(&Ps[kk * kAttP + ty * 4]);
+            const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int c = 0; c < DC; ++c) {
+                const float vv = Vs[kk * DP + tx * DC + c];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[i][c] = fmaf(av[i], vv, o[i][c]);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int qi = q0 + ty * 4 + i;
+        if (qi >= N) continue;
+        const float inv = 1.0f / l[i];
+        const long long off = base + qi * pitch;
+#pragma unroll
+        for (int c = 0; c < DC; ++c) {
+            const int cc = tx * DC + c;
+            if (cc < d) out[off + cc] = o[i][c] * inv * sigmoid_acc(g[off + cc]);
+        }
     }
 }
-
 
 // ------------------------------------------------------------------ fused pair-bias projection
 // LN(x).w_h = rstd * sum_c (x_c - mean) * (gamma_c w_hc) + sum_c beta_c w_hc
@@ -204,6 +288,8 @@ __global__ void __launch_bounds__(128) pair_bias_c128_h16_kernel(const T* __rest
                                                                  long long nn) {
     __shared__ float ws[16][128];
     __shared__ float cs[16];
+    umma::grid_trigger();
+    umma::grid_wait();
     for (int i = threadIdx.x; i < 16 * 128; i += 128) {
         const int c = i & 127;
         ws[i >> 7][c] = ld_as_float(w + i) * (gamma ? ld_as_float(gamma + c) : 1.0f);
@@ -277,76 +363,17 @@ __global__ void __launch_bounds__(128) pair_bias_c128_h16_kernel(const T* __rest
 }
 
 // ------------------------------------------------------------------ elementwise
-template <typename T>
-__global__ void gate_mul_mask_kernel(const float* __restrict__ g, const float* __restrict__ p,
-                                     int ld, const T* __restrict__ mask, float* __restrict__ dst,
-                                     long long rows, int C) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * C) return;
-    const long long r = i / C;
-    const int c = (int)(i % C);
-    const float mk = mask ? ld_as_float(mask + r) : 1.0f;
-    dst[i] = mk * sigmoid_acc(g[r * ld + c]) * p[r * ld + c];
-}
-__global__ void sigmoid_mul_kernel(const float* __restrict__ x, int ldx, const float* __restrict__ g,
-                                   int ldg, float* __restrict__ dst, long long rows, int C) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * C) return;
-    const long long r = i / C;
-    const int c = (int)(i % C);
-    dst[i] = x[r * ldx + c] * sigmoid_acc(g[r * ldg + c]);
-}
-__global__ void silu_mul_kernel(const float* __restrict__ a, const float* __restrict__ b, int ld,
-                                float* __restrict__ dst, long long rows, int C) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * C) return;
-    const long long r = i / C;
-    const int c = (int)(i % C);
-    const float av = a[r * ld + c];
-    dst[i] = av * sigmoid_acc(av) * b[r * ld + c];
-}
 __global__ void ada_combine_kernel(const float* __restrict__ g, const float* __restrict__ a,
                                    const float* __restrict__ s, float* __restrict__ dst,
                                    long long n) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = sigmoid_acc(g[i]) * a[i] + s[i];
 }
-template <typename T>
-__global__ void mask_to_bias_kernel(const T* __restrict__ mask, float* __restrict__ dst,
-                                    long long rows, int N, float inf, long long row_stride,
-                                    long long k_stride) {
+__global__ void swap_heads_kernel(const float* __restrict__ src, float* __restrict__ dst, long long B, long long nn, int H) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * N) return;
-    const long long r = i / N;
-    const int kk = (int)(i % N);
-    dst[i] = inf * (ld_as_float(mask + r * row_stride + kk * k_stride) - 1.0f);
-}
-template <typename T>
-__global__ void finalize_kernel(const float* __restrict__ upd, const float* __restrict__ gate,
-                                const T* residual, const T* __restrict__ mask, T* out,
-                                long long rows, int C, long long inner, long long outer_stride,
-                                long long inner_stride) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * C) return;
-    const long long r = i / C;
-    const int c = (int)(i % C);
-    const long long off = (r / inner) * outer_stride + (r % inner) * inner_stride + c;
-    float v = upd[i];
-    if (gate) v *= sigmoid_acc(gate[i]);
-    if (mask) v *= ld_as_float(mask + r);
-    if (residual) v += ld_as_float(residual + off);
-    st_from_float(out + off, v);
-}
-__global__ void permute_bias_kernel(const float* __restrict__ src, float* __restrict__ dst,
-                                    long long B, int N, int H) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long total = B * H * (long long)N * N;
-    if (i >= total) return;
-    const int kk = (int)(i % N);
-    const int qq = (int)((i / N) % N);
-    const int h = (int)((i / ((long long)N * N)) % H);
-    const long long b = i / ((long long)N * N * H);
-    dst[i] = src[((b * N + qq) * N + kk) * H + h];
+    if (i >= B * H * nn) return;
+    const long long h = (i / nn) % H, b = i / (nn * H);
+    dst[i] = src[(h * B + b) * nn + i % nn];
 }
 template <typename T>
 __global__ void to_f32_kernel(const T* __restrict__ src, float* __restrict__ dst, long long n) {
@@ -358,91 +385,67 @@ __global__ void to_f32_kernel(const T* __restrict__ src, float* __restrict__ dst
 
 // ------------------------------------------------------------------ host wrappers
 template <typename TX, typename TP>
-int layernorm(const TX* x, const TP* gamma, const TP* beta, float* y, long long rows, int C,
-              float eps, long long inner, long long outer_stride, long long inner_stride,
-              cudaStream_t stream) {
+int layernorm(const TX* x, const TP* gamma, const TP* beta, float* y, long long rows, int C, float eps, RowMap map,
+              cudaStream_t stream, const TP* proj_w, int H, float* proj) {
     if (rows <= 0) return OF3_OK;
     LaunchScope scope(20, stream);
-    layernorm_kernel<TX, TP><<<grid_for(rows, kThreads / 32), kThreads, 0, stream>>>(
-        x, gamma, beta, y, rows, C, eps, inner, outer_stride, inner_stride);
-    OF3_CUDA_CHECK(cudaGetLastError());
+    OF3_CUDA_CHECK(launch_chained(layernorm_kernel<TX, TP>, grid_for(rows, kThreads / 32), kThreads, 0, stream, x, gamma,
+                                  beta, y, rows, C, eps, map, proj_w, H, proj));
     return OF3_OK;
 }
-template int layernorm<float, float>(const float*, const float*, const float*, float*, long long, int,
-                                     float, long long, long long, long long, cudaStream_t);
-template int layernorm<__nv_bfloat16, __nv_bfloat16>(const __nv_bfloat16*, const __nv_bfloat16*,
-                                                     const __nv_bfloat16*, float*, long long, int,
-                                                     float, long long, long long, long long,
-                                                     cudaStream_t);
-template int layernorm<float, __nv_bfloat16>(const float*, const __nv_bfloat16*, const __nv_bfloat16*,
-                                             float*, long long, int, float, long long, long long,
-                                             long long, cudaStream_t);
+#define INSTANTIATE_LN(TX, TP)                                                                                       \
+    template int layernorm<TX, TP>(const TX*, const TP*, const TP*, float*, long long, int, float, RowMap, cudaStream_t, \
+                                   const TP*, int, float*);
+INSTANTIATE_LN(float, float)
+INSTANTIATE_LN(__nv_bfloat16, __nv_bfloat16)
 
-template <typename TW>
-int gemm_nt(const float* A, const TW* W, const TW* bias, float* out, const GemmDesc& d,
-            cudaStream_t stream) {
-    if (d.batch <= 0 || d.M <= 0 || d.N <= 0) return OF3_OK;
-    OF3_REQUIRE(d.batch <= 65535, OF3_ERR_SHAPE, "gemm_nt: batch %d > 65535", d.batch);
-    dim3 grid(ceil_div(d.N, kTN), ceil_div(d.M, kTM), d.batch);
-    OF3_REQUIRE(grid.y <= 65535, OF3_ERR_SHAPE, "gemm_nt: M %d too large for one launch", d.M);
+template <typename TP>
+int layernorm_planes(const float* x, const TP* gamma, const TP* beta, float* y, long long rows, int C, float eps,
+                     cudaStream_t stream) {
+    if (rows <= 0) return OF3_OK;
     LaunchScope scope(20, stream);
-    gemm_nt_kernel<TW><<<grid, 256, 0, stream>>>(A, W, bias, out, d);
-    OF3_CUDA_CHECK(cudaGetLastError());
+    OF3_CUDA_CHECK(launch_chained(layernorm_planes_kernel<TP>, grid_for(rows, 32), kThreads, 0, stream, x, gamma, beta, y,
+                                  rows, C, eps));
     return OF3_OK;
 }
-template int gemm_nt<float>(const float*, const float*, const float*, float*, const GemmDesc&,
-                            cudaStream_t);
-template int gemm_nt<__nv_bfloat16>(const float*, const __nv_bfloat16*, const __nv_bfloat16*, float*,
-                                    const GemmDesc&, cudaStream_t);
+template int layernorm_planes<float>(const float*, const float*, const float*, float*, long long, int, float, cudaStream_t);
+template int layernorm_planes<__nv_bfloat16>(const float*, const __nv_bfloat16*, const __nv_bfloat16*, float*, long long,
+                                             int, float, cudaStream_t);
 
-int attention(const float* q, const float* k, const float* v, const float* mask_bias,
-              const float* pair_bias, float* out, long long BB, int N, int H, int d, float scale,
-              long long rows_per_bias, cudaStream_t stream) {
-    OF3_REQUIRE(d >= 1 && d <= kAttMaxD, OF3_ERR_SHAPE, "attention: head dim %d not in [1, %d]", d,
-                kAttMaxD);
-    OF3_REQUIRE(H <= 65535, OF3_ERR_SHAPE, "attention: too many heads");
-    OF3_REQUIRE(ceil_div(N, kAttWarps) <= 65535, OF3_ERR_SHAPE, "attention: N %d too large", N);
-    if (BB <= 0) return OF3_OK;
-    dim3 grid((unsigned)BB, H, ceil_div(N, kAttWarps));
-    LaunchScope scope(20, stream);
-    attention_kernel<<<grid, kAttWarps * 32, 0, stream>>>(q, k, v, mask_bias, pair_bias, out, N, H, d,
-                                                          scale, rows_per_bias);
-    OF3_CUDA_CHECK(cudaGetLastError());
+template <int DP, typename T>
+static int attention_launch(const float* q, const float* k, const float* v, const float* g, const T* mask,
+                            long long mask_row, long long mask_k, float inf, const float* pair_bias, float* out,
+                            long long BB, int N, int H, int d, float scale, long long rows_per_bias, cudaStream_t st) {
+    constexpr int smem = att_smem_floats<DP>() * 4;
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(attention_kernel<DP, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        configured.mark();
+    }
+    LaunchScope scope(20, st);
+    OF3_CUDA_CHECK(launch_chained(attention_kernel<DP, T>, dim3((unsigned)BB, H, ceil_div(N, kAttQ)), 256, smem, st, q, k,
+                                  v, g, mask, mask_row, mask_k, inf, pair_bias, out, N, H, d, scale, rows_per_bias));
     return OF3_OK;
 }
-
 template <typename T>
-int gate_mul_mask(const float* g, const float* p, int ld, const T* mask, float* dst, long long rows,
-                  int C, cudaStream_t stream) {
-    if (rows <= 0) return OF3_OK;
-    LaunchScope scope(20, stream);
-    gate_mul_mask_kernel<T><<<grid_for(rows * C, kThreads), kThreads, 0, stream>>>(g, p, ld, mask, dst,
-                                                                                  rows, C);
-    OF3_CUDA_CHECK(cudaGetLastError());
-    return OF3_OK;
+int attention(const float* q, const float* k, const float* v, const float* g, const T* mask, long long mask_row,
+              long long mask_k, float inf, const float* pair_bias, float* out, long long BB, int N, int H, int d,
+              float scale, long long rows_per_bias, cudaStream_t st) {
+    OF3_REQUIRE(d >= 1 && d <= kAttMaxD, OF3_ERR_SHAPE, "attention: head dim %d not in [1, %d]", d, kAttMaxD);
+    OF3_REQUIRE(H <= 65535, OF3_ERR_SHAPE, "attention: too many heads");
+    OF3_REQUIRE(ceil_div(N, kAttQ) <= 65535, OF3_ERR_SHAPE, "attention: N %d too large", N);
+    if (BB <= 0) return OF3_OK;
+#define ATT(DP) attention_launch<DP, T>(q, k, v, g, mask, mask_row, mask_k, inf, pair_bias, out, BB, N, H, d, scale, \
+                                        rows_per_bias, st)
+    return d <= 16 ? ATT(16) : (d <= 32 ? ATT(32) : (d <= 48 ? ATT(48) : ATT(64)));
+#undef ATT
 }
-template int gate_mul_mask<float>(const float*, const float*, int, const float*, float*, long long,
-                                  int, cudaStream_t);
-template int gate_mul_mask<__nv_bfloat16>(const float*, const float*, int, const __nv_bfloat16*,
-                                          float*, long long, int, cudaStream_t);
+template int attention<float>(const float*, const float*, const float*, const float*, const float*, long long, long long,
+                              float, const float*, float*, long long, int, int, int, float, long long, cudaStream_t);
+template int attention<__nv_bfloat16>(const float*, const float*, const float*, const float*, const __nv_bfloat16*,
+                                      long long, long long, float, const float*, float*, long long, int, int, int, float,
+                                      long long, cudaStream_t);
 
-int sigmoid_mul(const float* x, int ldx, const float* g, int ldg, float* dst, long long rows, int C,
-                cudaStream_t stream) {
-    if (rows <= 0) return OF3_OK;
-    LaunchScope scope(20, stream);
-    sigmoid_mul_kernel<<<grid_for(rows * C, kThreads), kThreads, 0, stream>>>(x, ldx, g, ldg, dst,
-                                                                             rows, C);
-    OF3_CUDA_CHECK(cudaGetLastError());
-    return OF3_OK;
-}
-int silu_mul(const float* a, const float* b, int ld, float* dst, long long rows, int C,
-             cudaStream_t stream) {
-    if (rows <= 0) return OF3_OK;
-    LaunchScope scope(20, stream);
-    silu_mul_kernel<<<grid_for(rows * C, kThreads), kThreads, 0, stream>>>(a, b, ld, dst, rows, C);
-    OF3_CUDA_CHECK(cudaGetLastError());
-    return OF3_OK;
-}
 int ada_combine(const float* g, const float* a, const float* s, float* dst, long long n,
                 cudaStream_t stream) {
     if (n <= 0) return OF3_OK;
@@ -452,39 +455,6 @@ int ada_combine(const float* g, const float* a, const float* s, float* dst, long
     return OF3_OK;
 }
 template <typename T>
-int mask_to_bias(const T* mask, float* dst, long long rows, int N, float inf, long long row_stride,
-                 long long k_stride, cudaStream_t stream) {
-    if (rows <= 0) return OF3_OK;
-    LaunchScope scope(20, stream);
-    mask_to_bias_kernel<T><<<grid_for(rows * N, kThreads), kThreads, 0, stream>>>(
-        mask, dst, rows, N, inf, row_stride, k_stride);
-    OF3_CUDA_CHECK(cudaGetLastError());
-    return OF3_OK;
-}
-template int mask_to_bias<float>(const float*, float*, long long, int, float, long long, long long,
-                                 cudaStream_t);
-template int mask_to_bias<__nv_bfloat16>(const __nv_bfloat16*, float*, long long, int, float,
-                                         long long, long long, cudaStream_t);
-
-template <typename T>
-int finalize(const float* upd, const float* gate, const T* residual, const T* mask, T* out,
-             long long rows, int C, long long inner, long long outer_stride,
-             long long inner_stride, cudaStream_t stream) {
-    if (rows <= 0) return OF3_OK;
-    LaunchScope scope(20, stream);
-    finalize_kernel<T><<<grid_for(rows * C, kThreads), kThreads, 0, stream>>>(
-        upd, gate, residual, mask, out, rows, C, inner, outer_stride, inner_stride);
-    OF3_CUDA_CHECK(cudaGetLastError());
-    return OF3_OK;
-}
-template int finalize<float>(const float*, const float*, const float*, const float*, float*,
-                             long long, int, long long, long long, long long, cudaStream_t);
-template int finalize<__nv_bfloat16>(const float*, const float*, const __nv_bfloat16*,
-                                     const __nv_bfloat16*, __nv_bfloat16*, long long, int, long long,
-                                     long long, long long, cudaStream_t);
-
-
-template <typename T>
 int pair_bias_c128_h16(const T* z, const T* gamma, const T* beta, const T* w, float* dst, long long B,
                        long long positions_per_sample, cudaStream_t stream) {
     const long long nn = positions_per_sample;
@@ -492,8 +462,8 @@ int pair_bias_c128_h16(const T* z, const T* gamma, const T* beta, const T* w, fl
     if (rows <= 0) return OF3_OK;
     OF3_REQUIRE(((uintptr_t)z & 15) == 0, OF3_ERR_ALIGN, "pair_bias: z must be 16-byte aligned");
     LaunchScope scope(20, stream);
-    pair_bias_c128_h16_kernel<T><<<grid_for(rows, 128), 128, 0, stream>>>(z, gamma, beta, w, dst, rows, nn);
-    OF3_CUDA_CHECK(cudaGetLastError());
+    OF3_CUDA_CHECK(launch_chained(pair_bias_c128_h16_kernel<T>, grid_for(rows, 128), 128, 0, stream, z, gamma, beta, w,
+                                  dst, rows, nn));
     return OF3_OK;
 }
 template int pair_bias_c128_h16<float>(const float*, const float*, const float*, const float*, float*,
@@ -501,11 +471,11 @@ template int pair_bias_c128_h16<float>(const float*, const float*, const float*,
 template int pair_bias_c128_h16<__nv_bfloat16>(const __nv_bfloat16*, const __nv_bfloat16*, const __nv_bfloat16*,
                                                const __nv_bfloat16*, float*, long long, long long, cudaStream_t);
 
-int permute_bias(const float* src, float* dst, long long B, int N, int H, cudaStream_t stream) {
-    const long long total = B * H * (long long)N * N;
+int swap_heads(const float* src, float* dst, long long B, int N, int H, cudaStream_t stream) {
+    const long long nn = (long long)N * N, total = B * H * nn;
     if (total <= 0) return OF3_OK;
     LaunchScope scope(20, stream);
-    permute_bias_kernel<<<grid_for(total, kThreads), kThreads, 0, stream>>>(src, dst, B, N, H);
+    swap_heads_kernel<<<grid_for(total, kThreads), kThreads, 0, stream>>>(src, dst, B, nn, H);
     OF3_CUDA_CHECK(cudaGetLastError());
     return OF3_OK;
 }

@@ -11,6 +11,8 @@ from __future__ import annotations
 
 import torch
 
+from .lib import side_stream
+
 
 class GraphedModule:
     """``GraphedModule(fn, *example_args, warmup=2)(*args) -> the outputs of fn``, replayed from a CUDA graph.
@@ -28,7 +30,7 @@ class GraphedModule:
             raise ValueError("GraphedModule needs CUDA example arguments")
         dev = next(a.device for a in self._static_in if a is not None)
         cur = torch.cuda.current_stream(dev)
-        side = torch.cuda.Stream(dev)
+        side = side_stream(cur)   # shared, so that its workspace is there for the next graph
         side.wait_stream(cur)
         with torch.no_grad(), torch.cuda.stream(side):
             for _ in range(max(1, warmup)):   # workspaces, packed weights and caches exist before the capture

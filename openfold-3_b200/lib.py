@@ -219,6 +219,24 @@ def dtype_code(dtype: torch.dtype) -> int:
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 
 
+_side_streams: dict[tuple[int, int], torch.cuda.Stream] = {}
+
+
+def side_stream(main: torch.cuda.Stream) -> torch.cuda.Stream:
+    """The second stream of callers that run on ``main``. One per main stream and not one per module, so that a new
+    module finds the stream's workspace allocated; never ``main`` itself, whose workspace it must not share."""
+    key = (main.device_index, main.cuda_stream)
+    st = _side_streams.get(key)
+    if st is None:
+        st = torch.cuda.Stream(main.device_index)
+        while st.cuda_stream == main.cuda_stream:   # torch hands its streams out in turn
+            st = torch.cuda.Stream(main.device_index)
+        if len(_side_streams) >= 64:   # callers with ever-new streams
+            _side_streams.clear()
+        _side_streams[key] = st
+    return st
+
+
 def workspace(nbytes: int, device: torch.device, stream: torch.cuda.Stream | None = None) -> torch.Tensor:
     """Grow-only scratch buffer per (device, stream; default the current one); owned by torch, handed to the library
     per call."""

@@ -736,7 +736,6 @@ class PairFormerStack(_Tracked):
         self.tune_chunk_size = tune_chunk_size
         self.chunk_size_tuner = None  # nothing to tune: the kernels never materialise N^3 logits
         self.overlap_single_track = True   # run each block's single track on a second stream (CUDA only)
-        self._side_streams = {}
         self.blocks = nn.ModuleList([
             PairFormerBlock(c_s=c_s, c_z=c_z, c_hidden_pair_bias=c_hidden_pair_bias,
                             no_heads_pair_bias=no_heads_pair_bias, c_hidden_mul=c_hidden_mul,
@@ -767,9 +766,7 @@ class PairFormerStack(_Tracked):
         # N x 384 values) runs on a second stream under the pair stack of block i + 1. The one thing it needs from
         # z, the pair-bias projection, is computed on the main stream before the next block overwrites z in place.
         main = torch.cuda.current_stream(z.device)
-        side = self._side_streams.get(z.device)
-        if side is None:
-            side = self._side_streams[z.device] = torch.cuda.Stream(z.device)
+        side = lib.side_stream(main)
         lib.stream_wait(side, main)
         for b in self.blocks:
             if b._run_native(s, z, single_mask, pair_mask, _mask_trans, side):

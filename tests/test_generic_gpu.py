@@ -1,0 +1,29 @@
+"""The fp32 GEMM and attention tiles of the shape-generic family at their edges (32- and 128-row tiles, 64 queries x 64 keys,
+widths that no vector load divides), against the oracle: 1e-4 x RMS on the worst element, the bar of the validation mode."""
+
+import pytest
+import torch
+
+from cases import OF3, W, _PF_KW, oracle, pkg, rand_mask, rel_err, token_pair_mask
+
+pytestmark = pytest.mark.gpu
+ODD = dict(c_s=36, c_z=20, c_hidden_pair_bias=9, no_heads_pair_bias=4, c_hidden_mul=19, c_hidden_pair_att=14,
+           no_heads_pair=3, transition_n=2)
+
+
+@pytest.mark.parametrize("dims,B,N", [(OF3, 1, 1), (OF3, 2, 33), (OF3, 1, 65), (ODD, 2, 31), (ODD, 1, 130)])
+def test_fp32_block_matches_the_oracle(dims, B, N):
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(N)
+    P = W.pairformer_block_params(seed=41, final_std=None, **dims)
+    s, z = torch.randn(B, N, dims["c_s"], generator=g), torch.randn(B, N, N, dims["c_z"], generator=g)
+    sm = rand_mask((B, N), g, 0.9)
+    pm = token_pair_mask(sm)
+    ref = oracle.pairformer_block(s, z, sm, pm, P, "", dims["no_heads_pair"], dims["no_heads_pair_bias"])
+    blk = pkg.PairFormerBlock(**dims, **_PF_KW)
+    blk.load_state_dict(P, strict=True)
+    blk = blk.to(dev).eval()
+    with torch.no_grad():
+        got = blk(s.to(dev), z.to(dev), sm.to(dev), pm.to(dev))
+    for a, b in zip(got, ref):
+        assert rel_err(a.cpu(), b) < 1e-4, rel_err(a.cpu(), b)
