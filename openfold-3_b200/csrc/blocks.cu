@@ -2,6 +2,7 @@
 // same order as the module entry points of api.cu, issued by native code. A pair block is 13 launches and the single track of a block 9 more; from
 // Python, one layer call at a time, they cost about 13 us of host time each (400 us per block: the 4-block trunk at
 // N = 37 took 1.6 ms for 0.3 ms of device work, and so did N = 256).
+#include "fast_pairbias.cuh"
 #include "fast_single.cuh"
 #include "generic_ops.cuh"
 #include "modules.cuh"
@@ -110,6 +111,8 @@ int single_track(void* s, const void* z, const void* bias, BiasForm form, const 
 // several of them: with few rows the projections of one block (6 matrices of c_a x c_s) fill a fraction of the chip and
 // cost a launch each; with many rows one block fills it, and its planes should stay in L2 until they are read.
 constexpr size_t kCondGroupBytes = 32u << 20;
+// Room for the bias images of the blocks whose pair bias one pass over z projects (24 blocks up to N = 1150).
+constexpr size_t kBiasGroupBytes = 1u << 30;
 
 int diffusion_stack(void* a, const void* s, const void* z, const void* mask, const void* const* bias,
                     const of3_diffusion_dims& D, int dtype, int flags, int blocks, const of3_attn_pair_bias_params* pa,
@@ -148,6 +151,14 @@ int diffusion_stack(void* a, const void* s, const void* z, const void* mask, con
         }
         return OF3_OK;
     }
+    // pair biases projected in the call: several blocks per pass over z, as many as fit kBiasGroupBytes
+    const size_t per_bias = (size_t)D.Bz * of3_pair_bias_tiles_elems(D.N) * sizeof(bf16);
+    int nbias = 0;
+    if (bias == nullptr) {
+        const size_t fit = kBiasGroupBytes / per_bias;
+        nbias = fit < 1 ? 1 : (fit > (size_t)fast::kMaxBiasLayers ? fast::kMaxBiasLayers : (int)fit);
+        if (nbias > blocks) nbias = blocks;
+    }
     const size_t per_block = (size_t)rows * 6 * D.c_a * sizeof(bf16);
     int group = per_block ? (int)(kCondGroupBytes / per_block) : 1;
     if (group < 1) group = 1;
@@ -156,6 +167,7 @@ int diffusion_stack(void* a, const void* s, const void* z, const void* mask, con
     return ws.run([&](Arena& A) -> int {
         bf16* planes = (bf16*)A.take(group * per_block);
         bf16* sn = (bf16*)A.take((size_t)(2 * group + 1) * rows * D.c_s * sizeof(bf16));
+        bf16* tiles = nbias ? (bf16*)A.take(nbias * per_bias) : nullptr;
         const size_t mark = A.off;
         size_t need = A.off;
         for (int b0 = 0; b0 < blocks; b0 += group) {
@@ -174,9 +186,21 @@ int diffusion_stack(void* a, const void* s, const void* z, const void* mask, con
                 const int b = b0 + i;
                 const bf16* cond = planes ? planes + (size_t)i * 6 * rows * D.c_a : (const bf16*)256;
                 A.off = mark;
+                const bf16* bt = bias ? (const bf16*)bias[b] : (const bf16*)256;
+                if (bias == nullptr && A.base) {
+                    if (b % nbias == 0) {
+                        const int n = blocks - b < nbias ? blocks - b : nbias;
+                        fast::BiasLayer bl[fast::kMaxBiasLayers];
+                        for (int l = 0; l < n; ++l)
+                            bl[l] = {(const bf16*)pa[b + l].ln_z_w, (const bf16*)pa[b + l].ln_z_b, (const bf16*)pa[b + l].w_z};
+                        const int brc = fast::pair_bias_tiles((const bf16*)z, bl, n, tiles, D.Bz, D.N, st);
+                        if (brc) return brc;
+                    }
+                    bt = tiles + (size_t)(b % nbias) * (per_bias / sizeof(bf16));
+                }
                 int rc = fast::attn_pair_bias((const bf16*)a, (const bf16*)z, (const bf16*)s, (const bf16*)mask, (bf16*)a,
                                               D.Ba, D.Bz, D.N, D.c_a, D.c_s, D.H, D.d, D.inf, f, pa + b, A, st, nullptr,
-                                              bias ? (const bf16*)bias[b] : nullptr, cond);
+                                              bt, cond);
                 if (rc) return rc;
                 need = A.off > need ? A.off : need;
                 A.off = mark;

@@ -1,10 +1,19 @@
-// Pair-bias projection of the single track on the tensor pipe (bf16 z, c_z = 128, 16 heads):
-//   bias[h][pos] = sum_c LayerNorm_z(z[pos])[c] * W[h][c]          (attention_pair_bias.py:154-163)
-// One pass over z. Row tiles of 128 pair positions: TMA -> LayerNorm in place in the swizzled A operand
-// (one thread per row) -> one 128 x 16 x 128 tcgen05 GEMM against the resident 4 KB weight -> fp32 rows
-// written head-major. The LayerNorm pass is the long pole of every row-tile kernel here, so TWO sets of
-// four LayerNorm warps work on alternate tiles over a four-deep ring of z tiles; the thread-per-row SIMT
-// version (2048 FMAs and 512 shared-memory reads per row) took 188 us at N = 768.
+// Pair-bias projection of the single track and of the diffusion token stack on the tensor pipe (bf16 z, c_z = 128, 16
+// heads), for one layer or for several at once:
+//   bias_l[h][pos] = sum_c LayerNorm_l(z[pos])[c] * W_l[h][c]          (attention_pair_bias.py:154-163)
+// The layers differ in LayerNorm weights and projection only, so with W'_l = W_l * gamma_l (rounded to bf16 once per
+// launch, in the prologue) and the row's mean and 1 / std
+//   bias_l[h][pos] = rstd * (W'_l[h] . z[pos] - mean * sum_c W'_l[h][c]) + sum_c beta_l[c] W_l[h][c]
+// and z itself, unnormalised and unrounded, is the GEMM's operand: one pass over z for all layers, and no normalised tile
+// is written back to shared memory. (The operand error is one bf16 rounding per product, of the weight instead of the
+// activation; sums and the mean correction are fp32.)
+//
+// Per tile of 128 positions of a line: TMA -> per group of 128 output channels (8 layers x 16 heads) one 128 x 128 x 128
+// GEMM with the weights as the A operand, so that a TMEM lane is an output channel and its columns are consecutive
+// keys: a thread stores 32 bytes of a bias row at a time. Eight warps take the row statistics meanwhile.
+// Bound: HBM. 24 layers at N = 768 read 151 MB and write 453 MB, 94 us; one pass per layer (LayerNorm into the operand
+// tile, 2-byte stores) took 24 x 56 us.
+#include "fast_pairbias.cuh"
 #include "modules.cuh"
 #include "rowtile.cuh"
 #include "runtime.cuh"
@@ -17,51 +26,67 @@ using namespace umma;
 using namespace rowtile;
 
 constexpr int kKidPairBias = 9;
-constexpr int kStages = 4;
 constexpr int kHeads = 16;
-constexpr int kPbThreads = 32 * (2 + 8 + 4);  // producer, MMA, 2 x 4 LayerNorm warps, 4 epilogue warps
+constexpr int kZStages = 3;    // z tiles in flight
+constexpr int kRing = 4;       // row statistics of the last tiles: the epilogue trails the loads
+constexpr int kSlots = 4;      // TMEM slots of 128 columns
+constexpr int kStatWarps = 8;
+constexpr int kPbThreads = 32 * (2 + kStatWarps + 8);   // producer, MMA, statistics, two epilogue sets
 
+template <int G>   // groups of 128 output channels
 struct PbSmem {
-    static constexpr uint32_t kZ = 0;                              // 4 stages x 32 KB
-    static constexpr uint32_t kW = kStages * kTileBytes;           // 2 k-blocks x [16 rows x 128 B]
-    static constexpr uint32_t kGamma = kW + 4096;
-    static constexpr uint32_t kBeta = kGamma + 512;
-    static constexpr uint32_t kBars = kBeta + 512;
-    static constexpr uint32_t kTotal = kBars + 256;
-    static constexpr uint32_t kDyn = kTotal + 1024;
+    static constexpr uint32_t kW = 0;
+    static constexpr uint32_t kZ = G * kTileBytes;
+    static constexpr uint32_t kStat = kZ + kZStages * kTileBytes;    // ring x 2 x 128 floats: scale, scale * -mean
+    static constexpr uint32_t kConst = kStat + kRing * 1024;         // per channel: sum of W', constant term
+    static constexpr uint32_t kBars = kConst + G * 1024;
+    static constexpr uint32_t kDyn = kBars + 256 + 1024;
 };
 
+struct PbWeights {
+    const __nv_bfloat16 *ln_w[kMaxBiasLayers], *ln_b[kMaxBiasLayers], *w[kMaxBiasLayers];
+};
+
+// Output: with tiles != null the attention kernel's bias image of every layer (bf16, times log2(e), [layer][b*16 + h][key
+// block of 32][query row][32 keys], each 64-byte row in the 64-byte swizzle of a K-major A operand, keys past the end
+// zeros), lines = query rows; else (one layer) fp32 dst[line * 16 + h][position].
+template <int G>
 __global__ void __launch_bounds__(kPbThreads, 1)
-pair_bias_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmW,
-                    const __nv_bfloat16* __restrict__ ln_w, const __nv_bfloat16* __restrict__ ln_b,
-                    float* __restrict__ dst, __nv_bfloat16* __restrict__ tiles, int n_tok, long long rows, long long nn,
-                    int* status) {
+pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ PbWeights wts, int layers,
+                 float* __restrict__ dst, __nv_bfloat16* __restrict__ tiles, long long layer_stride, long long lines,
+                 int N, int* status) {
+    using Sm = PbSmem<G>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
-    float* gamma = reinterpret_cast<float*>(gbase + PbSmem::kGamma);
-    float* beta = reinterpret_cast<float*>(gbase + PbSmem::kBeta);
-    const uint32_t bars = sbase + PbSmem::kBars;
-    const uint32_t w_full = bars;
-    auto z_full = [&](int s) { return bars + 8u * (1 + s); };
-    auto z_empty = [&](int s) { return bars + 8u * (1 + kStages + s); };
-    auto a_ready = [&](int s) { return bars + 8u * (1 + 2 * kStages + s); };
-    auto slot_full = [&](int q) { return bars + 8u * (1 + 3 * kStages + q); };
-    auto slot_empty = [&](int q) { return bars + 8u * (3 + 3 * kStages + q); };
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + PbSmem::kBars + 160);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + PbSmem::kBars + 168);
+    float* stat = reinterpret_cast<float*>(gbase + Sm::kStat);
+    float2* chan = reinterpret_cast<float2*>(gbase + Sm::kConst);
+    const uint32_t bars = sbase + Sm::kBars;
+    auto z_full = [&](int s) { return bars + 8u * s; };
+    auto z_empty = [&](int s) { return bars + 8u * (kZStages + s); };
+    auto st_ready = [&](int r) { return bars + 8u * (2 * kZStages + r); };
+    auto st_free = [&](int r) { return bars + 8u * (2 * kZStages + kRing + r); };
+    auto slot_full = [&](int q) { return bars + 8u * (2 * kZStages + 2 * kRing + q); };
+    auto slot_empty = [&](int q) { return bars + 8u * (2 * kZStages + 2 * kRing + kSlots + q); };
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 200);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 208);
+    static_assert(8 * (2 * kZStages + 2 * kRing + 2 * kSlots) <= 200, "barrier block");
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long num_tiles = (rows + kRows - 1) / kRows;
+    const int tiles_per_line = (N + kRows - 1) / kRows;
+    const long long num_tiles = lines * tiles_per_line;
+    const float scale = tiles != nullptr ? 1.4426950408889634f : 1.0f;
 
     if (threadIdx.x == 0) {
-        mbar_init(w_full, 1);
-        for (int s = 0; s < kStages; ++s) {
+        for (int s = 0; s < kZStages; ++s) {
             mbar_init(z_full(s), 1);
-            mbar_init(z_empty(s), 1);
-            mbar_init(a_ready(s), 4);
+            mbar_init(z_empty(s), 1 + kStatWarps);
         }
-        for (int q = 0; q < 2; ++q) {
+        for (int r = 0; r < kRing; ++r) {
+            mbar_init(st_ready(r), kStatWarps);
+            mbar_init(st_free(r), 4 * G);
+        }
+        for (int q = 0; q < kSlots; ++q) {
             mbar_init(slot_full(q), 1);
             mbar_init(slot_empty(q), 4);
         }
@@ -69,118 +94,200 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
         mbar_fence_init();
         prefetch_tmap(&tmZ);
     }
-    if (threadIdx.x < 128) {
-        gamma[threadIdx.x] = ln_w ? __bfloat162float(ln_w[threadIdx.x]) : 1.0f;
-        beta[threadIdx.x] = ln_b ? __bfloat162float(ln_b[threadIdx.x]) : 0.0f;
+    // W' as swizzled operand tiles, 16 threads per channel; channels past the last layer are zeros
+    for (int idx = threadIdx.x; idx < G * 128 * 16; idx += kPbThreads) {
+        const int n = idx >> 4, seg = idx & 15, l = n >> 4, h = n & 15;
+        float cs = 0.f, cb = 0.f;
+        uint32_t o[4] = {0u, 0u, 0u, 0u};
+        if (l < layers) {
+            uint32_t wv[4], gv[4] = {0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u}, bv[4] = {0u, 0u, 0u, 0u};
+            ld_row8_any(wts.w[l] + h * kC + seg * 8, wv);
+            if (wts.ln_w[l]) ld_row8_any(wts.ln_w[l] + seg * 8, gv);
+            if (wts.ln_b[l]) ld_row8_any(wts.ln_b[l] + seg * 8, bv);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                o[e] = pack_bf16x2(bf16lo(wv[e]) * bf16lo(gv[e]), bf16hi(wv[e]) * bf16hi(gv[e]));
+                cs += bf16lo(o[e]) + bf16hi(o[e]);
+                cb = fmaf(bf16lo(wv[e]), bf16lo(bv[e]), fmaf(bf16hi(wv[e]), bf16hi(bv[e]), cb));
+            }
+        }
+        sts128(chunk_addr(sbase + Sm::kW + (n >> 7) * kTileBytes, n & 127, seg), make_uint4(o[0], o[1], o[2], o[3]));
+#pragma unroll
+        for (int w = 8; w > 0; w >>= 1) {
+            cs += __shfl_xor_sync(0xffffffffu, cs, w);
+            cb += __shfl_xor_sync(0xffffffffu, cb, w);
+        }
+        if (seg == 0) chan[n] = make_float2(cs, cb * scale);
     }
+    fence_proxy_async_smem();
     if (warp == 1) {
-        tmem_alloc(smem_u32((const void*)tmem_ptr), 32);
+        tmem_alloc(smem_u32((const void*)tmem_ptr), 512);
         tmem_relinquish();
     }
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_ptr;  // slot q = columns [16 q, 16 q + 16)
+    const uint32_t tmem_base = *tmem_ptr;
+    grid_trigger();
+    grid_wait();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
-            mbar_arrive_expect_tx(w_full, 4096);
-            for (int kb = 0; kb < 2; ++kb) tma_load_2d(sbase + PbSmem::kW + kb * 2048, &tmW, w_full, kb * 64, 0);
             uint32_t it = 0;
             for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
-                const int s = it % kStages;
-                if (!mbar_wait(z_empty(s), ((it / kStages) & 1u) ^ 1u, abort_flag)) {
+                const int s = it % kZStages;
+                if (!mbar_wait(z_empty(s), ((it / kZStages) & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidPairBias, 1);
                     break;
                 }
                 mbar_arrive_expect_tx(z_full(s), kTileBytes);
-                const uint32_t d = sbase + PbSmem::kZ + s * kTileBytes;
-                for (int kb = 0; kb < 2; ++kb) tma_load_2d(d + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, (int)(t * kRows));
+                const uint32_t d = sbase + Sm::kZ + s * kTileBytes;
+                for (int kb = 0; kb < 2; ++kb)
+                    tma_load_3d(d + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, (int)(t % tiles_per_line) * kRows,
+                                (int)(t / tiles_per_line));
             }
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
         if (lane == 0) {
-            constexpr uint32_t idesc = idesc_bf16_f32(128, kHeads);
-            bool ok = mbar_wait(w_full, 0, abort_flag);
-            if (!ok) report_wait_failure(status, abort_flag, kKidPairBias, 2);
-            uint32_t it = 0;
+            constexpr uint32_t idesc = idesc_bf16_f32(128, 128);
+            uint32_t it = 0, job = 0;
+            bool ok = true;
             for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
-                const int s = it % kStages, q = it & 1;
-                if (!mbar_wait(a_ready(s), (it / kStages) & 1u, abort_flag)) {
-                    report_wait_failure(status, abort_flag, kKidPairBias, 3);
+                const int s = it % kZStages;
+                if (!mbar_wait(z_full(s), (it / kZStages) & 1u, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidPairBias, 2);
                     break;
                 }
-                if (!mbar_wait(slot_empty(q), ((it >> 1) & 1u) ^ 1u, abort_flag)) {
-                    report_wait_failure(status, abort_flag, kKidPairBias, 4);
+                for (int g = 0; g < G; ++g, ++job) {
+                    const int q = job % kSlots;
+                    if (!mbar_wait(slot_empty(q), ((job / kSlots) & 1u) ^ 1u, abort_flag)) {
+                        report_wait_failure(status, abort_flag, kKidPairBias, 3);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    mma_rows<128>(tmem_base + q * 128, sbase + Sm::kW + g * kTileBytes, sbase + Sm::kZ + s * kTileBytes,
+                                  kKBlockBytes, idesc, false);
+                    mma_commit(slot_full(q));
+                }
+                if (ok) mma_commit(z_empty(s));
+            }
+        }
+    } else if (warp < 2 + kStatWarps) {
+        // ---------------------------------------------------------------- row statistics: 16 positions per warp
+        const int row = (warp - 2) * 16 + (lane & 15), half = lane >> 4;
+        uint32_t it = 0;
+        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+            const int s = it % kZStages, r = it % kRing;
+            if (!mbar_wait(z_full(s), (it / kZStages) & 1u, abort_flag) ||
+                !mbar_wait(st_free(r), ((it / kRing) & 1u) ^ 1u, abort_flag)) {
+                if (lane == 0) report_wait_failure(status, abort_flag, kKidPairBias, 4);
+                break;
+            }
+            uint32_t raw[32];
+            load_half_row(sbase + Sm::kZ + s * kTileBytes, row, half, raw);
+            float mean, rstd;
+            half_row_stats(raw, mean, rstd);
+            if (half == 0) {
+                const float p = rstd * scale;
+                stat[r * 256 + row] = p;
+                stat[r * 256 + 128 + row] = -p * mean;
+            }
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(z_empty(s));
+                mbar_arrive(st_ready(r));
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------- epilogue: thread = output channel
+        const int set = (warp - 2 - kStatWarps) >> 2, quad = warp & 3;
+        const int nkb = (N + 31) >> 5;
+        const long long hs = (long long)nkb * N * 32;   // elements per (sample, head) of the bias image
+        uint32_t it = 0, job = 0;
+        bool ok = true;
+        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
+            const long long line = t / tiles_per_line;
+            const int t0 = (int)(t % tiles_per_line) * kRows;
+            const int live = N - t0 < kRows ? N - t0 : kRows;                       // positions that exist
+            const int span = tiles != nullptr ? ((live + 31) & ~31) : live;         // positions to be written
+            const int r = it % kRing;
+            const float* p1 = stat + r * 256;
+            for (int g = 0; g < G; ++g, ++job) {
+                if ((int)(job & 1u) != set) continue;
+                const int q = job % kSlots;
+                if (!mbar_wait(st_ready(r), (it / kRing) & 1u, abort_flag) ||
+                    !mbar_wait(slot_full(q), (job / kSlots) & 1u, abort_flag)) {
+                    if (lane == 0) report_wait_failure(status, abort_flag, kKidPairBias, 5);
+                    ok = false;
                     break;
                 }
                 tc_fence_after_sync();
-                mma_k128(tmem_base + q * kHeads, sbase + PbSmem::kZ + s * kTileBytes, sbase + PbSmem::kW, 2048, idesc,
-                         false);
-                mma_commit(slot_full(q));
-                mma_commit(z_empty(s));
-            }
-        }
-    } else if (warp < 10) {
-        // ---------------------------------------------------------------- two LayerNorm sets, alternate tiles
-        const int set = (warp - 2) >> 2;
-        const int row = (warp & 3) * 32 + lane;  // any bijection warp -> 32 rows works here (no TMEM access)
-        uint32_t it = 0;
-        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
-            if ((int)(it & 1u) != set) continue;
-            const int s = it % kStages;
-            if (!mbar_wait(z_full(s), (it / kStages) & 1u, abort_flag)) {
-                if (lane == 0) report_wait_failure(status, abort_flag, kKidPairBias, 5);
-                break;
-            }
-            const uint32_t tile = sbase + PbSmem::kZ + s * kTileBytes;
-            uint32_t raw[64];
-            load_row(tile, row, raw);
-            float mean, rstd;
-            row_stats(raw, mean, rstd);
-            store_normalized_row(tile, row, raw, mean, rstd, gamma, beta);
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(a_ready(s));
-        }
-    } else {
-        // ---------------------------------------------------------------- epilogue warps (10..13)
-        const int quad = warp & 3;
-        const int row = quad * 32 + lane;
-        uint32_t it = 0;
-        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
-            const int q = it & 1;
-            if (!mbar_wait(slot_full(q), (it >> 1) & 1u, abort_flag)) {
-                if (lane == 0) report_wait_failure(status, abort_flag, kKidPairBias, 6);
-                break;
-            }
-            tc_fence_after_sync();
-            uint32_t r[16];
-            tmem_ld16(tmem_base + ((uint32_t)(quad * 32) << 16) + q * kHeads, r);
-            tmem_ld_wait();
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(slot_empty(q));
-            const long long pos = t * kRows + row;
-            if (pos < rows) {
-                const long long b = pos / nn, qk = pos - b * nn;
-                if (tiles != nullptr) {
-                    // the attention kernel's bias image: bf16, times log2(e), [b*16 + h][key block of 32][query row][32
-                    // keys], each 64-byte row in the 64-byte swizzle of a K-major A operand
-                    const int i = (int)(qk / n_tok), j = (int)(qk - (long long)i * n_tok);
-                    const long long nkb = (n_tok + 31) >> 5;
-                    const long long hs = nkb * n_tok * 32;   // elements per (sample, head)
-                    __nv_bfloat16* d = tiles + (b * kHeads) * hs + ((long long)(j >> 5) * n_tok + i) * 32 +
-                                       (((((j & 31) >> 3) ^ ((i >> 1) & 3)) << 3) | (j & 7));
+                const int n = g * 128 + quad * 32 + lane, l = n >> 4, h = n & 15;
+                if (g * 128 + quad * 32 < layers * kHeads) {   // the warp has a channel (a layer is half a warp)
+                    const float2 cc = chan[n];
+                    __nv_bfloat16* trow = nullptr;
+                    float* drow = nullptr;
+                    int sw = 0;
+                    const bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
+                    if (tiles != nullptr) {
+                        const long long b = line / N, i = line - b * N;
+                        sw = (int)(i >> 1) & 3;
+                        trow = tiles + l * layer_stride + (b * kHeads + h) * hs + i * 32;
+                    } else {
+                        drow = dst + (line * kHeads + h) * (long long)N + t0;
+                    }
+                    const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + q * 128;
+#pragma unroll 2
+                    for (int k0 = 0; k0 < span; k0 += 16) {
+                        uint32_t acc[16];
+                        tmem_ld16(taddr + k0, acc);
+                        float v[16];
+                        tmem_ld_wait();
 #pragma unroll
-                    for (int h = 0; h < kHeads; ++h)
-                        d[h * hs] = __float2bfloat16_rn(__uint_as_float(r[h]) * 1.4426950408889634f);
-                } else {
-                    float* d = dst + (b * kHeads) * nn + qk;
+                        for (int e = 0; e < 16; e += 4) {
+                            const float4 a = *reinterpret_cast<const float4*>(p1 + k0 + e);
+                            const float4 m = *reinterpret_cast<const float4*>(p1 + 128 + k0 + e);
+                            v[e] = fmaf(a.x, __uint_as_float(acc[e]), fmaf(m.x, cc.x, cc.y));
+                            v[e + 1] = fmaf(a.y, __uint_as_float(acc[e + 1]), fmaf(m.y, cc.x, cc.y));
+                            v[e + 2] = fmaf(a.z, __uint_as_float(acc[e + 2]), fmaf(m.z, cc.x, cc.y));
+                            v[e + 3] = fmaf(a.w, __uint_as_float(acc[e + 3]), fmaf(m.w, cc.x, cc.y));
+                        }
+                        if (tiles != nullptr && l < layers) {
+                            if (k0 + 16 > live) {   // keys past the end
 #pragma unroll
-                    for (int h = 0; h < kHeads; ++h) d[h * nn] = __uint_as_float(r[h]);
+                                for (int e = 0; e < 16; ++e)
+                                    if (k0 + e >= live) v[e] = 0.f;
+                            }
+                            // chunks c2 and c2 + 1 of the row lie at c2 ^ sw and (c2 + 1) ^ sw: one aligned pair
+                            const int c2 = (k0 >> 3) & 2;
+                            uint32_t o[8], w[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) o[e] = pack_bf16x2(v[2 * e], v[2 * e + 1]);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) w[e] = (sw & 1) ? o[e ^ 4] : o[e];
+                            stg256(trow + (long long)((t0 + k0) >> 5) * N * 32 + ((c2 ^ (sw & 2)) << 3), w);
+                        } else if (l < layers) {
+                            if (vec && k0 + 16 <= live) {
+#pragma unroll
+                                for (int e = 0; e < 16; e += 4)
+                                    *reinterpret_cast<float4*>(drow + k0 + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+                            } else {
+#pragma unroll
+                                for (int e = 0; e < 16; ++e)
+                                    if (k0 + e < live) drow[k0 + e] = v[e];
+                            }
+                        }
+                        __syncwarp();
+                    }
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(slot_empty(q));
+                    mbar_arrive(st_free(r));
                 }
             }
         }
@@ -190,72 +297,80 @@ pair_bias_tc_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
     __syncthreads();
     if (warp == 1) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, 32);
+        tmem_dealloc(tmem_base, 512);
+    }
+}
+
+template <int G>
+int launch_g(const CUtensorMap& tmZ, const PbWeights& wts, int layers, float* dst, __nv_bfloat16* tiles,
+             long long layer_stride, long long lines, int N, cudaStream_t st) {
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(pair_bias_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            PbSmem<G>::kDyn));
+        configured.mark();
+    }
+    const long long num_tiles = lines * ceil_div(N, kRows);
+    const int grid = (int)(num_tiles < sm_count() ? num_tiles : sm_count());
+    LaunchScope scope(kKidPairBias, st);
+    OF3_CUDA_CHECK(launch_chained(pair_bias_kernel<G>, grid, kPbThreads, PbSmem<G>::kDyn, st, tmZ, wts, layers, dst, tiles,
+                                  layer_stride, lines, N, device_status_ptr()));
+    return OF3_OK;
+}
+
+int launch(const __nv_bfloat16* z, const BiasLayer* layer, int layers, float* dst, __nv_bfloat16* tiles,
+           long long layer_stride, long long lines, int N, cudaStream_t st) {
+    if (lines <= 0 || N <= 0) return OF3_OK;
+    OF3_REQUIRE(((uintptr_t)z & 15) == 0, OF3_ERR_ALIGN, "pair_bias: z must be 16-byte aligned");
+    OF3_REQUIRE(((uintptr_t)tiles & 31) == 0, OF3_ERR_ALIGN, "pair_bias: bias tiles must be 32-byte aligned");
+    OF3_REQUIRE(lines < (1LL << 31), OF3_ERR_SHAPE, "pair_bias: too many pair positions");
+    OF3_REQUIRE(layers >= 1 && layers <= kMaxBiasLayers, OF3_ERR_ARG, "pair_bias: %d layers", layers);
+    PbWeights wts = {};
+    for (int l = 0; l < layers; ++l) {
+        wts.ln_w[l] = layer[l].ln_w;
+        wts.ln_b[l] = layer[l].ln_b;
+        wts.w[l] = layer[l].w;
+    }
+    CUtensorMap tmZ;
+    uint64_t dims[3] = {128, (uint64_t)N, (uint64_t)lines};
+    uint64_t str[2] = {256, (uint64_t)N * 256};
+    uint32_t box[3] = {64, 128, 1};
+    const int rc = make_tmap_bf16(&tmZ, z, 3, dims, str, box, 1);
+    if (rc) return rc;
+    switch ((layers * kHeads + 127) / 128) {
+        case 1: return launch_g<1>(tmZ, wts, layers, dst, tiles, layer_stride, lines, N, st);
+        case 2: return launch_g<2>(tmZ, wts, layers, dst, tiles, layer_stride, lines, N, st);
+        default: return launch_g<3>(tmZ, wts, layers, dst, tiles, layer_stride, lines, N, st);
     }
 }
 
 }  // namespace
-
-namespace {
-int pair_bias_launch(const __nv_bfloat16* z, const __nv_bfloat16* ln_w, const __nv_bfloat16* ln_b,
-                     const __nv_bfloat16* w, float* dst, __nv_bfloat16* tiles, int n_tok, long long B, long long nn,
-                     cudaStream_t st);
-}
 
 // dst[b][h][pos] (fp32) for B samples of nn pair positions each; z [B * nn][128] bf16.
 int pair_bias_c128_h16(const __nv_bfloat16* z, const __nv_bfloat16* ln_w, const __nv_bfloat16* ln_b,
                        const __nv_bfloat16* w, float* dst, long long B, long long nn, cudaStream_t st) {
-    return pair_bias_launch(z, ln_w, ln_b, w, dst, nullptr, 0, B, nn, st);
+    OF3_REQUIRE(nn < (1LL << 31) - 256, OF3_ERR_SHAPE, "pair_bias: too many pair positions");
+    const BiasLayer l{ln_w, ln_b, w};
+    return launch(z, &l, 1, dst, nullptr, 0, B, (int)nn, st);
 }
 
-// The same projection written straight into the bias image of the single-track attention kernel (bf16 tiles
-// [b*16 + h][key block of 32][N query rows][32], times log2(e)): no fp32 tensor in between. z [B][N][N][128].
-int pair_bias_tiles_c128_h16(const __nv_bfloat16* z, const __nv_bfloat16* ln_w, const __nv_bfloat16* ln_b,
-                             const __nv_bfloat16* w, __nv_bfloat16* tiles, long long B, int N, cudaStream_t st) {
-    if (N % 32 != 0) {   // the key padding of the last block must read as zeros
-        const size_t bytes = (size_t)B * kHeads * ((N + 31) / 32) * N * 32 * sizeof(__nv_bfloat16);
-        OF3_CUDA_CHECK(cudaMemsetAsync(tiles, 0, bytes, st));
+int pair_bias_tiles(const __nv_bfloat16* z, const BiasLayer* layer, int layers, __nv_bfloat16* tiles, long long B, int N,
+                    cudaStream_t st) {
+    const long long stride = B * kHeads * (long long)((N + 31) / 32) * N * 32;
+    for (int l0 = 0; l0 < layers; l0 += kMaxBiasLayers) {
+        const int n = layers - l0 < kMaxBiasLayers ? layers - l0 : kMaxBiasLayers;
+        const int rc = launch(z, layer + l0, n, nullptr, tiles + l0 * stride, stride, B * N, N, st);
+        if (rc) return rc;
     }
-    return pair_bias_launch(z, ln_w, ln_b, w, nullptr, tiles, N, B, (long long)N * N, st);
-}
-
-namespace {
-int pair_bias_launch(const __nv_bfloat16* z, const __nv_bfloat16* ln_w, const __nv_bfloat16* ln_b,
-                     const __nv_bfloat16* w, float* dst, __nv_bfloat16* tiles, int n_tok, long long B, long long nn,
-                     cudaStream_t st) {
-    const long long rows = B * nn;
-    if (rows <= 0) return OF3_OK;
-    OF3_REQUIRE(((uintptr_t)z & 15) == 0 && ((uintptr_t)w & 15) == 0, OF3_ERR_ALIGN,
-                "pair_bias: z and the weight must be 16-byte aligned");
-    OF3_REQUIRE(rows < (1LL << 31) - 256, OF3_ERR_SHAPE, "pair_bias: too many pair positions");
-    int rc;
-    CUtensorMap tmZ, tmW;
-    {
-        uint64_t dims[2] = {128, (uint64_t)rows};
-        uint64_t str[1] = {256};
-        uint32_t box[2] = {64, 128};
-        if ((rc = make_tmap_bf16(&tmZ, z, 2, dims, str, box, 1))) return rc;
-    }
-    {
-        uint64_t dims[2] = {128, (uint64_t)kHeads};
-        uint64_t str[1] = {256};
-        uint32_t box[2] = {64, (uint32_t)kHeads};
-        if ((rc = make_tmap_bf16(&tmW, w, 2, dims, str, box, 1))) return rc;
-    }
-    if (!device_configured(3)) {
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(pair_bias_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            PbSmem::kDyn));
-        device_mark_configured(3);
-    }
-    const long long num_tiles = (rows + kRows - 1) / kRows;
-    const int grid = (int)(num_tiles < sm_count() ? num_tiles : sm_count());
-    LaunchScope scope(kKidPairBias, st);
-    pair_bias_tc_kernel<<<grid, kPbThreads, PbSmem::kDyn, st>>>(tmZ, tmW, ln_w, ln_b, dst, tiles, n_tok, rows, nn,
-                                                                device_status_ptr());
-    OF3_CUDA_CHECK(cudaGetLastError());
     return OF3_OK;
 }
-}  // namespace
+
+// One layer's bias image (z [B][N][N][128]).
+int pair_bias_tiles_c128_h16(const __nv_bfloat16* z, const __nv_bfloat16* ln_w, const __nv_bfloat16* ln_b,
+                             const __nv_bfloat16* w, __nv_bfloat16* tiles, long long B, int N, cudaStream_t st) {
+    const BiasLayer l{ln_w, ln_b, w};
+    return pair_bias_tiles(z, &l, 1, tiles, B, N, st);
+}
 
 }  // namespace fast
 }  // namespace of3
