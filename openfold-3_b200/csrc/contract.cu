@@ -11,8 +11,8 @@
 //   warp 0     TMA producer     A tile 128x64, B tile BNx64 per k-block, 128B swizzle
 //   warp 1     MMA issuer       tcgen05.mma 128 x BN x 16, accumulators double-buffered in TMEM
 //   warps 2-5  epilogue         tcgen05.ld -> bf16 -> global (overlaps the next tile's main loop)
+#include "rowtile.cuh"
 #include "runtime.cuh"
-#include "umma.cuh"
 
 namespace of3 {
 namespace {
@@ -91,10 +91,9 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-                const int nt = (int)(t % num_nt);
-                const int mt = (int)((t / num_nt) % num_mt);
-                const int b = (int)(t / ((long long)num_nt * num_mt));
+            rowtile::TileWalk tw(blockIdx.x, gridDim.x, num_mt, num_nt);
+            for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, tw.next()) {
+                const int nt = tw.tile, mt = tw.line, b = tw.b;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % S;
                     const uint32_t ph = (it / S) & 1u;
@@ -154,10 +153,9 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         const int quad = warp & 3;  // TMEM lane quarter this warp may read
         uint32_t tcount = 0;
         bool ok = true;
-        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tcount) {
-            const int nt = (int)(t % num_nt);
-            const int mt = (int)((t / num_nt) % num_mt);
-            const int b = (int)(t / ((long long)num_nt * num_mt));
+        rowtile::TileWalk tw(blockIdx.x, gridDim.x, num_mt, num_nt);
+        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tcount, tw.next()) {
+            const int nt = tw.tile, mt = tw.line, b = tw.b;
             const uint32_t acc = tcount & 1u;
             const uint32_t acc_ph = (tcount >> 1) & 1u;
             if (!mbar_wait(tfull_bar(acc), acc_ph, abort_flag)) {

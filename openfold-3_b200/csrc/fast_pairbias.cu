@@ -75,6 +75,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_per_line = (N + kRows - 1) / kRows;
     const long long num_tiles = lines * tiles_per_line;
+    const int lines_per_sample = tiles != nullptr ? N : 1;
     const float scale = tiles != nullptr ? 1.4426950408889634f : 1.0f;
 
     if (threadIdx.x == 0) {
@@ -135,7 +136,8 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         // ---------------------------------------------------------------- TMA producer
         if (lane == 0) {
             uint32_t it = 0;
-            for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+            TileWalk tw(blockIdx.x, gridDim.x, lines_per_sample, tiles_per_line);
+            for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tw.next()) {
                 const int s = it % kZStages;
                 if (!mbar_wait(z_empty(s), ((it / kZStages) & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidPairBias, 1);
@@ -144,8 +146,8 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                 mbar_arrive_expect_tx(z_full(s), kTileBytes);
                 const uint32_t d = sbase + Sm::kZ + s * kTileBytes;
                 for (int kb = 0; kb < 2; ++kb)
-                    tma_load_3d(d + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, (int)(t % tiles_per_line) * kRows,
-                                (int)(t / tiles_per_line));
+                    tma_load_3d(d + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tw.tile * kRows,
+                                tw.b * lines_per_sample + tw.line);
             }
         }
     } else if (warp == 1) {
@@ -208,9 +210,9 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         const long long hs = (long long)nkb * N * 32;   // elements per (sample, head) of the bias image
         uint32_t it = 0, job = 0;
         bool ok = true;
-        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
-            const long long line = t / tiles_per_line;
-            const int t0 = (int)(t % tiles_per_line) * kRows;
+        TileWalk tw(blockIdx.x, gridDim.x, lines_per_sample, tiles_per_line);
+        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it, tw.next()) {
+            const int t0 = tw.tile * kRows;
             const int live = N - t0 < kRows ? N - t0 : kRows;                       // positions that exist
             const int span = tiles != nullptr ? ((live + 31) & ~31) : live;         // positions to be written
             const int r = it % kRing;
@@ -233,11 +235,10 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                     int sw = 0;
                     const bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
                     if (tiles != nullptr) {
-                        const long long b = line / N, i = line - b * N;
-                        sw = (int)(i >> 1) & 3;
-                        trow = tiles + l * layer_stride + (b * kHeads + h) * hs + i * 32;
+                        sw = (tw.line >> 1) & 3;
+                        trow = tiles + l * layer_stride + ((long long)tw.b * kHeads + h) * hs + tw.line * 32;
                     } else {
-                        drow = dst + (line * kHeads + h) * (long long)N + t0;
+                        drow = dst + ((long long)tw.b * kHeads + h) * N + t0;
                     }
                     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + q * 128;
 #pragma unroll 2

@@ -76,7 +76,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long num_tiles = (rows + kRows - 1) / kRows;
-    const long long my_tiles = (num_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    const long long my_tiles = tiles_of_block(num_tiles);
     const long long my_pairs = (my_tiles + 1) / 2;
 
     if (threadIdx.x == 0) {
@@ -392,7 +392,7 @@ transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long num_tiles = (rows + kRows - 1) / kRows;
-    const long long my_tiles = (num_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    const long long my_tiles = tiles_of_block(num_tiles);
 
     if (threadIdx.x == 0) {
         mbar_init(w_full, 1);

@@ -33,27 +33,16 @@ constexpr int kKidCore = 6;
 constexpr int kKidOut = 7;
 constexpr float kLog2e = 1.4426950408889634f;
 
-struct LineTile {
-    int b, line, t0;
-};
 // R = lines per sample (R == N for a whole pair tensor, N / P for a row shard)
-__device__ __forceinline__ LineTile line_tile(long long t, int R, int tiles_per_line) {
-    LineTile c;
-    c.t0 = (int)(t % tiles_per_line) * kRows;
-    const long long l = t / tiles_per_line;
-    c.line = (int)(l % R);
-    c.b = (int)(l / R);
-    return c;
-}
 // z tile of a line: rows (line, t0..t0+127) of the view; transposed view = z[b, t, line, :]
 template <int C, bool kTransposed>
 __device__ __forceinline__ void load_z_tile(uint32_t dst, const CUtensorMap* tm, uint32_t bar,
-                                            const LineTile& c, int R) {
+                                            const TileWalk& c, int R) {
     for (int kb = 0; kb < C / 64; ++kb) {
         if (kTransposed)
-            tma_load_4d(dst + kb * kKBlockBytes, tm, bar, kb * 64, c.line, c.t0, c.b);
+            tma_load_4d(dst + kb * kKBlockBytes, tm, bar, kb * 64, c.line, c.tile * kRows, c.b);
         else
-            tma_load_3d(dst + kb * kKBlockBytes, tm, bar, kb * 64, c.t0, c.b * R + c.line);
+            tma_load_3d(dst + kb * kKBlockBytes, tm, bar, kb * 64, c.tile * kRows, c.b * R + c.line);
     }
 }
 
@@ -167,13 +156,13 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
             for (int kb = 0; kb < C / 64; ++kb) tma_load_2d(sbase + Sm::kWb + kb * 2048, &tmWb, w_full, kb * 64, 0);
             grid_wait();
             uint32_t it = 0;
-            for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+            TileWalk tc(blockIdx.x, gridDim.x, R, tiles_per_line);
+            for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tc.next()) {
                 const int s = it % kSt;
                 if (!mbar_wait(z_empty(s), ((it / kSt) & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidProj, 1);
                     break;
                 }
-                const LineTile tc = line_tile(t, R, tiles_per_line);
                 mbar_arrive_expect_tx(z_full(s), tile_bytes<C>());
                 load_z_tile<C, kTransposed>(sbase + Sm::kZ + s * tile_bytes<C>(), &tmZ, z_full(s), tc, R);
             }
@@ -233,9 +222,9 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
         const float qscale = kLog2e * rsqrtf((float)D);
         uint32_t it = 0;
         bool ok = true;
-        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
-            const LineTile tc = line_tile(t, R, tiles_per_line);
-            const int pos = tc.t0 + row;
+        TileWalk tc(blockIdx.x, gridDim.x, R, tiles_per_line);
+        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it, tc.next()) {
+            const int pos = tc.tile * kRows + row;
             const bool valid = pos < npad;   // positions in [N, npad) are written as zeros (key padding)
             const bool live = pos < N;
             const int rpad = (R + 3) & ~3;
@@ -802,7 +791,7 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_per_line = (N + kRows - 1) / kRows;
     const long long num_tiles = (long long)B * R * tiles_per_line;
-    const long long my_tiles = (num_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    const long long my_tiles = tiles_of_block(num_tiles);
 
     if (threadIdx.x == 0) {
         mbar_init(w_full, 1);
@@ -845,10 +834,10 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
                 tma_load_2d(sbase + Sm::kWo + kb * C * 128, &tmWo, w_full, kb * 64, 0);
             }
             grid_wait();
-            for (long long lt = 0; lt < my_tiles; ++lt) {
+            TileWalk tc(blockIdx.x, gridDim.x, R, tiles_per_line);
+            for (long long lt = 0; lt < my_tiles; ++lt, tc.next()) {
                 const int g = (int)(lt & 1);
                 const uint32_t use = (uint32_t)(lt >> 1);
-                const LineTile tc = line_tile(blockIdx.x + lt * gridDim.x, R, tiles_per_line);
                 if (!mbar_wait(z_empty(g), (use & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidOut, 1);
                     break;
@@ -862,7 +851,7 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
                 mbar_arrive_expect_tx(o_full(g), tile_bytes<C>());
                 const uint32_t odst = sbase + Sm::kO + g * tile_bytes<C>();
                 for (int kb = 0; kb < C / 64; ++kb)
-                    tma_load_3d(odst + kb * kKBlockBytes, &tmO, o_full(g), kb * 64, tc.t0, tc.b * R + tc.line);
+                    tma_load_3d(odst + kb * kKBlockBytes, &tmO, o_full(g), kb * 64, tc.tile * kRows, tc.b * R + tc.line);
             }
         }
     } else if (warp == 1) {
@@ -909,9 +898,9 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
         const uint32_t ztile = sbase + Sm::kZ + g * tile_bytes<C>();
         const uint32_t otile = sbase + Sm::kO + g * tile_bytes<C>();
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * 256 + half * (C / 2);
-        for (long long lt = g; lt < my_tiles; lt += 2) {
+        TileWalk tc(blockIdx.x + g * gridDim.x, 2 * gridDim.x, R, tiles_per_line);
+        for (long long lt = g; lt < my_tiles; lt += 2, tc.next()) {
             const uint32_t use = (uint32_t)(lt >> 1);
-            const LineTile tc = line_tile(blockIdx.x + lt * gridDim.x, R, tiles_per_line);
             if (!mbar_wait(z_full(g), use & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidOut, 5);
                 break;
@@ -997,10 +986,10 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
                         asm volatile(
                             "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::
                                 "l"(reinterpret_cast<uint64_t>(&tmOut)),
-                            "r"(otile + kb * kKBlockBytes), "r"(kb * 64), "r"(tc.line), "r"(tc.t0), "r"(tc.b)
+                            "r"(otile + kb * kKBlockBytes), "r"(kb * 64), "r"(tc.line), "r"(tc.tile * kRows), "r"(tc.b)
                             : "memory");
                     } else {
-                        tma_store_3d(&tmOut, otile + kb * kKBlockBytes, kb * 64, tc.t0, tc.b * R + tc.line);
+                        tma_store_3d(&tmOut, otile + kb * kKBlockBytes, kb * 64, tc.tile * kRows, tc.b * R + tc.line);
                     }
                 }
                 tma_store_commit();

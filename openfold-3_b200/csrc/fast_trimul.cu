@@ -28,19 +28,7 @@ using namespace rowtile;
 constexpr int kKidIn = 2;
 constexpr int kKidOut = 3;
 
-struct TileCoord {
-    int b, fixed, t0;  // sample, fixed index (i), first row of the tile along the walking index
-};
 // R = lines per sample (R == N for a whole pair tensor, N / P for a row shard)
-__device__ __forceinline__ TileCoord tile_coord(long long t, int R, int tiles_per_line) {
-    TileCoord c;
-    c.t0 = (int)(t % tiles_per_line) * kRows;
-    const long long line = t / tiles_per_line;
-    c.fixed = (int)(line % R);
-    c.b = (int)(line / R);
-    return c;
-}
-
 // =====================================================================================
 // trimul_in
 // =====================================================================================
@@ -137,22 +125,23 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                     tma_load_2d(sbase + Sm::kW + kb * Sm::kWKb + w * C * 128, wm[w], w_full, kb * 64, 0);
             grid_wait();
             uint32_t it = 0;
-            for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+            TileWalk tw(blockIdx.x, gridDim.x, R, tiles_per_line);
+            for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tw.next()) {
                 const int s = it % kSt;
                 if (!mbar_wait(z_empty(s), ((it / kSt) & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidIn, 1);
                     break;
                 }
-                const TileCoord tc = tile_coord(t, R, tiles_per_line);
+                const int t0 = tw.tile * kRows;
                 mbar_arrive_expect_tx(z_full(s), tile_bytes<C>());
                 const uint32_t dst = sbase + Sm::kZ + s * tile_bytes<C>();
                 for (int kb = 0; kb < C / 64; ++kb) {
                     if (kOutgoing)
-                        tma_load_3d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tc.t0,
-                                    tc.b * R + tc.fixed);
+                        tma_load_3d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, t0,
+                                    tw.b * R + tw.line);
                     else
-                        tma_load_4d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tc.fixed, tc.t0,
-                                    tc.b);
+                        tma_load_4d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tw.line, t0,
+                                    tw.b);
                 }
             }
         }
@@ -203,7 +192,8 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         const int half = lane >> 4;
         grid_wait();
         uint32_t it = 0;
-        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+        TileWalk tw(blockIdx.x, gridDim.x, R, tiles_per_line);
+        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tw.next()) {
             const int s = it % kSt;
             if (!mbar_wait(z_full(s), (it / kSt) & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidIn, 5);
@@ -215,14 +205,14 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
             float mean, rstd;
             half_row_stats<C>(raw, mean, rstd);
             store_normalized_half_row<C>(tile, row, half, raw, mean, rstd, gamma, beta);
-            const TileCoord tc = tile_coord(t, R, tiles_per_line);
-            const int k = tc.t0 + row;
+            const int t0 = tw.tile * kRows;
+            const int k = t0 + row;
             float m = 0.f;   // positions past the end of the line are never stored
             if (k < N) {
                 m = 0.5f;
                 if (mask != nullptr) {
-                    const long long lin = kOutgoing ? ((long long)(tc.b * R + tc.fixed) * N + k)
-                                                    : ((long long)(tc.b * N + k) * R + tc.fixed);
+                    const long long lin = kOutgoing ? ((long long)(tw.b * R + tw.line) * N + k)
+                                                    : ((long long)(tw.b * N + k) * R + tw.line);
                     m = 0.5f * __bfloat162float(mask[lin]);
                 }
             }
@@ -252,10 +242,11 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + set * 256;
         grid_wait();
         uint32_t it = 0, use = 0;
-        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+        TileWalk tw(blockIdx.x, gridDim.x, R, tiles_per_line);
+        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tw.next()) {
             if (C == 64 && (it & 1u) != (uint32_t)set) continue;   // one job per tile: the sets take turns
-            const TileCoord tc = tile_coord(t, R, tiles_per_line);
-            const int kmax = (N - tc.t0 < kRows) ? N - tc.t0 : kRows;   // positions of the tile that exist
+            const int t0 = tw.tile * kRows;
+            const int kmax = (N - t0 < kRows) ? N - t0 : kRows;   // positions of the tile that exist
             if (!mbar_wait(slot_full(set), use & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidIn, 6);
                 break;
@@ -265,8 +256,8 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
             const float* mk = mask05 + (it % Sm::kMaskRing) * 128;
             // the line pitch ld is a multiple of 8 elements, so a 16-byte store that starts below N ends inside the
             // row; with a pitch that is a multiple of 16 (and 32-byte aligned planes) the same holds for 32 bytes
-            __nv_bfloat16* dst = plane + (long long)tc.b * ((C >> group_shift) * group_stride) +
-                                 (long long)tc.fixed * ld + tc.t0;
+            __nv_bfloat16* dst = plane + (long long)tw.b * ((C >> group_shift) * group_stride) +
+                                 (long long)tw.line * ld + t0;
             // 16 positions per pass; the TMEM load of the next pass is in flight while this one is computed
             auto emit = [&](const uint32_t (&p)[16], const uint32_t (&g)[16], int k0) {
                 uint32_t o[8];
@@ -404,22 +395,23 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                                 kb * 64, 0);
             grid_wait();
             uint32_t it = 0;
-            for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+            TileWalk tw(blockIdx.x, gridDim.x, R, tiles_per_line);
+            for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tw.next()) {
                 const int s = it & 1;
                 if (!mbar_wait(z_empty(s), ((it >> 1) & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidIn, 1);
                     break;
                 }
-                const TileCoord tc = tile_coord(t, R, tiles_per_line);
+                const int t0 = tw.tile * kRows;
                 mbar_arrive_expect_tx(z_full(s), kTileBytes);
                 const uint32_t dst = sbase + InSmem<128>::kZ + s * kTileBytes;
                 for (int kb = 0; kb < 2; ++kb) {
                     if (kOutgoing)
-                        tma_load_3d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tc.t0,
-                                    tc.b * R + tc.fixed);
+                        tma_load_3d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, t0,
+                                    tw.b * R + tw.line);
                     else
-                        tma_load_4d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tc.fixed, tc.t0,
-                                    tc.b);
+                        tma_load_4d(dst + kb * kKBlockBytes, &tmZ, z_full(s), kb * 64, tw.line, t0,
+                                    tw.b);
                 }
             }
         }
@@ -480,14 +472,15 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         const int row = quad * 32 + lane;
         uint32_t it = 0;
         bool ok = true;
-        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it) {
-            const TileCoord tc = tile_coord(t, R, tiles_per_line);
-            const int k = tc.t0 + row;
+        TileWalk tw(blockIdx.x, gridDim.x, R, tiles_per_line);
+        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it, tw.next()) {
+            const int t0 = tw.tile * kRows;
+            const int k = t0 + row;
             const bool valid = k < N;
             float m = 1.0f;
             if (valid && mask != nullptr) {
-                const long long lin = kOutgoing ? ((long long)(tc.b * R + tc.fixed) * N + k)
-                                                : ((long long)(tc.b * N + k) * R + tc.fixed);
+                const long long lin = kOutgoing ? ((long long)(tw.b * R + tw.line) * N + k)
+                                                : ((long long)(tw.b * N + k) * R + tw.line);
                 m = __bfloat162float(mask[lin]);
             }
             const float mh = 0.5f * m;
@@ -503,8 +496,8 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                 // rank when the planes are about to be exchanged
                 const long long cs = (long long)R * ld;
                 __nv_bfloat16* dst = (q == 0 ? a_t : b_t) +
-                                     (long long)tc.b * ((kC >> group_shift) * group_stride) +
-                                     (long long)tc.fixed * ld + k;
+                                     (long long)tw.b * ((kC >> group_shift) * group_stride) +
+                                     (long long)tw.line * ld + k;
                 const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + q * 256;
 #pragma unroll 1
                 for (int cb = 0; cb < 4; ++cb) {
@@ -594,7 +587,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     const int tiles_per_line = (N + kRows - 1) / kRows;
     const long long num_tiles = (long long)B * R * tiles_per_line;
     // tiles of this CTA alternate between the two groups: local tile index lt -> group lt & 1
-    const long long my_tiles = (num_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    const long long my_tiles = tiles_of_block(num_tiles);
 
     if (threadIdx.x == 0) {
         mbar_init(w_full, 1);
@@ -638,17 +631,18 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                 tma_load_2d(sbase + Sm::kWz + kb * C * 128, &tmWz, w_full, kb * 64, 0);
             }
             grid_wait();
-            for (long long lt = 0; lt < my_tiles; ++lt) {
+            TileWalk tw(blockIdx.x, gridDim.x, R, tiles_per_line);
+            for (long long lt = 0; lt < my_tiles; ++lt, tw.next()) {
                 const int g = (int)(lt & 1);
                 const uint32_t use = (uint32_t)(lt >> 1);
-                const TileCoord tc = tile_coord(blockIdx.x + lt * gridDim.x, R, tiles_per_line);
+                const int t0 = tw.tile * kRows;
                 if (!mbar_wait(x_empty(g), (use & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidOut, 1);
                     break;
                 }
                 // x tile: all 128 channels of positions (fixed, t0 .. t0+127), layout [c][j]
                 mbar_arrive_expect_tx(x_full(g), tile_bytes<C>());
-                tma_load_3d(sbase + Sm::kX + g * tile_bytes<C>(), &tmX, x_full(g), tc.t0, tc.fixed, tc.b * C);
+                tma_load_3d(sbase + Sm::kX + g * tile_bytes<C>(), &tmX, x_full(g), t0, tw.line, tw.b * C);
                 if (!mbar_wait(z_empty(g), (use & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidOut, 6);
                     break;
@@ -656,7 +650,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                 mbar_arrive_expect_tx(z_full(g), tile_bytes<C>());
                 const uint32_t zdst = sbase + Sm::kZ + g * tile_bytes<C>();
                 for (int kb = 0; kb < C / 64; ++kb)
-                    tma_load_3d(zdst + kb * kKBlockBytes, &tmZ, z_full(g), kb * 64, tc.t0, tc.b * R + tc.fixed);
+                    tma_load_3d(zdst + kb * kKBlockBytes, &tmZ, z_full(g), kb * 64, t0, tw.b * R + tw.line);
             }
         }
     } else if (warp == 1) {
@@ -690,9 +684,10 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
         const int gtid = (warp - 2 - g * 4) * 32 + lane;  // 0..127 inside the group
         const uint32_t ztile = sbase + Sm::kZ + g * tile_bytes<C>();
         const uint32_t xtile = sbase + Sm::kX + g * tile_bytes<C>();
-        for (long long lt = g; lt < my_tiles; lt += 2) {
+        TileWalk tw(blockIdx.x + g * gridDim.x, 2 * gridDim.x, R, tiles_per_line);
+        for (long long lt = g; lt < my_tiles; lt += 2, tw.next()) {
             const uint32_t use = (uint32_t)(lt >> 1);
-            const TileCoord tc = tile_coord(blockIdx.x + lt * gridDim.x, R, tiles_per_line);
+            const int t0 = tw.tile * kRows;
             if (!mbar_wait(x_full(g), use & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidOut, 4);
                 break;
@@ -762,7 +757,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
             group_sync(1 + g, 128);
             if (gtid == 0) {
                 for (int kb = 0; kb < C / 64; ++kb)
-                    tma_store_3d(&tmOut, ztile + kb * kKBlockBytes, kb * 64, tc.t0, tc.b * R + tc.fixed);
+                    tma_store_3d(&tmOut, ztile + kb * kKBlockBytes, kb * 64, t0, tw.b * R + tw.line);
                 tma_store_commit();
                 tma_store_wait_read<0>();
                 mbar_arrive(z_empty(g));

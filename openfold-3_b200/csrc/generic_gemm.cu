@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(G* BM / TM * BN / TN) gemm_kernel(const Args<T
             }
         } else if constexpr (EPI == kFinal) {
             const float mk = p.mask ? ld_as_float(p.mask + r) : 1.0f;
-            const long long off = (r / p.map.inner) * p.map.outer_stride + (r % p.map.inner) * p.map.inner_stride;
+            const long long off = row_offset(p.map, r);
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
                 const int c = col_of(j);

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kThreads) layernorm_kernel(const TX* __restric
     const int lane = threadIdx.x & 31;
     const long long r = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     if (r >= rows) return;
-    const TX* xr = x + (r / map.inner) * map.outer_stride + (r % map.inner) * map.inner_stride;
+    const TX* xr = x + row_offset(map, r);
     float* yr = y + r * C;
     const bool in_regs = C <= 32 * kLnRegs;
     float v[kLnRegs];

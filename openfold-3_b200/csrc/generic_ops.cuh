@@ -14,6 +14,15 @@ namespace generic {
 struct RowMap {
     long long inner, outer_stride, inner_stride;
 };
+#ifdef __CUDACC__
+__device__ __forceinline__ long long row_offset(const RowMap& m, long long r) {
+    if (((r | m.inner) >> 32) == 0) {   // a 64-bit division costs some 500 cycles
+        const uint32_t q = (uint32_t)r / (uint32_t)m.inner;
+        return q * m.outer_stride + (uint32_t)(r - (long long)q * m.inner) * m.inner_stride;
+    }
+    return (r / m.inner) * m.outer_stride + (r % m.inner) * m.inner_stride;
+}
+#endif
 inline RowMap dense_rows(long long rows, int C) { return RowMap{rows > 0 ? rows : 1, 0, C}; }
 
 // y[r, :] = LN(x[r, :]) * gamma + beta (gamma / beta may be null); y dense fp32 [rows, C] or null. With proj_w

@@ -60,7 +60,7 @@ __device__ __forceinline__ float sigmoid_of(float x) { return 1.0f / (1.0f + __e
 // One column group of 16 of this thread's row as attention operand images; `kind` is uniform over the tile.
 template <int D>
 __device__ __forceinline__ void store_images(const AttnImages& im, int kind, float qscale, const uint32_t (&r)[16],
-                                             int col0, long long row) {
+                                             int col0, long long row, long long bb, int pos) {
     constexpr int KD = SingleImage<D>::kKD, DV = SingleImage<D>::kDV;
     const int HD = im.H * D;
     if (kind == kOutG) {
@@ -71,8 +71,6 @@ __device__ __forceinline__ void store_images(const AttnImages& im, int kind, flo
         return;
     }
     const int n = im.rows_per_sample;
-    const long long bb = row / n;
-    const int pos = (int)(row - bb * n);
     const int nkb = (n + kSingleBK - 1) / kSingleBK, n_qt = (n + kSingleBQ - 1) / kSingleBQ;
     const int pad = nkb * kSingleBK - n;   // keys past the end of the last block: zeros, written by the first rows
 #pragma unroll
@@ -286,6 +284,11 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
             }
             tc_fence_after_sync();
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * Cfg::kAccStride + half * kCols;
+            [[maybe_unused]] int bb = 0, pos = 0;   // sample and position of the row
+            if constexpr (EPI == kEpiImages) {
+                bb = (int)((uint32_t)row / (uint32_t)ep.im.rows_per_sample);
+                pos = (int)row - bb * ep.im.rows_per_sample;
+            }
             float mk = 1.0f;
             if constexpr (EPI == kEpiResidual) {
                 if (ep.mask != nullptr && live) mk = __bfloat162float(ep.mask[row]);
@@ -299,7 +302,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                 const int col = c.nt * kWRows + half * kCols + c0;   // column inside the matrix
                 if (!live) continue;
                 if constexpr (EPI == kEpiImages) {
-                    store_images<D>(ep.im, ep.kind[c.g], ep.qscale, r, col, row);
+                    store_images<D>(ep.im, ep.kind[c.g], ep.qscale, r, col, row, bb, pos);
                 } else {
                     uint32_t o[8];
                     if constexpr (EPI == kEpiStore) {
