@@ -74,18 +74,20 @@ constexpr int kBK = 64;  // keys per key block = per attention step
 template <int D>
 __device__ __forceinline__ int qk_xor(int r) { return D == 32 ? (r >> 1) & 3 : (r >> 2) & 1; }
 
-// warps: 0 producer, 1 MMA issuer, 2..5 LayerNorm (one thread per row), 6..9 epilogue (TMEM slot 0: q, k;
-// slot 1: v and the 4-wide triangle bias). The bias projection is a fourth GEMM (N = 16 with 12 zero rows)
+// warps: 0 producer, 1 MMA issuer, 2..9 LayerNorm (two threads per row), 10..13 epilogue of TMEM slot 0 (q, k), 14..17 of
+// slot 1 (v and the 4-wide triangle bias): the epilogue is the longest part of a tile's chain. The bias projection is a fourth GEMM (N = 16 with 12 zero rows)
 // instead of 1024 FMAs per row inside the LayerNorm pass.
-constexpr int kProjThreads = 320;
+constexpr int kProjLnWarps = 8;
+constexpr int kProjThreads = 32 * (2 + kProjLnWarps + 8);
 constexpr int kBiasK = 32;  // keys per bias row
 // Pair-bias image: bf16, pre-scaled by log2(e), [b*4 + head][key block of 32][query row][32 keys]: the 128 rows
 // of a query tile and one key block are contiguous (one untiled bulk copy) and each 64-byte row is stored in the
 // 64-byte swizzle of a K-major tcgen05 A operand (16-byte chunk c of query row q at chunk c ^ ((q / 2) % 4)),
 // because the attention kernel adds the bias on the tensor pipe: S += bias_tile * I_32^T.
 
+// 64 channels: two CTAs share an SM (template stack, N = 300 x 4: 58 -> 49 us)
 template <int C, bool kTransposed>
-__global__ void __launch_bounds__(kProjThreads, 1)
+__global__ void __launch_bounds__(kProjThreads, C == 64 ? 2 : 1)
 triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmWq,
                     const __grid_constant__ CUtensorMap tmWk, const __grid_constant__ CUtensorMap tmWv,
                     const __grid_constant__ CUtensorMap tmWb,
@@ -119,7 +121,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
         for (int s = 0; s < kSt; ++s) {
             mbar_init(z_full(s), 1);
             mbar_init(z_empty(s), 1);
-            mbar_init(a_ready(s), 4);
+            mbar_init(a_ready(s), kProjLnWarps);
         }
         for (int q = 0; q < 2; ++q) {
             mbar_init(slot_full(q), 1);
@@ -195,9 +197,10 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
                 if (ok) mma_commit(z_empty(s));
             }
         }
-    } else if (warp < 6) {
-        // LayerNorm warps: normalise in place (the A operand of all four GEMMs)
-        const int row = (warp - 2) * 32 + lane;
+    } else if (warp < 2 + kProjLnWarps) {
+        // LayerNorm warps: normalise in place (the A operand of all four GEMMs); a warp takes 16 positions, lanes 0..15
+        // their first half of the channels, lanes 16..31 the other half
+        const int row = (warp - 2) * 16 + (lane & 15), half = lane >> 4;
         uint32_t it = 0;
         for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
             const int s = it % kSt;
@@ -206,105 +209,105 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
                 break;
             }
             const uint32_t tile = sbase + Sm::kZ + s * tile_bytes<C>();
-            uint32_t raw[C / 2];
-            load_row<C>(tile, row, raw);
+            uint32_t raw[C / 4];
+            load_half_row<C>(tile, row, half, raw);
             float mean, rstd;
-            row_stats<C>(raw, mean, rstd);
-            store_normalized_row<C>(tile, row, raw, mean, rstd, gamma, beta);
+            half_row_stats<C>(raw, mean, rstd);
+            store_normalized_half_row<C>(tile, row, half, raw, mean, rstd, gamma, beta);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(a_ready(s));
         }
     } else {
         // epilogue warps
+        const int set = (warp - 2 - kProjLnWarps) >> 2;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         const float qscale = kLog2e * rsqrtf((float)D);
+        const int rpad = (R + 3) & ~3;
+        const int nkb = npad >> 6;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
         uint32_t it = 0;
-        bool ok = true;
         TileWalk tc(blockIdx.x, gridDim.x, R, tiles_per_line);
-        for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++it, tc.next()) {
+        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tc.next()) {
             const int pos = tc.tile * kRows + row;
             const bool valid = pos < npad;   // positions in [N, npad) are written as zeros (key padding)
             const bool live = pos < N;
-            const int rpad = (R + 3) & ~3;
-            const int nkb = npad >> 6;
-            // ---- slot 0: q (columns [0, C)) and k ([C, 2C))
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
-            if (!mbar_wait(slot_full(0), it & 1u, abort_flag)) {
-                if (lane == 0) report_wait_failure(status, abort_flag, kKidProj, 6);
+            if (!mbar_wait(slot_full(set), it & 1u, abort_flag)) {
+                if (lane == 0) report_wait_failure(status, abort_flag, kKidProj, 6 + set);
                 break;
             }
             tc_fence_after_sync();
+            if (set == 0) {
+                // ---- slot 0: q (columns [0, C)) and k ([C, 2C))
 #pragma unroll 1
-            for (int qk = 0; qk < 2; ++qk) {
-                __nv_bfloat16* base = qk == 0 ? q_out : k_out;
-                const float sc = qk == 0 ? qscale : 1.0f;
+                for (int qk = 0; qk < 2; ++qk) {
+                    __nv_bfloat16* base = qk == 0 ? q_out : k_out;
+                    const float sl = live ? (qk == 0 ? qscale : 1.0f) : 0.f;
 #pragma unroll 1
-                for (int h = 0; h < kH; ++h) {
-                    uint32_t r[D];
-                    if constexpr (D == 32) tmem_ld32(taddr + qk * C + h * D, r);
-                    else tmem_ld16(taddr + qk * C + h * D, r);
-                    tmem_ld_wait();
-                    if (valid || qk == 0) {
-                        const long long bh = (long long)tc.b * kH + h;
-                        const long long rowidx = qk == 0
-                            ? ((bh * tiles_per_line + (pos >> 7)) * rpad + tc.line) * 128 + (pos & 127)
-                            : ((bh * nkb + (pos >> 6)) * rpad + tc.line) * kBK + (pos & 63);
-                        uint4* dst = reinterpret_cast<uint4*>(base + rowidx * D);
-                        const float sl = live ? sc : 0.f;
+                    for (int h = 0; h < kH; ++h) {
+                        uint32_t r[D];
+                        if constexpr (D == 32) tmem_ld32(taddr + qk * C + h * D, r);
+                        else tmem_ld16(taddr + qk * C + h * D, r);
+                        tmem_ld_wait();
+                        if (valid || qk == 0) {
+                            const long long bh = (long long)tc.b * kH + h;
+                            const long long rowidx = qk == 0
+                                ? ((bh * tiles_per_line + tc.tile) * rpad + tc.line) * 128 + row
+                                : ((bh * nkb + (pos >> 6)) * rpad + tc.line) * kBK + (pos & 63);
+                            __nv_bfloat16* dst = base + rowidx * D;
+                            // 32 bytes at a time: chunks c2 and c2 + 1 of the row lie at c2 ^ x and (c2 + 1) ^ x
+                            const int x = qk_xor<D>(pos);
 #pragma unroll
-                        for (int v4 = 0; v4 < D / 8; ++v4) {
-                            uint4 v;
-                            v.x = pack_bf16x2(sl * __uint_as_float(r[v4 * 8 + 0]), sl * __uint_as_float(r[v4 * 8 + 1]));
-                            v.y = pack_bf16x2(sl * __uint_as_float(r[v4 * 8 + 2]), sl * __uint_as_float(r[v4 * 8 + 3]));
-                            v.z = pack_bf16x2(sl * __uint_as_float(r[v4 * 8 + 4]), sl * __uint_as_float(r[v4 * 8 + 5]));
-                            v.w = pack_bf16x2(sl * __uint_as_float(r[v4 * 8 + 6]), sl * __uint_as_float(r[v4 * 8 + 7]));
-                            dst[v4 ^ qk_xor<D>(pos)] = v;
+                            for (int c2 = 0; c2 < D / 8; c2 += 2) {
+                                uint32_t o[8], w[8];
+#pragma unroll
+                                for (int e = 0; e < 8; ++e)
+                                    o[e] = pack_bf16x2(sl * __uint_as_float(r[c2 * 8 + 2 * e]),
+                                                       sl * __uint_as_float(r[c2 * 8 + 2 * e + 1]));
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) w[e] = (x & 1) ? o[e ^ 4] : o[e];
+                                stg256(dst + ((c2 ^ (x & 2)) << 3), w);
+                            }
                         }
                     }
                 }
-            }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(slot_empty(0));
-            // ---- slot 1: v, transposed
-            if (!mbar_wait(slot_full(1), it & 1u, abort_flag)) {
-                if (lane == 0) report_wait_failure(status, abort_flag, kKidProj, 7);
-                ok = false;
-                break;
-            }
-            tc_fence_after_sync();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(slot_empty(0));
+            } else {
+                // ---- slot 1: v, transposed; the triangle bias
 #pragma unroll 1
-            for (int h = 0; h < kH; ++h) {
-                uint32_t r[D];
-                if constexpr (D == 32) tmem_ld32(taddr + 2 * C + h * D, r);
-                else tmem_ld16(taddr + 2 * C + h * D, r);
-                tmem_ld_wait();
-                if (valid) {
-                    __nv_bfloat16* tile =
-                        vt_out + ((((long long)tc.b * kH + h) * nkb + (pos >> 6)) * rpad + tc.line) * (long long)(D * kBK);
-                    const int c = (pos & 63) >> 3, w = pos & 7;
+                for (int h = 0; h < kH; ++h) {
+                    uint32_t r[D];
+                    if constexpr (D == 32) tmem_ld32(taddr + 2 * C + h * D, r);
+                    else tmem_ld16(taddr + 2 * C + h * D, r);
+                    tmem_ld_wait();
+                    if (valid) {
+                        __nv_bfloat16* tile = vt_out + ((((long long)tc.b * kH + h) * nkb + (pos >> 6)) * rpad + tc.line) *
+                                                           (long long)(D * kBK);
+                        const int c = (pos & 63) >> 3, w = pos & 7;
 #pragma unroll
-                    for (int e = 0; e < D; ++e)
-                        tile[e * kBK + (((c ^ (e & 7)) << 3) | w)] =
-                            __float2bfloat16_rn(live ? __uint_as_float(r[e]) : 0.f);
+                        for (int e = 0; e < D; ++e)
+                            tile[e * kBK + (((c ^ (e & 7)) << 3) | w)] =
+                                __float2bfloat16_rn(live ? __uint_as_float(r[e]) : 0.f);
+                    }
                 }
-            }
-            uint32_t tbr[16];  // triangle bias of this position: columns 3C..3C+3, pre-scaled for exp2
-            tmem_ld16(taddr + 3 * C, tbr);
-            tmem_ld_wait();
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(slot_empty(1));
-            const int nkb32 = (N + kBiasK - 1) / kBiasK;
-            if (pos < nkb32 * kBiasK) {  // the key padding of the last row is read by the attention kernel: zeros
-                // row0 = index of this shard's first line among all query rows (the swizzle follows the global row)
-                const int kc = (((pos & 31) >> 3) ^ (((row0 + tc.line) >> 1) & 3)) * 8 + (pos & 7);
+                uint32_t tbr[16];  // triangle bias of this position: columns 3C..3C+3, pre-scaled for exp2
+                tmem_ld16(taddr + 3 * C, tbr);
+                tmem_ld_wait();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(slot_empty(1));
+                const int nkb32 = (N + kBiasK - 1) / kBiasK;
+                if (pos < nkb32 * kBiasK) {  // the key padding of the last row is read by the attention kernel: zeros
+                    // row0 = index of this shard's first line among all query rows (the swizzle follows the global row)
+                    const int kc = (((pos & 31) >> 3) ^ (((row0 + tc.line) >> 1) & 3)) * 8 + (pos & 7);
 #pragma unroll
-                for (int h = 0; h < kH; ++h)
-                    tb_out[((((long long)tc.b * kH + h) * nkb32 + (pos >> 5)) * R + tc.line) * kBiasK + kc] =
-                        __float2bfloat16_rn(live ? __uint_as_float(tbr[h]) * kLog2e : 0.f);
+                    for (int h = 0; h < kH; ++h)
+                        tb_out[((((long long)tc.b * kH + h) * nkb32 + (pos >> 5)) * R + tc.line) * kBiasK + kc] =
+                            __float2bfloat16_rn(live ? __uint_as_float(tbr[h]) * kLog2e : 0.f);
+                }
             }
         }
     }
@@ -753,13 +756,16 @@ struct AOutSmem {
     static constexpr uint32_t kParams = kO + 2 * tile_bytes<C>();  // gamma, beta
     static constexpr uint32_t kXch = kParams + 1024;          // 2 groups x 512 floats: LayerNorm partial sums
     static constexpr uint32_t kBars = kXch + 4096;
-    static constexpr uint32_t kTotal = kBars + 160;
+    static constexpr uint32_t kTotal = kBars + 192;
     static constexpr uint32_t kDyn = kTotal + 1024;
 };
 
-// producer, MMA issuer, 2 groups x 8 warps: a group alternates tiles with the other one; inside a group two threads
-// share a row (TMEM lane), each with 64 of its 128 channels through LayerNorm, gating and the output pass
-constexpr int kAOutThreads = 32 * (2 + 2 * 8);
+// Warps: 0 producer, 1 and 2 issue the GEMMs and the stores of the two row groups, then 2 groups x 8 warps: a group alternates
+// tiles with the other one; inside a group two threads share a row (TMEM lane), each with half of its channels through
+// LayerNorm, gating and the output pass. Each group has its own issuer: with one for both a group's output GEMM waited 5500
+// of a tile's 15300 cycles (N = 768) for the other group's next LayerNorm, and a row thread that waited for its TMA store to
+// leave the buffer held its group up for 2000; the issuer has that time, between a tile's last GEMM and the next LayerNorm.
+constexpr int kAOutThreads = 32 * (3 + 2 * 8);
 
 template <int C, bool kTransposed>
 __global__ void __launch_bounds__(kAOutThreads, 1)
@@ -785,8 +791,9 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
     auto g_full = [&](int g) { return bars + 8u * (7 + g); };
     auto a2_ready = [&](int g) { return bars + 8u * (9 + g); };
     auto d_full = [&](int g) { return bars + 8u * (11 + g); };
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 144);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 148);
+    auto out_ready = [&](int g) { return bars + 8u * (17 + g); };   // the group's result lies in the o buffer
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 160);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 164);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_per_line = (N + kRows - 1) / kRows;
@@ -804,6 +811,7 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
             mbar_init(g_full(g), 1);
             mbar_init(a2_ready(g), 8);
             mbar_init(d_full(g), 1);
+            mbar_init(out_ready(g), 8);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -824,7 +832,7 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr;
     grid_trigger();
-    if (warp >= 2) grid_wait();
+    if (warp >= 3) grid_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -854,52 +862,66 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
                     tma_load_3d(odst + kb * kKBlockBytes, &tmO, o_full(g), kb * 64, tc.tile * kRows, tc.b * R + tc.line);
             }
         }
-    } else if (warp == 1) {
+    } else if (warp <= 2) {
+        // ---------------------------------------------------------------- MMA issuer of row group g
         if (lane == 0) {
+            const int g = warp - 1;
             constexpr uint32_t idesc = idesc_bf16_f32(128, C);
             bool ok = mbar_wait(w_full, 0, abort_flag);
             if (!ok) report_wait_failure(status, abort_flag, kKidOut, 2);
-            // gate GEMM of tile lt is issued before the output GEMM of tile lt-1, so the two groups
-            // overlap: one gates its o tile while the other's gate GEMM runs
-            for (long long lt = 0; lt <= my_tiles && ok; ++lt) {
-                if (lt < my_tiles) {
-                    const int g = (int)(lt & 1);
-                    if (!mbar_wait(a1_ready(g), (uint32_t)(lt >> 1) & 1u, abort_flag)) {
-                        report_wait_failure(status, abort_flag, kKidOut, 3);
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    mma_rows<C>(tmem_base + g * 256, sbase + Sm::kZ + g * tile_bytes<C>(), sbase + Sm::kWg, C * 128, idesc,
-                                false);
-                    mma_commit(g_full(g));
-                    mma_commit(z_empty(g));
+            grid_wait();   // (the stores)
+            const uint32_t otile = sbase + Sm::kO + g * tile_bytes<C>();
+            TileWalk tc(blockIdx.x + g * gridDim.x, 2 * gridDim.x, R, tiles_per_line);
+            for (long long lt = g; lt < my_tiles && ok; lt += 2, tc.next()) {
+                const uint32_t par = (uint32_t)(lt >> 1) & 1u;
+                if (!mbar_wait(a1_ready(g), par, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidOut, 3);
+                    break;
                 }
-                if (lt >= 1) {
-                    const long long pt = lt - 1;
-                    const int g = (int)(pt & 1);
-                    if (!mbar_wait(a2_ready(g), (uint32_t)(pt >> 1) & 1u, abort_flag)) {
-                        report_wait_failure(status, abort_flag, kKidOut, 4);
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    mma_rows<C>(tmem_base + g * 256 + 128, sbase + Sm::kO + g * tile_bytes<C>(), sbase + Sm::kWo, C * 128,
-                                idesc, false);
-                    mma_commit(d_full(g));
+                tc_fence_after_sync();
+                mma_rows<C>(tmem_base + g * 256, sbase + Sm::kZ + g * tile_bytes<C>(), sbase + Sm::kWg, C * 128, idesc,
+                            false);
+                mma_commit(g_full(g));
+                mma_commit(z_empty(g));
+                if (!mbar_wait(a2_ready(g), par, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidOut, 4);
+                    break;
                 }
+                tc_fence_after_sync();
+                mma_rows<C>(tmem_base + g * 256 + 128, sbase + Sm::kO + g * tile_bytes<C>(), sbase + Sm::kWo, C * 128,
+                            idesc, false);
+                mma_commit(d_full(g));
+                if (!mbar_wait(out_ready(g), par, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidOut, 10);
+                    break;
+                }
+                for (int kb = 0; kb < C / 64; ++kb) {
+                    if (kTransposed) {
+                        asm volatile(
+                            "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::
+                                "l"(reinterpret_cast<uint64_t>(&tmOut)),
+                            "r"(otile + kb * kKBlockBytes), "r"(kb * 64), "r"(tc.line), "r"(tc.tile * kRows), "r"(tc.b)
+                            : "memory");
+                    } else {
+                        tma_store_3d(&tmOut, otile + kb * kKBlockBytes, kb * 64, tc.tile * kRows, tc.b * R + tc.line);
+                    }
+                }
+                tma_store_commit();
+                tma_store_wait_read<0>();
+                mbar_arrive(o_empty(g));
             }
+            tma_store_wait_all<0>();
         }
     } else {
-        const int g = (warp - 2) >> 3;
+        const int g = (warp - 3) >> 3;
         const int quad = warp & 3;
-        const int half = ((warp - 2) >> 2) & 1;   // half of the row's channels
+        const int half = ((warp - 3) >> 2) & 1;   // half of the row's channels
         const int row = quad * 32 + lane;
-        const int gtid = (warp - 2 - g * 8) * 32 + lane;
         float* xch = reinterpret_cast<float*>(gbase + Sm::kXch) + g * 512;
         const uint32_t ztile = sbase + Sm::kZ + g * tile_bytes<C>();
         const uint32_t otile = sbase + Sm::kO + g * tile_bytes<C>();
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * 256 + half * (C / 2);
-        TileWalk tc(blockIdx.x + g * gridDim.x, 2 * gridDim.x, R, tiles_per_line);
-        for (long long lt = g; lt < my_tiles; lt += 2, tc.next()) {
+        for (long long lt = g; lt < my_tiles; lt += 2) {
             const uint32_t use = (uint32_t)(lt >> 1);
             if (!mbar_wait(z_full(g), use & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidOut, 5);
@@ -979,25 +1001,9 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
             }
             tc_fence_before_sync();
             fence_proxy_async_smem();
-            group_sync(1 + g, 256);
-            if (gtid == 0) {
-                for (int kb = 0; kb < C / 64; ++kb) {
-                    if (kTransposed) {
-                        asm volatile(
-                            "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::
-                                "l"(reinterpret_cast<uint64_t>(&tmOut)),
-                            "r"(otile + kb * kKBlockBytes), "r"(kb * 64), "r"(tc.line), "r"(tc.tile * kRows), "r"(tc.b)
-                            : "memory");
-                    } else {
-                        tma_store_3d(&tmOut, otile + kb * kKBlockBytes, kb * 64, tc.tile * kRows, tc.b * R + tc.line);
-                    }
-                }
-                tma_store_commit();
-                tma_store_wait_read<0>();
-                mbar_arrive(o_empty(g));
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(out_ready(g));
         }
-        if (gtid == 0) tma_store_wait_all<0>();
     }
 
     tc_fence_before_sync();
@@ -1066,7 +1072,8 @@ int project_impl(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __n
     }
     if ((rc = set_attrs<C, kT>())) return rc;
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
-    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+    const int slots = sm_count() * (C == 128 ? 1 : 2);
+    const int grid = (int)(tiles < slots ? tiles : slots);
     typedef const __nv_bfloat16* P;
     LaunchScope scope(kKidProj, st);
     OF3_CUDA_CHECK(launch_chained(triattn_proj_kernel<C, kT>, grid, kProjThreads, ProjSmem<C>::kDyn, st, tmZ, tmW[0],
@@ -1129,6 +1136,7 @@ int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, 
                     __nv_bfloat16* tb, int B, int R, int N, int row0, bool transposed,
                     const of3_triattn_params* p, cudaStream_t st, int C) {
     OF3_REQUIRE(((uintptr_t)z & 15) == 0, OF3_ERR_ALIGN, "triattn: z must be 16-byte aligned");
+    OF3_REQUIRE((((uintptr_t)q | (uintptr_t)k) & 31) == 0, OF3_ERR_ALIGN, "triattn: q / k images must be 32-byte aligned");
     OF3_REQUIRE(!transposed || R == N, OF3_ERR_SHAPE, "triattn: transposed view needs the whole tensor");
     if (C == 128)
         return transposed ? project_impl<128, true>(z, q, k, vt, tb, B, R, N, row0, p, st)

@@ -548,14 +548,20 @@ struct OutSmem {
     static constexpr uint32_t kZ = 2 * kWBytes;                    // 2 groups: z tile, then output
     static constexpr uint32_t kX = kZ + 2 * tile_bytes<C>();       // 2 groups: x tile [c][j], then A
     static constexpr uint32_t kParams = kX + 2 * tile_bytes<C>();  // gamma_in, beta_in, gamma_out, beta_out
-    static constexpr uint32_t kBars = kParams + 4 * 512;
-    static constexpr uint32_t kTotal = kBars + 128;
+    static constexpr uint32_t kXch = kParams + 4 * 512;            // 2 groups x 512 floats: LayerNorm partial sums
+    static constexpr uint32_t kBars = kXch + 4096;
+    static constexpr uint32_t kTotal = kBars + 160;
     static constexpr uint32_t kDyn = kTotal + 1024;
 };
 
-// 64 channels: half the registers, tiles and tensor memory, so two CTAs share an SM (four tiles in flight)
+// Warps: 0 producer, 1 and 2 issue the GEMMs and the stores of the two row groups, then 2 groups x 8 warps, which alternate
+// tiles; two threads share a row, each with half of its channels. (One thread per row took 3400 + 4300 cycles for the two
+// LayerNorms and 3900 for the output of a tile's 17400 at N = 768: latency, with one warp of a group per scheduler; and the
+// row thread that waited for the store to leave its buffer another 1500.)
+constexpr int kOutThreads = 32 * (3 + 2 * 8);
+
 template <int C>
-__global__ void __launch_bounds__(320, C == 128 ? 1 : 2)
+__global__ void __launch_bounds__(kOutThreads, 1)
 trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmX,
                   const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ CUtensorMap tmWg,
                   const __grid_constant__ CUtensorMap tmWz, const __nv_bfloat16* __restrict__ ln_in_w,
@@ -564,6 +570,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                   int* status) {
     using Sm = OutSmem<C>;
     constexpr int kTm = 2 * C;   // tensor-memory columns of a group: gate, update
+    constexpr int CH = C / 2;   // channels per thread
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
@@ -580,8 +587,9 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     auto d_full = [&](int g) { return bars + 8u * (7 + g); };   // MMAs of the group's tile done
     auto z_full = [&](int g) { return bars + 8u * (9 + g); };   // TMA landed: z tile
     auto x_empty = [&](int g) { return bars + 8u * (11 + g); };  // MMAs have read the x buffer
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 112);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 116);
+    auto out_ready = [&](int g) { return bars + 8u * (13 + g); };  // the group's result lies in the z buffer
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 128);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 132);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_per_line = (N + kRows - 1) / kRows;
@@ -596,8 +604,9 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
             mbar_init(z_full(g), 1);
             mbar_init(x_empty(g), 1);
             mbar_init(z_empty(g), 1);
-            mbar_init(a_ready(g), 4);
+            mbar_init(a_ready(g), 8);
             mbar_init(d_full(g), 1);
+            mbar_init(out_ready(g), 8);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -620,7 +629,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr;
     grid_trigger();
-    if (warp >= 2) grid_wait();
+    if (warp >= 1) grid_wait();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -653,71 +662,81 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                     tma_load_3d(zdst + kb * kKBlockBytes, &tmZ, z_full(g), kb * 64, t0, tw.b * R + tw.line);
             }
         }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer
+    } else if (warp <= 2) {
+        // ---------------------------------------------------------------- GEMMs and stores of row group g
         if (lane == 0) {
+            const int g = warp - 1;
             constexpr uint32_t idesc = idesc_bf16_f32(128, C);
+            const uint32_t ztile = sbase + Sm::kZ + g * tile_bytes<C>();
             bool ok = mbar_wait(w_full, 0, abort_flag);
             if (!ok) report_wait_failure(status, abort_flag, kKidOut, 2);
-            for (long long lt = 0; lt < my_tiles && ok; ++lt) {
-                const int g = (int)(lt & 1);
-                const uint32_t use = (uint32_t)(lt >> 1);
-                if (!mbar_wait(a_ready(g), use & 1u, abort_flag)) {
+            TileWalk tw(blockIdx.x + g * gridDim.x, 2 * gridDim.x, R, tiles_per_line);
+            for (long long lt = g; lt < my_tiles && ok; lt += 2, tw.next()) {
+                const uint32_t par = (uint32_t)(lt >> 1) & 1u;
+                if (!mbar_wait(a_ready(g), par, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidOut, 3);
                     break;
                 }
                 tc_fence_after_sync();
                 // gate = LN_in(z) W_g^T -> columns [0,C); update = LN_out(x) W_z^T -> [C,2C)
-                mma_rows<C>(tmem_base + g * kTm, sbase + Sm::kZ + g * tile_bytes<C>(), sbase + Sm::kWg, C * 128, idesc,
-                            false);
+                mma_rows<C>(tmem_base + g * kTm, ztile, sbase + Sm::kWg, C * 128, idesc, false);
                 mma_rows<C>(tmem_base + g * kTm + C, sbase + Sm::kX + g * tile_bytes<C>(), sbase + Sm::kWz, C * 128, idesc,
                             false);
                 mma_commit(d_full(g));
                 mma_commit(x_empty(g));
+                if (!mbar_wait(out_ready(g), par, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidOut, 8);
+                    break;
+                }
+                for (int kb = 0; kb < C / 64; ++kb)
+                    tma_store_3d(&tmOut, ztile + kb * kKBlockBytes, kb * 64, tw.tile * kRows, tw.b * R + tw.line);
+                tma_store_commit();
+                tma_store_wait_read<0>();
+                mbar_arrive(z_empty(g));
             }
+            tma_store_wait_all<0>();
         }
     } else {
-        // ---------------------------------------------------------------- two row groups (warps 2..5, 6..9)
-        const int g = (warp - 2) >> 2;
+        // ---------------------------------------------------------------- two row groups
+        const int g = (warp - 3) >> 3;
         const int quad = warp & 3;
+        const int half = ((warp - 3) >> 2) & 1;   // which half of the row's channels
         const int row = quad * 32 + lane;
-        const int gtid = (warp - 2 - g * 4) * 32 + lane;  // 0..127 inside the group
         const uint32_t ztile = sbase + Sm::kZ + g * tile_bytes<C>();
         const uint32_t xtile = sbase + Sm::kX + g * tile_bytes<C>();
-        TileWalk tw(blockIdx.x + g * gridDim.x, 2 * gridDim.x, R, tiles_per_line);
-        for (long long lt = g; lt < my_tiles; lt += 2, tw.next()) {
+        float* xch = reinterpret_cast<float*>(gbase + Sm::kXch) + g * 512;
+        for (long long lt = g; lt < my_tiles; lt += 2) {
             const uint32_t use = (uint32_t)(lt >> 1);
-            const int t0 = tw.tile * kRows;
             if (!mbar_wait(x_full(g), use & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidOut, 4);
                 break;
             }
             float mean, rstd;
-            // --- x column of this position: C channels, [c][j] layout, stride 256 B
+            // --- half of the x column of this position: [c][j] layout, stride 256 B
             {
-                uint32_t xraw[C / 2];
-                const uint32_t col = xtile + row * 2;
+                uint32_t xraw[CH / 2];
+                const uint32_t col = xtile + row * 2 + half * (CH * 256);
 #pragma unroll
-                for (int i = 0; i < C / 2; ++i) {
+                for (int i = 0; i < CH / 2; ++i) {
                     uint32_t lo, hi;
                     if ((i & 7) == 0) asm volatile("" ::: "memory");  // cap the loads in flight per batch
                     asm volatile("ld.shared.u16 %0, [%1];" : "=r"(lo) : "r"(col + (2 * i) * 256));
                     asm volatile("ld.shared.u16 %0, [%1];" : "=r"(hi) : "r"(col + (2 * i + 1) * 256));
                     xraw[i] = lo | (hi << 16);
                 }
-                row_stats<C>(xraw, mean, rstd);
-                group_sync(1 + g, 128);  // everyone has read its column before rows overwrite the buffer
-                store_normalized_row<C>(xtile, row, xraw, mean, rstd, prm + 256, prm + 384);
+                // (behind its first barrier everyone has read its column: rows may overwrite the buffer)
+                half_row_stats_xwarp<C>(xraw, row, half, xch, 1 + g, 256, mean, rstd);
+                store_normalized_half_row<C>(xtile, row, half, xraw, mean, rstd, prm + 256, prm + 384);
             }
             // --- z row: keep the raw values for the residual, normalise in place (A operand 1)
             if (!mbar_wait(z_full(g), use & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidOut, 7);
                 break;
             }
-            uint32_t zraw[C / 2];
-            load_row<C>(ztile, row, zraw);
-            row_stats<C>(zraw, mean, rstd);
-            store_normalized_row<C>(ztile, row, zraw, mean, rstd, prm, prm + 128);
+            uint32_t zraw[CH / 2];
+            load_half_row<C>(ztile, row, half, zraw);
+            half_row_stats_xwarp<C>(zraw, row, half, xch, 1 + g, 256, mean, rstd);
+            store_normalized_half_row<C>(ztile, row, half, zraw, mean, rstd, prm, prm + 128);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(a_ready(g));
@@ -727,9 +746,9 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                 break;
             }
             tc_fence_after_sync();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * kTm;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + g * kTm + half * CH;
 #pragma unroll
-            for (int cb = 0; cb < C / 16; ++cb) {  // 16 channels per step
+            for (int cb = 0; cb < CH / 16; ++cb) {  // 16 channels per step
                 uint32_t gate[16], upd[16];
                 tmem_ld16(taddr + cb * 16, gate);
                 tmem_ld16(taddr + C + cb * 16, upd);
@@ -749,21 +768,14 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                         }
                         o[j] = pack_bf16x2(v0, v1);
                     }
-                    sts128(chunk_addr(ztile, row, cb * 2 + ch), make_uint4(o[0], o[1], o[2], o[3]));
+                    sts128(chunk_addr(ztile, row, half * (CH / 8) + cb * 2 + ch), make_uint4(o[0], o[1], o[2], o[3]));
                 }
             }
             tc_fence_before_sync();
             fence_proxy_async_smem();
-            group_sync(1 + g, 128);
-            if (gtid == 0) {
-                for (int kb = 0; kb < C / 64; ++kb)
-                    tma_store_3d(&tmOut, ztile + kb * kKBlockBytes, kb * 64, t0, tw.b * R + tw.line);
-                tma_store_commit();
-                tma_store_wait_read<0>();
-                mbar_arrive(z_empty(g));
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(out_ready(g));
         }
-        if (gtid == 0) tma_store_wait_all<0>();
     }
 
     tc_fence_before_sync();
@@ -833,7 +845,7 @@ int launch_out(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensor
     }
     typedef const __nv_bfloat16* P;
     LaunchScope scope(kKidOut, st);
-    OF3_CUDA_CHECK(launch_chained(trimul_out_kernel<C>, grid, 320, OutSmem<C>::kDyn, st, tmZ, tmX, tmOut, tmWg, tmWz,
+    OF3_CUDA_CHECK(launch_chained(trimul_out_kernel<C>, grid, kOutThreads, OutSmem<C>::kDyn, st, tmZ, tmX, tmOut, tmWg, tmWz,
                                   (P)p->ln_in_w, (P)p->ln_in_b, (P)p->ln_out_w, (P)p->ln_out_b, B, R, N, add_residual,
                                   device_status_ptr()));
     return OF3_OK;
@@ -927,8 +939,7 @@ int trimul_output(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat1
     if ((rc = weight_tmap(&tmWg, p->w_g, C))) return rc;
     if ((rc = weight_tmap(&tmWz, p->w_z, C))) return rc;
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
-    const int ctas = sm_count() * (C == 128 ? 1 : 2);
-    const int grid = (int)(tiles < ctas ? tiles : ctas);
+    const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     return C == 128 ? launch_out<128>(grid, st, tmZ, tmX, tmOut, tmWg, tmWz, p, B, R, N, add_residual)
                     : launch_out<64>(grid, st, tmZ, tmX, tmOut, tmWg, tmWz, p, B, R, N, add_residual);
 }
