@@ -5,9 +5,8 @@
 //   h  = silu(a) * b  -> bf16 -> shared memory as the next A operand (never leaves the SM)
 //   G2: y += h W_out[:, chunk]^T         (128x128x64, accumulated over the 8 chunks in TMEM)
 // then out = x + mask * y, TMA-stored. The 512-wide hidden activation (604 MB at N = 768 in the
-// reference's unfused path) never touches HBM. Two 128-row groups ping-pong on the tensor pipe
-// and share every weight chunk (streamed from L2 by TMA, double-buffered), which halves the
-// weight traffic per row.
+// reference's unfused path) never touches HBM. Two row groups of 128 rows share every weight chunk (streamed from L2
+// by TMA, double-buffered), which halves the weight traffic per row.
 // Reference: openfold3/core/model/layers/transition.py:225-271,
 //            openfold3/core/model/primitives/activations.py:33-61.
 #include "modules.cuh"
@@ -27,30 +26,64 @@ constexpr int kChunk = 64;
 constexpr int kNumChunks = kHidden / kChunk;  // 8
 
 
+// v[0..3]: partial sums of 4 rows, spread over the 16 lanes of a half warp -> the rows' sums, in every lane. The first
+// steps of the tree send the rows that the lane does not go on with: 3 + 2 + 4 shuffles instead of 4 x 4.
+__device__ __forceinline__ void row_sums(float (&v)[4], int lane) {
+#pragma unroll
+    for (int w = 2; w >= 1; w >>= 1) {   // w rows kept; the partner is 4 w lanes away
+        const bool up = lane & (4 * w);
+#pragma unroll
+        for (int r = 0; r < w; ++r) {
+            const float keep = up ? v[r + w] : v[r], send = up ? v[r] : v[r + w];
+            v[r] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * w);
+        }
+    }
+    float sum = v[0];   // of row (lane & 12) >> 2
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = __shfl_sync(0xffffffffu, sum, (lane & 16) + 4 * r);
+}
+
+// Keeps the compiler from carrying values computed from v[first .. first + 15] over this point.
+__device__ __forceinline__ void opaque(uint32_t (&v)[32], int first) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(v[first + i]));
+}
+
 struct TrSmem {
     static constexpr uint32_t kWStage = 49152;                 // [Wa|Wb] slab 32 KB + Wout chunk 16 KB
     static constexpr uint32_t kW = 0;                          // 2 stages
-    static constexpr uint32_t kX = 2 * kWStage;                // 2 groups x 32 KB (x tile / A / output)
-    static constexpr uint32_t kH = kX + 2 * kTileBytes;        // 2 groups x 16 KB
+    static constexpr uint32_t kX = 2 * kWStage;                // 3 x 32 KB (x tile / LN(x) / x again / output)
+    static constexpr uint32_t kH = kX + 3 * kTileBytes;        // 2 groups x 16 KB
     static constexpr uint32_t kParams = kH + 2 * kKBlockBytes; // gamma, beta
-    static constexpr uint32_t kXch = kParams + 1024;           // 2 groups x 512 floats: LayerNorm partial sums
-    static constexpr uint32_t kBars = kXch + 4096;
+    static constexpr uint32_t kBars = kParams + 1024;
     static constexpr uint32_t kTotal = kBars + 256;
     static constexpr uint32_t kDyn = kTotal + 1024;
 };
 
-// warps: 0 producer, 1 and 2 the MMA issuers of row group 0 and 1, 3..10 and 11..18 the two row groups: two
-// threads share a row (TMEM lane) and take half of its channels each through LayerNorm, half of every hidden chunk
-// through silu * mul, and half of the output row -- the per-row chains were the longest thing in the kernel.
-// One issuing thread for both groups was the critical path (in-kernel clock64 phases: 5000 cycles per hidden
-// chunk for 1536 cycles of tensor work -- it waited for one group's silu pass while the other group's next
-// GEMM was ready to go); each group now has its own issuer and the tensor pipe interleaves the two chains.
-constexpr int kTrThreads = 32 * (3 + 2 * 8);
+// warps: 0 weight producer, 1 and 2 the MMA issuers of row group 0 and 1, 3 the results' stores, 4..11 LayerNorm,
+// 12..19 and 20..27 the two row groups: two threads share a row (TMEM lane) and take half of every hidden chunk through
+// silu * mul, and half of the output row each.
+//
+// The tensor work of a tile is 6100 cycles; what kept a pair of tiles at 34400 (in-kernel clock phases at N = 768) was
+// what both groups did between two tiles at the same time, with the tensor pipe idle: store 2100, wait for the next x
+// 2600, LayerNorm 5300, output 1200. So the tiles are prepared ahead, by warps of their own: these hold the next tile,
+// normalised, in registers until one of the three x buffers is free (the CTA's tile t uses buffer t mod 3). The residual
+// is fetched once more from L2 into the buffer that the last G1 has released instead of staying in 32 registers of
+// every row thread.
+// What is left is near the shared memory's limit: a 128 x 128 x 16 MMA reads 8 KB in its 64 cycles, which is all that
+// the memory gives, and the weights, LN(x), h and the result are written beside it.
+// Both groups take the chunks in the same order, so that a row's result does not depend on where in the tensor it lies
+// (half a tile apart, with the cyclic sequence entered where it is, they would never wait for a buffer: 234 us instead
+// of 250). N = 768: 316 -> 250 us, N = 37: 25.8 -> 20.9.
+constexpr int kTrThreads = 32 * 28;
 
 __global__ void __launch_bounds__(kTrThreads, 1)
 transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmOut,
                   const __grid_constant__ CUtensorMap tmWa, const __grid_constant__ CUtensorMap tmWb,
-                  const __grid_constant__ CUtensorMap tmWo, const __nv_bfloat16* __restrict__ mask,
+                  const __grid_constant__ CUtensorMap tmWo, const __nv_bfloat16* x,   // x may be the output
+                  const __nv_bfloat16* __restrict__ mask,
                   const __nv_bfloat16* __restrict__ ln_w, const __nv_bfloat16* __restrict__ ln_b,
                   long long rows, int add_residual, int* status) {
     extern __shared__ uint8_t smem_raw[];
@@ -60,24 +93,25 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     const uint32_t bars = sbase + TrSmem::kBars;
     auto w_full = [&](int s) { return bars + 8u * (0 + s); };
     auto w_empty = [&](int s) { return bars + 8u * (2 + s); };
-    auto x_full = [&](int g) { return bars + 8u * (4 + g); };
-    auto x_empty = [&](int g) { return bars + 8u * (6 + g); };
-    auto a_ready = [&](int g) { return bars + 8u * (8 + g); };
-    auto d1_full = [&](int g) { return bars + 8u * (10 + g); };
-    auto d1_empty = [&](int g) { return bars + 8u * (12 + g); };
-    auto h_ready = [&](int g) { return bars + 8u * (14 + g); };
-    auto h_free = [&](int g) { return bars + 8u * (16 + g); };
-    auto d2_full = [&](int g) { return bars + 8u * (18 + g); };
-    auto d2_empty = [&](int g) { return bars + 8u * (20 + g); };
-    auto wo_full = [&](int s) { return bars + 8u * (22 + s); };   // W_out chunk of a weight stage (its own ring:
-    auto wo_empty = [&](int s) { return bars + 8u * (24 + s); };  // the slab is free long before the chunk's 2nd GEMM)
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + TrSmem::kBars + 224);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + TrSmem::kBars + 232);
+    auto wo_full = [&](int s) { return bars + 8u * (4 + s); };    // W_out chunk of a weight stage (its own ring:
+    auto wo_empty = [&](int s) { return bars + 8u * (6 + s); };   // the slab is free long before the chunk's 2nd GEMM)
+    auto a_ready = [&](int b) { return bars + 8u * (8 + b); };
+    auto x_empty = [&](int b) { return bars + 8u * (11 + b); };
+    auto d1_full = [&](int g) { return bars + 8u * (14 + g); };
+    auto d1_empty = [&](int g) { return bars + 8u * (16 + g); };
+    auto h_ready = [&](int g) { return bars + 8u * (18 + g); };
+    auto h_free = [&](int g) { return bars + 8u * (20 + g); };
+    auto d2_full = [&](int g) { return bars + 8u * (22 + g); };
+    auto d2_empty = [&](int g) { return bars + 8u * (24 + g); };
+    auto res_full = [&](int g) { return bars + 8u * (26 + g); };   // x is back in the tile's buffer
+    auto out_ready = [&](int g) { return bars + 8u * (28 + g); };  // the group's result lies in the tile's buffer
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + TrSmem::kBars + 240);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + TrSmem::kBars + 248);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long num_tiles = (rows + kRows - 1) / kRows;
-    const long long my_tiles = tiles_of_block(num_tiles);
-    const long long my_pairs = (my_tiles + 1) / 2;
+    const int my_tiles = (int)tiles_of_block((rows + kRows - 1) / kRows);
+    // group g's tiles are the CTA's tiles g, g + 2, ...
+    const int num_chunks = ((my_tiles + 1) >> 1) * kNumChunks;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) {
@@ -85,15 +119,18 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             mbar_init(w_empty(i), 2);  // both groups' issuers have consumed the [W_a|W_b] slab
             mbar_init(wo_full(i), 1);
             mbar_init(wo_empty(i), 2);
-            mbar_init(x_full(i), 1);
-            mbar_init(x_empty(i), 1);
-            mbar_init(a_ready(i), 8);
             mbar_init(d1_full(i), 1);
             mbar_init(d1_empty(i), 8);
             mbar_init(h_ready(i), 8);
             mbar_init(h_free(i), 1);
             mbar_init(d2_full(i), 1);
             mbar_init(d2_empty(i), 8);
+            mbar_init(res_full(i), 1);
+            mbar_init(out_ready(i), 8);
+        }
+        for (int i = 0; i < 3; ++i) {
+            mbar_init(x_empty(i), 1);
+            mbar_init(a_ready(i), 8);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -119,48 +156,36 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     // TMEM columns: group g -> D1 at g*256 + [0,128) ([a 64 | b 64]), D2 at g*256 + [128,256)
 
     if (warp == 0) {
-        // ---------------------------------------------------------------- TMA producer
+        // ---------------------------------------------------------------- weight producer
         if (lane == 0) {
-            uint32_t wi = 0;
             bool ok = true;
-            for (long long pi = 0; pi < my_pairs && ok; ++pi) {
-                for (int g = 0; g < 2; ++g) {
-                    const long long lt = pi * 2 + g;
-                    if (lt >= my_tiles) break;
-                    if (!mbar_wait(x_empty(g), ((uint32_t)pi & 1u) ^ 1u, abort_flag)) {
-                        report_wait_failure(status, abort_flag, kKidTrans, 1);
-                        ok = false;
-                        break;
-                    }
-                    const long long tile = blockIdx.x + lt * gridDim.x;
-                    mbar_arrive_expect_tx(x_full(g), kTileBytes);
-                    const uint32_t dst = sbase + TrSmem::kX + g * kTileBytes;
-                    // rows can exceed 2^31 only beyond any realistic N; tile*128 fits in int for N <= 46340
-                    tma_load_2d(dst, &tmX, x_full(g), 0, (int)(tile * kRows));
-                    tma_load_2d(dst + kKBlockBytes, &tmX, x_full(g), 64, (int)(tile * kRows));
+            auto load_slab = [&](int wi) -> bool {
+                const int s = wi & 1, c = wi & (kNumChunks - 1);
+                if (!mbar_wait(w_empty(s), ((uint32_t)(wi >> 1) & 1u) ^ 1u, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidTrans, 2);
+                    return false;
                 }
-                for (int c = 0; c < kNumChunks && ok; ++c, ++wi) {
-                    const int s = wi & 1;
-                    if (!mbar_wait(w_empty(s), ((wi >> 1) & 1u) ^ 1u, abort_flag)) {
-                        report_wait_failure(status, abort_flag, kKidTrans, 2);
-                        ok = false;
-                        break;
-                    }
-                    mbar_arrive_expect_tx(w_full(s), 2 * kKBlockBytes);
-                    const uint32_t w = sbase + TrSmem::kW + s * TrSmem::kWStage;
-                    for (int kb = 0; kb < 2; ++kb) {
-                        // slab k-block kb: rows [0,64) = W_a chunk, rows [64,128) = W_b chunk
-                        tma_load_2d(w + kb * kKBlockBytes, &tmWa, w_full(s), kb * 64, c * kChunk);
-                        tma_load_2d(w + kb * kKBlockBytes + 64 * 128, &tmWb, w_full(s), kb * 64, c * kChunk);
-                    }
-                    if (!mbar_wait(wo_empty(s), ((wi >> 1) & 1u) ^ 1u, abort_flag)) {
-                        report_wait_failure(status, abort_flag, kKidTrans, 12);
-                        ok = false;
-                        break;
-                    }
-                    mbar_arrive_expect_tx(wo_full(s), kKBlockBytes);
-                    tma_load_2d(w + 2 * kKBlockBytes, &tmWo, wo_full(s), c * kChunk, 0);
+                mbar_arrive_expect_tx(w_full(s), 2 * kKBlockBytes);
+                const uint32_t w = sbase + TrSmem::kW + s * TrSmem::kWStage;
+                for (int kb = 0; kb < 2; ++kb) {
+                    // slab k-block kb: rows [0,64) = W_a chunk, rows [64,128) = W_b chunk
+                    tma_load_2d(w + kb * kKBlockBytes, &tmWa, w_full(s), kb * 64, c * kChunk);
+                    tma_load_2d(w + kb * kKBlockBytes + 64 * 128, &tmWb, w_full(s), kb * 64, c * kChunk);
                 }
+                return true;
+            };
+            ok = load_slab(0);
+            for (int wi = 0; wi < num_chunks && ok; ++wi) {
+                // a slab's stage is released by the G1 two chunks before, and that comes before the G2 which releases
+                // this chunk's W_out stage
+                if (wi + 1 < num_chunks && !load_slab(wi + 1)) break;
+                const int s = wi & 1, c = wi & (kNumChunks - 1);
+                if (!mbar_wait(wo_empty(s), ((uint32_t)(wi >> 1) & 1u) ^ 1u, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidTrans, 12);
+                    break;
+                }
+                mbar_arrive_expect_tx(wo_full(s), kKBlockBytes);
+                tma_load_2d(sbase + TrSmem::kW + s * TrSmem::kWStage + 2 * kKBlockBytes, &tmWo, wo_full(s), c * kChunk, 0);
             }
         }
     } else if (warp <= 2) {
@@ -168,92 +193,189 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         if (lane == 0) {
             const int g = warp - 1;
             constexpr uint32_t idesc = idesc_bf16_f32(128, 128);
-            uint32_t wi = 0;
             bool ok = true;
             auto fail = [&](int site) {
                 report_wait_failure(status, abort_flag, kKidTrans, site);
                 ok = false;
             };
-            // Software-pipelined per tile: G1 of chunk c+1 is issued as soon as the row group has read D1 of
-            // chunk c, BEFORE waiting for that chunk's silu pass and its G2, so the row group finds its next
-            // accumulator ready when it comes back (the serial G2 -> weights -> G1 hop cost ~1900 cycles per chunk).
-            auto issue_g1 = [&](uint32_t widx, uint32_t c) -> bool {
-                const int s = widx & 1;
-                if (!mbar_wait(w_full(s), (widx >> 1) & 1u, abort_flag)) { fail(3); return false; }
-                if (!mbar_wait(d1_empty(g), (c & 1u) ^ 1u, abort_flag)) { fail(5); return false; }
+            auto skip_chunk = [&](int wi) {   // the other group's alone: keep both weight rings moving
+                const int s = wi & 1;
+                const uint32_t par = (uint32_t)(wi >> 1) & 1u;
+                if (!mbar_wait(w_full(s), par, abort_flag)) return fail(3);
+                mbar_arrive(w_empty(s));
+                if (!mbar_wait(wo_full(s), par, abort_flag)) return fail(13);
+                mbar_arrive(wo_empty(s));
+            };
+            // Software-pipelined: G1 of chunk i + 1 is issued as soon as the row group has read D1 of chunk i, BEFORE
+            // waiting for that chunk's silu pass and its G2, so the row group finds its next accumulator ready when it
+            // comes back; across the tiles' boundary too, if the next tile's LN(x) is there by then.
+            int t = g, buf = g;   // the CTA's tile that G1 is at, and its x buffer (t mod 3)
+            uint32_t use = 0;     // t / 3: how often the buffer has been used before
+            auto issue_g1 = [&](int i) -> bool {   // i: chunk, counted over the group's tiles
+                const int s = i & 1, c = i & (kNumChunks - 1);
+                if (c == 0 && !mbar_wait(a_ready(buf), use & 1u, abort_flag)) { fail(4); return false; }
+                if (!mbar_wait(w_full(s), (uint32_t)(i >> 1) & 1u, abort_flag)) { fail(3); return false; }
+                if (!mbar_wait(d1_empty(g), ((uint32_t)i & 1u) ^ 1u, abort_flag)) { fail(5); return false; }
                 tc_fence_after_sync();
-                mma_k128(tmem_base + g * 256, sbase + TrSmem::kX + g * kTileBytes,
+                mma_k128(tmem_base + g * 256, sbase + TrSmem::kX + buf * kTileBytes,
                          sbase + TrSmem::kW + s * TrSmem::kWStage, kKBlockBytes, idesc, false);
                 mma_commit(d1_full(g));
                 mma_commit(w_empty(s));
                 return true;
             };
-            for (long long pi = 0; pi < my_pairs && ok; ++pi) {
-                const bool have_tile = pi * 2 + g < my_tiles;  // the last pair may hold one tile only
-                const uint32_t ppar = (uint32_t)pi & 1u;
-                if (!have_tile) {  // keep both weight rings moving
-                    for (int c = 0; c < kNumChunks && ok; ++c, ++wi) {
-                        const int s = wi & 1;
-                        if (!mbar_wait(w_full(s), (wi >> 1) & 1u, abort_flag)) { fail(3); break; }
-                        mbar_arrive(w_empty(s));
-                        if (!mbar_wait(wo_full(s), (wi >> 1) & 1u, abort_flag)) { fail(13); break; }
-                        mbar_arrive(wo_empty(s));
+            const int n = ((my_tiles + 1 - g) >> 1) * kNumChunks;
+            if (ok && n > 0) ok = issue_g1(0);
+            for (int i = 0; i < n && ok; ++i) {
+                const int s = i & 1, c = i & (kNumChunks - 1);
+                bool late = false;    // the next tile's LN(x) is not there yet: its first G1 does not hold up this tile's last G2
+                if (c == kNumChunks - 1) {
+                    // the last G1 has read LN(x): fetch x once more (from L2) for the residual, under the silu pass
+                    if (!mbar_wait(d1_full(g), (uint32_t)i & 1u, abort_flag)) { fail(15); break; }
+                    if (add_residual) {
+                        const uint32_t xtile = sbase + TrSmem::kX + buf * kTileBytes;
+                        const int row0 = (int)((blockIdx.x + (long long)t * gridDim.x) * kRows);
+                        mbar_arrive_expect_tx(res_full(g), kTileBytes);
+                        tma_load_2d(xtile, &tmX, res_full(g), 0, row0);
+                        tma_load_2d(xtile + kKBlockBytes, &tmX, res_full(g), 64, row0);
+                    } else {
+                        mbar_arrive(res_full(g));
                     }
-                    continue;
+                    t += 2;
+                    buf += 2;
+                    if (buf >= 3) { buf -= 3; ++use; }
+                    late = i + 1 < n && !mbar_try_wait(a_ready(buf), use & 1u);
                 }
-                if (!mbar_wait(a_ready(g), ppar, abort_flag)) { fail(4); break; }
-                if (!issue_g1(wi, 0)) break;
-                for (int c = 0; c < kNumChunks && ok; ++c, ++wi) {
-                    const int s = wi & 1;
-                    const uint32_t cpar = (uint32_t)c & 1u;  // 8 chunks per tile: chunk parity is global
-                    if (c + 1 < kNumChunks && !issue_g1(wi + 1, c + 1)) break;
-                    if (c == 0 && !mbar_wait(d2_empty(g), ppar ^ 1u, abort_flag)) { fail(6); break; }
-                    if (!mbar_wait(wo_full(s), (wi >> 1) & 1u, abort_flag)) { fail(13); break; }
-                    if (!mbar_wait(h_ready(g), cpar, abort_flag)) { fail(7); break; }
-                    tc_fence_after_sync();
-                    const uint64_t ad = smem_desc_k_sw128(sbase + TrSmem::kH + g * kKBlockBytes);
-                    const uint64_t bd = smem_desc_k_sw128(sbase + TrSmem::kW + s * TrSmem::kWStage + 2 * kKBlockBytes);
+                if (i + 1 < n && !late && !issue_g1(i + 1)) break;
+                if (c == 0 && !mbar_wait(d2_empty(g), ((uint32_t)(i / kNumChunks) & 1u) ^ 1u, abort_flag)) { fail(6); break; }
+                if (!mbar_wait(wo_full(s), (uint32_t)(i >> 1) & 1u, abort_flag)) { fail(13); break; }
+                if (!mbar_wait(h_ready(g), (uint32_t)i & 1u, abort_flag)) { fail(7); break; }
+                tc_fence_after_sync();
+                const uint64_t ad = smem_desc_k_sw128(sbase + TrSmem::kH + g * kKBlockBytes);
+                const uint64_t bd = smem_desc_k_sw128(sbase + TrSmem::kW + s * TrSmem::kWStage + 2 * kKBlockBytes);
 #pragma unroll
-                    for (int k4 = 0; k4 < 4; ++k4)
-                        mma_bf16(tmem_base + g * 256 + 128, ad + 2u * k4, bd + 2u * k4, idesc,
-                                 (c != 0 || k4 != 0) ? 1u : 0u);
-                    mma_commit(h_free(g));
-                    if (c == kNumChunks - 1) mma_commit(d2_full(g));
-                    mma_commit(wo_empty(s));
+                for (int k4 = 0; k4 < 4; ++k4)
+                    mma_bf16(tmem_base + g * 256 + 128, ad + 2u * k4, bd + 2u * k4, idesc, (c != 0 || k4 != 0) ? 1u : 0u);
+                mma_commit(h_free(g));
+                if (c == kNumChunks - 1) mma_commit(d2_full(g));
+                mma_commit(wo_empty(s));
+                if (late && !issue_g1(i + 1)) break;
+            }
+            for (int i = n; i < num_chunks && ok; ++i) skip_chunk(i);
+        }
+    } else if (warp == 3) {
+        // ---------------------------------------------------------------- results out
+        if (lane == 0) {
+            uint32_t buf = 0;
+            for (int t = 0; t < my_tiles; ++t) {
+                if (!mbar_wait(out_ready(t & 1), (uint32_t)(t >> 1) & 1u, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidTrans, 14);
+                    break;
+                }
+                const uint32_t xtile = sbase + TrSmem::kX + buf * kTileBytes;
+                const int row0 = (int)((blockIdx.x + (long long)t * gridDim.x) * kRows);
+                tma_store_3d(&tmOut, xtile, 0, row0, 0);
+                tma_store_3d(&tmOut, xtile + kKBlockBytes, 64, row0, 0);
+                tma_store_commit();
+                if (t + 3 < my_tiles) {
+                    tma_store_wait_read<0>();
+                    mbar_arrive(x_empty(buf));
+                }
+                if (++buf == 3) buf = 0;
+            }
+            tma_store_wait_all<0>();
+        }
+    } else if (warp < 12) {
+        // ---------------------------------------------------------------- LayerNorm: 16 rows per warp and tile
+        // A half warp reads a row (coalesced), so that a thread holds 8 channels of 8 rows; see row_sums.
+        const int ch = lane & 15, sub = lane >> 4;
+        const int row0 = (warp - 4) * 16 + sub;
+        uint32_t buf = 0, use = 0;
+        for (int t = 0; t < my_tiles; ++t) {
+            const uint32_t xtile = sbase + TrSmem::kX + buf * kTileBytes;
+            const long long base = (blockIdx.x + (long long)t * gridDim.x) * kRows + row0;
+            const __nv_bfloat16* src = x + base * kC + ch * 8;
+            const int left = (int)min(rows - base, 16LL);   // rows 0, 2, ... 14 from here; the tensor may end before
+            uint32_t raw[32];
+#pragma unroll
+            for (int h = 0; h < 8; h += 4) {   // four rows at a time (registers)
+                float mean[4], rstd[4];
+                asm volatile("" ::: "memory");
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                    if (2 * (h + r) < left) v = *reinterpret_cast<const uint4*>(src + 2 * (h + r) * kC);
+                    uint32_t* o = &raw[(h + r) * 4];
+                    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    float a = 0.f, b = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { a += bf16lo(raw[(h + r) * 4 + i]); b += bf16hi(raw[(h + r) * 4 + i]); }
+                    mean[r] = a + b;
+                }
+                row_sums(mean, lane);
+                opaque(raw, h * 4);   // unpack again rather than keep 32 floats
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    mean[r] *= 1.0f / kC;
+                    float a = 0.f, b = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float x0 = bf16lo(raw[(h + r) * 4 + i]) - mean[r], x1 = bf16hi(raw[(h + r) * 4 + i]) - mean[r];
+                        a = fmaf(x0, x0, a);
+                        b = fmaf(x1, x1, b);
+                    }
+                    rstd[r] = a + b;
+                }
+                row_sums(rstd, lane);
+                opaque(raw, h * 4);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    rstd[r] = rsqrtf(rstd[r] * (1.0f / kC) + kLnEps);
+                    mean[r] *= -rstd[r];
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 ga = *reinterpret_cast<const float2*>(prm + ch * 8 + i * 2);
+                    const float2 be = *reinterpret_cast<const float2*>(prm + 128 + ch * 8 + i * 2);
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        uint32_t& v = raw[(h + r) * 4 + i];
+                        v = pack_bf16x2(fmaf(fmaf(bf16lo(v), rstd[r], mean[r]), ga.x, be.x),
+                                        fmaf(fmaf(bf16hi(v), rstd[r], mean[r]), ga.y, be.y));
+                    }
                 }
             }
+            if (!mbar_wait(x_empty(buf), (use & 1u) ^ 1u, abort_flag)) {
+                if (lane == 0) report_wait_failure(status, abort_flag, kKidTrans, 8);
+                break;
+            }
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                sts128(chunk_addr(xtile, row0 + 2 * r, ch), make_uint4(raw[r * 4], raw[r * 4 + 1], raw[r * 4 + 2], raw[r * 4 + 3]));
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(a_ready(buf));
+            if (++buf == 3) { buf = 0; ++use; }
         }
     } else {
         // ---------------------------------------------------------------- two row groups
-        const int g = (warp - 3) >> 3;
+        const int g = (warp - 12) >> 3;
         const int quad = warp & 3;
-        const int half = ((warp - 3) >> 2) & 1;
+        const int half = ((warp - 12) >> 2) & 1;
         const int row = quad * 32 + lane;
-        const int gtid = (warp - 3 - g * 8) * 32 + lane;
-        float* xch = reinterpret_cast<float*>(gbase + TrSmem::kXch) + g * 512;
-        const uint32_t xtile = sbase + TrSmem::kX + g * kTileBytes;
         const uint32_t htile = sbase + TrSmem::kH + g * kKBlockBytes;
         const uint32_t t_d1 = tmem_base + ((uint32_t)(quad * 32) << 16) + g * 256;
         const uint32_t t_d2 = t_d1 + 128;
         bool ok = true;
-        for (long long pi = 0; pi * 2 + g < my_tiles && ok; ++pi) {
-            const uint32_t ppar = (uint32_t)pi & 1u;
-            const long long tile = blockIdx.x + (pi * 2 + g) * gridDim.x;
-            const long long grow = tile * kRows + row;
-            if (!mbar_wait(x_full(g), ppar, abort_flag)) {
-                if (lane == 0) report_wait_failure(status, abort_flag, kKidTrans, 8);
-                break;
-            }
-            uint32_t raw[32];   // this thread's 64 channels of the row: kept for the residual
-            load_half_row(xtile, row, half, raw);
-            {
-                float mean, rstd;
-                half_row_stats_xwarp(raw, row, half, xch, 1 + g, 256, mean, rstd);
-                store_normalized_half_row(xtile, row, half, raw, mean, rstd, prm, prm + 128);
-            }
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(a_ready(g));
+        uint32_t ppar = 0;
+        int buf = g;
+        for (int t = g; t < my_tiles && ok; t += 2, ppar ^= 1u) {
+            const uint32_t xtile = sbase + TrSmem::kX + buf * kTileBytes;
+            buf += 2;
+            if (buf >= 3) buf -= 3;
+            const long long grow = (blockIdx.x + (long long)t * gridDim.x) * kRows + row;
             float m = 1.0f;
             if (mask != nullptr && grow < rows) m = __bfloat162float(mask[grow]);
 
@@ -272,6 +394,11 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     tmem_ld16(t_d1 + half * 32 + q * 16, a);
                     tmem_ld16(t_d1 + 64 + half * 32 + q * 16, b);
                     tmem_ld_wait();
+                    if (q == 1) {   // D1 is in registers: the next chunk's G1 may run under the rest of this pass
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(d1_empty(g));
+                    }
 #pragma unroll
                     for (int e = 0; e < 16; e += 2) {
                         const float a0 = __uint_as_float(a[e]), a1 = __uint_as_float(a[e + 1]);
@@ -280,9 +407,6 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                         hpk[q * 8 + e / 2] = pack_bf16x2(h0, h1);
                     }
                 }
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(d1_empty(g));
                 // the previous chunk's G2 must have consumed the H buffer before it is overwritten
                 if (!mbar_wait(h_free(g), cpar ^ 1u, abort_flag)) {
                     if (lane == 0) report_wait_failure(status, abort_flag, kKidTrans, 10);
@@ -302,44 +426,45 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidTrans, 11);
                 break;
             }
+            if (!mbar_wait(res_full(g), ppar, abort_flag)) {
+                if (lane == 0) report_wait_failure(status, abort_flag, kKidTrans, 16);
+                break;
+            }
             tc_fence_after_sync();
 #pragma unroll
             for (int cb = 0; cb < 4; ++cb) {
                 uint32_t y[16];
                 tmem_ld16(t_d2 + half * 64 + cb * 16, y);
                 tmem_ld_wait();
+                if (cb == 3) {
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(d2_empty(g));
+                }
 #pragma unroll
                 for (int ch = 0; ch < 2; ++ch) {
+                    const uint32_t xa = chunk_addr(xtile, row, half * 8 + cb * 2 + ch);
+                    const uint4 xv = lds128(xa);
+                    const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
                     uint32_t o[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int e = ch * 8 + j * 2;
-                        const uint32_t xr = raw[cb * 8 + ch * 4 + j];
                         float v0 = m * __uint_as_float(y[e]);
                         float v1 = m * __uint_as_float(y[e + 1]);
                         if (add_residual) {
-                            v0 += bf16lo(xr);
-                            v1 += bf16hi(xr);
+                            v0 += bf16lo(xw[j]);
+                            v1 += bf16hi(xw[j]);
                         }
                         o[j] = pack_bf16x2(v0, v1);
                     }
-                    sts128(chunk_addr(xtile, row, half * 8 + cb * 2 + ch), make_uint4(o[0], o[1], o[2], o[3]));
+                    sts128(xa, make_uint4(o[0], o[1], o[2], o[3]));
                 }
             }
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(d2_empty(g));
             fence_proxy_async_smem();
-            group_sync(1 + g, 256);
-            if (gtid == 0) {
-                tma_store_3d(&tmOut, xtile, 0, (int)(tile * kRows), 0);
-                tma_store_3d(&tmOut, xtile + kKBlockBytes, 64, (int)(tile * kRows), 0);
-                tma_store_commit();
-                tma_store_wait_read<0>();
-                mbar_arrive(x_empty(g));
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(out_ready(g));
         }
-        if (gtid == 0) tma_store_wait_all<0>();
     }
 
     tc_fence_before_sync();
@@ -363,11 +488,13 @@ struct Tr64Smem {
     static constexpr uint32_t kParams = kH + 4 * kKBlockBytes;   // gamma, beta
     static constexpr uint32_t kXch = kParams + 1024;
     static constexpr uint32_t kBars = kXch + 4096;
-    static constexpr uint32_t kTotal = kBars + 160;
+    static constexpr uint32_t kTotal = kBars + 192;
     static constexpr uint32_t kDyn = kTotal + 1024;
 };
 
-__global__ void __launch_bounds__(kTrThreads, 1)
+constexpr int kTr64Threads = 32 * (3 + 2 * 8);
+
+__global__ void __launch_bounds__(kTr64Threads, 1)
 transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmOut,
                     const __grid_constant__ CUtensorMap tmWa, const __grid_constant__ CUtensorMap tmWb,
                     const __grid_constant__ CUtensorMap tmWo, const __nv_bfloat16* __restrict__ mask,
@@ -387,8 +514,9 @@ transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     auto d1_full = [&](int g) { return bars + 8u * (11 + g); };
     auto h_ready = [&](int g) { return bars + 8u * (13 + g); };
     auto d2_full = [&](int g) { return bars + 8u * (15 + g); };
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 144);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 152);
+    auto out_ready = [&](int g) { return bars + 8u * (17 + g); };   // the group's result lies in the x buffer
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Sm::kBars + 160);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Sm::kBars + 168);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long num_tiles = (rows + kRows - 1) / kRows;
@@ -405,6 +533,7 @@ transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
             mbar_init(d1_full(g), 1);
             mbar_init(h_ready(g), 8);
             mbar_init(d2_full(g), 1);
+            mbar_init(out_ready(g), 8);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -446,6 +575,7 @@ transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     } else if (warp <= 2) {
         if (lane == 0) {
             const int g = warp - 1;
+            grid_wait();   // (the stores)
             bool ok = mbar_wait(w_full, 0, abort_flag);
             if (!ok) report_wait_failure(status, abort_flag, kKidTrans, 22);
             for (long long lt = g; lt < my_tiles && ok; lt += 2) {
@@ -466,14 +596,22 @@ transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
                 mma_rows<128>(tmem_base + g * 256, sbase + Sm::kH + g * 2 * kKBlockBytes, sbase + Sm::kWo, 8192,
                               idesc_bf16_f32(128, 64), false);
                 mma_commit(d2_full(g));
+                if (!mbar_wait(out_ready(g), ph, abort_flag)) {
+                    report_wait_failure(status, abort_flag, kKidTrans, 28);
+                    break;
+                }
+                tma_store_3d(&tmOut, xtile, 0, (int)((blockIdx.x + lt * gridDim.x) * kRows), 0);
+                tma_store_commit();
+                tma_store_wait_read<0>();
+                mbar_arrive(x_empty(g, (int)ph));
             }
+            tma_store_wait_all<0>();
         }
     } else {
         const int g = (warp - 3) >> 3;
         const int quad = warp & 3;
         const int half = ((warp - 3) >> 2) & 1;
         const int row = quad * 32 + lane;
-        const int gtid = (warp - 3 - g * 8) * 32 + lane;
         float* xch = reinterpret_cast<float*>(gbase + Sm::kXch) + g * 512;
         const uint32_t htile = sbase + Sm::kH + g * 2 * kKBlockBytes;
         const uint32_t td = tmem_base + ((uint32_t)(quad * 32) << 16) + g * 256;
@@ -553,15 +691,9 @@ transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
             }
             tc_fence_before_sync();
             fence_proxy_async_smem();
-            group_sync(1 + g, 256);
-            if (gtid == 0) {
-                tma_store_3d(&tmOut, xtile, 0, (int)(tile * kRows), 0);
-                tma_store_commit();
-                tma_store_wait_read<0>();
-                mbar_arrive(x_empty(g, b));
-            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(out_ready(g));
         }
-        if (gtid == 0) tma_store_wait_all<0>();
     }
 
     tc_fence_before_sync();
@@ -614,16 +746,21 @@ int transition(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bfloat16*
         device_mark_configured(4);
     }
     const long long tiles = (rows + kRows - 1) / kRows;
-    // two tiles per CTA pass share each weight chunk: aim for an even number of tiles per CTA
+    // Two tiles per CTA share each weight chunk: an even number of tiles per CTA, once every SM has one (with fewer tiles
+    // than SMs a tile has its SM's pipes to itself).
     long long grid = sm_count();
-    if (tiles < 2 * grid) grid = (tiles + 1) / 2;
+    if (tiles <= grid) grid = tiles;
+    else if (tiles < 2 * grid) grid = (tiles + 1) / 2;
     if (grid < 1) grid = 1;
     LaunchScope scope(kKidTrans, st);
     typedef const __nv_bfloat16* P;
     const int residual = (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0;
-    OF3_CUDA_CHECK(launch_chained(c == 128 ? transition_kernel : transition64_kernel, dim3((unsigned)grid), kTrThreads,
-                                  c == 128 ? TrSmem::kDyn : Tr64Smem::kDyn, st, tmX, tmOut, tmWa, tmWb, tmWo, mask,
-                                  (P)p->ln_w, (P)p->ln_b, rows, residual, device_status_ptr()));
+    if (c == 128)
+        OF3_CUDA_CHECK(launch_chained(transition_kernel, dim3((unsigned)grid), kTrThreads, TrSmem::kDyn, st, tmX, tmOut, tmWa,
+                                      tmWb, tmWo, x, mask, (P)p->ln_w, (P)p->ln_b, rows, residual, device_status_ptr()));
+    else
+        OF3_CUDA_CHECK(launch_chained(transition64_kernel, dim3((unsigned)grid), kTr64Threads, Tr64Smem::kDyn, st, tmX, tmOut,
+                                      tmWa, tmWb, tmWo, mask, (P)p->ln_w, (P)p->ln_b, rows, residual, device_status_ptr()));
     return OF3_OK;
 }
 
