@@ -10,7 +10,10 @@
 // Persistent, warp-specialised CTA (one per SM):
 //   warp 0     TMA producer     A tile 128x64, B tile BNx64 per k-block, 128B swizzle
 //   warp 1     MMA issuer       tcgen05.mma 128 x BN x 16, accumulators double-buffered in TMEM
-//   warps 2-5  epilogue         tcgen05.ld -> bf16 -> global (overlaps the next tile's main loop)
+//   warps 2-5  epilogue         tcgen05.ld -> bf16 -> global (overlaps the next tile's main loop); 32 bytes per store
+//                               where the pitch allows it (16-byte halves of a sector reach L2 one by one: N = 384 39 -> 29 us,
+//                               N = 768 114 -> 107)
+#include "modules.cuh"
 #include "rowtile.cuh"
 #include "runtime.cuh"
 
@@ -38,7 +41,7 @@ __global__ void __launch_bounds__(192, 1)
 contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    __nv_bfloat16* __restrict__ out, int M, int N, int K, int batch,
                    long long out_batch_stride, int ldo, int rows_per_block, long long row_block_stride,
-                   int a_shared, int* status) {
+                   int a_shared, int chan_shift, long long out_sample_stride, int wide, int* status) {
     using Cfg = ContractCfg<BN>;
     constexpr int S = Cfg::kStages;
     extern __shared__ uint8_t smem_raw[];
@@ -93,7 +96,12 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             bool ok = true;
             rowtile::TileWalk tw(blockIdx.x, gridDim.x, num_mt, num_nt);
             for (long long t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, tw.next()) {
-                const int nt = tw.tile, mt = tw.line, b = tw.b;
+                // maps: {k, row, 1, batch entry, 1}, or {k, row of its block, block, channel, sample}
+                const int a0 = tw.line * kBM, b0 = tw.tile * BN;
+                const int b = tw.b & (int)((1u << chan_shift) - 1u), smp = tw.b >> chan_shift;
+                const bool blocked = chan_shift != 31;
+                const int a_row = blocked ? 0 : a0, a_blk = blocked ? a0 >> kLineBlockShift : 0;
+                const int b_row = blocked ? 0 : b0, b_blk = blocked ? b0 >> kLineBlockShift : 0;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % S;
                     const uint32_t ph = (it / S) & 1u;
@@ -104,8 +112,8 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     }
                     mbar_arrive_expect_tx(full_bar(s), Cfg::kStageBytes);
                     const uint32_t sa = smem_base + s * Cfg::kStageBytes;
-                    tma_load_3d(sa, &tmA, full_bar(s), kb * kBK, mt * kBM, a_shared ? 0 : b);
-                    tma_load_3d(sa + Cfg::kABytes, &tmB, full_bar(s), kb * kBK, nt * BN, b);
+                    tma_load_5d(sa, &tmA, full_bar(s), kb * kBK, a_row, a_blk, a_shared ? 0 : b, smp);
+                    tma_load_5d(sa + Cfg::kABytes, &tmB, full_bar(s), kb * kBK, b_row, b_blk, b, smp);
                 }
             }
         }
@@ -166,13 +174,14 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             tc_fence_after_sync();
             const int row = mt * kBM + quad * 32 + lane;
             // rows_per_block > 0: output rows are grouped in blocks of that many rows and block q starts
-            // at q * row_block_stride (the layout a row-sharding all-to-all sends without a repack)
+            // at q * row_block_stride (the layout a row-sharding all-to-all sends without a repack, and the blocked one)
             long long roff = (long long)row * ldo;
             if (rows_per_block > 0) {
-                const int q = row / rows_per_block;
+                const int q = (uint32_t)row / (uint32_t)rows_per_block;
                 roff = (long long)q * row_block_stride + (long long)(row - q * rows_per_block) * ldo;
             }
-            __nv_bfloat16* orow = out + (long long)b * out_batch_stride + roff;
+            __nv_bfloat16* orow = out + (long long)(b >> chan_shift) * out_sample_stride +
+                                  (long long)(b & (int)((1u << chan_shift) - 1u)) * out_batch_stride + roff;
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN;
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
@@ -182,15 +191,19 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                 const int col0 = nt * BN + c * 32;
                 if (row < M) {
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) {
-                        const int col = col0 + g * 8;
+                    for (int g = 0; g < 2; ++g) {   // 16 columns: a sector of 32 bytes, whole where the pitch allows it
+                        const int col = col0 + g * 16;
+                        uint32_t o[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            o[e] = pack_bf16x2(__uint_as_float(r[g * 16 + 2 * e]), __uint_as_float(r[g * 16 + 2 * e + 1]));
                         if (col < N) {
-                            uint4 v;
-                            v.x = pack_bf16x2(__uint_as_float(r[g * 8 + 0]), __uint_as_float(r[g * 8 + 1]));
-                            v.y = pack_bf16x2(__uint_as_float(r[g * 8 + 2]), __uint_as_float(r[g * 8 + 3]));
-                            v.z = pack_bf16x2(__uint_as_float(r[g * 8 + 4]), __uint_as_float(r[g * 8 + 5]));
-                            v.w = pack_bf16x2(__uint_as_float(r[g * 8 + 6]), __uint_as_float(r[g * 8 + 7]));
-                            *reinterpret_cast<uint4*>(orow + col) = v;
+                            if (wide) {
+                                stg256(orow + col, o);
+                            } else {
+                                *reinterpret_cast<uint4*>(orow + col) = make_uint4(o[0], o[1], o[2], o[3]);
+                                if (col + 8 < N) *reinterpret_cast<uint4*>(orow + col + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+                            }
                         }
                     }
                 }
@@ -210,28 +223,33 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     }
 }
 
+// rows of `lines` lines in the blocked layout of contract_blocked_bf16, `box_rows` of them per copy
+int blocked_tmap(CUtensorMap* m, const __nv_bfloat16* x, int samples, int channels, int lines, int K, int ld, int box_rows) {
+    const uint64_t row = (uint64_t)ld * 2, chan = row << kLineBlockShift, blk = chan * channels;
+    const uint64_t blocks = (uint64_t)ceil_div(lines, 1 << kLineBlockShift);
+    uint64_t dims[5] = {(uint64_t)K, 1ull << kLineBlockShift, blocks, (uint64_t)channels, (uint64_t)samples};
+    uint64_t str[4] = {row, blk, chan, blk * blocks};
+    uint32_t box[5] = {kBK, 1u << kLineBlockShift, (uint32_t)box_rows >> kLineBlockShift, 1, 1};
+    return make_tmap_bf16(m, x, 5, dims, str, box, true);
+}
+// entries of `rows` rows, `entry` elements apart
+int plane_tmap(CUtensorMap* m, const __nv_bfloat16* x, int entries, int rows, int K, int ld, long long entry, int box_rows) {
+    uint64_t dims[5] = {(uint64_t)K, (uint64_t)rows, 1, (uint64_t)entries, 1};
+    uint64_t str[4] = {(uint64_t)ld * 2, (uint64_t)entry * 2, (uint64_t)entry * 2, (uint64_t)entry * 2};
+    uint32_t box[5] = {kBK, (uint32_t)box_rows, 1, 1, 1};
+    return make_tmap_bf16(m, x, 5, dims, str, box, true);
+}
+
+struct ContractOut {
+    __nv_bfloat16* out;
+    int ld, rows_per_block, chan_shift;   // chan_shift 31: the batch entries are not split into samples
+    long long batch_stride, row_block_stride, sample_stride;
+};
+
 template <int BN>
-int launch_contract(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, int batch,
-                    int M, int N, int K, int lda, int ldb, int ldo, long long a_bs, long long b_bs,
-                    long long o_bs, int rows_per_block, long long row_block_stride, cudaStream_t stream,
-                    int account_as) {
+int launch_contract(const CUtensorMap& tmA, const CUtensorMap& tmB, const ContractOut& o, int batch, int M, int N, int K,
+                    bool a_shared, cudaStream_t stream, int account_as) {
     using Cfg = ContractCfg<BN>;
-    CUtensorMap tmA, tmB;
-    {
-        // a_bs == 0: every batch entry multiplies the same A (several linear layers on one input)
-        uint64_t dims[3] = {(uint64_t)K, (uint64_t)M, (uint64_t)(a_bs == 0 ? 1 : batch)};
-        uint64_t str[2] = {(uint64_t)lda * 2, (uint64_t)(a_bs == 0 ? (long long)lda * M : a_bs) * 2};
-        uint32_t box[3] = {kBK, kBM, 1};
-        int rc = make_tmap_bf16(&tmA, a, 3, dims, str, box, true);
-        if (rc) return rc;
-    }
-    {
-        uint64_t dims[3] = {(uint64_t)K, (uint64_t)N, (uint64_t)batch};
-        uint64_t str[2] = {(uint64_t)ldb * 2, (uint64_t)b_bs * 2};
-        uint32_t box[3] = {kBK, BN, 1};
-        int rc = make_tmap_bf16(&tmB, b, 3, dims, str, box, true);
-        if (rc) return rc;
-    }
     constexpr int kAttrKey = BN == 256 ? 0 : (BN == 128 ? 1 : 2);  // per-device function attributes
     if (!device_configured(kAttrKey)) {
         OF3_CUDA_CHECK(cudaFuncSetAttribute(contract_nt_kernel<BN>,
@@ -243,9 +261,11 @@ int launch_contract(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat1
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     int* status = device_status_ptr();
     LaunchScope scope(account_as, stream);  // launch accounting: the triangle einsum or a plain linear layer
-    contract_nt_kernel<BN><<<grid, 192, Cfg::kSmemBytes, stream>>>(tmA, tmB, out, M, N, K, batch,
-                                                                   o_bs, ldo, rows_per_block, row_block_stride,
-                                                                   a_bs == 0 ? 1 : 0, status);
+    const int wide = o.ld % 16 == 0 && o.batch_stride % 16 == 0 && o.row_block_stride % 16 == 0 &&
+                     o.sample_stride % 16 == 0 && ((uintptr_t)o.out & 31) == 0;
+    contract_nt_kernel<BN><<<grid, 192, Cfg::kSmemBytes, stream>>>(tmA, tmB, o.out, M, N, K, batch, o.batch_stride, o.ld,
+                                                                   o.rows_per_block, o.row_block_stride, a_shared ? 1 : 0,
+                                                                   o.chan_shift, o.sample_stride, wide, status);
     OF3_CUDA_CHECK(cudaGetLastError());
     return OF3_OK;
 }
@@ -265,11 +285,35 @@ int contract_nt_bf16(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat
     OF3_REQUIRE(((uintptr_t)out & 15) == 0, OF3_ERR_ALIGN, "contract: out not 16-byte aligned");
     OF3_REQUIRE(rows_per_block >= 0 && row_block_stride % 8 == 0, OF3_ERR_ALIGN,
                 "contract: row block stride must be a multiple of 8 elements");
-    if (N > 128)
-        return launch_contract<256>(a, b, out, batch, M, N, K, lda, ldb, ldo, a_bs, b_bs, o_bs, rows_per_block,
-                                    row_block_stride, stream, account_as);
-    return launch_contract<128>(a, b, out, batch, M, N, K, lda, ldb, ldo, a_bs, b_bs, o_bs, rows_per_block,
-                                row_block_stride, stream, account_as);
+    const ContractOut o = {out, ldo, rows_per_block, 31, o_bs, row_block_stride, 0};
+    const int bn = N > 128 ? 256 : 128;
+    CUtensorMap tmA, tmB;
+    int rc;
+    // a_bs == 0: every batch entry multiplies the same A (several linear layers on one input)
+    if ((rc = plane_tmap(&tmA, a, a_bs == 0 ? 1 : batch, M, K, lda, a_bs == 0 ? (long long)lda * M : a_bs, kBM))) return rc;
+    if ((rc = plane_tmap(&tmB, b, batch, N, K, ldb, b_bs, bn))) return rc;
+    return bn == 256 ? launch_contract<256>(tmA, tmB, o, batch, M, N, K, a_bs == 0, stream, account_as)
+                     : launch_contract<128>(tmA, tmB, o, batch, M, N, K, a_bs == 0, stream, account_as);
+}
+
+// X = A B^T per sample and channel, all three as [sample][line / 8][channel][8][ld] with N lines of N positions.
+int contract_blocked_bf16(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, int samples, int channels,
+                          int N, int ld, cudaStream_t stream) {
+    OF3_REQUIRE(a && b && out && samples > 0 && N > 0, OF3_ERR_ARG, "contract: bad argument");
+    OF3_REQUIRE((channels & (channels - 1)) == 0, OF3_ERR_SHAPE, "contract: channels must be a power of two");
+    OF3_REQUIRE(ld % 8 == 0 && ld >= (int)align_up(N, 8) && ((uintptr_t)out & 15) == 0, OF3_ERR_ALIGN,
+                "contract: pitch or alignment");
+    int shift = 0;
+    while ((1 << shift) < channels) ++shift;
+    const long long chan = (long long)ld << kLineBlockShift, blk = chan * channels;
+    const ContractOut o = {out, ld, 1 << kLineBlockShift, shift, chan, blk, ceil_div(N, 1 << kLineBlockShift) * blk};
+    const int bn = N > 128 ? 256 : 128;
+    CUtensorMap tmA, tmB;
+    int rc;
+    if ((rc = blocked_tmap(&tmA, a, samples, channels, N, N, ld, kBM))) return rc;
+    if ((rc = blocked_tmap(&tmB, b, samples, channels, N, N, ld, bn))) return rc;
+    return bn == 256 ? launch_contract<256>(tmA, tmB, o, samples * channels, N, N, N, false, stream, 1)
+                     : launch_contract<128>(tmA, tmB, o, samples * channels, N, N, N, false, stream, 1);
 }
 
 }  // namespace of3

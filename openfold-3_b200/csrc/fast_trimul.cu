@@ -28,6 +28,47 @@ using namespace rowtile;
 constexpr int kKidIn = 2;
 constexpr int kKidOut = 3;
 
+// Where the channel-major tensors a_t, b_t and x_t keep channel c of a line: at channel(c) + line(l), its positions behind
+// one another. Planes: [c][line][ld], or one group of channels per destination rank when they are about to be exchanged.
+// Blocked (a whole pair tensor on this GPU): [line / 8][c][8][ld], so that what the tiles in flight write and read at one
+// time, all channels of some twenty lines, lies in a few megabytes. In planes the 32 channels of one store lie a plane
+// apart, and from 2 MB per plane on in as many pages. trimul_in, planes -> blocked: N = 768 149 -> 142 us, N = 1003
+// 369 -> 246, N = 2048 1.19 -> 1.01 ms; blocks of 32 lines are no faster.
+struct PlaneLayout {
+    int ld, group_shift, line_shift;
+    long long group_stride, chan_stride, block_stride, sample_stride;   // elements
+    __host__ __device__ long long channel(int c) const {
+        return (long long)(c >> group_shift) * group_stride + (long long)(c & ((1 << group_shift) - 1)) * chan_stride;
+    }
+    __host__ __device__ long long line(int l) const {
+        return (long long)(l >> line_shift) * block_stride + (long long)(l & (int)((1u << line_shift) - 1u)) * ld;
+    }
+};
+PlaneLayout plane_layout(int R, int ld, int C, int groups, long long group_stride) {
+    PlaneLayout pl;
+    pl.ld = ld;
+    pl.group_shift = C == 128 ? 7 : 6;
+    for (int g = groups; g > 1; g >>= 1) --pl.group_shift;
+    pl.line_shift = 31;
+    pl.chan_stride = (long long)R * ld;
+    pl.group_stride = groups == 1 ? C * pl.chan_stride : group_stride;
+    pl.block_stride = 0;
+    pl.sample_stride = groups * pl.group_stride;
+    return pl;
+}
+constexpr int kLineBlock = 1 << kLineBlockShift;
+PlaneLayout blocked_layout(int R, int ld, int C) {
+    PlaneLayout pl;
+    pl.ld = ld;
+    pl.group_shift = C == 128 ? 7 : 6;
+    pl.line_shift = kLineBlockShift;
+    pl.group_stride = 0;
+    pl.chan_stride = (long long)kLineBlock * ld;
+    pl.block_stride = C * pl.chan_stride;
+    pl.sample_stride = ceil_div(R, kLineBlock) * pl.block_stride;
+    return pl;
+}
+
 // R = lines per sample (R == N for a whole pair tensor, N / P for a row shard)
 // =====================================================================================
 // trimul_in
@@ -62,7 +103,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmWbg, const __nv_bfloat16* __restrict__ mask,
                  const __nv_bfloat16* __restrict__ ln_w, const __nv_bfloat16* __restrict__ ln_b,
                  __nv_bfloat16* __restrict__ a_t, __nv_bfloat16* __restrict__ b_t, int B, int R,
-                 int N, int ld, int group_shift, long long group_stride, int wide_stores, int* status) {
+                 int N, PlaneLayout pl, int wide_stores, int* status) {
     using Sm = InSmem<C>;
     constexpr int kSt = Sm::kStages;
     extern __shared__ uint8_t smem_raw[];
@@ -233,12 +274,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         const int lch = quad * 32 + lane;
         const bool is_b = C == 128 ? set == 1 : lch >= 64;
         const int c = lch & (C - 1);
-        const long long cs = (long long)R * ld;
-        // channel c lives at (c >> group_shift) * group_stride + (c & group_mask) * R * ld: one contiguous plane
-        // [C][R][ld] by default, or one group of channels per destination rank when the planes are about to be
-        // exchanged
-        __nv_bfloat16* plane = (is_b ? b_t : a_t) + (long long)(c >> group_shift) * group_stride +
-                               (long long)(c & ((1 << group_shift) - 1)) * cs;
+        __nv_bfloat16* plane = (is_b ? b_t : a_t) + pl.channel(c);
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + set * 256;
         grid_wait();
         uint32_t it = 0, use = 0;
@@ -256,8 +292,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
             const float* mk = mask05 + (it % Sm::kMaskRing) * 128;
             // the line pitch ld is a multiple of 8 elements, so a 16-byte store that starts below N ends inside the
             // row; with a pitch that is a multiple of 16 (and 32-byte aligned planes) the same holds for 32 bytes
-            __nv_bfloat16* dst = plane + (long long)tw.b * ((C >> group_shift) * group_stride) +
-                                 (long long)tw.line * ld + t0;
+            __nv_bfloat16* dst = plane + tw.b * pl.sample_stride + pl.line(tw.line) + t0;
             // 16 positions per pass; the TMEM load of the next pass is in flight while this one is computed
             auto emit = [&](const uint32_t (&p)[16], const uint32_t (&g)[16], int k0) {
                 uint32_t o[8];
@@ -324,7 +359,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
 
 // The same layer with the projections the other way round (the normalised tile is the A operand, a TMEM lane is a
 // position, its columns the output channels; N = 256 per MMA): a warp's store covers 32 consecutive positions of ONE
-// channel plane. Slower than the kernel above while a channel plane stays within a 2 MB page or so (170 against
+// channel plane. For planes only: slower than the kernel above while one stays within a 2 MB page or so (170 against
 // 151 us at N = 768: one 2-byte store per value), faster beyond (1.13 against 2.02 ms at N = 2048, where the 32
 // planes one store of the kernel above touches lie megabytes apart).
 constexpr int kInRowsThreads = 448;  // producer, MMA, 4 LayerNorm warps, 2 x 4 epilogue warps
@@ -336,7 +371,7 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                  const __grid_constant__ CUtensorMap tmWbg, const __nv_bfloat16* __restrict__ mask,
                  const __nv_bfloat16* __restrict__ ln_w, const __nv_bfloat16* __restrict__ ln_b,
                  __nv_bfloat16* __restrict__ a_t, __nv_bfloat16* __restrict__ b_t, int B, int R,
-                 int N, int ld, int group_shift, long long group_stride, int* status) {
+                 int N, PlaneLayout pl, int* status) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
@@ -491,13 +526,8 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
                     break;
                 }
                 tc_fence_after_sync();
-                // channel c lives at (c >> group_shift) * group_stride + (c & group_mask) * R * ld: one
-                // contiguous plane [128][R][ld] by default, or one group of channels per destination
-                // rank when the planes are about to be exchanged
-                const long long cs = (long long)R * ld;
-                __nv_bfloat16* dst = (q == 0 ? a_t : b_t) +
-                                     (long long)tw.b * ((kC >> group_shift) * group_stride) +
-                                     (long long)tw.line * ld + k;
+                const long long cs = pl.chan_stride;
+                __nv_bfloat16* dst = (q == 0 ? a_t : b_t) + tw.b * pl.sample_stride + pl.line(tw.line) + k;
                 const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + q * 256;
 #pragma unroll 1
                 for (int cb = 0; cb < 4; ++cb) {
@@ -509,8 +539,7 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
 #pragma unroll
                         for (int hf = 0; hf < 2; ++hf) {  // groups hold >= 16 channels: no boundary inside a half
                             const int c0 = cb * 32 + hf * 16;
-                            __nv_bfloat16* d0 = dst + (long long)(c0 >> group_shift) * group_stride +
-                                                (long long)(c0 & ((1 << group_shift) - 1)) * cs;
+                            __nv_bfloat16* d0 = dst + pl.channel(c0);
 #pragma unroll
                             for (int e = 0; e < 16; ++e) {
                                 // the same expression as the kernel above, so that both give the same bits:
@@ -566,8 +595,8 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                   const __grid_constant__ CUtensorMap tmOut, const __grid_constant__ CUtensorMap tmWg,
                   const __grid_constant__ CUtensorMap tmWz, const __nv_bfloat16* __restrict__ ln_in_w,
                   const __nv_bfloat16* __restrict__ ln_in_b, const __nv_bfloat16* __restrict__ ln_out_w,
-                  const __nv_bfloat16* __restrict__ ln_out_b, int B, int R, int N, int add_residual,
-                  int* status) {
+                  const __nv_bfloat16* __restrict__ ln_out_b, int B, int R, int N, int x_line_shift,
+                  int add_residual, int* status) {
     using Sm = OutSmem<C>;
     constexpr int kTm = 2 * C;   // tensor-memory columns of a group: gate, update
     constexpr int CH = C / 2;   // channels per thread
@@ -651,7 +680,8 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                 }
                 // x tile: all 128 channels of positions (fixed, t0 .. t0+127), layout [c][j]
                 mbar_arrive_expect_tx(x_full(g), tile_bytes<C>());
-                tma_load_3d(sbase + Sm::kX + g * tile_bytes<C>(), &tmX, x_full(g), t0, tw.line, tw.b * C);
+                tma_load_5d(sbase + Sm::kX + g * tile_bytes<C>(), &tmX, x_full(g), t0,
+                            tw.line & (int)((1u << x_line_shift) - 1u), tw.line >> x_line_shift, 0, tw.b);
                 if (!mbar_wait(z_empty(g), (use & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidOut, 6);
                     break;
@@ -804,7 +834,7 @@ int line_tmap(CUtensorMap* m, const void* z, int B, int R, int N, int C) {
 template <int C, bool kOutgoing>
 int launch_in(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensorMap* w, const __nv_bfloat16* mask,
               const __nv_bfloat16* lw, const __nv_bfloat16* lb, __nv_bfloat16* a_t, __nv_bfloat16* b_t, int B, int R,
-              int N, int ld, int group_shift, long long group_stride, int wide) {
+              int N, const PlaneLayout& pl, int wide) {
     static PerDeviceOnce configured;
     if (!configured.done()) {
         OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_in_kernel<C, kOutgoing>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -813,14 +843,13 @@ int launch_in(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensorM
     }
     LaunchScope scope(kKidIn, st);
     OF3_CUDA_CHECK(launch_chained(trimul_in_kernel<C, kOutgoing>, grid, kInThreads, InSmem<C>::kDyn, st, tmZ, w[0], w[1],
-                                  w[2], w[3], mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift, group_stride, wide,
-                                  device_status_ptr()));
+                                  w[2], w[3], mask, lw, lb, a_t, b_t, B, R, N, pl, wide, device_status_ptr()));
     return OF3_OK;
 }
 template <bool kOutgoing>
 int launch_in_rows(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensorMap* w, const __nv_bfloat16* mask,
                    const __nv_bfloat16* lw, const __nv_bfloat16* lb, __nv_bfloat16* a_t, __nv_bfloat16* b_t, int B, int R,
-                   int N, int ld, int group_shift, long long group_stride) {
+                   int N, const PlaneLayout& pl) {
     static PerDeviceOnce configured;
     if (!configured.done()) {
         OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_in_rows_kernel<kOutgoing>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -829,14 +858,13 @@ int launch_in_rows(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUte
     }
     LaunchScope scope(kKidIn, st);
     OF3_CUDA_CHECK(launch_chained(trimul_in_rows_kernel<kOutgoing>, grid, kInRowsThreads, InSmem<128>::kDyn, st, tmZ, w[0],
-                                  w[1], w[2], w[3], mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift, group_stride,
-                                  device_status_ptr()));
+                                  w[1], w[2], w[3], mask, lw, lb, a_t, b_t, B, R, N, pl, device_status_ptr()));
     return OF3_OK;
 }
 template <int C>
 int launch_out(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensorMap& tmX, const CUtensorMap& tmOut,
                const CUtensorMap& tmWg, const CUtensorMap& tmWz, const of3_trimul_params* p, int B, int R, int N,
-               int add_residual) {
+               int x_line_shift, int add_residual) {
     static PerDeviceOnce configured;
     if (!configured.done()) {
         OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_out_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -846,7 +874,7 @@ int launch_out(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensor
     typedef const __nv_bfloat16* P;
     LaunchScope scope(kKidOut, st);
     OF3_CUDA_CHECK(launch_chained(trimul_out_kernel<C>, grid, kOutThreads, OutSmem<C>::kDyn, st, tmZ, tmX, tmOut, tmWg, tmWz,
-                                  (P)p->ln_in_w, (P)p->ln_in_b, (P)p->ln_out_w, (P)p->ln_out_b, B, R, N, add_residual,
+                                  (P)p->ln_in_w, (P)p->ln_in_b, (P)p->ln_out_w, (P)p->ln_out_b, B, R, N, x_line_shift, add_residual,
                                   device_status_ptr()));
     return OF3_OK;
 }
@@ -859,17 +887,9 @@ bool trimul_supported(int c_z, int c_h) { return c_z == c_h && (c_z == 128 || c_
 // transposed_walk: z is [B][N][R][C] and a line runs along its FIRST index (line = second index),
 // which makes the incoming update the same K-major contraction as the outgoing one; with R != N this
 // is a row shard of N rows seen as R lines of N positions each.
-// groups > 1: the C channels are written as `groups` equal groups, group q of a_t at
-// a_t + q * group_stride (b_t likewise), so that each group can be sent to another rank as one block.
-int trimul_project(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* a_t, __nv_bfloat16* b_t,
-                   int B, int R, int N, int ld, bool transposed_walk, const of3_trimul_params* p,
-                   cudaStream_t st, int groups, long long group_stride, int C) {
+static int project(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* a_t, __nv_bfloat16* b_t, int B, int R,
+                   int N, const PlaneLayout& pl, bool transposed_walk, const of3_trimul_params* p, cudaStream_t st, int C) {
     OF3_REQUIRE(((uintptr_t)z & 15) == 0, OF3_ERR_ALIGN, "trimul: z must be 16-byte aligned");
-    OF3_REQUIRE(groups == 1 || groups == 2 || groups == 4 || groups == 8, OF3_ERR_ARG,
-                "trimul: channel groups must be 1, 2, 4 or 8 (got %d)", groups);
-    int group_shift = C == 128 ? 7 : 6;
-    for (int g = groups; g > 1; g >>= 1) --group_shift;
-    if (groups == 1) group_stride = (long long)C * R * ld;
     int rc;
     CUtensorMap tmZ, tmW[4];
     if (!transposed_walk) {
@@ -886,77 +906,79 @@ int trimul_project(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloa
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     // 32-byte stores need every channel row of a_t / b_t to start on a 32-byte boundary
-    const int wide = (ld % 16 == 0 && (group_stride % 16) == 0 && ((uintptr_t)a_t & 31) == 0 && ((uintptr_t)b_t & 31) == 0) ? 1 : 0;
+    const int wide = (pl.ld % 16 == 0 && pl.group_stride % 16 == 0 && ((uintptr_t)a_t & 31) == 0 && ((uintptr_t)b_t & 31) == 0) ? 1 : 0;
     // a channel plane of R lines: beyond about one 2 MB page the kernel whose stores stay inside one plane wins
-    const bool planes_far_apart = C == 128 && (long long)R * ld * (long long)sizeof(__nv_bfloat16) > (2LL << 20);
+    const bool planes_far_apart = C == 128 && pl.chan_stride * (long long)sizeof(__nv_bfloat16) > (2LL << 20);
     const __nv_bfloat16* lw = (const __nv_bfloat16*)p->ln_in_w;
     const __nv_bfloat16* lb = (const __nv_bfloat16*)p->ln_in_b;
     if (planes_far_apart)
-        return transposed_walk ? launch_in_rows<false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
-                                                       group_stride)
-                               : launch_in_rows<true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
-                                                      group_stride);
+        return transposed_walk ? launch_in_rows<false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, pl)
+                               : launch_in_rows<true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, pl);
     if (C == 128)
-        return transposed_walk ? launch_in<128, false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
-                                                       group_stride, wide)
-                               : launch_in<128, true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
-                                                      group_stride, wide);
-    return transposed_walk ? launch_in<64, false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
-                                                  group_stride, wide)
-                           : launch_in<64, true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, ld, group_shift,
-                                                 group_stride, wide);
+        return transposed_walk ? launch_in<128, false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, pl, wide)
+                               : launch_in<128, true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, pl, wide);
+    return transposed_walk ? launch_in<64, false>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, pl, wide)
+                           : launch_in<64, true>(grid, st, tmZ, tmW, mask, lw, lb, a_t, b_t, B, R, N, pl, wide);
 }
 
-// x = a_t . b_t^T per channel (a_t: R lines, b_t: all N lines), then LN_out / linear_z / gate / residual
-// on the R lines of z -> out (may alias z).
-int trimul_finish(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* a_t,
-                  const __nv_bfloat16* b_t, __nv_bfloat16* x_t, int B, int R, int N, int ld, int add_residual,
-                  const of3_trimul_params* p, cudaStream_t st, int C) {
-    OF3_REQUIRE(((uintptr_t)z & 15) == 0 && ((uintptr_t)out & 15) == 0, OF3_ERR_ALIGN,
-                "trimul: z/out must be 16-byte aligned");
-    int rc = contract_nt_bf16(a_t, b_t, x_t, B * C, R, N, N, ld, ld, ld, (long long)R * ld, (long long)N * ld,
-                              (long long)R * ld, st);
-    if (rc) return rc;
-    return trimul_output(z, out, x_t, B, R, N, ld, add_residual, p, st, C);
+// groups > 1: the C channels are written as `groups` equal groups, group q of a_t at
+// a_t + q * group_stride (b_t likewise), so that each group can be sent to another rank as one block.
+int trimul_project(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* a_t, __nv_bfloat16* b_t,
+                   int B, int R, int N, int ld, bool transposed_walk, const of3_trimul_params* p,
+                   cudaStream_t st, int groups, long long group_stride, int C) {
+    OF3_REQUIRE(groups == 1 || groups == 2 || groups == 4 || groups == 8, OF3_ERR_ARG,
+                "trimul: channel groups must be 1, 2, 4 or 8 (got %d)", groups);
+    return project(z, mask, a_t, b_t, B, R, N, plane_layout(R, ld, C, groups, group_stride), transposed_walk, p, st, C);
 }
 
 // LN_out(x) -> linear_z, gate from LN_in(z), residual: the part of the update after the contraction,
 // on R lines of z with x_t[b*C + c][line][j] (pitch ld)
-int trimul_output(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* x_t, int B, int R, int N, int ld,
-                  int add_residual, const of3_trimul_params* p, cudaStream_t st, int C) {
+static int output(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* x_t, int B, int R, int N,
+                  const PlaneLayout& pl, int add_residual, const of3_trimul_params* p, cudaStream_t st, int C) {
     OF3_REQUIRE(((uintptr_t)z & 15) == 0 && ((uintptr_t)out & 15) == 0 && ((uintptr_t)x_t & 15) == 0, OF3_ERR_ALIGN,
                 "trimul: z/out/x must be 16-byte aligned");
     int rc;
     CUtensorMap tmZ, tmOut, tmX, tmWg, tmWz;
     if ((rc = line_tmap(&tmZ, z, B, R, N, C))) return rc;
     if ((rc = line_tmap(&tmOut, out, B, R, N, C))) return rc;
-    {   // x_t[b*C + c][line][j], pitch ld: box = 128 positions j x 1 x C channels, no swizzle
-        uint64_t dims[3] = {(uint64_t)N, (uint64_t)R, (uint64_t)B * C};
-        uint64_t str[2] = {(uint64_t)ld * 2, (uint64_t)R * ld * 2};
-        uint32_t box[3] = {128, 1, (uint32_t)C};
-        if ((rc = make_tmap_bf16(&tmX, x_t, 3, dims, str, box, 0))) return rc;
+    {   // {position j, line of its block, block, channel, sample}: box = 128 positions of one line x C channels, no swizzle
+        const bool blocked = pl.line_shift == kLineBlockShift;
+        uint64_t dims[5] = {(uint64_t)N, (uint64_t)(blocked ? kLineBlock : R), (uint64_t)(blocked ? ceil_div(R, kLineBlock) : 1),
+                            (uint64_t)C, (uint64_t)B};
+        uint64_t str[4] = {(uint64_t)pl.ld * 2, (uint64_t)(blocked ? pl.block_stride : pl.sample_stride) * 2,
+                           (uint64_t)pl.chan_stride * 2, (uint64_t)pl.sample_stride * 2};
+        uint32_t box[5] = {128, 1, 1, (uint32_t)C, 1};
+        if ((rc = make_tmap_bf16(&tmX, x_t, 5, dims, str, box, 0))) return rc;
     }
     if ((rc = weight_tmap(&tmWg, p->w_g, C))) return rc;
     if ((rc = weight_tmap(&tmWz, p->w_z, C))) return rc;
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
-    return C == 128 ? launch_out<128>(grid, st, tmZ, tmX, tmOut, tmWg, tmWz, p, B, R, N, add_residual)
-                    : launch_out<64>(grid, st, tmZ, tmX, tmOut, tmWg, tmWz, p, B, R, N, add_residual);
+    return C == 128 ? launch_out<128>(grid, st, tmZ, tmX, tmOut, tmWg, tmWz, p, B, R, N, pl.line_shift, add_residual)
+                    : launch_out<64>(grid, st, tmZ, tmX, tmOut, tmWg, tmWz, p, B, R, N, pl.line_shift, add_residual);
+}
+
+// the same on planes [b*C + c][line][ld]
+int trimul_output(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* x_t, int B, int R, int N, int ld,
+                  int add_residual, const of3_trimul_params* p, cudaStream_t st, int C) {
+    return output(z, out, x_t, B, R, N, plane_layout(R, ld, C, 1, 0), add_residual, p, st, C);
 }
 
 int trimul(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N, int C,
            int flags, const of3_trimul_params* p, Arena& ws, cudaStream_t st) {
-    const int ld = (int)align_up(N, 8);
-    const size_t plane = (size_t)B * C * N * ld * sizeof(__nv_bfloat16);
-    __nv_bfloat16* a_t = (__nv_bfloat16*)ws.take(plane);
-    __nv_bfloat16* b_t = (__nv_bfloat16*)ws.take(plane);
-    __nv_bfloat16* x_t = (__nv_bfloat16*)ws.take(plane);
+    const int ld = (int)align_up(N, 16);   // (32-byte stores)
+    const PlaneLayout pl = blocked_layout(N, ld, C);
+    const size_t bytes = (size_t)B * pl.sample_stride * sizeof(__nv_bfloat16);
+    __nv_bfloat16* a_t = (__nv_bfloat16*)ws.take(bytes);
+    __nv_bfloat16* b_t = (__nv_bfloat16*)ws.take(bytes);
+    __nv_bfloat16* x_t = (__nv_bfloat16*)ws.take(bytes);
     if (!ws.base) return OF3_OK;
     OF3_REQUIRE(ws.ok(), OF3_ERR_WORKSPACE, "trimul: workspace too small (%zu needed)", ws.off);
     const bool outgoing = (flags & OF3_FLAG_OUTGOING) != 0;
-    int rc = trimul_project(z, mask, a_t, b_t, B, N, N, ld, !outgoing, p, st, 1, 0, C);
+    int rc = project(z, mask, a_t, b_t, B, N, N, pl, !outgoing, p, st, C);
     if (rc) return rc;
-    return trimul_finish(z, out, a_t, b_t, x_t, B, N, N, ld, (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, st, C);
+    if ((rc = contract_blocked_bf16(a_t, b_t, x_t, B, C, N, ld, st))) return rc;
+    return output(z, out, x_t, B, N, N, pl, (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, st, C);
 }
 
 }  // namespace fast

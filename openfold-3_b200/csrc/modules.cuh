@@ -43,9 +43,6 @@ int trimul_project(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloa
                    cudaStream_t st, int groups = 1, long long group_stride = 0, int C = 128);
 int trimul_output(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* x_t, int B, int R, int N, int ld,
                   int add_residual, const of3_trimul_params* p, cudaStream_t st, int C = 128);
-int trimul_finish(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat16* a_t,
-                  const __nv_bfloat16* b_t, __nv_bfloat16* x_t, int B, int R, int N, int ld, int add_residual,
-                  const of3_trimul_params* p, cudaStream_t st, int C = 128);
 size_t triattn_image_elems(int B, int R, int N, int C = 128);
 size_t triattn_bias_elems(int B, int R, int N);  // bf16 elements of the pair-bias image [B*4][key blocks][R][32]
 int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* vt,
@@ -100,6 +97,10 @@ int apb_dispatch(const void* a, const void* z, const void* s, const void* mask, 
 int cond_dispatch(const void* a, const void* s, const void* mask, void* out, long long rows, int c_a, int c_s, int n,
                   int dtype, int flags, const of3_cond_transition_params* p, Arena& ws, cudaStream_t st);
 
+// lines per block of the channel-major tensors of the triangle update, as a power of two
+constexpr int kLineBlockShift = 3;
+int contract_blocked_bf16(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, int samples, int channels,
+                          int N, int ld, cudaStream_t stream);
 int contract_nt_bf16(const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* out, int batch,
                      int M, int N, int K, int lda, int ldb, int ldo, long long a_bs, long long b_bs,
                      long long o_bs, cudaStream_t stream, int rows_per_block = 0, long long row_block_stride = 0,
