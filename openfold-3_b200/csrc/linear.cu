@@ -278,6 +278,22 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
             const uint32_t acc = tc & 1u;
             const long long row = (long long)c.mt * kBM + quad * 32 + lane;
             const bool live = row < rows;
+            const int colb = c.nt * kWRows + half * kCols;   // first column of this thread, inside the matrix
+            // The gate and residual values of the tile, all of them on their way under its GEMM: fetched 16 columns at a time
+            // between the TMEM loads, their latency was what a tile took (six times 1 us at BN = 192)
+            constexpr int kPre = EPI == kEpiResidual ? kCols / 16 : 1;
+            [[maybe_unused]] uint32_t gv[kPre][8], zv[kPre][8];
+            [[maybe_unused]] float mk = 1.0f;
+            if constexpr (EPI == kEpiResidual) {
+                if (live) {
+                    if (ep.mask != nullptr) mk = __bfloat162float(ep.mask[row]);
+#pragma unroll
+                    for (int p = 0; p < kPre; ++p) {
+                        if (ep.gate != nullptr) ld_row16(ep.gate + row * n + colb + p * 16, gv[p]);
+                        if (ep.residual != nullptr) ld_row16_any(ep.residual + row * n + colb + p * 16, zv[p]);
+                    }
+                }
+            }
             if (!mbar_wait(tfull(acc), (tc >> 1) & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKid, 4);
                 break;
@@ -289,17 +305,13 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                 bb = (int)((uint32_t)row / (uint32_t)ep.im.rows_per_sample);
                 pos = (int)row - bb * ep.im.rows_per_sample;
             }
-            float mk = 1.0f;
-            if constexpr (EPI == kEpiResidual) {
-                if (ep.mask != nullptr && live) mk = __bfloat162float(ep.mask[row]);
-            }
-#pragma unroll 1
+#pragma unroll(EPI == kEpiResidual ? kPre : 1)
             for (int c0 = 0; c0 < kCols; c0 += 16) {
                 uint32_t r[16], r2[16];
                 tmem_ld16(taddr + c0, r);
                 if constexpr (EPI == kEpiSwiglu) tmem_ld16(taddr + BN / 2 + c0, r2);
                 tmem_ld_wait();
-                const int col = c.nt * kWRows + half * kCols + c0;   // column inside the matrix
+                const int col = colb + c0;
                 if (!live) continue;
                 if constexpr (EPI == kEpiImages) {
                     store_images<D>(ep.im, ep.kind[c.g], ep.qscale, r, col, row, bb, pos);
@@ -323,8 +335,8 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
 #pragma unroll
                         for (int e = 0; e < 16; ++e) v[e] = mk * __uint_as_float(r[e]);
                         if (ep.gate != nullptr) {
-                            uint32_t g[8], b[8];
-                            ld_row16(ep.gate + row * n + col, g);
+                            const uint32_t (&g)[8] = gv[c0 / 16];
+                            uint32_t b[8];
                             ld_row16_any(ep.gate_bias + col, b);
 #pragma unroll
                             for (int e = 0; e < 8; ++e) {
@@ -333,8 +345,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                             }
                         }
                         if (ep.residual != nullptr) {
-                            uint32_t z[8];
-                            ld_row16_any(ep.residual + row * n + col, z);
+                            const uint32_t (&z)[8] = zv[c0 / 16];
 #pragma unroll
                             for (int e = 0; e < 8; ++e) {
                                 v[2 * e] += bf16lo(z[e]);
