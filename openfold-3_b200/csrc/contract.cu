@@ -88,6 +88,8 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr_smem;
+    grid_trigger();
+    grid_wait();
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
@@ -263,10 +265,9 @@ int launch_contract(const CUtensorMap& tmA, const CUtensorMap& tmB, const Contra
     LaunchScope scope(account_as, stream);  // launch accounting: the triangle einsum or a plain linear layer
     const int wide = o.ld % 16 == 0 && o.batch_stride % 16 == 0 && o.row_block_stride % 16 == 0 &&
                      o.sample_stride % 16 == 0 && ((uintptr_t)o.out & 31) == 0;
-    contract_nt_kernel<BN><<<grid, 192, Cfg::kSmemBytes, stream>>>(tmA, tmB, o.out, M, N, K, batch, o.batch_stride, o.ld,
-                                                                   o.rows_per_block, o.row_block_stride, a_shared ? 1 : 0,
-                                                                   o.chan_shift, o.sample_stride, wide, status);
-    OF3_CUDA_CHECK(cudaGetLastError());
+    OF3_CUDA_CHECK(launch_chained(contract_nt_kernel<BN>, grid, 192, Cfg::kSmemBytes, stream, tmA, tmB, o.out, M, N, K, batch,
+                                  o.batch_stride, o.ld, o.rows_per_block, o.row_block_stride, a_shared ? 1 : 0, o.chan_shift,
+                                  o.sample_stride, wide, status));
     return OF3_OK;
 }
 
