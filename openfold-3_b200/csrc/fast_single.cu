@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(256) ada_rows_kernel(const bf16* __restrict__ 
     const int lane = threadIdx.x & 31;
     const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= rows) return;
-    uint32_t g[NV][4], s[NV][4];   // in flight together with the row
+    uint32_t g[NV][4], s[NV][4], b[NV][4];   // in flight together with the row
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         const int c = (v * 32 + lane) * 8;
@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(256) ada_rows_kernel(const bf16* __restrict__ 
         const uint4 gv = *reinterpret_cast<const uint4*>(g_lin + r * C + c);
         const uint4 sv = *reinterpret_cast<const uint4*>(s_lin + r * C + c);
         g[v][0] = gv.x; g[v][1] = gv.y; g[v][2] = gv.z; g[v][3] = gv.w;
+        ld_row8_any(b_g + c, b[v]);
         s[v][0] = sv.x; s[v][1] = sv.y; s[v][2] = sv.z; s[v][3] = sv.w;
     }
     Row<NV> row;
@@ -179,12 +180,10 @@ __global__ void __launch_bounds__(256) ada_rows_kernel(const bf16* __restrict__ 
     for (int v = 0; v < NV; ++v) {
         const int c = (v * 32 + lane) * 8;
         if (c >= C) continue;
-        uint32_t b[4];
         float gf[8], sf[8], bf[8], o[8];
-        ld_row8_any(b_g + c, b);
         unpack8(g[v], gf);
         unpack8(s[v], sf);
-        unpack8(b, bf);
+        unpack8(b[v], bf);
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] = row.x[v * 8 + e] / (1.0f + __expf(-(gf[e] + bf[e]))) + sf[e];
         *reinterpret_cast<uint4*>(an + r * C + c) = pack8(o);
