@@ -2,8 +2,8 @@
 // the single track (c_s = 384) and of the diffusion token stack (c_a = 768, c_s = 384).
 //
 //   y = x W^T, x [rows][k], W [n][k], both K-major. Persistent CTA: warp 0 TMA producer (128-byte swizzled k-blocks of
-//   64), warp 1 MMA issuer (128 x BN x 16, accumulators double-buffered in TMEM), warps 2..9 the epilogue (two per 32
-//   rows, each half of the columns; thread = row).
+//   64), warp 1 MMA issuer (128 x BN x 16, accumulators double-buffered in TMEM), warps 2..17 the epilogue (four per 32
+//   rows, each a quarter of the columns; thread = row).
 //
 // What bounds them: a few hundred 128-row tiles with k = 384 .. 1536 are 3 - 15 us of L2 -> shared-memory traffic (every
 // tile streams its A and B panels) and, for short sequences, launch and fill latency; the separate passes that read the
@@ -24,7 +24,8 @@ typedef __nv_bfloat16 bf16;
 
 constexpr int kKid = 10;
 constexpr int kBM = 128, kBK = 64;
-constexpr int kThreads = 32 * (2 + 8);
+constexpr int kEpiParts = 4;   // epilogue warps per 32 rows, each with its part of the columns
+constexpr int kThreads = 32 * (2 + 4 * kEpiParts);
 constexpr float kLog2e = 1.4426950408889634f;
 
 enum Epi { kEpiStore, kEpiImages, kEpiSwiglu, kEpiResidual };
@@ -55,7 +56,14 @@ struct EpiArgs {
     const bf16 *residual, *gate, *gate_bias, *mask;
 };
 
-__device__ __forceinline__ float sigmoid_of(float x) { return 1.0f / (1.0f + __expf(-x)); }
+// 1 / (1 + exp(-x)) with the reciprocal refined by one Newton step, r (2 - d r): as close as the division, in a third of
+// its instructions. The clamp keeps d finite (0 * inf in the step): below -87 the result is 1.6e-38 instead of less.
+__device__ __forceinline__ float sigmoid_of(float x) {
+    const float d = 1.0f + __expf(-x > 87.0f ? 87.0f : -x);   // (a NaN stays one)
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
 
 // One column group of 16 of this thread's row as attention operand images; `kind` is uniform over the tile.
 template <int D>
@@ -173,7 +181,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(tfull(a), 1);
-            mbar_init(tempty(a), 8);
+            mbar_init(tempty(a), 4 * kEpiParts);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -268,9 +276,12 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
             }
         }
     } else {
-        // ---------------------------------------------------------------- epilogue: thread = row, half of the columns
-        const int quad = warp & 3, half = (warp - 2) >> 2;
-        constexpr int kCols = EPI == kEpiSwiglu ? BN / 4 : BN / 2;   // result columns per thread and tile
+        // ---------------------------------------------------------------- epilogue: thread = row, a part of the columns
+        // With two warps per 32 rows an epilogue took 7700 (images), 8900 (silu * mul) and 18100 (gate and residual) cycles
+        // for tiles whose GEMMs take 8300, 8300 and 14000 (in-kernel clock, 3840 rows of 768): latency, two warps per
+        // scheduler, and the divisions of the sigmoids.
+        const int quad = warp & 3, part = (warp - 2) >> 2;
+        constexpr int kCols = (EPI == kEpiSwiglu ? BN / 2 : BN) / kEpiParts;   // result columns per thread and tile
         grid_wait();
         uint32_t tc = 0;
         for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tc) {
@@ -278,13 +289,17 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
             const uint32_t acc = tc & 1u;
             const long long row = (long long)c.mt * kBM + quad * 32 + lane;
             const bool live = row < rows;
-            const int colb = c.nt * kWRows + half * kCols;   // first column of this thread, inside the matrix
+            const int colb = c.nt * kWRows + part * kCols;   // first column of this thread, inside the matrix
             // The gate and residual values of the tile, all of them on their way under its GEMM: fetched 16 columns at a time
             // between the TMEM loads, their latency was what a tile took (six times 1 us at BN = 192)
             constexpr int kPre = EPI == kEpiResidual ? kCols / 16 : 1;
             [[maybe_unused]] uint32_t gv[kPre][8], zv[kPre][8];
-            [[maybe_unused]] float mk = 1.0f;
+            [[maybe_unused]] float mk = 1.0f, bias0 = 0.f, bias1 = 0.f;   // gate biases of columns lane and 32 + lane
             if constexpr (EPI == kEpiResidual) {
+                if (ep.gate != nullptr) {
+                    if (lane < kCols) bias0 = __bfloat162float(ep.gate_bias[colb + lane]);
+                    if (32 + lane < kCols) bias1 = __bfloat162float(ep.gate_bias[colb + 32 + lane]);
+                }
                 if (live) {
                     if (ep.mask != nullptr) mk = __bfloat162float(ep.mask[row]);
 #pragma unroll
@@ -299,7 +314,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                 break;
             }
             tc_fence_after_sync();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * Cfg::kAccStride + half * kCols;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * Cfg::kAccStride + part * kCols;
             [[maybe_unused]] int bb = 0, pos = 0;   // sample and position of the row
             if constexpr (EPI == kEpiImages) {
                 bb = (int)((uint32_t)row / (uint32_t)ep.im.rows_per_sample);
@@ -312,7 +327,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                 if constexpr (EPI == kEpiSwiglu) tmem_ld16(taddr + BN / 2 + c0, r2);
                 tmem_ld_wait();
                 const int col = colb + c0;
-                if (!live) continue;
+                if (EPI != kEpiResidual && !live) continue;   // (its gate biases are shared by shuffles)
                 if constexpr (EPI == kEpiImages) {
                     store_images<D>(ep.im, ep.kind[c.g], ep.qscale, r, col, row, bb, pos);
                 } else {
@@ -336,12 +351,12 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                         for (int e = 0; e < 16; ++e) v[e] = mk * __uint_as_float(r[e]);
                         if (ep.gate != nullptr) {
                             const uint32_t (&g)[8] = gv[c0 / 16];
-                            uint32_t b[8];
-                            ld_row16_any(ep.gate_bias + col, b);
+                            const float bias = c0 < 32 ? bias0 : bias1;
 #pragma unroll
                             for (int e = 0; e < 8; ++e) {
-                                v[2 * e] *= sigmoid_of(bf16lo(g[e]) + bf16lo(b[e]));
-                                v[2 * e + 1] *= sigmoid_of(bf16hi(g[e]) + bf16hi(b[e]));
+                                const int src = (c0 & 31) + 2 * e;
+                                v[2 * e] *= sigmoid_of(bf16lo(g[e]) + __shfl_sync(0xffffffffu, bias, src));
+                                v[2 * e + 1] *= sigmoid_of(bf16hi(g[e]) + __shfl_sync(0xffffffffu, bias, src + 1));
                             }
                         }
                         if (ep.residual != nullptr) {
@@ -354,7 +369,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                         }
 #pragma unroll
                         for (int e = 0; e < 8; ++e) o[e] = pack_bf16x2(v[2 * e], v[2 * e + 1]);
-                        st_row16_any(ep.out + row * n + col, o);
+                        if (live) st_row16_any(ep.out + row * n + col, o);
                     }
                 }
             }
