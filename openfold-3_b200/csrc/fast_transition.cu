@@ -111,6 +111,9 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int my_tiles = (int)tiles_of_block((rows + kRows - 1) / kRows);
     // group g's tiles are the CTA's tiles g, g + 2, ...
+    // One tile only (a tensor of fewer tiles than SMs): both groups work on it, each on half of every chunk's columns and of
+    // the output's. The silu pass is the longest link of a lone tile's chain (trunk, N = 37, four blocks: 492 -> 489 us).
+    const bool solo = my_tiles == 1;
     const int num_chunks = ((my_tiles + 1) >> 1) * kNumChunks;
 
     if (threadIdx.x == 0) {
@@ -120,13 +123,13 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             mbar_init(wo_full(i), 1);
             mbar_init(wo_empty(i), 2);
             mbar_init(d1_full(i), 1);
-            mbar_init(d1_empty(i), 8);
-            mbar_init(h_ready(i), 8);
+            mbar_init(d1_empty(i), solo ? 16 : 8);
+            mbar_init(h_ready(i), solo ? 16 : 8);
             mbar_init(h_free(i), 1);
             mbar_init(d2_full(i), 1);
             mbar_init(d2_empty(i), 8);
             mbar_init(res_full(i), 1);
-            mbar_init(out_ready(i), 8);
+            mbar_init(out_ready(i), solo ? 16 : 8);
         }
         for (int i = 0; i < 3; ++i) {
             mbar_init(x_empty(i), 1);
@@ -152,7 +155,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_ptr;
     grid_trigger();
-    grid_wait();
+    if (warp != 0) grid_wait();   // (the weights do not depend on the kernel before this one)
     // TMEM columns: group g -> D1 at g*256 + [0,128) ([a 64 | b 64]), D2 at g*256 + [128,256)
 
     if (warp == 0) {
@@ -361,7 +364,8 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
     } else {
         // ---------------------------------------------------------------- two row groups
-        const int g = (warp - 12) >> 3;
+        const int own = (warp - 12) >> 3;      // group of these warps
+        const int g = solo ? 0 : own;          // group whose tile they work on
         const int quad = warp & 3;
         const int half = ((warp - 12) >> 2) & 1;
         const int row = quad * 32 + lane;
@@ -390,11 +394,12 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                 uint32_t hpk[16];  // 32 of the chunk's 64 hidden values of this row, packed bf16x2
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
+                    if (solo && q != own) continue;
                     uint32_t a[16], b[16];
                     tmem_ld16(t_d1 + half * 32 + q * 16, a);
                     tmem_ld16(t_d1 + 64 + half * 32 + q * 16, b);
                     tmem_ld_wait();
-                    if (q == 1) {   // D1 is in registers: the next chunk's G1 may run under the rest of this pass
+                    if (q == 1 || solo) {   // D1 is in registers: the next chunk's G1 may run under the rest of this pass
                         tc_fence_before_sync();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(d1_empty(g));
@@ -414,9 +419,11 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     break;
                 }
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch)
+                for (int ch = 0; ch < 4; ++ch) {
+                    if (solo && ch >> 1 != own) continue;
                     sts128(chunk_addr(htile, row, half * 4 + ch),
                            make_uint4(hpk[ch * 4], hpk[ch * 4 + 1], hpk[ch * 4 + 2], hpk[ch * 4 + 3]));
+                }
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(h_ready(g));
@@ -433,6 +440,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             tc_fence_after_sync();
 #pragma unroll
             for (int cb = 0; cb < 4; ++cb) {
+                if (solo && cb >> 1 != own) continue;
                 uint32_t y[16];
                 tmem_ld16(t_d2 + half * 64 + cb * 16, y);
                 tmem_ld_wait();
