@@ -94,10 +94,16 @@ struct InSmem {
 // outgoing: tmZ is 3-D {c, second index, b*N + first index}; incoming: 4-D {c, second, first, b}
 constexpr int kInLnWarps = 8;    // two threads per position
 constexpr int kInEpiSets = 2;    // epilogue warp sets, one per TMEM slot
-constexpr int kInThreads = 32 * (2 + kInLnWarps + 4 * kInEpiSets);  // producer, MMA, LayerNorm and epilogue warps
+// Warps per 32 channels of a set, each with its part of the positions: 64 channels have one job per tile, whose epilogue
+// is the longest step (template stack, N = 300 x 4: 55 -> 47 us with two); with 128 channels a second one gives nothing
+// (N = 768: 142 -> 150: registers).
+template <int C>
+constexpr int kInEpiParts = C == 128 ? 1 : 2;
+template <int C>
+constexpr int kInThreads = 32 * (2 + kInLnWarps + 4 * kInEpiSets * kInEpiParts<C>);  // producer, MMA, LayerNorm, epilogue
 
 template <int C, bool kOutgoing>
-__global__ void __launch_bounds__(kInThreads, 1)
+__global__ void __launch_bounds__(kInThreads<C>, 1)
 trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmWap,
                  const __grid_constant__ CUtensorMap tmWag, const __grid_constant__ CUtensorMap tmWbp,
                  const __grid_constant__ CUtensorMap tmWbg, const __nv_bfloat16* __restrict__ mask,
@@ -135,7 +141,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         }
         for (int q = 0; q < 2; ++q) {
             mbar_init(slot_full(q), 1);
-            mbar_init(slot_empty(q), 4);
+            mbar_init(slot_empty(q), 4 * kInEpiParts<C>);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -269,7 +275,10 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         // ---------------------------------------------------------------- epilogue warps: the first four take the a
         // projection (TMEM slot 0), the other four the b projection (slot 1); thread = output channel, columns =
         // positions
-        const int set = (warp - 2 - kInLnWarps) >> 2;   // TMEM slot of this set's jobs
+        constexpr int kParts = kInEpiParts<C>;
+        const int ew = warp - 2 - kInLnWarps;
+        const int set = ew / (4 * kParts);   // TMEM slot of this set's jobs
+        const int k_begin = ((ew >> 2) & (kParts - 1)) * (kRows / kParts);
         const int quad = warp & 3;
         const int lch = quad * 32 + lane;
         const bool is_b = C == 128 ? set == 1 : lch >= 64;
@@ -320,27 +329,38 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                     if (k0 + 8 < kmax) *reinterpret_cast<uint4*>(dst + k0 + 8) = make_uint4(o[4], o[5], o[6], o[7]);
                 }
             };
-            const int k_begin = 0, k_end = kmax;
-            uint32_t pa[16], ga[16], pb[16], gb[16];
-            if (k_begin < k_end) {
-                tmem_ld16(taddr + k_begin, pa);
-                tmem_ld16(taddr + 128 + k_begin, ga);
-            }
+            const int k_end = min(kmax, k_begin + kRows / kParts);
+            if constexpr (kParts > 1) {   // (the warps hide each other's loads)
 #pragma unroll 1
-            for (int k0 = k_begin; k0 < k_end; k0 += 32) {
-                tmem_ld_wait();
-                if (k0 + 16 < k_end) {
-                    tmem_ld16(taddr + k0 + 16, pb);
-                    tmem_ld16(taddr + 128 + k0 + 16, gb);
-                }
-                emit(pa, ga, k0);
-                if (k0 + 16 < k_end) {
+                for (int k0 = k_begin; k0 < k_end; k0 += 16) {
+                    uint32_t p[16], g[16];
+                    tmem_ld16(taddr + k0, p);
+                    tmem_ld16(taddr + 128 + k0, g);
                     tmem_ld_wait();
-                    if (k0 + 32 < k_end) {
-                        tmem_ld16(taddr + k0 + 32, pa);
-                        tmem_ld16(taddr + 128 + k0 + 32, ga);
+                    emit(p, g, k0);
+                }
+            } else {
+                uint32_t pa[16], ga[16], pb[16], gb[16];
+                if (k_begin < k_end) {
+                    tmem_ld16(taddr + k_begin, pa);
+                    tmem_ld16(taddr + 128 + k_begin, ga);
+                }
+#pragma unroll 1
+                for (int k0 = k_begin; k0 < k_end; k0 += 32) {
+                    tmem_ld_wait();
+                    if (k0 + 16 < k_end) {
+                        tmem_ld16(taddr + k0 + 16, pb);
+                        tmem_ld16(taddr + 128 + k0 + 16, gb);
                     }
-                    emit(pb, gb, k0 + 16);
+                    emit(pa, ga, k0);
+                    if (k0 + 16 < k_end) {
+                        tmem_ld_wait();
+                        if (k0 + 32 < k_end) {
+                            tmem_ld16(taddr + k0 + 32, pa);
+                            tmem_ld16(taddr + 128 + k0 + 32, ga);
+                        }
+                        emit(pb, gb, k0 + 16);
+                    }
                 }
             }
             tc_fence_before_sync();
@@ -842,7 +862,7 @@ int launch_in(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensorM
         configured.mark();
     }
     LaunchScope scope(kKidIn, st);
-    OF3_CUDA_CHECK(launch_chained(trimul_in_kernel<C, kOutgoing>, grid, kInThreads, InSmem<C>::kDyn, st, tmZ, w[0], w[1],
+    OF3_CUDA_CHECK(launch_chained(trimul_in_kernel<C, kOutgoing>, grid, kInThreads<C>, InSmem<C>::kDyn, st, tmZ, w[0], w[1],
                                   w[2], w[3], mask, lw, lb, a_t, b_t, B, R, N, pl, wide, device_status_ptr()));
     return OF3_OK;
 }
