@@ -11,7 +11,7 @@ from __future__ import annotations
 
 import torch
 
-from .lib import side_stream
+from .lib import holding, side_stream
 
 
 class GraphedModule:
@@ -38,7 +38,7 @@ class GraphedModule:
         cur.wait_stream(side)
         torch.cuda.synchronize(dev)
         self.graph = torch.cuda.CUDAGraph()
-        with torch.no_grad(), torch.cuda.graph(self.graph):
+        with torch.no_grad(), holding() as self._held, torch.cuda.graph(self.graph):
             self._static_out = fn(*self._static_in)
 
     def __call__(self, *args):

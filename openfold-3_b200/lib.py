@@ -7,7 +7,9 @@ library is missing or a call fails, a ``RuntimeError`` is raised.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import threading
 from ctypes import c_char_p, c_float, c_int, c_longlong, c_size_t, c_void_p
 from pathlib import Path
 
@@ -216,6 +218,29 @@ def dtype_code(dtype: torch.dtype) -> int:
     raise TypeError(f"unsupported activation dtype {dtype}: the kernels take bfloat16 or float32")
 
 
+# What a CUDA graph being captured reads besides the caller's tensors: packed weights, projected biases, workspaces. Their
+# owners replace them when parameters, pair tensors or sizes change, so the graph holds them itself.
+_captured = threading.local()
+
+
+@contextlib.contextmanager
+def holding():
+    """Collects, on this thread, what calls inside the block read by address: -> the list of those objects."""
+    outer, held = getattr(_captured, "held", None), []
+    _captured.held = held
+    try:
+        yield held
+    finally:
+        _captured.held = outer
+
+
+def hold(obj):
+    held = getattr(_captured, "held", None)
+    if held is not None:
+        held.append(obj)
+    return obj
+
+
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 
 
@@ -247,9 +272,9 @@ def workspace(nbytes: int, device: torch.device, stream: torch.cuda.Stream | Non
         buf = None
         _workspaces.pop(key, None)
         with torch.cuda.stream(st):   # allocated on the stream that uses it
-            buf = torch.empty(int(nbytes * 1.0) + 1024, dtype=torch.uint8, device=device)
+            buf = torch.empty(nbytes + 1024, dtype=torch.uint8, device=device)
         _workspaces[key] = buf
-    return buf
+    return hold(buf)
 
 
 def _ptr(t):

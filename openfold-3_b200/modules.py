@@ -182,13 +182,13 @@ class _PackedParams:
         if key != self._key:
             val = [None if t is None else t.detach().to(device=device, dtype=dtype).contiguous() for t in tensors]
             for group in adjacent:
-                if all(val[i] is not None for i in group):
+                if group and all(val[i] is not None for i in group):
                     block = torch.stack([val[i] for i in group])
                     for n, i in enumerate(group):
                         val[i] = block[n]
             self._val = tuple(val)
             self._key = key
-        return self._val
+        return lib.hold(self._val)
 
 
 def _param_watch():
@@ -234,7 +234,10 @@ class _BlockPlans:
         if (self._epoch != _structure_epoch or dtype != self._dtype or device != self._device
                 or (self._ref is not None and self._changed(self._watch))):
             self._build(block, dtype, device)
-        return None if self._ref is None or any(self._hooks) else self._ref
+        if self._ref is None or any(self._hooks):
+            return None
+        lib.hold(self._keep)
+        return self._ref
 
     def plan(self, block, *key):
         p = self._plans.get(key)
@@ -866,6 +869,7 @@ class DiffusionTransformer(_Tracked):
         self.hoist_pair_bias = True
         self._bias_cache = None   # (weakref to z, z._version, parameter versions, [bias per block])
         self._plans = _BlockPlans()
+        self._packed = _PackedParams()
 
     def _plan_submodules(self):
         blocks = list(self.blocks)
@@ -885,24 +889,21 @@ class DiffusionTransformer(_Tracked):
     def _native_params(self, dtype, device):
         """Parameter structs of all blocks. The projections of s lie back to back over the whole stack (the library
         computes those of several blocks in one launch)."""
-        conv = lambda t: None if t is None else t.detach().to(device=device, dtype=dtype).contiguous()  # noqa: E731
         layers = [m for b in self.blocks for m in (b.attention_pair_bias, b.conditioned_transition)]
-        cond = None
+        raw = [m._tensors() for m in layers]
+        first = [0]
+        for r in raw:
+            first.append(first[-1] + len(r))
+        group = ()
         if self.blocks[0].attention_pair_bias.use_ada_layer_norm:
-            raw = [m._tensors() for m in layers]
-            cond = torch.stack([r[i].detach().to(device=device, dtype=dtype) for m, r in zip(layers, raw)
-                                for i in m._cond_group]).view(len(layers), 3, *raw[0][layers[0]._cond_group[0]].shape)
-        vals = []
-        for n, m in enumerate(layers):
-            group = m._cond_group if cond is not None else ()
-            t = [None if i in group else conv(t) for i, t in enumerate(m._tensors())]
-            for j, i in enumerate(group):
-                t[i] = cond[n, j]
-            vals.append(t)
+            group = tuple(f + i for m, f in zip(layers, first) for i in m._cond_group)
+        # kept under the parameters themselves: a plan that is built again for another reason finds the same copies
+        packed = self._packed.get([t for r in raw for t in r], dtype, device, adjacent=(group,))
+        vals = [packed[a:b] for a, b in zip(first, first[1:])]
         attn = (lib.AttnPairBiasParams * len(self.blocks))(*[lib.AttnPairBiasParams(*_pointers(v)) for v in vals[0::2]])
         trans = (lib.CondTransitionParams * len(self.blocks))(
             *[lib.CondTransitionParams(*_pointers(v)) for v in vals[1::2]])
-        return (attn, trans), vals
+        return (attn, trans), packed
 
     def _native_plan(self, Ba, Bz, N, dtype, flags, with_bias):
         m = self.blocks[0].attention_pair_bias
@@ -921,6 +922,7 @@ class DiffusionTransformer(_Tracked):
         ac, zc, sc, m = m0._operands(a, z, s, mask)
         biases = self._pair_biases(z, token=st[0])
         flags = (lib.extra_flags | lib.FLAG_ADA_LN) | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
+        lib.hold(biases)
         plan = self._plans.plan(self, ac.shape[0], zc.shape[0], a.shape[-2], st[1], flags, biases[0] is not None)
         lib.diffusion_stack_forward(ac, sc, zc, m, biases, plan, st[1], flags, st[0])
         return True
@@ -958,7 +960,7 @@ class DiffusionTransformer(_Tracked):
         a = a.clone(memory_format=torch.contiguous_format)
         if not use_high_precision_attention and self._run_native(a, s, z, mask, _mask_trans):
             return a
-        biases = self._pair_biases(z)
+        biases = lib.hold(self._pair_biases(z))
         for b, pb in zip(self.blocks, biases):
             a = b(a, s, z, mask=mask, use_high_precision_attention=use_high_precision_attention,
                   _mask_trans=_mask_trans, _in_place=True, _pair_bias=pb)

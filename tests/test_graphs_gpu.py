@@ -70,3 +70,39 @@ def test_graphed_pairformer_stack_equals_eager(pkg):
             torch.cuda.synchronize()
             assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     pkg.lib.check_device_status()
+
+
+def test_a_graph_keeps_what_it_reads(pkg):
+    """Between capture and replay the stack is called for other sizes and pair tensors, its plan is built again and other
+    modules are made: nothing that the graph reads by address (packed weights, projected biases, workspace) is given back."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator().manual_seed(9)
+    model = pkg.DiffusionTransformer(**cases.DIFF, no_blocks=2, use_ada_layer_norm=True, n_query=None, n_key=None,
+                                     inf=1e9)
+    model.load_state_dict(pkg.weights.diffusion_stack_params(seed=21, no_blocks=2, **cases.DIFF), strict=True)
+    model = model.to(dev, bf).eval()
+
+    def draw(n):
+        return (torch.randn(1, 2, n, 768, generator=g).to(dev, bf), torch.randn(1, 2, n, 384, generator=g).to(dev, bf),
+                torch.randn(1, 1, n, n, 128, generator=g).to(dev, bf))
+
+    a, s, z = draw(40)
+    graphed = pkg.GraphedModule(lambda a, s: model(a, s, z), a, s)   # with the kept biases of z
+    want = graphed(a, s).clone()
+    with torch.no_grad():
+        model.eval()
+        pkg.LayerNorm(8)
+        for b in model.blocks:
+            b.attention_pair_bias.inf = 1e8
+        x = draw(150)
+        model(*x)
+        pkg.GraphedModule(model, *x)
+        model.float()(*(t.float() for t in draw(20)))   # and packs of another type take the place of these
+        model.to(bf)
+    torch.cuda.synchronize()
+    junk = [torch.full((1 << k,), float("nan"), device=dev) for k in range(8, 25) for _ in range(4)]   # freed memory
+    got = graphed(a, s)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    del junk
+    pkg.lib.check_device_status()
