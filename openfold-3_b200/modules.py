@@ -171,89 +171,109 @@ def _forward_only(module: nn.Module, *tensors):
 class _PackedParams:
     """Caches contiguous copies of a module's parameters in the activation dtype."""
 
-    def __init__(self):
-        self._key = None
-        self._val = None
+    _state = None   # (source tensors, key, copies), replaced as a whole: another thread sees one state or the other
+
+    def __reduce__(self):   # a copied or unpickled module packs its own
+        return (_PackedParams, ())
+
+    @property
+    def _val(self):
+        return None if self._state is None else self._state[2]
+
+    @_val.setter
+    def _val(self, val):
+        self._state = (*self._state[:2], val)
 
     def get(self, tensors, dtype, device, adjacent=()):
         """``adjacent``: groups of indices of equally shaped tensors whose copies are laid out back to back in one
         allocation (the library then runs linear layers that share an input as one launch)."""
         key = (dtype, device, tuple((t.data_ptr(), t._version) if t is not None else None for t in tensors))
-        if key != self._key:
+        st = self._state
+        # (the sources are held, so that a new tensor cannot come to lie at the address of one that is gone)
+        if st is None or st[1] != key or any(a is not b for a, b in zip(st[0], tensors)):
             val = [None if t is None else t.detach().to(device=device, dtype=dtype).contiguous() for t in tensors]
             for group in adjacent:
                 if group and all(val[i] is not None for i in group):
                     block = torch.stack([val[i] for i in group])
                     for n, i in enumerate(group):
                         val[i] = block[n]
-            self._val = tuple(val)
-            self._key = key
-        return lib.hold(self._val)
+            st = self._state = (tuple(tensors), key, tuple(val))
+        return lib.hold(st[2])
+
+
+_watch_module = None
 
 
 def _param_watch():
-    try:
-        from . import _param_watch as w
-    except ImportError as e:
-        raise RuntimeError("the _param_watch extension is missing: build it first (python __graft_entry__.py)") from e
-    return w
+    global _watch_module
+    if _watch_module is None:
+        try:
+            from . import _param_watch as w
+        except ImportError as e:
+            raise RuntimeError("the _param_watch extension is missing: build it first (python __graft_entry__.py)") from e
+        _watch_module = w
+    return _watch_module
 
 
-class _BlockPlans:
-    """A block's (or stack's) parameters as its native entry point takes them, and its plans per shape.
+class _Plan:
+    """What a native call of a block (or stack) needs, for one dtype and device. Nothing in it changes after it was built
+    but the cache of what depends on the shape."""
 
-    ``get`` returns the parameter structs, rebuilt when a parameter has another address or version, or the module tree
-    another structure, than when they were built; ``None`` when the call has to take the layer-by-layer path (hooks on
-    submodules, a submodule that is not this package's, parameters that track no versions)."""
+    __slots__ = ("dtype", "device", "epoch", "hooks", "watch", "params", "keep", "shapes")
 
-    def __init__(self):
-        self._epoch = -1
-        self._ref = None
-        self._plans = {}
-
-    def __reduce__(self):   # a copied or unpickled module builds its own
-        return (_BlockPlans, ())
-
-    def _build(self, block, dtype, device):
-        self._epoch = _structure_epoch
-        self._hooks, self._ref, self._plans = [], None, {}
-        self._dtype, self._device = dtype, device
+    def __init__(self, block, dtype, device):
+        self.dtype, self.device, self.epoch = dtype, device, _structure_epoch
+        self.hooks, self.watch, self.params, self.keep, self.shapes = [], None, None, None, {}
         plain = block._plan_submodules()
         if plain is None:
             return
         for m in plain:
-            self._hooks += [m._forward_hooks, m._forward_pre_hooks]
-        w = _param_watch()
-        self._changed = w.changed
-        self._watch = w.make([(m._parameters, n) for m in block.modules() for n, t in m._parameters.items()
-                              if t is not None])
-        if self._watch is not None:
-            self._ref, self._keep = block._native_params(dtype, device)
+            self.hooks += [m._forward_hooks, m._forward_pre_hooks]
+        self.watch = _param_watch().make([(m._parameters, n) for m in block.modules() for n, t in m._parameters.items()
+                                          if t is not None])
+        if self.watch is not None:
+            self.params, self.keep = block._native_params(dtype, device)
 
-    def get(self, block, dtype, device):
-        if (self._epoch != _structure_epoch or dtype != self._dtype or device != self._device
-                or (self._ref is not None and self._changed(self._watch))):
-            self._build(block, dtype, device)
-        if self._ref is None or any(self._hooks):
-            return None
-        lib.hold(self._keep)
-        return self._ref
+    def current(self, dtype, device):
+        return (dtype == self.dtype and device == self.device and self.epoch == _structure_epoch
+                and (self.watch is None or not _param_watch().changed(self.watch)))
 
-    def plan(self, block, *key):
-        p = self._plans.get(key)
+    def shape(self, block, *key):
+        p = self.shapes.get(key)
         if p is None:
-            if len(self._plans) >= 64:
-                self._plans.clear()
-            p = self._plans[key] = block._native_plan(*key)
+            if len(self.shapes) >= 64:
+                self.shapes.clear()
+            p = self.shapes[key] = block._native_plan(*key)
         return p
 
 
+class _BlockPlans:
+    """The plan of a block (or stack), built again when a parameter has another address or version, or the module tree
+    another structure, than when it was built. ``get``: ``None`` when the call has to take the layer-by-layer path (hooks on
+    submodules, a submodule that is not this package's, parameters that track no versions). Threads may share a module: each
+    works with the plan that it got."""
+
+    _plan = None
+
+    def __reduce__(self):   # a copied or unpickled module builds its own
+        return (_BlockPlans, ())
+
+    def get(self, block, dtype, device):
+        plan = self._plan
+        if plan is None or not plan.current(dtype, device):
+            plan = self._plan = _Plan(block, dtype, device)
+        if plan.params is None or any(plan.hooks):
+            return None
+        lib.hold(plan.keep)
+        return plan
+
+
 def _native_state(block, z):
-    """(parameter structs, dtype code) for the native path of ``block`` on z, or None."""
+    """(plan, dtype code) for the native path of ``block`` on z, or None."""
     if not z.is_cuda or block.training or z.dtype not in (torch.bfloat16, torch.float32):
         return None
-    ref = block._plans.get(block, z.dtype, z.device)
-    return None if ref is None else (ref, lib.dtype_code(z.dtype))
+    plan = block._plans.get(block, z.dtype, z.device)
+    return None if plan is None else (plan, lib.dtype_code(z.dtype))
 
 
 def _pointers(tensors):
@@ -618,8 +638,8 @@ class PairBlock(_Tracked):
             return False
         N = z.shape[-2]
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
-        plan = self._plans.plan(self, z.numel() // (N * N * z.shape[-1]), N, st[1], flags)
-        lib.pair_block_forward(z, pair_mask, plan, st[1], flags, st[0])
+        plan = st[0].shape(self, z.numel() // (N * N * z.shape[-1]), N, st[1], flags)
+        lib.pair_block_forward(z, pair_mask, plan, st[1], flags, st[0].params)
         return True
 
     def tri_mul_out_in(self, z, pair_mask, inplace_safe, use_cueq_triangle_kernels=False):
@@ -701,8 +721,8 @@ class PairFormerBlock(_Tracked):
         if st is None or s.dtype != z.dtype or s.shape[:-1] != z.shape[:-2]:
             return False
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
-        plan = self._plans.plan(self, z.numel() // (N * N * z.shape[-1]), N, st[1], flags)
-        lib.pairformer_block_forward(s, z, single_mask, pair_mask, plan, st[1], flags, st[0], side)
+        plan = st[0].shape(self, z.numel() // (N * N * z.shape[-1]), N, st[1], flags)
+        lib.pairformer_block_forward(s, z, single_mask, pair_mask, plan, st[1], flags, st[0].params, side)
         return True
 
     def forward(self, s, z, single_mask, pair_mask, chunk_size=None, use_deepspeed_evo_attention=False,
@@ -923,13 +943,13 @@ class DiffusionTransformer(_Tracked):
         biases = self._pair_biases(z, token=st[0])
         flags = (lib.extra_flags | lib.FLAG_ADA_LN) | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
         lib.hold(biases)
-        plan = self._plans.plan(self, ac.shape[0], zc.shape[0], a.shape[-2], st[1], flags, biases[0] is not None)
-        lib.diffusion_stack_forward(ac, sc, zc, m, biases, plan, st[1], flags, st[0])
+        plan = st[0].shape(self, ac.shape[0], zc.shape[0], a.shape[-2], st[1], flags, biases[0] is not None)
+        lib.diffusion_stack_forward(ac, sc, zc, m, biases, plan, st[1], flags, st[0].params)
         return True
 
     def _pair_biases(self, z, token=None):
         """The projected pair bias of every block, or Nones. ``token``: an object that stands for unchanged parameters
-        while it is the same (the native path's parameter structs)."""
+        while it is the same (the native path's plan)."""
         import weakref
 
         try:

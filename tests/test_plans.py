@@ -1,6 +1,9 @@
 """The parameter structs and packed weights that the native block calls work from: built once, kept while what they were
 built from stays the same, built again when it changes. Everything here runs without a GPU (no kernel is called)."""
 
+import sys
+import threading
+
 import torch
 
 CPU, BF = torch.device("cpu"), torch.bfloat16
@@ -43,3 +46,32 @@ def test_a_graph_holds_what_its_capture_read(pkg):
     assert any(h is stack._packed._val for h in held) and inner == ["inner"] and "inner" not in held
     pkg.lib.hold("outside")
     assert "outside" not in held
+
+
+def test_threads_that_share_a_module(pkg):
+    """Two types in turn on several threads, from the first call on: every thread gets a whole plan of its own type."""
+    blk = pkg.PairBlock(c_z=64, c_hidden_mul=64, c_hidden_pair_att=16, no_heads_pair=4, transition_type="swiglu",
+                        transition_n=2, pair_dropout=0.25, fuse_projection_weights=False, inf=1e9).eval().requires_grad_(False)
+    wrong, interval = [], sys.getswitchinterval()
+
+    def work(dtype):
+        try:
+            for _ in range(60):
+                plan = blk._plans.get(blk, dtype, CPU)
+                pointers = [plan.params.tri_mul_in.w_z, plan.params.pair_transition.w_out]
+                mine = [plan.keep[1][9], plan.keep[4][4]]
+                if plan.dtype != dtype or any(t.dtype != dtype for t in mine) or pointers != [t.data_ptr() for t in mine]:
+                    wrong.append("another thread's plan")
+        except Exception as e:   # noqa: BLE001
+            wrong.append(repr(e))
+
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=work, args=(d,)) for d in (BF, torch.float32) * 3]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(interval)
+    assert not wrong, wrong[:3]
