@@ -19,38 +19,20 @@ from functools import partialmethod
 
 import torch
 import torch.nn as nn
+from torch.nn.modules import module as _nn_module
 
 from . import init_config as lin_init
 from . import lib
 
 
 # --------------------------------------------------------------------------- primitives
-_structure_epoch = 0   # counts changes of what a cached block plan was built from (submodules, parameters, constants)
-
-
-class _Tracked(nn.Module):
-    """Base of this package's modules: assigning a public attribute (a submodule, a parameter, a constant such as
-    ``inf``) makes the block plans built so far be built again. Values of parameters are checked at every call."""
-
-    def __setattr__(self, name, value):
-        if name[0] != "_":
-            global _structure_epoch
-            _structure_epoch += 1
-        super().__setattr__(name, value)
-
-    def __delattr__(self, name):
-        global _structure_epoch
-        _structure_epoch += 1
-        super().__delattr__(name)
-
-
 def _trunc_normal_(w: torch.Tensor, scale: float, fan: int):
     # variance-scaled truncated normal on [-2, 2] sigma; 0.8796... is the std of that truncation
     std = math.sqrt(scale / max(1, fan)) / 0.87962566103423978
     nn.init.trunc_normal_(w, mean=0.0, std=std, a=-2.0 * std, b=2.0 * std)
 
 
-class Linear(_Tracked, nn.Linear):
+class Linear(nn.Linear):
     """Parameter holder with the reference's named initialisers
     (openfold3/core/model/primitives/linear.py:38-138). Called alone it is a plain library GEMM."""
 
@@ -84,7 +66,7 @@ class Linear(_Tracked, nn.Linear):
                 raise ValueError("Invalid init string.")
 
 
-class LayerNorm(_Tracked):
+class LayerNorm(nn.Module):
     """Parameter holder (openfold3/core/model/primitives/normalization.py:33-86)."""
 
     def __init__(self, c_in: int, create_scale: bool = True, create_offset: bool = True, eps=1e-5):
@@ -101,7 +83,7 @@ class LayerNorm(_Tracked):
         return nn.functional.layer_norm(x, self.c_in, w, b, self.eps)
 
 
-class AdaLN(_Tracked):
+class AdaLN(nn.Module):
     """Parameter holder for adaptive LayerNorm
     (openfold3/core/model/primitives/normalization.py:89-140); the arithmetic is fused into
     the kernels of the modules that own it."""
@@ -115,7 +97,7 @@ class AdaLN(_Tracked):
         self.linear_s = Linear(c_s, c_a, **linear_init_params.linear_s)
 
 
-class SwiGLU(_Tracked):
+class SwiGLU(nn.Module):
     """Parameter holder (openfold3/core/model/primitives/activations.py:33-61)."""
 
     def __init__(self, c_in: int, c_out: int, linear_init_params=lin_init.swiglu_init):
@@ -125,7 +107,7 @@ class SwiGLU(_Tracked):
         self.linear_b = Linear(c_in, c_out, **linear_init_params.linear_b)
 
 
-class Attention(_Tracked):
+class Attention(nn.Module):
     """Parameter holder for gated multi-head attention
     (openfold3/core/model/primitives/attention.py:199-268). ``c_hidden`` is per head."""
 
@@ -142,7 +124,7 @@ class Attention(_Tracked):
             self.linear_g = Linear(c_q, c_hidden * no_heads, **linear_init_params.linear_g)
 
 
-class DropoutRowwise(_Tracked):
+class DropoutRowwise(nn.Module):
     """Identity in eval mode (openfold3/core/model/primitives/dropout.py:57-58); training-mode
     shared dropout is outside the forward-only scope."""
 
@@ -216,27 +198,43 @@ def _param_watch():
 
 
 class _Plan:
-    """What a native call of a block (or stack) needs, for one dtype and device. Nothing in it changes after it was built
-    but the cache of what depends on the shape."""
+    """What a native call of a block (or stack) needs, for one dtype and device, and the means to tell whether it still
+    holds. Nothing in it changes after it was built but the cache of what depends on the shape.
 
-    __slots__ = ("dtype", "device", "epoch", "hooks", "watch", "params", "keep", "shapes")
+    ``called``: the modules that the layer-by-layer path runs as a caller would, with their hooks; ``layers``: those whose
+    parameters and constants the native path reads."""
 
-    def __init__(self, block, dtype, device):
-        self.dtype, self.device, self.epoch = dtype, device, _structure_epoch
-        self.hooks, self.watch, self.params, self.keep, self.shapes = [], None, None, None, {}
-        plain = block._plan_submodules()
-        if plain is None:
-            return
-        for m in plain:
-            self.hooks += [m._forward_hooks, m._forward_pre_hooks]
-        self.watch = _param_watch().make([(m._parameters, n) for m in block.modules() for n, t in m._parameters.items()
-                                          if t is not None])
-        if self.watch is not None:
+    __slots__ = ("dtype", "device", "hooks", "forwards", "watch", "held", "params", "keep", "shapes")
+
+    def __init__(self, block, called, layers, dtype, device):
+        self.dtype, self.device, self.params, self.keep, self.shapes = dtype, device, None, None, {}
+        self.hooks = [h for m in called for h in (m._forward_hooks, m._forward_pre_hooks)]
+        self.hooks += [_nn_module._global_forward_hooks, _nn_module._global_forward_pre_hooks]
+        self.forwards = [(c, c.forward) for c in {type(m) for m in called}]
+        tree = list(block.modules())
+        owned, children = [m._parameters for m in tree if m._parameters], [m._modules for m in tree if m._modules]
+        attrs = [(m.__dict__, n) for m in layers for n in m._plan_constants]
+        replaced = [(m.__dict__, "forward") for m in called]
+        replaced += [(m.__dict__, n) for m in (block, *called) for n in ("tri_mul_out_in", "tri_att_start_end")
+                     if isinstance(m, PairBlock)]
+        attrs += replaced
+        attrs += [(m.__dict__, "training") for m in called if isinstance(m, DropoutRowwise)]
+        w = _param_watch()
+        found = None
+        known = {id(t) for d in owned for t in d.values()}
+        # (a weight that is not a parameter, computed or a plain tensor, may change unseen: layer by layer)
+        if (not any(n in d for d, n in replaced) and not any("parametrizations" in m._modules for m in tree)
+                and all(t is None or id(t) in known for m in layers for t in m._tensors())):
+            found = w.make(owned, children, attrs)
+        self.watch, self.held = found or w.make([], owned + children, attrs)
+        if found:
             self.params, self.keep = block._native_params(dtype, device)
 
     def current(self, dtype, device):
-        return (dtype == self.dtype and device == self.device and self.epoch == _structure_epoch
-                and (self.watch is None or not _param_watch().changed(self.watch)))
+        return dtype == self.dtype and device == self.device and not _watch_module.changed(self.watch)
+
+    def usable(self):
+        return self.params is not None and not any(self.hooks) and all(c.forward is f for c, f in self.forwards)
 
     def shape(self, block, *key):
         p = self.shapes.get(key)
@@ -248,10 +246,10 @@ class _Plan:
 
 
 class _BlockPlans:
-    """The plan of a block (or stack), built again when a parameter has another address or version, or the module tree
-    another structure, than when it was built. ``get``: ``None`` when the call has to take the layer-by-layer path (hooks on
-    submodules, a submodule that is not this package's, parameters that track no versions). Threads may share a module: each
-    works with the plan that it got."""
+    """The plan of a block (or stack), built again when a parameter has another address or version, a module of the tree
+    other children or parameters, or a constant another value, than when it was built. ``get``: ``None`` when the call has to
+    take the layer-by-layer path (hooks, a submodule that is not this package's or whose ``forward`` was replaced, weights
+    that are not parameters or track no versions). Threads may share a module: each works with the plan that it got."""
 
     _plan = None
 
@@ -261,8 +259,9 @@ class _BlockPlans:
     def get(self, block, dtype, device):
         plan = self._plan
         if plan is None or not plan.current(dtype, device):
-            plan = self._plan = _Plan(block, dtype, device)
-        if plan.params is None or any(plan.hooks):
+            parts = block._plan_submodules()
+            plan = self._plan = None if parts is None else _Plan(block, *parts, dtype, device)
+        if plan is None or not plan.usable():
             return None
         lib.hold(plan.keep)
         return plan
@@ -287,7 +286,7 @@ def _mask_like(mask, shape, dtype):
 
 
 # --------------------------------------------------------------------------- triangle multiplication
-class TriangleMultiplicativeUpdate(_Tracked):
+class TriangleMultiplicativeUpdate(nn.Module):
     """AF3 Algorithms 12/13. Drop-in for
     openfold3/core/model/layers/triangular_multiplicative_update.py:123-503."""
 
@@ -304,11 +303,15 @@ class TriangleMultiplicativeUpdate(_Tracked):
         self.linear_b_g = Linear(c_z, c_hidden, **linear_init_params.linear_b_g)
         self._packed = _PackedParams()
 
+    _plan_constants = ("c_z", "c_hidden", "_outgoing")
+
+    def _tensors(self):
+        return (self.layer_norm_in.weight, self.layer_norm_in.bias, self.linear_a_p.weight,
+                self.linear_a_g.weight, self.linear_b_p.weight, self.linear_b_g.weight, self.linear_g.weight,
+                self.layer_norm_out.weight, self.layer_norm_out.bias, self.linear_z.weight)
+
     def _params(self, dtype, device):
-        return self._packed.get(
-            (self.layer_norm_in.weight, self.layer_norm_in.bias, self.linear_a_p.weight,
-             self.linear_a_g.weight, self.linear_b_p.weight, self.linear_b_g.weight, self.linear_g.weight,
-             self.layer_norm_out.weight, self.layer_norm_out.bias, self.linear_z.weight), dtype, device)
+        return self._packed.get(self._tensors(), dtype, device)
 
     def forward(self, z, mask=None, inplace_safe=False, use_cueq_triangle_kernels=False,
                 _add_with_inplace=False, _inplace_chunk_size=256):
@@ -335,7 +338,7 @@ class TriangleMultiplicationIncoming(TriangleMultiplicativeUpdate):
 
 
 # --------------------------------------------------------------------------- triangle attention
-class TriangleAttention(_Tracked):
+class TriangleAttention(nn.Module):
     """AF3 Algorithms 14/15. Drop-in for openfold3/core/model/layers/triangular_attention.py:30-179."""
 
     def __init__(self, c_in, c_hidden, no_heads, starting=True, inf=1e9, linear_init_params=lin_init.tri_att_init):
@@ -347,11 +350,15 @@ class TriangleAttention(_Tracked):
         self.mha = Attention(c_in, c_in, c_in, c_hidden, no_heads, linear_init_params=linear_init_params.mha)
         self._packed = _PackedParams()
 
+    _plan_constants = ("c_in", "c_hidden", "no_heads", "inf")
+
+    def _tensors(self):
+        return (self.layer_norm.weight, self.layer_norm.bias, self.linear_z.weight, self.mha.linear_q.weight,
+                self.mha.linear_k.weight, self.mha.linear_v.weight, self.mha.linear_g.weight,
+                self.mha.linear_o.weight)
+
     def _params(self, dtype, device):
-        return self._packed.get(
-            (self.layer_norm.weight, self.layer_norm.bias, self.linear_z.weight, self.mha.linear_q.weight,
-             self.mha.linear_k.weight, self.mha.linear_v.weight, self.mha.linear_g.weight,
-             self.mha.linear_o.weight), dtype, device)
+        return self._packed.get(self._tensors(), dtype, device)
 
     def _run(self, x, mask, transposed: bool, in_place: bool):
         N = x.shape[-2]
@@ -380,7 +387,7 @@ class TriangleAttentionEndingNode(TriangleAttention):
 
 
 # --------------------------------------------------------------------------- transitions
-class SwiGLUTransition(_Tracked):
+class SwiGLUTransition(nn.Module):
     """AF3 Algorithm 11. Drop-in for openfold3/core/model/layers/transition.py:225-271."""
 
     def __init__(self, c_in: int, n: int, linear_init_params=lin_init.swiglu_transition_init):
@@ -391,10 +398,14 @@ class SwiGLUTransition(_Tracked):
         self.linear_out = Linear(n * c_in, c_in, **linear_init_params.linear_out)
         self._packed = _PackedParams()
 
+    _plan_constants = ("c_in", "n")
+
+    def _tensors(self):
+        return (self.layer_norm.weight, self.layer_norm.bias, self.swiglu.linear_a.weight,
+                self.swiglu.linear_b.weight, self.linear_out.weight)
+
     def _params(self, dtype, device):
-        return self._packed.get(
-            (self.layer_norm.weight, self.layer_norm.bias, self.swiglu.linear_a.weight,
-             self.swiglu.linear_b.weight, self.linear_out.weight), dtype, device, adjacent=((2, 3),))
+        return self._packed.get(self._tensors(), dtype, device, adjacent=((2, 3),))
 
     def _run(self, x, mask, in_place: bool):
         xc = x.contiguous().view(-1, self.c_in)
@@ -410,7 +421,7 @@ class SwiGLUTransition(_Tracked):
         return self._run(x, mask, in_place=False)
 
 
-class ConditionedTransitionBlock(_Tracked):
+class ConditionedTransitionBlock(nn.Module):
     """AF3 Algorithm 25. Drop-in for openfold3/core/model/layers/transition.py:274-380."""
 
     def __init__(self, c_a: int, c_s: int, n: int, linear_init_params=lin_init.cond_transition_init):
@@ -421,6 +432,8 @@ class ConditionedTransitionBlock(_Tracked):
         self.linear_g = Linear(c_s, c_a, **linear_init_params.linear_g)
         self.linear_out = Linear(n * c_a, c_a, **linear_init_params.linear_out)
         self._packed = _PackedParams()
+
+    _plan_constants = ("c_a", "c_s", "n")
 
     def _tensors(self):
         ln = self.layer_norm
@@ -449,7 +462,7 @@ class ConditionedTransitionBlock(_Tracked):
 
 
 # --------------------------------------------------------------------------- attention with pair bias
-class AttentionPairBias(_Tracked):
+class AttentionPairBias(nn.Module):
     """AF3 Algorithm 24. Drop-in for openfold3/core/model/layers/attention_pair_bias.py:33-227."""
 
     def __init__(self, c_q, c_k, c_v, c_s, c_z, c_hidden, no_heads, use_ada_layer_norm=False, gating=True,
@@ -473,6 +486,8 @@ class AttentionPairBias(_Tracked):
         self.mha = Attention(c_q, c_k, c_v, c_hidden, no_heads, gating=gating,
                              linear_init_params=linear_init_params.mha)
         self._packed = _PackedParams()
+
+    _plan_constants = ("c_q", "c_s", "c_z", "c_hidden", "no_heads", "inf", "use_ada_layer_norm")
 
     def _tensors(self):
         if self.use_ada_layer_norm:
@@ -578,7 +593,7 @@ class AttentionPairBias(_Tracked):
 
 
 # --------------------------------------------------------------------------- blocks and stacks
-class PairBlock(_Tracked):
+class PairBlock(nn.Module):
     """Pair stack of one block. Drop-in for openfold3/core/model/latent/base_blocks.py:219-480."""
 
     def __init__(self, c_z, c_hidden_mul, c_hidden_pair_att, no_heads_pair, transition_type, transition_n,
@@ -603,19 +618,19 @@ class PairBlock(_Tracked):
         self._plans = _BlockPlans()
 
     def _plan_submodules(self):
-        """The submodules whose hooks the layer-by-layer path runs, or None if one is not this package's own."""
+        """(called, layers) of ``_Plan``, or None if the layers are not this package's own or do not fit together."""
         own = {"tri_mul_out": TriangleMultiplicationOutgoing, "tri_mul_in": TriangleMultiplicationIncoming,
                "tri_att_start": TriangleAttention, "tri_att_end": TriangleAttention, "pair_transition": SwiGLUTransition,
                "ps_dropout_row_layer": DropoutRowwise}
         if type(self) is not PairBlock or any(type(self._modules.get(n)) is not c for n, c in own.items()):
             return None
-        dims = {(m.c_z, m.c_hidden) for m in (self.tri_mul_out, self.tri_mul_in)}
-        att = {(m.c_in, m.c_hidden, m.no_heads, m.inf) for m in (self.tri_att_start, self.tri_att_end)}
-        if len(dims) != 1 or len(att) != 1 or self.tri_mul_in._outgoing or not self.tri_mul_out._outgoing:
+        mul, att = (self.tri_mul_out, self.tri_mul_in), (self.tri_att_start, self.tri_att_end)
+        widths = {m.c_z for m in mul} | {m.c_in for m in att} | {self.pair_transition.c_in}
+        if len(widths) != 1 or len({m.c_hidden for m in mul}) != 1 or len({(m.c_hidden, m.no_heads, m.inf) for m in att}) != 1:
             return None
-        if self.ps_dropout_row_layer.training:
+        if self.tri_mul_in._outgoing or not self.tri_mul_out._outgoing or self.ps_dropout_row_layer.training:
             return None
-        return [self.tri_mul_out, self.tri_mul_in, self.ps_dropout_row_layer]
+        return [*mul, self.ps_dropout_row_layer], [*mul, *att, self.pair_transition]
 
     def _native_params(self, dtype, device):
         parts = [m._params(dtype, device) for m in (self.tri_mul_out, self.tri_mul_in, self.tri_att_start,
@@ -673,7 +688,7 @@ class PairBlock(_Tracked):
         return z
 
 
-class PairFormerBlock(_Tracked):
+class PairFormerBlock(nn.Module):
     """Block of AF3 Algorithm 17. Drop-in for openfold3/core/model/latent/pairformer.py:38-213."""
 
     def __init__(self, c_s, c_z, c_hidden_pair_bias, no_heads_pair_bias, c_hidden_mul, c_hidden_pair_att,
@@ -697,10 +712,10 @@ class PairFormerBlock(_Tracked):
         own = {"pair_stack": PairBlock, "attn_pair_bias": AttentionPairBias, "single_transition": SwiGLUTransition}
         if type(self) is not PairFormerBlock or any(type(self._modules.get(n)) is not c for n, c in own.items()):
             return None
-        inner = self.pair_stack._plan_submodules()
-        if inner is None or self.attn_pair_bias.use_ada_layer_norm:
+        inner, attn, trans = self.pair_stack._plan_submodules(), self.attn_pair_bias, self.single_transition
+        if inner is None or attn.use_ada_layer_norm or attn.c_z != self.pair_stack.tri_mul_in.c_z or trans.c_in != attn.c_q:
             return None
-        return [self.pair_stack, *inner]
+        return [self.pair_stack, *inner[0]], [*inner[1], attn, trans]
 
     def _native_params(self, dtype, device):
         pair, keep = self.pair_stack._native_params(dtype, device)
@@ -745,7 +760,7 @@ class PairFormerBlock(_Tracked):
         return s, z
 
 
-class PairFormerStack(_Tracked):
+class PairFormerStack(nn.Module):
     """AF3 Algorithm 17. Drop-in for openfold3/core/model/latent/pairformer.py:217-464."""
 
     def __init__(self, c_s, c_z, c_hidden_pair_bias, no_heads_pair_bias, c_hidden_mul, c_hidden_pair_att,
@@ -806,7 +821,7 @@ class PairFormerStack(_Tracked):
         return s, z
 
 
-class PairStack(_Tracked):
+class PairStack(nn.Module):
     """Consecutive ``PairBlock``s applied to one pair tensor: the "pair stack only" workloads. The reference has no
     class for it; its callers keep a ``nn.ModuleList`` of ``PairBlock``s and call them in sequence with the same
     pair mask (openfold3/core/model/latent/template_module.py:148-189), which is what ``forward`` does.
@@ -835,7 +850,7 @@ class PairStack(_Tracked):
         return z
 
 
-class DiffusionTransformerBlock(_Tracked):
+class DiffusionTransformerBlock(nn.Module):
     """AF3 Algorithm 23 block. Drop-in for openfold3/core/model/layers/diffusion_transformer.py:30-179
     (the ``n_query is None`` token-level branch)."""
 
@@ -865,7 +880,7 @@ class DiffusionTransformerBlock(_Tracked):
         return a
 
 
-class DiffusionTransformer(_Tracked):
+class DiffusionTransformer(nn.Module):
     """AF3 Algorithm 23. Drop-in for openfold3/core/model/layers/diffusion_transformer.py:182-322."""
 
     def __init__(self, c_a, c_s, c_z, c_hidden, no_heads, no_blocks, n_transition, use_ada_layer_norm,
@@ -904,7 +919,9 @@ class DiffusionTransformer(_Tracked):
                   b.attention_pair_bias.use_ada_layer_norm, b.conditioned_transition.c_a, b.conditioned_transition.c_s,
                   b.conditioned_transition.n) for b in blocks}
         k = next(iter(kinds))
-        return blocks if len(kinds) == 1 and k[0] == k[7] and k[1] == k[8] else None
+        if len(kinds) != 1 or k[0] != k[7] or k[1] != k[8]:
+            return None
+        return blocks, [m for b in blocks for m in (b.attention_pair_bias, b.conditioned_transition)]
 
     def _native_params(self, dtype, device):
         """Parameter structs of all blocks. The projections of s lie back to back over the whole stack (the library

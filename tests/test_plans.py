@@ -4,6 +4,7 @@ built from stays the same, built again when it changes. Everything here runs wit
 import sys
 import threading
 
+import pytest
 import torch
 
 CPU, BF = torch.device("cpu"), torch.bfloat16
@@ -75,3 +76,89 @@ def test_threads_that_share_a_module(pkg):
     finally:
         sys.setswitchinterval(interval)
     assert not wrong, wrong[:3]
+
+
+def pair_block(pkg):
+    return pkg.PairBlock(c_z=64, c_hidden_mul=64, c_hidden_pair_att=16, no_heads_pair=4, transition_type="swiglu",
+                         transition_n=2, pair_dropout=0.25, fuse_projection_weights=False, inf=1e9).eval().requires_grad_(False)
+
+
+def test_an_unchanged_module_keeps_its_plan(pkg):
+    stack = diffusion(pkg)
+    plan = params(stack)
+    stack.eval()
+    stack.hoist_pair_bias = False
+    pkg.LayerNorm(8).eval()
+    assert plan is not None and params(stack) is plan
+
+
+EDITS = {
+    "replaced block": lambda s, o: s.blocks.__setitem__(0, o.blocks[0]),
+    "deleted block": lambda s, o: s.blocks.__delitem__(-1),
+    "appended block": lambda s, o: s.blocks.append(o.blocks[0]),
+    "inserted block": lambda s, o: s.blocks.insert(1, o.blocks[0]),
+    "swapped blocks": lambda s, o: s._modules["blocks"]._modules.update({"0": s.blocks[1], "1": s.blocks[0]}),
+    "another layer": lambda s, o: s.blocks[1].add_module("conditioned_transition", o.blocks[1].conditioned_transition),
+    "another linear": lambda s, o: setattr(s.blocks[1].attention_pair_bias.mha, "linear_o",
+                                           o.blocks[1].attention_pair_bias.mha.linear_o),
+    "another parameter": lambda s, o: s.blocks[1].conditioned_transition.linear_out.register_parameter(
+        "weight", torch.nn.Parameter(o.blocks[1].conditioned_transition.linear_out.weight.clone(), requires_grad=False)),
+}
+
+
+@pytest.mark.parametrize("edit", list(EDITS))
+def test_edits_of_the_module_tree_are_seen(pkg, edit):
+    """After the edit the structs say what those of a stack made that way say."""
+    stack, other = diffusion(pkg), diffusion(pkg)
+    params(stack, torch.float32)
+    EDITS[edit](stack, other)
+    plan = params(stack, torch.float32)
+    assert len(plan.params[0]) == len(stack.blocks)
+    for n, b in enumerate(stack.blocks):   # fp32 parameters are read where they are
+        assert plan.params[0][n].w_o == b.attention_pair_bias.mha.linear_o.weight.data_ptr()
+        assert plan.params[1][n].w_out == b.conditioned_transition.linear_out.weight.data_ptr()
+
+
+@pytest.mark.parametrize("change", ["inf", "c_hidden", "training"])
+def test_changed_constants_are_seen(pkg, change):
+    blk = pair_block(pkg)
+    plan = blk._plans.get(blk, BF, CPU)
+    if change == "inf":
+        blk.tri_att_start.inf = blk.tri_att_end.inf = 1e8
+        assert blk._plans.get(blk, BF, CPU).shape(blk, 1, 8, 0, 0).dims.inf_pair == 1e8
+    elif change == "c_hidden":   # the two directions no longer agree
+        blk.tri_mul_in.c_hidden = 32
+        assert blk._plans.get(blk, BF, CPU) is None
+    else:
+        blk.ps_dropout_row_layer.train()
+        assert blk._plans.get(blk, BF, CPU) is None
+    assert plan is not blk._plans._plan
+
+
+@pytest.mark.parametrize("how", ["instance", "class", "hook", "global hook", "plain tensor", "computed"])
+def test_what_the_native_call_would_pass_by_takes_the_layer_path(pkg, how, monkeypatch):
+    blk = pair_block(pkg)
+    assert blk._plans.get(blk, BF, CPU) is not None
+    seen = lambda *a, **k: None  # noqa: E731
+    if how == "instance":
+        blk.tri_mul_in.forward = seen
+    elif how == "class":
+        monkeypatch.setattr(pkg.TriangleMultiplicationIncoming, "forward", seen)
+    elif how == "hook":
+        blk.tri_mul_out.register_forward_hook(seen)
+    elif how == "global hook":
+        handle = torch.nn.modules.module.register_module_forward_hook(seen)
+    elif how == "plain tensor":   # may be written to without a trace in the module's parameters
+        lin = blk.pair_transition.linear_out
+        w = lin.weight.data
+        del lin.weight
+        lin.weight = w
+    else:
+        torch.nn.utils.parametrize.register_parametrization(blk.tri_att_end.linear_z, "weight", torch.nn.Identity())
+    try:
+        assert blk._plans.get(blk, BF, CPU) is None and blk._plans.get(blk, BF, CPU) is None
+    finally:
+        if how == "global hook":
+            handle.remove()
+            assert blk._plans.get(blk, BF, CPU) is not None
+
