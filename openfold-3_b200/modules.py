@@ -279,10 +279,26 @@ def _pointers(tensors):
     return [None if t is None else t.data_ptr() for t in tensors]
 
 
-def _mask_like(mask, shape, dtype):
+def _same_device(like, **others):
+    """The kernels take addresses: a tensor of another device, or of the host, must not get that far."""
+    for name, t in others.items():
+        if t is not None and t.device != like.device:
+            raise RuntimeError(f"{name} is on {t.device}, the call's tensors are on {like.device}")
+
+
+def _mask_like(mask, x):
+    """mask [*] for x [*, C], broadcast, in the dtype of x."""
     if mask is None:
         return None
-    return mask.to(dtype).expand(shape).contiguous()
+    _same_device(x, mask=mask)
+    return mask.to(x.dtype).expand(x.shape[:-1]).contiguous()
+
+
+def _pair_batch(z, c_z):
+    """B of a pair tensor z [*, N, N, c_z], or None if z is no such tensor (or empty)."""
+    if z.dim() < 3 or z.shape[-3] != z.shape[-2] or z.shape[-1] != c_z or z.numel() == 0:
+        return None
+    return z.numel() // (z.shape[-2] * z.shape[-2] * c_z)
 
 
 # --------------------------------------------------------------------------- triangle multiplication
@@ -321,7 +337,7 @@ class TriangleMultiplicativeUpdate(nn.Module):
         in_place = inplace_safe and _add_with_inplace and not use_cueq_triangle_kernels and z.is_contiguous()
         N = z.shape[-2]
         zc = z.contiguous().view(-1, N, N, self.c_z)
-        m = _mask_like(mask, z.shape[:-1], z.dtype)
+        m = _mask_like(mask, z)
         m = None if m is None else m.view(-1, N, N)
         out = zc if in_place else torch.empty_like(zc)
         lib.trimul_forward(zc, m, out, self._params(z.dtype, z.device), self.c_hidden, self._outgoing,
@@ -363,7 +379,7 @@ class TriangleAttention(nn.Module):
     def _run(self, x, mask, transposed: bool, in_place: bool):
         N = x.shape[-2]
         xc = x.contiguous().view(-1, N, N, self.c_in)
-        m = _mask_like(mask, x.shape[:-1], x.dtype)
+        m = _mask_like(mask, x)
         m = None if m is None else m.view(-1, N, N)
         out = xc if in_place else torch.empty_like(xc)
         lib.triattn_forward(xc, m, out, self._params(x.dtype, x.device), self.no_heads, self.c_hidden,
@@ -409,7 +425,7 @@ class SwiGLUTransition(nn.Module):
 
     def _run(self, x, mask, in_place: bool):
         xc = x.contiguous().view(-1, self.c_in)
-        m = _mask_like(mask, x.shape[:-1], x.dtype)
+        m = _mask_like(mask, x)
         m = None if m is None else m.view(-1)
         out = xc if in_place else torch.empty_like(xc)
         lib.transition_forward(xc, m, out, self._params(x.dtype, x.device), self.n, add_residual=in_place)
@@ -447,9 +463,10 @@ class ConditionedTransitionBlock(nn.Module):
         return self._packed.get(self._tensors(), dtype, device, adjacent=(self._cond_group, (4, 5)))
 
     def _run(self, a, s, mask, in_place: bool):
+        _same_device(a, s=s)
         ac = a.contiguous().view(-1, self.c_a)
         sc = s.expand(*a.shape[:-1], self.c_s).contiguous().view(-1, self.c_s)
-        m = _mask_like(mask, a.shape[:-1], a.dtype)
+        m = _mask_like(mask, a)
         m = None if m is None else m.view(-1)
         out = ac if in_place else torch.empty_like(ac)
         lib.cond_transition_forward(ac, sc, m, out, self._params(a.dtype, a.device), self.n,
@@ -530,9 +547,17 @@ class AttentionPairBias(nn.Module):
             return lib.pair_bias_project_tiles(zc, prm[8], prm[9], prm[10])
         return lib.pair_bias_project(zc, prm[8], prm[9], prm[10])
 
+    def _bias_fits(self, bias, zc):
+        """Whether ``bias`` is what ``project_pair_bias`` makes of a pair tensor of the shape of zc [Bz, N, N, C_z]."""
+        Bz, N = zc.shape[:2]
+        if bias.dtype == torch.bfloat16:
+            return bias.shape == (Bz, 16, (N + 31) // 32, N, 32)
+        return bias.dtype == torch.float32 and bias.shape == (Bz, self.no_heads, N, N)
+
     def _operands(self, a, z, s, mask):
         """a [Ba, N, C], z [Bz, N, N, C_z], s, mask as the kernels take them: samples that share a pair tensor are
         consecutive."""
+        _same_device(a, z=z, s=s)
         N = a.shape[-2]
         batch = a.shape[:-2]
         ac = a.contiguous().view(-1, N, self.c_q)
@@ -551,7 +576,7 @@ class AttentionPairBias(nn.Module):
             if s is None:
                 raise ValueError("AttentionPairBias with adaptive LayerNorm needs s")
             sc = s.expand(*batch, N, self.c_s).contiguous().view(-1, N, self.c_s)
-        m = _mask_like(mask, a.shape[:-1], a.dtype)
+        m = _mask_like(mask, a)
         m = None if m is None else m.view(-1, N)
         assert ac.shape[0] % zc.shape[0] == 0
         return ac, zc, sc, m
@@ -567,16 +592,15 @@ class AttentionPairBias(nn.Module):
                 a.add_(upd.to(a.dtype))
                 return a
             return upd.to(a.dtype)
-        N = a.shape[-2]
         ac, zc, sc, m = self._operands(a, z, s, mask)
         out = ac if in_place else torch.empty_like(ac)
         if pair_bias is not None and pair_bias.dtype == torch.bfloat16:   # bias tiles of the tensor-core attention
-            assert pair_bias.shape == (zc.shape[0], 16, (N + 31) // 32, N, 32) and a.dtype == torch.bfloat16
+            assert self._bias_fits(pair_bias, zc) and a.dtype == torch.bfloat16
             lib.attn_pair_bias_forward_pretiles(ac, pair_bias, sc, m, out, self._params(a.dtype, a.device),
                                                 self.no_heads, self.c_hidden, self.inf, self.use_ada_layer_norm,
                                                 add_residual=in_place)
         elif pair_bias is not None:
-            assert pair_bias.shape == (zc.shape[0], self.no_heads, N, N) and pair_bias.dtype == torch.float32
+            assert self._bias_fits(pair_bias, zc)
             lib.attn_pair_bias_forward_prebias(ac, pair_bias, sc, m, out, self._params(a.dtype, a.device),
                                                self.no_heads, self.c_hidden, self.inf, self.use_ada_layer_norm,
                                                add_residual=in_place)
@@ -649,11 +673,11 @@ class PairBlock(nn.Module):
     def _run_native(self, z, pair_mask, mask_trans):
         """In place on the contiguous z with the prepared mask; False if the native path does not take this call."""
         st = _native_state(self, z)
-        if st is None:
+        B = None if st is None else _pair_batch(z, self.tri_mul_out.c_z)
+        if B is None:   # (what has another shape is for the layers to refuse)
             return False
-        N = z.shape[-2]
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
-        plan = st[0].shape(self, z.numel() // (N * N * z.shape[-1]), N, st[1], flags)
+        plan = st[0].shape(self, B, z.shape[-2], st[1], flags)
         lib.pair_block_forward(z, pair_mask, plan, st[1], flags, st[0].params)
         return True
 
@@ -678,7 +702,7 @@ class PairBlock(nn.Module):
         _forward_only(self, z)
         self.ps_dropout_row_layer(z)  # raises in training mode with a non-zero rate
         z = z if inplace_safe and z.is_contiguous() else z.clone(memory_format=torch.contiguous_format)
-        pair_mask = _mask_like(pair_mask, z.shape[:-1], z.dtype)
+        pair_mask = _mask_like(pair_mask, z)
         if self._run_native(z, pair_mask, _mask_trans):
             return z
         z = self.tri_mul_out_in(z, pair_mask, inplace_safe=True)
@@ -732,11 +756,12 @@ class PairFormerBlock(nn.Module):
     def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None):
         """In place on contiguous s and z with prepared masks; False if the native path does not take this call."""
         st = _native_state(self, z)
-        N = z.shape[-2]
-        if st is None or s.dtype != z.dtype or s.shape[:-1] != z.shape[:-2]:
+        attn = self.attn_pair_bias
+        B = None if st is None else _pair_batch(z, attn.c_z)
+        if B is None or s.dtype != z.dtype or s.shape[:-1] != z.shape[:-2] or s.shape[-1] != attn.c_q:
             return False
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
-        plan = st[0].shape(self, z.numel() // (N * N * z.shape[-1]), N, st[1], flags)
+        plan = st[0].shape(self, B, z.shape[-2], st[1], flags)
         lib.pairformer_block_forward(s, z, single_mask, pair_mask, plan, st[1], flags, st[0].params, side)
         return True
 
@@ -745,11 +770,12 @@ class PairFormerBlock(nn.Module):
                 _attn_chunk_size=None):
         _forward_only(self, s, z)
         if z.is_cuda and not self.training:
+            _same_device(z, s=s)
             z = z if inplace_safe and z.is_contiguous() else z.clone(memory_format=torch.contiguous_format)
             s = s if inplace_safe and s.is_contiguous() else s.clone(memory_format=torch.contiguous_format)
             inplace_safe = True
-            pair_mask = _mask_like(pair_mask, z.shape[:-1], z.dtype)
-            single_mask = _mask_like(single_mask, s.shape[:-1], s.dtype)
+            pair_mask = _mask_like(pair_mask, z)
+            single_mask = _mask_like(single_mask, s)
             if self._run_native(s, z, single_mask, pair_mask, _mask_trans):
                 return s, z
         z = self.pair_stack(z=z, pair_mask=pair_mask, chunk_size=chunk_size, inplace_safe=inplace_safe,
@@ -792,8 +818,9 @@ class PairFormerStack(nn.Module):
         if not (inplace_safe and s.is_contiguous()):
             s = s.clone(memory_format=torch.contiguous_format)
         if z.is_cuda:   # prepared once for all blocks
-            pair_mask = _mask_like(pair_mask, z.shape[:-1], z.dtype)
-            single_mask = _mask_like(single_mask, s.shape[:-1], s.dtype)
+            _same_device(z, s=s)
+            pair_mask = _mask_like(pair_mask, z)
+            single_mask = _mask_like(single_mask, s)
         if not (self.overlap_single_track and z.is_cuda and len(self.blocks) > 1
                 and self.blocks[0].attn_pair_bias.can_hoist_pair_bias(z)):
             for b in self.blocks:
@@ -844,7 +871,7 @@ class PairStack(nn.Module):
         if not (inplace_safe and z.is_contiguous()):
             z = z.clone(memory_format=torch.contiguous_format)
         if z.is_cuda:   # prepared once for all blocks
-            pair_mask = _mask_like(pair_mask, z.shape[:-1], z.dtype)
+            pair_mask = _mask_like(pair_mask, z)
         for b in self.blocks:
             z = b(z, pair_mask, inplace_safe=True, _mask_trans=_mask_trans)
         return z
@@ -958,6 +985,8 @@ class DiffusionTransformer(nn.Module):
             return False
         ac, zc, sc, m = m0._operands(a, z, s, mask)
         biases = self._pair_biases(z, token=st[0])
+        if ac.numel() == 0 or not all(b is None or m0._bias_fits(b, zc) for b in biases):
+            return False   # (for the layers to refuse)
         flags = (lib.extra_flags | lib.FLAG_ADA_LN) | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
         lib.hold(biases)
         plan = st[0].shape(self, ac.shape[0], zc.shape[0], a.shape[-2], st[1], flags, biases[0] is not None)

@@ -1,0 +1,93 @@
+"""What the native block calls are given: tensors of other shapes or devices than the kernels read are refused on the host,
+as the layers refuse them. The library calls are recorded instead of made; nothing here needs a GPU."""
+
+import pytest
+import torch
+
+from cases import DIFF, OF3, _PF_KW
+
+BF = torch.bfloat16
+
+
+class OnGpu(torch.Tensor):
+    """A host tensor that passes for a CUDA one."""
+
+    is_cuda = property(lambda self: True)
+
+
+def gpu(*shape, dtype=BF):
+    return torch.zeros(shape, dtype=dtype).as_subclass(OnGpu)
+
+
+@pytest.fixture
+def calls(pkg, monkeypatch):
+    made = []
+    for name in ("pair_block_forward", "pairformer_block_forward", "diffusion_stack_forward", "trimul_forward",
+                 "triattn_forward", "transition_forward", "attn_pair_bias_forward", "attn_pair_bias_forward_pretiles",
+                 "attn_pair_bias_forward_prebias", "cond_transition_forward"):
+        monkeypatch.setattr(pkg.lib, name, lambda *a, _n=name, **k: made.append(_n))
+    monkeypatch.setattr(pkg.lib, "pair_bias_project_tiles",
+                        lambda z, *p: torch.zeros(z.shape[0], 16, (z.shape[1] + 31) // 32, z.shape[1], 32, dtype=BF))
+    return made
+
+
+@pytest.fixture(scope="module")
+def block(pkg):
+    return pkg.PairFormerBlock(**OF3, **_PF_KW).eval().to(BF).requires_grad_(False)
+
+
+@pytest.fixture(scope="module")
+def diffusion(pkg):
+    return pkg.DiffusionTransformer(**DIFF, no_blocks=2, use_ada_layer_norm=True, n_query=None, n_key=None,
+                                    inf=1e9).eval().to(BF).requires_grad_(False)
+
+
+def test_good_shapes_take_one_native_call(block, diffusion, calls):
+    with torch.no_grad():
+        block.pair_stack(gpu(1, 20, 20, 128), None)
+        block(gpu(2, 20, 384), gpu(2, 20, 20, 128), None, None)
+        diffusion(gpu(1, 3, 20, 768), gpu(1, 3, 20, 384), gpu(1, 1, 20, 20, 128))
+    assert calls == ["pair_block_forward", "pairformer_block_forward", "diffusion_stack_forward"]
+
+
+@pytest.mark.parametrize("z", [(1, 20, 20, 64), (1, 30, 20, 128), (1, 20, 30, 128), (0, 20, 20, 128), (20, 128)])
+def test_pair_block_refuses_other_pair_tensors(block, calls, z):
+    with torch.no_grad():
+        try:
+            block.pair_stack(gpu(*z), None)
+        except (RuntimeError, IndexError, AssertionError):
+            pass
+    assert "pair_block_forward" not in calls
+
+
+@pytest.mark.parametrize("s,z", [((1, 20, 128), (1, 20, 20, 128)), ((1, 20, 384), (1, 20, 20, 64)),
+                                 ((1, 20, 384), (1, 20, 40, 128)), ((1, 10, 384), (1, 20, 20, 128))])
+def test_pairformer_block_refuses_other_tensors(block, calls, s, z):
+    with torch.no_grad():
+        try:
+            block(gpu(*s), gpu(*z), None, None)
+        except (RuntimeError, AssertionError):
+            pass
+    assert "pairformer_block_forward" not in calls
+
+
+def test_kept_biases_of_another_batch_are_refused(diffusion, calls):
+    """Samples [2, 5] with pair tensors [1, 5]: the expanded pair tensor has ten entries, the kept biases five."""
+    with torch.no_grad(), pytest.raises(AssertionError):
+        diffusion(gpu(2, 5, 20, 768), gpu(2, 5, 20, 384), gpu(1, 5, 20, 20, 128))
+    assert calls == []
+
+
+def test_tensors_of_another_device_are_refused(block, diffusion, calls):
+    far = lambda *shape: torch.zeros(shape, dtype=BF, device="meta")  # noqa: E731
+    a, s, z = gpu(1, 2, 20, 768), gpu(1, 2, 20, 384), gpu(1, 1, 20, 20, 128)
+    with torch.no_grad():
+        for call in (lambda: block(far(1, 20, 384), gpu(1, 20, 20, 128), None, None),
+                     lambda: block(gpu(1, 20, 384), gpu(1, 20, 20, 128), far(1, 20), None),
+                     lambda: block.pair_stack(gpu(1, 20, 20, 128), far(1, 20, 20)),
+                     lambda: diffusion(a, far(1, 2, 20, 384), z),
+                     lambda: diffusion(a, s, far(1, 1, 20, 20, 128)),
+                     lambda: diffusion(a, s, z, mask=far(1, 2, 20))):
+            with pytest.raises(RuntimeError, match="is on meta"):
+                call()
+    assert calls == []
