@@ -929,7 +929,8 @@ class DiffusionTransformer(nn.Module):
         # 0.45 GB at N = 768; fp32 [*, H, N, N] for fp32 inputs) for as long as the caller passes the same, unmodified z; set to False to recompute them
         # in every call (what the reference does).
         self.hoist_pair_bias = True
-        self._bias_cache = None   # (weakref to z, z._version, parameter versions, [bias per block])
+        # (weakref to z, its version and address, (parameters, their addresses and versions), [bias per block], plan)
+        self._bias_cache = None
         self._plans = _BlockPlans()
         self._packed = _PackedParams()
 
@@ -1002,6 +1003,7 @@ class DiffusionTransformer(nn.Module):
             zv = z._version
         except RuntimeError:   # inference tensors do not track versions: nothing to key the cache on
             zv = None
+        zv = None if zv is None else (zv, z.data_ptr())
         c = self._bias_cache
         if (self.hoist_pair_bias and token is not None and c is not None and c[4] is token and c[0]() is z
                 and c[1] == zv and lib.extra_flags == 0):
@@ -1011,13 +1013,14 @@ class DiffusionTransformer(nn.Module):
             return [None] * len(apbs)
         if zv is None:
             return [m.project_pair_bias(z) for m in apbs]
-        pv = tuple((m.layer_norm_z.weight._version, m.linear_z.weight._version, m.linear_z.weight.data_ptr())
-                   for m in apbs)
-        if c is not None and c[0]() is z and c[1] == zv and c[2] == pv:
+        used = [t for m in apbs for t in (m.layer_norm_z.weight, m.layer_norm_z.bias, m.linear_z.weight) if t is not None]
+        pv = [(t.data_ptr(), t._version) for t in used]
+        if (c is not None and c[0]() is z and c[1] == zv and c[2][1] == pv and len(c[2][0]) == len(used)
+                and all(a is b for a, b in zip(c[2][0], used))):
             biases = c[3]
         else:
             biases = [m.project_pair_bias(z) for m in apbs]
-        self._bias_cache = (weakref.ref(z), zv, pv, biases, token)
+        self._bias_cache = (weakref.ref(z), zv, (used, pv), biases, token)
         return biases
 
     def forward(self, a, s, z, mask=None, use_deepspeed_evo_attention=False, use_cueq_triangle_kernels=False,

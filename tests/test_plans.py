@@ -162,3 +162,28 @@ def test_what_the_native_call_would_pass_by_takes_the_layer_path(pkg, how, monke
             handle.remove()
             assert blk._plans.get(blk, BF, CPU) is not None
 
+
+
+@pytest.mark.parametrize("change", ["layer_norm_z.weight", "layer_norm_z.bias", "linear_z.weight", "z", "data of z"])
+def test_kept_pair_biases_are_projected_again(pkg, monkeypatch, change):
+    """For new parameters (a new one starts at version 0, as the old one did) and new values of the pair tensor."""
+    stack = diffusion(pkg)
+    apb = stack.blocks[1].attention_pair_bias
+    projected = []
+    monkeypatch.setattr(pkg.AttentionPairBias, "can_hoist_pair_bias", lambda self, z: True)
+    monkeypatch.setattr(pkg.AttentionPairBias, "project_pair_bias", lambda self, z: projected.append(self) or z)
+    z = torch.zeros(1, 4, 4, 128)
+    token = params(stack, torch.float32)
+    first = stack._pair_biases(z, token)
+    assert stack._pair_biases(z, token) is first and len(projected) == 3
+    if change == "z":
+        z.add_(1)
+    elif change == "data of z":
+        z.data = torch.ones(1, 4, 4, 128)
+    else:
+        layer, name = change.split(".")
+        shape = (16, 128) if layer == "linear_z" else (128,)
+        setattr(getattr(apb, layer), name, torch.nn.Parameter(torch.ones(shape), requires_grad=False))
+    del projected[:]
+    assert stack._pair_biases(z, params(stack, torch.float32)) is not first and len(projected) == 3
+    assert stack._pair_biases(z) is not first and len(projected) == 3   # the layer path finds the new ones
