@@ -907,6 +907,14 @@ class DiffusionTransformerBlock(nn.Module):
         return a
 
 
+class _KeptBiases(tuple):
+    """The entry of ``DiffusionTransformer._bias_cache``. It stands for one pair tensor of this process: a copied or
+    unpickled stack starts without."""
+
+    def __reduce__(self):
+        return (type(None), ())
+
+
 class DiffusionTransformer(nn.Module):
     """AF3 Algorithm 23. Drop-in for openfold3/core/model/layers/diffusion_transformer.py:182-322."""
 
@@ -1020,7 +1028,7 @@ class DiffusionTransformer(nn.Module):
             biases = c[3]
         else:
             biases = [m.project_pair_bias(z) for m in apbs]
-        self._bias_cache = (weakref.ref(z), zv, (used, pv), biases, token)
+        self._bias_cache = _KeptBiases((weakref.ref(z), zv, (used, pv), biases, token))
         return biases
 
     def forward(self, a, s, z, mask=None, use_deepspeed_evo_attention=False, use_cueq_triangle_kernels=False,

@@ -1,6 +1,8 @@
 """The parameter structs and packed weights that the native block calls work from: built once, kept while what they were
 built from stays the same, built again when it changes. Everything here runs without a GPU (no kernel is called)."""
 
+import copy
+import pickle
 import sys
 import threading
 
@@ -187,3 +189,17 @@ def test_kept_pair_biases_are_projected_again(pkg, monkeypatch, change):
     del projected[:]
     assert stack._pair_biases(z, params(stack, torch.float32)) is not first and len(projected) == 3
     assert stack._pair_biases(z) is not first and len(projected) == 3   # the layer path finds the new ones
+
+
+@pytest.mark.parametrize("how", [copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))], ids=["deepcopy", "pickle"])
+def test_a_used_module_can_be_copied(pkg, monkeypatch, how):
+    """The copy packs its own weights, keeps no biases and has a plan of its own."""
+    stack = diffusion(pkg)
+    monkeypatch.setattr(pkg.AttentionPairBias, "can_hoist_pair_bias", lambda self, z: True)
+    monkeypatch.setattr(pkg.AttentionPairBias, "project_pair_bias", lambda self, z: z)
+    plan = params(stack)
+    stack._pair_biases(torch.zeros(1, 4, 4, 128), plan)
+    twin = how(stack)
+    assert twin._bias_cache is None and stack._bias_cache is not None
+    assert twin._packed._val is None and params(twin) is not plan and params(stack) is plan
+    assert params(twin).params[1][0].w_out != plan.params[1][0].w_out
