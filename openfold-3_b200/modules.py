@@ -267,6 +267,15 @@ class _BlockPlans:
         return plan
 
 
+class _Planned(nn.Module):
+    """Base of the modules that have a native call."""
+
+    def __setstate__(self, state):   # (a module pickled before it had one)
+        super().__setstate__(state)
+        self.__dict__.setdefault("_plans", _BlockPlans())
+        self.__dict__.setdefault("_packed", _PackedParams())
+
+
 def _native_state(block, z):
     """(plan, dtype code) for the native path of ``block`` on z, or None."""
     if not z.is_cuda or block.training or z.dtype not in (torch.bfloat16, torch.float32):
@@ -617,7 +626,7 @@ class AttentionPairBias(nn.Module):
 
 
 # --------------------------------------------------------------------------- blocks and stacks
-class PairBlock(nn.Module):
+class PairBlock(_Planned):
     """Pair stack of one block. Drop-in for openfold3/core/model/latent/base_blocks.py:219-480."""
 
     def __init__(self, c_z, c_hidden_mul, c_hidden_pair_att, no_heads_pair, transition_type, transition_n,
@@ -712,7 +721,7 @@ class PairBlock(nn.Module):
         return z
 
 
-class PairFormerBlock(nn.Module):
+class PairFormerBlock(_Planned):
     """Block of AF3 Algorithm 17. Drop-in for openfold3/core/model/latent/pairformer.py:38-213."""
 
     def __init__(self, c_s, c_z, c_hidden_pair_bias, no_heads_pair_bias, c_hidden_mul, c_hidden_pair_att,
@@ -915,7 +924,7 @@ class _KeptBiases(tuple):
         return (type(None), ())
 
 
-class DiffusionTransformer(nn.Module):
+class DiffusionTransformer(_Planned):
     """AF3 Algorithm 23. Drop-in for openfold3/core/model/layers/diffusion_transformer.py:182-322."""
 
     def __init__(self, c_a, c_s, c_z, c_hidden, no_heads, no_blocks, n_transition, use_ada_layer_norm,

@@ -203,3 +203,15 @@ def test_a_used_module_can_be_copied(pkg, monkeypatch, how):
     assert twin._bias_cache is None and stack._bias_cache is not None
     assert twin._packed._val is None and params(twin) is not plan and params(stack) is plan
     assert params(twin).params[1][0].w_out != plan.params[1][0].w_out
+
+
+def test_modules_pickled_without_plans(pkg):
+    """As a build that had no native calls pickled them."""
+    stack = diffusion(pkg)
+    for name in ("_plans", "_packed"):
+        del stack.__dict__[name]
+    blk = pair_block(pkg)
+    del blk.__dict__["_plans"]
+    assert params(pickle.loads(pickle.dumps(stack))) is not None
+    blk = pickle.loads(pickle.dumps(blk))
+    assert blk._plans.get(blk, BF, CPU) is not None
