@@ -335,6 +335,9 @@ int of3_attn_pair_bias_forward_prebias(const void* a, const float* pair_bias, co
  * of a batch lie back to back -- and the layer taking tiles [Bz][...]. A caller that applies the layer many
  * times to one pair tensor (a diffusion rollout) keeps the tiles. */
 long long of3_pair_bias_tiles_elems(int N);
+/* 1 if the layer's projected pair bias is taken as tiles (of3_attn_pair_bias_forward_pretiles, and the `bias` of
+ * of3_diffusion_stack_forward), 0 if as fp32 [Bz, H, N, N]. */
+int of3_pair_bias_takes_tiles(int N, int c_a, int c_s, int c_z, int H, int d, int dtype, int flags);
 int of3_pair_bias_project_tiles(const void* z, const void* ln_w, const void* ln_b, const void* w, void* tiles, int N,
                                 int c_z, int H, int dtype, void* stream);
 int of3_attn_pair_bias_forward_pretiles(const void* a, const void* bias_tiles, const void* s, const void* mask,

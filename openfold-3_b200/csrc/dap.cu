@@ -199,6 +199,10 @@ int of3_attn_pair_bias_forward_prebias(const void* a, const float* pair_bias, co
 
 long long of3_pair_bias_tiles_elems(int N) { return 16LL * ((N + 31) / 32) * N * 32; }
 
+int of3_pair_bias_takes_tiles(int N, int c_a, int c_s, int c_z, int H, int d, int dtype, int flags) {
+    return dtype == OF3_DTYPE_BF16 && fast::attn_pair_bias_supported(1, 1, N, c_a, c_s, c_z, H, d, flags) ? 1 : 0;
+}
+
 int of3_pair_bias_project_tiles(const void* z, const void* ln_w, const void* ln_b, const void* w, void* tiles, int N,
                                 int c_z, int H, int dtype, void* stream) {
     OF3_REQUIRE(z && w && tiles, OF3_ERR_ARG, "pair_bias_project_tiles: null pointer argument");

@@ -123,6 +123,7 @@ SIGNATURES = {
                                                    ctypes.POINTER(AttnPairBiasParams), c_void_p, c_size_t,
                                                    c_void_p]),
     "of3_pair_bias_tiles_elems": (c_longlong, [c_int]),
+    "of3_pair_bias_takes_tiles": (c_int, [c_int] * 8),
     "of3_pair_bias_project_tiles": (c_int, [c_void_p] * 5 + [c_int, c_int, c_int, c_int, c_void_p]),
     "of3_attn_pair_bias_forward_pretiles": (c_int, [c_void_p] * 5 + [c_int] * 7 + [c_float, c_int, c_int,
                                                     ctypes.POINTER(AttnPairBiasParams), c_void_p, c_size_t,

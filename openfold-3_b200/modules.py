@@ -539,10 +539,12 @@ class AttentionPairBias(nn.Module):
                 and z.dtype in (torch.bfloat16, torch.float32) and lib.extra_flags == 0)
 
     def _takes_bias_tiles(self, z) -> bool:
-        """bf16 on the tensor-core attention: the projection can be written as that kernel's own bias tiles."""
-        return (z.dtype == torch.bfloat16 and self.c_hidden in (24, 48) and self.c_q == 16 * self.c_hidden
-                and self.c_q % 64 == 0 and (not self.use_ada_layer_norm or self.c_s % 64 == 0)
-                and z.shape[-2] <= 8192)
+        """The attention is the tensor-core one, which takes the projection as its own bias tiles: the library's answer,
+        since the library reads them."""
+        flags = lib.extra_flags | (lib.FLAG_ADA_LN if self.use_ada_layer_norm else 0)
+        return bool(lib.load().of3_pair_bias_takes_tiles(z.shape[-2], self.c_q, self.c_s if self.use_ada_layer_norm else 0,
+                                                         self.c_z, self.no_heads, self.c_hidden, lib.dtype_code(z.dtype),
+                                                         flags))
 
     def project_pair_bias(self, z):
         """linear_z(LayerNorm_z(z)): the part of this layer that depends on z only (openfold3/core/model/layers/

@@ -55,3 +55,25 @@ def test_a_hook_takes_the_layer_path():
         h.remove()
         blk(s, z, None, None)
     assert seen == [z.shape]
+
+
+def test_kept_biases_where_the_attention_is_the_generic_one():
+    """c_s beyond the tensor-core layer's limit: the kept biases are fp32 tensors, read as such. Against the call that projects
+    its own: the same kernels but for the projection, whose operands are bf16 in one and fp32 in the other (2^-9 per product,
+    on a bias of order one in front of a softmax; the update is some 0.3 of the output): the bar of one bf16 block, 8e-3."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator().manual_seed(4)
+    st = pkg.DiffusionTransformer(c_a=768, c_s=2112, c_z=128, c_hidden=48, no_heads=16, no_blocks=1, n_transition=2,
+                                  use_ada_layer_norm=True, n_query=None, n_key=None, inf=1e9)
+    with torch.no_grad():
+        for p in st.parameters():
+            p.copy_(torch.randn(p.shape, generator=g) * (p.shape[-1] ** -0.5 if p.dim() > 1 else 0.1))
+    st = st.to(dev, bf).eval().requires_grad_(False)
+    a, s, z = (torch.randn(sh, generator=g).to(dev, bf) for sh in ((1, 2, 33, 768), (1, 2, 33, 2112), (1, 1, 33, 33, 128)))
+    with torch.no_grad():
+        kept = st(a, s, z)
+        assert st._bias_cache[3][0].dtype == torch.float32
+        st.hoist_pair_bias = False
+        own = st(a, s, z)
+    pkg.lib.check_device_status()
+    assert ((kept - own).float().norm() / own.float().norm()).item() < 8e-3

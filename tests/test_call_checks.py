@@ -91,3 +91,22 @@ def test_tensors_of_another_device_are_refused(block, diffusion, calls):
             with pytest.raises(RuntimeError, match="is on meta"):
                 call()
     assert calls == []
+
+
+@pytest.mark.parametrize("c_s,N,dtype", [(384, 20, BF), (384, 8192, BF), (384, 8193, BF), (2048, 20, BF), (2112, 20, BF),
+                                         (100, 20, BF), (384, 20, torch.float32)])
+def test_the_projected_bias_has_the_form_that_the_library_reads(pkg, monkeypatch, c_s, N, dtype):
+    """Sizes around the limits of the tensor-core attention and of its adaptive LayerNorm: bias tiles read as fp32 biases are
+    half as long as what is read."""
+    apb = pkg.AttentionPairBias(c_q=768, c_k=768, c_v=768, c_s=c_s, c_z=128, c_hidden=48, no_heads=16,
+                                use_ada_layer_norm=True)
+    made = []
+    monkeypatch.setattr(pkg.lib, "pair_bias_project_tiles", lambda *a: made.append("tiles"))
+    monkeypatch.setattr(pkg.lib, "pair_bias_project", lambda *a: made.append("f32"))
+    apb.project_pair_bias(torch.empty(1, N, N, 128, dtype=dtype, device="meta"))
+    lib = pkg.lib.load()
+    code, flags = pkg.lib.dtype_code(dtype), pkg.lib.FLAG_ADA_LN
+    fast = dtype == BF and c_s % 64 == 0 and c_s <= 2048 and N <= 8192
+    assert made == ["tiles" if fast else "f32"]
+    assert lib.of3_pair_bias_takes_tiles(N, 768, c_s, 128, 16, 48, code, flags) == fast
+    assert lib.of3_pair_bias_takes_tiles(N, 768, c_s, 128, 16, 48, code, flags | pkg.lib.FLAG_FORCE_GENERIC) == 0
