@@ -553,10 +553,12 @@ class AttentionPairBias(nn.Module):
         [*, H, N, N], or for bf16 inputs the attention kernel's own bf16 bias tiles [*, 16, N / 32, N, 32]."""
         N = z.shape[-2]
         zc = z.contiguous().view(-1, N, N, self.c_z)
-        prm = self._params(z.dtype, z.device)
+        # three tensors only: the copies of the whole layer would stand beside those of a stack's native call
+        packed = self.__dict__.setdefault("_packed_z", _PackedParams())
+        prm = packed.get((self.layer_norm_z.weight, self.layer_norm_z.bias, self.linear_z.weight), z.dtype, z.device)
         if self._takes_bias_tiles(z):
-            return lib.pair_bias_project_tiles(zc, prm[8], prm[9], prm[10])
-        return lib.pair_bias_project(zc, prm[8], prm[9], prm[10])
+            return lib.pair_bias_project_tiles(zc, *prm)
+        return lib.pair_bias_project(zc, *prm)
 
     def _bias_fits(self, bias, zc):
         """Whether ``bias`` is what ``project_pair_bias`` makes of a pair tensor of the shape of zc [Bz, N, N, C_z]."""

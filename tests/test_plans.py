@@ -215,3 +215,16 @@ def test_modules_pickled_without_plans(pkg):
     assert params(pickle.loads(pickle.dumps(stack))) is not None
     blk = pickle.loads(pickle.dumps(blk))
     assert blk._plans.get(blk, BF, CPU) is not None
+
+
+def test_projecting_pair_biases_packs_no_second_copy_of_the_layer(pkg, monkeypatch):
+    stack = diffusion(pkg)
+    monkeypatch.setattr(pkg.AttentionPairBias, "can_hoist_pair_bias", lambda self, z: True)
+    got = []
+    monkeypatch.setattr(pkg.lib, "pair_bias_project", lambda z, *prm: got.append(prm))
+    stack._pair_biases(torch.zeros(1, 4, 4, 128), params(stack, torch.float32))
+    for b, prm in zip(stack.blocks, got):
+        apb = b.attention_pair_bias
+        assert apb._packed._val is None
+        assert all(torch.equal(x, y) for x, y in zip(prm, (apb.layer_norm_z.weight, apb.layer_norm_z.bias, apb.linear_z.weight))
+                   if x is not None)
