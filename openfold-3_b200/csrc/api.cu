@@ -112,9 +112,7 @@ int of3_trimul_forward(const void* z, const void* mask, void* out, int B, int N,
     CHECK_DTYPE(dtype);
     OF3_REQUIRE(z && out && p && workspace, OF3_ERR_ARG, "trimul: null pointer argument");
     OF3_REQUIRE(B > 0 && N > 0 && c_z > 0 && c_h > 0, OF3_ERR_ARG, "trimul: non-positive size");
-    OF3_REQUIRE(p->ln_in_w && p->ln_in_b && p->w_a_p && p->w_a_g && p->w_b_p && p->w_b_g && p->w_g &&
-                    p->ln_out_w && p->ln_out_b && p->w_z,
-                OF3_ERR_ARG, "trimul: null parameter pointer");
+    OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "trimul: null parameter pointer");
     Arena ws(workspace, workspace_bytes);
     return trimul_dispatch(z, mask, out, B, N, c_z, c_h, dtype, flags, p, ws, (cudaStream_t)stream);
 }
@@ -132,8 +130,7 @@ int of3_triattn_forward(const void* z, const void* mask, void* out, int B, int N
     CHECK_DTYPE(dtype);
     OF3_REQUIRE(z && out && p && workspace, OF3_ERR_ARG, "triattn: null pointer argument");
     OF3_REQUIRE(B > 0 && N > 0 && c_z > 0 && H > 0 && d > 0, OF3_ERR_ARG, "triattn: non-positive size");
-    OF3_REQUIRE(p->ln_w && p->ln_b && p->w_bias && p->w_q && p->w_k && p->w_v && p->w_g && p->w_o,
-                OF3_ERR_ARG, "triattn: null parameter pointer");
+    OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "triattn: null parameter pointer");
     Arena ws(workspace, workspace_bytes);
     return triattn_dispatch(z, mask, out, B, N, c_z, H, d, inf, dtype, flags, p, ws,
                             (cudaStream_t)stream);
@@ -151,8 +148,7 @@ int of3_transition_forward(const void* x, const void* mask, void* out, long long
     CHECK_DTYPE(dtype);
     OF3_REQUIRE(x && out && p && workspace, OF3_ERR_ARG, "transition: null pointer argument");
     OF3_REQUIRE(rows > 0 && c > 0 && n > 0, OF3_ERR_ARG, "transition: non-positive size");
-    OF3_REQUIRE(p->ln_w && p->ln_b && p->w_a && p->w_b && p->w_out, OF3_ERR_ARG,
-                "transition: null parameter pointer");
+    OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "transition: null parameter pointer");
     Arena ws(workspace, workspace_bytes);
     return transition_dispatch(x, mask, out, rows, c, n, dtype, flags, p, ws, (cudaStream_t)stream);
 }
@@ -206,9 +202,7 @@ int of3_cond_transition_forward(const void* a, const void* s, const void* mask, 
     CHECK_DTYPE(dtype);
     OF3_REQUIRE(a && s && out && p && workspace, OF3_ERR_ARG, "cond_transition: null pointer argument");
     OF3_REQUIRE(rows > 0 && c_a > 0 && c_s > 0 && n > 0, OF3_ERR_ARG, "cond_transition: non-positive size");
-    OF3_REQUIRE(p->ada_ln_s_w && p->ada_w_g && p->ada_b_g && p->ada_w_s && p->w_a && p->w_b && p->w_g &&
-                    p->b_g && p->w_out,
-                OF3_ERR_ARG, "cond_transition: null parameter pointer");
+    OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "cond_transition: null parameter pointer");
     Arena ws(workspace, workspace_bytes);
     return cond_dispatch(a, s, mask, out, rows, c_a, c_s, n, dtype, flags, p, ws, (cudaStream_t)stream);
 }

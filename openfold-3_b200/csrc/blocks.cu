@@ -229,6 +229,10 @@ bool dims_ok(const of3_block_dims* d) {
 bool single_dims_ok(const of3_block_dims* d) {
     return d->c_s > 0 && d->no_heads_single > 0 && d->c_hidden_single > 0 && d->single_transition_n > 0;
 }
+bool complete_block(const of3_pair_block_params& p) {
+    return complete(p.tri_mul_out) && complete(p.tri_mul_in) && complete(p.tri_att_start) && complete(p.tri_att_end) &&
+           complete(p.pair_transition);
+}
 #define CHECK_BLOCK(what)                                                                                        \
     OF3_REQUIRE(dtype == OF3_DTYPE_BF16 || dtype == OF3_DTYPE_F32, OF3_ERR_ARG, what ": bad dtype %d", dtype);    \
     OF3_REQUIRE(dims_ok(dims), OF3_ERR_ARG, what ": non-positive size")
@@ -253,6 +257,7 @@ int of3_pair_block_forward(void* z, const void* pair_mask, const of3_block_dims*
                            const of3_pair_block_params* p, void* workspace, size_t workspace_bytes, void* stream) {
     CHECK_BLOCK("pair_block");
     OF3_REQUIRE(z && p && workspace, OF3_ERR_ARG, "pair_block: null pointer argument");
+    OF3_REQUIRE(complete_block(*p), OF3_ERR_ARG, "pair_block: null parameter pointer");
     Scratch ws{workspace, workspace_bytes};
     return pair_block(z, pair_mask, *dims, dtype, flags, p, ws, (cudaStream_t)stream);
 }
@@ -280,6 +285,8 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
     CHECK_BLOCK("pairformer_block");
     OF3_REQUIRE(single_dims_ok(dims), OF3_ERR_ARG, "pairformer_block: non-positive single-track size");
     OF3_REQUIRE(s && z && p && workspace && side_workspace, OF3_ERR_ARG, "pairformer_block: null pointer argument");
+    OF3_REQUIRE(complete_block(p->pair) && complete(p->attn, false, true) && complete(p->single_transition), OF3_ERR_ARG,
+                "pairformer_block: null parameter pointer");
     cudaStream_t main = (cudaStream_t)stream;
     const BiasForm form = bias_form(*dims, dtype, flags);
     const size_t tail = bias_bytes(*dims, form);
@@ -324,6 +331,10 @@ int of3_diffusion_stack_forward(void* a, const void* s, const void* z, const voi
     OF3_REQUIRE(diffusion_dims_ok(dims) && blocks > 0, OF3_ERR_ARG, "diffusion_stack: bad sizes");
     OF3_REQUIRE(a && s && (z || bias) && attn && transition && workspace, OF3_ERR_ARG,
                 "diffusion_stack: null pointer argument");
+    for (int b = 0; b < blocks; ++b)
+        OF3_REQUIRE(complete(attn[b], (flags & OF3_FLAG_ADA_LN) != 0, bias == nullptr) && complete(transition[b]) &&
+                        (bias == nullptr || bias[b] != nullptr),
+                    OF3_ERR_ARG, "diffusion_stack: null parameter pointer (block %d)", b);
     Scratch ws{workspace, workspace_bytes};
     return diffusion_stack(a, s, z, mask, bias, *dims, dtype, flags, blocks, attn, transition, ws, (cudaStream_t)stream);
 }

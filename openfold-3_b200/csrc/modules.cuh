@@ -83,6 +83,23 @@ int transition_wide(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bflo
                     int n, int flags, const of3_transition_params* p, Arena& ws, cudaStream_t st);
 }  // namespace fast
 
+// No parameter that the kernels read without asking is null (the optional ones: ln_z_b, b_q).
+inline bool complete(const of3_trimul_params& p) {
+    return p.ln_in_w && p.ln_in_b && p.w_a_p && p.w_a_g && p.w_b_p && p.w_b_g && p.w_g && p.ln_out_w && p.ln_out_b && p.w_z;
+}
+inline bool complete(const of3_triattn_params& p) {
+    return p.ln_w && p.ln_b && p.w_bias && p.w_q && p.w_k && p.w_v && p.w_g && p.w_o;
+}
+inline bool complete(const of3_transition_params& p) { return p.ln_w && p.ln_b && p.w_a && p.w_b && p.w_out; }
+inline bool complete(const of3_cond_transition_params& p) {
+    return p.ada_ln_s_w && p.ada_w_g && p.ada_b_g && p.ada_w_s && p.w_a && p.w_b && p.w_g && p.b_g && p.w_out;
+}
+// (the bias projection's parameters: only where the layer projects its own pair bias)
+inline bool complete(const of3_attn_pair_bias_params& p, bool ada, bool projects) {
+    if (!(p.w_q && p.w_k && p.w_v && p.w_g && p.w_o) || (projects && !(p.ln_z_w && p.w_z))) return false;
+    return ada ? p.ada_ln_s_w && p.ada_w_g && p.ada_b_g && p.ada_w_s && p.w_ada_out && p.b_ada_out : p.ln_a_w && p.ln_a_b;
+}
+
 // Kernel-family selection behind the module entry points (api.cu); with ws.base == nullptr they only measure the
 // workspace.
 int trimul_dispatch(const void* z, const void* mask, void* out, int B, int N, int c_z, int c_h, int dtype, int flags,

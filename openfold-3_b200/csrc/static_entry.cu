@@ -61,9 +61,7 @@ extern "C" int of3_trimul_forward_static(const void* z, const void* mask, void* 
                 "dtype %d is neither OF3_DTYPE_BF16 nor OF3_DTYPE_F32", dtype);
     OF3_REQUIRE(z && out && p, OF3_ERR_ARG, "trimul_static: null pointer argument");
     OF3_REQUIRE(B > 0 && N > 0 && c_z > 0 && c_h > 0, OF3_ERR_ARG, "trimul_static: non-positive size");
-    OF3_REQUIRE(p->ln_in_w && p->ln_in_b && p->w_a_p && p->w_a_g && p->w_b_p && p->w_b_g && p->w_g &&
-                    p->ln_out_w && p->ln_out_b && p->w_z,
-                OF3_ERR_ARG, "trimul_static: null parameter pointer");
+    OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "trimul_static: null parameter pointer");
     // size the chain first (no device work), reject what does not fit
     Arena probe(nullptr, 0);
     int rc = dtype == OF3_DTYPE_BF16

@@ -104,3 +104,50 @@ def test_modules_pack_grouped_weights_back_to_back(pkg):
     prm = tr._params(dt, dev)
     assert prm[3].data_ptr() - prm[2].data_ptr() == 4 * 384 * 384 * 2
     assert torch.equal(prm[3], tr.swiglu.linear_b.weight.to(dt))
+
+
+def _filled(struct):
+    """A parameter struct of addresses that nobody reads: the calls below are refused before the first launch."""
+    s = struct()
+    for name, kind in struct._fields_:
+        setattr(s, name, 4096 if kind is ctypes.c_void_p else _filled(kind))
+    return s
+
+
+def _pointer_fields(struct, prefix=()):
+    for name, kind in struct._fields_:
+        if kind is ctypes.c_void_p:
+            yield (*prefix, name)
+        else:
+            yield from _pointer_fields(kind, (*prefix, name))
+
+
+def test_block_entry_points_refuse_null_parameters(pkg):
+    """Every parameter that the kernels read without asking, as the layers' own entry points refuse them."""
+    L, lib = pkg.lib, pkg.lib.load()
+    dims = L.BlockDims(1, 8, 128, 128, 4, 32, 4, 384, 16, 24, 4, 1e9, 1e9)
+    diff = L.DiffusionDims(1, 1, 8, 768, 384, 128, 16, 48, 2, 1e9)
+    ref = ctypes.byref
+    calls = {
+        L.PairBlockParams: lambda p: lib.of3_pair_block_forward(4096, None, ref(dims), 0, 0, ref(p), 4096, 1 << 40, None),
+        L.PairformerBlockParams: lambda p: lib.of3_pairformer_block_forward(4096, 4096, None, None, ref(dims), 0, 0, ref(p),
+                                                                            4096, 1 << 40, 4096, 1 << 40, None, None),
+        L.AttnPairBiasParams: lambda p: lib.of3_diffusion_stack_forward(
+            4096, 4096, 4096, None, None, ref(diff), 0, L.FLAG_ADA_LN, 1, ref(p), ref(_filled(L.CondTransitionParams)), 4096,
+            1 << 40, None),
+        L.CondTransitionParams: lambda p: lib.of3_diffusion_stack_forward(
+            4096, 4096, 4096, None, None, ref(diff), 0, L.FLAG_ADA_LN, 1, ref(_filled(L.AttnPairBiasParams)), ref(p), 4096,
+            1 << 40, None),
+    }
+    optional = {"b_q", "ln_z_b"}
+    for struct, call in calls.items():
+        unused = optional | ({"ln_a_w", "ln_a_b"} if struct is L.AttnPairBiasParams else set())
+        for path in _pointer_fields(struct):
+            if path[-1] in unused or ("attn" in path and ("ada" in path[-1])):
+                continue
+            p = _filled(struct)
+            owner = p
+            for name in path[:-1]:
+                owner = getattr(owner, name)
+            setattr(owner, path[-1], None)
+            assert call(p) == -1 and b"null parameter" in lib.of3_last_error_string(), path
