@@ -846,18 +846,20 @@ class PairFormerStack(nn.Module):
         main = torch.cuda.current_stream(z.device)
         side = lib.side_stream(main)
         lib.stream_wait(side, main)
-        for b in self.blocks:
-            if b._run_native(s, z, single_mask, pair_mask, _mask_trans, side):
-                continue
-            z = b.pair_stack(z=z, pair_mask=pair_mask, chunk_size=chunk_size, inplace_safe=True,
-                             _mask_trans=_mask_trans)
-            bias = b.attn_pair_bias.project_pair_bias(z)
-            bias.record_stream(side)   # allocated on the main stream, last read on the second one
-            lib.stream_wait(side, main)
-            with torch.cuda.stream(side):
-                b.attn_pair_bias._run(s, z, None, single_mask, in_place=True, pair_bias=bias)
-                b.single_transition._run(s, single_mask if _mask_trans else None, in_place=True)
-        lib.stream_wait(main, side)
+        try:
+            for b in self.blocks:
+                if b._run_native(s, z, single_mask, pair_mask, _mask_trans, side):
+                    continue
+                z = b.pair_stack(z=z, pair_mask=pair_mask, chunk_size=chunk_size, inplace_safe=True,
+                                 _mask_trans=_mask_trans)
+                bias = b.attn_pair_bias.project_pair_bias(z)
+                bias.record_stream(side)   # allocated on the main stream, last read on the second one
+                lib.stream_wait(side, main)
+                with torch.cuda.stream(side):
+                    b.attn_pair_bias._run(s, z, None, single_mask, in_place=True, pair_bias=bias)
+                    b.single_transition._run(s, single_mask if _mask_trans else None, in_place=True)
+        finally:   # also on the way out of an error: s and the masks belong to the main stream
+            lib.stream_wait(main, side)
         return s, z
 
 

@@ -110,3 +110,22 @@ def test_the_projected_bias_has_the_form_that_the_library_reads(pkg, monkeypatch
     assert made == ["tiles" if fast else "f32"]
     assert lib.of3_pair_bias_takes_tiles(N, 768, c_s, 128, 16, 48, code, flags) == fast
     assert lib.of3_pair_bias_takes_tiles(N, 768, c_s, 128, 16, 48, code, flags | pkg.lib.FLAG_FORCE_GENERIC) == 0
+
+
+def test_a_failed_stack_call_still_joins_the_second_stream(pkg, calls, monkeypatch):
+    """The blocks before the failure have work on it that reads and writes tensors of the main stream."""
+    stack = pkg.PairFormerStack(**OF3, **_PF_KW, no_blocks=3, blocks_per_ckpt=None).eval().to(BF).requires_grad_(False)
+    waits = []
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: "main")
+    monkeypatch.setattr(pkg.lib, "side_stream", lambda main: "side")
+    monkeypatch.setattr(pkg.lib, "stream_wait", lambda waiter, signaler: waits.append((waiter, signaler)))
+
+    def call(*args):
+        calls.append("block")
+        if len(calls) == 2:
+            raise RuntimeError("second block")
+
+    monkeypatch.setattr(pkg.lib, "pairformer_block_forward", call)
+    with torch.no_grad(), pytest.raises(RuntimeError, match="second block"):
+        stack(gpu(1, 20, 384), gpu(1, 20, 20, 128), None, None)
+    assert calls == ["block", "block"] and waits == [("side", "main"), ("main", "side")]
