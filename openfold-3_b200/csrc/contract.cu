@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(192, 1)
 contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    __nv_bfloat16* __restrict__ out, int M, int N, int K, int batch,
                    long long out_batch_stride, int ldo, int rows_per_block, long long row_block_stride,
-                   int a_shared, int chan_shift, long long out_sample_stride, int wide, int* status) {
+                   int a_shared, int chan_shift, long long out_sample_stride, int wide_cols, int* status) {
     using Cfg = ContractCfg<BN>;
     constexpr int S = Cfg::kStages;
     extern __shared__ uint8_t smem_raw[];
@@ -200,7 +200,7 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                         for (int e = 0; e < 8; ++e)
                             o[e] = pack_bf16x2(__uint_as_float(r[g * 16 + 2 * e]), __uint_as_float(r[g * 16 + 2 * e + 1]));
                         if (col < N) {
-                            if (wide) {
+                            if (col + 16 <= wide_cols) {
                                 stg256(orow + col, o);
                             } else {
                                 *reinterpret_cast<uint4*>(orow + col) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -263,11 +263,14 @@ int launch_contract(const CUtensorMap& tmA, const CUtensorMap& tmB, const Contra
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
     int* status = device_status_ptr();
     LaunchScope scope(account_as, stream);  // launch accounting: the triangle einsum or a plain linear layer
-    const int wide = o.ld % 16 == 0 && o.batch_stride % 16 == 0 && o.row_block_stride % 16 == 0 &&
-                     o.sample_stride % 16 == 0 && ((uintptr_t)o.out & 31) == 0;
+    // 16 columns per store, up to the last column that is the output's: a general output ends at N rounded up to 8 (what lies
+    // behind it in the pitch is the caller's), the blocked one has its whole pitch to itself
+    const bool wide = o.ld % 16 == 0 && o.batch_stride % 16 == 0 && o.row_block_stride % 16 == 0 &&
+                      o.sample_stride % 16 == 0 && ((uintptr_t)o.out & 31) == 0;
+    const int wide_cols = !wide ? 0 : (o.chan_shift == 31 ? (int)align_up(N, 8) : o.ld);
     OF3_CUDA_CHECK(launch_chained(contract_nt_kernel<BN>, grid, 192, Cfg::kSmemBytes, stream, tmA, tmB, o.out, M, N, K, batch,
                                   o.batch_stride, o.ld, o.rows_per_block, o.row_block_stride, a_shared ? 1 : 0, o.chan_shift,
-                                  o.sample_stride, wide, status));
+                                  o.sample_stride, wide_cols, status));
     return OF3_OK;
 }
 

@@ -31,3 +31,23 @@ def test_triangle_update_matches_the_oracle(dims, B, N, outgoing):
     pkg.lib.check_device_status()
     got = got.float().cpu()
     assert rms_err(got, ref) < 8e-3 and rel_err(got, ref) < 8e-2, (rms_err(got, ref), rel_err(got, ref))
+
+
+@pytest.mark.parametrize("N", [8, 16, 20, 24, 40, 136, 200, 264])
+def test_the_contraction_leaves_the_rest_of_the_pitch_alone(N):
+    """Columns from N rounded up to 8 on belong to the caller (another result, or nothing: the last row may end the buffer),
+    whatever width the pitch would allow a store."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator().manual_seed(N)
+    M, K, batch, used = 130, 72, 3, (N + 7) // 8 * 8
+    ldo = (N + 15) // 16 * 16 + 16
+    a = torch.randn(batch, M, K, generator=g).to(dev, bf)
+    b = torch.randn(batch, N, K, generator=g).to(dev, bf)
+    whole = torch.full((batch, M, ldo), 7.0, dtype=bf, device=dev)
+    pkg.lib.contract_nt_bf16(a, b, whole)
+    torch.cuda.synchronize()
+    pkg.lib.check_device_status()
+    assert (whole[..., used:] == 7).all()
+    ref = torch.einsum("bik,bjk->bij", a.double(), b.double())
+    # operands as given, fp32 sums of 72 products, one rounding to bf16: 2^-9 relative and some 1e-6 of the sum's terms
+    assert ((whole[..., :N].double() - ref).abs() <= 2**-8 * ref.abs() + 1e-4).all()
