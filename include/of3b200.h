@@ -47,6 +47,7 @@ extern "C" {
 #define OF3_FLAG_OUTGOING 4    /* trimul: outgoing edges (else incoming) */
 #define OF3_FLAG_TRANSPOSED 8  /* triangle attention around the ending node */
 #define OF3_FLAG_ADA_LN 16     /* attention pair bias: adaptive LayerNorm conditioning on s */
+#define OF3_FLAG_CONTINUES 64  /* blocks: see of3_pair_block_forward */
 #define OF3_FLAG_NO_TRANSITION_MASK 32 /* blocks: the transitions ignore the mask (_mask_trans = False) */
 
 /* Message for the last non-zero return code seen by the calling thread. */
@@ -64,7 +65,9 @@ int of3_device_status_async(int* host4, void* stream);
  * come from a pool that grows on demand). of3_profile_read synchronises the device and returns the
  * launches since the last reset and the summed device time of the timed ones.
  * Kernel ids: 1 triangle contraction, 2 trimul projection/gate, 3 trimul output, 4 SwiGLU
- * transition, 5 attention projection, 6 attention core, 7 attention output, 20 generic kernels. */
+ * transition, 5 attention projection, 6 attention core, 7 attention output, 8 single-track rows, 9 pair-bias
+ * projection, 10 linear layers, 11 single-track attention core, 20 generic kernels; 0 those of all of them that were
+ * launched to start under the end of the kernel ahead of them in the stream (count only). */
 int of3_profile_enable(int on);
 int of3_profile_reset(void);
 int of3_profile_read(int kernel_id, long long* launches, float* total_ms);
@@ -225,6 +228,9 @@ int of3_cond_transition_forward(const void* a, const void* s, const void* mask, 
  * language takes longer than they run).
  * of3_pair_block_forward replaces PairBlock.forward (openfold3/core/model/latent/base_blocks.py:406-480), in place on
  * z [B, N, N, c_z]; pair_mask [B, N, N] or NULL.
+ * OF3_FLAG_CONTINUES (block calls): the last work enqueued on stream is another block call, and nothing has written
+ * this block's parameters since before that one; the block's first kernel then starts under the end of the previous
+ * block's last one, as the kernels inside a block do. Without it (always right) it starts after all work before it.
  * of3_pairformer_block_forward replaces PairFormerBlock.forward (openfold3/core/model/latent/pairformer.py:124-213), in
  * place on z and s [B, N, c_s]; single_mask [B, N] or NULL. With side_stream != NULL (and widths for which the pair-bias
  * projection has a kernel of its own: c_z = 128, 16 heads) the single track runs on side_stream behind the pair stack

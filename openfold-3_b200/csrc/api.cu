@@ -1,5 +1,6 @@
 // extern "C" entry points: argument checks, kernel-family selection, workspace sizing.
 #include "modules.cuh"
+#include "runtime.cuh"
 
 namespace of3 {
 
@@ -113,6 +114,7 @@ int of3_trimul_forward(const void* z, const void* mask, void* out, int B, int N,
     OF3_REQUIRE(z && out && p && workspace, OF3_ERR_ARG, "trimul: null pointer argument");
     OF3_REQUIRE(B > 0 && N > 0 && c_z > 0 && c_h > 0, OF3_ERR_ARG, "trimul: non-positive size");
     OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "trimul: null parameter pointer");
+    CallScope call;
     Arena ws(workspace, workspace_bytes);
     return trimul_dispatch(z, mask, out, B, N, c_z, c_h, dtype, flags, p, ws, (cudaStream_t)stream);
 }
@@ -131,6 +133,7 @@ int of3_triattn_forward(const void* z, const void* mask, void* out, int B, int N
     OF3_REQUIRE(z && out && p && workspace, OF3_ERR_ARG, "triattn: null pointer argument");
     OF3_REQUIRE(B > 0 && N > 0 && c_z > 0 && H > 0 && d > 0, OF3_ERR_ARG, "triattn: non-positive size");
     OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "triattn: null parameter pointer");
+    CallScope call;
     Arena ws(workspace, workspace_bytes);
     return triattn_dispatch(z, mask, out, B, N, c_z, H, d, inf, dtype, flags, p, ws,
                             (cudaStream_t)stream);
@@ -149,6 +152,7 @@ int of3_transition_forward(const void* x, const void* mask, void* out, long long
     OF3_REQUIRE(x && out && p && workspace, OF3_ERR_ARG, "transition: null pointer argument");
     OF3_REQUIRE(rows > 0 && c > 0 && n > 0, OF3_ERR_ARG, "transition: non-positive size");
     OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "transition: null parameter pointer");
+    CallScope call;
     Arena ws(workspace, workspace_bytes);
     return transition_dispatch(x, mask, out, rows, c, n, dtype, flags, p, ws, (cudaStream_t)stream);
 }
@@ -182,6 +186,7 @@ int of3_attn_pair_bias_forward(const void* a, const void* z, const void* s, cons
     }
     OF3_REQUIRE(p->ln_z_w && p->w_z && p->w_q && p->w_k && p->w_v && p->w_g && p->w_o, OF3_ERR_ARG,
                 "attn_pair_bias: null parameter pointer");
+    CallScope call;
     Arena ws(workspace, workspace_bytes);
     return apb_dispatch(a, z, s, mask, out, Ba, Bz, N, c_a, c_s, c_z, H, d, inf, dtype, flags, p, ws,
                         (cudaStream_t)stream);
@@ -203,6 +208,7 @@ int of3_cond_transition_forward(const void* a, const void* s, const void* mask, 
     OF3_REQUIRE(a && s && out && p && workspace, OF3_ERR_ARG, "cond_transition: null pointer argument");
     OF3_REQUIRE(rows > 0 && c_a > 0 && c_s > 0 && n > 0, OF3_ERR_ARG, "cond_transition: non-positive size");
     OF3_REQUIRE(complete(*p), OF3_ERR_ARG, "cond_transition: null parameter pointer");
+    CallScope call;
     Arena ws(workspace, workspace_bytes);
     return cond_dispatch(a, s, mask, out, rows, c_a, c_s, n, dtype, flags, p, ws, (cudaStream_t)stream);
 }

@@ -258,6 +258,7 @@ int of3_pair_block_forward(void* z, const void* pair_mask, const of3_block_dims*
     CHECK_BLOCK("pair_block");
     OF3_REQUIRE(z && p && workspace, OF3_ERR_ARG, "pair_block: null pointer argument");
     OF3_REQUIRE(complete_block(*p), OF3_ERR_ARG, "pair_block: null parameter pointer");
+    CallScope call((flags & OF3_FLAG_CONTINUES) != 0);
     Scratch ws{workspace, workspace_bytes};
     return pair_block(z, pair_mask, *dims, dtype, flags, p, ws, (cudaStream_t)stream);
 }
@@ -294,6 +295,7 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
     const size_t head = (workspace_bytes - tail) / 256 * 256;
     void* bias = (char*)workspace + head;
     Scratch ws{workspace, head}, ws_side{side_workspace, side_workspace_bytes};
+    CallScope call((flags & OF3_FLAG_CONTINUES) != 0);
     int rc;
     if ((rc = pair_block(z, pair_mask, *dims, dtype, flags, &p->pair, ws, main))) return rc;
     if (form == kBiasInLayer || side_stream == nullptr) {
@@ -335,6 +337,7 @@ int of3_diffusion_stack_forward(void* a, const void* s, const void* z, const voi
         OF3_REQUIRE(complete(attn[b], (flags & OF3_FLAG_ADA_LN) != 0, bias == nullptr) && complete(transition[b]) &&
                         (bias == nullptr || bias[b] != nullptr),
                     OF3_ERR_ARG, "diffusion_stack: null parameter pointer (block %d)", b);
+    CallScope call;
     Scratch ws{workspace, workspace_bytes};
     return diffusion_stack(a, s, z, mask, bias, *dims, dtype, flags, blocks, attn, transition, ws, (cudaStream_t)stream);
 }

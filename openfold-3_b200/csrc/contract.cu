@@ -327,6 +327,7 @@ extern "C" int of3_contract_nt_bf16(const void* a, const void* b, void* out, int
                                     int K, int lda, int ldb, int ldo, long long a_batch_stride,
                                     long long b_batch_stride, long long out_batch_stride,
                                     void* stream) {
+    of3::CallScope call;
     return of3::contract_nt_bf16((const __nv_bfloat16*)a, (const __nv_bfloat16*)b,
                                  (__nv_bfloat16*)out, batch, M, N, K, lda, ldb, ldo, a_batch_stride,
                                  b_batch_stride, out_batch_stride, (cudaStream_t)stream, 0, 0, 1);

@@ -95,6 +95,7 @@ int of3_attn_pair_bias_forward_rows(const void* a, const float* pair_bias_rows, 
     OF3_REQUIRE(dtype == OF3_DTYPE_BF16 && !(flags & OF3_FLAG_ADA_LN) &&
                     fast::attn_pair_bias_supported(1, 1, N, c_a, 0, 128, H, d, flags),
                 OF3_ERR_SHAPE, "attn_pair_bias_rows: bf16, 16 heads of 24 or 48 only");
+    CallScope call;
     Arena ws(workspace, workspace_bytes);
     return fast::attn_pair_bias_rows((const __nv_bfloat16*)a, pair_bias_rows, (const __nv_bfloat16*)mask,
                                      (__nv_bfloat16*)out_rows, N, row0, R, c_a, H, d, inf, flags, p, ws,
@@ -113,6 +114,7 @@ int of3_dap_trimul_project(const void* z_rows, const void* mask, void* ab, int l
     OF3_REQUIRE(lines > 0 && positions > 0, OF3_ERR_ARG, "dap_trimul_project: non-positive size");
     OF3_REQUIRE(world == 1 || world == 2 || world == 4 || world == 8, OF3_ERR_ARG,
                 "dap_trimul_project: world must be 1, 2, 4 or 8 (got %d)", world);
+    CallScope call;
     const int ld = (int)align_up(positions, 8);
     const long long plane = (long long)(128 / world) * lines * ld;  // one rank's channels of a (or b)
     __nv_bfloat16* a_t = (__nv_bfloat16*)ab;
@@ -125,6 +127,7 @@ int of3_dap_trimul_contract(const void* ab_all, void* x_blocks, int N, int chann
     OF3_REQUIRE(ab_all && x_blocks, OF3_ERR_ARG, "dap_trimul_contract: null pointer argument");
     OF3_REQUIRE(N > 0 && channels > 0 && rows_per_rank > 0 && N % rows_per_rank == 0, OF3_ERR_ARG,
                 "dap_trimul_contract: bad sizes N=%d channels=%d rows_per_rank=%d", N, channels, rows_per_rank);
+    CallScope call;
     const int ld = (int)align_up(N, 8);
     const __nv_bfloat16* a = (const __nv_bfloat16*)ab_all;
     const long long plane = (long long)N * ld;
@@ -137,6 +140,7 @@ int of3_dap_trimul_output(const void* z_rows, void* out_rows, const void* x_t, i
                           const of3_trimul_params* p, void* stream) {
     OF3_REQUIRE(z_rows && out_rows && x_t && p, OF3_ERR_ARG, "dap_trimul_output: null pointer argument");
     OF3_REQUIRE(R > 0 && N > 0, OF3_ERR_ARG, "dap_trimul_output: non-positive size");
+    CallScope call;
     return fast::trimul_output((const __nv_bfloat16*)z_rows, (__nv_bfloat16*)out_rows, (const __nv_bfloat16*)x_t, 1, R,
                                N, (int)align_up(N, 8), (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p,
                                (cudaStream_t)stream);
@@ -147,6 +151,7 @@ int of3_dap_triattn_project(const void* z_rows, void* q, void* k, void* vt, void
     OF3_REQUIRE(z_rows && q && k && vt && bias_rows && p, OF3_ERR_ARG, "dap_triattn_project: null pointer argument");
     OF3_REQUIRE(R > 0 && N > 0 && row0 >= 0 && row0 + R <= N, OF3_ERR_ARG,
                 "dap_triattn_project: bad sizes R=%d N=%d row0=%d", R, N, row0);
+    CallScope call;
     return fast::triattn_project((const __nv_bfloat16*)z_rows, (__nv_bfloat16*)q, (__nv_bfloat16*)k,
                                  (__nv_bfloat16*)vt, (__nv_bfloat16*)bias_rows, 1, R, N, row0, false, p,
                                  (cudaStream_t)stream);
@@ -158,6 +163,7 @@ int of3_dap_triattn_finish(const void* z_rows, const void* mask_rows, void* out_
     OF3_REQUIRE(z_rows && out_rows && q && k && vt && bias_all && o_scratch && p, OF3_ERR_ARG,
                 "dap_triattn_finish: null pointer argument");
     OF3_REQUIRE(R > 0 && N > 0, OF3_ERR_ARG, "dap_triattn_finish: non-positive size");
+    CallScope call;
     return fast::triattn_finish((const __nv_bfloat16*)z_rows, (const __nv_bfloat16*)mask_rows,
                                 (__nv_bfloat16*)out_rows, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
                                 (const __nv_bfloat16*)vt, (const __nv_bfloat16*)bias_all, (__nv_bfloat16*)o_scratch, 1, R,
@@ -168,6 +174,7 @@ int of3_pair_bias_project(const void* z_rows, const void* ln_w, const void* ln_b
                           long long positions, int c_z, int H, int dtype, void* stream) {
     OF3_REQUIRE(z_rows && w && bias_rows, OF3_ERR_ARG, "pair_bias_project: null pointer argument");
     OF3_REQUIRE(c_z == 128 && H == 16, OF3_ERR_SHAPE, "pair_bias_project: only c_z = 128, 16 heads");
+    CallScope call;
     if (dtype == OF3_DTYPE_BF16)
         return fast::pair_bias_c128_h16((const __nv_bfloat16*)z_rows, (const __nv_bfloat16*)ln_w,
                                         (const __nv_bfloat16*)ln_b, (const __nv_bfloat16*)w, bias_rows, 1, positions,
@@ -183,6 +190,7 @@ int of3_attn_pair_bias_forward_prebias(const void* a, const float* pair_bias, co
                                        size_t workspace_bytes, void* stream) {
     OF3_REQUIRE(a && pair_bias && out && p && workspace, OF3_ERR_ARG, "attn_pair_bias_prebias: null pointer argument");
     OF3_REQUIRE(Ba > 0 && Bz > 0 && Ba % Bz == 0 && N > 0, OF3_ERR_ARG, "attn_pair_bias_prebias: bad sizes");
+    CallScope call;
     Arena ws(workspace, workspace_bytes);
     if (dtype == OF3_DTYPE_BF16 && fast::attn_pair_bias_supported(Ba, Bz, N, c_a, c_s, 128, H, d, flags))
         return fast::attn_pair_bias((const __nv_bfloat16*)a, nullptr, (const __nv_bfloat16*)s,
@@ -208,6 +216,7 @@ int of3_pair_bias_project_tiles(const void* z, const void* ln_w, const void* ln_
     OF3_REQUIRE(z && w && tiles, OF3_ERR_ARG, "pair_bias_project_tiles: null pointer argument");
     OF3_REQUIRE(c_z == 128 && H == 16 && dtype == OF3_DTYPE_BF16 && N > 0, OF3_ERR_SHAPE,
                 "pair_bias_project_tiles: only bf16, c_z = 128, 16 heads");
+    CallScope call;
     return fast::pair_bias_tiles_c128_h16((const __nv_bfloat16*)z, (const __nv_bfloat16*)ln_w, (const __nv_bfloat16*)ln_b,
                                           (const __nv_bfloat16*)w, (__nv_bfloat16*)tiles, 1, N, (cudaStream_t)stream);
 }
@@ -220,6 +229,7 @@ int of3_attn_pair_bias_forward_pretiles(const void* a, const void* bias_tiles, c
     OF3_REQUIRE(Ba > 0 && Bz > 0 && Ba % Bz == 0 && N > 0, OF3_ERR_ARG, "attn_pair_bias_pretiles: bad sizes");
     OF3_REQUIRE(dtype == OF3_DTYPE_BF16 && fast::attn_pair_bias_supported(Ba, Bz, N, c_a, c_s, 128, H, d, flags),
                 OF3_ERR_SHAPE, "attn_pair_bias_pretiles: bias tiles only feed the bf16 tensor-core attention");
+    CallScope call;
     Arena ws(workspace, workspace_bytes);
     return fast::attn_pair_bias((const __nv_bfloat16*)a, nullptr, (const __nv_bfloat16*)s, (const __nv_bfloat16*)mask,
                                 (__nv_bfloat16*)out, Ba, Bz, N, c_a, c_s, H, d, inf, flags, p, ws, (cudaStream_t)stream,

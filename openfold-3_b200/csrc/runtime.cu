@@ -194,6 +194,18 @@ static std::vector<cudaEvent_t> g_pool;  // recycled events
 static long long g_launches[kMaxKernelIds] = {0};
 static bool g_prof_on = false;
 
+static std::atomic<long long> g_chained{0};
+static thread_local bool t_chain = false;
+
+CallScope::CallScope(bool continues) { t_chain = continues; }
+
+bool take_chain() {
+    const bool chained = t_chain;
+    t_chain = true;
+    if (chained) g_chained.fetch_add(1, std::memory_order_relaxed);
+    return chained;
+}
+
 static cudaEvent_t take_event() {
     if (!g_pool.empty()) {
         cudaEvent_t e = g_pool.back();
@@ -241,6 +253,7 @@ extern "C" int of3_profile_reset(void) {
     }
     of3::g_recs.clear();
     for (int i = 0; i < of3::kMaxKernelIds; ++i) of3::g_launches[i] = 0;
+    of3::g_chained = 0;
     return OF3_OK;
 }
 
@@ -249,7 +262,7 @@ extern "C" int of3_profile_read(int kernel_id, long long* launches, float* total
                 "of3_profile_read: bad argument");
     OF3_CUDA_CHECK(cudaDeviceSynchronize());
     std::lock_guard<std::mutex> lk(of3::g_mu);
-    *launches = of3::g_launches[kernel_id];
+    *launches = kernel_id == 0 ? of3::g_chained.load() : of3::g_launches[kernel_id];
     float sum = 0.f;
     for (auto& r : of3::g_recs) {
         if (r.kid != kernel_id) continue;

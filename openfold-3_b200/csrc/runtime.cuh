@@ -17,9 +17,9 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
 // Per-kernel launch accounting. Every launch site of this library opens a LaunchScope with its
 // kernel id: launches are always counted; when timing is enabled (of3_profile_enable) a CUDA event
 // pair is recorded around the launch on the launching stream, and of3_profile_read sums their
-// elapsed times. Ids: 1 contract, 2 trimul_in, 3 trimul_out, 4 transition, 5 triattn_proj,
+// elapsed times. Ids: 0 the launches of any kind that were chained to the one ahead (count only), 1 contract, 2 trimul_in, 3 trimul_out, 4 transition, 5 triattn_proj,
 // 6 triattn_core, 7 triattn_out, 8 single-track kernels, 9 pair-bias projection, 10 linear layers of the
-// single track (the contraction kernel as a plain GEMM), 20 the shape-generic SIMT kernels, 30 / 31 peer
+// single track, 11 single-track attention core, 20 the shape-generic SIMT kernels, 30 / 31 peer
 // barrier / pull.
 constexpr int kMaxKernelIds = 32;
 struct LaunchScope {
@@ -33,8 +33,18 @@ struct LaunchScope {
 // Work enqueued on `waiter` from now on starts after everything enqueued on `signaler` so far.
 int stream_wait(cudaStream_t waiter, cudaStream_t signaler);
 
+// One per call of an entry point that launches. Chained kernels load weights before umma::grid_wait(), which alone makes
+// the writes of the kernel ahead visible: so the first launch of a call, behind whatever the caller enqueued (an in-place
+// update of the weights, a conversion), is an ordinary one, and only launches behind a kernel of the same call are chained.
+// `continues`: the caller says that the kernel ahead is that of another call and no parameter was written since.
+struct CallScope {
+    explicit CallScope(bool continues = false);
+};
+bool take_chain();   // whether this thread's next launch may be chained
+
 // Launches a kernel that calls umma::grid_wait() before it touches anything another kernel wrote: its prologue (barrier
-// set-up, tensor-memory allocation, weight loads) overlaps the end of the kernel before it in the stream.
+// set-up, tensor-memory allocation, weight loads) overlaps the end of the kernel before it in the stream, where that is one
+// of the same call.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                   Args&&... args) {
@@ -47,7 +57,7 @@ inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = take_chain() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 

@@ -22,6 +22,7 @@
 #include <mutex>
 
 #include "modules.cuh"
+#include "runtime.cuh"
 
 namespace {
 
@@ -74,6 +75,7 @@ extern "C" int of3_trimul_forward_static(const void* z, const void* mask, void* 
                 B, N, c_z, c_h, probe.off, kStaticScratchBytes);
     void* scratch = nullptr;
     if ((rc = static_scratch(&scratch))) return rc;
+    CallScope call;
     Arena ws(scratch, kStaticScratchBytes);
     cudaStream_t st = (cudaStream_t)stream;
     if (dtype == OF3_DTYPE_BF16)

@@ -204,10 +204,11 @@ class _Plan:
     ``called``: the modules that the layer-by-layer path runs as a caller would, with their hooks; ``layers``: those whose
     parameters and constants the native path reads."""
 
-    __slots__ = ("dtype", "device", "hooks", "forwards", "watch", "held", "params", "keep", "shapes")
+    __slots__ = ("dtype", "device", "hooks", "forwards", "watch", "held", "params", "keep", "shapes", "called")
 
     def __init__(self, block, called, layers, dtype, device):
         self.dtype, self.device, self.params, self.keep, self.shapes = dtype, device, None, None, {}
+        self.called = False   # the copies of the weights may be the last work on the stream
         self.hooks = [h for m in called for h in (m._forward_hooks, m._forward_pre_hooks)]
         self.hooks += [_nn_module._global_forward_hooks, _nn_module._global_forward_pre_hooks]
         self.forwards = [(c, c.forward) for c in {type(m) for m in called}]
@@ -766,8 +767,9 @@ class PairFormerBlock(_Planned):
         d.single_transition_n, d.inf_single = self.single_transition.n, a.inf
         return lib.BlockPlan(d, dtype, flags, single=True)
 
-    def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None):
-        """In place on contiguous s and z with prepared masks; False if the native path does not take this call."""
+    def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None, continues=False):
+        """In place on contiguous s and z with prepared masks; False if the native path does not take this call.
+        ``continues``: the last work on the stream is another block's native call."""
         st = _native_state(self, z)
         attn = self.attn_pair_bias
         B = None if st is None else _pair_batch(z, attn.c_z)
@@ -775,6 +777,9 @@ class PairFormerBlock(_Planned):
             return False
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
         plan = st[0].shape(self, B, z.shape[-2], st[1], flags)
+        if continues and st[0].called:
+            flags |= lib.FLAG_CONTINUES
+        st[0].called = True
         lib.pairformer_block_forward(s, z, single_mask, pair_mask, plan, st[1], flags, st[0].params, side)
         return True
 
@@ -846,9 +851,11 @@ class PairFormerStack(nn.Module):
         main = torch.cuda.current_stream(z.device)
         side = lib.side_stream(main)
         lib.stream_wait(side, main)
+        native = False
         try:
             for b in self.blocks:
-                if b._run_native(s, z, single_mask, pair_mask, _mask_trans, side):
+                native = b._run_native(s, z, single_mask, pair_mask, _mask_trans, side, continues=native)
+                if native:
                     continue
                 z = b.pair_stack(z=z, pair_mask=pair_mask, chunk_size=chunk_size, inplace_safe=True,
                                  _mask_trans=_mask_trans)

@@ -1,6 +1,8 @@
 """The native block entry points against the layer-by-layer path of the same modules: the same kernels in the same order,
 so the same bits; parameters changed in place, replaced, or moved between calls are seen."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -77,3 +79,30 @@ def test_kept_biases_where_the_attention_is_the_generic_one():
         own = st(a, s, z)
     pkg.lib.check_device_status()
     assert ((kept - own).float().norm() / own.float().norm()).item() < 8e-3
+
+
+def test_the_first_launch_of_a_call_is_not_chained():
+    """It stands behind whatever the caller enqueued, an update of the weights for instance, which its loads ahead of the wait
+    must not overtake; all other launches of the tensor-core path are chained."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    L = pkg.lib.load()
+
+    def counts(call):
+        pkg.lib.profile_begin(timing=False)
+        with torch.no_grad():
+            call()
+        total = sum(n for n, _ in pkg.lib.profile_end().values())
+        chained, ms = ctypes.c_longlong(0), ctypes.c_float(0)
+        assert L.of3_profile_read(0, ctypes.byref(chained), ctypes.byref(ms)) == 0
+        return total, total - chained.value
+
+    st = pkg.PairFormerStack(**OF3, **_PF_KW, no_blocks=3, blocks_per_ckpt=None).to(dev, bf).eval().requires_grad_(False)
+    s, z = torch.randn(1, 20, 384, device=dev).to(bf), torch.randn(1, 20, 20, 128, device=dev).to(bf)
+    p = st.blocks[0].pair_stack
+    for layer in (p.tri_mul_out, p.tri_att_start, p.pair_transition):
+        assert counts(lambda: layer(z))[1] == 1
+    assert counts(lambda: p(z, None))[1] == 1
+    total, unchained = counts(lambda: st(s, z, None, None))   # the blocks' weights are packed in between
+    assert unchained == 3 and counts(lambda: st(s, z, None, None)) == (total, 1)
+    st.blocks[2].pair_stack.tri_att_end.mha.linear_o.weight.mul_(1.5)
+    assert counts(lambda: st(s, z, None, None)) == (total, 2)

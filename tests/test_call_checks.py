@@ -129,3 +129,24 @@ def test_a_failed_stack_call_still_joins_the_second_stream(pkg, calls, monkeypat
     with torch.no_grad(), pytest.raises(RuntimeError, match="second block"):
         stack(gpu(1, 20, 384), gpu(1, 20, 20, 128), None, None)
     assert calls == ["block", "block"] and waits == [("side", "main"), ("main", "side")]
+
+
+def test_only_blocks_behind_a_block_continue(pkg, monkeypatch):
+    """A block whose weights have just been packed, or written to, starts behind all work before it."""
+    stack = pkg.PairFormerStack(**OF3, **_PF_KW, no_blocks=3, blocks_per_ckpt=None).eval().to(BF).requires_grad_(False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: "main")
+    monkeypatch.setattr(pkg.lib, "side_stream", lambda main: "side")
+    monkeypatch.setattr(pkg.lib, "stream_wait", lambda *a: None)
+    flags = []
+    monkeypatch.setattr(pkg.lib, "pairformer_block_forward",
+                        lambda s, z, sm, pm, plan, dt, f, prm, side: flags.append(bool(f & pkg.lib.FLAG_CONTINUES)))
+
+    def call():
+        del flags[:]
+        with torch.no_grad():
+            stack(gpu(1, 20, 384), gpu(1, 20, 20, 128), None, None)
+        return flags
+
+    assert call() == [False, False, False] and call() == [False, True, True]
+    stack.blocks[1].single_transition.linear_out.weight.mul_(2)
+    assert call() == [False, False, True] and call() == [False, True, True]
