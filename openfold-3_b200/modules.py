@@ -212,8 +212,13 @@ class _Plan:
         self.hooks = [h for m in called for h in (m._forward_hooks, m._forward_pre_hooks)]
         self.hooks += [_nn_module._global_forward_hooks, _nn_module._global_forward_pre_hooks]
         self.forwards = [(c, c.forward) for c in {type(m) for m in called}]
-        tree = list(block.modules())
-        owned, children = [m._parameters for m in tree if m._parameters], [m._modules for m in tree if m._modules]
+        owned, children, tree = [], [], [block]
+        for m in tree:   # (grows)
+            if m._parameters:
+                owned.append(m._parameters)
+            if m._modules:
+                children.append(m._modules)
+                tree += [c for c in m._modules.values() if c is not None]
         attrs = [(m.__dict__, n) for m in layers for n in m._plan_constants]
         replaced = [(m.__dict__, "forward") for m in called]
         replaced += [(m.__dict__, n) for m in (block, *called) for n in ("tri_mul_out_in", "tri_att_start_end")
@@ -223,13 +228,14 @@ class _Plan:
         w = _param_watch()
         found = None
         known = {id(t) for d in owned for t in d.values()}
+        tensors = [m._tensors() for m in layers]
         # (a weight that is not a parameter, computed or a plain tensor, may change unseen: layer by layer)
-        if (not any(n in d for d, n in replaced) and not any("parametrizations" in m._modules for m in tree)
-                and all(t is None or id(t) in known for m in layers for t in m._tensors())):
+        if (not any(n in d for d, n in replaced) and not any("parametrizations" in c for c in children)
+                and all(t is None or id(t) in known for ts in tensors for t in ts)):
             found = w.make(owned, children, attrs)
         self.watch, self.held = found or w.make([], owned + children, attrs)
         if found:
-            self.params, self.keep = block._native_params(dtype, device)
+            self.params, self.keep = block._native_params(layers, tensors, dtype, device)
 
     def current(self, dtype, device):
         return dtype == self.dtype and device == self.device and not _watch_module.changed(self.watch)
@@ -311,8 +317,17 @@ def _pair_batch(z, c_z):
     return z.numel() // (z.shape[-2] * z.shape[-2] * c_z)
 
 
+class _Layer(nn.Module):
+    """Base of the layers: ``_tensors()`` lists the parameters that the kernels take, ``_packed`` keeps their copies."""
+
+    _adjacent = ()   # groups of _tensors() whose copies lie back to back
+
+    def _params(self, dtype, device):
+        return self._packed.get(self._tensors(), dtype, device, self._adjacent)
+
+
 # --------------------------------------------------------------------------- triangle multiplication
-class TriangleMultiplicativeUpdate(nn.Module):
+class TriangleMultiplicativeUpdate(_Layer):
     """AF3 Algorithms 12/13. Drop-in for
     openfold3/core/model/layers/triangular_multiplicative_update.py:123-503."""
 
@@ -335,9 +350,6 @@ class TriangleMultiplicativeUpdate(nn.Module):
         return (self.layer_norm_in.weight, self.layer_norm_in.bias, self.linear_a_p.weight,
                 self.linear_a_g.weight, self.linear_b_p.weight, self.linear_b_g.weight, self.linear_g.weight,
                 self.layer_norm_out.weight, self.layer_norm_out.bias, self.linear_z.weight)
-
-    def _params(self, dtype, device):
-        return self._packed.get(self._tensors(), dtype, device)
 
     def forward(self, z, mask=None, inplace_safe=False, use_cueq_triangle_kernels=False,
                 _add_with_inplace=False, _inplace_chunk_size=256):
@@ -364,7 +376,7 @@ class TriangleMultiplicationIncoming(TriangleMultiplicativeUpdate):
 
 
 # --------------------------------------------------------------------------- triangle attention
-class TriangleAttention(nn.Module):
+class TriangleAttention(_Layer):
     """AF3 Algorithms 14/15. Drop-in for openfold3/core/model/layers/triangular_attention.py:30-179."""
 
     def __init__(self, c_in, c_hidden, no_heads, starting=True, inf=1e9, linear_init_params=lin_init.tri_att_init):
@@ -382,9 +394,6 @@ class TriangleAttention(nn.Module):
         return (self.layer_norm.weight, self.layer_norm.bias, self.linear_z.weight, self.mha.linear_q.weight,
                 self.mha.linear_k.weight, self.mha.linear_v.weight, self.mha.linear_g.weight,
                 self.mha.linear_o.weight)
-
-    def _params(self, dtype, device):
-        return self._packed.get(self._tensors(), dtype, device)
 
     def _run(self, x, mask, transposed: bool, in_place: bool):
         N = x.shape[-2]
@@ -413,7 +422,7 @@ class TriangleAttentionEndingNode(TriangleAttention):
 
 
 # --------------------------------------------------------------------------- transitions
-class SwiGLUTransition(nn.Module):
+class SwiGLUTransition(_Layer):
     """AF3 Algorithm 11. Drop-in for openfold3/core/model/layers/transition.py:225-271."""
 
     def __init__(self, c_in: int, n: int, linear_init_params=lin_init.swiglu_transition_init):
@@ -430,8 +439,7 @@ class SwiGLUTransition(nn.Module):
         return (self.layer_norm.weight, self.layer_norm.bias, self.swiglu.linear_a.weight,
                 self.swiglu.linear_b.weight, self.linear_out.weight)
 
-    def _params(self, dtype, device):
-        return self._packed.get(self._tensors(), dtype, device, adjacent=((2, 3),))
+    _adjacent = ((2, 3),)
 
     def _run(self, x, mask, in_place: bool):
         xc = x.contiguous().view(-1, self.c_in)
@@ -447,7 +455,7 @@ class SwiGLUTransition(nn.Module):
         return self._run(x, mask, in_place=False)
 
 
-class ConditionedTransitionBlock(nn.Module):
+class ConditionedTransitionBlock(_Layer):
     """AF3 Algorithm 25. Drop-in for openfold3/core/model/layers/transition.py:274-380."""
 
     def __init__(self, c_a: int, c_s: int, n: int, linear_init_params=lin_init.cond_transition_init):
@@ -469,8 +477,7 @@ class ConditionedTransitionBlock(nn.Module):
 
     _cond_group = (1, 3, 6)   # the three projections of s among _tensors()
 
-    def _params(self, dtype, device):
-        return self._packed.get(self._tensors(), dtype, device, adjacent=(self._cond_group, (4, 5)))
+    _adjacent = (_cond_group, (4, 5))
 
     def _run(self, a, s, mask, in_place: bool):
         _same_device(a, s=s)
@@ -489,7 +496,7 @@ class ConditionedTransitionBlock(nn.Module):
 
 
 # --------------------------------------------------------------------------- attention with pair bias
-class AttentionPairBias(nn.Module):
+class AttentionPairBias(_Layer):
     """AF3 Algorithm 24. Drop-in for openfold3/core/model/layers/attention_pair_bias.py:33-227."""
 
     def __init__(self, c_q, c_k, c_v, c_s, c_z, c_hidden, no_heads, use_ada_layer_norm=False, gating=True,
@@ -530,9 +537,7 @@ class AttentionPairBias(nn.Module):
 
     _cond_group = (3, 5, 6)   # the three projections of s among _tensors()
 
-    def _params(self, dtype, device):
-        return self._packed.get(self._tensors(), dtype, device,
-                                adjacent=((11, 15, 13, 14), self._cond_group))   # q, g, k, v; the projections of s
+    _adjacent = ((11, 15, 13, 14), _cond_group)   # q, g, k, v; the projections of s
 
     def can_hoist_pair_bias(self, z) -> bool:
         """Whether ``project_pair_bias`` has a kernel for this layer (c_z = 128, 16 heads, bf16 or fp32)."""
@@ -670,9 +675,8 @@ class PairBlock(_Planned):
             return None
         return [*mul, self.ps_dropout_row_layer], [*mul, *att, self.pair_transition]
 
-    def _native_params(self, dtype, device):
-        parts = [m._params(dtype, device) for m in (self.tri_mul_out, self.tri_mul_in, self.tri_att_start,
-                                                    self.tri_att_end, self.pair_transition)]
+    def _native_params(self, layers, tensors, dtype, device):
+        parts = [m._packed.get(t, dtype, device, m._adjacent) for m, t in zip(layers, tensors)]
         kinds = (lib.TrimulParams, lib.TrimulParams, lib.TriattnParams, lib.TriattnParams, lib.TransitionParams)
         return lib.PairBlockParams(*[k(*_pointers(p)) for k, p in zip(kinds, parts)]), parts
 
@@ -755,9 +759,9 @@ class PairFormerBlock(_Planned):
             return None
         return [self.pair_stack, *inner[0]], [*inner[1], attn, trans]
 
-    def _native_params(self, dtype, device):
-        pair, keep = self.pair_stack._native_params(dtype, device)
-        attn, trans = self.attn_pair_bias._params(dtype, device), self.single_transition._params(dtype, device)
+    def _native_params(self, layers, tensors, dtype, device):
+        pair, keep = self.pair_stack._native_params(layers[:5], tensors[:5], dtype, device)
+        attn, trans = (m._packed.get(t, dtype, device, m._adjacent) for m, t in zip(layers[5:], tensors[5:]))
         return (lib.PairformerBlockParams(pair, lib.AttnPairBiasParams(*_pointers(attn)),
                                           lib.TransitionParams(*_pointers(trans))), (keep, attn, trans))
 
@@ -981,11 +985,9 @@ class DiffusionTransformer(_Planned):
             return None
         return blocks, [m for b in blocks for m in (b.attention_pair_bias, b.conditioned_transition)]
 
-    def _native_params(self, dtype, device):
+    def _native_params(self, layers, raw, dtype, device):
         """Parameter structs of all blocks. The projections of s lie back to back over the whole stack (the library
         computes those of several blocks in one launch)."""
-        layers = [m for b in self.blocks for m in (b.attention_pair_bias, b.conditioned_transition)]
-        raw = [m._tensors() for m in layers]
         first = [0]
         for r in raw:
             first.append(first[-1] + len(r))
