@@ -329,7 +329,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
 //                 registers. The pair-bias tiles [128 q x 32 k] (bf16, shared by both lines) are a second A operand
 //                 against a 32 x 32 identity: a bf16 value times 1.0 accumulated in fp32 is exact.
 //   softmax warps thread = query row = TMEM lane: S -> registers [+ mask bias where the block has masked keys], row
-//                 maximum, P = exp2(S - m), row sum, P rounded to bf16 into TMEM columns of its own
+//                 maximum, P = exp2(S - m) rounded to bf16, sum of the rounded values, P into TMEM columns of its own
 //   MMA warp      O[128 x D] += P_j V_j with P read from TMEM as the A operand
 // What bounds it: one exponential per logit (N = 768: 1.8e9 per launch, 402 us of the MUFU pipe at 1.9 GHz), and what a
 // softmax warp does besides, for the four lines of an SM keep that pipe busy only while one of them is in its
@@ -341,7 +341,10 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
 // TMEM columns of a line (128): S [0,64), P [64,96), O [96, 96 + D).
 // The running maximum m used for scaling is only raised when the row maximum exceeds it by more than 32
 // (2^32 head room in P, in bf16 as precise as below 1): then, and only then, the thread rescales its O row in TMEM and
-// its row sum. The result is exact: numerator and denominator always share one scale.
+// its row sum. The result is exact: numerator and denominator always share one scale, and one rounding of P: the row sum
+// adds the bf16 values that the GEMM reads (mixed-precision adds, N = 768 649 -> 666 us, N = 2048 11.07 -> 11.25 ms;
+// unpacking them for packed adds 681, 11.66). Summed before the rounding, what it does to the dominant keys of a row, up to
+// 2^-9, no longer cancels: 13 % more error in o where the values are alike.
 constexpr int kBQ = 128;      // queries per CTA
 constexpr int kMaxKeys = 2048;   // one CTA keeps a mask-bias row per line in shared memory
 constexpr int kKvStages = 2;     // ring of K + bias tiles, ring of V tiles
@@ -710,8 +713,8 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
                     const float p0 = ex2_approx(x[0]), p1 = ex2_approx(x[1]), p2 = ex2_approx(x[2]), p3 = ex2_approx(x[3]);
                     pk[e >> 1] = pack_bf16x2(p0, p1);
                     pk[(e >> 1) + 1] = pack_bf16x2(p2, p3);
-                    add2(l0, l1, p0, p1);
-                    add2(l2, l3, p2, p3);
+                    add_bf16x2(l0, l1, pk[e >> 1]);
+                    add_bf16x2(l2, l3, pk[(e >> 1) + 1]);
                 }
             };
             exps(0);

@@ -46,6 +46,18 @@ __device__ __forceinline__ void add2(float& x0, float& x1, float y0, float y1) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(a));
 }
 
+// x0 += low half, x1 += high half of two packed bf16 values (exact in fp32 up to the additions)
+__device__ __forceinline__ void add_bf16x2(float& x0, float& x1, uint32_t v) {
+    asm("{\n"
+        ".reg .b16 lo, hi;\n"
+        "mov.b32 {lo, hi}, %2;\n"
+        "add.rn.f32.bf16 %0, lo, %0;\n"
+        "add.rn.f32.bf16 %1, hi, %1;\n"
+        "}\n"
+        : "+f"(x0), "+f"(x1)
+        : "r"(v));
+}
+
 // Walks the row tiles t = first, first + step, ... of `lines` lines per sample and tiles_per_line tiles per line without a
 // division per tile: the 64-bit quotients and remainders of t took some 3900 cycles per tile in every warp's serial chain
 // (trimul_in at N = 768: of 10000).

@@ -28,3 +28,37 @@ def test_pair_block_matches_the_oracle(dims, B, N):
         got = blk(z.to(dev), m.to(dev, bf)).float().cpu()
     pkg.lib.check_device_status()
     assert rms_err(got, ref) < 8e-3 and rel_err(got, ref) < 8e-2, (rms_err(got, ref), rel_err(got, ref))
+
+
+@pytest.mark.parametrize("c,N", [(128, 320), (64, 300)])
+def test_numerator_and_denominator_of_the_softmax_round_alike(c, N):
+    """Values near one and rows that few keys dominate, the largest logit as a rule not in the first key block, so that the
+    probabilities of the dominant keys are rounded (2^-9): summed before that rounding, the row sum no longer cancels it. All
+    else of the layer is made exact (gate 1/2, output projection the identity, no bias), so the error against a double softmax
+    of the kernel's own bf16 operands is the final rounding of o and nothing more: 1.00 times it with matched sums, 1.13 with a
+    row sum of unrounded probabilities (both simulated in double)."""
+    dev, bf, H = torch.device("cuda:0"), torch.bfloat16, 4
+    g = torch.Generator().manual_seed(c)
+    wq, wk, wv = (torch.randn(c, c, generator=g) * (k * c ** -0.5) for k in (3.0, 1.0, 0.01))
+    wq[:, 0] = wk[:, 0] = 0
+    wv[:, 0] = 0.97
+    att = pkg.TriangleAttention(c, c // H, H)
+    with torch.no_grad():
+        att.layer_norm.weight[0], att.layer_norm.bias[0] = 0, 1   # channel 0 of the normalised rows is one
+        for lin, w in ((att.mha.linear_q, wq), (att.mha.linear_k, wk), (att.mha.linear_v, wv), (att.mha.linear_o, torch.eye(c)),
+                       (att.mha.linear_g, torch.zeros(c, c)), (att.linear_z, torch.zeros(H, c))):
+            lin.weight.copy_(w)
+    att = att.to(dev, bf).eval().requires_grad_(False)
+    z = torch.randn(N, N, c, generator=g).to(dev, bf)
+    with torch.no_grad():
+        got = 2 * att(z[None])[0, :4].double()
+    pkg.lib.check_device_status()
+    ln = torch.nn.functional.layer_norm(z[:4].float(), (c,)).to(bf).float()
+    ln[..., 0] = 1
+    q, k, v = (torch.nn.functional.linear(ln.double(), w.to(dev, bf).double()).float() for w in (wq, wk, wv))
+    q = (q * (1.4426950408889634 / (c // H) ** 0.5)).to(bf)
+    q, k, v = (t.to(bf).double().view(4, N, H, c // H) for t in (q, k, v))
+    p = torch.softmax(torch.einsum("bqhd,bkhd->bhqk", q, k) * 0.6931471805599453, -1)
+    exact = torch.einsum("bhqk,bkhd->bqhd", p, v).reshape(4, N, c)
+    rounding = (exact.to(bf).double() - exact).norm()
+    assert ((got - exact).norm() / rounding).item() < 1.04
