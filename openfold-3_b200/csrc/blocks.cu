@@ -291,10 +291,11 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
     cudaStream_t main = (cudaStream_t)stream;
     const BiasForm form = bias_form(*dims, dtype, flags);
     const size_t tail = bias_bytes(*dims, form);
-    OF3_REQUIRE(workspace_bytes >= tail, OF3_ERR_WORKSPACE, "pairformer_block: workspace too small");
-    const size_t head = (workspace_bytes - tail) / 256 * 256;
-    void* bias = (char*)workspace + head;
-    Scratch ws{workspace, head}, ws_side{side_workspace, side_workspace_bytes};
+    const Arena whole(workspace, workspace_bytes);   // its start aligned
+    OF3_REQUIRE(whole.cap >= tail, OF3_ERR_WORKSPACE, "pairformer_block: workspace too small");
+    const size_t head = (whole.cap - tail) / 256 * 256;
+    void* bias = whole.base + head;
+    Scratch ws{whole.base, head}, ws_side{side_workspace, side_workspace_bytes};
     CallScope call((flags & OF3_FLAG_CONTINUES) != 0);
     int rc;
     if ((rc = pair_block(z, pair_mask, *dims, dtype, flags, &p->pair, ws, main))) return rc;

@@ -41,12 +41,16 @@ int* device_status_ptr();  // lazily allocated once per device (not on the hot p
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Bump allocator over a caller-owned workspace.
+// Bump allocator over a caller-owned workspace, whatever its alignment: the *_workspace_bytes queries add the 256 bytes
+// that aligning its start may take (kernels store 32 bytes at a time into what lies in it).
 struct Arena {
     char* base;
     size_t cap;
     size_t off;
-    Arena(void* p, size_t n) : base((char*)p), cap(n), off(0) {}
+    Arena(void* p, size_t n) : base((char*)align_up((size_t)p, 256)), cap(n), off(0) {
+        const size_t lost = (size_t)(base - (char*)p);
+        cap = n > lost ? n - lost : 0;
+    }
     void* take(size_t bytes) {
         size_t o = align_up(off, 256);
         off = o + bytes;

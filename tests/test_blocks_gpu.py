@@ -106,3 +106,38 @@ def test_the_first_launch_of_a_call_is_not_chained():
     assert unchained == 3 and counts(lambda: st(s, z, None, None)) == (total, 1)
     st.blocks[2].pair_stack.tri_att_end.mha.linear_o.weight.mul_(1.5)
     assert counts(lambda: st(s, z, None, None)) == (total, 2)
+
+
+@pytest.mark.parametrize("offset", [1, 16, 255])
+def test_a_workspace_may_start_anywhere(monkeypatch, offset):
+    """A caller's workspace of exactly the bytes that were asked for, at any address: same bits."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator().manual_seed(2)
+    st = pkg.PairFormerStack(**OF3, **_PF_KW, no_blocks=2, blocks_per_ckpt=None)
+    st.load_state_dict(W.pairformer_stack_params(seed=5, no_blocks=2, **OF3))
+    diff = pkg.DiffusionTransformer(c_a=768, c_s=384, c_z=128, c_hidden=48, no_heads=16, no_blocks=1, n_transition=2,
+                                    use_ada_layer_norm=True, n_query=None, n_key=None, inf=1e9)
+    st, diff = (m.to(dev, bf).eval().requires_grad_(False) for m in (st, diff))
+    diff.hoist_pair_bias = False
+    s, z = torch.randn(1, 37, 384, generator=g).to(dev, bf), torch.randn(1, 37, 37, 128, generator=g).to(dev, bf)
+    a = torch.randn(1, 37, 768, generator=g).to(dev, bf)
+
+    def run():
+        with torch.no_grad():
+            blk = st.blocks[0]
+            return (*st(s, z, None, None), *blk(s, z, None, None), blk.pair_stack(z, None), diff(a, s, z),
+                    blk.attn_pair_bias(s, z), blk.single_transition(s), blk.pair_stack.tri_att_end(z))
+
+    want, kept = run(), []
+
+    def odd(nbytes, device, stream=None):
+        torch.cuda.synchronize()   # (made anew per call)
+        kept.append(torch.empty(nbytes + 512, dtype=torch.uint8, device=device))
+        assert kept[-1].data_ptr() % 256 == 0
+        return kept[-1][offset:offset + nbytes]
+
+    monkeypatch.setattr(pkg.lib, "workspace", odd)
+    got = run()
+    torch.cuda.synchronize()
+    pkg.lib.check_device_status()
+    assert len(kept) > 5 and all(torch.equal(x, y) for x, y in zip(got, want))
