@@ -37,7 +37,7 @@ template <int G>   // groups of 128 output channels
 struct PbSmem {
     static constexpr uint32_t kW = 0;
     static constexpr uint32_t kZ = G * kTileBytes;
-    static constexpr uint32_t kStat = kZ + kZStages * kTileBytes;    // ring x 2 x 128 floats: scale, scale * -mean
+    static constexpr uint32_t kStat = kZ + kZStages * kTileBytes;    // ring x 2 x 128 floats: 1 / std, -mean / std
     static constexpr uint32_t kConst = kStat + kRing * 1024;         // per channel: sum of W', constant term
     static constexpr uint32_t kBars = kConst + G * 1024;
     static constexpr uint32_t kDyn = kBars + 256 + 1024;
@@ -76,7 +76,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
     const int tiles_per_line = (N + kRows - 1) / kRows;
     const long long num_tiles = lines * tiles_per_line;
     const int lines_per_sample = tiles != nullptr ? N : 1;
-    const float scale = tiles != nullptr ? 1.4426950408889634f : 1.0f;
+    constexpr float kLog2e = 1.4426950408889634f;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kZStages; ++s) {
@@ -118,7 +118,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
             cs += __shfl_xor_sync(0xffffffffu, cs, w);
             cb += __shfl_xor_sync(0xffffffffu, cb, w);
         }
-        if (seg == 0) chan[n] = make_float2(cs, cb * scale);
+        if (seg == 0) chan[n] = make_float2(cs, cb);
     }
     fence_proxy_async_smem();
     if (warp == 1) {
@@ -193,9 +193,8 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
             float mean, rstd;
             half_row_stats(raw, mean, rstd);
             if (half == 0) {
-                const float p = rstd * scale;
-                stat[r * 256 + row] = p;
-                stat[r * 256 + 128 + row] = -p * mean;
+                stat[r * 256 + row] = rstd;
+                stat[r * 256 + 128 + row] = -rstd * mean;
             }
             __syncwarp();
             if (lane == 0) {
@@ -265,8 +264,10 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                             // chunks c2 and c2 + 1 of the row lie at c2 ^ sw and (c2 + 1) ^ sw: one aligned pair
                             const int c2 = (k0 >> 3) & 2;
                             uint32_t o[8], w[8];
+                            // scaled last, as the conversion of an fp32 bias is: a row shard, which takes that, gives
+                            // the same bits as the whole tensor
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) o[e] = pack_bf16x2(v[2 * e], v[2 * e + 1]);
+                            for (int e = 0; e < 8; ++e) o[e] = pack_bf16x2(v[2 * e] * kLog2e, v[2 * e + 1] * kLog2e);
 #pragma unroll
                             for (int e = 0; e < 8; ++e) w[e] = (sw & 1) ? o[e ^ 4] : o[e];
                             stg256(trow + (long long)((t0 + k0) >> 5) * N * 32 + ((c2 ^ (sw & 2)) << 3), w);

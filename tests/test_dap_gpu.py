@@ -337,3 +337,26 @@ def test_both_projection_kernels_of_the_triangle_update_give_the_same_bits(pkg):
             torch.cuda.synchronize()
             pkg.lib.check_device_status()
             assert torch.equal(whole[0, :, :, :R, :], shard[0])
+
+
+@pytest.mark.parametrize("P,N", [(2, 66), (4, 200)])
+def test_row_shards_give_the_bits_of_the_whole_tensor(pkg, P, N):
+    """One block on P virtual ranks: the phases are the same kernels, and each value is summed in the same order wherever its
+    row lies."""
+    dev, bf, R = torch.device("cuda:0"), torch.bfloat16, N // P
+    g = torch.Generator().manual_seed(N + 2)
+    stack = pkg.PairFormerStack(**cases.OF3, **cases._PF_KW, no_blocks=1, blocks_per_ckpt=None)
+    stack.load_state_dict(pkg.weights.pairformer_stack_params(seed=4, no_blocks=1, final_std=None, **cases.OF3))
+    stack = stack.to(dev, bf).eval().requires_grad_(False)
+    block, ops = stack.blocks[0], pkg.dap.CudaOps(dev)
+    z, s = torch.randn(1, N, N, 128, generator=g).to(dev, bf), torch.randn(1, N, 384, generator=g).to(dev, bf)
+    pm, sm = cases.rand_mask((1, N, N), g).to(dev, bf), cases.rand_mask((1, N), g).to(dev, bf)
+    with torch.no_grad():
+        s_ref, z_ref = stack(s, z, sm, pm)
+        shards = [z[0, r * R:(r + 1) * R].clone() for r in range(P)]
+        shards = _virtual_pair_block(ops, shards, pm[0], block.pair_stack, P)
+        rows = [ops.single_rows(s[0], ops.pair_bias_project(shards[r], block.attn_pair_bias), sm[0], block, r * R, R)
+                for r in range(P)]
+    torch.cuda.synchronize()
+    pkg.lib.check_device_status()
+    assert torch.equal(torch.cat(shards), z_ref[0]) and torch.equal(torch.cat(rows), s_ref[0])

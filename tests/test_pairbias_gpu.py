@@ -47,3 +47,23 @@ def test_projection_against_fp64(N, shift):
     bound = 5 * 2.0**-8 / 3**0.5
     assert cases.rel_err(got.cpu(), ref) < bound, cases.rel_err(got.cpu(), ref)
     pkg.lib.check_device_status()
+
+
+@pytest.mark.parametrize("N", [5, 66, 130])
+def test_bias_tiles_equal_a_converted_bias(N):
+    """The two forms of a projected bias give the same attention, bit for bit: row-sharded callers project fp32 rows, whole
+    tensors the tiles."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator().manual_seed(N)
+    apb = pkg.AttentionPairBias(c_q=384, c_k=384, c_v=384, c_s=384, c_z=128, c_hidden=24, no_heads=16)
+    with torch.no_grad():
+        for p in apb.parameters():
+            p.copy_(torch.randn(p.shape, generator=g) * (p.shape[-1] ** -0.5 if p.dim() > 1 else 0.3) + (1.0 if p.dim() == 1 else 0.0))
+    apb = apb.to(dev, bf).eval().requires_grad_(False)
+    a, z = torch.randn(2, N, 384, generator=g).to(dev, bf), (1 + torch.randn(2, N, N, 128, generator=g)).to(dev, bf)
+    prm = (apb.layer_norm_z.weight, apb.layer_norm_z.bias, apb.linear_z.weight)
+    with torch.no_grad():
+        outs = [apb._run(a, z, None, None, in_place=False, pair_bias=bias)
+                for bias in (None, pkg.lib.pair_bias_project_tiles(z, *prm), pkg.lib.pair_bias_project(z, *prm))]
+    pkg.lib.check_device_status()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[1], outs[2])
