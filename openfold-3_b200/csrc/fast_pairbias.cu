@@ -270,7 +270,8 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                             for (int e = 0; e < 8; ++e) o[e] = pack_bf16x2(v[2 * e] * kLog2e, v[2 * e + 1] * kLog2e);
 #pragma unroll
                             for (int e = 0; e < 8; ++e) w[e] = (sw & 1) ? o[e ^ 4] : o[e];
-                            stg256(trow + (long long)((t0 + k0) >> 5) * N * 32 + ((c2 ^ (sw & 2)) << 3), w);
+                            stg256_or_2x128(trow + (long long)((t0 + k0) >> 5) * N * 32 + ((c2 ^ (sw & 2)) << 3), w,
+                                            aligned32(tiles));
                         } else if (l < layers) {
                             if (vec && k0 + 16 <= live) {
 #pragma unroll
@@ -324,7 +325,7 @@ int launch(const __nv_bfloat16* z, const BiasLayer* layer, int layers, float* ds
            long long layer_stride, long long lines, int N, cudaStream_t st) {
     if (lines <= 0 || N <= 0) return OF3_OK;
     OF3_REQUIRE(((uintptr_t)z & 15) == 0, OF3_ERR_ALIGN, "pair_bias: z must be 16-byte aligned");
-    OF3_REQUIRE(((uintptr_t)tiles & 31) == 0, OF3_ERR_ALIGN, "pair_bias: bias tiles must be 32-byte aligned");
+    OF3_REQUIRE(((uintptr_t)tiles & 15) == 0, OF3_ERR_ALIGN, "pair_bias: bias tiles must be 16-byte aligned");
     OF3_REQUIRE(lines < (1LL << 31), OF3_ERR_SHAPE, "pair_bias: too many pair positions");
     OF3_REQUIRE(layers >= 1 && layers <= kMaxBiasLayers, OF3_ERR_ARG, "pair_bias: %d layers", layers);
     PbWeights wts = {};

@@ -267,7 +267,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
                                                        sl * __uint_as_float(r[c2 * 8 + 2 * e + 1]));
 #pragma unroll
                                 for (int e = 0; e < 8; ++e) w[e] = (x & 1) ? o[e ^ 4] : o[e];
-                                stg256(dst + ((c2 ^ (x & 2)) << 3), w);
+                                stg256_or_2x128(dst + ((c2 ^ (x & 2)) << 3), w, aligned32(base));
                             }
                         }
                     }
@@ -749,7 +749,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
 #pragma unroll
                     for (int e = 0; e < 8; ++e)
                         o[e] = pack_bf16x2(__uint_as_float(r[2 * e]) * inv, __uint_as_float(r[2 * e + 1]) * inv);
-                    if (qpos < N && line_valid) stg256(dst + part * 16, o);
+                    if (qpos < N && line_valid) stg256_or_2x128(dst + part * 16, o, aligned32(o_out));
                 }
             } else if (lane == 0) {
                 report_wait_failure(status, abort_flag, kKidCore, 10);
@@ -1158,7 +1158,8 @@ int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, 
                     __nv_bfloat16* tb, int B, int R, int N, int row0, bool transposed,
                     const of3_triattn_params* p, cudaStream_t st, int C) {
     OF3_REQUIRE(((uintptr_t)z & 15) == 0, OF3_ERR_ALIGN, "triattn: z must be 16-byte aligned");
-    OF3_REQUIRE((((uintptr_t)q | (uintptr_t)k) & 31) == 0, OF3_ERR_ALIGN, "triattn: q / k images must be 32-byte aligned");
+    OF3_REQUIRE((((uintptr_t)q | (uintptr_t)k | (uintptr_t)vt) & 15) == 0, OF3_ERR_ALIGN,
+                "triattn: q / k / v images must be 16-byte aligned");
     OF3_REQUIRE(!transposed || R == N, OF3_ERR_SHAPE, "triattn: transposed view needs the whole tensor");
     if (C == 128)
         return transposed ? project_impl<128, true>(z, q, k, vt, tb, B, R, N, row0, p, st)
@@ -1174,7 +1175,8 @@ int triattn_finish(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloa
                    const __nv_bfloat16* tb, __nv_bfloat16* o, int B, int R, int N, float inf,
                    bool transposed, int add_residual, const of3_triattn_params* p, cudaStream_t st, int C) {
     OF3_REQUIRE(((uintptr_t)tb & 15) == 0, OF3_ERR_ALIGN, "triattn: the pair-bias image must be 16-byte aligned");
-    OF3_REQUIRE(((uintptr_t)o & 31) == 0, OF3_ERR_ALIGN, "triattn: the attention output must be 32-byte aligned");
+    OF3_REQUIRE((((uintptr_t)o | (uintptr_t)q | (uintptr_t)k | (uintptr_t)vt) & 15) == 0, OF3_ERR_ALIGN,
+                "triattn: the attention's output and operand images must be 16-byte aligned");
     OF3_REQUIRE(((uintptr_t)z & 15) == 0 && ((uintptr_t)out & 15) == 0, OF3_ERR_ALIGN,
                 "triattn: z/out must be 16-byte aligned");
     OF3_REQUIRE(N <= kMaxKeys, OF3_ERR_SHAPE, "triattn: N %d above the %d keys one CTA keeps a mask row for", N,

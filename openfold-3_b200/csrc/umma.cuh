@@ -286,6 +286,16 @@ __device__ __forceinline__ void stg256(void* p, const uint32_t (&o)[8]) {
                  "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7])
                  : "memory");
 }
+// the same where a caller's buffer may start on a 16-byte boundary only; `wide`: it starts on a 32-byte one
+__device__ __forceinline__ void stg256_or_2x128(void* p, const uint32_t (&o)[8], bool wide) {
+    if (wide) {
+        stg256(p, o);
+    } else {
+        reinterpret_cast<uint4*>(p)[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        reinterpret_cast<uint4*>(p)[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+}
+__device__ __forceinline__ bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
 __device__ __forceinline__ void ld_row16(const __nv_bfloat16* p, uint32_t (&o)[8]) {
     const uint4 a = *reinterpret_cast<const uint4*>(p), b = *reinterpret_cast<const uint4*>(p + 8);
     o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;

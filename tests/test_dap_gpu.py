@@ -360,3 +360,39 @@ def test_row_shards_give_the_bits_of_the_whole_tensor(pkg, P, N):
     torch.cuda.synchronize()
     pkg.lib.check_device_status()
     assert torch.equal(torch.cat(shards), z_ref[0]) and torch.equal(torch.cat(rows), s_ref[0])
+
+
+def test_operand_images_need_16_byte_alignment_only(pkg, monkeypatch):
+    """q, k, v, bias image, attention output and bias tiles 16 bytes past a 32-byte boundary (where the kernels store 32 bytes
+    at a time): same bits."""
+    dev, bf, N = torch.device("cuda:0"), torch.bfloat16, 70
+    g = torch.Generator().manual_seed(1)
+    blk = pkg.PairFormerBlock(**cases.OF3, **cases._PF_KW)
+    blk.load_state_dict(pkg.weights.pairformer_block_params(seed=6))
+    blk = blk.to(dev, bf).eval().requires_grad_(False)
+    att, apb = blk.pair_stack.tri_att_start, blk.attn_pair_bias
+    z = torch.randn(N, N, 128, generator=g).to(dev, bf)
+    ops = pkg.dap.CudaOps(dev)
+    empty = torch.empty
+
+    def run():
+        z1 = z.clone()
+        qkv, tb = ops.triattn_project(z1, att)
+        ops.triattn_finish(z1, None, qkv, tb, att)
+        return z1, pkg.lib.pair_bias_project_tiles(z[None], apb.layer_norm_z.weight, apb.layer_norm_z.bias, apb.linear_z.weight)
+
+    def shifted(*shape, dtype=None, device=None):
+        shape = shape[0] if len(shape) == 1 and not isinstance(shape[0], int) else shape
+        n = 1
+        for d in shape:
+            n *= d
+        return empty(n + 8, dtype=dtype, device=device)[8:].view(tuple(shape))
+
+    want = run()
+    monkeypatch.setattr(torch, "empty", shifted)
+    monkeypatch.setattr(torch, "empty_like", lambda t: shifted(*t.shape, dtype=t.dtype, device=t.device))
+    got = run()
+    monkeypatch.undo()
+    torch.cuda.synchronize()
+    pkg.lib.check_device_status()
+    assert got[1].data_ptr() % 32 == 16 and all(torch.equal(a, b) for a, b in zip(got, want))
