@@ -150,6 +150,11 @@ def _forward_only(module: nn.Module, *tensors):
         )
 
 
+def _aligned(t):
+    """t, or a copy that starts where the tensor-core kernels can read it (a view of a larger buffer may start anywhere)."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _PackedParams:
     """Caches contiguous copies of a module's parameters in the activation dtype."""
 
@@ -173,7 +178,7 @@ class _PackedParams:
         st = self._state
         # (the sources are held, so that a new tensor cannot come to lie at the address of one that is gone)
         if st is None or st[1] != key or any(a is not b for a, b in zip(st[0], tensors)):
-            val = [None if t is None else t.detach().to(device=device, dtype=dtype).contiguous() for t in tensors]
+            val = [None if t is None else _aligned(t.detach().to(device=device, dtype=dtype).contiguous()) for t in tensors]
             for group in adjacent:
                 if group and all(val[i] is not None for i in group):
                     block = torch.stack([val[i] for i in group])
@@ -302,6 +307,13 @@ def _same_device(like, **others):
             raise RuntimeError(f"{name} is on {t.device}, the call's tensors are on {like.device}")
 
 
+def _in_place(x, out):
+    """x after the layer has written ``out``: x's own memory, or an aligned copy of it."""
+    if x.is_contiguous() and out.data_ptr() != x.data_ptr():
+        return x.copy_(out.view(x.shape))
+    return out.view(x.shape)
+
+
 def _mask_like(mask, x):
     """mask [*] for x [*, C], broadcast, in the dtype of x."""
     if mask is None:
@@ -311,8 +323,8 @@ def _mask_like(mask, x):
 
 
 def _pair_batch(z, c_z):
-    """B of a pair tensor z [*, N, N, c_z], or None if z is no such tensor (or empty)."""
-    if z.dim() < 3 or z.shape[-3] != z.shape[-2] or z.shape[-1] != c_z or z.numel() == 0:
+    """B of a pair tensor z [*, N, N, c_z], or None if z is no such tensor, empty, or not where the kernels can read it."""
+    if z.dim() < 3 or z.shape[-3] != z.shape[-2] or z.shape[-1] != c_z or z.numel() == 0 or z.data_ptr() % 16:
         return None
     return z.numel() // (z.shape[-2] * z.shape[-2] * c_z)
 
@@ -358,13 +370,13 @@ class TriangleMultiplicativeUpdate(_Layer):
         _forward_only(self, z)
         in_place = inplace_safe and _add_with_inplace and not use_cueq_triangle_kernels and z.is_contiguous()
         N = z.shape[-2]
-        zc = z.contiguous().view(-1, N, N, self.c_z)
+        zc = _aligned(z.contiguous()).view(-1, N, N, self.c_z)
         m = _mask_like(mask, z)
         m = None if m is None else m.view(-1, N, N)
         out = zc if in_place else torch.empty_like(zc)
         lib.trimul_forward(zc, m, out, self._params(z.dtype, z.device), self.c_hidden, self._outgoing,
                            add_residual=in_place)
-        return z if in_place else out.view(z.shape)
+        return _in_place(z, out) if in_place else out.view(z.shape)
 
 
 class TriangleMultiplicationOutgoing(TriangleMultiplicativeUpdate):
@@ -397,13 +409,13 @@ class TriangleAttention(_Layer):
 
     def _run(self, x, mask, transposed: bool, in_place: bool):
         N = x.shape[-2]
-        xc = x.contiguous().view(-1, N, N, self.c_in)
+        xc = _aligned(x.contiguous()).view(-1, N, N, self.c_in)
         m = _mask_like(mask, x)
         m = None if m is None else m.view(-1, N, N)
         out = xc if in_place else torch.empty_like(xc)
         lib.triattn_forward(xc, m, out, self._params(x.dtype, x.device), self.no_heads, self.c_hidden,
                             self.inf, transposed, add_residual=in_place)
-        return out.view(x.shape)
+        return _in_place(x, out) if in_place else out.view(x.shape)
 
     def forward(self, x, mask=None, chunk_size=None, use_deepspeed_evo_attention=False,
                 use_cueq_triangle_kernels=False, use_lma=False, inplace_safe=False):
@@ -442,12 +454,12 @@ class SwiGLUTransition(_Layer):
     _adjacent = ((2, 3),)
 
     def _run(self, x, mask, in_place: bool):
-        xc = x.contiguous().view(-1, self.c_in)
+        xc = _aligned(x.contiguous()).view(-1, self.c_in)
         m = _mask_like(mask, x)
         m = None if m is None else m.view(-1)
         out = xc if in_place else torch.empty_like(xc)
         lib.transition_forward(xc, m, out, self._params(x.dtype, x.device), self.n, add_residual=in_place)
-        return out.view(x.shape)
+        return _in_place(x, out) if in_place else out.view(x.shape)
 
     def forward(self, x, mask=None, chunk_size=None, ckpt_chunk_size=None):
         """x [*, N, C_in], mask [*, N] -> update [*, N, C_in]."""
@@ -558,7 +570,7 @@ class AttentionPairBias(_Layer):
         diffusion rollout -- compute it once and pass it to ``_run(pair_bias=...)``. An opaque tensor: fp32
         [*, H, N, N], or for bf16 inputs the attention kernel's own bf16 bias tiles [*, 16, N / 32, N, 32]."""
         N = z.shape[-2]
-        zc = z.contiguous().view(-1, N, N, self.c_z)
+        zc = _aligned(z.contiguous()).view(-1, N, N, self.c_z)
         # three tensors only: the copies of the whole layer would stand beside those of a stack's native call
         packed = self.__dict__.setdefault("_packed_z", _PackedParams())
         prm = packed.get((self.layer_norm_z.weight, self.layer_norm_z.bias, self.linear_z.weight), z.dtype, z.device)
@@ -587,9 +599,9 @@ class AttentionPairBias(_Layer):
         while lead < len(batch) and zb[lead] == batch[lead]:
             lead += 1
         if all(d == 1 for d in zb[lead:]):
-            zc = z.contiguous().view(-1, N, N, self.c_z)
+            zc = _aligned(z.contiguous()).view(-1, N, N, self.c_z)
         else:
-            zc = z.expand(*batch, N, N, self.c_z).contiguous().view(-1, N, N, self.c_z)
+            zc = _aligned(z.expand(*batch, N, N, self.c_z).contiguous()).view(-1, N, N, self.c_z)
         sc = None
         if self.use_ada_layer_norm:
             if s is None:
@@ -692,7 +704,7 @@ class PairBlock(_Planned):
         """In place on the contiguous z with the prepared mask; False if the native path does not take this call."""
         st = _native_state(self, z)
         B = None if st is None else _pair_batch(z, self.tri_mul_out.c_z)
-        if B is None:   # (what has another shape is for the layers to refuse)
+        if B is None:   # (what has another shape is for the layers to refuse, or, not aligned, to copy)
             return False
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
         plan = st[0].shape(self, B, z.shape[-2], st[1], flags)

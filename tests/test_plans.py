@@ -228,3 +228,19 @@ def test_projecting_pair_biases_packs_no_second_copy_of_the_layer(pkg, monkeypat
         assert apb._packed._val is None
         assert all(torch.equal(x, y) for x, y in zip(prm, (apb.layer_norm_z.weight, apb.layer_norm_z.bias, apb.linear_z.weight))
                    if x is not None)
+
+
+def test_parameters_of_a_flat_buffer(pkg):
+    """Views at odd offsets, as a flattened or sharded model keeps them: the copies start where the kernels can read them."""
+    stack = diffusion(pkg).to(BF)
+    flat = torch.zeros(1 + sum(p.numel() + 1 for p in stack.parameters()), dtype=BF)
+    at = 1
+    for p in stack.parameters():
+        flat[at:at + p.numel()].copy_(p.view(-1))
+        p.data = flat[at:at + p.numel()].view(p.shape)
+        at += p.numel() + 1
+    plan = params(stack)
+    assert any(p.data_ptr() % 16 for p in stack.parameters())
+    pointers = [getattr(s, n) for array in plan.params for s in array for n, _ in s._fields_]
+    assert pointers and all(p is None or p % 16 == 0 for p in pointers)
+    assert torch.equal(plan.keep[11], stack.blocks[0].attention_pair_bias.mha.linear_q.weight)

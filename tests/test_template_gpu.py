@@ -62,3 +62,38 @@ def test_numerator_and_denominator_of_the_softmax_round_alike(c, N):
     exact = torch.einsum("bhqk,bkhd->bqhd", p, v).reshape(4, N, c)
     rounding = (exact.to(bf).double() - exact).norm()
     assert ((got - exact).norm() / rounding).item() < 1.04
+
+
+@pytest.mark.parametrize("kind", ["template", "f32"])
+def test_tensors_that_start_anywhere(kind):
+    """A pair tensor one element into its buffer, in place and not: what a kernel cannot read where it lies is copied first.
+    Same bits as for an aligned one."""
+    dev, N = torch.device("cuda:0"), 20
+    dt = torch.bfloat16 if kind == "template" else torch.float32
+    dims = TEMPLATE if kind == "template" else PAIR
+    g = torch.Generator().manual_seed(3)
+    single = dict(c_s=384, c_hidden_pair_bias=24, no_heads_pair_bias=16)
+    blk = pkg.PairBlock(**dims, **_PF_KW) if kind == "template" else pkg.PairFormerBlock(**dims, **single, **_PF_KW)
+    with torch.no_grad():
+        for p in blk.parameters():
+            p.copy_(torch.randn(p.shape, generator=g) * (0.5 * p.shape[-1] ** -0.5 if p.dim() > 1 else 0.3))
+    blk = blk.to(dev, dt).eval().requires_grad_(False)
+    z, s = torch.randn(1, N, N, dims["c_z"], generator=g).to(dev, dt), torch.randn(1, N, 384, generator=g).to(dev, dt)
+    pair = blk if kind == "template" else blk.pair_stack
+    call = (lambda z, **k: (blk(z, None, **k),)) if kind == "template" else (lambda z, **k: blk(s.clone(), z, None, None, **k))
+    layers = (pair.tri_mul_in, pair.tri_att_start, pair.tri_att_end, pair.pair_transition)
+
+    def odd():
+        buf = torch.empty(z.numel() + 1, dtype=dt, device=dev)
+        return buf[1:].view(z.shape).copy_(z)
+
+    with torch.no_grad():
+        want, each = call(z.clone()), [m(z) for m in layers]
+        inside = odd()
+        assert inside.data_ptr() % 16
+        got = call(inside, inplace_safe=True)
+        assert got[-1].data_ptr() == inside.data_ptr()
+        for x in (got, call(odd())):
+            assert all(torch.equal(a, b) for a, b in zip(x, want))
+        assert all(torch.equal(m(odd()), w) for m, w in zip(layers, each))
+    pkg.lib.check_device_status()
