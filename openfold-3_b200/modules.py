@@ -688,7 +688,7 @@ class PairBlock(_Planned):
         return [*mul, self.ps_dropout_row_layer], [*mul, *att, self.pair_transition]
 
     def _native_params(self, layers, tensors, dtype, device):
-        parts = [m._packed.get(t, dtype, device, m._adjacent) for m, t in zip(layers, tensors)]
+        parts = [m._packed.get(t, dtype, device) for m, t in zip(layers, tensors)]   # (nothing here is read back to back)
         kinds = (lib.TrimulParams, lib.TrimulParams, lib.TriattnParams, lib.TriattnParams, lib.TransitionParams)
         return lib.PairBlockParams(*[k(*_pointers(p)) for k, p in zip(kinds, parts)]), parts
 
@@ -773,7 +773,7 @@ class PairFormerBlock(_Planned):
 
     def _native_params(self, layers, tensors, dtype, device):
         pair, keep = self.pair_stack._native_params(layers[:5], tensors[:5], dtype, device)
-        attn, trans = (m._packed.get(t, dtype, device, m._adjacent) for m, t in zip(layers[5:], tensors[5:]))
+        attn, trans = (m._packed.get(t, dtype, device) for m, t in zip(layers[5:], tensors[5:]))
         return (lib.PairformerBlockParams(pair, lib.AttnPairBiasParams(*_pointers(attn)),
                                           lib.TransitionParams(*_pointers(trans))), (keep, attn, trans))
 

@@ -244,3 +244,13 @@ def test_parameters_of_a_flat_buffer(pkg):
     pointers = [getattr(s, n) for array in plan.params for s in array for n, _ in s._fields_]
     assert pointers and all(p is None or p % 16 == 0 for p in pointers)
     assert torch.equal(plan.keep[11], stack.blocks[0].attention_pair_bias.mha.linear_q.weight)
+
+
+def test_a_block_copies_no_weights_that_can_be_read_where_they_are(pkg):
+    blk = pkg.PairFormerBlock(c_s=64, c_z=64, c_hidden_pair_bias=4, no_heads_pair_bias=16, c_hidden_mul=64, c_hidden_pair_att=16,
+                              no_heads_pair=4, transition_type="swiglu", transition_n=2, pair_dropout=0.25,
+                              fuse_projection_weights=False, inf=1e9).eval().to(BF).requires_grad_(False)
+    plan = blk._plans.get(blk, BF, CPU)
+    own = {p.data_ptr() for p in blk.parameters()}
+    pair, attn, trans = plan.keep
+    assert all(t is None or t.data_ptr() in own for ts in (*pair, attn, trans) for t in ts)
