@@ -224,7 +224,7 @@ int of3_cond_transition_forward(const void* a, const void* s, const void* mask, 
 
 /* ---- Whole blocks ------------------------------------------------------------------------
  * One call per block instead of one per layer: the block's layers are enqueued by native code (a block of a short
- * sequence is some thirty launches of a few microseconds, and issuing them one layer at a time from a scripting
+ * sequence is some twenty launches of a few microseconds, and issuing them one layer at a time from a scripting
  * language takes longer than they run).
  * of3_pair_block_forward replaces PairBlock.forward (openfold3/core/model/latent/base_blocks.py:406-480), in place on
  * z [B, N, N, c_z]; pair_mask [B, N, N] or NULL.
@@ -265,7 +265,8 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
  * diffusion_transformer.py:263-322, 116-179), in place on a [Ba, N, c_a]: per block attention with pair bias (AdaLN
  * variant with OF3_FLAG_ADA_LN), then the conditioned transition. s [Ba, N, c_s]; z [Bz, N, N, c_z] (Ba a multiple of
  * Bz, samples that share a pair tensor consecutive), or bias[block]: the blocks' pair biases, projected earlier
- * (of3_pair_bias_project_tiles for the bf16 tensor-core attention, else of3_pair_bias_project), and z NULL.
+ * (the form that of3_pair_bias_takes_tiles names: of3_pair_bias_project_tiles or of3_pair_bias_project), and z NULL.
+ * With z the workspace holds the bias images of up to 24 blocks, as many as fit 1 GiB (0.45 GB at N = 768, Bz = 1).
  * The projections of s are computed for several blocks per launch when those of all layers lie back to back:
  * [block][attention, transition][gate, shift, output gate][c_a][c_s]. */
 typedef struct {

@@ -1,7 +1,7 @@
 // Whole blocks of the Pairformer, and the whole diffusion token stack, behind one C call each: the same layers in the
-// same order as the module entry points of api.cu, issued by native code. A pair block is 13 launches and the single track of a block 9 more; from
-// Python, one layer call at a time, they cost about 13 us of host time each (400 us per block: the 4-block trunk at
-// N = 37 took 1.6 ms for 0.3 ms of device work, and so did N = 256).
+// same order as the module entry points of api.cu, issued by native code. A pair block is 13 launches and the single
+// track of a block 8 more; from Python, one layer call at a time, a block cost about 400 us of host time (the 4-block trunk
+// at N = 37 took 1.6 ms for 0.3 ms of device work, and so did N = 256).
 #include "fast_pairbias.cuh"
 #include "fast_single.cuh"
 #include "generic_ops.cuh"
@@ -111,7 +111,8 @@ int single_track(void* s, const void* z, const void* bias, BiasForm form, const 
 // several of them: with few rows the projections of one block (6 matrices of c_a x c_s) fill a fraction of the chip and
 // cost a launch each; with many rows one block fills it, and its planes should stay in L2 until they are read.
 constexpr size_t kCondGroupBytes = 32u << 20;
-// Room for the bias images of the blocks whose pair bias one pass over z projects (24 blocks up to N = 1150).
+// Room for the bias images of the blocks whose pair bias one pass over z projects (24 blocks up to N = 1150): 24 x 18.9 MB
+// of the workspace at N = 768, for 225 us instead of 24 passes of 56.
 constexpr size_t kBiasGroupBytes = 1u << 30;
 
 int diffusion_stack(void* a, const void* s, const void* z, const void* mask, const void* const* bias,

@@ -25,7 +25,7 @@ namespace {
 using namespace umma;
 typedef __nv_bfloat16 bf16;
 constexpr int kKidSingle = 8;
-constexpr int kKidLinear = 10;  // linear layers on the contraction kernel: accounted apart from the triangle einsum
+constexpr int kKidLinear = 10;  // linear layers, those on the contraction kernel too (accounted apart from the triangle einsum)
 constexpr float kEps = 1e-5f;
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -36,7 +36,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // ---------------------------------------------------------------- LayerNorm of rows, one warp per row
 // The row stays in registers: NV vectors of 8 values per lane (lane, lane + 32, ...), one 16-byte load each. (Re-reading
-// it three times with 2-byte loads, as for rows beyond 1024 values below, took 8 - 20 us for 3840 rows.)
+// it three times with 2-byte loads took 8 - 20 us for 3840 rows.)
 template <int NV>
 struct Row {
     float x[NV * 8];
@@ -230,7 +230,8 @@ int conditioning(const bf16* s, const CondLayer* layer, int layers, long long ro
     {
         // few rows: the layers are spread over blocks too
         const unsigned gx = row_blocks(rows);
-        unsigned gy = gx >= 296u ? 1u : (unsigned)(296 / gx + 1);
+        const unsigned want = 2u * (unsigned)sm_count();
+        unsigned gy = gx >= want ? 1u : want / gx + 1;
         if (gy > (unsigned)layers) gy = layers;
         LaunchScope scope(kKidSingle, st);
         BY_WIDTH(c_s, OF3_CUDA_CHECK(launch_chained(cond_rows_kernel<NV>, dim3(gx, gy), 256, 0, st, s, cw, layers, sn, rows,

@@ -5,7 +5,7 @@
 //               (tcgen05: the weights are the A operand, the normalised tile the B operand, so a TMEM lane is an
 //               output channel and its columns are the tile's 128 positions) -> mask * sigmoid(gate) * proj ->
 //               a, b stored CHANNEL-MAJOR with the contracted index innermost, a_t[c][i][k], b_t[c][j][k]:
-//               every epilogue thread writes its channel's 256 contiguous bytes with 16-byte stores.
+//               every epilogue thread writes its channel's 256 contiguous bytes with 32-byte stores.
 //               For the incoming update the tile walks z along its first index instead, so that
 //               both directions feed the same K-major x K-major contraction.
 //   contract    x_t[c][i][j] = sum_k a_t[c][i][k] * b_t[c][j][k]      (contract.cu)
@@ -379,9 +379,9 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
 
 // The same layer with the projections the other way round (the normalised tile is the A operand, a TMEM lane is a
 // position, its columns the output channels; N = 256 per MMA): a warp's store covers 32 consecutive positions of ONE
-// channel plane. For planes only: slower than the kernel above while one stays within a 2 MB page or so (170 against
-// 151 us at N = 768: one 2-byte store per value), faster beyond (1.13 against 2.02 ms at N = 2048, where the 32
-// planes one store of the kernel above touches lie megabytes apart).
+// channel plane. For planes only (row shards): slower than the kernel above while one stays within a 2 MB page or so (170
+// against 151 us for the planes of a whole tensor at N = 768: one 2-byte store per value), faster beyond (1.13 against
+// 2.02 ms at N = 2048, where the 32 planes that one store of the kernel above touches lie megabytes apart).
 constexpr int kInRowsThreads = 448;  // producer, MMA, 4 LayerNorm warps, 2 x 4 epilogue warps
 
 template <bool kOutgoing>

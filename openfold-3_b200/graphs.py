@@ -1,6 +1,6 @@
 """One CUDA graph per forward call of a module whose step is a long chain of small launches.
 
-The diffusion token stack is about 500 launches of a few microseconds each per step: issued one by one the GPU waits
+The diffusion token stack is about 220 launches of a few microseconds each per step: with few tokens the GPU may wait
 for the host between them. ``GraphedModule`` captures one forward call (all kernels, on every stream the module uses)
 into a ``torch.cuda.CUDAGraph`` and replays it; inputs are copied into the buffers the graph was captured with, so they
 may be device tensors or pinned host tensors (the copy is then the upload). Shapes, dtypes and which arguments are

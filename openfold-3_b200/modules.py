@@ -173,7 +173,7 @@ class _PackedParams:
 
     def get(self, tensors, dtype, device, adjacent=()):
         """``adjacent``: groups of indices of equally shaped tensors whose copies are laid out back to back in one
-        allocation (the library then runs linear layers that share an input as one launch)."""
+        allocation (the library then runs the projections of the conditioning s as one launch)."""
         key = (dtype, device, tuple((t.data_ptr(), t._version) if t is not None else None for t in tensors))
         st = self._state
         # (the sources are held, so that a new tensor cannot come to lie at the address of one that is gone)

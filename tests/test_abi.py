@@ -83,9 +83,9 @@ def test_state_dict_keys_match_reference_layout(pkg):
 
 
 def test_modules_pack_grouped_weights_back_to_back(pkg):
-    """Linear layers that share an input run as one launch when their weights lie back to back in memory (the
-    library compares addresses): the modules' parameter packer must lay q | g | k | v, the AdaLN pair and the
-    SwiGLU pair out that way, with unchanged values."""
+    """The projections of the conditioning run as one launch when their weights lie back to back in memory (the
+    library compares addresses): the modules' parameter packer must lay them out that way, and q | g | k | v and the
+    SwiGLU pair too, with unchanged values."""
     dt, dev = torch.bfloat16, torch.device("cpu")
     apb = pkg.AttentionPairBias(c_q=768, c_k=768, c_v=768, c_s=384, c_z=128, c_hidden=48, no_heads=16,
                                 use_ada_layer_norm=True, inf=1e9)

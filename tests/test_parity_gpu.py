@@ -183,8 +183,8 @@ def test_diffusion_stack_hoists_the_pair_bias_of_an_unchanged_pair_tensor(pkg, d
 
 
 def test_grouped_linear_launches_equal_separate_launches(pkg):
-    """q | g | k | v and the AdaLN / SwiGLU pairs run as one launch each when their weights lie back to back (how the
-    modules pack them); with every weight in an allocation of its own they run one by one. Same bits either way."""
+    """The projections of the conditioning run as one launch when their weights lie back to back (how the modules pack
+    them); with every weight in an allocation of its own they run one by one. Same bits either way."""
     dev = torch.device("cuda:0")
     bf = torch.bfloat16
     g = torch.Generator().manual_seed(77)
