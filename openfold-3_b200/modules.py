@@ -209,14 +209,16 @@ class _Plan:
     ``called``: the modules that the layer-by-layer path runs as a caller would, with their hooks; ``layers``: those whose
     parameters and constants the native path reads."""
 
-    __slots__ = ("dtype", "device", "hooks", "forwards", "watch", "held", "params", "keep", "shapes", "called")
+    __slots__ = ("dtype", "device", "forwards", "watch", "held", "params", "keep", "shapes", "called", "c_z", "c_s", "code")
 
     def __init__(self, block, called, layers, dtype, device):
         self.dtype, self.device, self.params, self.keep, self.shapes = dtype, device, None, None, {}
+        self.c_z, self.c_s = layers[0].c_z, getattr(layers[-2], "c_q", 0)   # (of a pair or Pairformer block)
+        self.code = lib.dtype_code(dtype)
         self.called = False   # the copies of the weights may be the last work on the stream
-        self.hooks = [h for m in called for h in (m._forward_hooks, m._forward_pre_hooks)]
-        self.hooks += [_nn_module._global_forward_hooks, _nn_module._global_forward_pre_hooks]
-        self.forwards = [(c, c.forward) for c in {type(m) for m in called}]
+        hooks = [h for m in called for h in (m._forward_hooks, m._forward_pre_hooks)]
+        hooks += [_nn_module._global_forward_hooks, _nn_module._global_forward_pre_hooks]
+        self.forwards = [(c, _OWN_FORWARDS[c]) for c in {type(m) for m in called}]
         owned, children, tree = [], [], [block]
         for m in tree:   # (grows)
             if m._parameters:
@@ -235,18 +237,21 @@ class _Plan:
         known = {id(t) for d in owned for t in d.values()}
         tensors = [m._tensors() for m in layers]
         # (a weight that is not a parameter, computed or a plain tensor, may change unseen: layer by layer)
-        if (not any(n in d for d, n in replaced) and not any("parametrizations" in c for c in children)
+        if (not any(hooks) and not any(n in d for d, n in replaced) and self.as_written() and not any("parametrizations" in c for c in children)
                 and all(t is None or id(t) in known for ts in tensors for t in ts)):
-            found = w.make(owned, children, attrs)
-        self.watch, self.held = found or w.make([], owned + children, attrs)
+            found = w.make(owned, children + hooks, attrs)
+        self.watch, self.held = found or w.make([], owned + children + hooks, attrs)
         if found:
             self.params, self.keep = block._native_params(layers, tensors, dtype, device)
 
     def current(self, dtype, device):
         return dtype == self.dtype and device == self.device and not _watch_module.changed(self.watch)
 
-    def usable(self):
-        return self.params is not None and not any(self.hooks) and all(c.forward is f for c, f in self.forwards)
+    def as_written(self):
+        for c, f in self.forwards:   # (classes may be patched)
+            if c.forward is not f:
+                return False
+        return True
 
     def shape(self, block, *key):
         p = self.shapes.get(key)
@@ -273,7 +278,7 @@ class _BlockPlans:
         if plan is None or not plan.current(dtype, device):
             parts = block._plan_submodules()
             plan = self._plan = None if parts is None else _Plan(block, *parts, dtype, device)
-        if plan is None or not plan.usable():
+        if plan is None or plan.params is None or not plan.as_written():
             return None
         lib.hold(plan.keep)
         return plan
@@ -289,22 +294,20 @@ class _Planned(nn.Module):
 
 
 def _native_state(block, z):
-    """(plan, dtype code) for the native path of ``block`` on z, or None."""
+    """The plan for the native path of ``block`` on z, or None."""
     if not z.is_cuda or block.training or z.dtype not in (torch.bfloat16, torch.float32):
         return None
-    plan = block._plans.get(block, z.dtype, z.device)
-    return None if plan is None else (plan, lib.dtype_code(z.dtype))
+    return block._plans.get(block, z.dtype, z.device)
 
 
 def _pointers(tensors):
     return [None if t is None else t.data_ptr() for t in tensors]
 
 
-def _same_device(like, **others):
+def _same_device(like, t, name):
     """The kernels take addresses: a tensor of another device, or of the host, must not get that far."""
-    for name, t in others.items():
-        if t is not None and t.device != like.device:
-            raise RuntimeError(f"{name} is on {t.device}, the call's tensors are on {like.device}")
+    if t is not None and t.device != like.device:
+        raise RuntimeError(f"{name} is on {t.device}, the call's tensors are on {like.device}")
 
 
 def _in_place(x, out):
@@ -318,15 +321,16 @@ def _mask_like(mask, x):
     """mask [*] for x [*, C], broadcast, in the dtype of x."""
     if mask is None:
         return None
-    _same_device(x, mask=mask)
+    _same_device(x, mask, "mask")
     return mask.to(x.dtype).expand(x.shape[:-1]).contiguous()
 
 
 def _pair_batch(z, c_z):
     """B of a pair tensor z [*, N, N, c_z], or None if z is no such tensor, empty, or not where the kernels can read it."""
-    if z.dim() < 3 or z.shape[-3] != z.shape[-2] or z.shape[-1] != c_z or z.numel() == 0 or z.data_ptr() % 16:
+    shape = z.shape
+    if len(shape) < 3 or shape[-3] != shape[-2] or shape[-1] != c_z or z.numel() == 0 or z.data_ptr() % 16:
         return None
-    return z.numel() // (z.shape[-2] * z.shape[-2] * c_z)
+    return z.numel() // (shape[-2] * shape[-2] * c_z)
 
 
 class _Layer(nn.Module):
@@ -492,7 +496,7 @@ class ConditionedTransitionBlock(_Layer):
     _adjacent = (_cond_group, (4, 5))
 
     def _run(self, a, s, mask, in_place: bool):
-        _same_device(a, s=s)
+        _same_device(a, s, "s")
         ac = a.contiguous().view(-1, self.c_a)
         sc = s.expand(*a.shape[:-1], self.c_s).contiguous().view(-1, self.c_s)
         m = _mask_like(mask, a)
@@ -588,7 +592,8 @@ class AttentionPairBias(_Layer):
     def _operands(self, a, z, s, mask):
         """a [Ba, N, C], z [Bz, N, N, C_z], s, mask as the kernels take them: samples that share a pair tensor are
         consecutive."""
-        _same_device(a, z=z, s=s)
+        _same_device(a, z, "z")
+        _same_device(a, s, "s")
         N = a.shape[-2]
         batch = a.shape[:-2]
         ac = a.contiguous().view(-1, N, self.c_q)
@@ -702,13 +707,13 @@ class PairBlock(_Planned):
 
     def _run_native(self, z, pair_mask, mask_trans):
         """In place on the contiguous z with the prepared mask; False if the native path does not take this call."""
-        st = _native_state(self, z)
-        B = None if st is None else _pair_batch(z, self.tri_mul_out.c_z)
+        plan = _native_state(self, z)
+        B = None if plan is None else _pair_batch(z, plan.c_z)
         if B is None:   # (what has another shape is for the layers to refuse, or, not aligned, to copy)
             return False
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
-        plan = st[0].shape(self, B, z.shape[-2], st[1], flags)
-        lib.pair_block_forward(z, pair_mask, plan, st[1], flags, st[0].params)
+        shape = plan.shape(self, B, z.shape[-2], plan.code, flags)
+        lib.pair_block_forward(z, pair_mask, shape, plan.code, flags, plan.params)
         return True
 
     def tri_mul_out_in(self, z, pair_mask, inplace_safe, use_cueq_triangle_kernels=False):
@@ -786,17 +791,16 @@ class PairFormerBlock(_Planned):
     def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None, continues=False):
         """In place on contiguous s and z with prepared masks; False if the native path does not take this call.
         ``continues``: the last work on the stream is another block's native call."""
-        st = _native_state(self, z)
-        attn = self.attn_pair_bias
-        B = None if st is None else _pair_batch(z, attn.c_z)
-        if B is None or s.dtype != z.dtype or s.shape[:-1] != z.shape[:-2] or s.shape[-1] != attn.c_q:
+        plan = _native_state(self, z)
+        B = None if plan is None else _pair_batch(z, plan.c_z)
+        if B is None or s.dtype != z.dtype or s.shape != (*z.shape[:-2], plan.c_s):
             return False
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
-        plan = st[0].shape(self, B, z.shape[-2], st[1], flags)
-        if continues and st[0].called:
+        shape = plan.shape(self, B, z.shape[-2], plan.code, flags)
+        if continues and plan.called:
             flags |= lib.FLAG_CONTINUES
-        st[0].called = True
-        lib.pairformer_block_forward(s, z, single_mask, pair_mask, plan, st[1], flags, st[0].params, side)
+        plan.called = True
+        lib.pairformer_block_forward(s, z, single_mask, pair_mask, shape, plan.code, flags, plan.params, side)
         return True
 
     def forward(self, s, z, single_mask, pair_mask, chunk_size=None, use_deepspeed_evo_attention=False,
@@ -804,7 +808,7 @@ class PairFormerBlock(_Planned):
                 _attn_chunk_size=None):
         _forward_only(self, s, z)
         if z.is_cuda and not self.training:
-            _same_device(z, s=s)
+            _same_device(z, s, "s")
             z = z if inplace_safe and z.is_contiguous() else z.clone(memory_format=torch.contiguous_format)
             s = s if inplace_safe and s.is_contiguous() else s.clone(memory_format=torch.contiguous_format)
             inplace_safe = True
@@ -852,7 +856,7 @@ class PairFormerStack(nn.Module):
         if not (inplace_safe and s.is_contiguous()):
             s = s.clone(memory_format=torch.contiguous_format)
         if z.is_cuda:   # prepared once for all blocks
-            _same_device(z, s=s)
+            _same_device(z, s, "s")
             pair_mask = _mask_like(pair_mask, z)
             single_mask = _mask_like(single_mask, s)
         if not (self.overlap_single_track and z.is_cuda and len(self.blocks) > 1
@@ -1022,20 +1026,20 @@ class DiffusionTransformer(_Planned):
 
     def _run_native(self, a, s, z, mask, mask_trans):
         """In place on the contiguous a; False if the native path does not take this call."""
-        st = _native_state(self, a)
-        if st is None or z.dtype != a.dtype or s is None or s.dtype != a.dtype:
+        plan = _native_state(self, a)
+        if plan is None or z.dtype != a.dtype or s is None or s.dtype != a.dtype:
             return False
         m0 = self.blocks[0].attention_pair_bias
         if not m0.use_ada_layer_norm:   # the attention takes no s then, the transitions still do
             return False
         ac, zc, sc, m = m0._operands(a, z, s, mask)
-        biases = self._pair_biases(z, token=st[0])
+        biases = self._pair_biases(z, token=plan)
         if ac.numel() == 0 or not all(b is None or m0._bias_fits(b, zc) for b in biases):
             return False   # (for the layers to refuse)
         flags = (lib.extra_flags | lib.FLAG_ADA_LN) | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
         lib.hold(biases)
-        plan = st[0].shape(self, ac.shape[0], zc.shape[0], a.shape[-2], st[1], flags, biases[0] is not None)
-        lib.diffusion_stack_forward(ac, sc, zc, m, biases, plan, st[1], flags, st[0].params)
+        shape = plan.shape(self, ac.shape[0], zc.shape[0], a.shape[-2], plan.code, flags, biases[0] is not None)
+        lib.diffusion_stack_forward(ac, sc, zc, m, biases, shape, plan.code, flags, plan.params)
         return True
 
     def _pair_biases(self, z, token=None):
@@ -1078,3 +1082,7 @@ class DiffusionTransformer(_Planned):
             a = b(a, s, z, mask=mask, use_high_precision_attention=use_high_precision_attention,
                   _mask_trans=_mask_trans, _in_place=True, _pair_bias=pb)
         return a
+
+
+_OWN_FORWARDS = {c: c.forward for c in (TriangleMultiplicationOutgoing, TriangleMultiplicationIncoming, DropoutRowwise, PairBlock,
+                                        DiffusionTransformerBlock)}
