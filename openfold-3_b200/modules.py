@@ -705,14 +705,18 @@ class PairBlock(_Planned):
     def _native_plan(self, B, N, dtype, flags):
         return lib.BlockPlan(self._native_dims(B, N), dtype, flags, single=False)
 
-    def _run_native(self, z, pair_mask, mask_trans):
-        """In place on the contiguous z with the prepared mask; False if the native path does not take this call."""
+    def _run_native(self, z, pair_mask, mask_trans, continues=False):
+        """In place on the contiguous z with the prepared mask; False if the native path does not take this call.
+        ``continues``: the last work on the stream is another block's native call."""
         plan = _native_state(self, z)
         B = None if plan is None else _pair_batch(z, plan.c_z)
         if B is None:   # (what has another shape is for the layers to refuse, or, not aligned, to copy)
             return False
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)
         shape = plan.shape(self, B, z.shape[-2], plan.code, flags)
+        if continues and plan.called:
+            flags |= lib.FLAG_CONTINUES
+        plan.called = True
         lib.pair_block_forward(z, pair_mask, shape, plan.code, flags, plan.params)
         return True
 
@@ -914,8 +918,12 @@ class PairStack(nn.Module):
             z = z.clone(memory_format=torch.contiguous_format)
         if z.is_cuda:   # prepared once for all blocks
             pair_mask = _mask_like(pair_mask, z)
+        native = False
         for b in self.blocks:
-            z = b(z, pair_mask, inplace_safe=True, _mask_trans=_mask_trans)
+            # the block's native call itself, where a call of the block would run nothing else: no caller's work in between
+            native = _runs_as_written(b) and b._run_native(z, pair_mask, _mask_trans, continues=native)
+            if not native:
+                z = b(z, pair_mask, inplace_safe=True, _mask_trans=_mask_trans)
         return z
 
 
@@ -1082,6 +1090,14 @@ class DiffusionTransformer(_Planned):
             a = b(a, s, z, mask=mask, use_high_precision_attention=use_high_precision_attention,
                   _mask_trans=_mask_trans, _in_place=True, _pair_bias=pb)
         return a
+
+
+def _runs_as_written(m):
+    """A call of m runs its own class's ``forward`` and nothing else."""
+    c = type(m)
+    return (c in _OWN_FORWARDS and c.forward is _OWN_FORWARDS[c] and "forward" not in m.__dict__
+            and not (m._forward_hooks or m._forward_pre_hooks or _nn_module._global_forward_hooks
+                     or _nn_module._global_forward_pre_hooks))
 
 
 _OWN_FORWARDS = {c: c.forward for c in (TriangleMultiplicationOutgoing, TriangleMultiplicationIncoming, DropoutRowwise, PairBlock,

@@ -4,7 +4,7 @@ as the layers refuse them. The library calls are recorded instead of made; nothi
 import pytest
 import torch
 
-from cases import DIFF, OF3, _PF_KW
+from cases import DIFF, OF3, PAIR, _PF_KW
 
 BF = torch.bfloat16
 
@@ -150,3 +150,23 @@ def test_only_blocks_behind_a_block_continue(pkg, monkeypatch):
     assert call() == [False, False, False] and call() == [False, True, True]
     stack.blocks[1].single_transition.linear_out.weight.mul_(2)
     assert call() == [False, False, True] and call() == [False, True, True]
+
+
+def test_a_pair_stack_continues_from_block_to_block(pkg, monkeypatch):
+    """But not past a block that is run by a call of its own, with its hooks."""
+    stack = pkg.PairStack(no_blocks=3, **{k: v for k, v in OF3.items() if k in PAIR}, **_PF_KW).eval().to(BF).requires_grad_(False)
+    flags, hooked = [], []
+    monkeypatch.setattr(pkg.lib, "pair_block_forward",
+                        lambda z, pm, plan, dt, f, prm: flags.append(bool(f & pkg.lib.FLAG_CONTINUES)))
+
+    def call():
+        del flags[:]
+        with torch.no_grad():
+            stack(gpu(1, 20, 20, 128), None)
+        return flags
+
+    assert call() == [False, False, False] and call() == [False, True, True]
+    hook = stack.blocks[1].register_forward_pre_hook(lambda m, args: hooked.append(m))
+    assert call() == [False, False, False] and hooked == [stack.blocks[1]]
+    hook.remove()
+    assert call() == [False, True, True]
