@@ -202,9 +202,13 @@ def _param_watch():
     return _watch_module
 
 
+_PAIR_BLOCK_STEPS = ("tri_mul_out_in", "tri_att_start_end")   # methods of PairBlock that its forward runs
+
+
 class _Plan:
     """What a native call of a block (or stack) needs, for one dtype and device, and the means to tell whether it still
-    holds. Nothing in it changes after it was built but the cache of what depends on the shape.
+    holds. Nothing in it changes after it was built but the cache of what depends on the shape. It refers to the parts of the
+    block (the watch needs them to live), never to the block itself, which would then live until the next garbage collection.
 
     ``called``: the modules that the layer-by-layer path runs as a caller would, with their hooks; ``layers``: those whose
     parameters and constants the native path reads."""
@@ -228,8 +232,7 @@ class _Plan:
                 tree += [c for c in m._modules.values() if c is not None]
         attrs = [(m.__dict__, n) for m in layers for n in m._plan_constants]
         replaced = [(m.__dict__, "forward") for m in called]
-        replaced += [(m.__dict__, n) for m in (block, *called) for n in ("tri_mul_out_in", "tri_att_start_end")
-                     if isinstance(m, PairBlock)]
+        replaced += [(m.__dict__, n) for m in called if isinstance(m, PairBlock) for n in _PAIR_BLOCK_STEPS]
         attrs += replaced
         attrs += [(m.__dict__, "training") for m in called if isinstance(m, DropoutRowwise)]
         w = _param_watch()
@@ -709,7 +712,7 @@ class PairBlock(_Planned):
         """In place on the contiguous z with the prepared mask; False if the native path does not take this call.
         ``continues``: the last work on the stream is another block's native call."""
         plan = _native_state(self, z)
-        B = None if plan is None else _pair_batch(z, plan.c_z)
+        B = None if plan is None or any(n in self.__dict__ for n in _PAIR_BLOCK_STEPS) else _pair_batch(z, plan.c_z)
         if B is None:   # (what has another shape is for the layers to refuse, or, not aligned, to copy)
             return False
         flags = lib.extra_flags | (0 if mask_trans else lib.FLAG_NO_TRANSITION_MASK)

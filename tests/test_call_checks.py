@@ -170,3 +170,12 @@ def test_a_pair_stack_continues_from_block_to_block(pkg, monkeypatch):
     assert call() == [False, False, False] and hooked == [stack.blocks[1]]
     hook.remove()
     assert call() == [False, True, True]
+
+
+def test_a_replaced_step_of_a_pair_block_is_run(pkg, calls):
+    blk = pkg.PairBlock(**{k: v for k, v in OF3.items() if k in PAIR}, **_PF_KW).eval().to(BF).requires_grad_(False)
+    seen = []
+    blk.tri_mul_out_in = lambda z, *a, **k: seen.append("step") or z
+    with torch.no_grad():
+        blk(gpu(1, 20, 20, 128), None)
+    assert seen == ["step"] and "pair_block_forward" not in calls

@@ -2,9 +2,11 @@
 built from stays the same, built again when it changes. Everything here runs without a GPU (no kernel is called)."""
 
 import copy
+import gc
 import pickle
 import sys
 import threading
+import weakref
 
 import pytest
 import torch
@@ -247,10 +249,30 @@ def test_parameters_of_a_flat_buffer(pkg):
 
 
 def test_a_block_copies_no_weights_that_can_be_read_where_they_are(pkg):
-    blk = pkg.PairFormerBlock(c_s=64, c_z=64, c_hidden_pair_bias=4, no_heads_pair_bias=16, c_hidden_mul=64, c_hidden_pair_att=16,
-                              no_heads_pair=4, transition_type="swiglu", transition_n=2, pair_dropout=0.25,
-                              fuse_projection_weights=False, inf=1e9).eval().to(BF).requires_grad_(False)
+    blk = pairformer_block(pkg).to(BF)
     plan = blk._plans.get(blk, BF, CPU)
     own = {p.data_ptr() for p in blk.parameters()}
     pair, attn, trans = plan.keep
     assert all(t is None or t.data_ptr() in own for ts in (*pair, attn, trans) for t in ts)
+
+
+def pairformer_block(pkg):
+    return pkg.PairFormerBlock(c_s=64, c_z=64, c_hidden_pair_bias=4, no_heads_pair_bias=16, c_hidden_mul=64, c_hidden_pair_att=16,
+                               no_heads_pair=4, transition_type="swiglu", transition_n=2, pair_dropout=0.25,
+                               fuse_projection_weights=False, inf=1e9).eval().requires_grad_(False)
+
+
+@pytest.mark.parametrize("make", [pair_block, pairformer_block, diffusion])
+def test_a_used_module_is_freed_with_its_last_reference(pkg, make):
+    """Its weights with it, without waiting for the garbage collector: a plan does not refer to the module it belongs to."""
+    m = make(pkg)
+    assert m._plans.get(m, BF, CPU) is not None
+    if make is pairformer_block:
+        assert m.pair_stack._plans.get(m.pair_stack, BF, CPU) is not None
+    gone = [weakref.ref(m), weakref.ref(next(m.parameters()))]
+    gc.disable()
+    try:
+        del m
+        assert all(r() is None for r in gone)
+    finally:
+        gc.enable()
