@@ -94,7 +94,8 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
                     const __nv_bfloat16* __restrict__ ln_w, const __nv_bfloat16* __restrict__ ln_b,
                     __nv_bfloat16* __restrict__ q_out,
                     __nv_bfloat16* __restrict__ k_out, __nv_bfloat16* __restrict__ vt_out,
-                    __nv_bfloat16* __restrict__ tb_out, int B, int R, int N, int npad, int row0, int* status) {
+                    __nv_bfloat16* __restrict__ tb_out, const __nv_bfloat16* __restrict__ mask,
+                    __nv_bfloat16* __restrict__ mask_t, int B, int R, int N, int npad, int row0, int* status) {
     using Sm = ProjSmem<C>;
     constexpr int kSt = Sm::kStages, D = C / kH;
     extern __shared__ uint8_t smem_raw[];
@@ -202,8 +203,15 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
         // their first half of the channels, lanes 16..31 the other half
         const int row = (warp - 2) * 16 + (lane & 15), half = lane >> 4;
         uint32_t it = 0;
-        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it) {
+        TileWalk tc(blockIdx.x, gridDim.x, R, tiles_per_line);
+        for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tc.next()) {
             const int s = it % kSt;
+            // The transposed view's mask column, as a row for the attention core: there every block of 128 queries and every
+            // head of a line would fetch a sector per key (N = 768: 85 of 762 us).
+            const int pos = tc.tile * kRows + row;
+            const bool copy_mask = kTransposed && mask != nullptr && half == 0 && pos < N;
+            __nv_bfloat16 mv = __float2bfloat16_rn(1.0f);
+            if (copy_mask) mv = mask[((long long)tc.b * N + pos) * N + tc.line];
             if (!mbar_wait(z_full(s), (it / kSt) & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidProj, 5);
                 break;
@@ -217,6 +225,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(a_ready(s));
+            if (copy_mask) mask_t[((long long)tc.b * R + tc.line) * npad + pos] = mv;
         }
     } else {
         // epilogue warps
@@ -325,16 +334,23 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
 // =====================================================================================
 // One CTA = one head, 128 queries and TWO lines of the pair tensor, 64 keys per step; two CTAs share an SM
 // (their prologues, epilogues and waits interleave). Per line and step j:
-//   MMA warp      S_j = Q K_j^T + Tb_j I^T: 128 x 64 logits in TMEM, issued as soon as the softmax warps have S_{j-1} in
+//   S warp        S_j = Q K_j^T + Tb_j I^T: 128 x 64 logits in TMEM, issued as soon as the softmax warps have S_{j-1} in
 //                 registers. The pair-bias tiles [128 q x 32 k] (bf16, shared by both lines) are a second A operand
 //                 against a 32 x 32 identity: a bf16 value times 1.0 accumulated in fp32 is exact.
 //   softmax warps thread = query row = TMEM lane: S -> registers [+ mask bias where the block has masked keys], row
 //                 maximum, P = exp2(S - m) rounded to bf16, sum of the rounded values, P into TMEM columns of its own
-//   MMA warp      O[128 x D] += P_j V_j with P read from TMEM as the A operand
-// What bounds it: one exponential per logit (N = 768: 1.8e9 per launch, 402 us of the MUFU pipe at 1.9 GHz), and what a
-// softmax warp does besides, for the four lines of an SM keep that pipe busy only while one of them is in its
-// exponentials. With nothing but the hand-offs left in the kernel it takes 410 us. Measured, us per launch at N = 768
-// (N = 2048: ms): 32 keys per step, two S buffers, P over S, row sum as a column of O: 759 (13.5). 64 keys per step, P over
+//   PV warp       O[128 x D] += P_j V_j with P read from TMEM as the A operand
+// What bounds it: one exponential per logit (N = 768: 1.8e9 per launch, 402 us of the MUFU pipe at 1.9 GHz), and the latency
+// of a step's hand-offs: polls, TMEM loads and stores, MMAs and commits go through the same queue as the exponentials of the
+// four softmax warps of a scheduler and take 50 - 100 cycles each behind them (a step of a line: 3260 cycles, of which 1790
+// exponentials, 940 waits for S and P V, 380 the load of S). The tensor pipe is not the limit: 298 cycles per line and step
+// in a loop of the same MMAs, of 815. Hence few such instructions in a row per warp: a warp per line issues S, a third one P V
+// (one warp for both: the next S queued behind P V); a K / bias stage is handed back by a commit behind S, not by the softmax
+// warps once they have read S (675 -> 660 us at N = 768, together 652); P V of the step before is awaited before the
+// exponentials, so that nothing divides these (644). Measured and worse: persistent blocks with 128 keys per step, two lines
+// per SM and the row sum on the tensor pipe 774 (two softmax warps per scheduler do not hide the hand-offs); no row maximum,
+// the block taken again where its sum overflows 733; all of P stored at the end of a step 701; S loaded in two halves 662.
+// Earlier steps, N = 768: 32 keys per step, two S buffers, P over S, row sum as a column of O: 759. 64 keys per step, P over
 // S: a step waits 1100 of its 3500 cycles for P V and the next S. P beside S, so that S_{j+1} is computed under the
 // softmax of S_j (the column of O for the row sum no longer fits, the threads take it: 28 us): with the bias added by
 // the threads 805 (it costs them 160), on the tensor pipe 682 (12.2).
@@ -350,7 +366,7 @@ constexpr int kMaxKeys = 2048;   // one CTA keeps a mask-bias row per line in sh
 constexpr int kKvStages = 2;     // ring of K + bias tiles, ring of V tiles
 constexpr int kLines = 2;     // lines per CTA
 constexpr int kLinePad = 4;   // the operand images pad the line count of a sample to a multiple of this
-// three warpgroups: producer and MMA warps; the softmax warps of line 0; of line 1
+// three warpgroups: producer, S of line 0, S of line 1, P V of both; the softmax warps of line 0; of line 1
 constexpr int kCoreThreads = 128 * (1 + kLines);
 // registers: the block is launched with 80 per thread (two blocks of 384 threads per SM); the issuing warpgroup gives up
 // what the softmax warpgroups, which hold a row of 64 logits, take. (The issuing warps need more than 32; with 96 for
@@ -377,12 +393,12 @@ struct CoreSmem {
     static uint32_t dyn_bytes(int nblk) { return kMb + kLines * nblk * kBK * 4 + 1024; }
 };
 
-template <int D, bool kTransposed>
+template <int D>
 __global__ void __launch_bounds__(kCoreThreads, 2)
 triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16* __restrict__ k_img,
                     const __nv_bfloat16* __restrict__ v_img, const __nv_bfloat16* __restrict__ tb_img,
-                    const __nv_bfloat16* __restrict__ mask, __nv_bfloat16* __restrict__ o_out, int B,
-                    int R, int N, float inf, int* status) {
+                    const __nv_bfloat16* __restrict__ mask, int mask_pitch, __nv_bfloat16* __restrict__ o_out, int R,
+                    int N, float inf, int* status) {
     using Sm = CoreSmem<D>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -424,7 +440,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
         mbar_init(q_full, 1);
         for (int s = 0; s < kSt; ++s) {
             mbar_init(kb_full(s), 1);
-            mbar_init(kb_empty(s), 4 * kLines);  // every softmax warp has read the S and the bias of the stage
+            mbar_init(kb_empty(s), kLines);      // each line's commit after the S that read the stage
             mbar_init(v_full(s), 1);
             mbar_init(v_empty(s), kLines);       // each line's commit after the P V that read the stage
         }
@@ -503,52 +519,60 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
             const uint32_t sb = __shfl_sync(0xffffffffu, sbase, 0);
             constexpr uint32_t idesc_s = idesc_bf16_f32(128, kBK);       // S: 128 x 64, K = D
             constexpr uint32_t idesc_b = idesc_bf16_f32(128, kBiasK);    // + bias: 128 x 32, K = 32
-            constexpr uint32_t idesc_o = idesc_bf16_f32(128, D);   // O: 128 x D, K = 64
             auto qk_desc = [](uint32_t a) { return D == 32 ? smem_desc_k_sw64(a) : smem_desc_k_sw32(a); };
-            bool ok = mbar_wait(q_full, 0, abort_flag);
-            if (!ok && lane == 0) report_wait_failure(status, abort_flag, kKidCore, 2);
+            const bool q_ok = mbar_wait(q_full, 0, abort_flag);
+            if (!q_ok && lane == 0) report_wait_failure(status, abort_flag, kKidCore, 2);
             const uint64_t qdesc = qk_desc(sb + Sm::kQ + L * Sm::kQBytes);
             const uint64_t identdesc = smem_desc_k_sw64(sb + Sm::kIdent);
             const uint32_t t_line = tm + L * 128;
             const int nkb32 = (N + kBiasK - 1) / kBiasK;
-            for (int i = 0; i <= nblk && ok; ++i) {
-                if (i < nblk) {   // S_i, once S_{i-1} is in registers
-                    const int ks = i % kSt;
-                    if (!mbar_wait(kb_full(ks), (i / kSt) & 1u, abort_flag)) {
-                        if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 3);
-                        break;
-                    }
-                    if (i > 0 && !mbar_wait(s_read(L), (i - 1) & 1u, abort_flag)) {
-                        if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 4);
-                        break;
-                    }
-                    tc_fence_after_sync();
-                    const uint64_t kdesc = qk_desc(sb + Sm::kK + (ks * kLines + L) * Sm::kKBytes);
-                    if (lane == 0) {
-#pragma unroll
-                        for (int kk = 0; kk < D / 16; ++kk)
-                            mma_bf16(t_line, qdesc + 2u * kk, kdesc + 2u * kk, idesc_s, kk != 0 ? 1u : 0u);
-                        const int nt = (2 * i + 1 < nkb32) ? 2 : 1;
-                        for (int t = 0; t < nt; ++t) {
-                            const uint64_t tbdesc = smem_desc_k_sw64(sb + Sm::kTb + (ks * 2 + t) * kTbTileBytes);
-                            mma_bf16(t_line + t * kBiasK, tbdesc, identdesc, idesc_b, 1u);
-                            mma_bf16(t_line + t * kBiasK, tbdesc + 2u, identdesc + 2u, idesc_b, 1u);
-                        }
-                        mma_commit(s_full(L));
-                    }
-                    __syncwarp();
+            for (int i = 0; i < nblk && q_ok; ++i) {   // S_i, once S_{i-1} is in registers
+                const int ks = i % kSt;
+                if (!mbar_wait(kb_full(ks), (i / kSt) & 1u, abort_flag)) {
+                    if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 3);
+                    break;
                 }
-                if (i > 0) {   // O += P_{i-1} V_{i-1}
-                    const int j = i - 1, vs = j % kSt;
-                    if (!mbar_wait(v_full(vs), (j / kSt) & 1u, abort_flag)) {
-                        if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 12);
-                        break;
+                if (i > 0 && !mbar_wait(s_read(L), (i - 1) & 1u, abort_flag)) {
+                    if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 4);
+                    break;
+                }
+                tc_fence_after_sync();
+                const uint64_t kdesc = qk_desc(sb + Sm::kK + (ks * kLines + L) * Sm::kKBytes);
+                if (lane == 0) {
+#pragma unroll
+                    for (int kk = 0; kk < D / 16; ++kk)
+                        mma_bf16(t_line, qdesc + 2u * kk, kdesc + 2u * kk, idesc_s, kk != 0 ? 1u : 0u);
+                    const int nt = (2 * i + 1 < nkb32) ? 2 : 1;
+                    for (int t = 0; t < nt; ++t) {
+                        const uint64_t tbdesc = smem_desc_k_sw64(sb + Sm::kTb + (ks * 2 + t) * kTbTileBytes);
+                        mma_bf16(t_line + t * kBiasK, tbdesc, identdesc, idesc_b, 1u);
+                        mma_bf16(t_line + t * kBiasK, tbdesc + 2u, identdesc + 2u, idesc_b, 1u);
                     }
+                    mma_commit(s_full(L));
+                    mma_commit(kb_empty(ks));
+                }
+                __syncwarp();
+            }
+        } else {
+            // ------------------------------------------------------------ the warp that issues O += P_j V_j of both lines
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const uint32_t sb = __shfl_sync(0xffffffffu, sbase, 0);
+            constexpr uint32_t idesc_o = idesc_bf16_f32(128, D);   // O: 128 x D, K = 64
+            bool ok = true;
+            for (int j = 0; j < nblk && ok; ++j) {
+                const int vs = j % kSt;
+                if (!mbar_wait(v_full(vs), (j / kSt) & 1u, abort_flag)) {
+                    if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 12);
+                    break;
+                }
+                for (int L = 0; L < kLines; ++L) {
                     if (!mbar_wait(p_ready(L), j & 1u, abort_flag)) {
                         if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 5);
+                        ok = false;
                         break;
                     }
                     tc_fence_after_sync();
+                    const uint32_t t_line = tm + L * 128;
                     const uint64_t vdesc = smem_desc_k_sw128(sb + Sm::kV + (vs * kLines + L) * Sm::kVBytes);
                     if (lane == 0) {
 #pragma unroll
@@ -587,11 +611,8 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
                 for (int e = 0; e < 8; ++e) {
                     const int k = c0 + e;
                     float m = 1.0f;
-                    if (mask != nullptr && k < N) {
-                        const long long mi = kTransposed ? ((long long)b * N + k) * N + line
-                                                         : ((long long)b * R + line) * N + k;
-                        m = __bfloat162float(mask[mi]);
-                    }
+                    if (mask != nullptr && k < N)
+                        m = __bfloat162float(mask[((long long)b * R + line) * mask_pitch + k]);
                     v[e] = (k < N) ? inf * (m - 1.0f) * kLog2e : -INFINITY;
                 }
                 bool any = false;
@@ -617,10 +638,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
         for (int j = 0; j < nblk && idle; ++j) {
             bool waited = mbar_wait(s_full(L), j & 1u, abort_flag);
             __syncwarp();
-            if (waited && lane == 0) {
-                mbar_arrive(s_read(L));
-                mbar_arrive(kb_empty(j % kSt));
-            }
+            if (waited && lane == 0) mbar_arrive(s_read(L));
             // (its arrival for step j must not count for step j - 1)
             if (waited && j > 0) waited = mbar_wait(pv_done(L), (j - 1) & 1u, abort_flag);
             if (!waited) {
@@ -631,7 +649,6 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
         }
         if (idle) ok = false;   // nothing to store
         for (int j = 0; j < nblk && ok; ++j) {
-            const int s = j % kSt;
             if (!mbar_wait(s_full(L), j & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 7);
                 ok = false;
@@ -644,10 +661,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
             tmem_ld_wait();
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(s_read(L));
-                mbar_arrive(kb_empty(s));   // S_j is complete: its K / bias stage can be refilled
-            }
+            if (lane == 0) mbar_arrive(s_read(L));
             float* sv = reinterpret_cast<float*>(sr);
             // + mask bias (blocks without a masked key skip it): (q.k + pair bias) + inf * (mask - 1); a masked
             // key ends at the same -1.44e9 in either order of the two additions, an unmasked one adds exactly 0
@@ -717,8 +731,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
                     add_bf16x2(l2, l3, pk[(e >> 1) + 1]);
                 }
             };
-            exps(0);
-            if (j > 0) {   // P_{j-1} has been read (long ago, as a rule)
+            if (j > 0) {   // P_{j-1} has been read
                 if (!mbar_wait(pv_done(L), (j - 1) & 1u, abort_flag)) {
                     if (lane == 0) report_wait_failure(status, abort_flag, kKidCore, 9);
                     ok = false;
@@ -726,6 +739,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
                 }
                 tc_fence_after_sync();
             }
+            exps(0);
             tmem_st16(trow + kColP, pk);
             exps(1);
             tmem_st16(trow + kColP + 16, pk);
@@ -1064,10 +1078,10 @@ int set_attrs() {
         OF3_CUDA_CHECK(cudaFuncSetAttribute(triattn_proj_kernel<C, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             ProjSmem<C>::kDyn));
         cudaFuncAttributes fa;   // a block launched with fewer registers would wait for the split for good
-        OF3_CUDA_CHECK(cudaFuncGetAttributes(&fa, triattn_core_kernel<C / kH, kT>));
+        OF3_CUDA_CHECK(cudaFuncGetAttributes(&fa, triattn_core_kernel<C / kH>));
         OF3_REQUIRE(fa.numRegs == kCoreRegsLaunch, OF3_ERR_DRIVER, "triattn_core is built with %d registers, not %d",
                     fa.numRegs, kCoreRegsLaunch);
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(triattn_core_kernel<C / kH, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(triattn_core_kernel<C / kH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             CoreSmem<C / kH>::dyn_bytes(kMaxKeys / kBK)));
         OF3_CUDA_CHECK(cudaFuncSetAttribute(triattn_out_kernel<C, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             AOutSmem<C>::kDyn));
@@ -1076,9 +1090,13 @@ int set_attrs() {
     return OF3_OK;
 }
 
+// elements per line of the mask rows that triattn_project writes for a transposed view
+int mask_pitch(int N) { return (int)align_up(N, kBK); }
+
 template <int C, bool kT>
 int project_impl(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* vt,
-                 __nv_bfloat16* tb, int B, int R, int N, int row0, const of3_triattn_params* p, cudaStream_t st) {
+                 __nv_bfloat16* tb, const __nv_bfloat16* mask, __nv_bfloat16* mask_t, int B, int R, int N, int row0,
+                 const of3_triattn_params* p, cudaStream_t st) {
     int rc;
     CUtensorMap tmZ, tmW[3], tmWb;
     if ((rc = z_tmap(&tmZ, z, B, R, N, C, kT))) return rc;
@@ -1099,13 +1117,13 @@ int project_impl(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __n
     typedef const __nv_bfloat16* P;
     LaunchScope scope(kKidProj, st);
     OF3_CUDA_CHECK(launch_chained(triattn_proj_kernel<C, kT>, grid, kProjThreads, ProjSmem<C>::kDyn, st, tmZ, tmW[0],
-                                  tmW[1], tmW[2], tmWb, (P)p->ln_w, (P)p->ln_b, q, k, vt, tb, B, R, N,
-                                  (int)align_up(N, kBK), row0, device_status_ptr()));
+                                  tmW[1], tmW[2], tmWb, (P)p->ln_w, (P)p->ln_b, q, k, vt, tb, mask, mask_t, B,
+                                  R, N, mask_pitch(N), row0, device_status_ptr()));
     return OF3_OK;
 }
 
 template <int C, bool kT>
-int finish_impl(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, const __nv_bfloat16* q,
+int finish_impl(const __nv_bfloat16* z, const __nv_bfloat16* mask, int pitch, __nv_bfloat16* out, const __nv_bfloat16* q,
                 const __nv_bfloat16* k, const __nv_bfloat16* vt, const __nv_bfloat16* tb, __nv_bfloat16* o, int B,
                 int R, int N, float inf, int add_residual, const of3_triattn_params* p, cudaStream_t st) {
     int rc;
@@ -1121,8 +1139,8 @@ int finish_impl(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16
     OF3_REQUIRE(ctas < (1LL << 31), OF3_ERR_SHAPE, "triattn: too many attention tiles");
     {
         LaunchScope scope(kKidCore, st);
-        OF3_CUDA_CHECK(launch_chained(triattn_core_kernel<C / kH, kT>, (unsigned)ctas, kCoreThreads,
-                                      CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK)), st, q, k, vt, tb, mask, o, B, R, N,
+        OF3_CUDA_CHECK(launch_chained(triattn_core_kernel<C / kH>, (unsigned)ctas, kCoreThreads,
+                                      CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK)), st, q, k, vt, tb, mask, pitch, o, R, N,
                                       inf, status));
     }
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
@@ -1151,25 +1169,30 @@ size_t triattn_bias_elems(int B, int R, int N) {
     return (size_t)B * kH * ceil_div(N, kBiasK) * R * kBiasK;
 }
 
+size_t triattn_mask_elems(int B, int N) { return (size_t)B * N * mask_pitch(N); }
+
 // q, k, v operand images and this shard's rows of the pair-bias image tb[(b*H + h)][key block][line][32]
 // from R lines of N positions; row0 = index of the shard's first line among all N query rows (0 for a whole
-// tensor). transposed: whole square tensors only.
+// tensor). transposed: whole square tensors only; their mask [B, N, N], where there is one, goes to mask_t
+// (triattn_mask_elems elements) with the view's lines as rows.
 int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* vt,
                     __nv_bfloat16* tb, int B, int R, int N, int row0, bool transposed,
-                    const of3_triattn_params* p, cudaStream_t st, int C) {
+                    const of3_triattn_params* p, cudaStream_t st, int C, const __nv_bfloat16* mask,
+                    __nv_bfloat16* mask_t) {
     OF3_REQUIRE(((uintptr_t)z & 15) == 0, OF3_ERR_ALIGN, "triattn: z must be 16-byte aligned");
     OF3_REQUIRE((((uintptr_t)q | (uintptr_t)k | (uintptr_t)vt) & 15) == 0, OF3_ERR_ALIGN,
                 "triattn: q / k / v images must be 16-byte aligned");
     OF3_REQUIRE(!transposed || R == N, OF3_ERR_SHAPE, "triattn: transposed view needs the whole tensor");
     if (C == 128)
-        return transposed ? project_impl<128, true>(z, q, k, vt, tb, B, R, N, row0, p, st)
-                          : project_impl<128, false>(z, q, k, vt, tb, B, R, N, row0, p, st);
-    return transposed ? project_impl<64, true>(z, q, k, vt, tb, B, R, N, row0, p, st)
-                      : project_impl<64, false>(z, q, k, vt, tb, B, R, N, row0, p, st);
+        return transposed ? project_impl<128, true>(z, q, k, vt, tb, mask, mask_t, B, R, N, row0, p, st)
+                          : project_impl<128, false>(z, q, k, vt, tb, mask, mask_t, B, R, N, row0, p, st);
+    return transposed ? project_impl<64, true>(z, q, k, vt, tb, mask, mask_t, B, R, N, row0, p, st)
+                      : project_impl<64, false>(z, q, k, vt, tb, mask, mask_t, B, R, N, row0, p, st);
 }
 
 // attention over the R lines with the pair-bias image of all N query rows (tb [(b*H + h)][key block][N][32]),
-// gate, output projection, residual.
+// gate, output projection, residual. mask: a row per line of the view, [B, R, N]; of a transposed view the rows that
+// triattn_project wrote.
 int triattn_finish(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out,
                    const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* vt,
                    const __nv_bfloat16* tb, __nv_bfloat16* o, int B, int R, int N, float inf,
@@ -1182,11 +1205,12 @@ int triattn_finish(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloa
     OF3_REQUIRE(N <= kMaxKeys, OF3_ERR_SHAPE, "triattn: N %d above the %d keys one CTA keeps a mask row for", N,
                 kMaxKeys);
     OF3_REQUIRE(!transposed || R == N, OF3_ERR_SHAPE, "triattn: transposed view needs the whole tensor");
+    const int pitch = transposed ? mask_pitch(N) : N;
     if (C == 128)
-        return transposed ? finish_impl<128, true>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
-                          : finish_impl<128, false>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
-    return transposed ? finish_impl<64, true>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
-                      : finish_impl<64, false>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
+        return transposed ? finish_impl<128, true>(z, mask, pitch, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
+                          : finish_impl<128, false>(z, mask, pitch, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
+    return transposed ? finish_impl<64, true>(z, mask, pitch, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
+                      : finish_impl<64, false>(z, mask, pitch, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
 }
 
 int triattn(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N, int C,
@@ -1198,12 +1222,13 @@ int triattn(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* ou
     __nv_bfloat16* vt = (__nv_bfloat16*)ws.take(img);
     __nv_bfloat16* o = (__nv_bfloat16*)ws.take(plane);
     __nv_bfloat16* tb = (__nv_bfloat16*)ws.take(triattn_bias_elems(B, N, N) * sizeof(__nv_bfloat16));
+    __nv_bfloat16* mask_t = (__nv_bfloat16*)ws.take(triattn_mask_elems(B, N) * sizeof(__nv_bfloat16));
     if (!ws.base) return OF3_OK;
     OF3_REQUIRE(ws.ok(), OF3_ERR_WORKSPACE, "triattn: workspace too small (%zu needed)", ws.off);
     const bool tr = (flags & OF3_FLAG_TRANSPOSED) != 0;
-    int rc = triattn_project(z, q, k, vt, tb, B, N, N, 0, tr, p, st, C);
+    int rc = triattn_project(z, q, k, vt, tb, B, N, N, 0, tr, p, st, C, mask, mask_t);
     if (rc) return rc;
-    return triattn_finish(z, mask, out, q, k, vt, tb, o, B, N, N, inf, tr,
+    return triattn_finish(z, (tr && mask != nullptr) ? mask_t : mask, out, q, k, vt, tb, o, B, N, N, inf, tr,
                           (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, st, C);
 }
 

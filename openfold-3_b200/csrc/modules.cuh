@@ -47,7 +47,9 @@ size_t triattn_image_elems(int B, int R, int N, int C = 128);
 size_t triattn_bias_elems(int B, int R, int N);  // bf16 elements of the pair-bias image [B*4][key blocks][R][32]
 int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* vt,
                     __nv_bfloat16* tb, int B, int R, int N, int row0, bool transposed,
-                    const of3_triattn_params* p, cudaStream_t st, int C = 128);
+                    const of3_triattn_params* p, cudaStream_t st, int C = 128, const __nv_bfloat16* mask = nullptr,
+                    __nv_bfloat16* mask_t = nullptr);
+size_t triattn_mask_elems(int B, int N);   // bf16 elements of mask_t: a transposed view's mask, a row per line
 int triattn_finish(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out,
                    const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* vt,
                    const __nv_bfloat16* tb, __nv_bfloat16* o, int B, int R, int N, float inf,

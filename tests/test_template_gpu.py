@@ -97,3 +97,24 @@ def test_tensors_that_start_anywhere(kind):
             assert all(torch.equal(a, b) for a, b in zip(x, want))
         assert all(torch.equal(m(odd()), w) for m, w in zip(layers, each))
     pkg.lib.check_device_status()
+
+
+@pytest.mark.parametrize("c,B,N", [(128, 1, 1), (128, 2, 37), (64, 2, 64), (128, 1, 65), (64, 1, 129), (128, 1, 200)])
+def test_ending_node_is_the_starting_node_of_the_transposed_tensor(c, B, N):
+    """The ending-node layer reads z and the mask in place, the mask through rows that its projection kernel writes: the same
+    bits as the starting-node layer on transposed copies, with masks that are not symmetric and without one."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator().manual_seed(N)
+    end, start = (pkg.TriangleAttention(c, c // 4, 4, starting=s) for s in (False, True))
+    with torch.no_grad():
+        for p, q in zip(end.parameters(), start.parameters()):
+            p.copy_(torch.randn(p.shape, generator=g) * (p.shape[-1] ** -0.5 if p.dim() > 1 else 0.3))
+            q.copy_(p)
+    end, start = (m.to(dev, bf).eval().requires_grad_(False) for m in (end, start))
+    z = torch.randn(B, N, N, c, generator=g).to(dev, bf)
+    m = rand_mask((B, N, N), g, 0.8).to(dev, bf)
+    with torch.no_grad():
+        for mask in (m, None):
+            want = start(z.transpose(1, 2).contiguous(), mask=None if mask is None else mask.transpose(1, 2).contiguous())
+            assert torch.equal(end(z, mask=mask), want.transpose(1, 2))
+    pkg.lib.check_device_status()
