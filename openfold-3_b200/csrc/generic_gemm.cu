@@ -9,6 +9,7 @@
 #include "generic_ops.cuh"
 #include "runtime.cuh"
 #include "umma.cuh"
+#include <type_traits>
 
 namespace of3 {
 namespace generic {
@@ -48,6 +49,17 @@ __device__ __forceinline__ bool vec_ok(const T* p, long long ld) {
     return (reinterpret_cast<uintptr_t>(p) & (4 * sizeof(T) - 1)) == 0 && (ld & 3) == 0;
 }
 
+__device__ __forceinline__ void store4(float* p, const float (&o)[4]) {
+    *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&o)[4]) {
+    *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool exists) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(dst)), "l"(src), "r"(exists ? 16 : 0)
+                 : "memory");
+}
+
 enum Epi { kStore, kGatedPlanes, kSwiglu, kFinal };
 
 template <typename T>
@@ -64,6 +76,143 @@ struct Args {
     T* final_out;
     RowMap map;
 };
+
+// What follows the product of a thread's TM x TN values: row_of(i), col_of(j) say where they lie.
+template <int BM, int BN, int TM, int TN, int EPI, typename T>
+__device__ __forceinline__ void epilogue(const Args<T>& p, const float (&v)[TM][TN], long long m0, int n0, int grp,
+                                         long long boff, int tx, int ty) {
+    constexpr int HN = BN / 2, HM = BM / 2, TN2 = TN / 2, TM2 = TM / 2;
+    const int n = p.n;
+    const long long M = p.M;
+    auto row_of = [&](int i) { return m0 + (i / TM2) * HM + ty * TM2 + i % TM2; };
+    auto col_of = [&](int j) { return n0 + (j / TN2) * HN + tx * TN2 + j % TN2; };   // kPaired: j < TN / 2 only
+    if constexpr (EPI == kGatedPlanes) {
+        float* out = p.out[grp];
+        const bool vo = vec_ok(out, M);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const long long r = row_of(hf * TM2);
+            float mk[TM2];
+#pragma unroll
+            for (int i = 0; i < TM2; ++i) mk[i] = (p.mask && r + i < M) ? ld_as_float(p.mask + r + i) : 1.0f;
+#pragma unroll
+            for (int j = 0; j < TN2; ++j) {
+                const int c = col_of(j);
+                if (c >= n) continue;
+                float o[TM2];
+#pragma unroll
+                for (int i = 0; i < TM2; ++i)
+                    o[i] = mk[i] * sigmoid_acc(v[hf * TM2 + i][TN2 + j]) * v[hf * TM2 + i][j];
+                float* d = out + (long long)c * M + r;
+                if (TM2 == 4 && vo && r + 3 < M) {
+                    *reinterpret_cast<float4*>(d) = make_float4(o[0], o[1], o[TM2 - 2], o[TM2 - 1]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < TM2; ++i)
+                        if (r + i < M) d[i] = o[i];
+                }
+            }
+        }
+        return;
+    }
+    if constexpr (EPI == kFinal && TN2 == 4) {
+        // Whole vectors, the gate and residual of TM2 rows ahead of the first store: the output may be the residual's
+        // own tensor, so that a load behind a store waits for it (with vector LayerNorm rows, one fp32 trunk block at
+        // N = 128: 1077 -> 1011 us).
+        const bool vec = (n & 3) == 0 && (p.map.inner_stride & 3) == 0 && (p.map.outer_stride & 3) == 0 &&
+                         vec_ok(p.final_out, 0) && (!p.residual || vec_ok(p.residual, 0)) && (!p.gate || vec_ok(p.gate, n));
+        if (vec) {
+#pragma unroll
+            for (int hm = 0; hm < 2; ++hm) {
+                float4 gt[TM2][2], rs[TM2][2];
+                float mk[TM2];
+                long long off[TM2];
+#pragma unroll
+                for (int i = 0; i < TM2; ++i) {
+                    const long long r = row_of(hm * TM2 + i);
+                    off[i] = r < M ? row_offset(p.map, r) : -1;
+                    mk[i] = (p.mask && r < M) ? ld_as_float(p.mask + r) : 1.0f;
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        const int c = col_of(hf * TN2), left = r < M ? n - c : 0;
+                        gt[i][hf] = p.gate ? load4(p.gate + r * n + c, left, true) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        rs[i][hf] = p.residual ? load4(p.residual + off[i] + c, left, true) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < TM2; ++i) {
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        const int c = col_of(hf * TN2);
+                        if (off[i] < 0 || c >= n) continue;
+                        const float ge[4] = {gt[i][hf].x, gt[i][hf].y, gt[i][hf].z, gt[i][hf].w};
+                        const float re[4] = {rs[i][hf].x, rs[i][hf].y, rs[i][hf].z, rs[i][hf].w};
+                        float o[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            o[j] = v[hm * TM2 + i][hf * TN2 + j];
+                            if (p.gate) o[j] *= sigmoid_acc(ge[j]);
+                            if (p.mask) o[j] *= mk[i];
+                            if (p.residual) o[j] += re[j];
+                        }
+                        store4(p.final_out + off[i] + c, o);
+                    }
+                }
+            }
+            return;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const long long r = row_of(i);
+        if (r >= M) continue;
+        if constexpr (EPI == kSwiglu) {
+            float* d = p.out[0] + r * n;
+            const int c = col_of(0);
+            float o[TN2];
+#pragma unroll
+            for (int j = 0; j < TN2; ++j) o[j] = v[i][j] * sigmoid_acc(v[i][j]) * v[i][TN2 + j];
+            if (TN2 == 4 && vec_ok(p.out[0], n) && c + 3 < n) {
+                *reinterpret_cast<float4*>(d + c) = make_float4(o[0], o[1], o[TN2 - 2], o[TN2 - 1]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < TN2; ++j)
+                    if (c + j < n) d[c + j] = o[j];
+            }
+        } else if constexpr (EPI == kStore) {
+            float* d = p.out[grp] + boff + r * n;
+            const bool vo = TN2 == 4 && vec_ok(p.out[grp] + boff, n);
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const int c = col_of(hf * TN2);
+                float o[TN2];
+#pragma unroll
+                for (int j = 0; j < TN2; ++j)
+                    o[j] = v[i][hf * TN2 + j] + ((p.bias[grp] && c + j < n) ? ld_as_float(p.bias[grp] + c + j) : 0.f);
+                if (vo && c + 3 < n) {
+                    *reinterpret_cast<float4*>(d + c) = make_float4(o[0], o[1], o[TN2 - 2], o[TN2 - 1]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < TN2; ++j)
+                        if (c + j < n) d[c + j] = o[j];
+                }
+            }
+        } else if constexpr (EPI == kFinal) {
+            const float mk = p.mask ? ld_as_float(p.mask + r) : 1.0f;
+            const long long off = row_offset(p.map, r);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int c = col_of(j);
+                if (c >= n) continue;
+                float o = v[i][j];
+                if (p.gate) o *= sigmoid_acc(p.gate[r * n + c]);
+                if (p.mask) o *= mk;
+                if (p.residual) o += ld_as_float(p.residual + off + c);
+                st_from_float(p.final_out + off + c, o);
+            }
+        }
+    }
+}
 
 // BM x BN tile; G groups of (BM / TM) x (BN / TN) threads, group g multiplies k = g (mod G quarters) of each slab. A
 // thread's rows are TM / 2 consecutive ones in each half of the tile, its columns TN / 2 in each half of the tile's BN;
@@ -222,79 +371,117 @@ __global__ void __launch_bounds__(G* BM / TM * BN / TN) gemm_kernel(const Args<T
             for (int q = 0; q < G - 1; ++q) v[i / TN][i % TN] += red[(q * TM * TN + i) * kGroupThreads + gt];
     }
 
-    auto row_of = [&](int i) { return m0 + (i / TM2) * HM + ty * TM2 + i % TM2; };
-    auto col_of = [&](int j) { return n0 + (j / TN2) * HN + tx * TN2 + j % TN2; };   // kPaired: j < TN / 2 only
-    if constexpr (EPI == kGatedPlanes) {
-        float* out = p.out[grp];
-        const bool vo = vec_ok(out, M);
+    epilogue<BM, BN, TM, TN, EPI, T>(p, v, m0, n0, grp, boff, tx, ty);
+}
+
+// The same product for fp32 operands in whole 16-byte vectors along k: slabs by cp.async as they lie, a thread's 8 x 8
+// products in pairs (even k, odd k), whose halves are added at the end: operands come from shared memory as the pairs that
+// fma.f32x2 takes, none is duplicated in registers. A row of a slab lies at the place that lets the lanes of a load, which
+// own rows 4 apart, hit neighbouring ones: pitch 20 floats, no bank conflict. Two blocks per SM, since a thread holds 128
+// sums: for the plain and the final epilogue the better kernel (one fp32 trunk block at N = 128: 1011 -> 978 us), for the
+// paired ones, whose exponentials three blocks of the kernel above overlap with products, the worse (swiglu 107 -> 119 us).
+// Both read 16 values per 64 products from shared memory, whose bandwidth (16 bytes x 32 lanes in four clocks) that takes
+// whole; 16 x 8 products per thread leave two blocks per SM and are slower (122 us).
+template <int EPI>
+__global__ void __launch_bounds__(128, 2) gemm_pairs_kernel(const Args<float> p) {
+    constexpr int BM = 128, BN = 64, TM = 8, TN = 8, BK = 16, kStages = 4, kPitch = BK + 4;
+    constexpr bool kPaired = EPI == kGatedPlanes || EPI == kSwiglu;
+    constexpr int HN = BN / 2;
+    extern __shared__ __align__(16) float slabs[];   // stages x (BM + BN) rows
+    umma::grid_trigger();
+    umma::grid_wait();
+    const int K = p.K, n = p.n;
+    const long long M = p.M, m0 = (long long)blockIdx.x * BM;
+    const int tiles_n = (n + (kPaired ? HN : BN) - 1) / (kPaired ? HN : BN);
+    const int grp = blockIdx.y / tiles_n;
+    const int n0 = (blockIdx.y % tiles_n) * (kPaired ? HN : BN);
+    const long long boff = (long long)blockIdx.z * p.a_batch;
+    const float* a = p.a + boff;
+    const float* w0 = (kPaired ? p.w[2 * grp] : p.w[grp]) + boff;
+    const float* w1 = kPaired ? p.w[2 * grp + 1] : w0;
+
+    // this thread's 16-byte vectors of a slab: row t / 4 + 32 i, k offset 4 (t % 4)
+    const int kc = (threadIdx.x & 3) * 4, lr = threadIdx.x >> 2;
+    const float* src[6];
+    float* dst[6];
+    bool in[6];
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-            const long long r = row_of(hf * TM2);
-            float mk[TM2];
-#pragma unroll
-            for (int i = 0; i < TM2; ++i) mk[i] = (p.mask && r + i < M) ? ld_as_float(p.mask + r + i) : 1.0f;
-#pragma unroll
-            for (int j = 0; j < TN2; ++j) {
-                const int c = col_of(j);
-                if (c >= n) continue;
-                float o[TM2];
-#pragma unroll
-                for (int i = 0; i < TM2; ++i)
-                    o[i] = mk[i] * sigmoid_acc(v[hf * TM2 + i][TN2 + j]) * v[hf * TM2 + i][j];
-                float* d = out + (long long)c * M + r;
-                if (TM2 == 4 && vo && r + 3 < M) {
-                    *reinterpret_cast<float4*>(d) = make_float4(o[0], o[1], o[TM2 - 2], o[TM2 - 1]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < TM2; ++i)
-                        if (r + i < M) d[i] = o[i];
-                }
-            }
+    for (int i = 0; i < 6; ++i) {
+        if (i < 4) {
+            const int r = lr + 32 * i;                     // 64 hm + 4 ty + e -> slot 64 hm + 16 e + ty
+            in[i] = m0 + r < M;
+            src[i] = a + (in[i] ? m0 + r : 0) * K + kc;
+            dst[i] = slabs + ((r & 64) + (r & 3) * 16 + ((r & 63) >> 2)) * kPitch + kc;
+        } else {
+            const int c = lr + 32 * (i - 4);               // 32 hf + 4 tx + e -> slot 32 hf + 8 e + tx
+            const int col = n0 + (kPaired ? c & 31 : c);
+            in[i] = col < n;
+            src[i] = (kPaired && c >= HN ? w1 : w0) + (long long)(in[i] ? col : 0) * K + kc;
+            dst[i] = slabs + (BM + (c & 32) + (c & 3) * 8 + ((c & 31) >> 2)) * kPitch + kc;
         }
-        return;
     }
+    const int slabs_k = (K + BK - 1) / BK;
+    auto fetch = [&](int ks) {
+        if (ks < slabs_k) {
+            const bool kin = ks * BK + kc < K;
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const long long r = row_of(i);
-        if (r >= M) continue;
-        if constexpr (EPI == kSwiglu) {
-            float* d = p.out[0] + r * n;
+            for (int i = 0; i < 6; ++i)
+                cp_async16(dst[i] + (ks % kStages) * ((BM + BN) * kPitch), kin ? src[i] + ks * BK : src[i] - kc, kin && in[i]);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    u64 acc[TM][TN];
 #pragma unroll
-            for (int j = 0; j < TN2; ++j)
-                if (col_of(j) < n) d[col_of(j)] = v[i][j] * sigmoid_acc(v[i][j]) * v[i][TN2 + j];
-        } else if constexpr (EPI == kStore) {
-            float* d = p.out[grp] + boff + r * n;
-            const bool vo = TN2 == 4 && vec_ok(p.out[grp] + boff, n);
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                const int c = col_of(hf * TN2);
-                float o[TN2];
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
 #pragma unroll
-                for (int j = 0; j < TN2; ++j)
-                    o[j] = v[i][hf * TN2 + j] + ((p.bias[grp] && c + j < n) ? ld_as_float(p.bias[grp] + c + j) : 0.f);
-                if (vo && c + 3 < n) {
-                    *reinterpret_cast<float4*>(d + c) = make_float4(o[0], o[1], o[TN2 - 2], o[TN2 - 1]);
-                } else {
+    for (int ks = 0; ks < kStages - 1; ++ks) fetch(ks);
+    for (int ks = 0; ks < slabs_k; ++ks) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        __syncthreads();
+        fetch(ks + kStages - 1);
+        const float* as = slabs + (ks % kStages) * ((BM + BN) * kPitch) + ty * kPitch;
+        const float* ws = slabs + (ks % kStages) * ((BM + BN) * kPitch) + (BM + tx) * kPitch;
 #pragma unroll
-                    for (int j = 0; j < TN2; ++j)
-                        if (c + j < n) d[c + j] = o[j];
-                }
-            }
-        } else if constexpr (EPI == kFinal) {
-            const float mk = p.mask ? ld_as_float(p.mask + r) : 1.0f;
-            const long long off = row_offset(p.map, r);
+        for (int q = 0; q < BK / 4; ++q) {
+            ulonglong2 av[TM];
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+                av[i] = *reinterpret_cast<const ulonglong2*>(as + ((i >> 2) * 64 + (i & 3) * 16) * kPitch + q * 4);
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
-                const int c = col_of(j);
-                if (c >= n) continue;
-                float o = v[i][j];
-                if (p.gate) o *= sigmoid_acc(p.gate[r * n + c]);
-                if (p.mask) o *= mk;
-                if (p.residual) o += ld_as_float(p.residual + off + c);
-                st_from_float(p.final_out + off + c, o);
+                const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(ws + ((j >> 2) * 32 + (j & 3) * 8) * kPitch + q * 4);
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    fma2(acc[i][j], av[i].x, wv.x);
+                    fma2(acc[i][j], av[i].y, wv.y);
+                }
             }
         }
     }
+    float v[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const float2 f = unpack2(acc[i][j]);
+            v[i][j] = f.x + f.y;
+        }
+    epilogue<BM, BN, TM, TN, EPI, float>(p, v, m0, n0, grp, boff, tx, ty);
+}
+constexpr int kPairsSmem = 4 * (128 + 64) * 20 * 4;
+
+template <int EPI>
+int launch_pairs(const Args<float>& p, dim3 grid, cudaStream_t st) {
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(gemm_pairs_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairsSmem));
+        configured.mark();
+    }
+    OF3_CUDA_CHECK(launch_chained(gemm_pairs_kernel<EPI>, grid, 128, kPairsSmem, st, p));
+    return OF3_OK;
 }
 
 template <int EPI, bool K_OUTER, typename T>
@@ -313,6 +500,12 @@ int launch(Args<T> p, int groups, int batch, cudaStream_t st) {
                 M, p.n, batch);
     const dim3 grid((unsigned)gx, (unsigned)gy, batch);
     LaunchScope scope(20, st);
+    if constexpr (std::is_same<T, float>::value && !K_OUTER) {
+        // where every operand, and every plane of a batch, comes in whole vectors along k
+        uintptr_t bits = reinterpret_cast<uintptr_t>(p.a) | (uintptr_t)(p.K & 3) << 2 | (uintptr_t)(p.a_batch & 3) << 2;
+        for (int i = 0; i < (kPaired ? 2 : 1) * groups; ++i) bits |= reinterpret_cast<uintptr_t>(p.w[i]);
+        if (large && (EPI == kStore || EPI == kFinal) && (bits & 15) == 0) return launch_pairs<EPI>(p, grid, st);
+    }
     if (large)
         OF3_CUDA_CHECK(launch_chained(gemm_kernel<128, 64, 8, 8, 1, EPI, K_OUTER, T>, grid, 128, 0, st, p));
     else

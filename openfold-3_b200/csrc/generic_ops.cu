@@ -2,6 +2,7 @@
 #include "generic_ops.cuh"
 #include "runtime.cuh"
 #include "umma.cuh"
+#include <type_traits>
 
 namespace of3 {
 namespace generic {
@@ -91,6 +92,70 @@ __global__ void __launch_bounds__(kThreads) layernorm_kernel(const TX* __restric
         } else {
             for (int c = lane; c < C; c += 32)
                 d = fmaf(norm(ld_as_float(xr + c), c), ld_as_float(proj_w + (long long)h * C + c), d);
+        }
+        d = warp_sum(d);
+        if (lane == 0) proj[(long long)h * rows + r] = d;
+    }
+}
+
+// The same for fp32 rows in whole 16-byte vectors, V of them per lane (C <= 128 V): at C = 128 a lane's loads, statistics and
+// stores are one of each instead of sixteen guarded passes.
+template <int V>
+__global__ void __launch_bounds__(kThreads) layernorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
+                                                                 const float* __restrict__ beta, float* __restrict__ y,
+                                                                 long long rows, int C, float eps, RowMap map,
+                                                                 const float* __restrict__ proj_w, int H,
+                                                                 float* __restrict__ proj) {
+    umma::grid_trigger();
+    umma::grid_wait();
+    const int lane = threadIdx.x & 31;
+    const long long r = (long long)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    if (r >= rows) return;
+    const float* xr = x + row_offset(map, r);
+    auto vec = [&](const float* p, int i, float fill) {
+        const int c = 4 * (lane + 32 * i);
+        return (p != nullptr && c < C) ? *reinterpret_cast<const float4*>(p + c) : make_float4(fill, fill, fill, fill);
+    };
+    float4 v[V], gm[V], bt[V];
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = vec(xr, i, 0.f);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        gm[i] = vec(gamma, i, 1.f);
+        bt[i] = vec(beta, i, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    const float mean = warp_sum(s) / (float)C;
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        if (4 * (lane + 32 * i) < C) {
+            v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean;
+            q += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+        }
+    }
+    const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)C + eps);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const int c = 4 * (lane + 32 * i);
+        if (c >= C) continue;
+        v[i].x = v[i].x * rstd * gm[i].x + bt[i].x;
+        v[i].y = v[i].y * rstd * gm[i].y + bt[i].y;
+        v[i].z = v[i].z * rstd * gm[i].z + bt[i].z;
+        v[i].w = v[i].w * rstd * gm[i].w + bt[i].w;
+        if (y) *reinterpret_cast<float4*>(y + r * C + c) = v[i];
+    }
+    for (int h = 0; h < H; ++h) {
+        float d = 0.f;
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            const float4 w = vec(proj_w + (long long)h * C, i, 0.f);
+            d = fmaf(v[i].x, w.x, d);
+            d = fmaf(v[i].y, w.y, d);
+            d = fmaf(v[i].z, w.z, d);
+            d = fmaf(v[i].w, w.w, d);
         }
         d = warp_sum(d);
         if (lane == 0) proj[(long long)h * rows + r] = d;
@@ -389,6 +454,16 @@ int layernorm(const TX* x, const TP* gamma, const TP* beta, float* y, long long 
               cudaStream_t stream, const TP* proj_w, int H, float* proj) {
     if (rows <= 0) return OF3_OK;
     LaunchScope scope(20, stream);
+    if constexpr (std::is_same<TX, float>::value) {
+        const uintptr_t bits = (uintptr_t)x | (uintptr_t)gamma | (uintptr_t)beta | (uintptr_t)y | (uintptr_t)proj_w;
+        const bool vec = (bits & 15) == 0 && ((C | map.inner_stride | map.outer_stride) & 3) == 0;
+        if (vec && C <= 512) {
+            OF3_CUDA_CHECK(launch_chained(C <= 128 ? layernorm_vec_kernel<1> : layernorm_vec_kernel<4>,
+                                          grid_for(rows, kThreads / 32), kThreads, 0, stream, x, gamma, beta, y, rows, C, eps,
+                                          map, proj_w, H, proj));
+            return OF3_OK;
+        }
+    }
     OF3_CUDA_CHECK(launch_chained(layernorm_kernel<TX, TP>, grid_for(rows, kThreads / 32), kThreads, 0, stream, x, gamma,
                                   beta, y, rows, C, eps, map, proj_w, H, proj));
     return OF3_OK;

@@ -27,3 +27,21 @@ def test_fp32_block_matches_the_oracle(dims, B, N):
         got = blk(s.to(dev), z.to(dev), sm.to(dev), pm.to(dev))
     for a, b in zip(got, ref):
         assert rel_err(a.cpu(), b) < 1e-4, rel_err(a.cpu(), b)
+
+
+@pytest.mark.parametrize("c_z,c_hidden_mul,heads,d,n,N", [(128, 128, 4, 32, 4, 101), (36, 20, 3, 12, 2, 141), (68, 36, 2, 18, 1, 139)])
+def test_fp32_pair_block_on_large_tiles(c_z, c_hidden_mul, heads, d, n, N):
+    """Enough rows for the 128 x 64 tiles, with a ragged last one; widths in whole vectors that divide neither a slab of 16 nor
+    a tile."""
+    dims = dict(c_z=c_z, c_hidden_mul=c_hidden_mul, c_hidden_pair_att=d, no_heads_pair=heads, transition_n=n)
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(N)
+    P = W.pair_block_params(seed=43, final_std=None, **dims)
+    z, m = torch.randn(1, N, N, c_z, generator=g), rand_mask((1, N, N), g, 0.9)
+    ref = oracle.pair_block(z, m, P, "", heads)
+    blk = pkg.PairBlock(**dims, **_PF_KW)
+    blk.load_state_dict(P, strict=True)
+    blk = blk.to(dev).eval()
+    with torch.no_grad():
+        got = blk(z.to(dev), m.to(dev)).cpu()
+    assert rel_err(got, ref) < 1e-4, rel_err(got, ref)
