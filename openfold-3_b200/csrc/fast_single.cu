@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) ada_rows_kernel(const bf16* __restrict__ 
         unpack8(s[v], sf);
         unpack8(b[v], bf);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = row.x[v * 8 + e] / (1.0f + __expf(-(gf[e] + bf[e]))) + sf[e];
+        for (int e = 0; e < 8; ++e) o[e] = fmaf(row.x[v * 8 + e], sigmoid_of(gf[e] + bf[e]), sf[e]);
         *reinterpret_cast<uint4*>(an + r * C + c) = pack8(o);
     }
 }

@@ -81,8 +81,26 @@ single_bias_kernel(const float* __restrict__ pair_bias, bf16* __restrict__ tb_im
     }
 }
 
+// V consecutive channels of the caller's row: 32 bytes where V = 16 and the address allows it
+template <int V>
+__device__ __forceinline__ void load_row(const bf16* p, uint32_t (&o)[V / 2]) {
+    if constexpr (V == 16) {
+        if (aligned32(p)) ldg256(p, o);
+        else ld_row16(p, o);
+    } else {
+        const uint4 v = *reinterpret_cast<const uint4*>(p);
+        o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+    }
+}
+template <int V>
+__device__ __forceinline__ void store_row(bf16* p, const uint32_t (&o)[V / 2]) {
+    if constexpr (V == 16) stg256_or_2x128(p, o, aligned32(p));
+    else *reinterpret_cast<uint4*>(p) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // ---------------------------------------------------------------- single_core
-// One CTA = (pair tensor z, head, 128 queries) for TWO samples ("lines") that share the pair bias; two CTAs per SM.
+// One CTA = (pair tensor z, head, 128 queries) for TWO samples ("lines") that share the pair bias (the last group of an odd
+// number of samples: one, and nothing is done for the other); two CTAs per SM.
 // Per line and 32-key step j:
 //   MMA warp      S_j = Q K_j^T + Tb_j I^T into TMEM slot j % 2 (the bias tile is a second A operand against a
 //                 32 x 32 identity: the tensor pipe adds it, exactly, in fp32)
@@ -92,6 +110,10 @@ single_bias_kernel(const float* __restrict__ pair_bias, bf16* __restrict__ tb_im
 // The running maximum m used for scaling is only raised when a row maximum exceeds it by more than 8 (2^8 head
 // room in P): then the thread rescales its O row in TMEM and its running sum. Numerator and denominator always
 // share one scale, so the result is exact.
+// What bounds it: one wave of blocks, each a chain of steps, and at both ends what no other block covers. Gate values fetched
+// behind the last P V, 16 bytes at a time, and divisions in the sigmoids made the epilogue 11000 cycles of some 60000 (5 x 768
+// tokens, 24 layers: 3630 -> 3456 us). Measured and not kept: 64 keys per step as in the triangle attention (with 48 channels
+// P then has one block of columns and two hand-offs per step: 3505 us), three V slots (one block per SM at N = 768: 3773).
 template <int D>
 __global__ void __launch_bounds__(kThreads, 2)
 single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_img, const bf16* __restrict__ v_img,
@@ -130,18 +152,18 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
     const int q0 = qt * kBQ;
     const int nblk = (N + kBK - 1) / kBK;
     const int nkp = nblk * kBK;
-    // a line past the last sample of z recomputes the group's first sample and is not stored
-    auto sample_of = [&](int L) { return (long long)z * rpb + ((grp * kLines + L < rpb) ? grp * kLines + L : grp * kLines); };
+    const int lines = rpb - grp * kLines < kLines ? rpb - grp * kLines : kLines;   // samples of this group
+    auto sample_of = [&](int L) { return (long long)z * rpb + grp * kLines + L; };
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
         for (int s = 0; s < kSt; ++s) {
             mbar_init(kb_full(s), 1);
-            mbar_init(kb_empty(s), 4 * kLines);  // every softmax warp has read the S that consumed the stage
+            mbar_init(kb_empty(s), lines);       // each line's commit after the S that read the stage
         }
         for (int s = 0; s < kVSt; ++s) {
             mbar_init(v_full(s), 1);
-            mbar_init(v_empty(s), kLines);       // each line's commit after the P V that read the stage
+            mbar_init(v_empty(s), lines);        // each line's commit after the P V that read the stage
         }
         for (int L = 0; L < kLines; ++L) {
             for (int s = 0; s < 2; ++s) {
@@ -185,36 +207,45 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
     if (warp == 0) {
         if (lane == 0) {
             const long long zh = (long long)z * H + h;
-            mbar_arrive_expect_tx(q_full, kLines * C::kQBytes);
-            for (int L = 0; L < kLines; ++L)
+            mbar_arrive_expect_tx(q_full, lines * C::kQBytes);
+            for (int L = 0; L < lines; ++L)
                 bulk_load(sbase + C::kQ + L * C::kQBytes,
                           q_img + (((sample_of(L) * H + h) * n_qt + qt) * kBQ) * (long long)KD, C::kQBytes, q_full);
             const int q_rows = (nq - q0 < kBQ) ? nq - q0 : kBQ;   // rows of the bias tile that exist
             const uint32_t tb_bytes = (uint32_t)q_rows * kBK * 2;
-            for (int j = 0; j < nblk; ++j) {
+            auto load_kb = [&](int j) {
                 const int s = j % kSt;
-                const uint32_t ph = ((j / kSt) & 1u) ^ 1u;
-                if (!mbar_wait(kb_empty(s), ph, abort_flag)) {
+                if (!mbar_wait(kb_empty(s), ((j / kSt) & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidSingleCore, 1);
-                    break;
+                    return false;
                 }
-                mbar_arrive_expect_tx(kb_full(s), kLines * C::kKBytes + tb_bytes);
-                for (int L = 0; L < kLines; ++L)
+                mbar_arrive_expect_tx(kb_full(s), lines * C::kKBytes + tb_bytes);
+                for (int L = 0; L < lines; ++L)
                     bulk_load(sbase + C::kK + (s * kLines + L) * C::kKBytes,
                               k_img + (((sample_of(L) * H + h) * nblk + j) * kBK) * (long long)KD, C::kKBytes,
                               kb_full(s));
                 bulk_load(sbase + C::kTb + s * C::kTbBytes, tb_img + ((zh * nblk + j) * (long long)nq + q0) * kBK,
                           tb_bytes, kb_full(s));
-                const int sv = j % kVSt;
-                if (!mbar_wait(v_empty(sv), ((j / kVSt) & 1u) ^ 1u, abort_flag)) {
+                return true;
+            };
+            auto load_v = [&](int j) {
+                const int s = j % kVSt;
+                if (!mbar_wait(v_empty(s), ((j / kVSt) & 1u) ^ 1u, abort_flag)) {
                     report_wait_failure(status, abort_flag, kKidSingleCore, 11);
-                    break;
+                    return false;
                 }
-                mbar_arrive_expect_tx(v_full(sv), kLines * C::kVBytes);
-                for (int L = 0; L < kLines; ++L)
-                    bulk_load(sbase + C::kV + (sv * kLines + L) * C::kVSlot,
+                mbar_arrive_expect_tx(v_full(s), lines * C::kVBytes);
+                for (int L = 0; L < lines; ++L)
+                    bulk_load(sbase + C::kV + (s * kLines + L) * C::kVSlot,
                               v_img + (((sample_of(L) * H + h) * nblk + j) * (long long)DV) * kBK, C::kVBytes,
-                              v_full(sv));
+                              v_full(s));
+                return true;
+            };
+            // K and bias run two blocks ahead of V: a V slot waits for P V, and what is behind it in this loop for as long
+            // (5 samples of 768 tokens, 24 layers: 3456 -> 3420 us)
+            for (int j = 0; j < nblk + 2; ++j) {
+                if (j < nblk && !load_kb(j)) break;
+                if (j >= 2 && !load_v(j - 2)) break;
             }
         }
     } else if (warp <= kLines) {
@@ -227,8 +258,9 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
         constexpr uint32_t idesc_s = idesc_bf16_f32(128, kBK);
         constexpr uint32_t idesc_o = idesc_bf16_f32(128, C::kON);
         auto kdesc_of = [](uint32_t a) { return KD == 32 ? smem_desc_k_sw64(a) : smem_desc_k_sw128(a); };
-        bool ok = mbar_wait(q_full, 0, abort_flag);
-        if (!ok && lane == 0) report_wait_failure(status, abort_flag, kKidSingleCore, 2);
+        bool ok = L < lines;
+        if (ok) ok = mbar_wait(q_full, 0, abort_flag);
+        if (!ok && L < lines && lane == 0) report_wait_failure(status, abort_flag, kKidSingleCore, 2);
         const uint64_t qdesc = kdesc_of(sb + C::kQ + L * C::kQBytes);
         const uint64_t identdesc = smem_desc_k_sw64(sb + C::kIdent);
         const uint32_t t_line = tm + L * 128;
@@ -255,6 +287,7 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
                 mma_bf16(d, tbdesc, identdesc, idesc_s, 1u);            // + pair bias
                 mma_bf16(d, tbdesc + 2u, identdesc + 2u, idesc_s, 1u);
                 mma_commit(s_full(L, s));
+                mma_commit(kb_empty(ks));
             }
             __syncwarp();
             return true;
@@ -289,13 +322,13 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         const int qpos = q0 + row;
-        const bool line_valid = grp * kLines + L < rpb;
+        bool ok = L < lines;
         const long long bb = sample_of(L);
         const uint32_t trow = tmem_base + ((uint32_t)(quad * 32) << 16) + L * 128;
         float* mbl = mbs + L * nkp;
         // Additive key mask of this sample, pre-scaled for exp2: inf * (mask - 1) * log2(e), -inf beyond N; one flag
         // per key block tells whether the block has any non-zero entry.
-        {
+        if (ok) {
             const int gt = (warp - 1 - kLines - 4 * L) * 32 + lane;  // 0..127 within the line's warps
             for (int base = 0; base < nkp; base += 128 * 8) {        // warp-uniform trip count (ballot below)
                 const int c0 = base + gt * 8;
@@ -321,7 +354,6 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
             group_sync(1 + L, 128);
         }
         float m_used = 0.f;
-        bool ok = true;
         for (int j = 0; j < nblk && ok; ++j) {
             const int s = j & 1;
             if (!mbar_wait(s_full(L, s), (j >> 1) & 1u, abort_flag)) {
@@ -333,10 +365,6 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
             uint32_t sr[32];
             tmem_ld32(trow + s * kBK, sr);
             tmem_ld_wait();
-            // S_j is in registers: the K / bias stage its GEMM read can be refilled
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(kb_empty(j % kSt));
             float sv[kBK];
 #pragma unroll
             for (int e = 0; e < 32; ++e) sv[e] = __uint_as_float(sr[e]);
@@ -412,36 +440,39 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
             if (lane == 0) mbar_arrive(p_ready(L, s));
         }
         if (ok) {
+            const bool store = qpos < nq;
+            const long long off = (bb * nq + qpos) * (long long)(H * D) + h * D;
+            // The row's gate, on its way under the last P V; whole sectors in and out (rows of heads of 48 are 96 bytes)
+            constexpr int kV = D % 16 == 0 ? 16 : 8;   // channels per access
+            uint32_t gw[D / kV][kV / 2];
+            if (store && gate != nullptr) {
+#pragma unroll
+                for (int c = 0; c < D / kV; ++c) load_row<kV>(gate + off + c * kV, gw[c]);
+            }
             if (mbar_wait(pv_done(L, (nblk - 1) & 1), ((nblk - 1) >> 1) & 1u, abort_flag)) {
                 tc_fence_after_sync();
                 const uint32_t lsum = tmem_ld1(trow + C::kColO + DV);
                 tmem_ld_wait();
                 const float inv = 1.0f / __uint_as_float(lsum);
-                const bool store = qpos < nq && line_valid;
-                const long long off = (bb * nq + qpos) * (long long)(H * D) + h * D;
 #pragma unroll
                 for (int part = 0; part < DV / 16; ++part) {
                     uint32_t r[16];
                     tmem_ld16(trow + C::kColO + part * 16, r);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int v8 = 0; v8 < 2; ++v8) {
-                        const int c0 = part * 16 + v8 * 8;
-                        if (c0 < D && store) {
-                            float fo[8];
+                    for (int c = part * 16 / kV; c < (part + 1) * 16 / kV && c < D / kV; ++c) {
+                        uint32_t o[kV / 2];
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) fo[e] = __uint_as_float(r[v8 * 8 + e]) * inv;
+                        for (int e = 0; e < kV / 2; ++e) {
+                            float f0 = __uint_as_float(r[c * kV % 16 + 2 * e]) * inv;
+                            float f1 = __uint_as_float(r[c * kV % 16 + 2 * e + 1]) * inv;
                             if (gate != nullptr) {
-                                const uint4 gw = *reinterpret_cast<const uint4*>(gate + off + c0);
-                                fo[0] *= sigmoidf_fast(bf16lo(gw.x)); fo[1] *= sigmoidf_fast(bf16hi(gw.x));
-                                fo[2] *= sigmoidf_fast(bf16lo(gw.y)); fo[3] *= sigmoidf_fast(bf16hi(gw.y));
-                                fo[4] *= sigmoidf_fast(bf16lo(gw.z)); fo[5] *= sigmoidf_fast(bf16hi(gw.z));
-                                fo[6] *= sigmoidf_fast(bf16lo(gw.w)); fo[7] *= sigmoidf_fast(bf16hi(gw.w));
+                                f0 *= sigmoid_of(bf16lo(gw[c][e]));
+                                f1 *= sigmoid_of(bf16hi(gw[c][e]));
                             }
-                            *reinterpret_cast<uint4*>(out + off + c0) =
-                                make_uint4(pack_bf16x2(fo[0], fo[1]), pack_bf16x2(fo[2], fo[3]),
-                                           pack_bf16x2(fo[4], fo[5]), pack_bf16x2(fo[6], fo[7]));
+                            o[e] = pack_bf16x2(f0, f1);
                         }
+                        if (store) store_row<kV>(out + off + c * kV, o);
                     }
                 }
             } else if (lane == 0) {

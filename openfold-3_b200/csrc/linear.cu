@@ -56,15 +56,6 @@ struct EpiArgs {
     const bf16 *residual, *gate, *gate_bias, *mask;
 };
 
-// 1 / (1 + exp(-x)) with the reciprocal refined by one Newton step, r (2 - d r): as close as the division, in a third of
-// its instructions. The clamp keeps d finite (0 * inf in the step): below -87 the result is 1.6e-38 instead of less.
-__device__ __forceinline__ float sigmoid_of(float x) {
-    const float d = 1.0f + __expf(-x > 87.0f ? 87.0f : -x);   // (a NaN stays one)
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    return fmaf(r, fmaf(-d, r, 1.0f), r);
-}
-
 // One column group of 16 of this thread's row as attention operand images; `kind` is uniform over the tile.
 template <int D>
 __device__ __forceinline__ void store_images(const AttnImages& im, int kind, float qscale, const uint32_t (&r)[16],
