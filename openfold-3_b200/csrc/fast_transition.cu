@@ -315,7 +315,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                 for (int r = 0; r < 4; ++r) {
                     float a = 0.f, b = 0.f;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) { a += bf16lo(raw[(h + r) * 4 + i]); b += bf16hi(raw[(h + r) * 4 + i]); }
+                    for (int i = 0; i < 4; ++i) { a = add_lo(raw[(h + r) * 4 + i], a); b = add_hi(raw[(h + r) * 4 + i], b); }
                     mean[r] = a + b;
                 }
                 row_sums(mean, lane);
@@ -326,7 +326,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     float a = 0.f, b = 0.f;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const float x0 = bf16lo(raw[(h + r) * 4 + i]) - mean[r], x1 = bf16hi(raw[(h + r) * 4 + i]) - mean[r];
+                        const float x0 = add_lo(raw[(h + r) * 4 + i], -mean[r]), x1 = add_hi(raw[(h + r) * 4 + i], -mean[r]);
                         a = fmaf(x0, x0, a);
                         b = fmaf(x1, x1, b);
                     }

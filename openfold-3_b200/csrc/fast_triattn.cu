@@ -1027,8 +1027,8 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
                         const uint32_t zr = zraw[cb * 8 + ch * 4 + j];
                         float v0 = __uint_as_float(upd[e]), v1 = __uint_as_float(upd[e + 1]);
                         if (add_residual) {
-                            v0 += bf16lo(zr);
-                            v1 += bf16hi(zr);
+                            v0 = add_lo(zr, v0);
+                            v1 = add_hi(zr, v1);
                         }
                         o[j] = pack_bf16x2(v0, v1);
                     }

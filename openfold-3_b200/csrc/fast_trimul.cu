@@ -607,7 +607,12 @@ struct OutSmem {
 // tiles; two threads share a row, each with half of its channels. (One thread per row took 3400 + 4300 cycles for the two
 // LayerNorms and 3900 for the output of a tile's 17400 at N = 768: latency, with one warp of a group per scheduler; and the
 // row thread that waited for the store to leave its buffer another 1500.)
-constexpr int kOutThreads = 32 * (3 + 2 * 8);
+constexpr int kOutThreads = 32 * (4 + 2 * 8);
+// registers: the block is launched with 96 per thread; the issuing warpgroup (its fourth warp is idle) gives up what the row
+// warps take, which hold half a row of z under the statistics of x (N = 768: 127 -> 119 us, with the
+// conversions for x and mixed adds for z that leave 20 bytes of spills; mixed adds for both: 122)
+constexpr int kOutRegsLaunch = 96, kOutRegsIssue = 64, kOutRegsRows = 104;
+static_assert(kOutRegsIssue + 4 * kOutRegsRows <= 5 * kOutRegsLaunch, "register split");
 
 template <int C>
 __global__ void __launch_bounds__(kOutThreads, 1)
@@ -679,6 +684,8 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
     const uint32_t tmem_base = *tmem_ptr;
     grid_trigger();
     if (warp >= 1) grid_wait();
+    if (warp < 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOutRegsIssue));
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kOutRegsRows));
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -746,11 +753,11 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
             }
             tma_store_wait_all<0>();
         }
-    } else {
+    } else if (warp >= 4) {
         // ---------------------------------------------------------------- two row groups
-        const int g = (warp - 3) >> 3;
+        const int g = (warp - 4) >> 3;
         const int quad = warp & 3;
-        const int half = ((warp - 3) >> 2) & 1;   // which half of the row's channels
+        const int half = ((warp - 4) >> 2) & 1;   // which half of the row's channels
         const int row = quad * 32 + lane;
         const uint32_t ztile = sbase + Sm::kZ + g * tile_bytes<C>();
         const uint32_t xtile = sbase + Sm::kX + g * tile_bytes<C>();
@@ -775,7 +782,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
                     xraw[i] = lo | (hi << 16);
                 }
                 // (behind its first barrier everyone has read its column: rows may overwrite the buffer)
-                half_row_stats_xwarp<C>(xraw, row, half, xch, 1 + g, 256, mean, rstd);
+                half_row_stats_xwarp<C, false>(xraw, row, half, xch, 1 + g, 256, mean, rstd);
                 store_normalized_half_row<C>(xtile, row, half, xraw, mean, rstd, prm + 256, prm + 384);
             }
             // --- z row: keep the raw values for the residual, normalise in place (A operand 1)
@@ -887,6 +894,10 @@ int launch_out(int grid, cudaStream_t st, const CUtensorMap& tmZ, const CUtensor
                int x_line_shift, int add_residual) {
     static PerDeviceOnce configured;
     if (!configured.done()) {
+        cudaFuncAttributes fa;   // a block launched with fewer registers would wait for the split for good
+        OF3_CUDA_CHECK(cudaFuncGetAttributes(&fa, trimul_out_kernel<C>));
+        OF3_REQUIRE(fa.numRegs == kOutRegsLaunch, OF3_ERR_DRIVER, "trimul_out is built with %d registers, not %d", fa.numRegs,
+                    kOutRegsLaunch);
         OF3_CUDA_CHECK(cudaFuncSetAttribute(trimul_out_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             OutSmem<C>::kDyn));
         configured.mark();

@@ -58,6 +58,21 @@ __device__ __forceinline__ void add_bf16x2(float& x0, float& x1, uint32_t v) {
         : "r"(v));
 }
 
+// Low / high half of a pair of bf16 values + f, in one instruction: no conversion ahead of it and no register for one, which
+// in kernels at their register limit is worth more than the instruction (N = 768: triangle attention output 104 -> 95 us, no
+// spills left there; N = 256: pair transition 39.8 -> 38.2). The same bits as a conversion and an add; where a product comes
+// first, that pair is an fma and stays one. Packed fma.f32x2 for the normalisation: slower throughout (attention output 109).
+__device__ __forceinline__ float add_lo(uint32_t v, float f) {
+    float d;
+    asm("{\n.reg .b16 lo, hi;\nmov.b32 {lo, hi}, %1;\nadd.rn.f32.bf16 %0, lo, %2;\n}\n" : "=f"(d) : "r"(v), "f"(f));
+    return d;
+}
+__device__ __forceinline__ float add_hi(uint32_t v, float f) {
+    float d;
+    asm("{\n.reg .b16 lo, hi;\nmov.b32 {lo, hi}, %1;\nadd.rn.f32.bf16 %0, hi, %2;\n}\n" : "=f"(d) : "r"(v), "f"(f));
+    return d;
+}
+
 // Walks the row tiles t = first, first + step, ... of `lines` lines per sample and tiles_per_line tiles per line without a
 // division per tile: the 64-bit quotients and remainders of t took some 3900 cycles per tile in every warp's serial chain
 // (trimul_in at N = 768: of 10000).
@@ -158,7 +173,7 @@ __device__ __forceinline__ void row_stats(const uint32_t (&raw)[C / 2], float& m
         for (int i = 0; i < C / 4; i += 4) {
 #pragma unroll
             for (int a = 0; a < 4; ++a)
-                s[h * 4 + a] += bf16lo(raw[h * (C / 4) + i + a]) + bf16hi(raw[h * (C / 4) + i + a]);
+                s[h * 4 + a] += add_lo(raw[h * (C / 4) + i + a], bf16hi(raw[h * (C / 4) + i + a]));
         }
     }
     mean = (((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]))) * (1.0f / C);
@@ -171,7 +186,7 @@ __device__ __forceinline__ void row_stats(const uint32_t (&raw)[C / 2], float& m
         for (int i = 0; i < C / 4; i += 4) {
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const float x0 = bf16lo(raw[h * (C / 4) + i + a]) - mean, x1 = bf16hi(raw[h * (C / 4) + i + a]) - mean;
+                const float x0 = add_lo(raw[h * (C / 4) + i + a], -mean), x1 = add_hi(raw[h * (C / 4) + i + a], -mean);
                 v[h * 4 + a] = fmaf(x0, x0, v[h * 4 + a]);
                 v[h * 4 + a] = fmaf(x1, x1, v[h * 4 + a]);
             }
@@ -227,25 +242,27 @@ __device__ __forceinline__ void load_half_row(uint32_t tile, int row, int half, 
         raw[ch * 4 + 3] = v.w;
     }
 }
-// Sum, and sum of squared deviations, of this thread's half of a row's values.
-template <int C = kC>
+// Sum, and sum of squared deviations, of this thread's half of a row's values. kMixed: by mixed-precision adds (the same bits).
+template <int C = kC, bool kMixed = true>
 __device__ __forceinline__ float half_row_sum(const uint32_t (&raw)[C / 4]) {
     float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < C / 4; i += 4) {
 #pragma unroll
-        for (int a = 0; a < 4; ++a) s[a] += bf16lo(raw[i + a]) + bf16hi(raw[i + a]);
+        for (int a = 0; a < 4; ++a)
+            s[a] += kMixed ? add_lo(raw[i + a], bf16hi(raw[i + a])) : bf16lo(raw[i + a]) + bf16hi(raw[i + a]);
     }
     return (s[0] + s[1]) + (s[2] + s[3]);
 }
-template <int C = kC>
+template <int C = kC, bool kMixed = true>
 __device__ __forceinline__ float half_row_sqdev(const uint32_t (&raw)[C / 4], float mean) {
     float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int i = 0; i < C / 4; i += 4) {
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            const float x0 = bf16lo(raw[i + a]) - mean, x1 = bf16hi(raw[i + a]) - mean;
+            const float x0 = kMixed ? add_lo(raw[i + a], -mean) : bf16lo(raw[i + a]) - mean;
+            const float x1 = kMixed ? add_hi(raw[i + a], -mean) : bf16hi(raw[i + a]) - mean;
             v[a] = fmaf(x0, x0, v[a]);
             v[a] = fmaf(x1, x1, v[a]);
         }
@@ -264,14 +281,14 @@ __device__ __forceinline__ void half_row_stats(const uint32_t (&raw)[C / 4], flo
 }
 // the two halves of a row belong to the same lane of two warps of a group of `nthreads` threads: the partial
 // results cross through xch (2 x 256 floats of shared memory) and two named barriers (id)
-template <int C = kC>
+template <int C = kC, bool kMixed = true>
 __device__ __forceinline__ void half_row_stats_xwarp(const uint32_t (&raw)[C / 4], int row, int half, float* xch,
                                                      int bar_id, int nthreads, float& mean, float& rstd) {
-    const float sum = half_row_sum<C>(raw);
+    const float sum = half_row_sum<C, kMixed>(raw);
     xch[half * 128 + row] = sum;
     group_sync(bar_id, nthreads);
     mean = (sum + xch[(half ^ 1) * 128 + row]) * (1.0f / C);
-    const float var = half_row_sqdev<C>(raw, mean);
+    const float var = half_row_sqdev<C, kMixed>(raw, mean);
     xch[256 + half * 128 + row] = var;
     group_sync(bar_id, nthreads);
     rstd = rsqrtf((var + xch[256 + (half ^ 1) * 128 + row]) * (1.0f / C) + kLnEps);
