@@ -39,7 +39,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // it three times with 2-byte loads took 8 - 20 us for 3840 rows.)
 template <int NV>
 struct Row {
-    float x[NV * 8];
+    float x[NV * 8], mean, rstd;
     __device__ __forceinline__ void load(const bf16* p, int C, int lane) {
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -55,7 +55,7 @@ struct Row {
         float s = 0.f;
 #pragma unroll
         for (int i = 0; i < NV * 8; ++i) s += x[i];
-        const float mean = warp_sum(s) / (float)C;
+        mean = warp_sum(s) / (float)C;
         float q = 0.f;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -67,7 +67,7 @@ struct Row {
                 q = fmaf(d, d, q);
             }
         }
-        const float rstd = rsqrtf(warp_sum(q) / (float)C + kEps);
+        rstd = rsqrtf(warp_sum(q) / (float)C + kEps);
 #pragma unroll
         for (int i = 0; i < NV * 8; ++i) x[i] *= rstd;
     }
@@ -176,17 +176,47 @@ __global__ void __launch_bounds__(256) ada_rows_kernel(const bf16* __restrict__ 
     Row<NV> row;
     row.load(a + r * C, C, lane);
     row.normalize(C, lane);
+    auto store = [&](int c, const float (&x)[8], const uint32_t (&gv)[4], const uint32_t (&sv)[4], const uint32_t (&bv)[4],
+                     auto divide) {
+        float gf[8], sf[8], bf[8], o[8];
+        unpack8(gv, gf);
+        unpack8(sv, sf);
+        unpack8(bv, bf);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = divide(x[e], 1.0f + __expf(-(gf[e] + bf[e]))) + sf[e];
+        *reinterpret_cast<uint4*>(an + r * C + c) = pack8(o);
+    };
+    // quotient_of's range: gates above -44 (a normalised value is at most sqrt(C))
+    float dmax = 1.0f;
+    uint32_t xmin = 0xffffffffu;   // of the bits of |x|, doubled, minus one: zero is in the range
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         const int c = (v * 32 + lane) * 8;
         if (c >= C) continue;
-        float gf[8], sf[8], bf[8], o[8];
-        unpack8(g[v], gf);
-        unpack8(s[v], sf);
-        unpack8(b[v], bf);
+        float x[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = fmaf(row.x[v * 8 + e], sigmoid_of(gf[e] + bf[e]), sf[e]);
-        *reinterpret_cast<uint4*>(an + r * C + c) = pack8(o);
+        for (int e = 0; e < 8; ++e) x[e] = row.x[v * 8 + e];
+        store(c, x, g[v], s[v], b[v], [&](float xe, float d) {
+            dmax = fmaxf(dmax, d);
+            xmin = min(xmin, 2u * __float_as_uint(xe) - 1u);
+            return quotient_of(xe, d);
+        });
+    }
+    if (dmax <= 0x1p64f && xmin >= 2u * __float_as_uint(0x1p-60f) - 1u) return;
+    // A closed gate, as a rule: the lane's values once more, by the division. Behind the loop and as one of its own, since
+    // divisions between the vectors above cost a short call 3 us per launch in instructions fetched and never run.
+#pragma unroll 1
+    for (int c = lane * 8; c < C; c += 256) {
+        uint32_t av[4], gv[4], sv[4], bv[4];
+        ld_row8_any(a + r * C + c, av);
+        ld_row8_any(g_lin + r * C + c, gv);
+        ld_row8_any(s_lin + r * C + c, sv);
+        ld_row8_any(b_g + c, bv);
+        float x[8];
+        unpack8(av, x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] = (x[e] - row.mean) * row.rstd;
+        store(c, x, gv, sv, bv, [](float xe, float d) { return xe / d; });
     }
 }
 

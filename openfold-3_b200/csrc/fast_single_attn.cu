@@ -454,6 +454,7 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
                 const uint32_t lsum = tmem_ld1(trow + C::kColO + DV);
                 tmem_ld_wait();
                 const float inv = 1.0f / __uint_as_float(lsum);
+                float gmin = 0.f;
 #pragma unroll
                 for (int part = 0; part < DV / 16; ++part) {
                     uint32_t r[16];
@@ -461,18 +462,32 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
                     tmem_ld_wait();
 #pragma unroll
                     for (int c = part * 16 / kV; c < (part + 1) * 16 / kV && c < D / kV; ++c) {
+                        float f[kV];
+#pragma unroll
+                        for (int e = 0; e < kV; ++e) f[e] = __uint_as_float(r[c * kV % 16 + e]) * inv;
+                        if (gate != nullptr) {
+#pragma unroll
+                            for (int e = 0; e < kV; ++e) {
+                                const float ge = (e & 1) ? bf16hi(gw[c][e >> 1]) : bf16lo(gw[c][e >> 1]);
+                                gmin = fminf(gmin, ge);
+                                f[e] *= rcp_of(1.0f + __expf(-ge));
+                            }
+                        }
                         uint32_t o[kV / 2];
 #pragma unroll
-                        for (int e = 0; e < kV / 2; ++e) {
-                            float f0 = __uint_as_float(r[c * kV % 16 + 2 * e]) * inv;
-                            float f1 = __uint_as_float(r[c * kV % 16 + 2 * e + 1]) * inv;
-                            if (gate != nullptr) {
-                                f0 *= sigmoid_of(bf16lo(gw[c][e]));
-                                f1 *= sigmoid_of(bf16hi(gw[c][e]));
-                            }
-                            o[e] = pack_bf16x2(f0, f1);
-                        }
+                        for (int e = 0; e < kV / 2; ++e) o[e] = pack_bf16x2(f[2 * e], f[2 * e + 1]);
                         if (store) store_row<kV>(out + off + c * kV, o);
+                    }
+                }
+                // A row with a closed gate, past the range of rcp_of: once more by the division (exactly 0 where the
+                // exponential overflows). A loop of its own, which costs nothing where it is not run.
+                if (__any_sync(0xffffffffu, store && gate != nullptr && gmin < kSigmoidMin)) {
+#pragma unroll 1
+                    for (int c = 0; c < D; ++c) {
+                        const uint32_t acc = tmem_ld1(trow + C::kColO + c);
+                        tmem_ld_wait();
+                        if (store)
+                            out[off + c] = __float2bfloat16_rn(__uint_as_float(acc) * inv * sigmoidf_fast(__bfloat162float(gate[off + c])));
                     }
                 }
             } else if (lane == 0) {

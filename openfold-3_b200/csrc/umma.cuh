@@ -280,14 +280,25 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
-// 1 / (1 + exp(-x)) with the reciprocal refined by one Newton step, r (2 - d r): as close as the division, in a third of
-// its instructions. The clamp keeps d finite (0 * inf in the step): below -87 the result is 1.6e-38 instead of less.
-__device__ __forceinline__ float sigmoid_of(float x) {
-    const float d = 1.0f + __expf(-x > 87.0f ? 87.0f : -x);   // (a NaN stays one)
+// The bits of 1.0f / d for 1 <= d < 2^126, without the branch for other values, which keeps the divisions of a row one behind
+// the other: the approximation within one unit in the last place, then one Newton step r + r (1 - d r), whose residual is exact
+// (Markstein 1990). Equal to the division for every float of that range.
+__device__ __forceinline__ float rcp_of(float d) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
     return fmaf(r, fmaf(-d, r, 1.0f), r);
 }
+// The bits of x / d for 2^-60 <= |x| < 2^60 or x = 0, and 1 <= d <= 2^64 (NaN stays NaN): Markstein's theorem, a product with
+// the rounded reciprocal corrected by its exact remainder (which loses the sign of a zero); nothing here underflows. 2.6e10
+// random pairs equal the division.
+__device__ __forceinline__ float quotient_of(float x, float d) {
+    const float y = rcp_of(d), q = x * y;
+    return copysignf(fmaf(fmaf(-d, q, x), y, q), x);
+}
+// 1 / (1 + exp(-x)): the bits of the division down to x = -87; below that 1.6e-38 instead of less, which keeps d in range
+// (a NaN stays one).
+constexpr float kSigmoidMin = -87.0f;
+__device__ __forceinline__ float sigmoid_of(float x) { return rcp_of(1.0f + __expf(-x > -kSigmoidMin ? -kSigmoidMin : -x)); }
 
 // 32 bytes of global memory per thread (one full sector); p 32-byte aligned
 __device__ __forceinline__ void stg256(void* p, const uint32_t (&o)[8]) {
