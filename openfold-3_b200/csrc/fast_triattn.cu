@@ -209,7 +209,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
             // The transposed view's mask column, as a row for the attention core: there every block of 128 queries and every
             // head of a line would fetch a sector per key (N = 768: 85 of 762 us).
             const int pos = tc.tile * kRows + row;
-            const bool copy_mask = kTransposed && mask != nullptr && half == 0 && pos < N;
+            const bool copy_mask = kTransposed && mask_t != nullptr && half == 0 && pos < N;
             __nv_bfloat16 mv = __float2bfloat16_rn(1.0f);
             if (copy_mask) mv = mask[((long long)tc.b * N + pos) * N + tc.line];
             if (!mbar_wait(z_full(s), (it / kSt) & 1u, abort_flag)) {
@@ -397,8 +397,7 @@ template <int D>
 __global__ void __launch_bounds__(kCoreThreads, 2)
 triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16* __restrict__ k_img,
                     const __nv_bfloat16* __restrict__ v_img, const __nv_bfloat16* __restrict__ tb_img,
-                    const __nv_bfloat16* __restrict__ mask, int mask_pitch, __nv_bfloat16* __restrict__ o_out, int R,
-                    int N, float inf, int* status) {
+                    const MaskView mask, __nv_bfloat16* __restrict__ o_out, int R, int N, float inf, int* status) {
     using Sm = CoreSmem<D>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -433,7 +432,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
     const int q0 = qt * kBQ;
     const int nblk = (N + kBK - 1) / kBK;
     const int nkp = nblk * kBK;
-    // lines past the end of the sample recompute the first line of the group and are not stored
+    // (a line past the end of the sample: the images' padding line, unwritten, with the mask of the group's first; not stored)
     auto line_of = [&](int L) { return (line0 + L < R) ? line0 + L : line0; };
 
     if (threadIdx.x == 0) {
@@ -602,7 +601,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
         // independent of each other) while the first copies and GEMMs are already under way.
         {
             const int gt = quad * 32 + lane;  // 0..127 within the line's warps
-            const int line = line_of(L);
+            const __nv_bfloat16* mrow = mask.p + (b * mask.batch + (long long)line_of(L) * mask.line);
             for (int base = 0; base < nkp; base += 128 * 8) {   // warp-uniform trip count (ballot below)
                 const int c0 = base + gt * 8;
                 const bool active = c0 < nkp;
@@ -611,8 +610,8 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
                 for (int e = 0; e < 8; ++e) {
                     const int k = c0 + e;
                     float m = 1.0f;
-                    if (mask != nullptr && k < N)
-                        m = __bfloat162float(mask[((long long)b * R + line) * mask_pitch + k]);
+                    if (mask.p != nullptr && k < N)
+                        m = __bfloat162float(mrow[k * mask.key]);
                     v[e] = (k < N) ? inf * (m - 1.0f) * kLog2e : -INFINITY;
                 }
                 bool any = false;
@@ -1090,9 +1089,6 @@ int set_attrs() {
     return OF3_OK;
 }
 
-// elements per line of the mask rows that triattn_project writes for a transposed view
-int mask_pitch(int N) { return (int)align_up(N, kBK); }
-
 template <int C, bool kT>
 int project_impl(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* vt,
                  __nv_bfloat16* tb, const __nv_bfloat16* mask, __nv_bfloat16* mask_t, int B, int R, int N, int row0,
@@ -1118,12 +1114,12 @@ int project_impl(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __n
     LaunchScope scope(kKidProj, st);
     OF3_CUDA_CHECK(launch_chained(triattn_proj_kernel<C, kT>, grid, kProjThreads, ProjSmem<C>::kDyn, st, tmZ, tmW[0],
                                   tmW[1], tmW[2], tmWb, (P)p->ln_w, (P)p->ln_b, q, k, vt, tb, mask, mask_t, B,
-                                  R, N, mask_pitch(N), row0, device_status_ptr()));
+                                  R, N, triattn_mask_pitch(N), row0, device_status_ptr()));
     return OF3_OK;
 }
 
 template <int C, bool kT>
-int finish_impl(const __nv_bfloat16* z, const __nv_bfloat16* mask, int pitch, __nv_bfloat16* out, const __nv_bfloat16* q,
+int finish_impl(const __nv_bfloat16* z, const MaskView& mask, __nv_bfloat16* out, const __nv_bfloat16* q,
                 const __nv_bfloat16* k, const __nv_bfloat16* vt, const __nv_bfloat16* tb, __nv_bfloat16* o, int B,
                 int R, int N, float inf, int add_residual, const of3_triattn_params* p, cudaStream_t st) {
     int rc;
@@ -1140,8 +1136,8 @@ int finish_impl(const __nv_bfloat16* z, const __nv_bfloat16* mask, int pitch, __
     {
         LaunchScope scope(kKidCore, st);
         OF3_CUDA_CHECK(launch_chained(triattn_core_kernel<C / kH>, (unsigned)ctas, kCoreThreads,
-                                      CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK)), st, q, k, vt, tb, mask, pitch, o, R, N,
-                                      inf, status));
+                                      CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK)), st, q, k, vt, tb, mask, o, R, N, inf,
+                                      status));
     }
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
@@ -1169,12 +1165,12 @@ size_t triattn_bias_elems(int B, int R, int N) {
     return (size_t)B * kH * ceil_div(N, kBiasK) * R * kBiasK;
 }
 
-size_t triattn_mask_elems(int B, int N) { return (size_t)B * N * mask_pitch(N); }
+int triattn_mask_pitch(int N) { return (int)align_up(N, kBK); }
 
 // q, k, v operand images and this shard's rows of the pair-bias image tb[(b*H + h)][key block][line][32]
 // from R lines of N positions; row0 = index of the shard's first line among all N query rows (0 for a whole
-// tensor). transposed: whole square tensors only; their mask [B, N, N], where there is one, goes to mask_t
-// (triattn_mask_elems elements) with the view's lines as rows.
+// tensor). transposed: whole square tensors only; where mask_t is given, their mask [B, N, N] goes there with the view's lines
+// as rows of triattn_mask_pitch elements.
 int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* vt,
                     __nv_bfloat16* tb, int B, int R, int N, int row0, bool transposed,
                     const of3_triattn_params* p, cudaStream_t st, int C, const __nv_bfloat16* mask,
@@ -1183,6 +1179,7 @@ int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, 
     OF3_REQUIRE((((uintptr_t)q | (uintptr_t)k | (uintptr_t)vt) & 15) == 0, OF3_ERR_ALIGN,
                 "triattn: q / k / v images must be 16-byte aligned");
     OF3_REQUIRE(!transposed || R == N, OF3_ERR_SHAPE, "triattn: transposed view needs the whole tensor");
+    OF3_REQUIRE(mask_t == nullptr || mask != nullptr, OF3_ERR_ARG, "triattn: mask rows without a mask");
     if (C == 128)
         return transposed ? project_impl<128, true>(z, q, k, vt, tb, mask, mask_t, B, R, N, row0, p, st)
                           : project_impl<128, false>(z, q, k, vt, tb, mask, mask_t, B, R, N, row0, p, st);
@@ -1191,9 +1188,8 @@ int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, 
 }
 
 // attention over the R lines with the pair-bias image of all N query rows (tb [(b*H + h)][key block][N][32]),
-// gate, output projection, residual. mask: a row per line of the view, [B, R, N]; of a transposed view the rows that
-// triattn_project wrote.
-int triattn_finish(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out,
+// gate, output projection, residual.
+int triattn_finish(const __nv_bfloat16* z, const MaskView& mask, __nv_bfloat16* out,
                    const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* vt,
                    const __nv_bfloat16* tb, __nv_bfloat16* o, int B, int R, int N, float inf,
                    bool transposed, int add_residual, const of3_triattn_params* p, cudaStream_t st, int C) {
@@ -1205,12 +1201,11 @@ int triattn_finish(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloa
     OF3_REQUIRE(N <= kMaxKeys, OF3_ERR_SHAPE, "triattn: N %d above the %d keys one CTA keeps a mask row for", N,
                 kMaxKeys);
     OF3_REQUIRE(!transposed || R == N, OF3_ERR_SHAPE, "triattn: transposed view needs the whole tensor");
-    const int pitch = transposed ? mask_pitch(N) : N;
     if (C == 128)
-        return transposed ? finish_impl<128, true>(z, mask, pitch, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
-                          : finish_impl<128, false>(z, mask, pitch, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
-    return transposed ? finish_impl<64, true>(z, mask, pitch, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
-                      : finish_impl<64, false>(z, mask, pitch, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
+        return transposed ? finish_impl<128, true>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
+                          : finish_impl<128, false>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
+    return transposed ? finish_impl<64, true>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
+                      : finish_impl<64, false>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
 }
 
 int triattn(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* out, int B, int N, int C,
@@ -1222,14 +1217,16 @@ int triattn(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* ou
     __nv_bfloat16* vt = (__nv_bfloat16*)ws.take(img);
     __nv_bfloat16* o = (__nv_bfloat16*)ws.take(plane);
     __nv_bfloat16* tb = (__nv_bfloat16*)ws.take(triattn_bias_elems(B, N, N) * sizeof(__nv_bfloat16));
-    __nv_bfloat16* mask_t = (__nv_bfloat16*)ws.take(triattn_mask_elems(B, N) * sizeof(__nv_bfloat16));
+    const int pitch = triattn_mask_pitch(N);
+    __nv_bfloat16* mask_t = (__nv_bfloat16*)ws.take((size_t)B * N * pitch * sizeof(__nv_bfloat16));
     if (!ws.base) return OF3_OK;
     OF3_REQUIRE(ws.ok(), OF3_ERR_WORKSPACE, "triattn: workspace too small (%zu needed)", ws.off);
     const bool tr = (flags & OF3_FLAG_TRANSPOSED) != 0;
+    if (!tr || mask == nullptr) mask_t = nullptr;
     int rc = triattn_project(z, q, k, vt, tb, B, N, N, 0, tr, p, st, C, mask, mask_t);
     if (rc) return rc;
-    return triattn_finish(z, (tr && mask != nullptr) ? mask_t : mask, out, q, k, vt, tb, o, B, N, N, inf, tr,
-                          (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, st, C);
+    const MaskView view = mask_t != nullptr ? mask_rows(mask_t, N, pitch) : mask_rows(mask, N, N);
+    return triattn_finish(z, view, out, q, k, vt, tb, o, B, N, N, inf, tr, (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, st, C);
 }
 
 }  // namespace fast
