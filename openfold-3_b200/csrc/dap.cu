@@ -164,7 +164,7 @@ int of3_dap_triattn_finish(const void* z_rows, const void* mask_rows, void* out_
                 "dap_triattn_finish: null pointer argument");
     OF3_REQUIRE(R > 0 && N > 0, OF3_ERR_ARG, "dap_triattn_finish: non-positive size");
     CallScope call;
-    return fast::triattn_finish((const __nv_bfloat16*)z_rows, fast::mask_rows((const __nv_bfloat16*)mask_rows, R, N),
+    return fast::triattn_finish((const __nv_bfloat16*)z_rows, {(const __nv_bfloat16*)mask_rows, N, false},
                                 (__nv_bfloat16*)out_rows, (const __nv_bfloat16*)q, (const __nv_bfloat16*)k,
                                 (const __nv_bfloat16*)vt, (const __nv_bfloat16*)bias_all, (__nv_bfloat16*)o_scratch, 1, R,
                                 N, inf, false, (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, (cudaStream_t)stream);

@@ -393,11 +393,13 @@ struct CoreSmem {
     static uint32_t dyn_bytes(int nblk) { return kMb + kLines * nblk * kBK * 4 + 1024; }
 };
 
-template <int D>
+// kColumns: where the mask of a transposed view is read in place (strides that are not constants cost the short calls 0.3 %)
+template <int D, bool kColumns>
 __global__ void __launch_bounds__(kCoreThreads, 2)
 triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16* __restrict__ k_img,
                     const __nv_bfloat16* __restrict__ v_img, const __nv_bfloat16* __restrict__ tb_img,
-                    const MaskView mask, __nv_bfloat16* __restrict__ o_out, int R, int N, float inf, int* status) {
+                    const __nv_bfloat16* __restrict__ mask, int mask_pitch, __nv_bfloat16* __restrict__ o_out, int R,
+                    int N, float inf, int* status) {
     using Sm = CoreSmem<D>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -601,7 +603,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
         // independent of each other) while the first copies and GEMMs are already under way.
         {
             const int gt = quad * 32 + lane;  // 0..127 within the line's warps
-            const __nv_bfloat16* mrow = mask.p + (b * mask.batch + (long long)line_of(L) * mask.line);
+            const int line = line_of(L);
             for (int base = 0; base < nkp; base += 128 * 8) {   // warp-uniform trip count (ballot below)
                 const int c0 = base + gt * 8;
                 const bool active = c0 < nkp;
@@ -610,8 +612,11 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
                 for (int e = 0; e < 8; ++e) {
                     const int k = c0 + e;
                     float m = 1.0f;
-                    if (mask.p != nullptr && k < N)
-                        m = __bfloat162float(mrow[k * mask.key]);
+                    if (mask != nullptr && k < N) {
+                        const long long mi = kColumns ? ((long long)b * mask_pitch + k) * mask_pitch + line
+                                                      : ((long long)b * R + line) * mask_pitch + k;
+                        m = __bfloat162float(mask[mi]);
+                    }
                     v[e] = (k < N) ? inf * (m - 1.0f) * kLog2e : -INFINITY;
                 }
                 bool any = false;
@@ -1076,12 +1081,14 @@ int set_attrs() {
     if (!configured.done()) {
         OF3_CUDA_CHECK(cudaFuncSetAttribute(triattn_proj_kernel<C, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             ProjSmem<C>::kDyn));
-        cudaFuncAttributes fa;   // a block launched with fewer registers would wait for the split for good
-        OF3_CUDA_CHECK(cudaFuncGetAttributes(&fa, triattn_core_kernel<C / kH>));
-        OF3_REQUIRE(fa.numRegs == kCoreRegsLaunch, OF3_ERR_DRIVER, "triattn_core is built with %d registers, not %d",
-                    fa.numRegs, kCoreRegsLaunch);
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(triattn_core_kernel<C / kH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            CoreSmem<C / kH>::dyn_bytes(kMaxKeys / kBK)));
+        for (auto* core : {triattn_core_kernel<C / kH, false>, triattn_core_kernel<C / kH, true>}) {
+            cudaFuncAttributes fa;   // a block launched with fewer registers would wait for the split for good
+            OF3_CUDA_CHECK(cudaFuncGetAttributes(&fa, core));
+            OF3_REQUIRE(fa.numRegs == kCoreRegsLaunch, OF3_ERR_DRIVER, "triattn_core is built with %d registers, not %d",
+                        fa.numRegs, kCoreRegsLaunch);
+            OF3_CUDA_CHECK(cudaFuncSetAttribute(core, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                CoreSmem<C / kH>::dyn_bytes(kMaxKeys / kBK)));
+        }
         OF3_CUDA_CHECK(cudaFuncSetAttribute(triattn_out_kernel<C, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             AOutSmem<C>::kDyn));
         configured.mark();
@@ -1135,9 +1142,9 @@ int finish_impl(const __nv_bfloat16* z, const MaskView& mask, __nv_bfloat16* out
     OF3_REQUIRE(ctas < (1LL << 31), OF3_ERR_SHAPE, "triattn: too many attention tiles");
     {
         LaunchScope scope(kKidCore, st);
-        OF3_CUDA_CHECK(launch_chained(triattn_core_kernel<C / kH>, (unsigned)ctas, kCoreThreads,
-                                      CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK)), st, q, k, vt, tb, mask, o, R, N, inf,
-                                      status));
+        auto* core = mask.columns ? triattn_core_kernel<C / kH, true> : triattn_core_kernel<C / kH, false>;
+        OF3_CUDA_CHECK(launch_chained(core, (unsigned)ctas, kCoreThreads, CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK)), st, q,
+                                      k, vt, tb, mask.p, mask.pitch, o, R, N, inf, status));
     }
     const long long tiles = (long long)B * R * ceil_div(N, kRows);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
@@ -1201,6 +1208,7 @@ int triattn_finish(const __nv_bfloat16* z, const MaskView& mask, __nv_bfloat16* 
     OF3_REQUIRE(N <= kMaxKeys, OF3_ERR_SHAPE, "triattn: N %d above the %d keys one CTA keeps a mask row for", N,
                 kMaxKeys);
     OF3_REQUIRE(!transposed || R == N, OF3_ERR_SHAPE, "triattn: transposed view needs the whole tensor");
+    OF3_REQUIRE(!mask.columns || transposed, OF3_ERR_ARG, "triattn: mask by columns of a view that is not transposed");
     if (C == 128)
         return transposed ? finish_impl<128, true>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st)
                           : finish_impl<128, false>(z, mask, out, q, k, vt, tb, o, B, R, N, inf, add_residual, p, st);
@@ -1217,15 +1225,18 @@ int triattn(const __nv_bfloat16* z, const __nv_bfloat16* mask, __nv_bfloat16* ou
     __nv_bfloat16* vt = (__nv_bfloat16*)ws.take(img);
     __nv_bfloat16* o = (__nv_bfloat16*)ws.take(plane);
     __nv_bfloat16* tb = (__nv_bfloat16*)ws.take(triattn_bias_elems(B, N, N) * sizeof(__nv_bfloat16));
+    const bool tr = (flags & OF3_FLAG_TRANSPOSED) != 0;
+    if (!ws.base && !tr) return OF3_OK;
+    OF3_REQUIRE(!ws.base || ws.ok(), OF3_ERR_WORKSPACE, "triattn: workspace too small (%zu needed)", ws.off);
+    // Mask rows of the ending node, 0.1 % of the workspace: where they do not fit (a workspace of the starting node's size),
+    // the attention reads the mask in place (N = 768: 85 us more).
     const int pitch = triattn_mask_pitch(N);
     __nv_bfloat16* mask_t = (__nv_bfloat16*)ws.take((size_t)B * N * pitch * sizeof(__nv_bfloat16));
     if (!ws.base) return OF3_OK;
-    OF3_REQUIRE(ws.ok(), OF3_ERR_WORKSPACE, "triattn: workspace too small (%zu needed)", ws.off);
-    const bool tr = (flags & OF3_FLAG_TRANSPOSED) != 0;
-    if (!tr || mask == nullptr) mask_t = nullptr;
+    if (!tr || mask == nullptr || !ws.ok()) mask_t = nullptr;
     int rc = triattn_project(z, q, k, vt, tb, B, N, N, 0, tr, p, st, C, mask, mask_t);
     if (rc) return rc;
-    const MaskView view = mask_t != nullptr ? mask_rows(mask_t, N, pitch) : mask_rows(mask, N, N);
+    const MaskView view = mask_t != nullptr ? MaskView{mask_t, pitch, false} : MaskView{mask, N, tr && mask != nullptr};
     return triattn_finish(z, view, out, q, k, vt, tb, o, B, N, N, inf, tr, (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0, p, st, C);
 }
 

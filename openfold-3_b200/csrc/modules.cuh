@@ -45,14 +45,13 @@ int trimul_output(const __nv_bfloat16* z, __nv_bfloat16* out, const __nv_bfloat1
                   int add_residual, const of3_trimul_params* p, cudaStream_t st, int C = 128);
 size_t triattn_image_elems(int B, int R, int N, int C = 128);
 size_t triattn_bias_elems(int B, int R, int N);  // bf16 elements of the pair-bias image [B*4][key blocks][R][32]
-// The mask of a view's lines: of sample b, line l and key k at p[b * batch + l * line + k * key]; p null: no mask.
+// The mask of a view's lines, p null: none. Of sample b, line l and key k at p[(b * lines + l) * pitch + k], or of a transposed
+// view in place, by columns, at p[(b * pitch + k) * pitch + l].
 struct MaskView {
     const __nv_bfloat16* p;
-    long long batch;
-    int line, key;
+    int pitch;
+    bool columns;
 };
-inline MaskView mask_rows(const __nv_bfloat16* p, int R, int pitch) { return {p, (long long)R * pitch, pitch, 1}; }
-inline MaskView mask_columns(const __nv_bfloat16* p, int N) { return {p, (long long)N * N, 1, N}; }
 int triattn_project(const __nv_bfloat16* z, __nv_bfloat16* q, __nv_bfloat16* k, __nv_bfloat16* vt,
                     __nv_bfloat16* tb, int B, int R, int N, int row0, bool transposed,
                     const of3_triattn_params* p, cudaStream_t st, int C = 128, const __nv_bfloat16* mask = nullptr,

@@ -50,6 +50,19 @@ def test_workspace_queries_need_no_gpu(pkg):
         assert lib.of3_cond_transition_workspace_bytes(128, 768, 384, 2, dt, 0) > 0
 
 
+@pytest.mark.parametrize("B,N,c", [(1, 1, 128), (2, 37, 64), (1, 2048, 128)])
+def test_only_the_ending_node_asks_for_mask_rows(pkg, B, N, c):
+    """Operand images, output and bias tiles are what both nodes need; a row of the mask per line, in whole blocks of 64 keys,
+    the ending node's alone. (Each array starts on 256 bytes, and so does the first.)"""
+    up = lambda x, to: (x + to - 1) // to * to  # noqa: E731
+    start, end = (pkg.lib.load().of3_triattn_workspace_bytes(B, N, c, 4, c // 4, 0, flags)
+                  for flags in (0, pkg.lib.FLAG_TRANSPOSED))
+    images = 3 * B * up(N, 4) * up(N, 128) * c * 2
+    rest = up(B * N * N * c * 2, 256) + B * 4 * up(N, 32) * N * 2
+    assert start <= images + rest + 256
+    assert up(start, 256) + B * N * up(N, 64) * 2 == end
+
+
 def test_no_cpu_fallback(pkg):
     """CPU tensors are refused: there is no path that avoids the CUDA library."""
     m = pkg.TriangleMultiplicationOutgoing(128, 128).eval()

@@ -118,3 +118,19 @@ def test_ending_node_is_the_starting_node_of_the_transposed_tensor(c, B, N):
             want = start(z.transpose(1, 2).contiguous(), mask=None if mask is None else mask.transpose(1, 2).contiguous())
             assert torch.equal(end(z, mask=mask), want.transpose(1, 2))
     pkg.lib.check_device_status()
+
+
+def test_the_ending_node_in_a_workspace_of_the_starting_nodes_size(monkeypatch):
+    """No room for mask rows: the mask is read in place, the same bits; without a mask there is nothing to make room for."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator().manual_seed(3)
+    layer = pkg.TriangleAttention(128, 32, 4, starting=False).to(dev, bf).eval().requires_grad_(False)
+    for p in layer.parameters():
+        p.copy_(torch.randn(p.shape, generator=g) * (p.shape[-1] ** -0.5 if p.dim() > 1 else 0.3))
+    z, m = torch.randn(2, 70, 70, 128, generator=g).to(dev, bf), rand_mask((2, 70, 70), g, 0.8).to(dev, bf)
+    want = [layer(z, mask=mask) for mask in (m, None)]
+    size = pkg.lib.load().of3_triattn_workspace_bytes(2, 70, 128, 4, 32, 0, 0)
+    monkeypatch.setattr(pkg.lib, "workspace", lambda nbytes, device, stream=None: torch.empty(size, dtype=torch.uint8, device=device))
+    for mask, w in zip((m, None), want):
+        assert torch.equal(layer(z, mask=mask), w)
+    pkg.lib.check_device_status()
