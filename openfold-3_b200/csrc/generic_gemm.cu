@@ -385,20 +385,18 @@ __global__ void __launch_bounds__(G* BM / TM * BN / TN) gemm_kernel(const Args<T
 template <int EPI>
 __global__ void __launch_bounds__(128, 2) gemm_pairs_kernel(const Args<float> p) {
     constexpr int BM = 128, BN = 64, TM = 8, TN = 8, BK = 16, kStages = 4, kPitch = BK + 4;
-    constexpr bool kPaired = EPI == kGatedPlanes || EPI == kSwiglu;
-    constexpr int HN = BN / 2;
+    static_assert(EPI == kStore || EPI == kFinal, "one weight per group");
     extern __shared__ __align__(16) float slabs[];   // stages x (BM + BN) rows
     umma::grid_trigger();
     umma::grid_wait();
     const int K = p.K, n = p.n;
     const long long M = p.M, m0 = (long long)blockIdx.x * BM;
-    const int tiles_n = (n + (kPaired ? HN : BN) - 1) / (kPaired ? HN : BN);
+    const int tiles_n = (n + BN - 1) / BN;
     const int grp = blockIdx.y / tiles_n;
-    const int n0 = (blockIdx.y % tiles_n) * (kPaired ? HN : BN);
+    const int n0 = (blockIdx.y % tiles_n) * BN;
     const long long boff = (long long)blockIdx.z * p.a_batch;
     const float* a = p.a + boff;
-    const float* w0 = (kPaired ? p.w[2 * grp] : p.w[grp]) + boff;
-    const float* w1 = kPaired ? p.w[2 * grp + 1] : w0;
+    const float* w = p.w[grp] + boff;
 
     // this thread's 16-byte vectors of a slab: row t / 4 + 32 i, k offset 4 (t % 4)
     const int kc = (threadIdx.x & 3) * 4, lr = threadIdx.x >> 2;
@@ -414,9 +412,8 @@ __global__ void __launch_bounds__(128, 2) gemm_pairs_kernel(const Args<float> p)
             dst[i] = slabs + ((r & 64) + (r & 3) * 16 + ((r & 63) >> 2)) * kPitch + kc;
         } else {
             const int c = lr + 32 * (i - 4);               // 32 hf + 4 tx + e -> slot 32 hf + 8 e + tx
-            const int col = n0 + (kPaired ? c & 31 : c);
-            in[i] = col < n;
-            src[i] = (kPaired && c >= HN ? w1 : w0) + (long long)(in[i] ? col : 0) * K + kc;
+            in[i] = n0 + c < n;
+            src[i] = w + (long long)(in[i] ? n0 + c : 0) * K + kc;
             dst[i] = slabs + (BM + (c & 32) + (c & 3) * 8 + ((c & 31) >> 2)) * kPitch + kc;
         }
     }
@@ -500,11 +497,11 @@ int launch(Args<T> p, int groups, int batch, cudaStream_t st) {
                 M, p.n, batch);
     const dim3 grid((unsigned)gx, (unsigned)gy, batch);
     LaunchScope scope(20, st);
-    if constexpr (std::is_same<T, float>::value && !K_OUTER) {
+    if constexpr (std::is_same<T, float>::value && !K_OUTER && !kPaired) {
         // where every operand, and every plane of a batch, comes in whole vectors along k
         uintptr_t bits = reinterpret_cast<uintptr_t>(p.a) | (uintptr_t)(p.K & 3) << 2 | (uintptr_t)(p.a_batch & 3) << 2;
-        for (int i = 0; i < (kPaired ? 2 : 1) * groups; ++i) bits |= reinterpret_cast<uintptr_t>(p.w[i]);
-        if (large && (EPI == kStore || EPI == kFinal) && (bits & 15) == 0) return launch_pairs<EPI>(p, grid, st);
+        for (int i = 0; i < groups; ++i) bits |= reinterpret_cast<uintptr_t>(p.w[i]);
+        if (large && (bits & 15) == 0) return launch_pairs<EPI>(p, grid, st);
     }
     if (large)
         OF3_CUDA_CHECK(launch_chained(gemm_kernel<128, 64, 8, 8, 1, EPI, K_OUTER, T>, grid, 128, 0, st, p));
