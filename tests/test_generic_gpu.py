@@ -45,3 +45,21 @@ def test_fp32_pair_block_on_large_tiles(c_z, c_hidden_mul, heads, d, n, N):
     with torch.no_grad():
         got = blk(z.to(dev), m.to(dev)).cpu()
     assert rel_err(got, ref) < 1e-4, rel_err(got, ref)
+
+
+@pytest.mark.parametrize("c_hidden_mul,B,N", [(128, 1, 68), (128, 2, 132), (36, 1, 140)])
+def test_fp32_contraction_in_whole_vectors(c_hidden_mul, B, N):
+    """N in whole vectors and enough planes for the 128 x 64 tiles: the outgoing update's N x N products, a plane per batch
+    entry, read in vectors along k, with ragged row and column tiles and a ragged last slab of k."""
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(N)
+    z, m = torch.randn(B, N, N, 32, generator=g), rand_mask((B, N, N), g, 0.9)
+    for cls in (pkg.TriangleMultiplicationOutgoing, pkg.TriangleMultiplicationIncoming):
+        layer = cls(32, c_hidden_mul)
+        with torch.no_grad():
+            for p in layer.parameters():
+                p.copy_(torch.randn(p.shape, generator=g) * (p.shape[-1] ** -0.5 if p.dim() > 1 else 0.3))
+            P = {"l." + k: v.clone() for k, v in layer.state_dict().items()}
+            ref = oracle.triangle_multiplicative_update(z, m, P, "l.", outgoing=cls is pkg.TriangleMultiplicationOutgoing)
+            got = layer.to(dev).eval()(z.to(dev), mask=m.to(dev)).cpu()
+        assert rel_err(got, ref) < 1e-4, rel_err(got, ref)
