@@ -237,16 +237,21 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                     const float rs = p1[row], nm = p1[128 + row];
                     tmem_ld_wait();
                     if (row < span) {
-                        const int key = ((((row & 31) >> 3) ^ ((tw.line >> 1) & 3)) << 3) | (row & 7);
-                        __nv_bfloat16* trow = tiles + (long long)tw.b * kHeads * hs + (long long)(pos >> 5) * N * 32 +
-                                              tw.line * 32 + key;
-                        float* drow = dst + (long long)tw.b * kHeads * N + pos;
-#pragma unroll
-                        for (int h = 0; h < kHeads; ++h) {
+                        auto value = [&](int h) {
                             const float2 cc = chan[h];
-                            const float v = fmaf(rs, __uint_as_float(acc[h]), fmaf(nm, cc.x, cc.y));
-                            if (tiles != nullptr) trow[h * hs] = __float2bfloat16_rn(pos < N ? v * kLog2e : 0.f);
-                            else drow[(long long)h * N] = v;
+                            return fmaf(rs, __uint_as_float(acc[h]), fmaf(nm, cc.x, cc.y));
+                        };
+                        if (tiles != nullptr) {
+                            const int key = ((((row & 31) >> 3) ^ ((tw.line >> 1) & 3)) << 3) | (row & 7);
+                            __nv_bfloat16* trow = tiles + (long long)tw.b * kHeads * hs + (long long)(pos >> 5) * N * 32 +
+                                                  tw.line * 32 + key;
+#pragma unroll
+                            for (int h = 0; h < kHeads; ++h)
+                                trow[h * hs] = __float2bfloat16_rn(pos < N ? value(h) * kLog2e : 0.f);
+                        } else {
+                            float* drow = dst + (long long)tw.b * kHeads * N + pos;
+#pragma unroll
+                            for (int h = 0; h < kHeads; ++h) drow[(long long)h * N] = value(h);
                         }
                     }
                     tc_fence_before_sync();
@@ -260,16 +265,8 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                 const int n = g * 128 + quad * 32 + lane, l = n >> 4, h = n & 15;
                 if (g * 128 + quad * 32 < layers * kHeads) {   // the warp has a channel (a layer is half a warp)
                     const float2 cc = chan[n];
-                    __nv_bfloat16* trow = nullptr;
-                    float* drow = nullptr;
-                    int sw = 0;
-                    const bool vec = (N & 3) == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
-                    if (tiles != nullptr) {
-                        sw = (tw.line >> 1) & 3;
-                        trow = tiles + l * layer_stride + ((long long)tw.b * kHeads + h) * hs + tw.line * 32;
-                    } else {
-                        drow = dst + ((long long)tw.b * kHeads + h) * N + t0;
-                    }
+                    const int sw = (tw.line >> 1) & 3;
+                    __nv_bfloat16* trow = tiles + l * layer_stride + ((long long)tw.b * kHeads + h) * hs + tw.line * 32;
                     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + q * 128;
 #pragma unroll 2
                     for (int k0 = 0; k0 < span; k0 += 16) {
@@ -286,7 +283,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                             v[e + 2] = fmaf(a.z, __uint_as_float(acc[e + 2]), fmaf(m.z, cc.x, cc.y));
                             v[e + 3] = fmaf(a.w, __uint_as_float(acc[e + 3]), fmaf(m.w, cc.x, cc.y));
                         }
-                        if (tiles != nullptr && l < layers) {
+                        if (l < layers) {
                             if (k0 + 16 > live) {   // keys past the end
 #pragma unroll
                                 for (int e = 0; e < 16; ++e)
@@ -303,16 +300,6 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
                             for (int e = 0; e < 8; ++e) w[e] = (sw & 1) ? o[e ^ 4] : o[e];
                             stg256_or_2x128(trow + (long long)((t0 + k0) >> 5) * N * 32 + ((c2 ^ (sw & 2)) << 3), w,
                                             aligned32(tiles));
-                        } else if (l < layers) {
-                            if (vec && k0 + 16 <= live) {
-#pragma unroll
-                                for (int e = 0; e < 16; e += 4)
-                                    *reinterpret_cast<float4*>(drow + k0 + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
-                            } else {
-#pragma unroll
-                                for (int e = 0; e < 16; ++e)
-                                    if (k0 + e < live) drow[k0 + e] = v[e];
-                            }
                         }
                         __syncwarp();
                     }
@@ -359,6 +346,7 @@ int launch(const __nv_bfloat16* z, const BiasLayer* layer, int layers, float* ds
     OF3_REQUIRE(((uintptr_t)tiles & 15) == 0, OF3_ERR_ALIGN, "pair_bias: bias tiles must be 16-byte aligned");
     OF3_REQUIRE(lines < (1LL << 31), OF3_ERR_SHAPE, "pair_bias: too many pair positions");
     OF3_REQUIRE(layers >= 1 && layers <= kMaxBiasLayers, OF3_ERR_ARG, "pair_bias: %d layers", layers);
+    OF3_REQUIRE(tiles != nullptr || layers == 1, OF3_ERR_ARG, "pair_bias: fp32 output of %d layers", layers);
     PbWeights wts = {};
     for (int l = 0; l < layers; ++l) {
         wts.ln_w[l] = layer[l].ln_w;
