@@ -66,3 +66,14 @@ def test_closed_adaptive_gates():
     assert not _run(layer, *x).any()
     layer.layer_norm_a.linear_g.bias.fill_(-3.0)
     assert _run(layer, *x).any()
+
+
+def test_closed_and_open_output_gates():
+    """The output projection's gate: one where open; closed, it leaves at most 1.6e-38 of the update."""
+    x, layer = _inputs(True), _layer(True)
+    layer.layer_norm_a.linear_g.bias.fill_(100.0)
+    half = _run(layer, *x)
+    layer.linear_ada_out.bias.fill_(100.0)
+    assert half.any() and torch.equal(_run(layer, *x), 2 * half)
+    layer.linear_ada_out.bias.fill_(-100.0)
+    assert (_run(layer, *x).double().abs() <= 4e-38 * half.double().abs()).all()
