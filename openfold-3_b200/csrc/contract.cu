@@ -93,7 +93,7 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             bool ok = true;
             rowtile::TileWalk tw(blockIdx.x, gridDim.x, num_mt, num_nt);
@@ -121,7 +121,7 @@ contract_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(kBM, BN);
             uint32_t it = 0, tcount = 0;
             bool ok = true;

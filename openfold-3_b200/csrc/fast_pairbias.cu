@@ -138,7 +138,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             TileWalk tw(blockIdx.x, gridDim.x, lines_per_sample, tiles_per_line);
             for (long long t = blockIdx.x; t < num_tiles; t += gridDim.x, ++it, tw.next()) {
@@ -156,7 +156,7 @@ pair_bias_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(128, kOne ? kHeads : 128);
             uint32_t it = 0, job = 0;
             bool ok = true;

@@ -205,7 +205,7 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
     grid_wait();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             const long long zh = (long long)z * H + h;
             mbar_arrive_expect_tx(q_full, lines * C::kQBytes);
             for (int L = 0; L < lines; ++L)
@@ -280,7 +280,7 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
             const uint64_t kdesc = kdesc_of(sb + C::kK + (ks * kLines + L) * C::kKBytes);
             const uint64_t tbdesc = smem_desc_k_sw64(sb + C::kTb + ks * C::kTbBytes);
             const uint32_t d = t_line + s * kBK;
-            if (lane == 0) {
+            if (elect_one()) {
 #pragma unroll
                 for (int kk = 0; kk < C::kKSteps; ++kk)
                     mma_bf16(d, qdesc + 2u * kk, kdesc + 2u * kk, idesc_s, kk ? 1u : 0u);
@@ -306,7 +306,7 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
             }
             tc_fence_after_sync();
             const uint64_t vdesc = smem_desc_k_sw64(sb + C::kV + (vs * kLines + L) * C::kVSlot);
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t a_p = t_line + (j & 1) * kBK;
                 mma_bf16_ts(t_line + C::kColO, a_p, vdesc, idesc_o, j != 0 ? 1u : 0u);
                 mma_bf16_ts(t_line + C::kColO, a_p + 8u, vdesc + 2u, idesc_o, 1u);

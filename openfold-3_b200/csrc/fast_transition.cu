@@ -161,7 +161,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 
     if (warp == 0) {
         // ---------------------------------------------------------------- weight producer
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             auto load_slab = [&](int wi) -> bool {
                 const int s = wi & 1, c = wi & (kNumChunks - 1);
@@ -194,7 +194,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
     } else if (warp <= 2) {
         // ---------------------------------------------------------------- MMA issuer of row group g
-        if (lane == 0) {
+        if (elect_one()) {
             const int g = warp - 1;
             constexpr uint32_t idesc = idesc_bf16_f32(128, 128);
             bool ok = true;
@@ -268,7 +268,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
     } else if (warp == 3) {
         // ---------------------------------------------------------------- results out
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t buf = 0;
             for (int t = 0; t < my_tiles; ++t) {
                 if (!mbar_wait(out_ready(t & 1), (uint32_t)(t >> 1) & 1u, abort_flag)) {
@@ -564,7 +564,7 @@ transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
     // TMEM: group g: D1 = [a 128 | b 128] at g * 256; D2 (64 columns) over the a half once D1 has been read
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(w_full, 49152);
             tma_load_2d(sbase + Sm::kWab, &tmWa, w_full, 0, 0);
             tma_load_2d(sbase + Sm::kWab + 16384, &tmWb, w_full, 0, 0);
@@ -582,7 +582,7 @@ transition64_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
             }
         }
     } else if (warp <= 2) {
-        if (lane == 0) {
+        if (elect_one()) {
             const int g = warp - 1;
             grid_wait();   // (the stores)
             bool ok = mbar_wait(w_full, 0, abort_flag);

@@ -149,7 +149,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
     // TMEM: slot 0 = [q|k] columns [0,2C), slot 1 = v columns [2C,3C) + triangle bias [3C,3C+16)
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(w_full, C / 64 * (Sm::kWKb + 2048));
             const CUtensorMap* wm[3] = {&tmWq, &tmWk, &tmWv};
             for (int w = 0; w < 3; ++w)
@@ -171,7 +171,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = mbar_wait(w_full, 0, abort_flag);
             if (!ok) report_wait_failure(status, abort_flag, kKidProj, 2);
             uint32_t it = 0;
@@ -875,7 +875,7 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
     if (warp >= 3) grid_wait();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(w_full, 2 * Sm::kWBytes);
             for (int kb = 0; kb < C / 64; ++kb) {
                 tma_load_2d(sbase + Sm::kWg + kb * C * 128, &tmWg, w_full, kb * 64, 0);
@@ -904,7 +904,7 @@ triattn_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constan
         }
     } else if (warp <= 2) {
         // ---------------------------------------------------------------- MMA issuer of row group g
-        if (lane == 0) {
+        if (elect_one()) {
             const int g = warp - 1;
             constexpr uint32_t idesc = idesc_bf16_f32(128, C);
             bool ok = mbar_wait(w_full, 0, abort_flag);

@@ -163,7 +163,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(w_full, C / 64 * Sm::kWKb);
             // slab order: C = 128: a_p, a_g, b_p, b_g; C = 64: a_p, b_p | a_g, b_g
             const CUtensorMap* wm[4] = {&tmWap, C == 128 ? &tmWag : &tmWbp, C == 128 ? &tmWbp : &tmWag, &tmWbg};
@@ -194,7 +194,7 @@ trimul_in_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(128, 128);
             bool ok = mbar_wait(w_full, 0, abort_flag);
             if (!ok) report_wait_failure(status, abort_flag, kKidIn, 2);
@@ -441,7 +441,7 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(w_full, 2 * InSmem<128>::kWKb);
             const CUtensorMap* wm[4] = {&tmWap, &tmWag, &tmWbp, &tmWbg};
             for (int w = 0; w < 4; ++w)
@@ -472,7 +472,7 @@ trimul_in_rows_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_cons
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(128, 256);
             bool ok = mbar_wait(w_full, 0, abort_flag);
             if (!ok) report_wait_failure(status, abort_flag, kKidIn, 2);
@@ -689,7 +689,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             mbar_arrive_expect_tx(w_full, 2 * Sm::kWBytes);
             for (int kb = 0; kb < C / 64; ++kb) {
                 tma_load_2d(sbase + Sm::kWg + kb * C * 128, &tmWg, w_full, kb * 64, 0);
@@ -721,7 +721,7 @@ trimul_out_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_constant
         }
     } else if (warp <= 2) {
         // ---------------------------------------------------------------- GEMMs and stores of row group g
-        if (lane == 0) {
+        if (elect_one()) {
             const int g = warp - 1;
             constexpr uint32_t idesc = idesc_bf16_f32(128, C);
             const uint32_t ztile = sbase + Sm::kZ + g * tile_bytes<C>();

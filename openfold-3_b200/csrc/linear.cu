@@ -191,7 +191,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             auto load_w = [&](const Tile& c, int kb, int s) {
                 const uint32_t sw = sbase + s * Cfg::kStageBytes + Cfg::kABytes;
                 if constexpr (EPI == kEpiSwiglu) {
@@ -236,7 +236,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = idesc_bf16_f32(kBM, BN);
             uint32_t it = 0, tc = 0;
             bool ok = true;

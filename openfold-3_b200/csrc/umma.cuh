@@ -80,6 +80,16 @@ __device__ __forceinline__ void report_wait_failure(int* status, volatile int* a
     }
 }
 
+// One lane of a converged warp, always the same. The instructions that one thread issues for the CTA (tcgen05.mma and commit,
+// TMA) take their operands from uniform registers; behind a test of the lane index the compiler has to allow for several
+// threads with operands of their own, and each such instruction costs 50 - 65 cycles of the issuing warp instead of 4 (commit)
+// to 40 (a 128 x 32 x 16 product, which is what it takes to execute).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p)::"memory");
+    return p != 0;
+}
+
 // ---------------------------------------------------------------- proxies / fences
 // Makes generic-proxy writes to shared memory visible to the async proxy (TMA, tcgen05.mma).
 __device__ __forceinline__ void fence_proxy_async_smem() {
