@@ -111,6 +111,10 @@ int single_track(void* s, const void* z, const void* bias, BiasForm form, const 
 // several of them: with few rows the projections of one block (6 matrices of c_a x c_s) fill a fraction of the chip and
 // cost a launch each; with many rows one block fills it, and its planes should stay in L2 until they are read.
 constexpr size_t kCondGroupBytes = 32u << 20;
+// Room for the normalised rows of the conditioning ahead of those projections: one launch for several groups of blocks, of
+// which each alone waits for the kernel ahead and for its own start (5 x 768 tokens: 24 launches of 5.1 us -> 5 of 13.8, 5 x 500:
+// 24 of 5.1 -> 3 of 20.2).
+constexpr size_t kCondRowsBytes = 32u << 20;
 // Room for the bias images of the blocks whose pair bias one pass over z projects (24 blocks up to N = 1150): 24 x 18.9 MB
 // of the workspace at N = 768, for 225 us instead of 24 passes of 56.
 constexpr size_t kBiasGroupBytes = 1u << 30;
@@ -165,9 +169,13 @@ int diffusion_stack(void* a, const void* s, const void* z, const void* mask, con
     if (group < 1) group = 1;
     if (group > blocks) group = blocks;
     if (group > fast::kMaxCondBatch / 2) group = fast::kMaxCondBatch / 2;
-    return ws.run([&](Arena& A) -> int {
+    int rows_group = (int)(kCondRowsBytes / ((size_t)rows * 2 * D.c_s * sizeof(bf16)));   // blocks per launch of the rows
+    if (rows_group > fast::kMaxCondBatch / 2) rows_group = fast::kMaxCondBatch / 2;
+    if (rows_group > blocks) rows_group = blocks;
+    rows_group = rows_group < group ? group : rows_group / group * group;
+    auto run = [&](Arena& A, int rows_group) -> int {
         bf16* planes = (bf16*)A.take(group * per_block);
-        bf16* sn = (bf16*)A.take((size_t)(2 * group + 1) * rows * D.c_s * sizeof(bf16));
+        bf16* sn = (bf16*)A.take((size_t)(2 * rows_group + 1) * rows * D.c_s * sizeof(bf16));
         bf16* tiles = nbias ? (bf16*)A.take(nbias * per_bias) : nullptr;
         const size_t mark = A.off;
         size_t need = A.off;
@@ -175,12 +183,16 @@ int diffusion_stack(void* a, const void* s, const void* z, const void* mask, con
             const int nb = blocks - b0 < group ? blocks - b0 : group;
             if (A.base) {
                 OF3_REQUIRE(A.ok(), OF3_ERR_WORKSPACE, "diffusion stack: workspace too small (%zu needed)", A.off);
-                fast::CondLayer layer[fast::kMaxCondBatch];
-                for (int i = 0; i < nb; ++i) {
-                    layer[2 * i] = fast::cond_layer(pa + b0 + i);
-                    layer[2 * i + 1] = fast::cond_layer(pt + b0 + i);
+                const int r0 = b0 / rows_group * rows_group, nr = blocks - r0 < rows_group ? blocks - r0 : rows_group;
+                fast::CondLayer layer[fast::kMaxCondBatch];   // of the blocks [r0, r0 + nr)
+                for (int i = 0; i < nr; ++i) {
+                    layer[2 * i] = fast::cond_layer(pa + r0 + i);
+                    layer[2 * i + 1] = fast::cond_layer(pt + r0 + i);
                 }
-                const int rc = fast::conditioning((const bf16*)s, layer, 2 * nb, rows, D.c_a, D.c_s, sn, planes, st);
+                int rc = b0 == r0 ? fast::conditioning_rows((const bf16*)s, layer, 2 * nr, rows, D.c_s, sn, st) : OF3_OK;
+                if (rc == OF3_OK)
+                    rc = fast::conditioning_planes(sn, 2 * (b0 - r0), 2 * nr, layer + 2 * (b0 - r0), 2 * nb, rows, D.c_a, D.c_s,
+                                                   planes, st);
                 if (rc) return rc;
             }
             for (int i = 0; i < nb; ++i) {
@@ -215,6 +227,12 @@ int diffusion_stack(void* a, const void* s, const void* z, const void* mask, con
         }
         A.off = need;
         return OF3_OK;
+    };
+    return ws.run([&](Arena& A) -> int {
+        if (!A.base) return run(A, rows_group);
+        Arena whole(nullptr, 0);   // a workspace without room for more takes the rows of one group at a time
+        const int rc = run(whole, rows_group);
+        return rc ? rc : run(A, whole.off <= A.cap ? rows_group : group);
     });
 }
 

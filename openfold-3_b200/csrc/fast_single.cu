@@ -252,30 +252,35 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
 
-int conditioning(const bf16* s, const CondLayer* layer, int layers, long long rows, int c_a, int c_s, bf16* sn,
-                 bf16* planes, cudaStream_t st) {
+int conditioning_rows(const bf16* s, const CondLayer* layer, int layers, long long rows, int c_s, bf16* sn,
+                      cudaStream_t st) {
     OF3_REQUIRE(layers >= 1 && layers <= kMaxCondLayers, OF3_ERR_ARG, "conditioning: %d layers", layers);
     CondWeights cw = {};
     for (int l = 0; l < layers; ++l) cw.w[l] = layer[l].ln_s_w;
-    {
-        // few rows: the layers are spread over blocks too
-        const unsigned gx = row_blocks(rows);
-        const unsigned want = 2u * (unsigned)sm_count();
-        unsigned gy = gx >= want ? 1u : want / gx + 1;
-        if (gy > (unsigned)layers) gy = layers;
-        LaunchScope scope(kKidSingle, st);
-        BY_WIDTH(c_s, OF3_CUDA_CHECK(launch_chained(cond_rows_kernel<NV>, dim3(gx, gy), 256, 0, st, s, cw, layers, sn, rows,
-                                                    c_s)));
-    }
+    // few rows: the layers are spread over blocks too
+    const unsigned gx = row_blocks(rows);
+    const unsigned want = 2u * (unsigned)sm_count();
+    unsigned gy = gx >= want ? 1u : want / gx + 1;
+    if (gy > (unsigned)layers) gy = layers;
+    LaunchScope scope(kKidSingle, st);
+    BY_WIDTH(c_s, OF3_CUDA_CHECK(launch_chained(cond_rows_kernel<NV>, dim3(gx, gy), 256, 0, st, s, cw, layers, sn, rows,
+                                                c_s)));
+    return OF3_OK;
+}
+
+int conditioning_planes(const bf16* sn, int first, int raw_slice, const CondLayer* layer, int layers, long long rows,
+                        int c_a, int c_s, bf16* planes, cudaStream_t st) {
+    const bf16* x0 = sn + first * rows * c_s;
+    const int raw_rel = raw_slice - first;
     const long long wsz = (long long)c_a * c_s, plane = rows * c_a;
     auto grouped = [&](int l) {   // the layer's own three matrices
         return layer[l].w_s == layer[l].w_g + wsz && layer[l].w_out == layer[l].w_g + 2 * wsz && aligned16(layer[l].w_g);
     };
     bool all = true;
     for (int l = 0; l < layers; ++l) all = all && grouped(l) && layer[l].w_g == layer[0].w_g + 3 * l * wsz;
-    if (all) return linear_conditioning(sn, rows, c_s, c_a, layer[0].w_g, layers, layers + 1, layers, planes, st);
+    if (all) return linear_conditioning(x0, rows, c_s, c_a, layer[0].w_g, layers, raw_rel + 1, raw_rel, planes, st);
     for (int l = 0; l < layers; ++l) {
-        const bf16 *x = sn + l * rows * c_s, *raw = sn + layers * rows * c_s;
+        const bf16 *x = x0 + l * rows * c_s, *raw = x0 + raw_rel * rows * c_s;
         bf16* y = planes + 3 * l * plane;
         int rc;
         if ((rc = linear_bf16(x, layer[l].w_g, y, rows, c_a, c_s, st))) return rc;
@@ -283,6 +288,12 @@ int conditioning(const bf16* s, const CondLayer* layer, int layers, long long ro
         if ((rc = linear_bf16(raw, layer[l].w_out, y + 2 * plane, rows, c_a, c_s, st))) return rc;
     }
     return OF3_OK;
+}
+
+int conditioning(const bf16* s, const CondLayer* layer, int layers, long long rows, int c_a, int c_s, bf16* sn,
+                 bf16* planes, cudaStream_t st) {
+    const int rc = conditioning_rows(s, layer, layers, rows, c_s, sn, st);
+    return rc ? rc : conditioning_planes(sn, 0, layers, layer, layers, rows, c_a, c_s, planes, st);
 }
 
 // bf16, one pair tensor per group of samples; c_a = H * d a multiple of 64; d in {24, 48}.

@@ -23,6 +23,12 @@ inline CondLayer cond_layer(const of3_cond_transition_params* p) {
 constexpr int kMaxCondBatch = 48;
 int conditioning(const __nv_bfloat16* s, const CondLayer* layer, int layers, long long rows, int c_a, int c_s,
                  __nv_bfloat16* sn, __nv_bfloat16* planes, cudaStream_t st);
+// The two launches apart: the normalised rows of `layers` layers (and s itself, slice `layers`) into sn; the planes of
+// `layers` of them, from slice `first` on, where s is slice `raw`.
+int conditioning_rows(const __nv_bfloat16* s, const CondLayer* layer, int layers, long long rows, int c_s, __nv_bfloat16* sn,
+                      cudaStream_t st);
+int conditioning_planes(const __nv_bfloat16* sn, int first, int raw, const CondLayer* layer, int layers, long long rows,
+                        int c_a, int c_s, __nv_bfloat16* planes, cudaStream_t st);
 
 // operand images of the attention kernel in the workspace
 struct SingleImages {
