@@ -72,6 +72,46 @@ __device__ __forceinline__ void store_images(const AttnImages& im, int kind, flo
     const int n = im.rows_per_sample;
     const int nkb = (n + kSingleBK - 1) / kSingleBK, n_qt = (n + kSingleBQ - 1) / kSingleBQ;
     const int pad = nkb * kSingleBK - n;   // keys past the end of the last block: zeros, written by the first rows
+    if constexpr (D % 16 == 0 && KD == 64) {
+        // 16 channels of one head: two neighbouring chunks of the row, which the swizzle keeps inside one 32-byte sector. Rows of
+        // different lanes are different lines, and the memory pipe takes a line at a time: two stores of 16 bytes cost twice
+        // one of 32 (5 x 768 tokens: 21.5 -> 19.2 us per launch).
+        if (kind != kOutV) {
+            const int h = col0 / D, c = (col0 - h * D) >> 3;
+            float f[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(r[e]);
+            if (kind == kOutQ) {
+                if (im.q_bias) {
+                    uint32_t b[8];
+                    ld_row16_any(im.q_bias + col0, b);
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) f[e] += (e & 1) ? bf16hi(b[e >> 1]) : bf16lo(b[e >> 1]);
+                }
+#pragma unroll
+                for (int e = 0; e < 16; ++e) f[e] *= qscale;
+            }
+            uint32_t o[8];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {   // odd rows: the chunks change places
+                const uint32_t lo = pack_bf16x2(f[2 * e], f[2 * e + 1]), hi = pack_bf16x2(f[8 + 2 * e], f[9 + 2 * e]);
+                o[e] = pos & 1 ? hi : lo;
+                o[4 + e] = pos & 1 ? lo : hi;
+            }
+            if (kind == kOutQ) {
+                uint8_t* t = reinterpret_cast<uint8_t*>(im.q) +
+                             ((bb * im.H + h) * n_qt + (pos >> 7)) * (long long)(kSingleBQ * KD * 2);
+                stg256(t + (single_chunk_off<KD>(pos & 127, c) & ~31u), o);
+            } else {
+                uint8_t* t0 = reinterpret_cast<uint8_t*>(im.k) + (bb * im.H + h) * nkb * (long long)(kSingleBK * KD * 2);
+                stg256(t0 + (pos >> 5) * (long long)(kSingleBK * KD * 2) + (single_chunk_off<KD>(pos & 31, c) & ~31u), o);
+                const uint32_t zero[8] = {};
+                for (int p = n + pos; p < n + pad; p += n)
+                    stg256(t0 + (p >> 5) * (long long)(kSingleBK * KD * 2) + (single_chunk_off<KD>(p & 31, c) & ~31u), zero);
+            }
+            return;
+        }
+    }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int col = col0 + half * 8;
@@ -295,8 +335,8 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                     if (ep.mask != nullptr) mk = __bfloat162float(ep.mask[row]);
 #pragma unroll
                     for (int p = 0; p < kPre; ++p) {
-                        if (ep.gate != nullptr) ld_row16(ep.gate + row * n + colb + p * 16, gv[p]);
-                        if (ep.residual != nullptr) ld_row16_any(ep.residual + row * n + colb + p * 16, zv[p]);
+                        if (ep.gate != nullptr) ld_row16_wide(ep.gate + row * n + colb + p * 16, gv[p]);
+                        if (ep.residual != nullptr) ld_row16_wide(ep.residual + row * n + colb + p * 16, zv[p]);
                     }
                 }
             }

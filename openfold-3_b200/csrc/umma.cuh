@@ -353,6 +353,12 @@ __device__ __forceinline__ void ld_row16_any(const __nv_bfloat16* p, uint32_t (&
     ld_row8_any(p, o);
     ld_row8_any(p + 8, o + 4);
 }
+// 32 bytes at a time where the row starts on a sector: rows of different lanes, which the memory pipe takes one by one, so that
+// two loads of 16 bytes take twice as long
+__device__ __forceinline__ void ld_row16_wide(const __nv_bfloat16* p, uint32_t (&o)[8]) {
+    if (aligned32(p)) ldg256(p, o);
+    else ld_row16_any(p, o);
+}
 __device__ __forceinline__ void st_row16_any(__nv_bfloat16* p, const uint32_t (&o)[8]) {
     if ((reinterpret_cast<uintptr_t>(p) & 31) == 0) {
         stg256(p, o);
