@@ -79,6 +79,10 @@ struct TrSmem {
 // of 250). N = 768: 316 -> 250 us, N = 37: 25.8 -> 20.9.
 constexpr int kTrThreads = 32 * 28;
 
+// kSolo: one tile per CTA (a tensor of no more tiles than SMs), whose chunks alternate between both groups' D1 and h buffers, so
+// that G1 runs two chunks ahead of the silu pass instead of one: N = 24 ... 111 18.7 -> 16.9 us per launch. An instantiation of
+// its own: with the choice made in the kernel N = 768 took 241 instead of 224 us (registers).
+template <bool kSolo>
 __global__ void __launch_bounds__(kTrThreads, 1)
 transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmOut,
                   const __grid_constant__ CUtensorMap tmWa, const __grid_constant__ CUtensorMap tmWb,
@@ -111,10 +115,9 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int my_tiles = (int)tiles_of_block((rows + kRows - 1) / kRows);
     // group g's tiles are the CTA's tiles g, g + 2, ...
-    // One tile only (a tensor of fewer tiles than SMs): both groups work on it, each on half of every chunk's columns and of
-    // the output's. The silu pass is the longest link of a lone tile's chain: 22.1 -> 21.8 us at N = 37, a pair block (20 in
-    // a graph) 95.0 -> 94.5, N = 24 93.9 -> 93.6, N = 136 148.3 -> 148.2; the runs of a side differ by 0.1.
-    const bool solo = my_tiles == 1;
+    // One tile only (also the last of an odd number): both groups work on it, each on half of every chunk's columns and of the
+    // output's. The silu pass is the longest link of a lone tile's chain.
+    const bool solo = kSolo || my_tiles == 1;
     const int num_chunks = ((my_tiles + 1) >> 1) * kNumChunks;
 
     if (threadIdx.x == 0) {
@@ -219,22 +222,27 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                 const int s = i & 1, c = i & (kNumChunks - 1);
                 if (c == 0 && !mbar_wait(a_ready(buf), use & 1u, abort_flag)) { fail(4); return false; }
                 if (!mbar_wait(w_full(s), (uint32_t)(i >> 1) & 1u, abort_flag)) { fail(3); return false; }
-                if (!mbar_wait(d1_empty(g), ((uint32_t)i & 1u) ^ 1u, abort_flag)) { fail(5); return false; }
+                const int d = kSolo ? i & 1 : g;
+                if (!mbar_wait(d1_empty(d), ((uint32_t)(kSolo ? i >> 1 : i) & 1u) ^ 1u, abort_flag)) { fail(5); return false; }
                 tc_fence_after_sync();
-                mma_k128(tmem_base + g * 256, sbase + TrSmem::kX + buf * kTileBytes,
+                mma_k128(tmem_base + d * 256, sbase + TrSmem::kX + buf * kTileBytes,
                          sbase + TrSmem::kW + s * TrSmem::kWStage, kKBlockBytes, idesc, false);
-                mma_commit(d1_full(g));
+                mma_commit(d1_full(d));
                 mma_commit(w_empty(s));
                 return true;
             };
             const int n = ((my_tiles + 1 - g) >> 1) * kNumChunks;
+            const int ahead = kSolo ? 2 : 1;
             if (ok && n > 0) ok = issue_g1(0);
+            if (ok && n > 0 && kSolo) ok = issue_g1(1);
             for (int i = 0; i < n && ok; ++i) {
                 const int s = i & 1, c = i & (kNumChunks - 1);
+                const int d = kSolo ? i & 1 : g;                        // D1 and h buffers of the chunk
+                const uint32_t dpar = (uint32_t)(kSolo ? i >> 1 : i) & 1u;
                 bool late = false;    // the next tile's LN(x) is not there yet: its first G1 does not hold up this tile's last G2
                 if (c == kNumChunks - 1) {
                     // the last G1 has read LN(x): fetch x once more (from L2) for the residual, under the silu pass
-                    if (!mbar_wait(d1_full(g), (uint32_t)i & 1u, abort_flag)) { fail(15); break; }
+                    if (!mbar_wait(d1_full(d), dpar, abort_flag)) { fail(15); break; }
                     if (add_residual) {
                         const uint32_t xtile = sbase + TrSmem::kX + buf * kTileBytes;
                         const int row0 = (int)((blockIdx.x + (long long)t * gridDim.x) * kRows);
@@ -249,20 +257,20 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     if (buf >= 3) { buf -= 3; ++use; }
                     late = i + 1 < n && !mbar_try_wait(a_ready(buf), use & 1u);
                 }
-                if (i + 1 < n && !late && !issue_g1(i + 1)) break;
+                if (i + ahead < n && !late && !issue_g1(i + ahead)) break;
                 if (c == 0 && !mbar_wait(d2_empty(g), ((uint32_t)(i / kNumChunks) & 1u) ^ 1u, abort_flag)) { fail(6); break; }
                 if (!mbar_wait(wo_full(s), (uint32_t)(i >> 1) & 1u, abort_flag)) { fail(13); break; }
-                if (!mbar_wait(h_ready(g), (uint32_t)i & 1u, abort_flag)) { fail(7); break; }
+                if (!mbar_wait(h_ready(d), dpar, abort_flag)) { fail(7); break; }
                 tc_fence_after_sync();
-                const uint64_t ad = smem_desc_k_sw128(sbase + TrSmem::kH + g * kKBlockBytes);
+                const uint64_t ad = smem_desc_k_sw128(sbase + TrSmem::kH + d * kKBlockBytes);
                 const uint64_t bd = smem_desc_k_sw128(sbase + TrSmem::kW + s * TrSmem::kWStage + 2 * kKBlockBytes);
 #pragma unroll
                 for (int k4 = 0; k4 < 4; ++k4)
                     mma_bf16(tmem_base + g * 256 + 128, ad + 2u * k4, bd + 2u * k4, idesc, (c != 0 || k4 != 0) ? 1u : 0u);
-                mma_commit(h_free(g));
+                mma_commit(h_free(d));
                 if (c == kNumChunks - 1) mma_commit(d2_full(g));
                 mma_commit(wo_empty(s));
-                if (late && !issue_g1(i + 1)) break;
+                if (late && !issue_g1(i + 1)) break;   // (several tiles: one chunk ahead)
             }
             for (int i = n; i < num_chunks && ok; ++i) skip_chunk(i);
         }
@@ -370,9 +378,8 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         const int quad = warp & 3;
         const int half = ((warp - 12) >> 2) & 1;
         const int row = quad * 32 + lane;
-        const uint32_t htile = sbase + TrSmem::kH + g * kKBlockBytes;
-        const uint32_t t_d1 = tmem_base + ((uint32_t)(quad * 32) << 16) + g * 256;
-        const uint32_t t_d2 = t_d1 + 128;
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
+        const uint32_t t_d2 = t_lane + g * 256 + 128;
         bool ok = true;
         uint32_t ppar = 0;
         int buf = g;
@@ -385,8 +392,11 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             if (mask != nullptr && grow < rows) m = __bfloat162float(mask[grow]);
 
             for (int c = 0; c < kNumChunks; ++c) {
-                const uint32_t cpar = (uint32_t)c & 1u;
-                if (!mbar_wait(d1_full(g), cpar, abort_flag)) {
+                const int d = kSolo ? c & 1 : g;
+                const uint32_t cpar = (uint32_t)(kSolo ? c >> 1 : c) & 1u;
+                const uint32_t htile = sbase + TrSmem::kH + d * kKBlockBytes;
+                const uint32_t t_d1 = t_lane + d * 256;
+                if (!mbar_wait(d1_full(d), cpar, abort_flag)) {
                     if (lane == 0) report_wait_failure(status, abort_flag, kKidTrans, 9);
                     ok = false;
                     break;
@@ -403,7 +413,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     if (q == 1 || solo) {   // D1 is in registers: the next chunk's G1 may run under the rest of this pass
                         tc_fence_before_sync();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(d1_empty(g));
+                        if (lane == 0) mbar_arrive(d1_empty(d));
                     }
 #pragma unroll
                     for (int e = 0; e < 16; e += 2) {
@@ -414,7 +424,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                     }
                 }
                 // the previous chunk's G2 must have consumed the H buffer before it is overwritten
-                if (!mbar_wait(h_free(g), cpar ^ 1u, abort_flag)) {
+                if (!mbar_wait(h_free(d), cpar ^ 1u, abort_flag)) {
                     if (lane == 0) report_wait_failure(status, abort_flag, kKidTrans, 10);
                     ok = false;
                     break;
@@ -427,7 +437,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(h_ready(g));
+                if (lane == 0) mbar_arrive(h_ready(d));
             }
             if (!ok) break;
             if (!mbar_wait(d2_full(g), ppar, abort_flag)) {
@@ -748,7 +758,9 @@ int transition(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bfloat16*
         if ((rc = make_tmap_bf16(&tmWo, p->w_out, 2, dimo, stro, boxo, true))) return rc;
     }
     if (!device_configured(4)) {
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(transition_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(transition_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            TrSmem::kDyn));
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(transition_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             TrSmem::kDyn));
         OF3_CUDA_CHECK(cudaFuncSetAttribute(transition64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             Tr64Smem::kDyn));
@@ -765,8 +777,8 @@ int transition(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bfloat16*
     typedef const __nv_bfloat16* P;
     const int residual = (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0;
     if (c == 128)
-        OF3_CUDA_CHECK(launch_chained(transition_kernel, dim3((unsigned)grid), kTrThreads, TrSmem::kDyn, st, tmX, tmOut, tmWa,
-                                      tmWb, tmWo, x, mask, (P)p->ln_w, (P)p->ln_b, rows, residual, device_status_ptr()));
+        OF3_CUDA_CHECK(launch_chained(tiles <= grid ? transition_kernel<true> : transition_kernel<false>, dim3((unsigned)grid),
+                                      kTrThreads, TrSmem::kDyn, st, tmX, tmOut, tmWa, tmWb, tmWo, x, mask, (P)p->ln_w, (P)p->ln_b, rows, residual, device_status_ptr()));
     else
         OF3_CUDA_CHECK(launch_chained(transition64_kernel, dim3((unsigned)grid), kTr64Threads, Tr64Smem::kDyn, st, tmX, tmOut,
                                       tmWa, tmWb, tmWo, mask, (P)p->ln_w, (P)p->ln_b, rows, residual, device_status_ptr()));
