@@ -153,14 +153,14 @@ __global__ void __launch_bounds__(256) cond_rows_kernel(const bf16* __restrict__
 }
 
 // an = sigmoid(g_lin + b_g) * LN(a) + s_lin (normalization.py:121-140)
-template <int NV>
-__global__ void __launch_bounds__(256) ada_rows_kernel(const bf16* __restrict__ a, const bf16* __restrict__ g_lin,
+template <int NV, int ROWS>
+__global__ void __launch_bounds__(32 * ROWS) ada_rows_kernel(const bf16* __restrict__ a, const bf16* __restrict__ g_lin,
                                                        const bf16* __restrict__ b_g, const bf16* __restrict__ s_lin,
                                                        bf16* __restrict__ an, long long rows, int C) {
     grid_trigger();
     grid_wait();
     const int lane = threadIdx.x & 31;
-    const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const long long r = (long long)blockIdx.x * ROWS + (threadIdx.x >> 5);
     if (r >= rows) return;
     uint32_t g[NV][4], s[NV][4], b[NV][4];   // in flight together with the row
 #pragma unroll
@@ -224,6 +224,7 @@ __global__ void __launch_bounds__(256) ada_rows_kernel(const bf16* __restrict__ 
     do {                                                    \
         if ((C) <= 256) { constexpr int NV = 1; CALL; }     \
         else if ((C) <= 512) { constexpr int NV = 2; CALL; } \
+        else if ((C) <= 768) { constexpr int NV = 3; CALL; } \
         else if ((C) <= 1024) { constexpr int NV = 4; CALL; } \
         else { constexpr int NV = 8; CALL; }                \
     } while (0)
@@ -238,8 +239,18 @@ int ln_rows(const bf16* x, const bf16* gamma, const bf16* beta, bf16* y, long lo
 }
 int ada_rows(const bf16* a, const bf16* planes, const bf16* b_g, bf16* an, long long rows, int C, cudaStream_t st) {
     LaunchScope scope(kKidSingle, st);
-    BY_WIDTH(C, OF3_CUDA_CHECK(launch_chained(ada_rows_kernel<NV>, row_blocks(rows), 256, 0, st, a, planes, b_g,
-                                              planes + rows * C, an, rows, C)));
+    auto launch = [&](auto* kernel, int per_block) {
+        return launch_chained(kernel, (unsigned)((rows + per_block - 1) / per_block), 32 * per_block, 0, st, a, planes, b_g,
+                              planes + rows * C, an, rows, C);
+    };
+    // Rows per block, by the step of 24 blocks (c_a = 768) with three vectors per lane and 2 / 4 / 8 rows, and with four and 8, us:
+    // 111 rows 923 / 939 / 942, 952; 900 rows 1510 / 1505 / 1528, 1492; 1200 rows 1670 / 1660 / 1700, 1657; 2500 rows 2294 /
+    // 2288 / 2317, 2363; 3840 rows 3075 / 3075 / 3100, 3135. Few rows: every row's chain on a scheduler of its own; many: blocks
+    // that fit side by side; in between, as long as there is an SM for every 8 rows, these leave the others to the next kernel.
+    const long long sms = sm_count();
+    if (rows <= 2 * sms) BY_WIDTH(C, OF3_CUDA_CHECK(launch(ada_rows_kernel<NV, 2>, 2)));
+    else if (rows > 4 * sms && rows <= 8 * sms && C > 512 && C <= 768) OF3_CUDA_CHECK(launch(ada_rows_kernel<4, 8>, 8));
+    else BY_WIDTH(C, OF3_CUDA_CHECK(launch(ada_rows_kernel<NV, 4>, 4)));
     return OF3_OK;
 }
 // y = x w^T on the contraction kernel
