@@ -778,7 +778,8 @@ int transition(const __nv_bfloat16* x, const __nv_bfloat16* mask, __nv_bfloat16*
     const int residual = (flags & OF3_FLAG_ADD_RESIDUAL) ? 1 : 0;
     if (c == 128)
         OF3_CUDA_CHECK(launch_chained(tiles <= grid ? transition_kernel<true> : transition_kernel<false>, dim3((unsigned)grid),
-                                      kTrThreads, TrSmem::kDyn, st, tmX, tmOut, tmWa, tmWb, tmWo, x, mask, (P)p->ln_w, (P)p->ln_b, rows, residual, device_status_ptr()));
+                                      kTrThreads, TrSmem::kDyn, st, tmX, tmOut, tmWa, tmWb, tmWo, x, mask, (P)p->ln_w,
+                                      (P)p->ln_b, rows, residual, device_status_ptr()));
     else
         OF3_CUDA_CHECK(launch_chained(transition64_kernel, dim3((unsigned)grid), kTr64Threads, Tr64Smem::kDyn, st, tmX, tmOut,
                                       tmWa, tmWb, tmWo, mask, (P)p->ln_w, (P)p->ln_b, rows, residual, device_status_ptr()));

@@ -514,7 +514,8 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
             // ------------------------------------------------------------ one MMA-issuing warp per line
             // The whole warp walks the loop and lane 0 issues: with warp-uniform control flow and operands (the
             // shuffles tell the compiler so) descriptors and addresses live in uniform registers, instead of being
-            // moved there one by one in front of every tcgen05.mma of a single-lane loop.
+            // moved there one by one in front of every tcgen05.mma of a single-lane loop. (With elect_one() in these loops,
+            // where an MMA costs the warp 40 instead of 50 - 65 cycles and a commit 4 instead of 46: N = 768 683 us against 670.)
             const int L = __shfl_sync(0xffffffffu, warp, 0) - 1;
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint32_t sb = __shfl_sync(0xffffffffu, sbase, 0);
