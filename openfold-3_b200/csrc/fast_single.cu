@@ -153,14 +153,16 @@ __global__ void __launch_bounds__(256) cond_rows_kernel(const bf16* __restrict__
 }
 
 // an = sigmoid(g_lin + b_g) * LN(a) + s_lin (normalization.py:121-140)
-template <int NV, int ROWS>
-__global__ void __launch_bounds__(32 * ROWS) ada_rows_kernel(const bf16* __restrict__ a, const bf16* __restrict__ g_lin,
-                                                       const bf16* __restrict__ b_g, const bf16* __restrict__ s_lin,
-                                                       bf16* __restrict__ an, long long rows, int C) {
+constexpr int kAdaRows = 4;   // per block
+template <int NV>
+__global__ void __launch_bounds__(32 * kAdaRows) ada_rows_kernel(const bf16* __restrict__ a, const bf16* __restrict__ g_lin,
+                                                                 const bf16* __restrict__ b_g,
+                                                                 const bf16* __restrict__ s_lin, bf16* __restrict__ an,
+                                                                 long long rows, int C) {
     grid_trigger();
     grid_wait();
     const int lane = threadIdx.x & 31;
-    const long long r = (long long)blockIdx.x * ROWS + (threadIdx.x >> 5);
+    const long long r = (long long)blockIdx.x * kAdaRows + (threadIdx.x >> 5);
     if (r >= rows) return;
     uint32_t g[NV][4], s[NV][4], b[NV][4];   // in flight together with the row
 #pragma unroll
@@ -237,21 +239,43 @@ int ln_rows(const bf16* x, const bf16* gamma, const bf16* beta, bf16* y, long lo
     BY_WIDTH(C, OF3_CUDA_CHECK(launch_chained(ln_rows_kernel<NV>, row_blocks(rows), 256, 0, st, x, gamma, beta, y, rows, C)));
     return OF3_OK;
 }
+// How many blocks of the AdaLN rows an SM may hold: as many as spread them evenly over the SMs, by a request for shared memory
+// that the kernel does not use. The blocks start while the kernel ahead drains, and without a limit they gather on the SMs that
+// it has left first, where each then waits for the others' loads; the next kernel, one block per SM, starts behind the fullest.
+// (Alone, unchained, the kernel takes the same time with and without.) Step of 24 blocks in a graph, c_a = 768, us, without a
+// limit / at most 1 / 2 / 3 / 4 blocks per SM, medians whose runs differ by up to 0.3 %:
+//   rows  111   867 /  911 /  866 /  860 /  873      rows 1184  1685 / 1720 / 1648 / 1655 / 1674
+//         150   938 /  915 /  927 /  940 /  928           1300  1764 / 1846 / 1772 / 1738 / 1752
+//         250   954 /  951 /  958 /  956 /  957           1500  1561 / 1657 / 1584 / 1533 / 1551
+//         450  1152 / 1054 / 1064 / 1154 / 1160           1775  1859 / 1981 / 1890 / 1851 / 1851
+//         592  1233 / 1223 / 1228 / 1239 / 1247           1900  1886 / 2061 / 1927 / 1916 / 1882
+//         700  1281 / 1311 / 1261 / 1283 / 1291           2200  1970 / 2156 / 2025 / 2020 / 1977
+//         900  1517 / 1528 / 1470 / 1480 / 1504           2750  2295 / 2580 / 2417 / 2370 / 2362
+// c_a = 384: 450 rows 820 / - / 819 / 824 / 838, 1000 1176 / - / 1138 / 1141 / 1154, 1500 1113 / - / 1127 / 1083 / 1090, 2000
+// 1307 / - / 1308 / 1304 / 1262, 3840 1954 / - / 2078 / 2016 / 1981. With fewer than two rows per SM a limit of one lost 5 % at
+// 111 rows and gained 2 % at 150: two. Past four blocks per SM they fill the chip anyway: no limit.
+int ada_blocks_per_sm(long long rows) {
+    const long long sms = sm_count(), per_sm = (rows + kAdaRows * sms - 1) / (kAdaRows * sms);
+    return rows < 2 * sms ? 2 : (per_sm <= 4 ? (int)per_sm : 0);
+}
+template <int NV>
+int ada_rows_width(const bf16* a, const bf16* planes, const bf16* b_g, bf16* an, long long rows, int C, cudaStream_t st) {
+    constexpr int kSmBytes = 228 << 10, kReserved = 1 << 10;   // shared memory of an SM; of it, the system's per block
+    const int limit = ada_blocks_per_sm(rows);
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(ada_rows_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            kSmBytes - kReserved));
+        configured.mark();
+    }
+    OF3_CUDA_CHECK(launch_chained(ada_rows_kernel<NV>, (unsigned)((rows + kAdaRows - 1) / kAdaRows), 32 * kAdaRows,
+                                  limit ? kSmBytes / limit - kReserved : 0, st, a, planes, b_g, planes + rows * C, an, rows,
+                                  C));
+    return OF3_OK;
+}
 int ada_rows(const bf16* a, const bf16* planes, const bf16* b_g, bf16* an, long long rows, int C, cudaStream_t st) {
     LaunchScope scope(kKidSingle, st);
-    auto launch = [&](auto* kernel, int per_block) {
-        return launch_chained(kernel, (unsigned)((rows + per_block - 1) / per_block), 32 * per_block, 0, st, a, planes, b_g,
-                              planes + rows * C, an, rows, C);
-    };
-    // Rows per block, by the step of 24 blocks (c_a = 768) with three vectors per lane and 2 / 4 / 8 rows, and with four and 8, us:
-    // 111 rows 923 / 939 / 942, 952; 900 rows 1510 / 1505 / 1528, 1492; 1200 rows 1670 / 1660 / 1700, 1657; 2500 rows 2294 /
-    // 2288 / 2317, 2363; 3840 rows 3075 / 3075 / 3100, 3135. Few rows: every row's chain on a scheduler of its own; many: blocks
-    // that fit side by side; in between, as long as there is an SM for every 8 rows, these leave the others to the next kernel.
-    const long long sms = sm_count();
-    if (rows <= 2 * sms) BY_WIDTH(C, OF3_CUDA_CHECK(launch(ada_rows_kernel<NV, 2>, 2)));
-    else if (rows > 4 * sms && rows <= 8 * sms && C > 512 && C <= 768) OF3_CUDA_CHECK(launch(ada_rows_kernel<4, 8>, 8));
-    else BY_WIDTH(C, OF3_CUDA_CHECK(launch(ada_rows_kernel<NV, 4>, 4)));
-    return OF3_OK;
+    BY_WIDTH(C, return ada_rows_width<NV>(a, planes, b_g, an, rows, C, st));
 }
 // y = x w^T on the contraction kernel
 int linear_bf16(const bf16* x, const bf16* w, bf16* y, long long rows, int out_dim, int in_dim, cudaStream_t st) {

@@ -1,7 +1,7 @@
-"""The diffusion token stack over the numbers of rows at which its launches change: rows per block of the adaptive LayerNorm
-(up to two and four rows per SM, up to eight, more), blocks whose conditioning rows share a launch (2000 rows: ten, then two),
-key counts that are no multiple of a key block. The stack against its blocks called one by one, bit for bit: there every block
-has launches of its own. And the lone-tile instantiation of the pair transition against the other one, bit for bit."""
+"""The diffusion token stack over the numbers of rows at which its launches change: blocks whose conditioning rows share a launch
+(2000 rows: ten, then two), key counts that are no multiple of a key block. The stack against its blocks called one by one, bit
+for bit: there every block has launches of its own. The adaptive LayerNorm's rows against the same rows in calls of a few. And
+the lone-tile instantiation of the pair transition against the other one, bit for bit."""
 
 import pytest
 import torch
@@ -35,6 +35,27 @@ def test_stack_equals_its_blocks(N, samples, blocks):
             want = blk(want, s, z, mask=m)
     pkg.lib.check_device_status()
     assert torch.isfinite(got).all() and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("rows", [5, 111, 296, 301, 593, 1185, 1777, 2370])
+def test_adaptive_rows_equal_those_of_short_calls(rows):
+    """One to four blocks per SM, no limit; every seventh row's gates below -44, where the sigmoid's division is taken."""
+    dev, bf = torch.device("cuda:0"), torch.bfloat16
+    g = torch.Generator().manual_seed(rows)
+    blk = _stack(1, g).blocks[0].conditioned_transition
+    blk.layer_norm.linear_g.weight.zero_()
+    blk.layer_norm.linear_g.weight[:, 0] = 20.0
+    blk.layer_norm.layer_norm_s.weight.fill_(1.0)
+    blk.layer_norm.linear_g.bias.zero_()
+    a, s = (torch.randn(1, rows, c, generator=g) for c in (768, 384))
+    s[..., 0] = 1.0
+    s[:, ::7, 0] = -3.0
+    a, s = a.to(dev, bf), s.to(dev, bf)
+    with torch.no_grad():
+        whole = blk(a, s, mask=None)
+        parts = [blk(a[:, i:i + 67].contiguous(), s[:, i:i + 67].contiguous(), mask=None) for i in range(0, rows, 67)]
+    pkg.lib.check_device_status()
+    assert torch.isfinite(whole).all() and whole.any() and torch.equal(whole, torch.cat(parts, 1))
 
 
 @pytest.mark.parametrize("rows", [1, 127, 128 * 147 + 1, 128 * 148])
