@@ -268,7 +268,9 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
  * (the form that of3_pair_bias_takes_tiles names: of3_pair_bias_project_tiles or of3_pair_bias_project), and z NULL.
  * With z the workspace holds the bias images of up to 24 blocks, as many as fit 1 GiB (0.45 GB at N = 768, Bz = 1).
  * The projections of s are computed for several blocks per launch when those of all layers lie back to back:
- * [block][attention, transition][gate, shift, output gate][c_a][c_s]. */
+ * [block][attention, transition][gate, shift, output gate][c_a][c_s]. The workspace holds the normalised rows of s that
+ * several such launches read (up to 32 MiB). One that falls short by no more than the rows of all but one launch's blocks
+ * is taken too, at a launch of rows per launch of projections; a shorter one is OF3_ERR_WORKSPACE. */
 typedef struct {
     int Ba, Bz, N, c_a, c_s, c_z, H, d, n;
     float inf;

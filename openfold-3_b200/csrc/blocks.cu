@@ -230,7 +230,9 @@ int diffusion_stack(void* a, const void* s, const void* z, const void* mask, con
     };
     return ws.run([&](Arena& A) -> int {
         if (!A.base) return run(A, rows_group);
-        Arena whole(nullptr, 0);   // a workspace without room for more takes the rows of one group at a time
+        // A workspace without room for more takes the rows of one group at a time: a caller's buffer may be of the size that was
+        // asked for before rows were shared. (The sizing of one block: under 1 us of a call's host time.)
+        Arena whole(nullptr, 0);
         const int rc = run(whole, rows_group);
         return rc ? rc : run(A, whole.off <= A.cap ? rows_group : group);
     });

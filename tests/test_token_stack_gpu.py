@@ -75,7 +75,8 @@ def test_a_transition_of_lone_tiles_equals_that_of_several(rows):
 
 
 def test_a_workspace_without_room_for_shared_launches_is_taken(monkeypatch):
-    """The conditioning rows of three blocks (group of one: 1 + 2 slices of 2000 x 384) in a workspace short of the other two's."""
+    """The conditioning rows of three blocks (group of one: 1 + 2 slices of 2000 x 384) in a workspace short of the other two's;
+    one that is shorter by 256 bytes (and the 256 of its alignment) more is refused."""
     N, samples, blocks = 400, 5, 3
     g = torch.Generator().manual_seed(1)
     st = _stack(blocks, g)
@@ -86,5 +87,8 @@ def test_a_workspace_without_room_for_shared_launches_is_taken(monkeypatch):
         want = st(a, s, z, mask=None)
         monkeypatch.setattr(pkg.lib, "workspace", lambda n, *k, **kw: real(n, *k, **kw)[: n - short])
         got = st(a, s, z, mask=None)
+        monkeypatch.setattr(pkg.lib, "workspace", lambda n, *k, **kw: real(n, *k, **kw)[: n - short - 512])
+        with pytest.raises(RuntimeError, match="workspace too small"):
+            st(a, s, z, mask=None)
     pkg.lib.check_device_status()
     assert torch.equal(got, want)
