@@ -1,7 +1,8 @@
-"""The diffusion token stack over the numbers of rows at which its launches change: blocks whose conditioning rows share a launch
-(2000 rows: ten, then two), key counts that are no multiple of a key block. The stack against its blocks called one by one, bit
-for bit: there every block has launches of its own. The adaptive LayerNorm's rows against the same rows in calls of a few. And
-the lone-tile instantiation of the pair transition against the other one, bit for bit."""
+"""The diffusion token stack over the numbers of rows at which its launches change: blocks whose conditioning rows, and fewer
+whose projections, share a launch (2000 rows: ten, then two, and one), key counts that are no multiple of a key block. The stack
+against its blocks called one by one, bit for bit: there every block has launches of its own. The adaptive LayerNorm's rows
+against the same rows in calls of a few. And the lone-tile instantiation of the pair transition against the other one, bit for
+bit."""
 
 import pytest
 import torch
@@ -20,8 +21,15 @@ def _stack(blocks, g):
     return st.to("cuda:0", torch.bfloat16).eval().requires_grad_(False)
 
 
-@pytest.mark.parametrize("N,samples,blocks", [(1, 1, 2), (31, 3, 2), (148, 2, 2), (99, 3, 2), (119, 5, 2), (237, 5, 2), (400, 5, 12)])
-def test_stack_equals_its_blocks(N, samples, blocks):
+# 700 rows: projections of 5 blocks per launch, rows of 20, then 4; 900: 4 and 24; 1400: 2 and 14, then 10
+@pytest.mark.parametrize("N,samples,blocks", [(1, 1, 2), (31, 3, 2), (148, 2, 2), (99, 3, 2), (119, 5, 2), (237, 5, 2), (400, 5, 12),
+                                              (350, 2, 24), (300, 3, 24), (280, 5, 24)])
+@pytest.mark.parametrize("packed", [True, False])
+def test_stack_equals_its_blocks(N, samples, blocks, packed, monkeypatch):
+    """``packed``: the stack's projections of s lie back to back, or each layer has launches of its own."""
+    if not packed:
+        for layer in (pkg.AttentionPairBias, pkg.ConditionedTransitionBlock):
+            monkeypatch.setattr(layer, "_cond_group", ())
     g = torch.Generator().manual_seed(N)
     st = _stack(blocks, g)
     a, s = (torch.randn(1, samples, N, c, generator=g).to("cuda:0", torch.bfloat16) for c in (768, 384))
