@@ -250,8 +250,8 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
         }
     } else if (warp <= kLines) {
         // ---------------------------------------------------------------- one MMA-issuing warp per line
-        // The whole warp walks the loop and lane 0 issues: with warp-uniform control flow and operands descriptors
-        // and addresses live in uniform registers.
+        // The whole warp walks the loop and an elected lane issues: with warp-uniform control flow and operands
+        // descriptors and addresses live in uniform registers.
         const int L = __shfl_sync(0xffffffffu, warp, 0) - 1;
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
         const uint32_t sb = __shfl_sync(0xffffffffu, sbase, 0);

@@ -80,8 +80,9 @@ struct TrSmem {
 constexpr int kTrThreads = 32 * 28;
 
 // kSolo: one tile per CTA (a tensor of no more tiles than SMs), whose chunks alternate between both groups' D1 and h buffers, so
-// that G1 runs two chunks ahead of the silu pass instead of one: N = 24 ... 111 18.7 -> 16.9 us per launch. An instantiation of
-// its own: with the choice made in the kernel N = 768 took 241 instead of 224 us (registers).
+// that G1 runs two chunks ahead of the silu pass instead of one: N = 24 / 37 / 64 / 111 / 137, unchained, 14.1 / 14.2 / 14.3 / 14.7 /
+// 15.0 -> 12.7 / 12.8 / 13.0 / 13.6 / 14.0 us (with 36 instead of 12 bytes of registers spilled). An instantiation of its own: with
+// the choice made in the kernel N = 768 took 241 instead of 224 us (registers).
 template <bool kSolo>
 __global__ void __launch_bounds__(kTrThreads, 1)
 transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmOut,
@@ -115,8 +116,9 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int my_tiles = (int)tiles_of_block((rows + kRows - 1) / kRows);
     // group g's tiles are the CTA's tiles g, g + 2, ...
-    // One tile only (also the last of an odd number): both groups work on it, each on half of every chunk's columns and of the
-    // output's. The silu pass is the longest link of a lone tile's chain.
+    // One tile only (kSolo, or a CTA with one where others have two): both groups work on it, each on half of every chunk's
+    // columns and of the output's. The silu pass is the longest link of a lone tile's chain. (The last of three tiles or more
+    // is its group's alone.)
     const bool solo = kSolo || my_tiles == 1;
     const int num_chunks = ((my_tiles + 1) >> 1) * kNumChunks;
 

@@ -5,10 +5,11 @@
 //   64), warp 1 MMA issuer (128 x BN x 16, accumulators double-buffered in TMEM), warps 2..17 the epilogue (four per 32
 //   rows, each a quarter of the columns; thread = row).
 //
-// What bounds them: a few hundred 128-row tiles with k = 384 .. 1536, two to four per CTA, whose epilogues are a third of their
-// time (3840 rows of 768: images 19.3 us, 14.2 with nothing computed or stored there) and, for short sequences, launch and fill
-// latency; the separate passes that read the products back (attention operand images, silu * mul, gates, residuals) cost as
-// much again as 11 launches per block.
+// What bounds them: a few hundred 128-row tiles with k = 384 .. 1536, and for short sequences launch and fill latency. At 3840
+// rows of 768 a CTA has two to four tiles of the images, gate / up and conditioning projections, of which the epilogues are a
+// quarter to a third (images 19.3 us, 14.2 with nothing computed or stored there; conditioning 16.0, 10.9 without stores), and
+// one of the output projections (120 tiles of 192 columns), whose epilogue nothing hides. The separate passes that would read
+// the products back (attention operand images, silu * mul, gates, residuals) cost as much again as 11 launches per block.
 // So the product leaves the SM in the form its consumer reads, and BN is chosen per call (pick_bn).
 #include "linear.cuh"
 #include "modules.cuh"
