@@ -8,9 +8,11 @@
 // What bounds them: a few hundred 128-row tiles with k = 384 .. 1536, and for short sequences launch and fill latency. At 3840
 // rows of 768 a CTA has two to four tiles of the images, gate / up and conditioning projections, of which the epilogues are a
 // quarter to a third (images 19.3 us, 14.2 with nothing computed or stored there; conditioning 16.0, 10.9 without stores), and
-// one of the output projections (120 tiles of 192 columns), whose epilogue nothing hides. The separate passes that would read
+// one of the output projections (120 tiles of 192 columns), whose panels arrive at 115 GB/s per SM (64 bytes per cycle). The separate passes that would read
 // the products back (attention operand images, silu * mul, gates, residuals) cost as much again as 11 launches per block.
 // So the product leaves the SM in the form its consumer reads, and BN is chosen per call (pick_bn).
+#include <type_traits>
+
 #include "linear.cuh"
 #include "modules.cuh"
 #include "rowtile.cuh"
@@ -30,20 +32,34 @@ constexpr int kEpiParts = 4;   // epilogue warps per 32 rows, each with its part
 constexpr int kThreads = 32 * (2 + 4 * kEpiParts);
 constexpr float kLog2e = 1.4426950408889634f;
 
-enum Epi { kEpiStore, kEpiImages, kEpiSwiglu, kEpiResidual };
+// kEpiStaged: kEpiResidual with the gate's, the residual's and the output's tile in shared memory, moved by TMA. Rows of the
+// caller's tensors that lie in different lanes cost the memory pipe a line at a time, behind the operand panels: at 3840 rows of
+// 768 the gates of a tile of 192 columns arrived 7.4 us after its start, when its product of k = 768 was done at 4.5 us. Staged,
+// gates and product are there after 5 and 6 us, and the tile ends at 8.3 instead of 11.9 us (k = 1536: 12.3 instead of 15.2).
+// Step of 24 blocks, c_a = 768: 5 x 1024 tokens 4334 -> 4225 us, 5 x 768 2995 -> 2924, 5 x 500 2249 -> 2214, 3 x 300 1403 ->
+// 1390, 111 923 both. With BN = 256 two stages of operands would be left: at most 192.
+enum Epi { kEpiStore, kEpiImages, kEpiSwiglu, kEpiResidual, kEpiStaged };
 
-template <int BN>
+template <int BN, int EPI>
 struct LinCfg {
     static constexpr int kABytes = kBM * kBK * 2;
     static constexpr int kStageBytes = kABytes + BN * kBK * 2;
-    static constexpr int kStages = BN == 256 ? 4 : (BN == 192 ? 5 : (BN == 128 ? 6 : 8));
+    static constexpr int kPlaneBytes = EPI == kEpiStaged ? kBM * BN * 2 : 0;   // a tile of the gate, and one of the residual / output
+    static constexpr int kStages = EPI == kEpiStaged ? (BN == 192 ? 3 : (BN == 128 ? 5 : 8))
+                                                     : (BN == 256 ? 4 : (BN == 192 ? 5 : (BN == 128 ? 6 : 8)));
     static constexpr int kAccStride = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);
     static constexpr int kTmemCols = 2 * kAccStride;
-    static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;
+    static constexpr int kPlanes = kStages * kStageBytes;            // offsets
+    static constexpr int kBars = kPlanes + 2 * kPlaneBytes;
+    static constexpr int kSmemBytes = kBars + 1024 + 256;
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory of a block");
 };
 
 struct LinMaps {
     CUtensorMap a, w[4];
+};
+struct StagedMaps : LinMaps {
+    CUtensorMap gate, residual, out;   // boxes of 64 columns and 128 rows
 };
 struct EpiArgs {
     // kEpiStore
@@ -173,21 +189,22 @@ __device__ __forceinline__ void store_images(const AttnImages& im, int kind, flo
 
 template <int BN, int EPI, int D>
 __global__ void __launch_bounds__(kThreads, 1)
-linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long rows, int K, int n, int num_mats,
-              int* status) {
-    using Cfg = LinCfg<BN>;
+linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, StagedMaps, LinMaps> maps, const EpiArgs ep,
+              long long rows, int K, int n, int num_mats, int* status) {
+    using Cfg = LinCfg<BN, EPI>;
     constexpr int S = Cfg::kStages;
     constexpr int kWRows = EPI == kEpiSwiglu ? BN / 2 : BN;   // rows of each weight matrix in a tile
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
-    const uint32_t bars = sbase + S * Cfg::kStageBytes;
+    const uint32_t bars = sbase + Cfg::kBars;
     auto full = [&](int s) { return bars + 8u * s; };
     auto empty = [&](int s) { return bars + 8u * (S + s); };
     auto tfull = [&](int a) { return bars + 8u * (2 * S + a); };
     auto tempty = [&](int a) { return bars + 8u * (2 * S + 2 + a); };
-    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + S * Cfg::kStageBytes + 8 * (2 * S + 4));
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + S * Cfg::kStageBytes + 8 * (2 * S + 4) + 8);
+    const uint32_t planes_full = bars + 8u * (2 * S + 4);
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + Cfg::kBars + 8 * (2 * S + 5));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + Cfg::kBars + 8 * (2 * S + 5) + 8);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int num_mt = (int)((rows + kBM - 1) / kBM);
@@ -216,6 +233,7 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
             mbar_init(tfull(a), 1);
             mbar_init(tempty(a), 4 * kEpiParts);
         }
+        mbar_init(planes_full, 1);
         *abort_flag = 0;
         mbar_fence_init();
         prefetch_tmap(&maps.a);
@@ -316,7 +334,25 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
         const int quad = warp & 3, part = (warp - 2) >> 2;
         constexpr int kCols = (EPI == kEpiSwiglu ? BN / 2 : BN) / kEpiParts;   // result columns per thread and tile
         grid_wait();
+        // kEpiStaged: a tile's gate and residual, by one thread, which also stores the tile ahead
+        [[maybe_unused]] auto load_planes = [&](int t) {
+            if constexpr (EPI == kEpiStaged) {
+                const Tile c = tile_of(t);
+                const bool gate = ep.gate != nullptr, residual = ep.residual != nullptr;
+                mbar_arrive_expect_tx(planes_full, (gate + residual) * Cfg::kPlaneBytes);
+                for (int b = 0; b < BN / 64; ++b) {
+                    if (gate) tma_load_2d(sbase + Cfg::kPlanes + b * (kBM * 128), &maps.gate, planes_full, c.nt * BN + b * 64, c.mt * kBM);
+                }
+                for (int b = 0; b < BN / 64; ++b) {
+                    if (residual)
+                        tma_load_2d(sbase + Cfg::kPlanes + Cfg::kPlaneBytes + b * (kBM * 128), &maps.residual, planes_full,
+                                    c.nt * BN + b * 64, c.mt * kBM);
+                }
+            }
+        };
+        if (EPI == kEpiStaged && threadIdx.x == 64) load_planes(blockIdx.x);
         uint32_t tc = 0;
+        bool ok = true;   // kEpiStaged: a warp whose wait ran out still takes part in the barriers of the tiles that are left
         for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tc) {
             const Tile c = tile_of(t);
             const uint32_t acc = tc & 1u;
@@ -328,11 +364,40 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
             constexpr int kPre = EPI == kEpiResidual ? kCols / 16 : 1;
             [[maybe_unused]] uint32_t gv[kPre][8], zv[kPre][8];
             [[maybe_unused]] float mk = 1.0f, bias0 = 0.f, bias1 = 0.f;   // gate biases of columns lane and 32 + lane
-            if constexpr (EPI == kEpiResidual) {
+            [[maybe_unused]] float sg[EPI == kEpiStaged ? kCols : 1];
+            // this thread's eight columns from `col` (of the tile) on in a plane
+            [[maybe_unused]] auto plane = [&](int which, int col) {
+                return reinterpret_cast<uint4*>(gbase + Cfg::kPlanes + which * Cfg::kPlaneBytes + (col >> 6) * (kBM * 128) +
+                                                sw128_offset(quad * 32 + lane, col & 63));
+            };
+            if constexpr (EPI == kEpiResidual || EPI == kEpiStaged) {
                 if (ep.gate != nullptr) {
                     if (lane < kCols) bias0 = __bfloat162float(ep.gate_bias[colb + lane]);
                     if (32 + lane < kCols) bias1 = __bfloat162float(ep.gate_bias[colb + 32 + lane]);
                 }
+            }
+            if constexpr (EPI == kEpiStaged) {
+                if (live && ep.mask != nullptr) mk = __bfloat162float(ep.mask[row]);
+                if (ok && !mbar_wait(planes_full, tc & 1u, abort_flag)) {
+                    if (lane == 0) report_wait_failure(status, abort_flag, kKid, 5);
+                    ok = false;
+                }
+                // the gates' sigmoids, under the product: two special-function results per value, 1.7 us of a tile of 192 columns
+                if (ep.gate != nullptr && ok) {
+#pragma unroll
+                    for (int e0 = 0; e0 < kCols; e0 += 8) {
+                        const uint4 g = *plane(0, part * kCols + e0);
+                        const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const float ge = e & 1 ? bf16hi(gw[e >> 1]) : bf16lo(gw[e >> 1]);
+                            sg[e0 + e] = sigmoid_of(ge + __shfl_sync(0xffffffffu, e0 < 32 ? bias0 : bias1, (e0 + e) & 31));
+                            asm volatile("" : "+f"(sg[e0 + e]));   // not behind the wait
+                        }
+                    }
+                }
+            }
+            if constexpr (EPI == kEpiResidual) {
                 if (live) {
                     if (ep.mask != nullptr) mk = __bfloat162float(ep.mask[row]);
 #pragma unroll
@@ -342,10 +407,11 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                     }
                 }
             }
-            if (!mbar_wait(tfull(acc), (tc >> 1) & 1u, abort_flag)) {
+            if (ok && !mbar_wait(tfull(acc), (tc >> 1) & 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKid, 4);
-                break;
+                ok = false;
             }
+            if (EPI != kEpiStaged && !ok) break;
             tc_fence_after_sync();
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * Cfg::kAccStride + part * kCols;
             [[maybe_unused]] int bb = 0, pos = 0;   // sample and position of the row
@@ -353,16 +419,36 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
                 bb = (int)((uint32_t)row / (uint32_t)ep.im.rows_per_sample);
                 pos = (int)row - bb * ep.im.rows_per_sample;
             }
-#pragma unroll(EPI == kEpiResidual ? kPre : 1)
+#pragma unroll(EPI == kEpiResidual ? kPre : (EPI == kEpiStaged ? kCols / 16 : 1))
             for (int c0 = 0; c0 < kCols; c0 += 16) {
+                if (EPI == kEpiStaged && !ok) break;
                 uint32_t r[16], r2[16];
                 tmem_ld16(taddr + c0, r);
                 if constexpr (EPI == kEpiSwiglu) tmem_ld16(taddr + BN / 2 + c0, r2);
                 tmem_ld_wait();
                 const int col = colb + c0;
-                if (EPI != kEpiResidual && !live) continue;   // (its gate biases are shared by shuffles)
+                if (EPI != kEpiResidual && EPI != kEpiStaged && !live) continue;   // (its gate biases are shared by shuffles)
                 if constexpr (EPI == kEpiImages) {
                     store_images<D>(ep.im, ep.kind[c.g], ep.qscale, r, col, row, bb, pos);
+                } else if constexpr (EPI == kEpiStaged) {
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint4* p = plane(1, part * kCols + c0 + h * 8);
+                        float v[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            v[e] = __fmul_rn(mk, __uint_as_float(r[h * 8 + e]));
+                            if (ep.gate != nullptr) v[e] = __fmul_rn(v[e], sg[c0 + h * 8 + e]);   // not one fma with the residual
+                        }
+                        if (ep.residual != nullptr) {
+                            const uint4 z = *p;
+                            const uint32_t zw[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) v[e] += e & 1 ? bf16hi(zw[e >> 1]) : bf16lo(zw[e >> 1]);
+                        }
+                        *p = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                                        pack_bf16x2(v[6], v[7]));
+                    }
                 } else {
                     uint32_t o[8];
                     if constexpr (EPI == kEpiStore) {
@@ -409,7 +495,21 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty(acc));
+            if constexpr (EPI == kEpiStaged) {
+                fence_proxy_async_smem();
+                rowtile::group_sync(1, 128 * kEpiParts);
+                if (threadIdx.x == 64 && ok) {
+                    for (int b = 0; b < BN / 64; ++b)
+                        tma_store_2d(&maps.out, sbase + Cfg::kPlanes + Cfg::kPlaneBytes + b * (kBM * 128), c.nt * BN + b * 64, c.mt * kBM);
+                    tma_store_commit();
+                    if (t + (int)gridDim.x < num_tiles) {
+                        tma_store_wait_read<0>();
+                        load_planes(t + gridDim.x);
+                    }
+                }
+            }
         }
+        if (EPI == kEpiStaged && threadIdx.x == 64) tma_store_wait_all<0>();
     }
 
     tc_fence_before_sync();
@@ -423,14 +523,14 @@ linear_kernel(const __grid_constant__ LinMaps maps, const EpiArgs ep, long long 
 // Column tile: the number of waves of 148 CTAs times the panels a tile streams (128 rows of x and BN of the weights per
 // k-block, plus a constant for its fill and epilogue). Wide tiles move fewer bytes, narrow ones fill the chip when there
 // are few rows; a BN that does not divide the matrix is out.
-int pick_bn(long long rows, int n, int mats, bool swiglu) {
+int pick_bn(long long rows, int n, int mats, bool swiglu, int widest = 256) {
     const long long sms = sm_count(), mt = (rows + kBM - 1) / kBM;
     const int cand[4] = {256, 192, 128, 64};
     int best = 0;
     long long best_cost = 0;
     for (int bn : cand) {
         const int wr = swiglu ? bn / 2 : bn;
-        if (n % wr != 0 || (swiglu && (bn == 64 || bn == 192))) continue;
+        if (bn > widest || n % wr != 0 || (swiglu && (bn == 64 || bn == 192))) continue;
         const long long tiles = mt * (n / wr) * (swiglu ? 1 : mats);
         const long long cost = (tiles + sms - 1) / sms * (128 + bn + 64);
         if (best == 0 || cost < best_cost) {
@@ -443,9 +543,9 @@ int pick_bn(long long rows, int n, int mats, bool swiglu) {
 
 template <int BN, int EPI, int D>
 int launch(const LinearIn& in, const EpiArgs& ep, int slices, int w_rows, cudaStream_t st) {
-    using Cfg = LinCfg<BN>;
+    using Cfg = LinCfg<BN, EPI>;
     constexpr int kWRows = EPI == kEpiSwiglu ? BN / 2 : BN;
-    LinMaps maps;
+    std::conditional_t<EPI == kEpiStaged, StagedMaps, LinMaps> maps;
     int rc;
     {
         uint64_t dims[3] = {(uint64_t)in.k, (uint64_t)in.rows, (uint64_t)slices};
@@ -461,6 +561,15 @@ int launch(const LinearIn& in, const EpiArgs& ep, int slices, int w_rows, cudaSt
         if ((rc = make_tmap_bf16(&maps.w[i], in.w[i], 2, dims, str, box, 1))) return rc;
     }
     for (int i = tensors; i < 4; ++i) maps.w[i] = maps.w[0];
+    if constexpr (EPI == kEpiStaged) {
+        const uint64_t dims[2] = {(uint64_t)in.n, (uint64_t)in.rows};
+        const uint64_t str[1] = {(uint64_t)in.n * 2};
+        const uint32_t box[2] = {64, kBM};
+        if ((rc = make_tmap_bf16(&maps.out, ep.out, 2, dims, str, box, 1))) return rc;
+        maps.gate = maps.residual = maps.out;
+        if (ep.gate && (rc = make_tmap_bf16(&maps.gate, ep.gate, 2, dims, str, box, 1))) return rc;
+        if (ep.residual && (rc = make_tmap_bf16(&maps.residual, ep.residual, 2, dims, str, box, 1))) return rc;
+    }
     static PerDeviceOnce configured;
     if (!configured.done()) {
         OF3_CUDA_CHECK(cudaFuncSetAttribute(linear_kernel<BN, EPI, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -480,8 +589,9 @@ template <int EPI, int D>
 int dispatch(const LinearIn& in, const EpiArgs& ep, int slices, int w_rows, cudaStream_t st) {
     OF3_REQUIRE(in.k % kBK == 0 && in.n % 64 == 0, OF3_ERR_SHAPE, "linear: widths %d x %d are not multiples of 64", in.n,
                 in.k);
-    switch (pick_bn(in.rows, in.n, in.num_w, EPI == kEpiSwiglu)) {
-        case 256: return launch<256, EPI, D>(in, ep, slices, w_rows, st);
+    switch (pick_bn(in.rows, in.n, in.num_w, EPI == kEpiSwiglu, EPI == kEpiResidual || EPI == kEpiStaged ? 192 : 256)) {
+        case 256:
+            if constexpr (EPI != kEpiResidual && EPI != kEpiStaged) return launch<256, EPI, D>(in, ep, slices, w_rows, st);
         case 192:
             if constexpr (EPI != kEpiSwiglu) return launch<192, EPI, D>(in, ep, slices, w_rows, st);
         case 128: return launch<128, EPI, D>(in, ep, slices, w_rows, st);
@@ -524,7 +634,8 @@ int linear_residual(const LinearIn& in, const bf16* residual, const bf16* gate, 
     ep.gate = gate;
     ep.gate_bias = gate_bias;
     ep.mask = mask;
-    return dispatch<kEpiResidual, 0>(in, ep, 1, in.n, st);
+    const bool tma = (((uintptr_t)residual | (uintptr_t)gate | (uintptr_t)out) & 15) == 0;
+    return tma ? dispatch<kEpiStaged, 0>(in, ep, 1, in.n, st) : dispatch<kEpiResidual, 0>(in, ep, 1, in.n, st);
 }
 
 }  // namespace fast
