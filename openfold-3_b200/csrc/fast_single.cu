@@ -284,6 +284,7 @@ int linear_bf16(const bf16* x, const bf16* w, bf16* y, long long rows, int out_d
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+bool even(const void* p) { return ((uintptr_t)p & 3) == 0; }   // pairs of channels
 
 }  // namespace
 
@@ -370,8 +371,9 @@ int attn_pair_bias(const bf16* a, const bf16* z, const bf16* s, const bf16* mask
         const LinearIn in{an, rows, c_a, c_a,
                           {(const bf16*)p->w_q, (const bf16*)p->w_g, (const bf16*)p->w_k, (const bf16*)p->w_v}, 4};
         const LinearOut kinds[4] = {kOutQ, kOutG, kOutK, kOutV};
-        if ((rc = linear_attn_images(in, kinds, AttnImages{im.q, im.k, im.v, g, (const bf16*)p->b_q, N, H, d}, st)))
-            return rc;
+        const AttnImages images{im.q, im.k, im.v, g, (const bf16*)p->b_q, N, H, d};
+        const bool few = token_images_supported(Ba, N, c_a, d);
+        if ((rc = (few ? token_attn_images : linear_attn_images)(in, kinds, images, st))) return rc;
     }
     SingleBias bias;
     bias.tiles = bias_tiles;
@@ -382,8 +384,10 @@ int attn_pair_bias(const bf16* a, const bf16* z, const bf16* s, const bf16* mask
     bias.w = (const bf16*)p->w_z;
     if ((rc = single_attn(im, g, bias, tb, mask, og, Ba, N, N, H, d, inf, Ba / Bz, st))) return rc;
     const LinearIn in{og, rows, c_a, c_a, {(const bf16*)p->w_o}, 1};
-    return linear_residual(in, (flags & OF3_FLAG_ADD_RESIDUAL) ? a : nullptr, ada ? cond + 2 * rows * c_a : nullptr,
-                           (const bf16*)p->b_ada_out, nullptr, out, st);
+    const bool few = token_residual_supported(rows, c_a) && even(a) && even(out);
+    return (few ? token_residual : linear_residual)(in, (flags & OF3_FLAG_ADD_RESIDUAL) ? a : nullptr,
+                                                    ada ? cond + 2 * rows * c_a : nullptr, (const bf16*)p->b_ada_out, nullptr, out,
+                                                    st);
 }
 
 // ConditionedTransitionBlock (transition.py:325-339): AdaLN -> SwiGLU -> linear_out, gated by sigmoid(linear_g(s)).
@@ -408,9 +412,10 @@ int cond_transition(const bf16* a, const bf16* s, const bf16* mask, bf16* out, l
     }
     if ((rc = ada_rows(a, cond, (const bf16*)p->ada_b_g, an, rows, c_a, st))) return rc;
     const LinearIn up{an, rows, c_a, hid, {(const bf16*)p->w_a, (const bf16*)p->w_b}, 2};
-    if ((rc = linear_swiglu(up, h, st))) return rc;
+    if ((rc = (token_swiglu_supported(rows, hid) ? token_swiglu : linear_swiglu)(up, h, st))) return rc;
     const LinearIn down{h, rows, hid, c_a, {(const bf16*)p->w_out}, 1};
-    return linear_residual(down, (flags & OF3_FLAG_ADD_RESIDUAL) ? a : nullptr, cond + 2 * rows * c_a,
+    const bool few = token_residual_supported(rows, c_a) && even(a) && even(out);
+    return (few ? token_residual : linear_residual)(down, (flags & OF3_FLAG_ADD_RESIDUAL) ? a : nullptr, cond + 2 * rows * c_a,
                            (const bf16*)p->b_g, mask, out, st);
 }
 

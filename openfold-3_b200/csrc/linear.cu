@@ -8,8 +8,9 @@
 // What bounds them: a few hundred 128-row tiles with k = 384 .. 1536, and for short sequences launch and fill latency. At 3840
 // rows of 768 a CTA has two to four tiles of the images, gate / up and conditioning projections, of which the epilogues are a
 // quarter to a third (images 19.3 us, 14.2 with nothing computed or stored there; conditioning 16.0, 10.9 without stores), and
-// one of the output projections (120 tiles of 192 columns), whose panels arrive at 115 GB/s per SM (64 bytes per cycle). The separate passes that would read
-// the products back (attention operand images, silu * mul, gates, residuals) cost as much again as 11 launches per block.
+// one of the output projections (120 tiles of 192 columns), whose panels arrive at 115 GB/s per SM (64 bytes per cycle). The
+// separate passes that would read the products back (attention operand images, silu * mul, gates, residuals) cost as much again
+// as 11 launches per block.
 // So the product leaves the SM in the form its consumer reads, and BN is chosen per call (pick_bn).
 #include <type_traits>
 

@@ -41,5 +41,15 @@ int linear_swiglu(const LinearIn& in, __nv_bfloat16* h, cudaStream_t st);
 int linear_residual(const LinearIn& in, const __nv_bfloat16* residual, const __nv_bfloat16* gate,
                     const __nv_bfloat16* gate_bias, const __nv_bfloat16* mask, __nv_bfloat16* out, cudaStream_t st);
 
+// The same where a call has few tokens (token_linear.cu): tiles of 64 or 128 output channels by 16 to 64 tokens. residual and out
+// start on 4 bytes.
+bool token_images_supported(int samples, int tokens, int c, int d);
+bool token_swiglu_supported(long long rows, int hidden);
+bool token_residual_supported(long long rows, int c);
+int token_attn_images(const LinearIn& in, const LinearOut* kinds, const AttnImages& im, cudaStream_t st);
+int token_swiglu(const LinearIn& in, __nv_bfloat16* h, cudaStream_t st);
+int token_residual(const LinearIn& in, const __nv_bfloat16* residual, const __nv_bfloat16* gate,
+                   const __nv_bfloat16* gate_bias, const __nv_bfloat16* mask, __nv_bfloat16* out, cudaStream_t st);
+
 }  // namespace fast
 }  // namespace of3

@@ -1,6 +1,9 @@
-"""The output projections of the single track, whose gate, residual and result pass through shared memory where the caller's
-tensors start on 16 bytes, against the same call on tensors that do not (every thread then reads and writes rows of its own): the
-same products, gates and sums in the same order, so the same bits. Rows: part of a tile, its edges, several tiles per block."""
+"""The linear layers of the single track and of the diffusion token stack in their several forms, bit for bit.
+
+The output projections, whose gate, residual and result pass through shared memory where the caller's tensors start on 16 bytes,
+against the same call on tensors that do not (every thread then reads and writes rows of its own): the same products, gates and
+sums in the same order. Rows: part of a tile, its edges, several tiles per block. The launches for few tokens against those of
+128-row tiles."""
 
 import pytest
 import torch
@@ -48,3 +51,37 @@ def test_staged_rows_equal_direct_ones(rows, c, gated, residual):
     pkg.lib.check_device_status()
     assert torch.isfinite(outs[0]).all() and outs[0].any()
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+def _diffusion_block(g):
+    blk = pkg.DiffusionTransformerBlock(c_a=768, c_s=384, c_z=128, c_hidden=48, no_heads=16, n_transition=2,
+                                        use_ada_layer_norm=True, n_query=None, n_key=None, inf=1e9)
+    with torch.no_grad():
+        for p in blk.parameters():
+            p.copy_(torch.randn(p.shape, generator=g) * (0.03 if p.dim() > 1 else 0.3) + (1.0 if p.dim() == 1 else 0.0))
+    return blk.to("cuda:0", torch.bfloat16).eval().requires_grad_(False)
+
+
+# Tiles of 16, 32 and 64 tokens, one and several of them, per sample and over the rows of all samples; key blocks that end inside,
+# at and before a tile's end; 370: the last sizes that one wave of 64-token tiles takes (three launches, then two, then one)
+@pytest.mark.parametrize("N,samples", [(1, 1), (1, 3), (15, 1), (16, 1), (17, 2), (31, 1), (32, 1), (33, 3), (48, 1), (64, 1), (65, 1),
+                                       (75, 5), (96, 1), (111, 1), (129, 1), (185, 2), (192, 1), (193, 1), (370, 1), (384, 1),
+                                       (385, 1), (768, 1), (769, 1)])
+def test_few_tokens_equal_rows_of_a_larger_call(N, samples):
+    """The launches for few tokens against the 128-row ones, which the same samples take in a call of many: the same products in the
+    same order, so the same bits."""
+    g = torch.Generator().manual_seed(N)
+    blk = _diffusion_block(g)
+    many = max(samples + 1, -(-800 // N))
+    many += many % 2
+    if N < 32:
+        many = 60   # more samples than one wave of tiles
+    a, s = (torch.randn(1, many, N, c, generator=g).to("cuda:0", torch.bfloat16) for c in (768, 384))
+    z = torch.randn(1, 1, N, N, 128, generator=g).to("cuda:0", torch.bfloat16)
+    m = (torch.rand(1, 1, N, generator=g) < 0.9).to("cuda:0", torch.bfloat16)
+    m[..., 0] = 1
+    with torch.no_grad():
+        want = blk(a, s, z, mask=m)[:, :samples]
+        got = blk(a[:, :samples].contiguous(), s[:, :samples].contiguous(), z, mask=m)
+    pkg.lib.check_device_status()
+    assert torch.isfinite(got).all() and got.any() and torch.equal(got, want)
