@@ -9,7 +9,7 @@
  *    > 0 a cudaError_t. of3_last_error_string() describes the last failure of the calling
  *    thread. Nothing throws or aborts.
  *  - dtype: OF3_DTYPE_BF16 (bf16 storage, fp32 accumulation and statistics) or
- *    OF3_DTYPE_F32 (fp32 storage and true fp32 arithmetic: the validation mode). Activations,
+ *    OF3_DTYPE_F32 (fp32 storage and fp32 arithmetic: the validation mode). Activations,
  *    masks and parameters of one call share the dtype.
  *  - Every buffer is owned by the caller. Entry points enqueue work on `stream` and return;
  *    they allocate nothing (except a 64-byte per-device status block on first use) and keep

@@ -1,11 +1,11 @@
-// fp32 GEMMs of the shape-generic family on the FMA pipe, with the element-wise step that follows in the epilogue.
+// fp32 GEMMs of the shape-generic family, with the element-wise step that follows in the epilogue.
 //
-// Bound: 128 fp32 FMA per SM and clock (75 TFLOP/s); the operands of these layers sit in L2. Tiles of 128 x 64 with 8 x 8
-// products per thread read 16 values from shared memory per 64 FMA (packed fma.f32x2: half the issue slots), the next
-// k-slab is in registers while this one is multiplied. Layers with few rows take 32 x 32 tiles whose k-slab is split over
-// four groups of threads (the chain over k = 1536 on 24 large tiles is what such a layer waits for).
-// The 64 x 64 kernel with 4 x 4 products, scalar shared-memory reads and separate element-wise kernels ran the 128-token
-// trunk block at 8.5 TFLOP/s.
+// Large layers of fp32 operands run on the tensor cores as products of three bf16 parts (gemm_split_kernel): below the FMA pipe's
+// error, and past its 75 TFLOP/s. Few rows, and bf16 weights, stay on the FMA pipe: tiles of 128 x 64 with 8 x 8 products per
+// thread (packed fma.f32x2; the next k-slab is in registers while this one is multiplied), and where there are few of these, or
+// the operands are fp32, 32 x 32 tiles whose k-slab is split over four groups of threads (the chain over k = 1536 on 24 large tiles
+// is what such a layer waits for). Fp32 trunk block, FMA pipe alone / now, us: N = 48 429 / 369, 64 520 / 434, 128 955 / 695, 250
+// 3310 / 2246.
 #include "generic_ops.cuh"
 #include "runtime.cuh"
 #include "umma.cuh"
@@ -49,17 +49,9 @@ __device__ __forceinline__ bool vec_ok(const T* p, long long ld) {
     return (reinterpret_cast<uintptr_t>(p) & (4 * sizeof(T) - 1)) == 0 && (ld & 3) == 0;
 }
 
-__device__ __forceinline__ void store4(float* p, const float (&o)[4]) {
-    *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
-}
 __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&o)[4]) {
     *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
 }
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool exists) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(umma::smem_u32(dst)), "l"(src), "r"(exists ? 16 : 0)
-                 : "memory");
-}
-
 enum Epi { kStore, kGatedPlanes, kSwiglu, kFinal };
 
 template <typename T>
@@ -374,110 +366,534 @@ __global__ void __launch_bounds__(G* BM / TM * BN / TN) gemm_kernel(const Args<T
     epilogue<BM, BN, TM, TN, EPI, T>(p, v, m0, n0, grp, boff, tx, ty);
 }
 
-// The same product for fp32 operands in whole 16-byte vectors along k: slabs by cp.async as they lie, a thread's 8 x 8
-// products in pairs (even k, odd k), whose halves are added at the end: operands come from shared memory as the pairs that
-// fma.f32x2 takes, none is duplicated in registers. A row of a slab lies at the place that lets the lanes of a load, which
-// own rows 4 apart, hit neighbouring ones: pitch 20 floats, no bank conflict. Two blocks per SM, since a thread holds 128
-// sums: for the plain and the final epilogue the better kernel (one fp32 trunk block at N = 128: 1011 -> 978 us), for the
-// paired ones, whose exponentials three blocks of the kernel above overlap with products, the worse (swiglu 107 -> 119 us).
-// Both read 16 values per 64 products from shared memory, whose bandwidth (16 bytes x 32 lanes in four clocks) that takes
-// whole; 16 x 8 products per thread leave two blocks per SM and are slower (122 us).
-template <int EPI>
-__global__ void __launch_bounds__(128, 2) gemm_pairs_kernel(const Args<float> p) {
-    constexpr int BM = 128, BN = 64, TM = 8, TN = 8, BK = 16, kStages = 4, kPitch = BK + 4;
-    static_assert(EPI == kStore || EPI == kFinal, "one weight per group");
-    extern __shared__ __align__(16) float slabs[];   // stages x (BM + BN) rows
-    umma::grid_trigger();
-    umma::grid_wait();
-    const int K = p.K, n = p.n;
-    const long long M = p.M, m0 = (long long)blockIdx.x * BM;
-    const int tiles_n = (n + BN - 1) / BN;
-    const int grp = blockIdx.y / tiles_n;
-    const int n0 = (blockIdx.y % tiles_n) * BN;
-    const long long boff = (long long)blockIdx.z * p.a_batch;
-    const float* a = p.a + boff;
-    const float* w = p.w[grp] + boff;
+// ---------------------------------------------------------------- fp32 products on the tensor cores
+// An fp32 value is the sum of three bf16 values of 8 bits each (exact where none of them is below 2^-133, and fp32 itself is not
+// denormal), and a product of two such values the sum of the six of their products that are above 2^-26 of it. The products of
+// the leading parts are summed by the tensor core over 64 k at a time, each such sum is added up in fp32 by the epilogue's threads;
+// the other five, 2^-8 of them and less, have an accumulator of their own. (The tensor core cuts sums off instead of rounding
+// them: in one accumulator over all of k the error grows to 1e-5 at k = 1536.) RMS error of 128 x 64 products against fp64, normal
+// operands, FFMA in order / as pairs along k / this: k = 64 1.5e-7 / 1.1e-7 / 7.1e-8, 128 2.0e-7 / 1.5e-7 / 7.4e-8, 512 4.0e-7 /
+// 2.9e-7 / 8.9e-8, 1536 7.0e-7 / 4.9e-7 / 1.2e-7; operands around 1: k = 128 1.7e-7 / 9.2e-8 / 3.3e-8.
+// A tile with a value that is not finite, or that bf16 would round to infinity, is computed once more on the FMA pipe.
+//
+// Tiles of 128 rows by BN columns; warps 0..7 convert (loads of the next k-block are on their way under this one's conversions),
+// 8..15 the epilogue (two per 32 rows, thread = row), 16 issues the MMAs.
+constexpr int kSplitThreads = 32 * 20;
+// registers: the block is launched with 96 per thread; the issuing warpgroup gives up what the epilogue takes, which holds 64 sums
+// beside the gates and residuals that are on their way
+constexpr int kSplitRegsLaunch = 96, kSplitRegsIssue = 32, kSplitRegsConvert = 104, kSplitRegsEpi = 120;
+static_assert(2 * kSplitRegsConvert + 2 * kSplitRegsEpi + kSplitRegsIssue <= 5 * kSplitRegsLaunch, "register split");
+// kFinal: gate, residual and output in whole vectors of four columns (an absent one is aligned)
+__host__ __device__ inline bool final_vec(const Args<float>& p) {
+    const uintptr_t bits = reinterpret_cast<uintptr_t>(p.final_out) | reinterpret_cast<uintptr_t>(p.residual) | reinterpret_cast<uintptr_t>(p.gate);
+    return (bits & 15) == 0 && (p.n & 3) == 0 && (p.map.inner_stride & 3) == 0 && (p.map.outer_stride & 3) == 0;
+}
 
-    // this thread's 16-byte vectors of a slab: row t / 4 + 32 i, k offset 4 (t % 4)
-    const int kc = (threadIdx.x & 3) * 4, lr = threadIdx.x >> 2;
-    const float* src[6];
-    float* dst[6];
-    bool in[6];
+template <int BN>
+struct SplitCfg {
+    static constexpr int kAPlane = 128 * 128, kWPlane = BN * 128;   // bytes: 64 bf16 per row, 128-byte swizzle
+    static constexpr int kStage = 3 * (kAPlane + kWPlane);
+    static constexpr int kBars = 2 * kStage;
+    static constexpr int kSmem = kBars + 256 + 1024;
+    static_assert(kSmem <= 227 * 1024, "shared memory of a block");
+    static constexpr int kTmem = 4 * BN;   // leading sums of even and odd k-blocks; small sums of even and odd tiles
+};
+
+// x0 and x1 less the halves of v, a pair of bf16 values
+__device__ __forceinline__ void sub_pair(float& x0, float& x1, uint32_t v) {
+    const uint32_t neg = v ^ 0x80008000u;
+    asm("{\n.reg .b16 lo, hi;\nmov.b32 {lo, hi}, %2;\nadd.rn.f32.bf16 %0, lo, %0;\nadd.rn.f32.bf16 %1, hi, %1;\n}\n"
+        : "+f"(x0), "+f"(x1)
+        : "r"(neg));
+}
+// Eight values into three planes of a stage, at d; bits 15 and 31 of `special`: an exponent of 254 or 255 as bf16
+__device__ __forceinline__ void split8(float (&x)[8], uint8_t* d, int plane, uint32_t& special) {
+    uint32_t u[4];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        if (i < 4) {
-            const int r = lr + 32 * i;                     // 64 hm + 4 ty + e -> slot 64 hm + 16 e + ty
-            in[i] = m0 + r < M;
-            src[i] = a + (in[i] ? m0 + r : 0) * K + kc;
-            dst[i] = slabs + ((r & 64) + (r & 3) * 16 + ((r & 63) >> 2)) * kPitch + kc;
-        } else {
-            const int c = lr + 32 * (i - 4);               // 32 hf + 4 tx + e -> slot 32 hf + 8 e + tx
-            in[i] = n0 + c < n;
-            src[i] = w + (long long)(in[i] ? n0 + c : 0) * K + kc;
-            dst[i] = slabs + (BM + (c & 32) + (c & 3) * 8 + ((c & 31) >> 2)) * kPitch + kc;
+    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            u[i] = pack_bf16x2(x[2 * i], x[2 * i + 1]);
+            if (q == 0) special |= (u[i] & 0x7f007f00u) + 0x01000100u;
+            if (q < 2) sub_pair(x[2 * i], x[2 * i + 1], u[i]);
         }
+        *reinterpret_cast<uint4*>(d + q * plane) = make_uint4(u[0], u[1], u[2], u[3]);
     }
-    const int slabs_k = (K + BK - 1) / BK;
-    auto fetch = [&](int ks) {
-        if (ks < slabs_k) {
-            const bool kin = ks * BK + kc < K;
+}
+
+// eight consecutive values, `n` of which exist
+__device__ __forceinline__ void load8(const float* p, int n, bool vec, float (&x)[8]) {
+    const float4 a = load4(p, n, vec), b = load4(p + 4, n - 4, vec);
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+__device__ __forceinline__ void load8(const float* p, int n, float (&x)[8]) {   // n a multiple of four, p on 16 bytes
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+    if (n >= 4) a = reinterpret_cast<const float4*>(p)[0];
+    if (n >= 8) b = reinterpret_cast<const float4*>(p)[1];
+    x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+    x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+__device__ __forceinline__ void store8(float* p, const float (&o)[8], int n) {   // the first n
+    if (n >= 8 && umma::aligned32(p)) {
+        uint32_t u[8];
 #pragma unroll
-            for (int i = 0; i < 6; ++i)
-                cp_async16(dst[i] + (ks % kStages) * ((BM + BN) * kPitch), kin ? src[i] + ks * BK : src[i] - kc, kin && in[i]);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        for (int i = 0; i < 8; ++i) u[i] = __float_as_uint(o[i]);
+        umma::stg256(p, u);
+    } else if (n >= 8 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        reinterpret_cast<float4*>(p)[0] = make_float4(o[0], o[1], o[2], o[3]);
+        reinterpret_cast<float4*>(p)[1] = make_float4(o[4], o[5], o[6], o[7]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i < n) p[i] = o[i];
+    }
+}
+
+// kWhole: k in whole k-blocks, and operands in whole vectors along it. kShort (kFinal): at most two k-blocks, and gate, residual and
+// output in whole vectors (an instantiation of its own: both forms in one kernel spilled 1100 bytes of registers)
+template <int BN, int EPI, bool K_OUTER, bool kWhole, bool kShort>
+__global__ void __launch_bounds__(kSplitThreads, 1)
+gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
+    using namespace umma;
+    using C = SplitCfg<BN>;
+    constexpr bool kPaired = EPI == kGatedPlanes || EPI == kSwiglu;
+    constexpr int HN = BN / 2, kCols = kPaired ? HN : BN;   // columns of the result per tile
+    constexpr int kRun = BN / 4;                            // an epilogue thread's columns: kRun in each half of the tile
+    constexpr int kItemsA = 4, kItemsW = BN / 32;           // vectors of eight k per converting thread and k-block
+    constexpr int kKid = 20;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
+    const uint32_t bars = sbase + C::kBars;
+    auto full = [&](int s) { return bars + 8u * s; };             // a stage is converted
+    auto empty = [&](int s) { return bars + 8u * (2 + s); };      // its products are done
+    auto main_full = [&](int s) { return bars + 8u * (4 + s); };  // leading sums of a k-block
+    auto main_free = [&](int s) { return bars + 8u * (6 + s); };
+    auto small_full = [&](int s) { return bars + 8u * (8 + s); };   // small sums of a tile
+    auto small_free = [&](int s) { return bars + 8u * (10 + s); };
+    volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + C::kBars + 96);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + C::kBars + 104);
+    volatile int* special = reinterpret_cast<volatile int*>(gbase + C::kBars + 112);   // [4] tile numbers (of this CTA, from 1)
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int K = p.K, n = p.n;
+    const long long M = p.M;
+    const int num_kb = (K + 63) / 64;
+    const uint32_t row_tiles = (uint32_t)((M + 127) / 128), col_tiles = (uint32_t)(n + kCols - 1) / kCols;
+    const uint32_t num_tiles = row_tiles * col_tiles * (uint32_t)(groups * batch);   // (below 2^31)
+    struct Tile {
+        long long m0, boff;
+        int grp, n0;
     };
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
-    u64 acc[TM][TN];
+    auto tile_of = [&](uint32_t t) {   // row tiles innermost: CTAs that run at the same time share the weights
+        Tile c;
+        uint32_t q = t / row_tiles;
+        c.m0 = (t - q * row_tiles) * 128LL;
+        const uint32_t q2 = q / col_tiles;
+        c.n0 = (int)(q - q2 * col_tiles) * kCols;
+        q = q2 / (uint32_t)groups;
+        c.grp = (int)(q2 - q * groups);
+        c.boff = q * p.a_batch;
+        return c;
+    };
+    auto weight_row = [&](const Tile& c, int j, int& col) {   // row j of the weight tile: its matrix, and its row there
+        col = c.n0 + (kPaired ? j % HN : j);
+        return kPaired ? (j < HN ? p.w[2 * c.grp] : p.w[2 * c.grp + 1]) : p.w[c.grp] + c.boff;
+    };
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(full(s), 8);
+            mbar_init(empty(s), 1);
+            mbar_init(main_full(s), 1);
+            mbar_init(main_free(s), 8);
+            mbar_init(small_full(s), 1);
+            mbar_init(small_free(s), 8);
+        }
+        for (int i = 0; i < 4; ++i) special[i] = 0;
+        *abort_flag = 0;
+        mbar_fence_init();
+    }
+    if (warp == 16) {
+        tmem_alloc(smem_u32((const void*)tmem_ptr), C::kTmem);
+        tmem_relinquish();
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_ptr;
+    grid_trigger();
+    if (warp >= 8) grid_wait();
+
+    if (warp < 8) {
+        // ---------------------------------------------------------------- conversion
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSplitRegsConvert));
+        const long long step_a = K_OUTER ? M : 1, step_w = K_OUTER ? n : 1;   // from one k to the next
+        // the tile's operands, and where the thread's vectors of the first k-block lie; rows past the end: the last one
+        const float *a0 = nullptr, *w0 = nullptr, *w1 = nullptr;
+        uint32_t oa[kItemsA] = {}, ow[kItemsW] = {};
+        static_assert(!kPaired || (!K_OUTER && kItemsW % 2 == 0), "the second half of the vectors is of the second weight");
+        bool va = kWhole, vw = kWhole;
+        float xa[kItemsA][8], xw[kItemsW][8];
+        // a k-block's vector v: rows of k next to one another: eight lanes per row; K_OUTER: a row per lane
+        auto row_of = [&](int v, int rows) { return K_OUTER ? v % rows : v >> 3; };
+        auto chunk_of = [&](int v, int rows) { return K_OUTER ? v / rows : v & 7; };
+        auto fetch = [&](const float* src, long long step, bool vec, int k, float (&x)[8]) {
+            if constexpr (K_OUTER) {
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+                for (int e = 0; e < 8; ++e) x[e] = kWhole || k + e < K ? src[e * step] : 0.f;
+            } else if constexpr (kWhole) {
+                const float4 u = reinterpret_cast<const float4*>(src)[0], w = reinterpret_cast<const float4*>(src)[1];
+                x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+                x[4] = w.x; x[5] = w.y; x[6] = w.z; x[7] = w.w;
+            } else {
+                load8(src, K - k, vec, x);
+            }
+        };
+        auto fetch_a = [&](int i, int kb) {
+            const int v = threadIdx.x + i * 256;
+            fetch(a0 + kb * 64 * step_a + oa[i], step_a, va, kb * 64 + chunk_of(v, 128) * 8, xa[i]);
+        };
+        auto fetch_w = [&](int i, int kb) {
+            const int v = threadIdx.x + i * 256;
+            fetch((kPaired && i >= kItemsW / 2 ? w1 : w0) + kb * 64 * step_w + ow[i], step_w, vw, kb * 64 + chunk_of(v, BN) * 8, xw[i]);
+        };
+        auto open = [&](uint32_t t) {
+            const Tile c = tile_of(t);
+            int col;
+            a0 = p.a + c.boff + (K_OUTER ? c.m0 : c.m0 * K);
+            w0 = weight_row(c, 0, col);
+            w1 = weight_row(c, BN - 1, col);
+            if (!kWhole && !K_OUTER) {
+                va = vec_ok(a0, K);
+                vw = vec_ok(w0, K) && vec_ok(w1, K);
+            }
+            const uint32_t last_row = (uint32_t)min(M - 1 - c.m0, 127LL);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+            for (int i = 0; i < kItemsA; ++i) {
+                const int v = threadIdx.x + i * 256;
+                const uint32_t r = min((uint32_t)row_of(v, 128), last_row);
+                oa[i] = r * (K_OUTER ? 1u : (uint32_t)K) + chunk_of(v, 128) * 8 * (uint32_t)step_a;
+            }
 #pragma unroll
-    for (int ks = 0; ks < kStages - 1; ++ks) fetch(ks);
-    for (int ks = 0; ks < slabs_k; ++ks) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
-        __syncthreads();
-        fetch(ks + kStages - 1);
-        const float* as = slabs + (ks % kStages) * ((BM + BN) * kPitch) + ty * kPitch;
-        const float* ws = slabs + (ks % kStages) * ((BM + BN) * kPitch) + (BM + tx) * kPitch;
+            for (int i = 0; i < kItemsW; ++i) {
+                const int v = threadIdx.x + i * 256;
+                weight_row(c, row_of(v, BN), col);
+                ow[i] = (uint32_t)min(col, n - 1) * (K_OUTER ? 1u : (uint32_t)K) + chunk_of(v, BN) * 8 * (uint32_t)step_w;
+            }
+        };
+        bool ok = true;
+        uint32_t it = 0;
+        int seq = 0;
+        open(blockIdx.x);
+        if (p.a_batch != 0) grid_wait();   // (batched products: no weights)
 #pragma unroll
-        for (int q = 0; q < BK / 4; ++q) {
-            ulonglong2 av[TM];
+        for (int i = 0; i < kItemsW; ++i) fetch_w(i, 0);
+        if (p.a_batch == 0) grid_wait();
 #pragma unroll
-            for (int i = 0; i < TM; ++i)
-                av[i] = *reinterpret_cast<const ulonglong2*>(as + ((i >> 2) * 64 + (i & 3) * 16) * kPitch + q * 4);
+        for (int i = 0; i < kItemsA; ++i) fetch_a(i, 0);
+        for (uint32_t t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++seq) {
+            uint32_t bad = 0;
+            for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                const int s = it & 1;
+                if (!mbar_wait(empty(s), ((it >> 1) & 1u) ^ 1u, abort_flag)) {
+                    if (lane == 0) report_wait_failure(status, abort_flag, kKid, 1);
+                    ok = false;
+                    break;
+                }
+                uint8_t* const stage = gbase + s * C::kStage;
+                const bool last = kb + 1 == num_kb, more = !last || t + gridDim.x < num_tiles;
+                const int next = last ? 0 : kb + 1;
+                if (last && more) open(t + gridDim.x);
 #pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const ulonglong2 wv = *reinterpret_cast<const ulonglong2*>(ws + ((j >> 2) * 32 + (j & 3) * 8) * kPitch + q * 4);
+                for (int i = 0; i < kItemsA; ++i) {
+                    const int v = threadIdx.x + i * 256;
+                    split8(xa[i], stage + sw128_offset(row_of(v, 128), chunk_of(v, 128) * 8), C::kAPlane, bad);
+                    if (more) fetch_a(i, next);
+                }
 #pragma unroll
-                for (int i = 0; i < TM; ++i) {
-                    fma2(acc[i][j], av[i].x, wv.x);
-                    fma2(acc[i][j], av[i].y, wv.y);
+                for (int i = 0; i < kItemsW; ++i) {
+                    const int v = threadIdx.x + i * 256;
+                    split8(xw[i], stage + 3 * C::kAPlane + sw128_offset(row_of(v, BN), chunk_of(v, BN) * 8), C::kWPlane, bad);
+                    if (more) fetch_w(i, next);
+                }
+                if (bad & 0x80008000u) special[seq & 3] = seq + 1;
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full(s));
+            }
+        }
+    } else if (warp >= 16) {
+        // ---------------------------------------------------------------- MMA issuer
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kSplitRegsIssue));
+        if (warp == 16 && elect_one()) {
+            constexpr uint32_t idesc = idesc_bf16_f32(128, BN);
+            uint32_t it = 0, tc = 0;
+            bool ok = true;
+            for (uint32_t t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tc) {
+                const uint32_t d_small = tmem_base + 2 * BN + (tc & 1u) * BN;
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    const int s = it & 1;
+                    if (!mbar_wait(full(s), (it >> 1) & 1u, abort_flag) || !mbar_wait(main_free(s), ((it >> 1) & 1u) ^ 1u, abort_flag) ||
+                        (kb == 0 && !mbar_wait(small_free(tc & 1u), ((tc >> 1) & 1u) ^ 1u, abort_flag))) {
+                        report_wait_failure(status, abort_flag, kKid, 2);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    const uint32_t sa = sbase + s * C::kStage, sw = sa + 3 * C::kAPlane;
+                    auto products = [&](int pa, int pw, uint32_t d, bool fresh) {
+                        const uint64_t ad = smem_desc_k_sw128(sa + pa * C::kAPlane), wd = smem_desc_k_sw128(sw + pw * C::kWPlane);
+#pragma unroll
+                        for (int k4 = 0; k4 < 4; ++k4) mma_bf16(d, ad + 2u * k4, wd + 2u * k4, idesc, fresh && k4 == 0 ? 0u : 1u);
+                    };
+                    products(0, 0, tmem_base + s * BN, true);
+                    mma_commit(main_full(s));
+                    products(2, 0, d_small, kb == 0);
+                    products(1, 1, d_small, false);
+                    products(0, 2, d_small, false);
+                    products(1, 0, d_small, false);
+                    products(0, 1, d_small, false);
+                    mma_commit(empty(s));
+                }
+                if (ok) mma_commit(small_full(tc & 1u));
+            }
+        }
+    } else {
+        // ---------------------------------------------------------------- epilogue: thread = row, kRun columns of each half
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSplitRegsEpi));
+        const int quad = warp & 3, part = (warp - 8) >> 2;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + part * kRun;
+        uint32_t it = 0, tc = 0;
+        for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tc) {
+            const Tile c = tile_of(t);
+            const long long r = c.m0 + quad * 32 + lane;
+            const bool live = r < M;
+            const float mk = (EPI == kGatedPlanes || EPI == kFinal) && p.mask && live ? p.mask[r] : 1.0f;
+            const uint32_t t_small = 2 * BN + (tc & 1u) * BN;
+            auto col_of = [&](int e) { return c.n0 + part * kRun + (e < kRun ? e : HN + e - kRun); };
+            auto add16 = [&](uint32_t col, float (&v)[16]) {
+                uint32_t u[16];
+                tmem_ld16(taddr + col, u);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 16; ++e) v[e] += __uint_as_float(u[e]);
+            };
+            auto wait_main = [&] {
+                if (mbar_wait(main_full(it & 1), (it >> 1) & 1u, abort_flag)) return true;
+                if (lane == 0) report_wait_failure(status, abort_flag, kKid, 3);
+                return false;
+            };
+            auto wait_small = [&] {
+                if (mbar_wait(small_full(tc & 1u), (tc >> 1) & 1u, abort_flag)) return true;
+                if (lane == 0) report_wait_failure(status, abort_flag, kKid, 4);
+                return false;
+            };
+            auto free_main = [&](uint32_t s) {
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(main_free(s));
+            };
+            // one value of the result from its product (and that of the paired weight)
+            auto result = [&](int e, float x, float y) {
+                const int col = col_of(e);
+                if (!live || col >= n) return;
+                if constexpr (EPI == kGatedPlanes) {
+                    p.out[c.grp][(long long)col * M + r] = mk * sigmoid_acc(y) * x;
+                } else if constexpr (EPI == kSwiglu) {
+                    p.out[0][r * n + col] = x * sigmoid_acc(x) * y;
+                } else if constexpr (EPI == kFinal) {
+                    if (p.gate) x *= sigmoid_acc(p.gate[r * n + col]);
+                    if (p.mask) x *= mk;
+                    const long long at = row_offset(p.map, r) + col;
+                    p.final_out[at] = x + (p.residual ? p.residual[at] : 0.f);
+                } else {
+                    p.out[c.grp][c.boff + r * n + col] = x + (p.bias[c.grp] ? p.bias[c.grp][col] : 0.f);
+                }
+            };
+            // a tile with values that the split does not take: its products on the FMA pipe
+            auto redo = [&] {
+                auto dot = [&](int e) {
+                    int col;
+                    const float* w = weight_row(c, part * kRun + (e < kRun ? e : HN + e - kRun), col);
+                    float x = 0.f;
+                    if (live && col < n)
+                        for (int k = 0; k < K; ++k)
+                            x = K_OUTER ? fmaf(p.a[c.boff + (long long)k * M + r], w[(long long)k * n + col], x)
+                                        : fmaf(p.a[c.boff + r * K + k], w[(long long)col * K + k], x);
+                    return x;
+                };
+#pragma unroll 1
+                for (int e = 0; e < (kPaired ? kRun : 2 * kRun); ++e) result(e, dot(e), kPaired ? dot(kRun + e) : 0.f);
+            };
+            // all of the thread's columns, 16 by 16
+            auto sum_up = [&](float (&v)[2 * kRun / 16][16]) {
+                auto add = [&](uint32_t col) {
+#pragma unroll
+                    for (int e0 = 0; e0 < 2 * kRun; e0 += 16) add16(col + (e0 < kRun ? e0 : HN + e0 - kRun), v[e0 / 16]);
+                };
+#pragma unroll
+                for (int e = 0; e < 2 * kRun; ++e) v[e / 16][e % 16] = 0.f;
+                for (int kb = 0; kb < num_kb; ++kb, ++it) {
+                    if (!wait_main()) return false;
+                    tc_fence_after_sync();
+                    add((it & 1) * BN);
+                    free_main(it & 1);
+                }
+                if (!wait_small()) return false;
+                tc_fence_after_sync();
+                add(t_small);
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(small_free(tc & 1u));
+                return true;
+            };
+            if constexpr (EPI == kFinal) {
+                const long long off = live ? row_offset(p.map, r) : 0;
+                const bool vec = kShort || final_vec(p);
+                // Gates and residuals of 16 columns from e0 on: ahead of the stores before them, which may be to the residual's own rows
+                struct Ahead {
+                    float gate[2][8], residual[2][8];
+                };
+                auto fetch = [&](int e0, Ahead& a) {
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const int col = col_of(e0 + 8 * q), left = live ? n - col : 0;
+                        if (p.gate) load8(p.gate + r * n + col, left, a.gate[q]);
+                        if (p.residual) load8(p.residual + off + col, left, a.residual[q]);
+                    }
+                };
+                auto finish = [&](float (&v)[16], const Ahead& a) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (p.gate) v[j] *= sigmoid_acc(a.gate[j >> 3][j & 7]);
+                        if (p.mask) v[j] *= mk;
+                        if (p.residual) v[j] += a.residual[j >> 3][j & 7];
+                    }
+                };
+                auto put = [&](int e0, const float (&v)[16]) {
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const int col = col_of(e0 + 8 * q);
+                        float o[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) o[j] = v[8 * q + j];
+                        if (live) store8(p.final_out + off + col, o, n - col);
+                    }
+                };
+                if constexpr (kShort) {
+                    // both leading sums stay where they are until they are added up, 16 columns at a time
+                    Ahead a[2];
+                    fetch(0, a[0]);
+                    fetch(16, a[1]);
+                    bool ok = wait_main();
+                    const uint32_t s0 = it++ & 1;
+                    if (ok && num_kb == 2) {
+                        ok = wait_main();
+                        ++it;
+                    }
+                    if (!ok || !wait_small()) break;
+                    tc_fence_after_sync();
+                    const bool bad = special[tc & 3] == (int)tc + 1;
+#pragma unroll
+                    for (int e0 = 0; e0 < 2 * kRun; e0 += 16) {
+                        const uint32_t at = e0 < kRun ? e0 : HN + e0 - kRun;
+                        float v[16];
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) v[e] = 0.f;
+                        add16(s0 * BN + at, v);
+                        if (num_kb == 2) add16((s0 ^ 1u) * BN + at, v);
+                        add16(t_small + at, v);
+                        if (e0 + 16 == 2 * kRun) {
+                            free_main(s0);
+                            if (num_kb == 2) free_main(s0 ^ 1u);
+                            if (lane == 0) mbar_arrive(small_free(tc & 1u));
+                        }
+                        if (bad) continue;
+                        finish(v, a[e0 / 16 % 2]);
+                        if (e0 + 32 < 2 * kRun) fetch(e0 + 32, a[e0 / 16 % 2]);
+                        put(e0, v);
+                    }
+                    if (bad) redo();
+                } else {
+                    float v[2 * kRun / 16][16];
+                    if (!sum_up(v)) break;
+                    if (special[tc & 3] == (int)tc + 1) {
+                        redo();
+                    } else if (!vec) {
+#pragma unroll
+                        for (int e = 0; e < 2 * kRun; ++e) result(e, v[e / 16][e % 16], 0.f);
+                    } else {
+                        Ahead a;
+                        fetch(0, a);
+#pragma unroll
+                        for (int e0 = 0; e0 < 2 * kRun; e0 += 16) {
+                            finish(v[e0 / 16], a);
+                            if (e0 + 16 < 2 * kRun) fetch(e0 + 16, a);
+                            put(e0, v[e0 / 16]);
+                        }
+                    }
+                }
+            } else {
+                float v[2 * kRun / 16][16];
+                if (!sum_up(v)) break;
+                if (special[tc & 3] == (int)tc + 1) {
+                    redo();
+                    continue;
+                }
+                if (!live) continue;
+                auto at = [&](int e) { return v[e / 16][e % 16]; };
+                if constexpr (EPI == kGatedPlanes) {
+                    float* out = p.out[c.grp];
+#pragma unroll
+                    for (int j = 0; j < kRun; ++j)
+                        if (col_of(j) < n) out[(long long)col_of(j) * M + r] = mk * sigmoid_acc(at(kRun + j)) * at(j);
+                } else {
+#pragma unroll
+                    for (int e0 = 0; e0 < (EPI == kSwiglu ? kRun : 2 * kRun); e0 += 8) {
+                        const int col = col_of(e0);
+                        float o[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float x = at(e0 + j);
+                            if constexpr (EPI == kSwiglu) o[j] = x * sigmoid_acc(x) * at(kRun + e0 + j);
+                            else o[j] = x + (p.bias[c.grp] && col + j < n ? p.bias[c.grp][col + j] : 0.f);
+                        }
+                        store8((EPI == kSwiglu ? p.out[0] : p.out[c.grp] + c.boff) + r * n + col, o, n - col);
+                    }
                 }
             }
         }
     }
-    float v[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const float2 f = unpack2(acc[i][j]);
-            v[i][j] = f.x + f.y;
-        }
-    epilogue<BM, BN, TM, TN, EPI, float>(p, v, m0, n0, grp, boff, tx, ty);
-}
-constexpr int kPairsSmem = 4 * (128 + 64) * 20 * 4;
 
-template <int EPI>
-int launch_pairs(const Args<float>& p, dim3 grid, cudaStream_t st) {
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == 16) {
+        tc_fence_after_sync();
+        tmem_dealloc(tmem_base, C::kTmem);
+    }
+}
+
+template <int BN, int EPI, bool K_OUTER, bool kWhole, bool kShort = false>
+int launch_split(const Args<float>& p, int groups, int batch, cudaStream_t st) {
+    using C = SplitCfg<BN>;
+    constexpr int kCols = EPI == kGatedPlanes || EPI == kSwiglu ? BN / 2 : BN;
     static PerDeviceOnce configured;
     if (!configured.done()) {
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(gemm_pairs_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairsSmem));
+        cudaFuncAttributes fa;   // a block launched with fewer registers would wait for the split for good
+        OF3_CUDA_CHECK(cudaFuncGetAttributes(&fa, gemm_split_kernel<BN, EPI, K_OUTER, kWhole, kShort>));
+        OF3_REQUIRE(fa.numRegs == kSplitRegsLaunch, OF3_ERR_DRIVER, "the split product is built with %d registers, not %d", fa.numRegs,
+                    kSplitRegsLaunch);
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(gemm_split_kernel<BN, EPI, K_OUTER, kWhole, kShort>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            C::kSmem));
         configured.mark();
     }
-    OF3_CUDA_CHECK(launch_chained(gemm_pairs_kernel<EPI>, grid, 128, kPairsSmem, st, p));
+    const long long tiles = (p.M + 127) / 128 * ((p.n + kCols - 1) / kCols) * groups * batch;
+    OF3_REQUIRE(tiles < (1LL << 31), OF3_ERR_SHAPE, "gemm: %lld rows, %d columns, batch %d", p.M, p.n, batch);
+    LaunchScope scope(20, st);
+    OF3_CUDA_CHECK(launch_chained(gemm_split_kernel<BN, EPI, K_OUTER, kWhole, kShort>, (unsigned)(tiles < sm_count() ? tiles : sm_count()),
+                                  kSplitThreads, C::kSmem, st, p, batch, groups, device_status_ptr()));
     return OF3_OK;
 }
 
@@ -489,24 +905,37 @@ int launch(Args<T> p, int groups, int batch, cudaStream_t st) {
     auto tiles = [&](int bm, int bn) {
         return ((M + bm - 1) / bm) * ((p.n + bn - 1) / bn) * groups * (long long)batch;
     };
-    // large tiles once they give every SM at least one
-    const bool large = tiles(128, kPaired ? 32 : 64) >= sm_count();
+    if constexpr (std::is_same<T, float>::value) {
+        // Tensor cores once the small tiles of the FMA kernel would come in more than four waves. Device time, us, FMA / tensor, cold:
+        // 576 rows: 4 x 128 columns 7.8 / 11.9; 2304 rows: 128 columns 8.0 / 12.4 (two waves), 4 x 128 22.3 / 12.5 (eight)
+        if (tiles(32, kPaired ? 16 : 32) > 4 * sm_count()) {
+            bool whole = p.K % 64 == 0;
+            if (!K_OUTER) {
+                whole = whole && (reinterpret_cast<uintptr_t>(p.a) & 15) == 0 && (p.a_batch & 3) == 0;
+                for (int i = 0; i < groups * (kPaired ? 2 : 1); ++i) whole = whole && (reinterpret_cast<uintptr_t>(p.w[i]) & 15) == 0;
+            }
+            if constexpr (EPI == kFinal) {
+                if (whole && p.K <= 128 && final_vec(p)) return launch_split<128, EPI, K_OUTER, true, true>(p, groups, batch, st);
+            }
+            return whole ? launch_split<128, EPI, K_OUTER, true>(p, groups, batch, st)
+                         : launch_split<128, EPI, K_OUTER, false>(p, groups, batch, st);
+        }
+    }
+    // Otherwise small tiles; with bf16 weights, large ones once they give every SM at least one
+    const bool large = !std::is_same<T, float>::value && tiles(128, kPaired ? 32 : 64) >= sm_count();
     const int bm = large ? 128 : 32, bn = large ? (kPaired ? 32 : 64) : (kPaired ? 16 : 32);
     const long long gx = (M + bm - 1) / bm, gy = (long long)((p.n + bn - 1) / bn) * groups;
     OF3_REQUIRE(batch <= 65535 && gy <= 65535 && gx < (1LL << 31), OF3_ERR_SHAPE, "gemm: %lld rows, %d columns, batch %d",
                 M, p.n, batch);
     const dim3 grid((unsigned)gx, (unsigned)gy, batch);
     LaunchScope scope(20, st);
-    if constexpr (std::is_same<T, float>::value && !K_OUTER && !kPaired) {
-        // where every operand, and every plane of a batch, comes in whole vectors along k
-        uintptr_t bits = reinterpret_cast<uintptr_t>(p.a) | (uintptr_t)(p.K & 3) << 2 | (uintptr_t)(p.a_batch & 3) << 2;
-        for (int i = 0; i < groups; ++i) bits |= reinterpret_cast<uintptr_t>(p.w[i]);
-        if (large && (bits & 15) == 0) return launch_pairs<EPI>(p, grid, st);
+    if constexpr (!std::is_same<T, float>::value) {
+        if (large) {
+            OF3_CUDA_CHECK(launch_chained(gemm_kernel<128, 64, 8, 8, 1, EPI, K_OUTER, T>, grid, 128, 0, st, p));
+            return OF3_OK;
+        }
     }
-    if (large)
-        OF3_CUDA_CHECK(launch_chained(gemm_kernel<128, 64, 8, 8, 1, EPI, K_OUTER, T>, grid, 128, 0, st, p));
-    else
-        OF3_CUDA_CHECK(launch_chained(gemm_kernel<32, 32, 4, 4, 4, EPI, K_OUTER, T>, grid, 256, 0, st, p));
+    OF3_CUDA_CHECK(launch_chained(gemm_kernel<32, 32, 4, 4, 4, EPI, K_OUTER, T>, grid, 256, 0, st, p));
     return OF3_OK;
 }
 

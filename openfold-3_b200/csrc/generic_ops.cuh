@@ -1,7 +1,7 @@
 // Shape-generic SIMT kernels (any channel width, head count, sequence length).
 //
-// They back (1) the fp32 validation mode, where every product and sum is true fp32 (no
-// tensor cores, no TF32), and (2) bf16 storage with shapes the tcgen05 kernels do not
+// They back (1) the fp32 validation mode, where every product and sum is fp32 or nearer to the exact value (large matrix
+// products as sums of bf16 products on the tensor cores, generic_gemm.cu; no TF32), and (2) bf16 storage with shapes the tcgen05 kernels do not
 // cover. Storage type T is float or __nv_bfloat16; intermediates are always fp32.
 #pragma once
 #include "common.cuh"

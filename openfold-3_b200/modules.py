@@ -623,7 +623,7 @@ class AttentionPairBias(_Layer):
     def _run(self, a, z, s, mask, in_place: bool, high_precision: bool = False, pair_bias=None):
         """``high_precision`` (the reference's ``use_high_precision_attention``, which computes logits and softmax
         in fp32: openfold3/core/model/primitives/attention.py:99-120, 314-339): bf16 inputs are evaluated by the
-        fp32 validation kernels (true fp32 products everywhere) and the result is rounded once at the end."""
+        fp32 validation kernels (fp32 products everywhere) and the result is rounded once at the end."""
         if high_precision and a.dtype != torch.float32:
             f32 = lambda t: None if t is None else t.float()
             upd = self._run(f32(a), f32(z), f32(s), f32(mask), in_place=False)
