@@ -4,7 +4,7 @@
 // error, and past its 75 TFLOP/s. Few rows, and bf16 weights, stay on the FMA pipe: tiles of 128 x 64 with 8 x 8 products per
 // thread (packed fma.f32x2; the next k-slab is in registers while this one is multiplied), and where there are few of these, or
 // the operands are fp32, 32 x 32 tiles whose k-slab is split over four groups of threads (the chain over k = 1536 on 24 large tiles
-// is what such a layer waits for). Fp32 trunk block, FMA pipe alone / now, us: N = 48 429 / 369, 64 520 / 434, 128 955 / 695, 250
+// is what such a layer waits for). Fp32 trunk block, FMA pipe alone / as here, us: N = 48 429 / 369, 64 520 / 434, 128 955 / 695, 250
 // 3310 / 2246.
 #include "generic_ops.cuh"
 #include "runtime.cuh"

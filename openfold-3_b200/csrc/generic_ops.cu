@@ -220,7 +220,7 @@ template <int DP>
 constexpr int att_smem_floats() { return 2 * DP * kAttP + kAttK * DP + kAttK * kAttP + kAttK; }
 
 template <int DP, typename T>
-__global__ void __launch_bounds__(256) attention_kernel(const float* __restrict__ q, const float* __restrict__ k,
+__global__ void __launch_bounds__(256, DP <= 32 ? 3 : 2) attention_kernel(const float* __restrict__ q, const float* __restrict__ k,
                                                         const float* __restrict__ v, const float* g,
                                                         const T* __restrict__ mask, long long mask_row,
                                                         long long mask_k, float inf, const float* __restrict__ pair_bias,
@@ -252,21 +252,44 @@ __global__ void __launch_bounds__(256) attention_kernel(const float* __restrict_
 #pragma unroll
         for (int c = 0; c < DC; ++c) o[i][c] = 0.f;
     }
-    for (int k0 = 0; k0 < N; k0 += kAttK) {
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < kAttK * DP; idx += 256) {
-            const int i = idx / DP, c = idx % DP;
+    // A key block's keys and values, in registers while the block before them is multiplied: fetched between the barriers they, and
+    // the pair bias fetched where it is added, were most of a block's time (fp32 trunk block: N = 128 695 -> 677 us, 250 2246 -> 2143, with three blocks per SM)
+    constexpr int kVecs = kAttK * DP / 256;
+    float rk[kVecs], rv[kVecs], rm = 0.f;
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < kVecs; ++u) {
+            const int i = (threadIdx.x + u * 256) / DP, c = (threadIdx.x + u * 256) % DP;
             const bool in = k0 + i < N && c < d;
             const long long off = base + (k0 + i) * pitch + c;
-            Ks[c * kAttP + i] = in ? k[off] : 0.f;
-            Vs[i * DP + c] = in ? v[off] : 0.f;
+            rk[u] = in ? k[off] : 0.f;
+            rv[u] = in ? v[off] : 0.f;
         }
         if (threadIdx.x < kAttK) {
             const int kk = k0 + threadIdx.x;
-            Ms[threadIdx.x] = kk >= N ? -INFINITY
-                              : (mask ? inf * (ld_as_float(mask + bb * mask_row + kk * mask_k) - 1.0f) : 0.f);
+            rm = kk >= N ? -INFINITY : (mask ? inf * (ld_as_float(mask + bb * mask_row + kk * mask_k) - 1.0f) : 0.f);
         }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < N; k0 += kAttK) {
         __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kVecs; ++u) {
+            const int i = (threadIdx.x + u * 256) / DP, c = (threadIdx.x + u * 256) % DP;
+            Ks[c * kAttP + i] = rk[u];
+            Vs[i * DP + c] = rv[u];
+        }
+        if (threadIdx.x < kAttK) Ms[threadIdx.x] = rm;
+        __syncthreads();
+        float bias[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int qi = q0 + ty * 4 + i, kk = k0 + tx * 4 + j;
+                bias[i][j] = pb && qi < N && kk < N ? pb[(long long)qi * N + kk] : 0.f;
+            }
+        if (k0 + kAttK < N) fetch(k0 + kAttK);
         float s[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -285,13 +308,10 @@ __global__ void __launch_bounds__(256) attention_kernel(const float* __restrict_
         float p[4][4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int qi = q0 + ty * 4 + i;
             float mx = -INFINITY;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int kk = k0 + tx * 4 + j;
-                float x = s[i][j] * scale + Ms[tx * 4 + j];
-                if (pb && qi < N && kk < N) x += pb[(long long)qi * N + kk];
+                const float x = s[i][j] * scale + Ms[tx * 4 + j] + bias[i][j];
                 s[i][j] = x;
                 mx = fmaxf(mx, x);
             }
