@@ -46,9 +46,68 @@ __device__ __forceinline__ void row_sums(float (&v)[4], int lane) {
 }
 
 // Keeps the compiler from carrying values computed from v[first .. first + 15] over this point.
-__device__ __forceinline__ void opaque(uint32_t (&v)[32], int first) {
+template <int N>
+__device__ __forceinline__ void opaque(uint32_t (&v)[N], int first) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(v[first + i]));
+}
+
+// LN of rows 0, 2, .. 2 (NR - 1) from src on, of which those below `left` exist: eight channels of each, packed. A half warp reads a
+// row (coalesced).
+template <int NR>
+__device__ __forceinline__ void normalize_rows(const __nv_bfloat16* src, int left, int ch, int lane, const float* prm,
+                                               uint32_t (&raw)[NR * 4]) {
+#pragma unroll
+    for (int h = 0; h < NR; h += 4) {   // four rows at a time (registers)
+        float mean[4], rstd[4];
+        asm volatile("" ::: "memory");
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (2 * (h + r) < left) v = *reinterpret_cast<const uint4*>(src + 2 * (h + r) * kC);
+            uint32_t* o = &raw[(h + r) * 4];
+            o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float a = 0.f, b = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { a = add_lo(raw[(h + r) * 4 + i], a); b = add_hi(raw[(h + r) * 4 + i], b); }
+            mean[r] = a + b;
+        }
+        row_sums(mean, lane);
+        opaque(raw, h * 4);   // unpack again rather than keep 32 floats
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            mean[r] *= 1.0f / kC;
+            float a = 0.f, b = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float x0 = add_lo(raw[(h + r) * 4 + i], -mean[r]), x1 = add_hi(raw[(h + r) * 4 + i], -mean[r]);
+                a = fmaf(x0, x0, a);
+                b = fmaf(x1, x1, b);
+            }
+            rstd[r] = a + b;
+        }
+        row_sums(rstd, lane);
+        opaque(raw, h * 4);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            rstd[r] = rsqrtf(rstd[r] * (1.0f / kC) + kLnEps);
+            mean[r] *= -rstd[r];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 ga = *reinterpret_cast<const float2*>(prm + ch * 8 + i * 2);
+            const float2 be = *reinterpret_cast<const float2*>(prm + 128 + ch * 8 + i * 2);
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                uint32_t& v = raw[(h + r) * 4 + i];
+                v = pack_bf16x2(fmaf(fmaf(bf16lo(v), rstd[r], mean[r]), ga.x, be.x),
+                                fmaf(fmaf(bf16hi(v), rstd[r], mean[r]), ga.y, be.y));
+            }
+        }
+    }
 }
 
 struct TrSmem {
@@ -81,7 +140,8 @@ constexpr int kTrThreads = 32 * 28;
 
 // kSolo: one tile per CTA (a tensor of no more tiles than SMs), whose chunks alternate between both groups' D1 and h buffers, so
 // that G1 runs two chunks ahead of the silu pass instead of one: N = 24 / 37 / 64 / 111 / 137, unchained, 14.1 / 14.2 / 14.3 / 14.7 /
-// 15.0 -> 12.7 / 12.8 / 13.0 / 13.6 / 14.0 us (with 36 instead of 12 bytes of registers spilled). An instantiation of its own: with
+// 15.0 -> 12.7 / 12.8 / 13.0 / 13.6 / 14.0 us. The LayerNorm of its tile is shared by the LayerNorm warps and the first row group,
+// four rows per half warp instead of eight in two turns, each of which waited for its loads (N = 37, four pair blocks: 349 -> 344). An instantiation of its own: with
 // the choice made in the kernel N = 768 took 241 instead of 224 us (registers).
 template <bool kSolo>
 __global__ void __launch_bounds__(kTrThreads, 1)
@@ -139,7 +199,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
         for (int i = 0; i < 3; ++i) {
             mbar_init(x_empty(i), 1);
-            mbar_init(a_ready(i), 8);
+            mbar_init(a_ready(i), kSolo ? 16 : 8);
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -298,7 +358,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             }
             tma_store_wait_all<0>();
         }
-    } else if (warp < 12) {
+    } else if (!kSolo && warp < 12) {
         // ---------------------------------------------------------------- LayerNorm: 16 rows per warp and tile
         // A half warp reads a row (coalesced), so that a thread holds 8 channels of 8 rows; see row_sums.
         const int ch = lane & 15, sub = lane >> 4;
@@ -310,57 +370,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             const __nv_bfloat16* src = x + base * kC + ch * 8;
             const int left = (int)min(rows - base, 16LL);   // rows 0, 2, ... 14 from here; the tensor may end before
             uint32_t raw[32];
-#pragma unroll
-            for (int h = 0; h < 8; h += 4) {   // four rows at a time (registers)
-                float mean[4], rstd[4];
-                asm volatile("" ::: "memory");
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (2 * (h + r) < left) v = *reinterpret_cast<const uint4*>(src + 2 * (h + r) * kC);
-                    uint32_t* o = &raw[(h + r) * 4];
-                    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-                }
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    float a = 0.f, b = 0.f;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) { a = add_lo(raw[(h + r) * 4 + i], a); b = add_hi(raw[(h + r) * 4 + i], b); }
-                    mean[r] = a + b;
-                }
-                row_sums(mean, lane);
-                opaque(raw, h * 4);   // unpack again rather than keep 32 floats
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    mean[r] *= 1.0f / kC;
-                    float a = 0.f, b = 0.f;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float x0 = add_lo(raw[(h + r) * 4 + i], -mean[r]), x1 = add_hi(raw[(h + r) * 4 + i], -mean[r]);
-                        a = fmaf(x0, x0, a);
-                        b = fmaf(x1, x1, b);
-                    }
-                    rstd[r] = a + b;
-                }
-                row_sums(rstd, lane);
-                opaque(raw, h * 4);
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    rstd[r] = rsqrtf(rstd[r] * (1.0f / kC) + kLnEps);
-                    mean[r] *= -rstd[r];
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 ga = *reinterpret_cast<const float2*>(prm + ch * 8 + i * 2);
-                    const float2 be = *reinterpret_cast<const float2*>(prm + 128 + ch * 8 + i * 2);
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        uint32_t& v = raw[(h + r) * 4 + i];
-                        v = pack_bf16x2(fmaf(fmaf(bf16lo(v), rstd[r], mean[r]), ga.x, be.x),
-                                        fmaf(fmaf(bf16hi(v), rstd[r], mean[r]), ga.y, be.y));
-                    }
-                }
-            }
+            normalize_rows<8>(src, left, ch, lane, prm, raw);
             if (!mbar_wait(x_empty(buf), (use & 1u) ^ 1u, abort_flag)) {
                 if (lane == 0) report_wait_failure(status, abort_flag, kKidTrans, 8);
                 break;
@@ -375,6 +385,22 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
     } else {
         // ---------------------------------------------------------------- two row groups
+        if constexpr (kSolo) {
+            // the tile's LayerNorm, eight rows per warp: by the LayerNorm warps and the first row group, which has no row yet
+            if (warp < 20) {
+                const int ch = lane & 15, row0 = (warp - 4) * 8 + (lane >> 4);
+                const long long base = blockIdx.x * (long long)kRows + row0;
+                uint32_t raw[16];
+                normalize_rows<4>(x + base * kC + ch * 8, (int)min(rows - base, 8LL), ch, lane, prm, raw);
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    sts128(chunk_addr(sbase + TrSmem::kX, row0 + 2 * r, ch),
+                           make_uint4(raw[r * 4], raw[r * 4 + 1], raw[r * 4 + 2], raw[r * 4 + 3]));
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(a_ready(0));
+            }
+        }
         const int own = (warp - 12) >> 3;      // group of these warps
         const int g = solo ? 0 : own;          // group whose tile they work on
         const int quad = warp & 3;
@@ -382,7 +408,7 @@ transition_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         const int row = quad * 32 + lane;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16);
         const uint32_t t_d2 = t_lane + g * 256 + 128;
-        bool ok = true;
+        bool ok = !kSolo || warp >= 12;
         uint32_t ppar = 0;
         int buf = g;
         for (int t = g; t < my_tiles && ok; t += 2, ppar ^= 1u) {
