@@ -48,6 +48,7 @@ extern "C" {
 #define OF3_FLAG_TRANSPOSED 8  /* triangle attention around the ending node */
 #define OF3_FLAG_ADA_LN 16     /* attention pair bias: adaptive LayerNorm conditioning on s */
 #define OF3_FLAG_CONTINUES 64  /* blocks: see of3_pair_block_forward */
+#define OF3_FLAG_LAST 128      /* of3_pairformer_block_forward: no block follows whose pair stack the single track would run beside */
 #define OF3_FLAG_NO_TRANSITION_MASK 32 /* blocks: the transitions ignore the mask (_mask_trans = False) */
 
 /* Message for the last non-zero return code seen by the calling thread. */
@@ -236,7 +237,8 @@ int of3_cond_transition_forward(const void* a, const void* s, const void* mask, 
  * projection has a kernel of its own: c_z = 128, 16 heads) the single track runs on side_stream behind the pair stack
  * of the same block, so that it overlaps the pair stack of the next block: the caller makes side_stream wait for
  * stream before the first block and stream wait for side_stream after the last one (of3_stream_wait), and gives the
- * single track a workspace of its own. */
+ * single track a workspace of its own. OF3_FLAG_LAST tells that no block follows: the single track then takes launches
+ * that spread over the chip. */
 typedef struct {
     of3_trimul_params tri_mul_out, tri_mul_in;
     of3_triattn_params tri_att_start, tri_att_end;

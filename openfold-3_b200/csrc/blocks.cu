@@ -86,7 +86,7 @@ int project_bias(const void* z, void* bias, const of3_block_dims& D, BiasForm fo
 
 int single_track(void* s, const void* z, const void* bias, BiasForm form, const void* mask, const of3_block_dims& D,
                  int dtype, int flags, const of3_pairformer_block_params* p, Scratch& ws, cudaStream_t st) {
-    const int f = (flags & OF3_FLAG_FORCE_GENERIC) | OF3_FLAG_ADD_RESIDUAL;
+    const int f = (flags & (OF3_FLAG_FORCE_GENERIC | fast::kFlagBeside)) | OF3_FLAG_ADD_RESIDUAL;
     int rc = ws.run([&](Arena& a) {
         if (form == kBiasTiles)
             return fast::attn_pair_bias((const __nv_bfloat16*)s, nullptr, nullptr, (const __nv_bfloat16*)mask,
@@ -331,7 +331,8 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
     if ((rc = stream_wait(main, side))) return rc;
     if ((rc = project_bias(z, bias, *dims, form, &p->attn, main))) return rc;
     if ((rc = stream_wait(side, main))) return rc;
-    return single_track(s, nullptr, bias, form, single_mask, *dims, dtype, flags, p, ws_side, side);
+    const int beside = (flags & OF3_FLAG_LAST) ? 0 : fast::kFlagBeside;
+    return single_track(s, nullptr, bias, form, single_mask, *dims, dtype, flags | beside, p, ws_side, side);
 }
 
 size_t of3_diffusion_stack_workspace_bytes(const of3_diffusion_dims* dims, int dtype, int flags, int blocks,

@@ -284,6 +284,10 @@ int linear_bf16(const bf16* x, const bf16* w, bf16* y, long long rows, int out_d
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+// Launches for few tokens fill the chip with short blocks. Beside a pair stack (kFlagBeside) each of these makes a block of it late,
+// while a pair stack of few tokens leaves SMs idle. Trunk of four blocks, us, 128-row tiles in all blocks / in all but the last / in
+// none: N = 24 408 / - / 399, 37 411 / - / 406, 64 417 / - / 409, 80 442 / 436 / 449, 96 450 / 444 / 458, 128 473 / 467 / 485.
+bool alone(long long rows, int flags) { return !(flags & kFlagBeside) || rows <= kBesideRows; }
 bool even(const void* p) { return ((uintptr_t)p & 3) == 0; }   // pairs of channels
 
 }  // namespace
@@ -372,7 +376,7 @@ int attn_pair_bias(const bf16* a, const bf16* z, const bf16* s, const bf16* mask
                           {(const bf16*)p->w_q, (const bf16*)p->w_g, (const bf16*)p->w_k, (const bf16*)p->w_v}, 4};
         const LinearOut kinds[4] = {kOutQ, kOutG, kOutK, kOutV};
         const AttnImages images{im.q, im.k, im.v, g, (const bf16*)p->b_q, N, H, d};
-        const bool few = token_images_supported(Ba, N, c_a, d);
+        const bool few = token_images_supported(Ba, N, c_a, d) && alone(rows, flags);
         if ((rc = (few ? token_attn_images : linear_attn_images)(in, kinds, images, st))) return rc;
     }
     SingleBias bias;
@@ -384,7 +388,7 @@ int attn_pair_bias(const bf16* a, const bf16* z, const bf16* s, const bf16* mask
     bias.w = (const bf16*)p->w_z;
     if ((rc = single_attn(im, g, bias, tb, mask, og, Ba, N, N, H, d, inf, Ba / Bz, st))) return rc;
     const LinearIn in{og, rows, c_a, c_a, {(const bf16*)p->w_o}, 1};
-    const bool few = token_residual_supported(rows, c_a) && even(a) && even(out);
+    const bool few = token_residual_supported(rows, c_a) && alone(rows, flags) && even(a) && even(out);
     return (few ? token_residual : linear_residual)(in, (flags & OF3_FLAG_ADD_RESIDUAL) ? a : nullptr,
                                                     ada ? cond + 2 * rows * c_a : nullptr, (const bf16*)p->b_ada_out, nullptr, out,
                                                     st);
@@ -468,9 +472,10 @@ int transition_wide(const bf16* x, const bf16* mask, bf16* out, long long rows, 
     int rc;
     if ((rc = ln_rows(x, (const bf16*)p->ln_w, (const bf16*)p->ln_b, xn, rows, c, st))) return rc;
     const LinearIn up{xn, rows, c, hid, {(const bf16*)p->w_a, (const bf16*)p->w_b}, 2};
-    if ((rc = linear_swiglu(up, h, st))) return rc;
+    if ((rc = (token_swiglu_supported(rows, hid) && alone(rows, flags) ? token_swiglu : linear_swiglu)(up, h, st))) return rc;
     const LinearIn down{h, rows, hid, c, {(const bf16*)p->w_out}, 1};
-    return linear_residual(down, (flags & OF3_FLAG_ADD_RESIDUAL) ? x : nullptr, nullptr, nullptr, mask, out, st);
+    const bool few = token_residual_supported(rows, c) && alone(rows, flags) && even(x) && even(out);
+    return (few ? token_residual : linear_residual)(down, (flags & OF3_FLAG_ADD_RESIDUAL) ? x : nullptr, nullptr, nullptr, mask, out, st);
 }
 
 }  // namespace fast

@@ -5,6 +5,10 @@
 namespace of3 {
 namespace fast {
 
+// Internal flag of the single-track layers, beside the public ones: other kernels run at the same time (the next block's pair stack).
+constexpr int kFlagBeside = 1 << 20;
+constexpr int kBesideRows = 64;
+
 // The three projections of the conditioning s that an AdaLN layer needs, planes [3][rows][c_a]: gate and shift of the
 // adaptive LayerNorm (without the gate's bias), output gate (without its bias).
 struct CondLayer {

@@ -36,7 +36,6 @@ constexpr int kThreads = 32 * (2 + 4 * kParts);
 constexpr int kGroup = 3;            // k-blocks of a stage
 constexpr int kMaxStages = 8;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kD = 48;               // channels per head
 
 enum Epi { kImages, kSwiglu, kResidual };
 
@@ -81,7 +80,8 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[N]) {
     else tmem_ld4(taddr, r);
 }
 
-template <int BF, int NT, int EPI>
+// D: channels per head (kImages)
+template <int BF, int NT, int EPI, int D>
 __global__ void __launch_bounds__(kThreads, 1)
 token_linear_kernel(const __grid_constant__ TokMaps maps, const TokArgs ar, int rows, int K, int n, int tok_tiles,
                     int* status) {
@@ -284,13 +284,14 @@ token_linear_kernel(const __grid_constant__ TokMaps maps, const TokArgs ar, int 
             } else {
                 static_assert(EPI != kImages || BF == 128, "lanes of the tile");
                 const AttnImages& im = ar.im;
-                const int kind = ar.kind[g], HD = im.H * kD;
+                constexpr int KD = SingleImage<D>::kKD, DV = SingleImage<D>::kDV;
+                const int kind = ar.kind[g], HD = im.H * D;
                 const int nkb = (ns + kSingleBK - 1) / kSingleBK, n_qt = (ns + kSingleBQ - 1) / kSingleBQ;
                 const int f = nt * kOut + quad * 32 + lane;   // channel, in its matrix
-                const int h = f / kD, d = f - h * kD;
+                const int h = f / D, d = f - h * D;
                 const long long bh = (long long)bb * im.H + h;
                 if (kind == kOutV) {
-                    // tile [48 channels][32 keys], 64-byte rows: this channel's keys, a chunk of eight (or half a one) at a time;
+                    // tile [DV channels][32 keys], 64-byte rows: this channel's keys, a chunk of eight (or half a one) at a time;
                     // keys past the end of the last block are zeros
                     constexpr int kRun = kTok < 8 ? kTok : 8;
 #pragma unroll
@@ -301,7 +302,7 @@ token_linear_kernel(const __grid_constant__ TokMaps maps, const TokArgs ar, int 
 #pragma unroll
                         for (int e = 0; e < kRun; e += 2)
                             o[e / 2] = pack_bf16x2(p + e < ns ? v[i + e] : 0.f, p + e + 1 < ns ? v[i + e + 1] : 0.f);
-                        bf16* t = im.v + ((bh * nkb + (p >> 5)) * kD + d) * kSingleBK +
+                        bf16* t = im.v + ((bh * nkb + (p >> 5)) * DV + d) * kSingleBK +
                                   (((((p & 31) >> 3) ^ ((d >> 1) & 3)) << 3) | (p & 7));
                         if constexpr (kRun == 8) *reinterpret_cast<uint4*>(t) = make_uint4(o[0], o[1], o[2], o[3]);
                         else *reinterpret_cast<uint2*>(t) = make_uint2(o[0], o[1]);
@@ -309,8 +310,10 @@ token_linear_kernel(const __grid_constant__ TokMaps maps, const TokArgs ar, int 
                 } else {
                     const float qb = kind == kOutQ && im.q_bias ? __bfloat162float(im.q_bias[f]) : 0.f;
                     const int dp = d & ~1;   // (an even channel and the next one lie in one head and chunk)
-                    uint8_t* const q = reinterpret_cast<uint8_t*>(im.q) + bh * n_qt * (long long)(kSingleBQ * 128);
-                    uint8_t* const k = reinterpret_cast<uint8_t*>(im.k) + bh * nkb * (long long)(kSingleBK * 128);
+                    constexpr int kRow = KD * 2;   // bytes of an image's row
+                    const bool last = D < KD && D <= 32 && dp >= D - 8;   // 24 channels: chunk 3 of the row pads K with zeros
+                    uint8_t* const q = reinterpret_cast<uint8_t*>(im.q) + bh * n_qt * (long long)(kSingleBQ * kRow);
+                    uint8_t* const k = reinterpret_cast<uint8_t*>(im.k) + bh * nkb * (long long)(kSingleBK * kRow);
 #pragma unroll
                     for (int i = 0; i < kTok; i += 2) {
                         float v0 = v[i], v1 = v[i + 1];
@@ -324,13 +327,18 @@ token_linear_kernel(const __grid_constant__ TokMaps maps, const TokArgs ar, int 
                         }
                         const uint32_t o = pair_channels(v0, v1, lane);
                         const int p = tok + i + (lane & 1);
-                        const uint32_t in_row = single_chunk_off<64>(p & 7, dp >> 3) - (p & 7) * 128 + (dp & 7) * 2;
+                        auto in_row = [&](int c) {   // chunk c of row p, from the row's start
+                            return single_chunk_off<KD>(p & 7, c) - (p & 7) * kRow + (dp & 7) * 2;
+                        };
                         if (kind == kOutG) {
                             if (p < ns) *reinterpret_cast<uint32_t*>(im.g + ((long long)bb * ns + p) * HD + (f & ~1)) = o;
-                        } else if (kind == kOutQ) {   // tiles of 128 rows of 128 bytes, one behind the other
-                            if (p < ns) *reinterpret_cast<uint32_t*>(q + (long long)p * 128 + in_row) = o;
-                        } else {                      // and of 32
-                            if (p < nkb * kSingleBK) *reinterpret_cast<uint32_t*>(k + (long long)p * 128 + in_row) = p < ns ? o : 0u;
+                        } else {   // tiles of 128 (32) rows, one behind the other
+                            const bool is_q = kind == kOutQ;
+                            uint8_t* const row = (is_q ? q : k) + (long long)p * kRow;
+                            if (p < (is_q ? ns : nkb * kSingleBK)) {
+                                *reinterpret_cast<uint32_t*>(row + in_row(dp >> 3)) = p < ns ? o : 0u;
+                                if (last) *reinterpret_cast<uint32_t*>(row + in_row((dp >> 3) + 1)) = 0u;
+                            }
                         }
                     }
                 }
@@ -347,7 +355,7 @@ token_linear_kernel(const __grid_constant__ TokMaps maps, const TokArgs ar, int 
     }
 }
 
-template <int BF, int NT, int EPI>
+template <int BF, int NT, int EPI, int D>
 int launch(const TokArgs& ar, const LinearIn& in, int tok_tiles, int grid, cudaStream_t st) {
     using C = Cfg<BF, NT>;
     TokMaps maps;
@@ -368,26 +376,26 @@ int launch(const TokArgs& ar, const LinearIn& in, int tok_tiles, int grid, cudaS
     constexpr int smem = C::kStages * C::kStageBytes + C::kFixed;
     static PerDeviceOnce configured;
     if (!configured.done()) {
-        OF3_CUDA_CHECK(cudaFuncSetAttribute(token_linear_kernel<BF, NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(token_linear_kernel<BF, NT, EPI, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured.mark();
     }
     LaunchScope scope(kKid, st);
-    OF3_CUDA_CHECK(launch_chained(token_linear_kernel<BF, NT, EPI>, grid, kThreads, smem, st, maps, ar, (int)in.rows, in.k, in.n,
+    OF3_CUDA_CHECK(launch_chained(token_linear_kernel<BF, NT, EPI, D>, grid, kThreads, smem, st, maps, ar, (int)in.rows, in.k, in.n,
                                   tok_tiles, device_status_ptr()));
     return OF3_OK;
 }
 
 // Tokens per tile: the fewest that one wave of CTAs covers, since a tile's loads and epilogue grow with them and its products
 // hardly do. `samples`: tiles lie in one sample each.
-template <int BF, int EPI>
+template <int BF, int EPI, int D = 0>
 int by_tokens(const TokArgs& ar, const LinearIn& in, int samples, int channel_tiles, cudaStream_t st) {
     // (kImages: whole key blocks of 32, of which the tiles write the end as zeros)
     const int ns = EPI == kImages ? ((int)(in.rows / samples) + 31) / 32 * 32 : (int)in.rows;
     auto tiles = [&](int nt) { return samples * ((ns + nt - 1) / nt); };
     auto fits = [&](int nt) { return tiles(nt) * channel_tiles <= sm_count(); };
-    if (fits(16)) return launch<BF, 16, EPI>(ar, in, tiles(16), tiles(16) * channel_tiles, st);
-    if (fits(32)) return launch<BF, 32, EPI>(ar, in, tiles(32), tiles(32) * channel_tiles, st);
-    return launch<BF, 64, EPI>(ar, in, tiles(64), tiles(64) * channel_tiles, st);
+    if (fits(16)) return launch<BF, 16, EPI, D>(ar, in, tiles(16), tiles(16) * channel_tiles, st);
+    if (fits(32)) return launch<BF, 32, EPI, D>(ar, in, tiles(32), tiles(32) * channel_tiles, st);
+    return launch<BF, 64, EPI, D>(ar, in, tiles(64), tiles(64) * channel_tiles, st);
 }
 
 }  // namespace
@@ -398,7 +406,7 @@ static bool one_wave(long long samples, long long tokens, int channel_tiles) {
     return samples * ((tokens + 63) / 64) * channel_tiles <= sm_count();
 }
 bool token_images_supported(int samples, int tokens, int c, int d) {
-    return c % 128 == 0 && d == kD && one_wave(samples, tokens, 4 * c / 128);
+    return c % 128 == 0 && (d == 24 || d == 48) && one_wave(samples, tokens, 4 * c / 128);
 }
 bool token_swiglu_supported(long long rows, int hidden) { return hidden % 64 == 0 && one_wave(1, rows, hidden / 64); }
 bool token_residual_supported(long long rows, int c) { return c % 64 == 0 && one_wave(1, rows, c / 64); }
@@ -408,7 +416,8 @@ int token_attn_images(const LinearIn& in, const LinearOut* kinds, const AttnImag
     ar.im = im;
     for (int i = 0; i < in.num_w; ++i) ar.kind[i] = kinds[i];
     ar.qscale = kLog2e * (1.0f / sqrtf((float)im.D));
-    return by_tokens<128, kImages>(ar, in, (int)(in.rows / im.rows_per_sample), in.n / 128 * in.num_w, st);
+    const int samples = (int)(in.rows / im.rows_per_sample), tiles = in.n / 128 * in.num_w;
+    return im.D == 24 ? by_tokens<128, kImages, 24>(ar, in, samples, tiles, st) : by_tokens<128, kImages, 48>(ar, in, samples, tiles, st);
 }
 
 int token_swiglu(const LinearIn& in, bf16* h, cudaStream_t st) {

@@ -795,9 +795,9 @@ class PairFormerBlock(_Planned):
         d.single_transition_n, d.inf_single = self.single_transition.n, a.inf
         return lib.BlockPlan(d, dtype, flags, single=True)
 
-    def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None, continues=False):
+    def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None, continues=False, last=True):
         """In place on contiguous s and z with prepared masks; False if the native path does not take this call.
-        ``continues``: the last work on the stream is another block's native call."""
+        ``continues``: the last work on the stream is another block's native call; ``last``: no block follows."""
         plan = _native_state(self, z)
         B = None if plan is None else _pair_batch(z, plan.c_z)
         if B is None or s.dtype != z.dtype or s.shape != (*z.shape[:-2], plan.c_s):
@@ -806,6 +806,8 @@ class PairFormerBlock(_Planned):
         shape = plan.shape(self, B, z.shape[-2], plan.code, flags)
         if continues and plan.called:
             flags |= lib.FLAG_CONTINUES
+        if last:
+            flags |= lib.FLAG_LAST
         plan.called = True
         lib.pairformer_block_forward(s, z, single_mask, pair_mask, shape, plan.code, flags, plan.params, side)
         return True
@@ -881,7 +883,8 @@ class PairFormerStack(nn.Module):
         native = False
         try:
             for b in self.blocks:
-                native = b._run_native(s, z, single_mask, pair_mask, _mask_trans, side, continues=native)
+                native = b._run_native(s, z, single_mask, pair_mask, _mask_trans, side, continues=native,
+                                       last=b is self.blocks[-1])
                 if native:
                     continue
                 z = b.pair_stack(z=z, pair_mask=pair_mask, chunk_size=chunk_size, inplace_safe=True,

@@ -85,3 +85,25 @@ def test_few_tokens_equal_rows_of_a_larger_call(N, samples):
         got = blk(a[:, :samples].contiguous(), s[:, :samples].contiguous(), z, mask=m)
     pkg.lib.check_device_status()
     assert torch.isfinite(got).all() and got.any() and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("N,samples", [(1, 2), (7, 1), (16, 1), (33, 2), (64, 1), (100, 1), (129, 2), (500, 1), (768, 1)])
+def test_few_tokens_of_the_single_track(N, samples):
+    """The same for the attention of the trunk's single track (16 heads of 24, whose images pad k to 32)."""
+    g = torch.Generator().manual_seed(N)
+    layer = pkg.AttentionPairBias(c_q=384, c_k=384, c_v=384, c_s=None, c_z=128, c_hidden=24, no_heads=16)
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.copy_(torch.randn(p.shape, generator=g) * (0.05 if p.dim() > 1 else 0.3) + (1.0 if p.dim() == 1 else 0.0))
+    layer = layer.to("cuda:0", torch.bfloat16).eval().requires_grad_(False)
+    many = max(samples + 1, -(-1700 // N)) if N > 12 else 200   # more tiles than one wave takes
+    a = torch.randn(many, N, 384, generator=g).to("cuda:0", torch.bfloat16)
+    z = torch.randn(samples, N, N, 128, generator=g).to("cuda:0", torch.bfloat16)
+    z = torch.cat([z, z[:1].expand(many - samples, -1, -1, -1)])
+    m = (torch.rand(many, N, generator=g) < 0.9).to("cuda:0", torch.bfloat16)
+    m[:, 0] = 1
+    with torch.no_grad():
+        want = layer(a, z, mask=m)[:samples]
+        got = layer(a[:samples].contiguous(), z[:samples].contiguous(), mask=m[:samples].contiguous())
+    pkg.lib.check_device_status()
+    assert torch.isfinite(got).all() and got.any() and torch.equal(got, want)
