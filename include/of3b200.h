@@ -49,6 +49,7 @@ extern "C" {
 #define OF3_FLAG_ADA_LN 16     /* attention pair bias: adaptive LayerNorm conditioning on s */
 #define OF3_FLAG_CONTINUES 64  /* blocks: see of3_pair_block_forward */
 #define OF3_FLAG_LAST 128      /* of3_pairformer_block_forward: no block follows whose pair stack the single track would run beside */
+#define OF3_FLAG_BIAS_SLOT(k) ((k) << 8) /* of3_pairformer_block_forward, k = 0 .. 3 */
 #define OF3_FLAG_NO_TRANSITION_MASK 32 /* blocks: the transitions ignore the mask (_mask_trans = False) */
 
 /* Message for the last non-zero return code seen by the calling thread. */
@@ -238,7 +239,10 @@ int of3_cond_transition_forward(const void* a, const void* s, const void* mask, 
  * of the same block, so that it overlaps the pair stack of the next block: the caller makes side_stream wait for
  * stream before the first block and stream wait for side_stream after the last one (of3_stream_wait), and gives the
  * single track a workspace of its own. OF3_FLAG_LAST tells that no block follows: the single track then takes launches
- * that spread over the chip. */
+ * that spread over the chip. OF3_FLAG_BIAS_SLOT(k): which of the workspace's rooms for the projected pair bias this block
+ * takes (where it has four; else the first). Before it takes the first one, stream waits for side_stream, whose last single
+ * track may still read it; before the others it does not: they belong to the second to fourth block of a run whose first
+ * took slot 0, or to the first blocks after stream has waited for side_stream. */
 typedef struct {
     of3_trimul_params tri_mul_out, tri_mul_in;
     of3_triattn_params tri_att_start, tri_att_end;

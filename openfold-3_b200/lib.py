@@ -20,6 +20,7 @@ LIB_PATH = Path(__file__).resolve().parent / "libof3b200.so"
 DTYPE_BF16, DTYPE_F32 = 0, 1
 FLAG_ADD_RESIDUAL, FLAG_FORCE_GENERIC, FLAG_OUTGOING, FLAG_TRANSPOSED, FLAG_ADA_LN = 1, 2, 4, 8, 16
 FLAG_NO_TRANSITION_MASK, FLAG_CONTINUES, FLAG_LAST = 32, 64, 128
+BIAS_SLOTS, BIAS_SLOT_SHIFT = 4, 8   # FLAG_BIAS_SLOT(k) = k << BIAS_SLOT_SHIFT
 MODULE_TRIMUL, MODULE_TRIATTN, MODULE_TRANSITION = 1, 2, 3
 
 _lib = None

@@ -795,9 +795,10 @@ class PairFormerBlock(_Planned):
         d.single_transition_n, d.inf_single = self.single_transition.n, a.inf
         return lib.BlockPlan(d, dtype, flags, single=True)
 
-    def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None, continues=False, last=True):
+    def _run_native(self, s, z, single_mask, pair_mask, mask_trans, side=None, continues=False, last=True, run=0):
         """In place on contiguous s and z with prepared masks; False if the native path does not take this call.
-        ``continues``: the last work on the stream is another block's native call; ``last``: no block follows."""
+        ``continues``: the last work on the stream is another block's native call; ``last``: no block follows;
+        ``run``: native calls of the stack before this one (its room for the pair bias: 1, 2, 3, 0, ... in turn)."""
         plan = _native_state(self, z)
         B = None if plan is None else _pair_batch(z, plan.c_z)
         if B is None or s.dtype != z.dtype or s.shape != (*z.shape[:-2], plan.c_s):
@@ -808,6 +809,8 @@ class PairFormerBlock(_Planned):
             flags |= lib.FLAG_CONTINUES
         if last:
             flags |= lib.FLAG_LAST
+        if side is not None:
+            flags |= (run + 1) % lib.BIAS_SLOTS << lib.BIAS_SLOT_SHIFT
         plan.called = True
         lib.pairformer_block_forward(s, z, single_mask, pair_mask, shape, plan.code, flags, plan.params, side)
         return True
@@ -880,12 +883,13 @@ class PairFormerStack(nn.Module):
         main = torch.cuda.current_stream(z.device)
         side = lib.side_stream(main)
         lib.stream_wait(side, main)
-        native = False
+        native, run = False, 0
         try:
             for b in self.blocks:
                 native = b._run_native(s, z, single_mask, pair_mask, _mask_trans, side, continues=native,
-                                       last=b is self.blocks[-1])
+                                       last=b is self.blocks[-1], run=run)
                 if native:
+                    run += 1
                     continue
                 z = b.pair_stack(z=z, pair_mask=pair_mask, chunk_size=chunk_size, inplace_safe=True,
                                  _mask_trans=_mask_trans)
