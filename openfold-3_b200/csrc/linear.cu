@@ -188,10 +188,16 @@ __device__ __forceinline__ void store_images(const AttnImages& im, int kind, flo
     }
 }
 
+// A last wave of 256-wide tiles that takes at most half of the SMs runs as twice as many tiles of half the columns: a half tile takes
+// about 0.6 of a whole one, whose time the wave otherwise costs. A step of 24 blocks whose wave has 64 tiles (5 x 768 tokens) 2959 ->
+// 2920 us, 36 (5 x 1024) 4287 -> 4234, 20 (5 x 350) 1833 -> 1798; fuller waves stay whole and as fast (92 tiles, 5 x 500: 2231).
+template <int BN, int EPI>
+__host__ __device__ constexpr bool has_halves() { return BN == 256 && (EPI == kEpiImages || EPI == kEpiSwiglu); }
+
 template <int BN, int EPI, int D>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, StagedMaps, LinMaps> maps, const EpiArgs ep,
-              long long rows, int K, int n, int num_mats, int* status) {
+              long long rows, int K, int n, int num_mats, int whole_tiles, int* status) {
     using Cfg = LinCfg<BN, EPI>;
     constexpr int S = Cfg::kStages;
     constexpr int kWRows = EPI == kEpiSwiglu ? BN / 2 : BN;   // rows of each weight matrix in a tile
@@ -213,11 +219,19 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
     // kEpiSwiglu: matrices 0 and 1 share a tile; otherwise a tile lies inside one matrix
     const int num_nt = EPI == kEpiSwiglu ? nt_per_mat : nt_per_mat * num_mats;
     const int num_kb = K / kBK;
-    const int num_tiles = num_mt * num_nt;
-    // a tile: row tile mt (innermost: concurrent CTAs share the weight panel), matrix g, column tile inside it
-    struct Tile { int mt, g, nt; };
+    // The tiles from whole_tiles on come in two halves of their columns (kHalves)
+    constexpr bool kHalves = has_halves<BN, EPI>();
+    const int num_tiles = kHalves ? 2 * num_mt * num_nt - whole_tiles : num_mt * num_nt;
+    // a tile: row tile mt (innermost: concurrent CTAs share the weight panel), matrix g, column tile inside it; which half
+    struct Tile { int mt, g, nt, half; bool whole; };
     auto tile_of = [&](int t) {
         Tile c;
+        c.whole = !kHalves || t < whole_tiles;
+        c.half = 0;
+        if (!c.whole) {
+            c.half = (t - whole_tiles) & 1;
+            t = whole_tiles + ((t - whole_tiles) >> 1);
+        }
         c.mt = t % num_mt;
         const int q = t / num_mt;
         c.g = EPI == kEpiSwiglu ? 0 : q / nt_per_mat;
@@ -255,7 +269,13 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
         if (elect_one()) {
             auto load_w = [&](const Tile& c, int kb, int s) {
                 const uint32_t sw = sbase + s * Cfg::kStageBytes + Cfg::kABytes;
-                if constexpr (EPI == kEpiSwiglu) {
+                if constexpr (kHalves) {   // boxes of half a tile's rows
+                    const int mats = EPI == kEpiSwiglu ? 2 : 1, boxes = c.whole ? 2 : 1;
+                    for (int m = 0; m < mats; ++m)
+                        for (int b = 0; b < boxes; ++b)
+                            tma_load_2d(sw + (m * boxes + b) * (kWRows / 2) * 128, &maps.w[EPI == kEpiSwiglu ? m : c.g], full(s), kb * kBK,
+                                        c.nt * kWRows + (b + c.half) * (kWRows / 2));
+                } else if constexpr (EPI == kEpiSwiglu) {
                     tma_load_2d(sw, &maps.w[0], full(s), kb * kBK, c.nt * kWRows);
                     tma_load_2d(sw + kWRows * 128, &maps.w[1], full(s), kb * kBK, c.nt * kWRows);
                 } else if constexpr (EPI == kEpiStore) {
@@ -272,7 +292,7 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
             const Tile first = tile_of(blockIdx.x);
             const int ahead = num_kb < S ? num_kb : S;
             for (int kb = 0; kb < ahead; ++kb) {
-                mbar_arrive_expect_tx(full(kb), Cfg::kStageBytes);
+                mbar_arrive_expect_tx(full(kb), Cfg::kStageBytes);   // (a CTA's first tile is a whole one)
                 load_w(first, kb, kb);
             }
             grid_wait();
@@ -289,7 +309,7 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
                         ok = false;
                         break;
                     }
-                    mbar_arrive_expect_tx(full(s), Cfg::kStageBytes);
+                    mbar_arrive_expect_tx(full(s), c.whole ? Cfg::kStageBytes : Cfg::kABytes + BN / 2 * kBK * 2);
                     load_a(c, kb, s);
                     load_w(c, kb, s);
                 }
@@ -298,7 +318,6 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
         if (elect_one()) {
-            constexpr uint32_t idesc = idesc_bf16_f32(kBM, BN);
             uint32_t it = 0, tc = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tc) {
@@ -309,6 +328,7 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
                 }
                 tc_fence_after_sync();
                 const uint32_t d = tmem_base + acc * Cfg::kAccStride;
+                const uint32_t idesc = !kHalves || t < whole_tiles ? idesc_bf16_f32(kBM, BN) : idesc_bf16_f32(kBM, BN / 2);
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % S;
                     if (!mbar_wait(full(s), (it / S) & 1u, abort_flag)) {
@@ -359,7 +379,8 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
             const uint32_t acc = tc & 1u;
             const long long row = (long long)c.mt * kBM + quad * 32 + lane;
             const bool live = row < rows;
-            const int colb = c.nt * kWRows + part * kCols;   // first column of this thread, inside the matrix
+            const int cols = c.whole ? kCols : kCols / 2;
+            const int colb = c.nt * kWRows + c.half * (kWRows / 2) + part * cols;   // first column of this thread, inside the matrix
             // The gate and residual values of the tile, all of them on their way under its GEMM: fetched 16 columns at a time
             // between the TMEM loads, their latency was what a tile took (six times 1 us at BN = 192)
             constexpr int kPre = EPI == kEpiResidual ? kCols / 16 : 1;
@@ -414,18 +435,19 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
             }
             if (EPI != kEpiStaged && !ok) break;
             tc_fence_after_sync();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * Cfg::kAccStride + part * kCols;
+            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * Cfg::kAccStride + part * cols;
+            const uint32_t second = c.whole ? BN / 2 : BN / 4;   // kEpiSwiglu: the other matrix' columns
             [[maybe_unused]] int bb = 0, pos = 0;   // sample and position of the row
             if constexpr (EPI == kEpiImages) {
                 bb = (int)((uint32_t)row / (uint32_t)ep.im.rows_per_sample);
                 pos = (int)row - bb * ep.im.rows_per_sample;
             }
 #pragma unroll(EPI == kEpiResidual ? kPre : (EPI == kEpiStaged ? kCols / 16 : 1))
-            for (int c0 = 0; c0 < kCols; c0 += 16) {
+            for (int c0 = 0; c0 < (kHalves ? cols : kCols); c0 += 16) {
                 if (EPI == kEpiStaged && !ok) break;
                 uint32_t r[16], r2[16];
                 tmem_ld16(taddr + c0, r);
-                if constexpr (EPI == kEpiSwiglu) tmem_ld16(taddr + BN / 2 + c0, r2);
+                if constexpr (EPI == kEpiSwiglu) tmem_ld16(taddr + second + c0, r2);
                 tmem_ld_wait();
                 const int col = colb + c0;
                 if (EPI != kEpiResidual && EPI != kEpiStaged && !live) continue;   // (its gate biases are shared by shuffles)
@@ -523,7 +545,8 @@ linear_kernel(const __grid_constant__ std::conditional_t<EPI == kEpiStaged, Stag
 
 // Column tile: the number of waves of 148 CTAs times the panels a tile streams (128 rows of x and BN of the weights per
 // k-block, plus a constant for its fill and epilogue). Wide tiles move fewer bytes, narrow ones fill the chip when there
-// are few rows; a BN that does not divide the matrix is out.
+// are few rows; a BN that does not divide the matrix is out. (A last wave of halves counted as one of half the width picks 256
+// where 192 ties: 5 x 350, 4 x 500 and 5 x 450 tokens within 0.2% of each other.)
 int pick_bn(long long rows, int n, int mats, bool swiglu, int widest = 256) {
     const long long sms = sm_count(), mt = (rows + kBM - 1) / kBM;
     const int cand[4] = {256, 192, 128, 64};
@@ -558,7 +581,7 @@ int launch(const LinearIn& in, const EpiArgs& ep, int slices, int w_rows, cudaSt
     for (int i = 0; i < tensors; ++i) {
         uint64_t dims[2] = {(uint64_t)in.k, (uint64_t)w_rows};
         uint64_t str[1] = {(uint64_t)in.k * 2};
-        uint32_t box[2] = {kBK, (uint32_t)kWRows};
+        uint32_t box[2] = {kBK, (uint32_t)(has_halves<BN, EPI>() ? kWRows / 2 : kWRows)};
         if ((rc = make_tmap_bf16(&maps.w[i], in.w[i], 2, dims, str, box, 1))) return rc;
     }
     for (int i = tensors; i < 4; ++i) maps.w[i] = maps.w[0];
@@ -578,11 +601,12 @@ int launch(const LinearIn& in, const EpiArgs& ep, int slices, int w_rows, cudaSt
         configured.mark();
     }
     const long long tiles = ((in.rows + kBM - 1) / kBM) * (in.n / kWRows) * (EPI == kEpiSwiglu ? 1 : in.num_w);
-    OF3_REQUIRE(tiles < (1LL << 31) && in.rows < (1LL << 31), OF3_ERR_SHAPE, "linear: too many rows");
+    OF3_REQUIRE(tiles < (1LL << 30) && in.rows < (1LL << 31), OF3_ERR_SHAPE, "linear: too many rows");
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
+    const int rest = (int)(tiles % grid), whole = (int)tiles - (has_halves<BN, EPI>() && 2 * rest <= grid ? rest : 0);
     LaunchScope scope(kKid, st);
     OF3_CUDA_CHECK(launch_chained(linear_kernel<BN, EPI, D>, grid, kThreads, Cfg::kSmemBytes, st, maps, ep, in.rows, in.k,
-                                  in.n, in.num_w, device_status_ptr()));
+                                  in.n, in.num_w, whole, device_status_ptr()));
     return OF3_OK;
 }
 

@@ -87,6 +87,24 @@ def test_few_tokens_equal_rows_of_a_larger_call(N, samples):
     assert torch.isfinite(got).all() and got.any() and torch.equal(got, want)
 
 
+# 12 column tiles of 256 (queries to gates; the hidden channels) times 14, 25, 30, 31 and 40 row tiles on 148 SMs: a last wave of 20
+# tiles, of 4, of 64 and of 36, in halves, and one of 76, whole; the last row tile full and in part
+@pytest.mark.parametrize("N,samples", [(350, 5), (1050, 3), (768, 5), (987, 4), (1024, 5)])
+def test_halves_of_the_last_wave_equal_whole_tiles(N, samples):
+    """A step whose last wave of wide tiles is half empty, its tiles in two, against every sample by itself."""
+    g = torch.Generator().manual_seed(N)
+    blk = _diffusion_block(g)
+    a, s = (torch.randn(1, samples, N, c, generator=g).to("cuda:0", torch.bfloat16) for c in (768, 384))
+    z = torch.randn(1, 1, N, N, 128, generator=g).to("cuda:0", torch.bfloat16)
+    m = (torch.rand(1, 1, N, generator=g) < 0.9).to("cuda:0", torch.bfloat16)
+    m[..., 0] = 1
+    with torch.no_grad():
+        got = blk(a, s, z, mask=m)
+        want = torch.cat([blk(a[:, i:i + 1].contiguous(), s[:, i:i + 1].contiguous(), z, mask=m) for i in range(samples)], 1)
+    pkg.lib.check_device_status()
+    assert torch.isfinite(got).all() and got.any() and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("N,samples", [(1, 2), (7, 1), (16, 1), (33, 2), (64, 1), (100, 1), (129, 2), (500, 1), (768, 1)])
 def test_few_tokens_of_the_single_track(N, samples):
     """The same for the attention of the trunk's single track (16 heads of 24, whose images pad k to 32)."""
