@@ -146,6 +146,9 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
     const uint32_t tmem_base = *tmem_ptr;
     grid_trigger();
     if (warp >= 2) grid_wait();
+    // 128 channels, lone tiles: the LayerNorm warps, done with theirs, take k and half of v's heads. With trimul_in's share of the
+    // positions, four blocks of the trunk: N = 37 408.1 -> 404.7 us, 64 406.9 -> 402.8, 100 447.9 -> 445.8. (64 channels: registers.)
+    const bool solo = C == 128 && num_tiles <= (long long)gridDim.x;
     // TMEM: slot 0 = [q|k] columns [0,2C), slot 1 = v columns [2C,3C) + triangle bias [3C,3C+16)
 
     if (warp == 0) {
@@ -227,9 +230,12 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
             if (lane == 0) mbar_arrive(a_ready(s));
             if (copy_mask) mask_t[((long long)tc.b * R + tc.line) * npad + pos] = mv;
         }
-    } else {
+    }
+    if (warp >= (solo ? 2 : 2 + kProjLnWarps)) {
         // epilogue warps
-        const int set = (warp - 2 - kProjLnWarps) >> 2;
+        const bool helper = C == 128 && warp < 2 + kProjLnWarps, shared = solo && !helper;
+        const int set = ((warp - 2) >> 2) & 1;
+        const int qk_end = shared ? 1 : 2, h_end = shared ? kH / 2 : kH;
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
         const float qscale = kLog2e * rsqrtf((float)D);
@@ -250,7 +256,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
             if (set == 0) {
                 // ---- slot 0: q (columns [0, C)) and k ([C, 2C))
 #pragma unroll 1
-                for (int qk = 0; qk < 2; ++qk) {
+                for (int qk = helper ? 1 : 0; qk < qk_end; ++qk) {
                     __nv_bfloat16* base = qk == 0 ? q_out : k_out;
                     const float sl = live ? (qk == 0 ? qscale : 1.0f) : 0.f;
 #pragma unroll 1
@@ -283,11 +289,11 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
                 }
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(slot_empty(0));
+                if (lane == 0 && !helper) mbar_arrive(slot_empty(0));
             } else {
                 // ---- slot 1: v, transposed; the triangle bias
 #pragma unroll 1
-                for (int h = 0; h < kH; ++h) {
+                for (int h = helper ? kH / 2 : 0; h < h_end; ++h) {
                     uint32_t r[D];
                     if constexpr (D == 32) tmem_ld32(taddr + 2 * C + h * D, r);
                     else tmem_ld16(taddr + 2 * C + h * D, r);
@@ -302,6 +308,7 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
                                 __float2bfloat16_rn(live ? __uint_as_float(r[e]) : 0.f);
                     }
                 }
+                if (helper) break;
                 uint32_t tbr[16];  // triangle bias of this position: columns 3C..3C+3, pre-scaled for exp2
                 tmem_ld16(taddr + 3 * C, tbr);
                 tmem_ld_wait();
