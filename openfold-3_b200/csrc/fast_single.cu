@@ -386,7 +386,7 @@ int attn_pair_bias(const bf16* a, const bf16* z, const bf16* s, const bf16* mask
     bias.ln_w = (const bf16*)p->ln_z_w;
     bias.ln_b = (const bf16*)p->ln_z_b;
     bias.w = (const bf16*)p->w_z;
-    if ((rc = single_attn(im, g, bias, tb, mask, og, Ba, N, N, H, d, inf, Ba / Bz, st))) return rc;
+    if ((rc = single_attn(im, g, bias, tb, mask, og, Ba, N, N, H, d, inf, Ba / Bz, !(flags & kFlagBeside), st))) return rc;
     const LinearIn in{og, rows, c_a, c_a, {(const bf16*)p->w_o}, 1};
     const bool few = token_residual_supported(rows, c_a) && alone(rows, flags) && even(a) && even(out);
     return (few ? token_residual : linear_residual)(in, (flags & OF3_FLAG_ADD_RESIDUAL) ? a : nullptr,
@@ -452,7 +452,7 @@ int attn_pair_bias_rows(const bf16* a, const float* pair_bias_rows, const bf16* 
     }
     SingleBias bias;
     bias.f32 = pair_bias_rows;
-    if ((rc = single_attn(im, g, bias, tb, mask, og, 1, N, R, H, d, inf, 1, st))) return rc;
+    if ((rc = single_attn(im, g, bias, tb, mask, og, 1, N, R, H, d, inf, 1, false, st))) return rc;
     const LinearIn in{og, R, c_a, c_a, {(const bf16*)p->w_o}, 1};
     return linear_residual(in, (flags & OF3_FLAG_ADD_RESIDUAL) ? a + (long long)row0 * c_a : nullptr, nullptr, nullptr,
                            nullptr, out_rows, st);

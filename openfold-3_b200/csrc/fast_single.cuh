@@ -47,7 +47,7 @@ struct SingleBias {
 };
 int single_attn(const SingleImages& im, const __nv_bfloat16* gate, const SingleBias& bias, __nv_bfloat16* tb,
                 const __nv_bfloat16* mask, __nv_bfloat16* out, int BB, int N, int nq, int H, int d, float inf,
-                int rows_per_bias, cudaStream_t st);
+                int rows_per_bias, bool spread, cudaStream_t st);
 
 }  // namespace fast
 }  // namespace of3

@@ -1,6 +1,6 @@
 // Attention of the single track and of the diffusion token stack on the tensor pipe (bf16, 16 heads of 24 or 48):
 // the streaming core of the triangle attention (csrc/fast_triattn.cu) with one (pair tensor, head, 128 queries) and
-// two samples per CTA.
+// one or two samples per CTA.
 //
 //   operand images  q / k / v projections as pre-swizzled operand tiles (linear.cu): q with its bias added and scaled
 //                   by log2(e)/sqrt(d), K-dim padded with zeros to 32 (d = 24) or 64 (d = 48); k likewise per key
@@ -8,7 +8,7 @@
 //   single_bias     pair bias fp32 [zh][nq][N] -> bf16 tiles [zh][key block][nq][32], pre-scaled by log2(e), each
 //                   64-byte row in the 64-byte swizzle of a K-major A operand (callers that project the bias
 //                   themselves get these tiles straight from csrc/fast_pairbias.cu and skip this kernel)
-//   single_core     per CTA and 32-key step: S = Q K^T + bias I^T (tcgen05, TMEM), online softmax by one thread per
+//   single_core     a CTA takes one or two samples; per CTA and 32-key step: S = Q K^T + bias I^T (tcgen05, TMEM), online softmax by one thread per
 //                   query row (exp2, lazy rescaling), P (bf16) back into TMEM over S as the A operand of
 //                   O += P [V; 1] (the row of ones makes the tensor pipe accumulate the row sum l); epilogue
 //                   O / l * sigmoid(gate) -> og [rows, H*d]
@@ -34,12 +34,15 @@ constexpr int kKidSingleCore = 11;   // the attention core
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kBQ = kSingleBQ;   // queries per CTA and line
 constexpr int kBK = kSingleBK;   // keys per step
-constexpr int kLines = 2;  // samples per CTA: they share the pair-bias tiles
+// Lines (samples) per CTA: two share the pair-bias tiles; one where that leaves fewer lines per SM (core_impl)
+template <int kLines>
 constexpr int kThreads = 32 * (1 + kLines + 4 * kLines);  // producer, one MMA warp per line, softmax warps
+template <int kLines>
+constexpr int kCtasPerSm = kLines == 1 ? 3 : 2;
 constexpr float kRescaleThreshold = 8.0f;
 constexpr int kMaxKeysSingle = 8192;  // one flag byte per key block, 256 of them
 
-template <int D>
+template <int D, int kLines>
 struct Cfg {
     static constexpr int kKD = SingleImage<D>::kKD;
     static constexpr int kKSteps = (D + 15) / 16;        // K = 16 steps that hold data
@@ -99,8 +102,8 @@ __device__ __forceinline__ void store_row(bf16* p, const uint32_t (&o)[V / 2]) {
 }
 
 // ---------------------------------------------------------------- single_core
-// One CTA = (pair tensor z, head, 128 queries) for TWO samples ("lines") that share the pair bias (the last group of an odd
-// number of samples: one, and nothing is done for the other); two CTAs per SM.
+// One CTA = (pair tensor z, head, 128 queries) for ONE sample ("line"), three CTAs per SM, or for TWO that share the pair bias
+// (the last of an odd number of samples: one, and nothing is done for the other), two CTAs per SM; core_impl chooses.
 // Per line and 32-key step j:
 //   MMA warp      S_j = Q K_j^T + Tb_j I^T into TMEM slot j % 2 (the bias tile is a second A operand against a
 //                 32 x 32 identity: the tensor pipe adds it, exactly, in fp32)
@@ -114,12 +117,12 @@ __device__ __forceinline__ void store_row(bf16* p, const uint32_t (&o)[V / 2]) {
 // behind the last P V, 16 bytes at a time, and divisions in the sigmoids made the epilogue 11000 cycles of some 60000 (5 x 768
 // tokens, 24 layers: 3630 -> 3456 us). Measured and not kept: 64 keys per step as in the triangle attention (with 48 channels
 // P then has one block of columns and two hand-offs per step: 3505 us), three V slots (one block per SM at N = 768: 3773).
-template <int D>
-__global__ void __launch_bounds__(kThreads, 2)
+template <int D, int kLines>
+__global__ void __launch_bounds__(kThreads<kLines>, kCtasPerSm<kLines>)
 single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_img, const bf16* __restrict__ v_img,
                    const bf16* __restrict__ tb_img, const bf16* __restrict__ mask, const bf16* __restrict__ gate,
-                   bf16* __restrict__ out, int N, int nq, int H, int rpb, float inf, int* status) {
-    using C = Cfg<D>;
+                   bf16* __restrict__ out, int N, int nq, int H, int rpb, int pairs, float inf, int* status) {
+    using C = Cfg<D, kLines>;
     constexpr int KD = C::kKD, DV = C::kDV, kSt = C::kStages, kVSt = C::kVStages;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -144,15 +147,18 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_qt = (nq + kBQ - 1) / kBQ;
-    const int gpz = (rpb + kLines - 1) / kLines;   // CTAs per (z, head, query tile)
-    const int grp = blockIdx.x % gpz;
-    const int qt = (blockIdx.x / gpz) % n_qt;
-    const int h = (blockIdx.x / (gpz * n_qt)) % H;
-    const int z = blockIdx.x / (gpz * n_qt * H);
+    // CTAs of kLines samples first, `pairs` of them; then those of the last sample of an odd number
+    const bool odd = kLines == 2 && (int)blockIdx.x >= pairs;
+    const int b = odd ? (int)blockIdx.x - pairs : (int)blockIdx.x;
+    const int gpz = odd ? 1 : rpb / kLines;   // CTAs of the kind per (z, head, query tile)
+    const int grp = odd ? rpb / kLines : b % gpz;
+    const int qt = (b / gpz) % n_qt;
+    const int h = (b / (gpz * n_qt)) % H;
+    const int z = b / (gpz * n_qt * H);
     const int q0 = qt * kBQ;
     const int nblk = (N + kBK - 1) / kBK;
     const int nkp = nblk * kBK;
-    const int lines = rpb - grp * kLines < kLines ? rpb - grp * kLines : kLines;   // samples of this group
+    const int lines = odd ? 1 : kLines;   // samples of this group
     auto sample_of = [&](int L) { return (long long)z * rpb + grp * kLines + L; };
 
     if (threadIdx.x == 0) {
@@ -504,18 +510,44 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
     }
 }
 
+template <int D, int kLines>
+int launch_core(const SingleImages& im, const bf16* g, const bf16* tb, const bf16* mask, bf16* out, int BB, int N, int nq,
+                int H, float inf, int rpb, uint32_t smem, cudaStream_t st) {
+    // the size depends on N and function attributes are per device: set on every launch (a host-side store)
+    OF3_CUDA_CHECK(cudaFuncSetAttribute(single_core_kernel<D, kLines>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const long long each = (long long)(BB / rpb) * H * ceil_div(nq, kBQ), pairs = each * (rpb / kLines);
+    const long long grid = pairs + (rpb % kLines ? each : 0);
+    LaunchScope scope(kKidSingleCore, st);
+    OF3_CUDA_CHECK(launch_chained(single_core_kernel<D, kLines>, dim3((unsigned)grid), kThreads<kLines>, smem, st, im.q, im.k,
+                                  im.v, tb, mask, g, out, N, nq, H, rpb, (int)pairs, inf, device_status_ptr()));
+    return OF3_OK;
+}
+
+// One line per CTA where the chip takes all lines at once (three per SM), two above. A line's step is a chain of hand-offs: an SM
+// with four lines needs some 1900 cycles for a step of each, with fewer up to half of that, so the launch takes as long as its
+// fullest SM. Under the launch before, whose blocks end one by one, the SMs that are free first took two CTAs of two lines each
+// while others stayed empty. So a CTA takes shared memory of which an SM has only as many shares as the lines need (not beside
+// another stack, whose blocks want to share the SM). Steps of 24 blocks, two lines per CTA -> this: 111 tokens 759 -> 755 us,
+// 5 x 111 1046 -> 959, 1024 1571 -> 1480, 3 x 300 1393 -> 1241, 2 x 700 1797 -> 1597, 5 x 500 2225 -> 2108, 5 x 640 2634 -> 2539
+// (lines per SM of the last four: 1, 2, 3, 3). Without the shares 3 x 300 1293, 3 x 400 1599 (with 1436). More lines, two per CTA:
+// the pairs first and the odd samples behind them, which end the launch sooner than pairs do (5 x 1024: 4214 -> 4091).
 template <int D>
 int core_impl(const SingleImages& im, const bf16* g, const bf16* tb, const bf16* mask, bf16* out, int BB, int N, int nq,
-              int H, float inf, int rpb, cudaStream_t st) {
-    const int nkb = ceil_div(N, kBK), n_qt = ceil_div(nq, kBQ);
-    const uint32_t smem = Cfg<D>::dyn_bytes(nkb * kBK);
-    // the size depends on N and function attributes are per device: set on every launch (a host-side store)
-    OF3_CUDA_CHECK(cudaFuncSetAttribute(single_core_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const long long grid = (long long)(BB / rpb) * H * n_qt * ceil_div(rpb, kLines);
-    LaunchScope scope(kKidSingleCore, st);
-    OF3_CUDA_CHECK(launch_chained(single_core_kernel<D>, dim3((unsigned)grid), kThreads, smem, st, im.q, im.k, im.v, tb,
-                                  mask, g, out, N, nq, H, rpb, inf, device_status_ptr()));
-    return OF3_OK;
+              int H, float inf, int rpb, bool spread, cudaStream_t st) {
+    const int nkp = ceil_div(N, kBK) * kBK;
+    const long long lines = (long long)BB * H * ceil_div(nq, kBQ), sms = sm_count();
+    uint32_t smem = Cfg<D, 1>::dyn_bytes(nkp);
+    constexpr uint32_t kSmBytes = 228 * 1024, kReserved = 1024;   // shared memory of an SM, of it per CTA
+    int fit = (int)(kSmBytes / (smem + kReserved));
+    if (fit > kCtasPerSm<1>) fit = kCtasPerSm<1>;
+    if (rpb > 1 && lines > fit * sms)
+        return launch_core<D, 2>(im, g, tb, mask, out, BB, N, nq, H, inf, rpb, Cfg<D, 2>::dyn_bytes(nkp), st);
+    const long long per_sm = (lines + sms - 1) / sms;
+    if (spread && per_sm < fit) {
+        const uint32_t more = kSmBytes / (uint32_t)(per_sm + 1) - kReserved + 1024;   // one more would not fit
+        smem = smem > more ? smem : more;
+    }
+    return launch_core<D, 1>(im, g, tb, mask, out, BB, N, nq, H, inf, rpb, smem, st);
 }
 
 }  // namespace
@@ -523,16 +555,16 @@ int core_impl(const SingleImages& im, const bf16* g, const bf16* tb, const bf16*
 // d in {24, 48}; H * d a multiple of 8 (16-byte rows per head); N within the mask row a CTA keeps.
 bool single_attn_tc_supported(int N, int H, int d) {
     if (!(d == 24 || d == 48) || N < 1 || N > kMaxKeysSingle || H * d % 64 != 0) return false;
-    const size_t smem = d == 24 ? Cfg<24>::dyn_bytes(ceil_div(N, kBK) * kBK) : Cfg<48>::dyn_bytes(ceil_div(N, kBK) * kBK);
+    const size_t smem = d == 24 ? Cfg<24, 2>::dyn_bytes(ceil_div(N, kBK) * kBK) : Cfg<48, 2>::dyn_bytes(ceil_div(N, kBK) * kBK);
     return smem <= 227 * 1024;
 }
 
 SingleImages take_single_images(Arena& ws, int BB, int N, int nq, int H, int d) {
     const size_t n_qt = ceil_div(nq, kBQ), nkb = ceil_div(N, kBK), bh = (size_t)BB * H;
     SingleImages im;
-    im.q = (bf16*)ws.take(bh * n_qt * (d == 24 ? Cfg<24>::kQBytes : Cfg<48>::kQBytes));
-    im.k = (bf16*)ws.take(bh * nkb * (d == 24 ? Cfg<24>::kKBytes : Cfg<48>::kKBytes));
-    im.v = (bf16*)ws.take(bh * nkb * (d == 24 ? Cfg<24>::kVBytes : Cfg<48>::kVBytes));
+    im.q = (bf16*)ws.take(bh * n_qt * (d == 24 ? Cfg<24, 1>::kQBytes : Cfg<48, 1>::kQBytes));
+    im.k = (bf16*)ws.take(bh * nkb * (d == 24 ? Cfg<24, 1>::kKBytes : Cfg<48, 1>::kKBytes));
+    im.v = (bf16*)ws.take(bh * nkb * (d == 24 ? Cfg<24, 1>::kVBytes : Cfg<48, 1>::kVBytes));
     return im;
 }
 
@@ -541,7 +573,7 @@ SingleImages take_single_images(Arena& ws, int BB, int N, int nq, int H, int d) 
 //                                                       + inf * (mask[bb, j] - 1) + pair_bias[bb / rpb, h, i, j]) v
 // g, out: [BB, nq, H*d]; mask [BB, N] or null; tb: room for the bias tiles where they are not given.
 int single_attn(const SingleImages& im, const bf16* g, const SingleBias& bias, bf16* tb, const bf16* mask, bf16* out,
-                int BB, int N, int nq, int H, int d, float inf, int rows_per_bias, cudaStream_t st) {
+                int BB, int N, int nq, int H, int d, float inf, int rows_per_bias, bool spread, cudaStream_t st) {
     OF3_REQUIRE(single_attn_tc_supported(N, H, d), OF3_ERR_SHAPE, "single attention: N %d, H %d, d %d not supported",
                 N, H, d);
     OF3_REQUIRE(rows_per_bias > 0 && BB % rows_per_bias == 0, OF3_ERR_SHAPE,
@@ -560,8 +592,8 @@ int single_attn(const SingleImages& im, const bf16* g, const SingleBias& bias, b
         const int rc = pair_bias_tiles_c128_h16(bias.z, bias.ln_w, bias.ln_b, bias.w, tb, Bz, N, st);
         if (rc) return rc;
     }
-    return d == 24 ? core_impl<24>(im, g, tiles, mask, out, BB, N, nq, H, inf, rows_per_bias, st)
-                   : core_impl<48>(im, g, tiles, mask, out, BB, N, nq, H, inf, rows_per_bias, st);
+    return d == 24 ? core_impl<24>(im, g, tiles, mask, out, BB, N, nq, H, inf, rows_per_bias, spread, st)
+                   : core_impl<48>(im, g, tiles, mask, out, BB, N, nq, H, inf, rows_per_bias, spread, st);
 }
 
 }  // namespace fast
