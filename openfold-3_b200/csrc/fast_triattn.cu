@@ -1139,6 +1139,11 @@ int z_tmap(CUtensorMap* m, const void* z, int B, int R, int N, int C, bool trans
     return make_tmap_bf16(m, z, 4, dims, str, box, 1);
 }
 
+// Shared memory for a block of the core that leaves no room for a second one on its SM (228 KB, 1 KB of them the system's per block):
+// where no SM need take two, since the blocks start while the launch before drains and would gather on the SMs that it has left first.
+// Trunk of four blocks: N = 37 403.8 -> 399.9 us, 50 409 -> 394, 64 403 -> 391, 74 433 -> 418; template of 60 134 -> 127.
+constexpr uint32_t kCoreAlone = 114 * 1024;
+
 template <int C, bool kT>
 int set_attrs() {
     static PerDeviceOnce configured;
@@ -1151,7 +1156,7 @@ int set_attrs() {
             OF3_REQUIRE(fa.numRegs == kCoreRegsLaunch, OF3_ERR_DRIVER, "triattn_core is built with %d registers, not %d",
                         fa.numRegs, kCoreRegsLaunch);
             OF3_CUDA_CHECK(cudaFuncSetAttribute(core, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                CoreSmem<C / kH>::dyn_bytes(kMaxKeys / kBK)));
+                                                max(CoreSmem<C / kH>::dyn_bytes(kMaxKeys / kBK), kCoreAlone)));
         }
         for (auto* out : {triattn_out_kernel<C, kT, false>, triattn_out_kernel<C, kT, true>})
             OF3_CUDA_CHECK(cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, AOutSmem<C>::kDyn));
@@ -1211,8 +1216,9 @@ int finish_impl(const __nv_bfloat16* z, const MaskView& mask, __nv_bfloat16* out
     {
         LaunchScope scope(kKidCore, st);
         auto* core = mask.columns ? triattn_core_kernel<C / kH, true> : triattn_core_kernel<C / kH, false>;
-        OF3_CUDA_CHECK(launch_chained(core, (unsigned)ctas, kCoreThreads, CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK)), st, q,
-                                      k, vt, tb, mask.p, mask.pitch, o, R, N, inf, status));
+        uint32_t smem = CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK));
+        if (ctas <= sm_count()) smem = max(smem, kCoreAlone);
+        OF3_CUDA_CHECK(launch_chained(core, (unsigned)ctas, kCoreThreads, smem, st, q, k, vt, tb, mask.p, mask.pitch, o, R, N, inf, status));
     }
     const long long tiles = (long long)oB * oR * ceil_div(oN, kRows);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());
