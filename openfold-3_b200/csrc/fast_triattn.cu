@@ -340,7 +340,8 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
 // triattn_core
 // =====================================================================================
 // One CTA = one head, 128 queries and TWO lines of the pair tensor, 64 keys per step; two CTAs share an SM
-// (their prologues, epilogues and waits interleave). Per line and step j:
+// (their prologues, epilogues and waits interleave). Few lines: ONE per CTA, up to three CTAs per SM (finish_impl).
+// Per line and step j:
 //   S warp        S_j = Q K_j^T + Tb_j I^T: 128 x 64 logits in TMEM, issued as soon as the softmax warps have S_{j-1} in
 //                 registers. The pair-bias tiles [128 q x 32 k] (bf16, shared by both lines) are a second A operand
 //                 against a 32 x 32 identity: a bf16 value times 1.0 accumulated in fp32 is exact.
@@ -371,20 +372,24 @@ triattn_proj_kernel(const __grid_constant__ CUtensorMap tmZ, const __grid_consta
 constexpr int kBQ = 128;      // queries per CTA
 constexpr int kMaxKeys = 2048;   // one CTA keeps a mask-bias row per line in shared memory
 constexpr int kKvStages = 2;     // ring of K + bias tiles, ring of V tiles
-constexpr int kLines = 2;     // lines per CTA
 constexpr int kLinePad = 4;   // the operand images pad the line count of a sample to a multiple of this
-// three warpgroups: producer, S of line 0, S of line 1, P V of both; the softmax warps of line 0; of line 1
+// three warpgroups: producer, S of line 0, S of line 1, P V of both; the softmax warps of line 0; of line 1 (one line: producer, S,
+// P V and an idle warp; the softmax warps)
+template <int kLines>
 constexpr int kCoreThreads = 128 * (1 + kLines);
-// registers: the block is launched with 80 per thread (two blocks of 384 threads per SM); the issuing warpgroup gives up
+template <int kLines>
+constexpr int kCorePerSm = kLines == 1 ? 3 : 2;
+// registers: the block is launched with 80 per thread (two blocks of 384 threads per SM, or three of 256); the issuing warpgroup gives up
 // what the softmax warpgroups, which hold a row of 64 logits, take. (The issuing warps need more than 32; with 96 for
 // the softmax warps it is no faster.)
 constexpr int kCoreRegsLaunch = 80, kCoreRegsIssue = 64, kCoreRegsSoftmax = 88;
-static_assert(kCoreRegsIssue + 2 * kCoreRegsSoftmax <= 3 * kCoreRegsLaunch, "register split");
+static_assert(kCoreRegsIssue + 2 * kCoreRegsSoftmax <= 3 * kCoreRegsLaunch && kCoreRegsIssue + kCoreRegsSoftmax <= 2 * kCoreRegsLaunch,
+              "register split");
 constexpr float kRescaleThreshold = 32.0f;
 constexpr uint32_t kTbTileBytes = kBQ * kBiasK * 2;    // 8192: 128 query rows x 32 keys
 constexpr uint32_t kColP = 64, kColO = 96;
 
-template <int D>
+template <int D, int kLines>
 struct CoreSmem {
     static constexpr uint32_t kQBytes = kBQ * D * 2;
     static constexpr uint32_t kKBytes = kBK * D * 2;
@@ -401,13 +406,13 @@ struct CoreSmem {
 };
 
 // kColumns: where the mask of a transposed view is read in place (strides that are not constants cost the short calls 0.3 %)
-template <int D, bool kColumns>
-__global__ void __launch_bounds__(kCoreThreads, 2)
+template <int D, bool kColumns, int kLines>
+__global__ void __launch_bounds__(kCoreThreads<kLines>, kCorePerSm<kLines>)
 triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16* __restrict__ k_img,
                     const __nv_bfloat16* __restrict__ v_img, const __nv_bfloat16* __restrict__ tb_img,
                     const __nv_bfloat16* __restrict__ mask, int mask_pitch, __nv_bfloat16* __restrict__ o_out, int R,
                     int N, float inf, int* status) {
-    using Sm = CoreSmem<D>;
+    using Sm = CoreSmem<D, kLines>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t sbase = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* gbase = smem_raw + (sbase - smem_u32(smem_raw));
@@ -462,7 +467,7 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
         mbar_fence_init();
     }
     // 32 x 32 identity, bf16, K-major with the 64-byte swizzle: element (n, n) of row n
-    for (int idx = threadIdx.x; idx < 32 * 16; idx += kCoreThreads) {
+    for (int idx = threadIdx.x; idx < 32 * 16; idx += kCoreThreads<kLines>) {
         const int n = idx >> 4, w = idx & 15;  // row, 32-bit word of the row (2 elements)
         const int k = w * 2;                   // first element of the word
         uint32_t v = 0;
@@ -562,8 +567,8 @@ triattn_core_kernel(const __nv_bfloat16* __restrict__ q_img, const __nv_bfloat16
                 }
                 __syncwarp();
             }
-        } else {
-            // ------------------------------------------------------------ the warp that issues O += P_j V_j of both lines
+        } else if (warp == kLines + 1) {
+            // ------------------------------------------------------------ the warp that issues O += P_j V_j of all lines
             const uint32_t tm = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint32_t sb = __shfl_sync(0xffffffffu, sbase, 0);
             constexpr uint32_t idesc_o = idesc_bf16_f32(128, D);   // O: 128 x D, K = 64
@@ -1139,10 +1144,8 @@ int z_tmap(CUtensorMap* m, const void* z, int B, int R, int N, int C, bool trans
     return make_tmap_bf16(m, z, 4, dims, str, box, 1);
 }
 
-// Shared memory for a block of the core that leaves no room for a second one on its SM (228 KB, 1 KB of them the system's per block):
-// where no SM need take two, since the blocks start while the launch before drains and would gather on the SMs that it has left first.
-// Trunk of four blocks: N = 37 403.8 -> 399.9 us, 50 409 -> 394, 64 403 -> 391, 74 433 -> 418; template of 60 134 -> 127.
-constexpr uint32_t kCoreAlone = 114 * 1024;
+// Shared memory of which an SM (228 KB, 1 KB of them the system's per block) has per_sm shares and no more
+constexpr uint32_t core_share(int per_sm) { return 228 * 1024 / (uint32_t)(per_sm + 1); }
 
 template <int C, bool kT>
 int set_attrs() {
@@ -1150,13 +1153,14 @@ int set_attrs() {
     if (!configured.done()) {
         OF3_CUDA_CHECK(cudaFuncSetAttribute(triattn_proj_kernel<C, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             ProjSmem<C>::kDyn));
-        for (auto* core : {triattn_core_kernel<C / kH, false>, triattn_core_kernel<C / kH, true>}) {
+        for (auto* core : {triattn_core_kernel<C / kH, false, 1>, triattn_core_kernel<C / kH, true, 1>,
+                           triattn_core_kernel<C / kH, false, 2>, triattn_core_kernel<C / kH, true, 2>}) {
             cudaFuncAttributes fa;   // a block launched with fewer registers would wait for the split for good
             OF3_CUDA_CHECK(cudaFuncGetAttributes(&fa, core));
             OF3_REQUIRE(fa.numRegs == kCoreRegsLaunch, OF3_ERR_DRIVER, "triattn_core is built with %d registers, not %d",
                         fa.numRegs, kCoreRegsLaunch);
             OF3_CUDA_CHECK(cudaFuncSetAttribute(core, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                max(CoreSmem<C / kH>::dyn_bytes(kMaxKeys / kBK), kCoreAlone)));
+                                                max(CoreSmem<C / kH, 2>::dyn_bytes(kMaxKeys / kBK), core_share(1))));
         }
         for (auto* out : {triattn_out_kernel<C, kT, false>, triattn_out_kernel<C, kT, true>})
             OF3_CUDA_CHECK(cudaFuncSetAttribute(out, cudaFuncAttributeMaxDynamicSharedMemorySize, AOutSmem<C>::kDyn));
@@ -1211,14 +1215,24 @@ int finish_impl(const __nv_bfloat16* z, const MaskView& mask, __nv_bfloat16* out
     if ((rc = weight_tmap(&tmWo, p->w_o, C))) return rc;
     if ((rc = set_attrs<C, kT>())) return rc;
     int* status = device_status_ptr();
-    const long long ctas = (long long)B * ceil_div(R, kLines) * kH * ceil_div(N, kBQ);
-    OF3_REQUIRE(ctas < (1LL << 31), OF3_ERR_SHAPE, "triattn: too many attention tiles");
+    const long long lines = (long long)B * R * kH * ceil_div(N, kBQ), pairs = (long long)B * ceil_div(R, 2) * kH * ceil_div(N, kBQ);
+    OF3_REQUIRE(pairs < (1LL << 31), OF3_ERR_SHAPE, "triattn: too many attention tiles");
+    // One line per block where the chip takes all lines at once, and room for as many blocks per SM as spread them evenly: blocks start
+    // while the projections drain, and gathered on the SMs that these had left first; the launch ends with its fullest SM. Trunk of
+    // four blocks, us, two lines per block / also with a share of the SM where there are no more blocks than SMs / one line: N = 37
+    // (one line per SM) 403.8 / 400.0 / 375.5, 50 409 / 395 / 392, 64 (two) 403 / 391.0 / 387.4, 80 (three) - / 430.4 / 420.1, 111 - /
+    // 451.5 / 449.7; pair stack of 37 343.6 / 316.9 with one line, template of 60 134.3 / 127.9 / 126.8.
+    const bool one = lines <= kCorePerSm<1> * (long long)sm_count();
+    const long long ctas = one ? lines : pairs;
+    const int nblk = ceil_div(N, kBK);
+    uint32_t smem = one ? CoreSmem<C / kH, 1>::dyn_bytes(nblk) : CoreSmem<C / kH, 2>::dyn_bytes(nblk);
+    if (one) smem = max(smem, core_share((int)((lines + sm_count() - 1) / sm_count())));
     {
         LaunchScope scope(kKidCore, st);
-        auto* core = mask.columns ? triattn_core_kernel<C / kH, true> : triattn_core_kernel<C / kH, false>;
-        uint32_t smem = CoreSmem<C / kH>::dyn_bytes(ceil_div(N, kBK));
-        if (ctas <= sm_count()) smem = max(smem, kCoreAlone);
-        OF3_CUDA_CHECK(launch_chained(core, (unsigned)ctas, kCoreThreads, smem, st, q, k, vt, tb, mask.p, mask.pitch, o, R, N, inf, status));
+        auto* core = mask.columns ? (one ? triattn_core_kernel<C / kH, true, 1> : triattn_core_kernel<C / kH, true, 2>)
+                                  : (one ? triattn_core_kernel<C / kH, false, 1> : triattn_core_kernel<C / kH, false, 2>);
+        OF3_CUDA_CHECK(launch_chained(core, (unsigned)ctas, one ? kCoreThreads<1> : kCoreThreads<2>, smem, st, q, k, vt, tb, mask.p,
+                                      mask.pitch, o, R, N, inf, status));
     }
     const long long tiles = (long long)oB * oR * ceil_div(oN, kRows);
     const int grid = (int)(tiles < sm_count() ? tiles : sm_count());

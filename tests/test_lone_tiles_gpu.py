@@ -1,5 +1,5 @@
 """Kernels whose blocks have one tile each, which all of a block's warps share, against the same rows in a tensor of several tiles per
-block: a pair block on one sample and on as many as give every block more than one tile, with and without a mask, both nodes of the
+block: a pair block on one sample and on as many as give every block more than one tile (and the attention two lines per block), with and without a mask, both nodes of the
 attention and both directions of the update, bit for bit. The output of the attention takes a view that is not transposed as one
 line: its tiles cross lines and samples."""
 
@@ -21,7 +21,7 @@ def _block(dims, g):
 
 
 @pytest.mark.parametrize("dims", [PAIR, TEMPLATE], ids=["c128", "c64"])
-@pytest.mark.parametrize("N", [1, 2, 17, 37, 64, 100, 127, 128, 129, 148])
+@pytest.mark.parametrize("N", [1, 2, 17, 37, 38, 64, 75, 100, 111, 112, 127, 128, 129, 148])
 @pytest.mark.parametrize("masked", [False, True])
 def test_a_lone_tile_equals_one_of_several(dims, N, masked):
     g = torch.Generator().manual_seed(N)
