@@ -1222,6 +1222,7 @@ int finish_impl(const __nv_bfloat16* z, const MaskView& mask, __nv_bfloat16* out
     // four blocks, us, two lines per block / also with a share of the SM where there are no more blocks than SMs / one line: N = 37
     // (one line per SM) 403.8 / 400.0 / 375.5, 50 409 / 395 / 392, 64 (two) 403 / 391.0 / 387.4, 80 (three) - / 430.4 / 420.1, 111 - /
     // 451.5 / 449.7; pair stack of 37 343.6 / 316.9 with one line, template of 60 134.3 / 127.9 / 126.8.
+    // Past three lines per SM two per block: N = 112 447 us against 465 with one, 128 457 / 477, 148 711 / 728, 4 x 60 template 172 / 178.
     const bool one = lines <= kCorePerSm<1> * (long long)sm_count();
     const long long ctas = one ? lines : pairs;
     const int nblk = ceil_div(N, kBK);

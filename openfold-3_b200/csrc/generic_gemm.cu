@@ -908,7 +908,8 @@ int launch(Args<T> p, int groups, int batch, cudaStream_t st) {
     if constexpr (std::is_same<T, float>::value) {
         // Tensor cores once the small tiles of the FMA kernel would come in more than four waves. Device time, us, FMA / tensor, cold:
         // 576 rows: 4 x 128 columns 7.8 / 11.9; 2304 rows: 128 columns 8.0 / 12.4 (two waves), 4 x 128 22.3 / 12.5 (eight)
-        if (tiles(32, kPaired ? 16 : 32) > 4 * sm_count()) {
+        // (silu * up later: block of 25 tokens, 640 tiles, 314.5 / 320.2; of 26, 704, 310.4 / 311.4; of 27, 736, 311.2 / 303.9)
+        if (5 * tiles(32, kPaired ? 16 : 32) > (EPI == kSwiglu ? 24 : 20) * sm_count()) {
             bool whole = p.K % 64 == 0;
             if (!K_OUTER) {
                 whole = whole && (reinterpret_cast<uintptr_t>(p.a) & 15) == 0 && (p.a_batch & 3) == 0;
