@@ -41,6 +41,7 @@ template <int kLines>
 constexpr int kCtasPerSm = kLines == 1 ? 3 : 2;
 constexpr float kRescaleThreshold = 8.0f;
 constexpr int kMaxKeysSingle = 8192;  // one flag byte per key block, 256 of them
+constexpr int kMaxSmem = 227 * 1024;  // shared memory of a CTA
 
 template <int D, int kLines>
 struct Cfg {
@@ -513,8 +514,12 @@ single_core_kernel(const bf16* __restrict__ q_img, const bf16* __restrict__ k_im
 template <int D, int kLines>
 int launch_core(const SingleImages& im, const bf16* g, const bf16* tb, const bf16* mask, bf16* out, int BB, int N, int nq,
                 int H, float inf, int rpb, uint32_t smem, cudaStream_t st) {
-    // the size depends on N and function attributes are per device: set on every launch (a host-side store)
-    OF3_CUDA_CHECK(cudaFuncSetAttribute(single_core_kernel<D, kLines>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // Sizes depend on N and on the lines of a call, and the limit is the kernel's, for all threads of the process: the largest, once
+    static PerDeviceOnce configured;
+    if (!configured.done()) {
+        OF3_CUDA_CHECK(cudaFuncSetAttribute(single_core_kernel<D, kLines>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem));
+        configured.mark();
+    }
     const long long each = (long long)(BB / rpb) * H * ceil_div(nq, kBQ), pairs = each * (rpb / kLines);
     const long long grid = pairs + (rpb % kLines ? each : 0);
     LaunchScope scope(kKidSingleCore, st);
@@ -556,7 +561,7 @@ int core_impl(const SingleImages& im, const bf16* g, const bf16* tb, const bf16*
 bool single_attn_tc_supported(int N, int H, int d) {
     if (!(d == 24 || d == 48) || N < 1 || N > kMaxKeysSingle || H * d % 64 != 0) return false;
     const size_t smem = d == 24 ? Cfg<24, 2>::dyn_bytes(ceil_div(N, kBK) * kBK) : Cfg<48, 2>::dyn_bytes(ceil_div(N, kBK) * kBK);
-    return smem <= 227 * 1024;
+    return smem <= kMaxSmem;
 }
 
 SingleImages take_single_images(Arena& ws, int BB, int N, int nq, int H, int d) {
