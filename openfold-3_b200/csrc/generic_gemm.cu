@@ -727,8 +727,9 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
 #pragma unroll 1
                 for (int e = 0; e < (kPaired ? kRun : 2 * kRun); ++e) result(e, dot(e), kPaired ? dot(kRun + e) : 0.f);
             };
-            // all of the thread's columns, 16 by 16
-            auto sum_up = [&](float (&v)[2 * kRun / 16][16]) {
+            // all of the thread's columns, 16 by 16. marked: the tile's, read ahead of the arrivals (of one k-block each, the tile after
+            // next could otherwise be multiplied and the one behind it, whose mark takes the same place, be converted)
+            auto sum_up = [&](float (&v)[2 * kRun / 16][16], bool& marked) {
                 auto add = [&](uint32_t col) {
 #pragma unroll
                     for (int e0 = 0; e0 < 2 * kRun; e0 += 16) add16(col + (e0 < kRun ? e0 : HN + e0 - kRun), v[e0 / 16]);
@@ -742,6 +743,7 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     free_main(it & 1);
                 }
                 if (!wait_small()) return false;
+                marked = special[tc & 3] == (int)tc + 1;
                 tc_fence_after_sync();
                 add(t_small);
                 tc_fence_before_sync();
@@ -818,8 +820,9 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     if (bad) redo();
                 } else {
                     float v[2 * kRun / 16][16];
-                    if (!sum_up(v)) break;
-                    if (special[tc & 3] == (int)tc + 1) {
+                    bool marked;
+                    if (!sum_up(v, marked)) break;
+                    if (marked) {
                         redo();
                     } else if (!vec) {
 #pragma unroll
@@ -837,8 +840,9 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                 }
             } else {
                 float v[2 * kRun / 16][16];
-                if (!sum_up(v)) break;
-                if (special[tc & 3] == (int)tc + 1) {
+                bool marked;
+                if (!sum_up(v, marked)) break;
+                if (marked) {
                     redo();
                     continue;
                 }

@@ -87,3 +87,24 @@ def test_values_that_bf16_parts_cannot_hold():
         rms = want[fits, k].pow(2).mean().sqrt()
         assert fits.any() and ((got[:, k].double() - want[:, k]).abs()[fits] <= 2.0 ** -20 * (3 * rms + want[fits, k].abs())).all()
         assert torch.isinf(got[:, k][want[:, k].abs() > 3.5e38]).all()
+
+
+# k of one k-block (whole, ragged) and of several; gate / up of 128 channels, the final product of 64 and 72, and both in each call
+@pytest.mark.parametrize("c,n", [(64, 1), (36, 2), (128, 4)])
+def test_special_values_in_every_tile(c, n):
+    """An infinity or a NaN in every 128 rows, many tiles per block: only its own row is not finite. The others are sums in order on the
+    FMA pipe: k roundings of at most 2^-24 of sums that grow to the last one, sqrt(k / 6) 2^-24 RMS, 9.2 x 2^-24 at k = 512, and as
+    much again at most from the layer before and the residual."""
+    rows = 45000
+    g = torch.Generator().manual_seed(c)
+    p = _params(c, n, g)
+    x = torch.randn(rows, c, generator=g).to(DEV)
+    bad = torch.zeros(rows, dtype=torch.bool, device=DEV)
+    bad[torch.arange(5, rows, 128)] = True
+    want = _reference(x.double(), torch.ones(rows, dtype=torch.double, device=DEV), [t.double() for t in p])
+    x[bad, 3] = float("inf")
+    x[133::256, 3] = float("nan")
+    out = x.clone()
+    pkg.lib.transition_forward(out, torch.ones(rows, device=DEV), out, p, n, True)
+    pkg.lib.check_device_status()
+    assert not torch.isfinite(out[bad]).any() and rms_err(out[~bad], want[~bad]) < 2.0 ** -20
