@@ -374,7 +374,9 @@ __global__ void __launch_bounds__(G* BM / TM * BN / TN) gemm_kernel(const Args<T
 // them: in one accumulator over all of k the error grows to 1e-5 at k = 1536.) RMS error of 128 x 64 products against fp64, normal
 // operands, FFMA in order / as pairs along k / this: k = 64 1.5e-7 / 1.1e-7 / 7.1e-8, 128 2.0e-7 / 1.5e-7 / 7.4e-8, 512 4.0e-7 /
 // 2.9e-7 / 8.9e-8, 1536 7.0e-7 / 4.9e-7 / 1.2e-7; operands around 1: k = 128 1.7e-7 / 9.2e-8 / 3.3e-8.
-// A tile with a value that is not finite, or that bf16 would round to infinity, is computed once more on the FMA pipe.
+// A tile with a value of 2^127 and more, an infinity or a NaN is computed once more on the FMA pipe. Where a product of two values may
+// be beyond fp32's range (2^55 of one of them and more, for k below 2^17) its parts can be infinities of either sign: of a tile with
+// such values the rows are computed once more where a sum of their warp is not finite.
 //
 // Tiles of 128 rows by BN columns; warps 0..7 convert (loads of the next k-block are on their way under this one's conversions),
 // 8..15 the epilogue (two per 32 rows, thread = row), 16 issues the MMAs.
@@ -406,15 +408,21 @@ __device__ __forceinline__ void sub_pair(float& x0, float& x1, uint32_t v) {
         : "+f"(x0), "+f"(x1)
         : "r"(neg));
 }
-// Eight values into three planes of a stage, at d; bits 15 and 31 of `special`: an exponent of 254 or 255 as bf16
-__device__ __forceinline__ void split8(float (&x)[8], uint8_t* d, int plane, uint32_t& special) {
+// The largest of the magnitudes; NaN of a NaN
+__device__ __forceinline__ float max_abs(float m, float x0, float x1) {
+    asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(x0), "f"(x1));
+    return m;
+}
+// Eight values into three planes of a stage, at d; their largest magnitude
+__device__ __forceinline__ void split8(float (&x)[8], uint8_t* d, int plane, float& largest) {
     uint32_t u[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) largest = max_abs(largest, x[2 * i], x[2 * i + 1]);
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             u[i] = pack_bf16x2(x[2 * i], x[2 * i + 1]);
-            if (q == 0) special |= (u[i] & 0x7f007f00u) + 0x01000100u;
             if (q < 2) sub_pair(x[2 * i], x[2 * i + 1], u[i]);
         }
         *reinterpret_cast<uint4*>(d + q * plane) = make_uint4(u[0], u[1], u[2], u[3]);
@@ -474,7 +482,9 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
     auto small_free = [&](int s) { return bars + 8u * (10 + s); };
     volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + C::kBars + 96);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + C::kBars + 104);
-    volatile int* special = reinterpret_cast<volatile int*>(gbase + C::kBars + 112);   // [4] tile numbers (of this CTA, from 1)
+    // marks of tiles: [4] tile numbers (of this CTA, from 1). Values that the parts do not hold; values whose sums are to be looked at
+    volatile int* special = reinterpret_cast<volatile int*>(gbase + C::kBars + 112);
+    volatile int* doubtful = special + 4;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int K = p.K, n = p.n;
@@ -511,7 +521,7 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
             mbar_init(small_full(s), 1);
             mbar_init(small_free(s), 8);
         }
-        for (int i = 0; i < 4; ++i) special[i] = 0;
+        for (int i = 0; i < 4; ++i) special[i] = doubtful[i] = 0;
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -594,7 +604,7 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
 #pragma unroll
         for (int i = 0; i < kItemsA; ++i) fetch_a(i, 0);
         for (uint32_t t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++seq) {
-            uint32_t bad = 0;
+            float largest = 0.f;
             for (int kb = 0; kb < num_kb; ++kb, ++it) {
                 const int s = it & 1;
                 if (!mbar_wait(empty(s), ((it >> 1) & 1u) ^ 1u, abort_flag)) {
@@ -609,16 +619,19 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
 #pragma unroll
                 for (int i = 0; i < kItemsA; ++i) {
                     const int v = threadIdx.x + i * 256;
-                    split8(xa[i], stage + sw128_offset(row_of(v, 128), chunk_of(v, 128) * 8), C::kAPlane, bad);
+                    split8(xa[i], stage + sw128_offset(row_of(v, 128), chunk_of(v, 128) * 8), C::kAPlane, largest);
                     if (more) fetch_a(i, next);
                 }
 #pragma unroll
                 for (int i = 0; i < kItemsW; ++i) {
                     const int v = threadIdx.x + i * 256;
-                    split8(xw[i], stage + 3 * C::kAPlane + sw128_offset(row_of(v, BN), chunk_of(v, BN) * 8), C::kWPlane, bad);
+                    split8(xw[i], stage + 3 * C::kAPlane + sw128_offset(row_of(v, BN), chunk_of(v, BN) * 8), C::kWPlane, largest);
                     if (more) fetch_w(i, next);
                 }
-                if (bad & 0x80008000u) special[seq & 3] = seq + 1;
+                if (!(largest < 0x1p55f)) {
+                    doubtful[seq & 3] = seq + 1;
+                    if (!(largest < 0x1p127f)) special[seq & 3] = seq + 1;
+                }
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full(s));
@@ -667,6 +680,7 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
         const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + part * kRun;
         uint32_t it = 0, tc = 0;
         for (uint32_t t = blockIdx.x; t < num_tiles; t += gridDim.x, ++tc) {
+            __syncwarp();   // (lanes part where rows end, and in redo)
             const Tile c = tile_of(t);
             const long long r = c.m0 + quad * 32 + lane;
             const bool live = r < M;
@@ -712,8 +726,14 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     p.out[c.grp][c.boff + r * n + col] = x + (p.bias[c.grp] ? p.bias[c.grp][col] : 0.f);
                 }
             };
-            // a tile with values that the split does not take: its products on the FMA pipe
-            auto redo = [&] {
+            auto sound = [](const float (&v)[16]) {
+                float chk = 0.f;
+#pragma unroll
+                for (int e = 0; e < 16; ++e) chk = fmaf(v[e], 0.f, chk);
+                return chk == 0.f;
+            };
+            // columns of a tile that the split does not take: their products on the FMA pipe
+            auto redo = [&](int first, int end) {
                 auto dot = [&](int e) {
                     int col;
                     const float* w = weight_row(c, part * kRun + (e < kRun ? e : HN + e - kRun), col);
@@ -725,11 +745,11 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     return x;
                 };
 #pragma unroll 1
-                for (int e = 0; e < (kPaired ? kRun : 2 * kRun); ++e) result(e, dot(e), kPaired ? dot(kRun + e) : 0.f);
+                for (int e = first; e < end; ++e) result(e, dot(e), kPaired ? dot(kRun + e) : 0.f);
             };
-            // all of the thread's columns, 16 by 16. marked: the tile's, read ahead of the arrivals (of one k-block each, the tile after
-            // next could otherwise be multiplied and the one behind it, whose mark takes the same place, be converted)
-            auto sum_up = [&](float (&v)[2 * kRun / 16][16], bool& marked) {
+            // all of the thread's columns, 16 by 16. The marks are read ahead of the arrivals (of one k-block each, the tile after next
+            // could otherwise be multiplied and the one behind it, whose marks take the same place, be converted)
+            auto sum_up = [&](float (&v)[2 * kRun / 16][16], bool& again) {
                 auto add = [&](uint32_t col) {
 #pragma unroll
                     for (int e0 = 0; e0 < 2 * kRun; e0 += 16) add16(col + (e0 < kRun ? e0 : HN + e0 - kRun), v[e0 / 16]);
@@ -743,12 +763,18 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     free_main(it & 1);
                 }
                 if (!wait_small()) return false;
-                marked = special[tc & 3] == (int)tc + 1;
+                again = special[tc & 3] == (int)tc + 1;
+                const bool look = doubtful[tc & 3] == (int)tc + 1;
                 tc_fence_after_sync();
                 add(t_small);
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(small_free(tc & 1u));
+                if (look) {
+#pragma unroll
+                    for (int q = 0; q < 2 * kRun / 16; ++q) again |= !sound(v[q]);
+                    again = __any_sync(0xffffffffu, again);
+                }
                 return true;
             };
             if constexpr (EPI == kFinal) {
@@ -797,7 +823,8 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     }
                     if (!ok || !wait_small()) break;
                     tc_fence_after_sync();
-                    const bool bad = special[tc & 3] == (int)tc + 1;
+                    const bool marked = special[tc & 3] == (int)tc + 1, look = doubtful[tc & 3] == (int)tc + 1;
+                    uint32_t again = 0;   // a bit per 16 columns
 #pragma unroll
                     for (int e0 = 0; e0 < 2 * kRun; e0 += 16) {
                         const uint32_t at = e0 < kRun ? e0 : HN + e0 - kRun;
@@ -812,18 +839,21 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                             if (num_kb == 2) free_main(s0 ^ 1u);
                             if (lane == 0) mbar_arrive(small_free(tc & 1u));
                         }
-                        if (bad) continue;
+                        const bool bad = look && __any_sync(0xffffffffu, marked || !sound(v));
                         finish(v, a[e0 / 16 % 2]);
                         if (e0 + 32 < 2 * kRun) fetch(e0 + 32, a[e0 / 16 % 2]);
-                        put(e0, v);
+                        if (bad) again |= 1u << (e0 / 16);
+                        else put(e0, v);
                     }
-                    if (bad) redo();
+#pragma unroll 1
+                    for (int q = 0; again >> q; ++q)
+                        if (again >> q & 1u) redo(16 * q, 16 * q + 16);
                 } else {
                     float v[2 * kRun / 16][16];
-                    bool marked;
-                    if (!sum_up(v, marked)) break;
-                    if (marked) {
-                        redo();
+                    bool again;
+                    if (!sum_up(v, again)) break;
+                    if (again) {
+                        redo(0, 2 * kRun);
                     } else if (!vec) {
 #pragma unroll
                         for (int e = 0; e < 2 * kRun; ++e) result(e, v[e / 16][e % 16], 0.f);
@@ -840,10 +870,10 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                 }
             } else {
                 float v[2 * kRun / 16][16];
-                bool marked;
-                if (!sum_up(v, marked)) break;
-                if (marked) {
-                    redo();
+                bool again;
+                if (!sum_up(v, again)) break;
+                if (again) {
+                    redo(0, kPaired ? kRun : 2 * kRun);
                     continue;
                 }
                 if (!live) continue;
@@ -913,7 +943,7 @@ int launch(Args<T> p, int groups, int batch, cudaStream_t st) {
         // Tensor cores once the small tiles of the FMA kernel would come in more than four waves. Device time, us, FMA / tensor, cold:
         // 576 rows: 4 x 128 columns 7.8 / 11.9; 2304 rows: 128 columns 8.0 / 12.4 (two waves), 4 x 128 22.3 / 12.5 (eight)
         // (silu * up later: block of 25 tokens, 640 tiles, 314.5 / 320.2; of 26, 704, 310.4 / 311.4; of 27, 736, 311.2 / 303.9)
-        if (5 * tiles(32, kPaired ? 16 : 32) > (EPI == kSwiglu ? 24 : 20) * sm_count()) {
+        if (5 * tiles(32, kPaired ? 16 : 32) > (EPI == kSwiglu ? 24 : 20) * sm_count() && p.K < 1 << 17) {
             bool whole = p.K % 64 == 0;
             if (!K_OUTER) {
                 whole = whole && (reinterpret_cast<uintptr_t>(p.a) & 15) == 0 && (p.a_batch & 3) == 0;

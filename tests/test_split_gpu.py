@@ -108,3 +108,26 @@ def test_special_values_in_every_tile(c, n):
     pkg.lib.transition_forward(out, torch.ones(rows, device=DEV), out, p, n, True)
     pkg.lib.check_device_status()
     assert not torch.isfinite(out[bad]).any() and rms_err(out[~bad], want[~bad]) < 2.0 ** -20
+
+
+# one k-block, ragged and whole, two of them, and many
+@pytest.mark.parametrize("c,n", [(36, 1), (32, 2), (64, 2), (128, 4)])
+def test_products_beyond_the_range(c, n):
+    """Operands that bf16 parts hold, products that fp32 does not: infinities of their sign, and nothing else changes."""
+    rows = 20001
+    g = torch.Generator().manual_seed(c)
+    p = _params(c, n, g)
+    p[3] *= 2.0 ** 24
+    p[4][7] = 0
+    p[4][7, 11] = 1.003e38
+    x = torch.randn(rows, c, generator=g).to(DEV)
+    mask = torch.ones(rows, device=DEV)
+    out = x.clone()
+    pkg.lib.transition_forward(out, mask, out, p, n, True)
+    pkg.lib.check_device_status()
+    want = _reference(x.double(), mask.double(), [t.double() for t in p])
+    beyond = want[:, 7].abs() > 3.5e38
+    assert beyond.sum() > rows // 2 and torch.isinf(out[beyond, 7]).all()
+    assert torch.equal(out[beyond, 7] > 0, want[beyond, 7] > 0)
+    cols = torch.arange(c, device=DEV) != 7
+    assert torch.isfinite(out[:, cols]).all() and rms_err(out[:, cols], want[:, cols]) < 2.0 ** -20   # (redone ones: see above)
