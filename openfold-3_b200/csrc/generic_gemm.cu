@@ -367,16 +367,22 @@ __global__ void __launch_bounds__(G* BM / TM * BN / TN) gemm_kernel(const Args<T
 }
 
 // ---------------------------------------------------------------- fp32 products on the tensor cores
-// An fp32 value is the sum of three bf16 values of 8 bits each (exact where none of them is below 2^-133, and fp32 itself is not
-// denormal), and a product of two such values the sum of the six of their products that are above 2^-26 of it. The products of
-// the leading parts are summed by the tensor core over 64 k at a time, each such sum is added up in fp32 by the epilogue's threads;
-// the other five, 2^-8 of them and less, have an accumulator of their own. (The tensor core cuts sums off instead of rounding
-// them: in one accumulator over all of k the error grows to 1e-5 at k = 1536.) RMS error of 128 x 64 products against fp64, normal
+// An fp32 value of 2^-110 and more is the sum of three bf16 values of 8 bits each, and a product of two such values the sum of the six
+// of their products that are above 2^-26 of it (G. Henry, P. T. P. Tang, A. Heinecke, "Leveraging the bfloat16 Artificial Intelligence
+// Datatype For Higher-Precision Computations", 2019). The products of the leading parts are summed by the tensor core over 64 k at a
+// time, each such sum is added up in fp32 by the epilogue's threads; the other five, 2^-8 of them and less, have an accumulator of
+// their own. (The tensor core cuts sums off instead of rounding them: in one accumulator over all of k the error grows to 1e-5 at
+// k = 1536.) RMS error of 128 x 64 products against fp64, normal
 // operands, FFMA in order / as pairs along k / this: k = 64 1.5e-7 / 1.1e-7 / 7.1e-8, 128 2.0e-7 / 1.5e-7 / 7.4e-8, 512 4.0e-7 /
 // 2.9e-7 / 8.9e-8, 1536 7.0e-7 / 4.9e-7 / 1.2e-7; operands around 1: k = 128 1.7e-7 / 9.2e-8 / 3.3e-8.
 // A tile with a value of 2^127 and more, an infinity or a NaN is computed once more on the FMA pipe. Where a product of two values may
 // be beyond fp32's range (2^55 of one of them and more, for k below 2^17) its parts can be infinities of either sign: of a tile with
-// such values the rows are computed once more where a sum of their warp is not finite.
+// such values the rows are computed once more where a sum of their warp is not finite. At the other end the parts miss up to 2^-134 of
+// a value below 2^-110, and of products below 2^-126 more is cut off than an fma rounds away (31 x 2^-149 against 6.5, RMS, k = 512).
+// Values that are zero or 2^-50 and more have neither. A tile with others, and with none of 2^55 and more, misses at most 2^-61 in a
+// sum: its rows are computed once more where a sum of their warp is below 2^-34. (An addition and half a minimum per value: fp32 trunk
+// block N = 128 683.6 -> 692 us. From the bf16 parts' remainder, which is zero where nothing is missed, 703; a minimum of all values
+// first, and zeros told apart behind it, 696.)
 //
 // Tiles of 128 rows by BN columns; warps 0..7 convert (loads of the next k-block are on their way under this one's conversions),
 // 8..15 the epilogue (two per 32 rows, thread = row), 16 issues the MMAs.
@@ -413,11 +419,16 @@ __device__ __forceinline__ float max_abs(float m, float x0, float x1) {
     asm("max.NaN.abs.f32 %0, %0, %1, %2;" : "+f"(m) : "f"(x0), "f"(x1));
     return m;
 }
-// Eight values into three planes of a stage, at d; their largest magnitude
-__device__ __forceinline__ void split8(float (&x)[8], uint8_t* d, int plane, float& largest) {
+// Orders the magnitudes of values, with zero behind all others
+__host__ __device__ constexpr uint32_t nonzero_order(uint32_t bits) { return bits + bits - 1u; }
+// Eight values into three planes of a stage, at d; their largest magnitude, and the order of the smallest that is not zero
+__device__ __forceinline__ void split8(float (&x)[8], uint8_t* d, int plane, float& largest, uint32_t& smallest) {
     uint32_t u[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) largest = max_abs(largest, x[2 * i], x[2 * i + 1]);
+    for (int i = 0; i < 4; ++i) {
+        largest = max_abs(largest, x[2 * i], x[2 * i + 1]);
+        smallest = __vimin3_u32(smallest, nonzero_order(__float_as_uint(x[2 * i])), nonzero_order(__float_as_uint(x[2 * i + 1])));
+    }
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
 #pragma unroll
@@ -482,9 +493,10 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
     auto small_free = [&](int s) { return bars + 8u * (10 + s); };
     volatile uint32_t* tmem_ptr = reinterpret_cast<volatile uint32_t*>(gbase + C::kBars + 96);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + C::kBars + 104);
-    // marks of tiles: [4] tile numbers (of this CTA, from 1). Values that the parts do not hold; values whose sums are to be looked at
+    // marks of tiles: [4] tile numbers (of this CTA, from 1). Values that the parts do not hold; large and small ones, whose sums are to
+    // be looked at
     volatile int* special = reinterpret_cast<volatile int*>(gbase + C::kBars + 112);
-    volatile int* doubtful = special + 4;
+    volatile int *large = special + 4, *small = special + 8;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int K = p.K, n = p.n;
@@ -521,7 +533,7 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
             mbar_init(small_full(s), 1);
             mbar_init(small_free(s), 8);
         }
-        for (int i = 0; i < 4; ++i) special[i] = doubtful[i] = 0;
+        for (int i = 0; i < 12; ++i) special[i] = 0;
         *abort_flag = 0;
         mbar_fence_init();
     }
@@ -605,6 +617,7 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
         for (int i = 0; i < kItemsA; ++i) fetch_a(i, 0);
         for (uint32_t t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++seq) {
             float largest = 0.f;
+            uint32_t smallest = ~0u;
             for (int kb = 0; kb < num_kb; ++kb, ++it) {
                 const int s = it & 1;
                 if (!mbar_wait(empty(s), ((it >> 1) & 1u) ^ 1u, abort_flag)) {
@@ -619,19 +632,20 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
 #pragma unroll
                 for (int i = 0; i < kItemsA; ++i) {
                     const int v = threadIdx.x + i * 256;
-                    split8(xa[i], stage + sw128_offset(row_of(v, 128), chunk_of(v, 128) * 8), C::kAPlane, largest);
+                    split8(xa[i], stage + sw128_offset(row_of(v, 128), chunk_of(v, 128) * 8), C::kAPlane, largest, smallest);
                     if (more) fetch_a(i, next);
                 }
 #pragma unroll
                 for (int i = 0; i < kItemsW; ++i) {
                     const int v = threadIdx.x + i * 256;
-                    split8(xw[i], stage + 3 * C::kAPlane + sw128_offset(row_of(v, BN), chunk_of(v, BN) * 8), C::kWPlane, largest);
+                    split8(xw[i], stage + 3 * C::kAPlane + sw128_offset(row_of(v, BN), chunk_of(v, BN) * 8), C::kWPlane, largest, smallest);
                     if (more) fetch_w(i, next);
                 }
                 if (!(largest < 0x1p55f)) {
-                    doubtful[seq & 3] = seq + 1;
+                    large[seq & 3] = seq + 1;
                     if (!(largest < 0x1p127f)) special[seq & 3] = seq + 1;
                 }
+                if (smallest < nonzero_order(0x26800000u)) small[seq & 3] = seq + 1;   // 2^-50
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(full(s));
@@ -726,11 +740,23 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     p.out[c.grp][c.boff + r * n + col] = x + (p.bias[c.grp] ? p.bias[c.grp][col] : 0.f);
                 }
             };
-            auto sound = [](const float (&v)[16]) {
-                float chk = 0.f;
+            struct Marks {
+                bool all, look;   // compute the tile once more; look at its sums
+                float least;      // the smallest magnitude of a sound one
+            };
+            auto marks = [&] {
+                const int id = (int)tc + 1;
+                const bool l = large[tc & 3] == id, s = small[tc & 3] == id;
+                return Marks{special[tc & 3] == id || (l && s), l || s, s ? 0x1p-34f : 0.f};
+            };
+            auto sound = [](const float (&v)[16], float least) {
+                float chk = 0.f, mn = v[0];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) chk = fmaf(v[e], 0.f, chk);
-                return chk == 0.f;
+                for (int e = 0; e < 16; ++e) {
+                    chk = fmaf(v[e], 0.f, chk);
+                    mn = fminf(fabsf(mn), fabsf(v[e]));
+                }
+                return chk == 0.f && fabsf(mn) >= least;
             };
             // columns of a tile that the split does not take: their products on the FMA pipe
             auto redo = [&](int first, int end) {
@@ -763,16 +789,16 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     free_main(it & 1);
                 }
                 if (!wait_small()) return false;
-                again = special[tc & 3] == (int)tc + 1;
-                const bool look = doubtful[tc & 3] == (int)tc + 1;
+                const Marks m = marks();
+                again = m.all;
                 tc_fence_after_sync();
                 add(t_small);
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(small_free(tc & 1u));
-                if (look) {
+                if (m.look) {
 #pragma unroll
-                    for (int q = 0; q < 2 * kRun / 16; ++q) again |= !sound(v[q]);
+                    for (int q = 0; q < 2 * kRun / 16; ++q) again |= !sound(v[q], m.least);
                     again = __any_sync(0xffffffffu, again);
                 }
                 return true;
@@ -823,7 +849,7 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                     }
                     if (!ok || !wait_small()) break;
                     tc_fence_after_sync();
-                    const bool marked = special[tc & 3] == (int)tc + 1, look = doubtful[tc & 3] == (int)tc + 1;
+                    const Marks m = marks();
                     uint32_t again = 0;   // a bit per 16 columns
 #pragma unroll
                     for (int e0 = 0; e0 < 2 * kRun; e0 += 16) {
@@ -839,7 +865,7 @@ gemm_split_kernel(const Args<float> p, int batch, int groups, int* status) {
                             if (num_kb == 2) free_main(s0 ^ 1u);
                             if (lane == 0) mbar_arrive(small_free(tc & 1u));
                         }
-                        const bool bad = look && __any_sync(0xffffffffu, marked || !sound(v));
+                        const bool bad = m.look && __any_sync(0xffffffffu, m.all || !sound(v, m.least));
                         finish(v, a[e0 / 16 % 2]);
                         if (e0 + 32 < 2 * kRun) fetch(e0 + 32, a[e0 / 16 % 2]);
                         if (bad) again |= 1u << (e0 / 16);

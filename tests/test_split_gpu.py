@@ -131,3 +131,34 @@ def test_products_beyond_the_range(c, n):
     assert torch.equal(out[beyond, 7] > 0, want[beyond, 7] > 0)
     cols = torch.arange(c, device=DEV) != 7
     assert torch.isfinite(out[:, cols]).all() and rms_err(out[:, cols], want[:, cols]) < 2.0 ** -20   # (redone ones: see above)
+
+
+# hidden values below and beside the parts' reach (2^-110) against weights that bring the sums back, at both ends of what the parts'
+# products take; products whose parts are denormal; one k-block, ragged and whole, two of them, and many
+@pytest.mark.parametrize("up,out", [(2.0 ** -118, 1.0), (2.0 ** -118, 2.0 ** 50), (2.0 ** -118, 2.0 ** 100), (2.0 ** -112, 2.0 ** 50),
+                                    (2.0 ** -60, 2.0 ** -62), (2.0 ** -40, 2.0 ** -80), (2.0 ** -49, 2.0 ** -49)])
+@pytest.mark.parametrize("c,n", [(36, 1), (32, 2), (64, 2), (128, 4)])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_small_operands(up, out, c, n, mixed):
+    """Products of small values are as good as those of ordinary ones, alone and beside them (mixed: half of the hidden channels are
+    ordinary, and half of the output's columns are without them). As sums in order on the FMA pipe at most: see above."""
+    rows = 20001
+    g = torch.Generator().manual_seed(c)
+    p = _params(c, n, g)
+    half, rest = n * c // 2, c // 2
+    p[3][:half if mixed else n * c] *= up
+    p[4] *= out
+    if mixed:
+        p[4][:rest, half:] = 0
+    x = torch.randn(rows, c, generator=g).to(DEV)
+    mask = torch.ones(rows, device=DEV)
+    got = torch.empty_like(x)
+    pkg.lib.transition_forward(x, mask, got, p, n, False)
+    pkg.lib.check_device_status()
+    q = [t.double() for t in p]
+    y = F.layer_norm(x.double(), (c,), q[0], q[1], 1e-5)
+    want = (F.silu(y @ q[2].T) * (y @ q[3].T)) @ q[4].T
+    for cols in ((slice(0, rest), slice(rest, c)) if mixed else (slice(0, c),)):
+        y, w = got[:, cols].double(), want[:, cols]
+        keep = 2.0 ** -149 / w.pow(2).mean().sqrt()   # (what fp32 itself does not hold)
+        assert rms_err(y, w) < 2.0 ** -20 + keep, (rms_err(y, w), keep)
