@@ -125,3 +125,36 @@ def test_few_tokens_of_the_single_track(N, samples):
         got = layer(a[:samples].contiguous(), z[:samples].contiguous(), mask=m[:samples].contiguous())
     pkg.lib.check_device_status()
     assert torch.isfinite(got).all() and got.any() and torch.equal(got, want)
+
+
+# more rows than one wave of 64-token tiles takes in any of the products: 768 of 768 channels, 1536 of 384
+@pytest.mark.parametrize("N,samples", [(1, 1), (1, 3), (7, 1), (15, 1), (16, 1), (17, 2), (31, 1)])
+@pytest.mark.parametrize("track", ["diffusion", "single"])
+def test_fewest_tokens_equal_rows_of_a_large_call(N, samples, track):
+    """The smallest calls, all of whose products are launches for few tokens, against a call that has none of these."""
+    g = torch.Generator().manual_seed(N + samples)
+    many = (801 if track == "diffusion" else 1601) // N + 1
+    c = 768 if track == "diffusion" else 384
+    a, s = (torch.randn(many, N, k, generator=g).to("cuda:0", torch.bfloat16) for k in (c, 384))
+    z = torch.randn(1, N, N, 128, generator=g).to("cuda:0", torch.bfloat16)
+    m = (torch.rand(1, N, generator=g) < 0.9).to("cuda:0", torch.bfloat16)
+    m[:, 0] = 1
+    if track == "diffusion":
+        blk = _diffusion_block(g)
+        run = lambda k: blk(a[None, :k].contiguous(), s[None, :k].contiguous(), z[None], mask=m[None])[0]  # noqa: E731
+    else:
+        layer = pkg.AttentionPairBias(c_q=c, c_k=c, c_v=c, c_s=None, c_z=128, c_hidden=24, no_heads=16)
+        up = pkg.SwiGLUTransition(c_in=c, n=4)
+        with torch.no_grad():
+            for p in (*layer.parameters(), *up.parameters()):
+                p.copy_(torch.randn(p.shape, generator=g) * (0.05 if p.dim() > 1 else 0.3) + (1.0 if p.dim() == 1 else 0.0))
+        layer, up = (x.to("cuda:0", torch.bfloat16).eval().requires_grad_(False) for x in (layer, up))
+
+        def run(k):
+            zk, mk = z.expand(k, -1, -1, -1).contiguous(), m.expand(k, -1).contiguous()
+            x = a[:k] + layer(a[:k].contiguous(), zk, mask=mk)
+            return x + up(x, mask=mk)
+    with torch.no_grad():
+        want, got = run(many)[:samples], run(samples)
+    pkg.lib.check_device_status()
+    assert torch.isfinite(got).all() and got.any() and torch.equal(got, want)
