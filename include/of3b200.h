@@ -240,7 +240,7 @@ int of3_cond_transition_forward(const void* a, const void* s, const void* mask, 
  * stream before the first block and stream wait for side_stream after the last one (of3_stream_wait), and gives the
  * single track a workspace of its own. OF3_FLAG_LAST tells that no block follows: the single track then takes launches
  * that spread over the chip. OF3_FLAG_BIAS_SLOT(k): which of the workspace's rooms for the projected pair bias this block
- * takes (where it has four; else the first). Before it takes the first one, stream waits for side_stream, whose last single
+ * takes (where it has four, of up to 8 MB each; else the first). Before it takes the first one, stream waits for side_stream, whose last single
  * track may still read it; before the others it does not: they belong to the second to fourth block of a run whose first
  * took slot 0, or to the first blocks after stream has waited for side_stream. */
 typedef struct {

@@ -71,12 +71,16 @@ BiasForm bias_form(const of3_block_dims& D, int dtype, int flags) {
 }
 // Rooms for the projected bias in a block's workspace. With one, every block's projection waits for the single track of the block
 // ahead, which ended long before; but a wait for another stream takes the place of the chain between two kernels (N = 256: 5.9 instead
-// of 1.1 us). Trunk, one room / four, us: 4 blocks of 128 474 / 460, 256 1229 / 1217, 384 2428 / 2407, 12 of 256 3562 / 3475.
+// of 1.1 us). Trunk, one room / four, us: 4 blocks of 128 474 / 460, 256 1229 / 1217, 384 2428 / 2407, 12 of 256 3562 / 3475, 8 of 320
+// 3764 / 3748, 448 7326 / 7248, 512 8960 / 8856. Where a room is larger (16 N^2 values: 8 MB at 512) one: 640 15033 / 15041, 768 23017 /
+// 23062, and three more would be 57 MB at 768, 0.4 GB at 2048.
 constexpr int kBiasSlots = 4;
+constexpr size_t kBiasSlotMost = 8 << 20;
 size_t bias_bytes(const of3_block_dims& D, BiasForm f) {
     if (f == kBiasTiles) return (size_t)D.B * of3_pair_bias_tiles_elems(D.N) * sizeof(__nv_bfloat16);
     return f == kBiasF32 ? (size_t)D.B * D.no_heads_single * D.N * D.N * sizeof(float) : 0;
 }
+size_t rooms_bytes(size_t one) { return (one <= kBiasSlotMost ? kBiasSlots : 1) * align_up(one, 256); }
 
 int project_bias(const void* z, void* bias, const of3_block_dims& D, BiasForm form, const of3_attn_pair_bias_params* p,
                  cudaStream_t st) {
@@ -301,7 +305,7 @@ size_t of3_pairformer_block_workspace_bytes(const of3_block_dims* dims, int dtyp
         return ws.need + 256;
     }
     if (pair_block(nullptr, nullptr, *dims, dtype, flags, &p.pair, ws, nullptr)) return 0;
-    return align_up(ws.need, 256) + (form == kBiasInLayer ? 0 : kBiasSlots * align_up(bias_bytes(*dims, form), 256)) + 256;
+    return align_up(ws.need, 256) + rooms_bytes(bias_bytes(*dims, form)) + 256;
 }
 
 int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, const void* pair_mask,
@@ -322,9 +326,10 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
     Scratch sizing{nullptr, 0};
     int slot = side_stream != nullptr ? (flags >> 8) & (kBiasSlots - 1) : 0;
     size_t tail = one;
-    if (form != kBiasInLayer && pair_block(nullptr, nullptr, *dims, dtype, flags, &p->pair, sizing, nullptr) == OF3_OK &&
-        whole.cap >= align_up(sizing.need, 256) + kBiasSlots * align_up(one, 256))
-        tail = kBiasSlots * align_up(one, 256);
+    if (form != kBiasInLayer && one <= kBiasSlotMost &&
+        pair_block(nullptr, nullptr, *dims, dtype, flags, &p->pair, sizing, nullptr) == OF3_OK &&
+        whole.cap >= align_up(sizing.need, 256) + rooms_bytes(one))
+        tail = rooms_bytes(one);
     else
         slot = 0;
     const size_t head = (whole.cap - tail) / 256 * 256;
@@ -339,7 +344,7 @@ int of3_pairformer_block_forward(void* s, void* z, const void* single_mask, cons
     }
     // The pair stack never reads s, so the single track (a chain of small, launch-bound kernels) runs on the side
     // stream under the next block's pair stack. What it needs of z, the pair bias, is projected here, before the next
-    // block overwrites z, into the one bias buffer: behind the previous block's single track, which read it.
+    // block overwrites z, into a room of its own, or into the first: behind the single tracks that read it.
     cudaStream_t side = (cudaStream_t)side_stream;
     if (slot == 0 && (rc = stream_wait(main, side))) return rc;
     if ((rc = project_bias(z, bias, *dims, form, &p->attn, main))) return rc;

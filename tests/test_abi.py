@@ -63,6 +63,19 @@ def test_only_the_ending_node_asks_for_mask_rows(pkg, B, N, c):
     assert up(start, 256) + B * N * up(N, 64) * 2 == end
 
 
+@pytest.mark.parametrize("dt,bytes_per,N,rooms", [(0, 2, 512, 4), (0, 2, 544, 1), (0, 2, 768, 1), (0, 2, 2048, 1),
+                                                  (1, 4, 362, 4), (1, 4, 363, 1), (1, 4, 1024, 1)])
+def test_rooms_for_the_pair_bias_in_a_workspace(pkg, dt, bytes_per, N, rooms):
+    """Beside the layers' own: four of 16 N^2 values up to 8 MB each, one above."""
+    lib = pkg.lib
+    d = lib.BlockDims(B=1, N=N, c_z=128, c_hidden_mul=128, no_heads_pair=4, c_hidden_pair_att=32, pair_transition_n=4, c_s=384,
+                      no_heads_single=16, c_hidden_single=24, single_transition_n=4, inf_pair=1e9, inf_single=1e9)
+    pair = lib.load().of3_pair_block_workspace_bytes(ctypes.byref(d), dt, 0)
+    both = lib.load().of3_pairformer_block_workspace_bytes(ctypes.byref(d), dt, 0, 0)
+    room = 16 * N * N * bytes_per
+    assert pair > 0 and 0 <= both - pair - rooms * room < (rooms + 2) * 256
+
+
 def test_no_cpu_fallback(pkg):
     """CPU tensors are refused: there is no path that avoids the CUDA library."""
     m = pkg.TriangleMultiplicationOutgoing(128, 128).eval()
