@@ -968,8 +968,10 @@ int launch(Args<T> p, int groups, int batch, cudaStream_t st) {
     if constexpr (std::is_same<T, float>::value) {
         // Tensor cores once the small tiles of the FMA kernel would come in more than four waves. Device time, us, FMA / tensor, cold:
         // 576 rows: 4 x 128 columns 7.8 / 11.9; 2304 rows: 128 columns 8.0 / 12.4 (two waves), 4 x 128 22.3 / 12.5 (eight)
-        // (silu * up later: block of 25 tokens, 640 tiles, 314.5 / 320.2; of 26, 704, 310.4 / 311.4; of 27, 736, 311.2 / 303.9)
-        if (5 * tiles(32, kPaired ? 16 : 32) > (EPI == kSwiglu ? 24 : 20) * sm_count() && p.K < 1 << 17) {
+        // (silu * up of short k later, for the sake of blocks: trunk of 25 tokens (k = 128, 640 tiles) 310.3 / 317.6, 26 (704) 305.8 / 309.0,
+        // template of 49 (k = 64, 608) 350 / 352, but 51 (656) 348 / 344. Of longer k not: a transition alone of 192 channels, 445 rows,
+        // 51.5 / 33.8; 256, 317 50.7 / 39.3; 384, 200 90.7 / 54.1; 768, 221 125.2 / 108.7)
+        if (5 * tiles(32, kPaired ? 16 : 32) > (EPI == kSwiglu && p.K <= 128 ? 24 : 20) * sm_count() && p.K < 1 << 17) {
             bool whole = p.K % 64 == 0;
             if (!K_OUTER) {
                 whole = whole && (reinterpret_cast<uintptr_t>(p.a) & 15) == 0 && (p.a_batch & 3) == 0;
