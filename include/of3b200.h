@@ -9,8 +9,9 @@
  *    > 0 a cudaError_t. of3_last_error_string() describes the last failure of the calling
  *    thread. Nothing throws or aborts.
  *  - dtype: OF3_DTYPE_BF16 (bf16 storage, fp32 accumulation and statistics) or
- *    OF3_DTYPE_F32 (fp32 storage and fp32 arithmetic: the validation mode). Activations,
- *    masks and parameters of one call share the dtype.
+ *    OF3_DTYPE_F32 (fp32 storage and fp32 arithmetic, large products as sums of bf16 products
+ *    that are no further from the exact value: the validation mode). Activations, masks and
+ *    parameters of one call share the dtype.
  *  - Every buffer is owned by the caller. Entry points enqueue work on `stream` and return;
  *    they allocate nothing (except a 64-byte per-device status block on first use) and keep
  *    no reference after the enqueued work completes. `workspace` must hold at least the
